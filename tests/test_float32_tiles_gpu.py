@@ -1,11 +1,12 @@
-"""The 32-bit kernels that work in register tiles, alone: the product at the edges of its tiles and of its slices of k."""
+"""The 32-bit kernels that work in register tiles, alone: the product at the edges of its tiles and of its slices of k, and
+the attention over rows with several tokens against the general kernel and a plain float64 attention."""
 
 import math
 
 import pytest
 import torch
 
-from test_kernels_gpu import ops, rand  # noqa: F401  (ops: a fixture)
+from test_kernels_gpu import build_paged_case, ops, rand, ref_attention_row, tiles_for  # noqa: F401  (ops: a fixture)
 
 pytestmark = pytest.mark.gpu
 
@@ -23,3 +24,36 @@ def test_product_at_tile_edges(ops, cuda_device, M, N, K):
     wide = torch.full((M, N + 3), 7.0, device=cuda_device)
     ops.gemm_nt_simt(rand((M, K), torch.float32, cuda_device, 1).repeat(1, 2)[:, :K], w, out=wide[:, :N])
     assert torch.equal(wide[:, :N], got) and bool((wide[:, N:] == 7.0).all())
+
+
+@pytest.mark.parametrize("nh,nkv,hd,page,window,chunk,softcap,sink", [
+    (4, 2, 16, 4, 0, 0, 0.0, False), (16, 8, 128, 16, 0, 0, 0.0, False), (6, 2, 64, 8, 24, 0, 0.0, True),
+    (9, 1, 68, 16, 0, 40, 0.0, False), (40, 1, 112, 16, 0, 0, 5.0, True), (3, 3, 100, 32, 70, 0, 0.0, False)])
+def test_attention_against_the_general_kernel(ops, cuda_device, nh, nkv, hd, page, window, chunk, softcap, sink):
+    q_lens, ctx = [1, 37, 2, 150, 64, 129], [130, 0, 63, 3, 64, 200]
+    q, cache, meta, Ks, Vs, qs = build_paged_case(cuda_device, torch.float32, nh, nkv, hd, page, q_lens, ctx, 100)
+    sinks = rand((nh,), torch.float32, cuda_device, 5) if sink else None
+    status = ops.new_status(cuda_device)
+    common = (meta["row_q_start"], meta["row_q_len"], meta["row_ctx"], nh, nkv, hd, window, 1 / math.sqrt(hd), status)
+    masks = dict(chunk=chunk, sinks=sinks, softcap=softcap)
+    tokens = ops.attention_tile_tokens(nh // nkv)
+    general = ops.paged_attention(q, cache, meta["table"], *tiles_for(q_lens, tokens, cuda_device), tokens, *common, **masks)
+    wide = ops.paged_prefill_tile_tokens()
+    out = torch.full_like(q, 7.0)
+    ops.paged_attention_f32(q, cache, meta["table"], *tiles_for(q_lens, wide, cuda_device, only_multi=True), wide, *common, out, **masks)
+    ops.check_status(status)
+    assert bool((out[:1] == 7.0).all())                   # the single token is another kernel's
+    # Two float32 softmax averages of values around one: a few roundings of the scores' products and of the sums.
+    assert (out[1:] - general[1:]).abs().max() <= 2e-5
+    if not (chunk or softcap or sink):
+        got, cursor = out.double().cpu().view(-1, nh, hd), 0
+        for r, n in enumerate(q_lens):
+            expected = ref_attention_row(qs[r].double(), Ks[r].double(), Vs[r].double(), ctx[r], n, window, nh, nkv)
+            assert n == 1 or (got[cursor:cursor + n] - expected).abs().max() <= 4e-5
+            cursor += n
+
+
+def test_attention_refuses_what_it_does_not_take(ops):
+    assert ops.paged_attention_f32_supported(64, 1, 128, torch.float32)
+    for nh, nkv, hd, dtype in ((65, 1, 64, torch.float32), (4, 2, 132, torch.float32), (4, 2, 30, torch.float32), (4, 2, 64, torch.bfloat16)):
+        assert not ops.paged_attention_f32_supported(nh, nkv, hd, dtype)

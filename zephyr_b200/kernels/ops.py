@@ -101,6 +101,10 @@ _SIGNATURES = {
                                 c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                                 c_int, c_float, c_float, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p,
                                 c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p],
+    "zb_paged_attention_f32_supported": [c_int, c_int, c_int],
+    "zb_paged_attention_f32": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
+                               c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p,
+                               c_void_p, c_void_p],
     "zb_heads_attention_tile_tokens": [c_int, c_int, c_int, c_int, c_int],
     "zb_heads_attention_tile_keys": [c_int, c_int, c_int, c_int],
     "zb_heads_attention": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
@@ -1063,6 +1067,33 @@ def paged_attention(q: torch.Tensor, kv_cache: torch.Tensor, block_table: torch.
         int(shared_kv), _ptr(head_slopes), _ptr(sinks), int(keep_first), int(pool), _ptr(pool_cache),
         _ptr(pool_table), pool_blocks, pool_pages, int(cross_values), int(out_dtype == torch.float32 and q.dtype != torch.float32),
         _ptr(r1), _ptr(r2), _ptr(score_mix), DTYPE_CODE[q.dtype], _ptr(status), _stream()), "paged_attention")
+    return out
+
+
+def paged_attention_f32_supported(nh: int, nkv: int, hd: int, dtype: torch.dtype) -> bool:
+    """True if the tiled 32-bit kernel takes this shape: float32, heads of a multiple of 4 up to 128, up to 64 query
+    heads per key/value head."""
+    return dtype == torch.float32 and bool(library().zb_paged_attention_f32_supported(nh, nkv, hd))
+
+
+def paged_attention_f32(q: torch.Tensor, kv_cache: torch.Tensor, block_table: torch.Tensor, tile_row: torch.Tensor,
+                        tile_q0: torch.Tensor, tile_tokens: int, row_q_start: torch.Tensor, row_q_len: torch.Tensor,
+                        row_ctx: torch.Tensor, nh: int, nkv: int, hd: int, window: int, scale: float, status: torch.Tensor,
+                        out: torch.Tensor, chunk: int = 0, sinks: torch.Tensor | None = None, softcap: float = 0.0) -> torch.Tensor:
+    """What ``paged_attention`` does in float32, for rows that bring several tokens (tiles of ``tile_tokens`` tokens, which
+    the kernel cuts among its CTAs): causal, with a window, a chunked mask, sinks and a bound on the scores."""
+    _cuda(q, kv_cache, block_table, tile_row, tile_q0, row_q_start, row_q_len, row_ctx, status, sinks, out)
+    _i32(block_table, tile_row, tile_q0, row_q_start, row_q_len, row_ctx)
+    _require(sinks is None or (sinks.dtype == torch.float32 and sinks.is_contiguous() and sinks.numel() == nh),
+             "one float32 sink per query head")
+    _require(q.dim() == 2 and q.is_contiguous() and q.shape[1] == nh * hd and q.dtype == torch.float32, "q must be float32 [T, heads * hd]")
+    _require(out.shape == q.shape and out.dtype == torch.float32 and out.is_contiguous(), "out must be like q")
+    pages, page_size = _cache_geometry(kv_cache, nkv, hd, hd, torch.float32)
+    _check(library().zb_paged_attention_f32(
+        _ptr(out), _ptr(q), _ptr(kv_cache), _ptr(block_table), block_table.shape[1], page_size, pages, block_table.shape[0],
+        _ptr(tile_row), _ptr(tile_q0), tile_row.numel(), int(tile_tokens), _ptr(row_q_start), _ptr(row_q_len), _ptr(row_ctx),
+        nh, nkv, hd, int(window), int(chunk), float(scale), float(softcap), _ptr(sinks), _ptr(status), _stream()),
+        "paged_attention_f32")
     return out
 
 

@@ -66,6 +66,10 @@ from .base import POSITION_ENCODINGS, Mixer, StepContext, lookup, register_mixer
 class Attention(Mixer):
     graph_safe = True
 
+    # New tokens per request, on average, from which on a float32 step's rows with several tokens run in tiles of 64
+    # query rows: below, most of a tile would be empty (see csrc/attention_f32.cu).
+    FLOAT32_TILES_FROM = 16
+
     def __init__(self, spec: MixerSpec, weights: Mapping[str, torch.Tensor], dtype: torch.dtype,
                  device: torch.device | str):
         p = spec.params
@@ -186,6 +190,7 @@ class Attention(Mixer):
         # tokens a second at 8 requests, 11305 against 11143 at 64.
         self.fuse_decode_rows = 32
         self.fast_prefill = self.score_slopes is None and ops.paged_prefill_supported(self.nh, self.nkv, self.hd, dtype)
+        self.float32_tiles = self.score_slopes is None and ops.paged_attention_f32_supported(self.nh, self.nkv, self.hd, dtype)
         self.prefill_tile_tokens = ops.paged_prefill_tile_tokens()
 
     def _init_general(self, p) -> None:
@@ -224,6 +229,8 @@ class Attention(Mixer):
             self.heads_tile_tokens = ops.heads_attention_tile_tokens(self.nh, self.nkv, self.hd, self.vd, self.dtype)
         self.fast_decode = equal and not self.windowed and ops.paged_decode_supported(self.nh, self.nkv, self.hd, self.dtype)
         self.fast_prefill = equal and ops.paged_prefill_supported(self.nh, self.nkv, self.hd, self.dtype)
+        self.float32_tiles = (equal and not self.windowed and self.distance_bias is None and self.score_mix is None
+                              and ops.paged_attention_f32_supported(self.nh, self.nkv, self.hd, self.dtype))
         self.prefill_tile_tokens = ops.paged_prefill_tile_tokens()
 
     def score_slopes_wanted(self) -> bool:
@@ -360,6 +367,12 @@ class Attention(Mixer):
                                   *common, out=out, **masks)
         if decode_done and prefill_done:
             return out
+        if self.float32_tiles and q.shape[0] >= self.FLOAT32_TILES_FROM * ctx.num_rows:
+            tile_row, tile_q0 = ctx.tiles[(self.prefill_tile_tokens, "multi")]
+            prefill_done = True
+            if tile_row.numel() > 0:
+                ops.paged_attention_f32(q, cache, table, tile_row, tile_q0, self.prefill_tile_tokens, ctx.row_q_start, ctx.row_q_len,
+                                        ctx.row_ctx, *common, out=out, **masks)
         which = "multi" if decode_done else ("single" if prefill_done else "all")
         tile_row, tile_q0 = ctx.tiles[(self.tile_tokens, which)]
         if tile_row.numel() > 0:
