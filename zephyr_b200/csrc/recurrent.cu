@@ -288,17 +288,49 @@ __global__ void causal_conv_silu_kernel(const ConvArgs a, const int* token_row, 
   }
 }
 
-// The form that runs wherever the shapes allow it (bfloat16, an even number of channels, aligned rows):
-// a CTA takes CONV_TILE consecutive tokens of the stream and 128 channels, a thread two adjacent
-// channels, which it walks down the tile with the last inputs in registers: one 4-byte load and one
-// 4-byte store a token.  Where a tile crosses from one request to the next the window starts again
-// from that request's state.  The tile's rows, slots and first tokens are looked up once, into shared
-// memory.
-constexpr int CONV_TILE = 32;
+// The form for runs of tokens (rows that start on a vector's boundary): a CTA takes CONV_RUN consecutive tokens of the
+// stream, a thread VEC neighbouring channels of them.  Bound by latency where a thread walks its tokens one load
+// behind the other, so it asks for all its inputs, the TAPS - 1 before the first token among them, before it uses any
+// (they come again from the cache for the next CTA); inputs before a request's first new token come from its state.
+// TAPS: the taps of the kernel, `taps` of them in use (the others, at the old end, are skipped).
+constexpr int CONV_RUN = 8;
 
-__global__ void __launch_bounds__(64) causal_conv_silu_tile_kernel(const ConvArgs a, const int* token_row, int tokens) {
-  __shared__ int first_s[CONV_TILE], slot_s[CONV_TILE];       // per token: index within its request's new tokens, slot
-  const int t0 = blockIdx.x * CONV_TILE, nt = min(CONV_TILE, tokens - t0);
+template <typename T, int VEC>
+__device__ __forceinline__ void conv_load(float (&x)[VEC], const T* p) {
+  if constexpr (VEC == 4) {
+    const float4 v = load4(p);
+    x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+  } else if constexpr (sizeof(T) == 4) {
+    const float2 v = *reinterpret_cast<const float2*>(p);
+    x[0] = v.x; x[1] = v.y;
+  } else {
+    const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
+    x[0] = v.x; x[1] = v.y;
+  }
+}
+template <typename T, int VEC>
+__device__ __forceinline__ void conv_store(T* p, const float (&y)[VEC]) {
+  if constexpr (VEC == 4) store4(p, make_float4(y[0], y[1], y[2], y[3]));
+  else if constexpr (sizeof(T) == 4) *reinterpret_cast<float2*>(p) = make_float2(y[0], y[1]);
+  else *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(y[0], y[1]);
+}
+
+template <typename T, int VEC, int TAPS>
+__global__ void __launch_bounds__(128) causal_conv_silu_run_kernel(const ConvArgs a, const int* token_row, int tokens) {
+  __shared__ int first_s[CONV_RUN], slot_s[CONV_RUN];         // per token: index within its request's new tokens, slot
+  const int t0 = blockIdx.x * CONV_RUN, nt = min(CONV_RUN, tokens - t0);
+  const int c = (blockIdx.y * blockDim.x + threadIdx.x) * VEC;
+  const bool works = c < a.C;
+  const int skipped = TAPS - a.taps;
+  const T* x = static_cast<const T*>(a.x);
+  float in[TAPS - 1 + CONV_RUN][VEC];
+#pragma unroll
+  for (int i = 0; i < TAPS - 1 + CONV_RUN; ++i) {
+    const int t = t0 - (TAPS - 1) + i;
+#pragma unroll
+    for (int v = 0; v < VEC; ++v) in[i][v] = 0.0f;
+    if (works && i >= skipped && t >= 0 && t < tokens) conv_load<T, VEC>(in[i], x + t * a.x_stride + c);
+  }
   if (threadIdx.x < nt) {
     const int row = token_row[t0 + threadIdx.x];
     const int slot = a.slots[row];
@@ -306,56 +338,59 @@ __global__ void __launch_bounds__(64) causal_conv_silu_tile_kernel(const ConvArg
     slot_s[threadIdx.x] = slot;
     if (slot < 0 || slot >= a.num_slots) report(a.status, STATUS_ROW_OUT_OF_RANGE, slot, row);
   }
-  __syncthreads();
-  const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 2;
-  if (c >= a.C) return;
-  const int first = CONV_MAX_TAPS - a.taps;
   const float* wp = static_cast<const float*>(a.w);
-  float w[CONV_MAX_TAPS][2], win[CONV_MAX_TAPS][2];
+  float w[TAPS][VEC], bias[VEC];
 #pragma unroll
-  for (int j = 0; j < CONV_MAX_TAPS; ++j) {
-    w[j][0] = j >= first ? wp[c * a.taps + (j - first)] : 0.0f;
-    w[j][1] = j >= first ? wp[(c + 1) * a.taps + (j - first)] : 0.0f;
-    win[j][0] = win[j][1] = 0.0f;
+  for (int v = 0; v < VEC; ++v) {
+    bias[v] = works ? static_cast<const float*>(a.bias)[c + v] : 0.0f;
+#pragma unroll
+    for (int j = 0; j < TAPS; ++j) w[j][v] = works && j >= skipped ? wp[(c + v) * a.taps + (j - skipped)] : 0.0f;
   }
-  const float bias0 = static_cast<const float*>(a.bias)[c], bias1 = static_cast<const float*>(a.bias)[c + 1];
-  const __nv_bfloat16* x = static_cast<const __nv_bfloat16*>(a.x);
-  __nv_bfloat16* out = static_cast<__nv_bfloat16*>(a.out);
-  for (int k = 0; k < nt; ++k) {
+  __syncthreads();
+  if (!works) return;
+  T* out = static_cast<T*>(a.out);
+#pragma unroll
+  for (int k = 0; k < CONV_RUN; ++k) {
+    if (k >= nt) break;
     const int i = first_s[k], slot = slot_s[k];
     if (slot < 0 || slot >= a.num_slots) continue;
-    if (k == 0 || i == 0) {
-      // The window before this token: inputs i - taps + 1 .. i - 1, from x or, before the request's first
-      // new token, from its state.  win[j + 1] is what win[j] will be after the shift below.
+    float acc[VEC];
+#pragma unroll
+    for (int v = 0; v < VEC; ++v) acc[v] = 0.0f;
+    if (i >= TAPS - 1) {
+#pragma unroll
+      for (int j = 0; j < TAPS; ++j)
+        if (j >= skipped) {
+#pragma unroll
+          for (int v = 0; v < VEC; ++v) acc[v] = fmaf(w[j][v], in[k + j][v], acc[v]);
+        }
+    } else {
       const float* state = a.state + static_cast<long long>(slot) * a.slot_stride;
 #pragma unroll
-      for (int j = 0; j < CONV_MAX_TAPS; ++j) {
-        if (j > first) {
-          const int back = CONV_MAX_TAPS - j;          // win[j] holds the input `back` tokens before this one
-          if (i - back >= 0) {
-            const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(
-                x + static_cast<long long>(t0 + k - back) * a.x_stride + c));
-            win[j][0] = v.x; win[j][1] = v.y;
-          } else {
-            const float2 v = *reinterpret_cast<const float2*>(state + static_cast<long long>(a.taps - 1 + i - back) * a.C + c);
-            win[j][0] = v.x; win[j][1] = v.y;
-          }
+      for (int j = 0; j < TAPS; ++j)
+        if (j >= skipped) {
+          const int back = TAPS - 1 - j;
+#pragma unroll
+          for (int v = 0; v < VEC; ++v)
+            acc[v] = fmaf(w[j][v], i >= back ? in[k + j][v] : state[static_cast<long long>(a.taps - 1 + i - back) * a.C + c + v], acc[v]);
         }
-      }
     }
 #pragma unroll
-    for (int j = 0; j + 1 < CONV_MAX_TAPS; ++j) { win[j][0] = win[j + 1][0]; win[j][1] = win[j + 1][1]; }
-    const float2 now = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(
-        x + static_cast<long long>(t0 + k) * a.x_stride + c));
-    win[CONV_MAX_TAPS - 1][0] = now.x; win[CONV_MAX_TAPS - 1][1] = now.y;
-    float acc0 = 0.0f, acc1 = 0.0f;
-#pragma unroll
-    for (int j = 0; j < CONV_MAX_TAPS; ++j) {
-      acc0 = fmaf(w[j][0], win[j][0], acc0);
-      acc1 = fmaf(w[j][1], win[j][1], acc1);
-    }
-    *reinterpret_cast<__nv_bfloat162*>(out + static_cast<long long>(t0 + k) * a.C + c) =
-        __floats2bfloat162_rn(silu_f(acc0 + bias0), silu_f(acc1 + bias1));
+    for (int v = 0; v < VEC; ++v) acc[v] = silu_f(acc[v] + bias[v]);
+    conv_store<T, VEC>(out + static_cast<long long>(t0 + k) * a.C + c, acc);
+  }
+}
+
+template <typename T>
+static void conv_run_launch(const ConvArgs& a, const int* token_row, int tokens, bool four, cudaStream_t s) {
+  const int vectors = a.C / (four ? 4 : 2);
+  const dim3 grid((tokens + CONV_RUN - 1) / CONV_RUN, (vectors + 127) / 128);
+  if (a.taps <= 4) {
+    if (four) causal_conv_silu_run_kernel<T, 4, 4><<<grid, 128, 0, s>>>(a, token_row, tokens);
+    else causal_conv_silu_run_kernel<T, 2, 4><<<grid, 128, 0, s>>>(a, token_row, tokens);
+  } else {
+    if (four) causal_conv_silu_run_kernel<T, 4, 8><<<grid, 128, 0, s>>>(a, token_row, tokens);
+    else causal_conv_silu_run_kernel<T, 2, 8><<<grid, 128, 0, s>>>(a, token_row, tokens);
   }
 }
 
@@ -940,19 +975,20 @@ ZB_API int zb_causal_conv_silu(void* out, const void* x, long long x_stride, flo
   auto s = static_cast<cudaStream_t>(stream);
   if (tokens <= 0) return OK;
   const dim3 grid((tokens + CONV_TOKENS - 1) / CONV_TOKENS, (C + 127) / 128), per_row((C + 127) / 128, rows);
+  // Runs pay where requests bring several tokens; a step of single tokens has nothing to share.
+  auto aligned = [&](int vec) {
+    const size_t bytes = vec * (dtype == DTYPE_F32 ? 4 : 2);
+    return C % vec == 0 && x_stride % vec == 0 && w_dtype == DTYPE_F32 && reinterpret_cast<uintptr_t>(x) % bytes == 0 &&
+           reinterpret_cast<uintptr_t>(out) % bytes == 0;
+  };
+  const bool runs = tokens >= 4 * rows && aligned(2);
   if (dtype == DTYPE_F32) {
-    causal_conv_silu_kernel<float><<<grid, 128, 0, s>>>(a, token_row, tokens);
+    if (runs) conv_run_launch<float>(a, token_row, tokens, aligned(4), s);
+    else causal_conv_silu_kernel<float><<<grid, 128, 0, s>>>(a, token_row, tokens);
     if (write_state && taps > 1) conv_state_update_kernel<float><<<per_row, 128, 0, s>>>(a);
   } else {
-    const bool pairs = C % 2 == 0 && x_stride % 2 == 0 && slot_stride % 2 == 0 && w_dtype == DTYPE_F32 &&
-                       reinterpret_cast<uintptr_t>(x) % 4 == 0 && reinterpret_cast<uintptr_t>(out) % 4 == 0 &&
-                       reinterpret_cast<uintptr_t>(state) % 8 == 0;
-    // Tiles pay where requests bring runs of tokens; a step of single tokens has nothing to slide over.
-    if (pairs && tokens >= 4 * rows)
-      causal_conv_silu_tile_kernel<<<dim3((tokens + CONV_TILE - 1) / CONV_TILE, (C / 2 + 63) / 64), 64, 0, s>>>(
-          a, token_row, tokens);
-    else
-      causal_conv_silu_kernel<__nv_bfloat16><<<grid, 128, 0, s>>>(a, token_row, tokens);
+    if (runs) conv_run_launch<__nv_bfloat16>(a, token_row, tokens, aligned(4), s);
+    else causal_conv_silu_kernel<__nv_bfloat16><<<grid, 128, 0, s>>>(a, token_row, tokens);
     if (write_state && taps > 1) conv_state_update_kernel<__nv_bfloat16><<<per_row, 128, 0, s>>>(a);
   }
   return launch_result();
