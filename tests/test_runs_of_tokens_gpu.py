@@ -36,3 +36,36 @@ def test_convolution_over_runs(cuda_device, dtype, channels, taps, offset):
         assert (out[start:start + n].double() - expected).abs().max() <= bound * max(1.0, float(expected.abs().max()))
         if taps > 1:
             assert torch.equal(state[slot].view(taps - 1, channels).double(), inputs[len(inputs) - taps + 1:])
+
+
+def test_the_delta_rule_on_both_paths(cuda_device):
+    """A step whose rows bring runs goes block by block, single tokens one by one: a request cut either way ends in the
+    same outputs and the same state, also where keys repeat (the block's matrix is then far from the unit matrix) and
+    where a decay is so strong that a block forgets its start."""
+    from zephyr_b200.kernels import ops
+
+    heads, groups, dim, vdim, T = 4, 2, 128, 128, 83
+    g = torch.Generator().manual_seed(5)
+    q, k, v = (torch.randn(T, n, generator=g).to(cuda_device) for n in (groups * dim, groups * dim, heads * vdim))
+    k[20:40] = k[20]                                       # one key twenty times over
+    ba = (torch.randn(T, 2 * heads, generator=g) * 1.5).to(cuda_device)
+    ba[50:53, heads:] = 60.0                               # decays of e^-60 and less
+    a_log, dt_bias = (torch.randn(heads, generator=g) * 0.5).to(cuda_device), torch.zeros(heads, device=cuda_device)
+    i32 = lambda values: torch.tensor(values, dtype=torch.int32, device=cuda_device)
+    status = ops.new_status(cuda_device)
+
+    def run(cuts):
+        state, out, at = torch.zeros(1, heads * dim * vdim, device=cuda_device), [], 0
+        for n in cuts:
+            part = slice(at, at + n)
+            out.append(ops.delta_rule(q[part], k[part], v[part], ba[part, :heads], ba[part, heads:], a_log, dt_bias, heads, groups,
+                                      dim, vdim, state, i32([0]), i32([0]), i32([n]), status, q_scale=dim ** -0.5))
+            at += n
+        ops.check_status(status)
+        return torch.cat(out), state
+
+    assert ops.DELTA_BLOCKS_FROM <= 17
+    single, blocks, mixed = run([1] * T), run([T]), run([17, 3, 30, 1, 32])
+    for other in (blocks, mixed):
+        for x, y in zip(single, other):       # float32 sums in another order
+            assert (x - y).abs().max() <= 1e-5 * max(1.0, float(x.abs().max()))

@@ -17,6 +17,9 @@
 //                 written back at its end, so a prompt may be cut anywhere.  In the slot a head's state
 //                 lies [V][D] (a column's channels together).
 //
+// Where requests bring runs of tokens, two other kernels take their place (delta_blocks, delta_block_scan below): the
+// same rule, block by block of 16 tokens.
+//
 // Everything here is float32; the values v are read in the model's type.
 #include "common.cuh"
 #include "mma.cuh"
@@ -299,6 +302,329 @@ __global__ void __launch_bounds__(DS_THREADS) delta_scan_kernel(const DeltaScanA
   }
 }
 
+// ------------------------------------------------------------------------------------------------ blocks of tokens
+// Token by token the recurrence is a chain: the state's read-out with k, u, the write, 0.26 us a token whatever the SMs
+// could do besides.  Over a block of B tokens, with S the state at its start, c_t the sum of the logarithms of the
+// decays up to token t, R_k = S^T k_t and R_q = S^T q_t,
+//
+//   v'_t = v_t - e^(c_t) R_k(t)
+//   u    = (I + A)^-1 diag(beta) v',   A_tj = beta_t e^(c_t - c_j) (k_t . k_j) for j < t
+//   o_t  = e^(c_t) R_q(t) + sum_{j <= t} e^(c_t - c_j) (q_t . k_j) u_j
+//   S   <- e^(c_B) S + sum_j e^(c_B - c_j) k_j u_j^T
+//
+// so the chain is one read-out and one write a block, both plain products.  All but the products with S and v' depends
+// on the block alone: delta_blocks makes, for all blocks side by side, the unit vectors (a block's k and q with their
+// tokens side by side, the layout that the products read) and per head
+//
+//   Tu = diag(e^(c_B - c_t)) (I + A)^-1 diag(beta)       (what the write takes is Tu v')
+//   M  = P (I + A)^-1 diag(beta),  P_tj = e^(c_t - c_j) (q_t . k_j)   (o = e^(c) R_q + M v')
+//
+// and delta_block_scan walks a request's blocks.  Exponents are differences of sums within a block, never positive.
+// Tokens behind a portion's end have beta 0 and decay 1.  Block p of row r has the number row_q_start[r] / B + r + p.
+constexpr int DB = 16;                     // tokens of a block
+constexpr int DB_THREADS = 256;
+constexpr int DB_COLS = 16;                // value columns of a CTA
+constexpr int DB_COEF = 2 * DB * DB + 2 * DB;      // Tu and M, both [j][t], e^(c_t), e^(c_B) and padding
+
+struct DeltaBlocksArgs {
+  float* qk;               // [blocks][qk_heads][DP][2 DB]: k of the block's tokens, then q
+  float* coef;             // [blocks][heads][DB_COEF]
+  const void* q; long long q_stride;
+  const void* k; long long k_stride;
+  const float* b; const float* a; long long ba_stride;
+  const float* a_log; const float* dt_bias;
+  const int* row_q_start; const int* row_q_len;
+  int rows, qk_heads, heads, D;
+  float q_scale, unit_eps;
+};
+
+// DP: the channels padded with zeros.
+template <typename T, int DP>
+__global__ void __launch_bounds__(DB_THREADS) delta_blocks_kernel(const DeltaBlocksArgs a) {
+  extern __shared__ __align__(16) float db_smem[];
+  constexpr int ST = DP + 1;
+  float* x_s = db_smem;                    // [2 DB][ST]: k, q
+  float* kk_s = x_s + 2 * DB * ST;         // [DB][DB]
+  float* qk_s = kk_s + DB * DB;
+  float* t_s = qk_s + DB * DB;             // [DB][DB]: (I + A)^-1 diag(beta)
+  float* c_s = t_s + DB * DB;              // [DB]
+  float* beta_s = c_s + DB;
+  __shared__ int found;
+  const int block = blockIdx.x, group = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) found = -1;
+  __syncthreads();
+  for (int r = tid; r < a.rows; r += DB_THREADS) {
+    const int p = block - (a.row_q_start[r] / DB + r);
+    if (p >= 0 && p * DB < a.row_q_len[r]) found = r;       // at most one row
+  }
+  __syncthreads();
+  const int row = found;
+  if (row < 0) return;
+  const int begin = (block - (a.row_q_start[row] / DB + row)) * DB, n = min(DB, a.row_q_len[row] - begin);
+  const long long t0 = a.row_q_start[row] + begin;
+  for (int i = warp; i < 2 * DB; i += DB_THREADS / 32) {
+    const bool is_q = i >= DB;
+    const int t = i % DB;
+    const T* src = is_q ? static_cast<const T*>(a.q) + (t0 + t) * a.q_stride + group * a.D
+                        : static_cast<const T*>(a.k) + (t0 + t) * a.k_stride + group * a.D;
+    float x[DP / 32], ss = 0.0f;
+#pragma unroll
+    for (int j = 0; j < DP / 32; ++j) {
+      const int d = lane + 32 * j;
+      x[j] = t < n && d < a.D ? to_float(src[d]) : 0.0f;
+      ss = fmaf(x[j], x[j], ss);
+    }
+    const float inv = (is_q ? a.q_scale : 1.0f) / sqrtf(warp_sum(ss) + a.unit_eps);
+#pragma unroll
+    for (int j = 0; j < DP / 32; ++j) x_s[i * ST + lane + 32 * j] = t < n ? x[j] * inv : 0.0f;
+  }
+  __syncthreads();
+  float4* to = reinterpret_cast<float4*>(a.qk + (static_cast<long long>(block) * a.qk_heads + group) * DP * 2 * DB);
+  for (int e = tid; e < DP * 2 * DB / 4; e += DB_THREADS) {
+    const int d = e / (2 * DB / 4), i = e % (2 * DB / 4) * 4;
+    to[e] = make_float4(x_s[i * ST + d], x_s[(i + 1) * ST + d], x_s[(i + 2) * ST + d], x_s[(i + 3) * ST + d]);
+  }
+  const int t = tid / DB, j = tid % DB;
+  {
+    float kk[2] = {0.0f, 0.0f}, qk[2] = {0.0f, 0.0f};
+    const float* kt = x_s + t * ST;
+    const float* qt = x_s + (DB + t) * ST;
+    const float* kj = x_s + j * ST;
+#pragma unroll 8
+    for (int d = 0; d < DP; ++d) {
+      kk[d & 1] = fmaf(kt[d], kj[d], kk[d & 1]);
+      qk[d & 1] = fmaf(qt[d], kj[d], qk[d & 1]);
+    }
+    kk_s[tid] = kk[0] + kk[1];
+    qk_s[tid] = qk[0] + qk[1];
+  }
+  const int per = a.heads / a.qk_heads;
+  for (int h = group * per; h < (group + 1) * per; ++h) {
+    __syncthreads();                       // the products are there, and the head before is done
+    if (tid < 32) {
+      float c = 0.0f, beta = 0.0f;
+      if (lane < n) {
+        const long long at = (t0 + lane) * a.ba_stride + h;
+        beta = 1.0f / (1.0f + expf(-a.b[at]));
+        c = -expf(a.a_log[h]) * softplus_d(a.a[at] + a.dt_bias[h]);
+      }
+#pragma unroll
+      for (int o = 1; o < DB; o <<= 1) {
+        const float before = __shfl_up_sync(0xffffffffu, c, o);
+        if (lane >= o) c += before;
+      }
+      if (lane < DB) {
+        c_s[lane] = c;
+        beta_s[lane] = beta;
+      }
+    }
+    __syncthreads();
+    float* coef = a.coef + (static_cast<long long>(block) * a.heads + h) * DB_COEF;
+    if (tid < DB) {
+      // A column of the inverse by forward substitution, times beta of the column.
+      float x[DB];
+#pragma unroll
+      for (int i = 0; i < DB; ++i) {
+        float sum = i == tid ? 1.0f : 0.0f;
+#pragma unroll
+        for (int m = 0; m < i; ++m) sum = fmaf(-beta_s[i] * expf(c_s[i] - c_s[m]) * kk_s[i * DB + m], x[m], sum);
+        x[i] = sum;
+      }
+      const float last = c_s[DB - 1];
+#pragma unroll
+      for (int i = 0; i < DB; ++i) {
+        t_s[i * DB + tid] = x[i] * beta_s[tid];
+        coef[tid * DB + i] = expf(last - c_s[i]) * x[i] * beta_s[tid];
+      }
+      coef[2 * DB * DB + tid] = expf(c_s[tid]);
+      if (tid == 0) coef[2 * DB * DB + DB] = expf(last);
+    }
+    __syncthreads();
+    float m = 0.0f;
+    for (int i = 0; i <= t; ++i) m = fmaf(expf(c_s[t] - c_s[i]) * qk_s[t * DB + i], t_s[i * DB + j], m);
+    coef[DB * DB + j * DB + t] = m;
+  }
+}
+
+struct DeltaBlockScanArgs {
+  float* out;              // [T, heads * V]
+  const float* qk;
+  const float* coef;
+  const void* v; long long v_stride;
+  float* state; long long slot_stride;     // slot s at state + s * slot_stride: [heads][V][D]
+  const int* slots; const int* row_q_start; const int* row_q_len;
+  int heads, qk_heads, D, V, num_slots, write_state;
+  int* status;
+};
+
+// A CTA owns a request, a head and DB_COLS value columns; its state lies in registers (two channels by four columns a
+// thread) and, for the read-outs, in shared memory.  A block: every warp forms the read-outs of all 32 rows (k and q)
+// over its share of the channels, 4 x 4 a thread; the warps' sums are added and v' made; u and o from the block's
+// matrices; the state.  The next block's operands are copied meanwhile.
+template <typename T, int DP>
+__global__ void __launch_bounds__(DB_THREADS) delta_block_scan_kernel(const DeltaBlockScanArgs a) {
+  extern __shared__ __align__(16) float db_smem[];
+  constexpr int QK_ST = 2 * DB + 4, S_ST = DB_COLS + 4, RED_ST = 2 * DB + 4;
+  constexpr int stage_floats = DP * QK_ST + DB_COEF;
+  float* stages = db_smem;                                   // two of [DP][QK_ST] and the coefficients
+  float* s_s = stages + 2 * stage_floats;                    // [DP][S_ST]
+  float* red_s = s_s + DP * S_ST;                            // [warps][DB_COLS][RED_ST]
+  float* vp_s = red_s + DB_THREADS / 32 * DB_COLS * RED_ST;  // [DB_COLS][DB]: v'
+  float* u_s = vp_s + DB_COLS * DB;                          // [DB][S_ST]: what the write takes
+  float* o_s = u_s + DB * S_ST;                              // [DB][S_ST]
+  const int row = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * DB_COLS;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int slot = a.slots[row];
+  if (slot < 0 || slot >= a.num_slots) {
+    if (tid == 0) report(a.status, STATUS_ROW_OUT_OF_RANGE, slot, row);
+    return;
+  }
+  const int n = a.row_q_len[row], blocks = (n + DB - 1) / DB;
+  const long long t0 = a.row_q_start[row];
+  const int first = a.row_q_start[row] / DB + row;
+  const int group = head / (a.heads / a.qk_heads);
+
+  auto copy_block = [&](int p, float* stage) {
+    const float* qk = a.qk + (static_cast<long long>(first + p) * a.qk_heads + group) * DP * 2 * DB;
+    for (int e = tid; e < DP * 2 * DB / 4; e += DB_THREADS) {
+      const int d = e / (2 * DB / 4), i = e % (2 * DB / 4) * 4;
+      cp_async_16(stage + d * QK_ST + i, qk + e * 4, true);
+    }
+    const float* coef = a.coef + (static_cast<long long>(first + p) * a.heads + head) * DB_COEF;
+    for (int e = tid; e < DB_COEF / 4; e += DB_THREADS) cp_async_16(stage + DP * QK_ST + e * 4, coef + e * 4, true);
+    cp_async_commit();
+  };
+  // This thread's token and column in the small products.
+  const int my_t = tid % DB, my_c = tid / DB;
+  const T* v = static_cast<const T*>(a.v) + t0 * a.v_stride + head * a.V + col0 + my_c;
+  auto fetch_v = [&](int p) {
+    const int t = p * DB + my_t;
+    return t < n && col0 + my_c < a.V ? to_float(v[t * a.v_stride]) : 0.0f;
+  };
+  // This thread's part of the state: channels d0 and d0 + 1, columns c0 .. c0 + 3.
+  const int d0 = tid / 4 * 2, c0 = tid % 4 * 4;
+  const bool holds = d0 < DP;
+  float S[2][4];
+  float* state = a.state + static_cast<long long>(slot) * a.slot_stride + (static_cast<long long>(head) * a.V + col0) * a.D;
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      S[i][c] = holds && d0 + i < a.D && col0 + c0 + c < a.V ? state[static_cast<long long>(c0 + c) * a.D + d0 + i] : 0.0f;
+  auto store_state = [&]() {
+    if (holds) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i) *reinterpret_cast<float4*>(s_s + (d0 + i) * S_ST + c0) = make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
+    }
+  };
+  store_state();
+  float v_now = 0.0f;
+  if (blocks > 0) {
+    copy_block(0, stages);
+    v_now = fetch_v(0);
+  }
+  for (int p = 0; p < blocks; ++p) {
+    const float* stage = stages + (p & 1) * stage_floats;
+    const float* coef = stage + DP * QK_ST;
+    cp_async_wait<0>();
+    __syncthreads();             // the block and the state are there; the other buffer is no longer read
+    float v_next = 0.0f;
+    if (p + 1 < blocks) {
+      copy_block(p + 1, stages + ((p + 1) & 1) * stage_floats);
+      v_next = fetch_v(p + 1);
+    }
+    {
+      const int i0 = (lane & 7) * 4, rc = (lane >> 3) * 4;
+      float acc[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
+#pragma unroll
+      for (int u = 0; u < DP / 8; ++u) {
+        const int d = warp * (DP / 8) + u;
+        float x[4], y[4];
+        *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(stage + d * QK_ST + i0);
+        *reinterpret_cast<float4*>(y) = *reinterpret_cast<const float4*>(s_s + d * S_ST + rc);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) acc[c][i] = fmaf(x[i], y[c], acc[c][i]);
+      }
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        *reinterpret_cast<float4*>(red_s + (warp * DB_COLS + rc + c) * RED_ST + i0) = make_float4(acc[c][0], acc[c][1], acc[c][2], acc[c][3]);
+    }
+    __syncthreads();
+    float rk = 0.0f, rq = 0.0f;
+#pragma unroll
+    for (int w = 0; w < DB_THREADS / 32; ++w) {
+      rk += red_s[(w * DB_COLS + my_c) * RED_ST + my_t];
+      rq += red_s[(w * DB_COLS + my_c) * RED_ST + DB + my_t];
+    }
+    const float lead = coef[2 * DB * DB + my_t], whole = coef[2 * DB * DB + DB];
+    vp_s[my_c * DB + my_t] = v_now - lead * rk;
+    __syncthreads();
+    {
+      float u = 0.0f, o = 0.0f;
+#pragma unroll
+      for (int j = 0; j < DB; j += 4) {
+        float x[4];
+        *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(vp_s + my_c * DB + j);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          u = fmaf(coef[(j + i) * DB + my_t], x[i], u);
+          o = fmaf(coef[DB * DB + (j + i) * DB + my_t], x[i], o);
+        }
+      }
+      u_s[my_t * S_ST + my_c] = u;
+      o_s[my_t * S_ST + my_c] = fmaf(lead, rq, o);
+    }
+    __syncthreads();
+    {
+      const int t = p * DB + tid / DB_COLS, c = tid % DB_COLS;
+      if (t < n && col0 + c < a.V)
+        a.out[(t0 + t) * a.heads * a.V + static_cast<long long>(head) * a.V + col0 + c] = o_s[tid / DB_COLS * S_ST + c];
+    }
+    if (holds) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) S[i][c] *= whole;
+#pragma unroll
+      for (int j = 0; j < DB; j += 4) {
+        float k0[4], k1[4];
+        *reinterpret_cast<float4*>(k0) = *reinterpret_cast<const float4*>(stage + d0 * QK_ST + j);
+        *reinterpret_cast<float4*>(k1) = *reinterpret_cast<const float4*>(stage + (d0 + 1) * QK_ST + j);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          float u[4];
+          *reinterpret_cast<float4*>(u) = *reinterpret_cast<const float4*>(u_s + (j + i) * S_ST + c0);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            S[0][c] = fmaf(k0[i], u[c], S[0][c]);
+            S[1][c] = fmaf(k1[i], u[c], S[1][c]);
+          }
+        }
+      }
+    }
+    store_state();               // (nobody reads the state's tile between the barriers above and the next one)
+    v_now = v_next;
+  }
+  if (!a.write_state || !holds) return;
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      if (d0 + i < a.D && col0 + c0 + c < a.V) state[static_cast<long long>(c0 + c) * a.D + d0 + i] = S[i][c];
+}
+
+template <int DP>
+constexpr size_t delta_blocks_smem() { return sizeof(float) * (2 * DB * (DP + 1) + 3 * DB * DB + 2 * DB); }
+template <int DP>
+constexpr size_t delta_block_scan_smem() {
+  return sizeof(float) * (2 * (DP * (2 * DB + 4) + DB_COEF) + DP * (DB_COLS + 4) + DB_THREADS / 32 * DB_COLS * (2 * DB + 4) +
+                          DB_COLS * DB + 2 * DB * (DB_COLS + 4));
+}
+
 }  // namespace zb
 
 using namespace zb;
@@ -373,4 +699,47 @@ ZB_API int zb_delta_scan(float* out, const float* q, const float* k, const void*
   auto s = static_cast<cudaStream_t>(stream);
   return dtype == DTYPE_F32 ? delta_scan_dispatch<float>(a, rows, tokens, s)
                             : delta_scan_dispatch<__nv_bfloat16>(a, rows, tokens, s);
+}
+
+// The blocks' form takes up to this many key channels per head.
+ZB_API int zb_delta_block_max_channels() { return 128; }
+ZB_API int zb_delta_block_tokens() { return DB; }
+// Floats of workspace a block needs: its unit vectors and its matrices.
+ZB_API int zb_delta_block_floats(int qk_heads, int heads, int D) { return qk_heads * (D <= 64 ? 64 : 128) * 2 * DB + heads * DB_COEF; }
+
+template <typename T, int DP>
+static int delta_block_launch(const DeltaBlocksArgs& b, const DeltaBlockScanArgs& a, int rows, int blocks, cudaStream_t s) {
+  constexpr int first = static_cast<int>(delta_blocks_smem<DP>()), second = static_cast<int>(delta_block_scan_smem<DP>());
+  if (cuda_failed(cudaFuncSetAttribute(delta_block_scan_kernel<T, DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, second)))
+    return ERR_CUDA;
+  delta_blocks_kernel<T, DP><<<dim3(blocks, b.qk_heads), DB_THREADS, first, s>>>(b);
+  delta_block_scan_kernel<T, DP><<<dim3(rows, a.heads, (a.V + DB_COLS - 1) / DB_COLS), DB_THREADS, second, s>>>(a);
+  return launch_result();
+}
+
+// The rule over runs of tokens, block by block.  `ws`: (tokens / block tokens + rows) * zb_delta_block_floats floats,
+// 16-byte aligned, contents irrelevant.  The rows' tokens lie behind one another in the stream, row_q_start ascending.
+ZB_API int zb_delta_block_scan(float* out, const void* q, long long q_stride, const void* k, long long k_stride, const void* v,
+                               long long v_stride, const float* b, const float* a, long long ba_stride, const float* a_log,
+                               const float* dt_bias, float* state, long long slot_stride, const int* slots, const int* row_q_start,
+                               const int* row_q_len, int rows, int tokens, int qk_heads, int heads, int D, int V, int num_slots,
+                               int write_state, float q_scale, float unit_eps, float* ws, int dtype, int* status, void* stream) {
+  if (rows < 0 || tokens < 0 || qk_heads <= 0 || heads <= 0 || heads % qk_heads != 0 || D <= 0 || V <= 0 || num_slots <= 0)
+    return ERR_BAD_ARGUMENT;
+  if (D > zb_delta_block_max_channels() || heads > 65535 || (V + DB_COLS - 1) / DB_COLS > 65535) return ERR_UNSUPPORTED;
+  if (rows == 0 || tokens == 0) return OK;
+  if (ws == nullptr || reinterpret_cast<uintptr_t>(ws) % 16 != 0) return ERR_BAD_ARGUMENT;
+  const int blocks = tokens / DB + rows, dp = D <= 64 ? 64 : 128;
+  DeltaBlocksArgs g;
+  g.qk = ws; g.coef = ws + static_cast<long long>(blocks) * qk_heads * dp * 2 * DB; g.q = q; g.q_stride = q_stride; g.k = k;
+  g.k_stride = k_stride; g.b = b; g.a = a; g.ba_stride = ba_stride; g.a_log = a_log; g.dt_bias = dt_bias;
+  g.row_q_start = row_q_start; g.row_q_len = row_q_len; g.rows = rows; g.qk_heads = qk_heads; g.heads = heads; g.D = D;
+  g.q_scale = q_scale; g.unit_eps = unit_eps;
+  DeltaBlockScanArgs c;
+  c.out = out; c.qk = g.qk; c.coef = g.coef; c.v = v; c.v_stride = v_stride; c.state = state; c.slot_stride = slot_stride;
+  c.slots = slots; c.row_q_start = row_q_start; c.row_q_len = row_q_len; c.heads = heads; c.qk_heads = qk_heads; c.D = D; c.V = V;
+  c.num_slots = num_slots; c.write_state = write_state; c.status = status;
+  auto s = static_cast<cudaStream_t>(stream);
+  if (dtype == DTYPE_F32) return dp == 64 ? delta_block_launch<float, 64>(g, c, rows, blocks, s) : delta_block_launch<float, 128>(g, c, rows, blocks, s);
+  return dp == 64 ? delta_block_launch<__nv_bfloat16, 64>(g, c, rows, blocks, s) : delta_block_launch<__nv_bfloat16, 128>(g, c, rows, blocks, s);
 }

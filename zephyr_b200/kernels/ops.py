@@ -124,6 +124,12 @@ _SIGNATURES = {
     "zb_delta_scan": [c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_longlong,
                       c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                       c_void_p, c_void_p],
+    "zb_delta_block_max_channels": [],
+    "zb_delta_block_tokens": [],
+    "zb_delta_block_floats": [c_int, c_int, c_int],
+    "zb_delta_block_scan": [c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p,
+                            c_longlong, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+                            c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p, c_int, c_void_p, c_void_p],
     "zb_residual_rms_norm": [c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_int, c_float, c_float, c_int,
                              c_int, c_int, c_void_p],
     "zb_route_biased": [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
@@ -1237,6 +1243,9 @@ def delta_max_channels() -> int:
     return library().zb_delta_max_channels()
 
 
+DELTA_BLOCKS_FROM = 16       # new tokens per request, on average, from which on the delta rule runs block by block
+
+
 def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b: torch.Tensor, a: torch.Tensor,
                a_log: torch.Tensor, dt_bias: torch.Tensor, heads: int, qk_heads: int, key_dim: int, value_dim: int,
                state: torch.Tensor, slots: torch.Tensor, row_q_start: torch.Tensor, row_q_len: torch.Tensor,
@@ -1262,7 +1271,17 @@ def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b: torch.Tenso
     _require(heads % qk_heads == 0, "heads must be a multiple of the q/k heads")
     _require(state.dim() == 2 and state.dtype == torch.float32 and state.stride(1) == 1
              and state.shape[1] == heads * key_dim * value_dim, "state must be float32 [slots, heads * value_dim * key_dim]")
-    dev = v.device
+    dev, lib, rows = v.device, library(), slots.numel()
+    out = torch.empty((T, heads * value_dim), dtype=torch.float32, device=dev)
+    if T >= DELTA_BLOCKS_FROM * rows and key_dim <= lib.zb_delta_block_max_channels():
+        ws = torch.empty(((T // lib.zb_delta_block_tokens() + rows) * lib.zb_delta_block_floats(qk_heads, heads, key_dim),),
+                         dtype=torch.float32, device=dev)
+        _check(lib.zb_delta_block_scan(
+            _ptr(out), _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(b), _ptr(a), b.stride(0), _ptr(a_log),
+            _ptr(dt_bias), _ptr(state), state.stride(0), _ptr(slots), _ptr(row_q_start), _ptr(row_q_len), rows, T, qk_heads, heads,
+            key_dim, value_dim, state.shape[0], int(write_state), float(q_scale), float(unit_eps), _ptr(ws), DTYPE_CODE[v.dtype],
+            _ptr(status), _stream()), "delta_block_scan", kernels=2)
+        return out
     qn = torch.empty((T, qk_heads * key_dim), dtype=torch.float32, device=dev)
     kn = torch.empty_like(qn)
     beta = torch.empty((T, heads), dtype=torch.float32, device=dev)
@@ -1270,7 +1289,6 @@ def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b: torch.Tenso
     _check(library().zb_delta_gates(_ptr(qn), _ptr(kn), _ptr(beta), _ptr(decay), _ptr(q), q.stride(0), _ptr(k), k.stride(0),
                                     _ptr(b), _ptr(a), b.stride(0), _ptr(a_log), _ptr(dt_bias), T, qk_heads, heads, key_dim,
                                     float(q_scale), float(unit_eps), DTYPE_CODE[v.dtype], _stream()), "delta_gates")
-    out = torch.empty((T, heads * value_dim), dtype=torch.float32, device=dev)
     _check(library().zb_delta_scan(_ptr(out), _ptr(qn), _ptr(kn), _ptr(v), v.stride(0), _ptr(beta), _ptr(decay), _ptr(state),
                                    state.stride(0), _ptr(slots), _ptr(row_q_start), _ptr(row_q_len), slots.numel(), T, heads,
                                    heads // qk_heads, key_dim, value_dim, state.shape[0], int(write_state),
