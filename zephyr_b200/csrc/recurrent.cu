@@ -292,6 +292,8 @@ __global__ void causal_conv_silu_kernel(const ConvArgs a, const int* token_row, 
 // stream, a thread VEC neighbouring channels of them.  Bound by latency where a thread walks its tokens one load
 // behind the other, so it asks for all its inputs, the TAPS - 1 before the first token among them, before it uses any
 // (they come again from the cache for the next CTA); inputs before a request's first new token come from its state.
+// 2048 tokens: 2560 bfloat16 channels 15.5 us (21.7 us walked 32 tokens a thread), 4096 float32 channels 20.6 us (69.6 us
+// with a thread a channel and token).
 // TAPS: the taps of the kernel, `taps` of them in use (the others, at the old end, are skipped).
 constexpr int CONV_RUN = 8;
 
@@ -340,9 +342,15 @@ __global__ void __launch_bounds__(128) causal_conv_silu_run_kernel(const ConvArg
   }
   const float* wp = static_cast<const float*>(a.w);
   float w[TAPS][VEC], bias[VEC];
+  const bool quads = a.taps == 4 && reinterpret_cast<uintptr_t>(wp) % 16 == 0;      // a channel's weights in one read
 #pragma unroll
   for (int v = 0; v < VEC; ++v) {
     bias[v] = works ? static_cast<const float*>(a.bias)[c + v] : 0.0f;
+    if (TAPS == 4 && quads) {
+      const float4 four = works ? load4(wp + (c + v) * 4) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      w[0][v] = four.x; w[1][v] = four.y; w[2][v] = four.z; w[3][v] = four.w;
+      continue;
+    }
 #pragma unroll
     for (int j = 0; j < TAPS; ++j) w[j][v] = works && j >= skipped ? wp[(c + v) * a.taps + (j - skipped)] : 0.0f;
   }
