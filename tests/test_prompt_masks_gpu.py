@@ -1,0 +1,60 @@
+"""The prompt kernel on tcgen05 with a window that keeps the first tokens and with a chunked mask, at the edges of its tiles of
+128 keys, against a plain float64 attention and against the mma.sync kernel."""
+
+import math
+
+import pytest
+import torch
+
+from test_kernels_gpu import build_paged_case, ops, rand, tiles_for  # noqa: F401  (ops: a fixture)
+
+pytestmark = pytest.mark.gpu
+
+
+def plain(q, K, V, ctx, nh, nkv, window, keep, chunk, sinks, softcap):
+    T = q.shape[0]
+    i, j = torch.arange(ctx, ctx + T)[:, None], torch.arange(ctx + T)[None, :]
+    seen = j <= i
+    if window:
+        seen = seen & (i - j < window)
+    if chunk:
+        seen = seen & (i // chunk == j // chunk)
+    seen = seen | ((j <= i) & (j < keep))                  # kept first tokens stay through either mask
+    out = []
+    for h in range(nh):
+        s = q[:, h].double() @ K[:, h // (nh // nkv)].double().T / math.sqrt(128)
+        if softcap:
+            s = softcap * torch.tanh(s / softcap)
+        s = s.masked_fill(~seen, -math.inf)
+        if sinks is not None:
+            s = torch.cat([s, sinks[h].double().expand(T, 1)], dim=1)
+        out.append(torch.softmax(s, -1)[:, :ctx + T] @ V[:, h // (nh // nkv)].double())
+    return torch.stack(out, 1)
+
+
+@pytest.mark.parametrize("window,keep,chunk,softcap,sink,page", [
+    (100, 1, 0, 0.0, False, 16), (64, 64, 0, 0.0, True, 16), (200, 128, 0, 0.0, False, 8), (130, 129, 0, 0.0, True, 32),
+    (1, 300, 0, 0.0, False, 16), (300, 70, 0, 20.0, True, 16), (1000, 64, 0, 0.0, False, 16), (0, 0, 100, 0.0, True, 16),
+    (0, 0, 128, 0.0, False, 16), (90, 0, 256, 0.0, False, 64), (60, 40, 200, 0.0, False, 16)])
+def test_kept_windows_and_chunks(ops, cuda_device, window, keep, chunk, softcap, sink, page):
+    nh, nkv, hd, q_lens, ctx = 4, 2, 128, [37, 300, 2, 129, 128], [0, 5, 400, 255, 256]
+    q, cache, meta, Ks, Vs, qs = build_paged_case(cuda_device, torch.bfloat16, nh, nkv, hd, page, q_lens, ctx, 300)
+    sinks = rand((nh,), torch.float32, cuda_device, 5) if sink else None
+    status, got = ops.new_status(cuda_device), {}
+    for tcgen05 in (True, False):
+        ops.USE_TCGEN05_PREFILL = tcgen05
+        try:
+            got[tcgen05] = ops.paged_prefill(q, cache, meta["table"], *tiles_for(q_lens, ops.paged_prefill_tile_tokens(), cuda_device),
+                                             meta["row_q_start"], meta["row_q_len"], meta["row_ctx"], nh, nkv, hd, window,
+                                             1 / math.sqrt(hd), status, torch.empty_like(q), chunk=chunk, sinks=sinks,
+                                             softcap=softcap, keep_first=keep)
+        finally:
+            ops.USE_TCGEN05_PREFILL = True
+    ops.check_status(status)
+    # Weights and the result are rounded to bfloat16 (2^-9 each, of values around one to four).
+    assert (got[True].float() - got[False].float()).abs().max() <= 3 * 2.0 ** -7
+    cursor = 0
+    for r, n in enumerate(q_lens):
+        expected = plain(qs[r], Ks[r], Vs[r], ctx[r], nh, nkv, window, keep, chunk, sinks.cpu() if sink else None, softcap)
+        assert (got[True][cursor:cursor + n].double().cpu().view(n, nh, hd) - expected).abs().max() <= 1.6e-2 * 2
+        cursor += n

@@ -25,8 +25,12 @@
 //     shift it is given as long as it is given everywhere; the bound keeps exp2 far from
 //     overflow).  A row's two threads tell each other their largest score every tile, so both
 //     take the same decisions.
+// A window may keep the first tokens of a sequence, and a chunk may bound what a query sees: masks of the same loop
+// (3000 tokens, 16/8 heads, window 1024 with 64 kept tokens: 80 us, 151 us on the mma.sync kernel; 2125 tokens in chunks
+// of 1024: 37 us, 68 us there).
 // Math and masking as in attention_prefill.cu and attention_simt.cu (causal, lower-right aligned on
-// the cached context, optional window; probabilities rounded to bfloat16 for the second product;
+// the cached context, optional window, whose first tokens may be kept, and optional chunk; probabilities rounded to
+// bfloat16 for the second product;
 // reference: src/layer/paged_attention.cpp:118-296, deps/ttl/src/kernels/attention/attention.cu:58-170).
 // Every wait is bounded and reports instead of hanging; TMEM is given back on every path.
 #include <map>
@@ -71,6 +75,8 @@ struct PrefillTcArgs {
   const int* row_ctx;            // [R]
   int max_blocks, page_shift, num_pages, num_rows;
   int nh, nkv, window;
+  int chunk;                     // > 0: a query at position p sees only keys j with j / chunk == p / chunk
+  int keep_first;                // with a window: keys below this position stay visible to every later query
   float scale_log2;
   float softcap_log2;            // > 0: scores are softcap * tanh(scale * s / softcap); this is softcap * log2(e)
   float scale_over_cap;          // scale / softcap
@@ -161,8 +167,9 @@ __device__ __forceinline__ void softmax_pass(unsigned tmem_row, unsigned (&words
   row_sum = (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
 }
 
-// BIASED_SCORES: with the distance bias (a form of its own, so that the other keeps its registers).
-template <bool BIASED_SCORES>
+// BIASED_SCORES: with the distance bias (a form of its own, so that the other keeps its registers).  KEPT: with a window
+// that keeps the first tokens (likewise).
+template <bool BIASED_SCORES, bool KEPT>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 paged_prefill_tc_kernel(const __grid_constant__ PrefillTcArgs a) {
   // Shared memory holds keys and values only (three stages of each, tiles of 32 KB on 1024-byte
@@ -212,9 +219,19 @@ paged_prefill_tc_kernel(const __grid_constant__ PrefillTcArgs a) {
 
   // Keys any query of this tile may see: [lo, hi).
   const int hi = ctx + q0 + n_tok;
-  const int lo = a.window > 0 ? max(0, ctx + q0 - a.window + 1) : 0;
+  int lo = a.window > 0 ? max(0, ctx + q0 - a.window + 1) : 0;
+  if (!BIASED_SCORES && a.chunk > 0) lo = max(lo, (ctx + q0) / a.chunk * a.chunk);
+  // First tokens that a window keeps, [0, kept), are tiles of their own in front as soon as some row has left a key
+  // behind; what follows them is the window's (and the chunk's) alone.
+  int kept = 0;
+  if (KEPT && max(hi - a.window, a.chunk > 0 ? (hi - 1) / a.chunk * a.chunk : 0) > 0) kept = min(a.keep_first, hi);
+  lo = max(lo, kept);
   const int first_tile = lo / TC_BN * TC_BN;
-  const int n_tiles = (hi - first_tile + TC_BN - 1) / TC_BN;
+  const int kept_tiles = KEPT ? (kept + TC_BN - 1) / TC_BN : 0;
+  const int n_tiles = kept_tiles + (lo < hi ? (hi - first_tile + TC_BN - 1) / TC_BN : 0);
+  auto tile_start = [&](int j) { return KEPT && j < kept_tiles ? j * TC_BN : first_tile + (j - kept_tiles) * TC_BN; };
+  auto run_lo = [&](int j) { return KEPT && j < kept_tiles ? 0 : lo; };                // the positions a tile's rows are taken from
+  auto run_hi = [&](int j) { return KEPT && j < kept_tiles ? kept : hi; };
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
@@ -295,7 +312,7 @@ paged_prefill_tc_kernel(const __grid_constant__ PrefillTcArgs a) {
     const int first_id = (lt >> 5) * 8 + (lt & 31);
     int ahead_tile = -1, ahead_page[2] = {0, 0};
     auto look_up = [&](int j, int (&page)[2]) {
-      const int k0 = first_tile + j * TC_BN;
+      const int k0 = tile_start(j);
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         const int id = first_id + 16 * u;
@@ -304,7 +321,7 @@ paged_prefill_tc_kernel(const __grid_constant__ PrefillTcArgs a) {
       }
     };
     auto issue_tiled = [&](int j) {
-      const int stage = j % TC_STAGES, k0 = first_tile + j * TC_BN;
+      const int stage = j % TC_STAGES, k0 = tile_start(j);
       unsigned char* dst = kv_s + stage * 2 * TC_TILE_BYTES + kv * TC_TILE_BYTES;
       unsigned long long* bar = &kv_full[kv * TC_STAGES + stage];
       if (lt == 0) mbar_arrive_expect_tx(bar, TC_TILE_BYTES);
@@ -335,7 +352,7 @@ paged_prefill_tc_kernel(const __grid_constant__ PrefillTcArgs a) {
     auto issue_plain = [&](int j) {
       const int stage = j % TC_STAGES;
       unsigned char* dst = kv_s + stage * 2 * TC_TILE_BYTES + kv * TC_TILE_BYTES + dst_base;
-      const int k0 = first_tile + j * TC_BN;
+      const int k0 = tile_start(j), rows_lo = run_lo(j), rows_hi = run_hi(j);
 #pragma unroll 1
       for (int part = 0; part < 2; ++part) {
         // The page ids of 16 of this thread's 32 rows first, all at once: a lookup per copy would put
@@ -344,12 +361,12 @@ paged_prefill_tc_kernel(const __grid_constant__ PrefillTcArgs a) {
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           const int pos = k0 + row_in_4 + 4 * (16 * part + i), block = pos >> a.page_shift;
-          page[i] = pos >= lo && pos < hi ? (block < a.max_blocks ? table[block] : -1) : 0;
+          page[i] = pos >= rows_lo && pos < rows_hi ? (block < a.max_blocks ? table[block] : -1) : 0;
         }
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           const int r = row_in_4 + 4 * (16 * part + i), pos = k0 + r;
-          bool ok = pos >= lo && pos < hi;
+          bool ok = pos >= rows_lo && pos < rows_hi;
           const __nv_bfloat16* src = a.kv_cache;
           if (ok) {
             if (page[i] <= 0 || page[i] >= a.num_pages) {
@@ -373,9 +390,9 @@ paged_prefill_tc_kernel(const __grid_constant__ PrefillTcArgs a) {
         give_up(-1);
         break;
       }
-      const int k0 = first_tile + j * TC_BN;
+      const int k0 = tile_start(j);
       if (trace && lt == 0 && j < 64) trace[256 + 4 * j + kv] = tc_timer_ns();
-      if (a.tiled && k0 >= lo && k0 + TC_BN <= hi) issue_tiled(j); else issue_plain(j);
+      if (a.tiled && k0 >= run_lo(j) && k0 + TC_BN <= run_hi(j)) issue_tiled(j); else issue_plain(j);
     }
   } else if (warp == TC_MMA_WARP) {
     // ------------------------------------------------------------- the thread that issues products
@@ -450,8 +467,16 @@ paged_prefill_tc_kernel(const __grid_constant__ PrefillTcArgs a) {
     constexpr bool biased = BIASED_SCORES;
     const float r1 = biased ? a.bias_r1[head] : 0.0f, r2 = biased ? a.bias_r2[head] : 0.0f;
     bool failed = false;
+    // The last position that this row's window and chunk leave out, and the first key that all rows of the CTA see.
+    int passed = a.window > 0 ? qp - a.window : -1;
+    int open_from = a.window > 0 ? ctx + q0 + TC_BM - a.window : 0;
+    if (!BIASED_SCORES && a.chunk > 0) {
+      passed = max(passed, qp / a.chunk * a.chunk - 1);
+      open_from = max(open_from, (ctx + q0 + TC_BM - 1) / a.chunk * a.chunk);
+    }
     for (int j = 0; j < n_tiles; ++j) {
-      const int k0 = first_tile + j * TC_BN;
+      const int k0 = tile_start(j);
+      const bool in_kept = KEPT && j < kept_tiles;
       // Whether to go on is decided by the warp as one: the tensor-memory instructions below are
       // for all of its lanes together.
       const int buffer = j & 1;
@@ -460,8 +485,7 @@ paged_prefill_tc_kernel(const __grid_constant__ PrefillTcArgs a) {
       tc_fence_after_sync();
       if (trace && threadIdx.x == 0 && j < 64) trace[4 * j + 1] = tc_timer_ns();
       // Most tiles lie wholly in every row's past (and inside its window): no mask to evaluate.
-      const bool open_tile = k0 + TC_BN - 1 <= ctx + q0 && k0 >= lo &&
-                             (a.window == 0 || k0 > ctx + q0 + TC_BM - 1 - a.window);
+      const bool open_tile = k0 + TC_BN - 1 <= ctx + q0 && (in_kept ? k0 + TC_BN <= kept : k0 >= lo && k0 >= open_from);
       // One pass forms the probabilities with the shift the row already has and notes the row's
       // largest score; only if that has outgrown the shift by 2^8 (always for a row's first keys) is
       // the shift moved, O and the sum rescaled, and the pass repeated.  Per score the pass costs a
@@ -472,24 +496,27 @@ paged_prefill_tc_kernel(const __grid_constant__ PrefillTcArgs a) {
       for (int attempt = 0; attempt < 2; ++attempt) {
         const float neg_shift = m_used == -INFINITY ? 0.0f : -m_used;
         float raw_max = -INFINITY, row_sum = 0.0f;
-        const int after = a.window > 0 ? qp - a.window - k0 : -(1 << 30);
+        const int after = in_kept ? -1 : passed - k0, last = (in_kept ? min(qp, kept - 1) : qp) - k0;
+        const int first = run_lo(j) - k0;
         if (capped) {
           if (open_tile)
-            softmax_pass<false, TC_CAPPED>(tmem_s, words, half, a.scale_over_cap, neg_shift, 0, 0, 0, raw_max, row_sum, a.softcap_log2);
+            softmax_pass<false, TC_CAPPED>(tmem_s, words, half, a.scale_over_cap, neg_shift, 0, 0, 0, raw_max, row_sum,
+                                                  a.softcap_log2);
           else
-            softmax_pass<true, TC_CAPPED>(tmem_s, words, half, a.scale_over_cap, neg_shift, qp - k0, lo - k0, after, raw_max,
-                                          row_sum, a.softcap_log2);
+            softmax_pass<true, TC_CAPPED>(tmem_s, words, half, a.scale_over_cap, neg_shift, last, first, after,
+                                                raw_max, row_sum, a.softcap_log2);
         } else if (biased) {
           if (open_tile)
-            softmax_pass<false, TC_BIASED>(tmem_s, words, half, a.scale_log2, neg_shift, qp - k0, 0, 0, raw_max, row_sum, 0.0f,
-                                           r1, r2);
+            softmax_pass<false, TC_BIASED>(tmem_s, words, half, a.scale_log2, neg_shift, last, 0, 0, raw_max, row_sum, 0.0f,
+                                                  r1, r2);
           else
-            softmax_pass<true, TC_BIASED>(tmem_s, words, half, a.scale_log2, neg_shift, qp - k0, lo - k0, after, raw_max, row_sum,
-                                          0.0f, r1, r2);
+            softmax_pass<true, TC_BIASED>(tmem_s, words, half, a.scale_log2, neg_shift, last, first, after, raw_max,
+                                                row_sum, 0.0f, r1, r2);
         } else if (open_tile) {
           softmax_pass<false, TC_PLAIN>(tmem_s, words, half, a.scale_log2, neg_shift, 0, 0, 0, raw_max, row_sum);
         } else {
-          softmax_pass<true, TC_PLAIN>(tmem_s, words, half, a.scale_log2, neg_shift, qp - k0, lo - k0, after, raw_max, row_sum);
+          softmax_pass<true, TC_PLAIN>(tmem_s, words, half, a.scale_log2, neg_shift, last, first, after, raw_max,
+                                             row_sum);
         }
         if (attempt == 0) {
           // The row's largest score is the larger of its halves'.
@@ -647,17 +674,20 @@ ZB_API int zb_paged_prefill_tc_supported(int nh, int nkv, int hd, int dtype, int
 }
 
 // Attention of the tiles' tokens (tiles of 128 new tokens of one request) over their requests'
-// pages; writes those tokens' rows of `out`.  Arguments as zb_paged_prefill_masked without the chunked mask:
+// pages; writes those tokens' rows of `out`.  Arguments as zb_paged_prefill_masked:
 // `softcap` > 0 bounds the scaled scores by softcap * tanh(. / softcap); `keys_only`: a page holds keys alone
 // and they are the values too; `sinks` (null, or one float32 per query head) join the softmax's denominator;
-// `bias_r1`, `bias_r2` (null, or one float32 per query head each; not with a softcap) bias the distances.
+// `bias_r1`, `bias_r2` (null, or one float32 per query head each; not with a softcap, a chunk or kept tokens) bias the distances;
+// `keep_first` (with a window): keys below this position stay visible.
 ZB_API int zb_paged_prefill_tc_masked(void* out, const void* q, const void* kv_cache, const int* block_table,
                                       int max_blocks, int page_size, int num_pages, int num_rows, const int* tile_row,
                                       const int* tile_q0, int n_tiles, const int* row_q_start, const int* row_q_len,
-                                      const int* row_ctx, int nh, int nkv, int hd, int window, float scale, float softcap,
-                                      int keys_only, const float* sinks, const float* bias_r1, const float* bias_r2,
+                                      const int* row_ctx, int nh, int nkv, int hd, int window, int chunk, int keep_first, float scale,
+                                      float softcap, int keys_only, const float* sinks, const float* bias_r1, const float* bias_r2,
                                       int* status, void* stream) {
-  if ((bias_r1 == nullptr) != (bias_r2 == nullptr) || (bias_r1 != nullptr && softcap > 0.0f) || n_tiles < 0 || page_size <= 0 || window < 0 || softcap < 0.0f) return ERR_BAD_ARGUMENT;
+  if ((bias_r1 == nullptr) != (bias_r2 == nullptr) || (bias_r1 != nullptr && softcap > 0.0f) || n_tiles < 0 || page_size <= 0 || window < 0 || softcap < 0.0f ||
+      chunk < 0 || keep_first < 0 || (keep_first > 0 && window <= 0) || (bias_r1 != nullptr && (keep_first > 0 || chunk > 0)))
+    return ERR_BAD_ARGUMENT;
   if (!zb_paged_prefill_tc_supported(nh, nkv, hd, DTYPE_BF16, page_size)) return ERR_UNSUPPORTED;
   if (reinterpret_cast<uintptr_t>(q) % 16 != 0 || reinterpret_cast<uintptr_t>(out) % 16 != 0 ||
       reinterpret_cast<uintptr_t>(kv_cache) % 16 != 0)
@@ -677,7 +707,7 @@ ZB_API int zb_paged_prefill_tc_masked(void* out, const void* q, const void* kv_c
   a.max_blocks = max_blocks; a.num_pages = num_pages; a.num_rows = num_rows;
   a.page_shift = 0;
   while ((1 << a.page_shift) < page_size) ++a.page_shift;
-  a.nh = nh; a.nkv = nkv; a.window = window;
+  a.nh = nh; a.nkv = nkv; a.window = window; a.chunk = chunk; a.keep_first = keep_first;
   a.scale_log2 = scale * 1.4426950408889634f;
   a.softcap_log2 = softcap * 1.4426950408889634f;
   a.scale_over_cap = softcap > 0.0f ? scale / softcap : 0.0f;
@@ -687,7 +717,8 @@ ZB_API int zb_paged_prefill_tc_masked(void* out, const void* q, const void* kv_c
   a.status = status;
   a.trace = prefill_tc_trace();
   const size_t smem = 2 * TC_STAGES * TC_TILE_BYTES;
-  auto kernel = bias_r1 != nullptr ? paged_prefill_tc_kernel<true> : paged_prefill_tc_kernel<false>;
+  auto kernel = bias_r1 != nullptr ? paged_prefill_tc_kernel<true, false>
+                : keep_first > 0   ? paged_prefill_tc_kernel<false, true> : paged_prefill_tc_kernel<false, false>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
     return ERR_CUDA;
   kernel<<<dim3(nh, n_tiles), TC_THREADS, smem, static_cast<cudaStream_t>(stream)>>>(a);
@@ -699,6 +730,6 @@ ZB_API int zb_paged_prefill_tc(void* out, const void* q, const void* kv_cache, c
                                int n_tiles, const int* row_q_start, const int* row_q_len, const int* row_ctx, int nh,
                                int nkv, int hd, int window, float scale, int* status, void* stream) {
   return zb_paged_prefill_tc_masked(out, q, kv_cache, block_table, max_blocks, page_size, num_pages, num_rows, tile_row,
-                                    tile_q0, n_tiles, row_q_start, row_q_len, row_ctx, nh, nkv, hd, window, scale, 0.0f, 0,
+                                    tile_q0, n_tiles, row_q_start, row_q_len, row_ctx, nh, nkv, hd, window, 0, 0, scale, 0.0f, 0,
                                     nullptr, nullptr, nullptr, status, stream);
 }

@@ -184,8 +184,8 @@ _SIGNATURES = {
     "zb_paged_prefill_tc_supported": [c_int, c_int, c_int, c_int, c_int],
     "zb_paged_prefill_tc_set_trace": [c_void_p],
     "zb_paged_prefill_tc_masked": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
-                                   c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_int,
-                                   c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
+                                   c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float,
+                                   c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
     "zb_paged_prefill_tc": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
                             c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p],
     "zb_gemm_small_supported": [c_int, c_int, c_int],
@@ -1557,9 +1557,9 @@ def paged_prefill(q: torch.Tensor, kv_cache: torch.Tensor, block_table: torch.Te
     """Tensor-core attention for rows with several new tokens, cut into tiles of
     ``paged_prefill_tile_tokens()``; writes those tokens' rows of ``out``.  ``chunk``, ``sinks``, ``softcap`` and
     ``distance_bias`` as in ``paged_attention``, ``keys_only`` as its ``shared_kv``.  Head size 128 runs on tcgen05
-    with the accumulators in tensor memory (every form but the chunked mask), other sizes and chunked masks
-    on mma.sync.  ``keep_first``, ``pool`` with its store, and ``cross_values`` (``out`` is then
-    [T, nh * nkv * hd], bfloat16 or float32) as in ``paged_attention``: these run on mma.sync.  ``by_group``: every
+    with the accumulators in tensor memory, other sizes on mma.sync.  ``keep_first``, ``pool`` with its store, and
+    ``cross_values`` (``out`` is then [T, nh * nkv * hd], bfloat16 or float32) as in ``paged_attention``: the last two, and
+    kept tokens or a chunk beside a distance bias, run on mma.sync.  ``by_group``: every
     tile is one new token (the tiles of single-token rows), and a CTA's query rows are the heads that share a
     key/value head: a decoded token's keys and values stream once a group."""
     _cuda(q, kv_cache, block_table, tile_row, tile_q0, row_q_start, row_q_len, row_ctx, status, out, pool_cache, pool_table)
@@ -1583,13 +1583,14 @@ def paged_prefill(q: torch.Tensor, kv_cache: torch.Tensor, block_table: torch.Te
                  and pool_cache.is_contiguous(), "a pooled store has the pages' shape and a table row per request")
         pool_pages, pool_blocks = pool_cache.shape[0], pool_table.shape[1]
     r1, r2 = _distance_bias(distance_bias, nh)
-    tensor_memory = (USE_TCGEN05_PREFILL and not chunk and not windowed and not (softcap and r1 is not None)
+    tensor_memory = (USE_TCGEN05_PREFILL and not (pool or cross_values or by_group or (keep_first and window <= 0))
+                     and not ((softcap or keep_first or chunk) and r1 is not None)
                      and bool(library().zb_paged_prefill_tc_supported(nh, nkv, hd, DTYPE_CODE[q.dtype], page_size)))
     common = (_ptr(out), _ptr(q), _ptr(kv_cache), _ptr(block_table), block_table.shape[1], page_size, pages,
               block_table.shape[0], _ptr(tile_row), _ptr(tile_q0), tile_row.numel(), _ptr(row_q_start), _ptr(row_q_len),
               _ptr(row_ctx), nh, nkv, hd, int(window))
     if tensor_memory:
-        _check(library().zb_paged_prefill_tc_masked(*common, float(scale), float(softcap), int(keys_only), _ptr(sinks),
+        _check(library().zb_paged_prefill_tc_masked(*common, int(chunk), int(keep_first), float(scale), float(softcap), int(keys_only), _ptr(sinks),
                                                     _ptr(r1), _ptr(r2), _ptr(status), _stream()), "paged_prefill")
     elif windowed or r1 is not None:
         _check(library().zb_paged_prefill_windowed(*common, int(chunk), float(scale), float(softcap), int(keys_only),
