@@ -69,3 +69,45 @@ def test_the_delta_rule_on_both_paths(cuda_device):
     for other in (blocks, mixed):
         for x, y in zip(single, other):       # float32 sums in another order
             assert (x - y).abs().max() <= 1e-5 * max(1.0, float(x.abs().max()))
+
+
+@pytest.mark.parametrize("heads,per,dim,vdim", [(4, 2, 128, 64), (6, 3, 64, 20), (3, 1, 40, 36), (2, 2, 16, 130), (40, 8, 128, 64), (2, 1, 8, 9)])
+def test_the_state_space_walk(cuda_device, heads, per, dim, vdim):
+    """Portions of 33 to 200 tokens and their pieces' edges, from states of their own into them, against the plain
+    recurrence; one head's decays are strong (e^-80 a token), one's next to none, both within a piece."""
+    from zephyr_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(heads * dim + vdim)
+    lengths, slots, groups = [64, 33, 200, 65, 63], [1, 4, 0, 3, 2], heads // per
+    T = sum(lengths)
+    bf = lambda *shape: torch.randn(*shape, generator=g).to(torch.bfloat16)
+    q, k, v, dt = bf(T, groups * dim), bf(T, groups * dim), bf(T, heads * vdim), bf(T, heads)
+    a_log, dt_bias, skip = torch.randn(heads, generator=g), torch.randn(heads, generator=g) - 1.0, torch.randn(heads, generator=g)
+    a_log[0], a_log[-1] = 3.0, -8.0
+    dt[100:103] = 4.0                                       # strong steps in the middle of a piece
+    state = torch.randn(5, heads * dim * vdim + 3, generator=g)[:, :heads * dim * vdim]
+    dev = lambda t: t.to(cuda_device)
+    held = dev(torch.cat([state, torch.zeros(5, 3)], dim=1))[:, :heads * dim * vdim]
+    i32 = lambda values: torch.tensor(values, dtype=torch.int32, device=cuda_device)
+    starts = [sum(lengths[:i]) for i in range(len(lengths))]
+    status = ops.new_status(cuda_device)
+    before = ops.LAUNCH_COUNTS.get("state_walk", 0)
+    out = ops.decayed_state_scan("state_space", dev(q), dev(k), dev(v), heads, dim, vdim, held, i32(slots), i32(starts), i32(lengths),
+                                 status, dt=dev(dt), dt_bias=dev(dt_bias), a_log=dev(a_log), skip=dev(skip), heads_per_group=per)
+    ops.check_status(status)
+    assert ops.LAUNCH_COUNTS["state_walk"] == before + 2
+    for start, n, slot in zip(starts, lengths, slots):
+        S = state[slot].double().view(heads, dim, vdim).clone()
+        step = torch.nn.functional.softplus(dt[start:start + n].double() + dt_bias.double())
+        decay = torch.exp(-torch.exp(a_log.double()) * step)
+        own = torch.arange(heads) // per
+        expected = []
+        for i in range(n):
+            qi, ki = (x[start + i].double().view(groups, dim)[own] for x in (q, k))
+            vi = v[start + i].double().view(heads, vdim)
+            S = S * decay[i].view(-1, 1, 1) + (ki * step[i].view(-1, 1)).unsqueeze(-1) * vi.unsqueeze(1)
+            expected.append(torch.einsum("hdv,hd->hv", S, qi) + skip.double().view(-1, 1) * vi)
+        expected = torch.stack(expected).reshape(n, -1)
+        # float32 sums of products that are exact, decays good to a few roundings.
+        assert (out[start:start + n].cpu().double() - expected).abs().max() <= 3e-6 * max(1.0, float(expected.abs().max()))
+        assert (held[slot].cpu().double() - S.reshape(-1)).abs().max() <= 3e-6 * max(1.0, float(S.abs().max()))

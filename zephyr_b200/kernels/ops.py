@@ -155,6 +155,12 @@ _SIGNATURES = {
                      c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p],
     "zb_retention_step": [c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_float, c_float, c_void_p, c_void_p, c_longlong,
                           c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
+    "zb_walk_max_channels": [],
+    "zb_walk_piece_tokens": [],
+    "zb_walk_piece_floats": [c_int, c_int, c_int, c_int],
+    "zb_state_walk": [c_int, c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p,
+                      c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
+                      c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p],
     "zb_rotate_qk": [c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_float, c_void_p, c_int, c_int, c_int, c_void_p],
     "zb_gated_group_rms_norm": [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_int,
                                 c_float, c_int, c_int, c_int, c_void_p],
@@ -712,6 +718,23 @@ def state_scan_max_channels() -> int:
     return library().zb_state_scan_max_channels()
 
 
+WALK_FROM = 32      # new tokens per request, on average, from which on a step's recurrences with one decay a head walk in pieces
+
+
+def _state_walk(mode: int, out, q, k, v, heads: int, key_dim: int, value_dim: int, state, slots, row_q_start, row_q_len, status,
+                write_state: bool, dt=None, dt_bias=None, a_log=None, skip=None, decay=None, heads_per_group: int = 1) -> None:
+    """The recurrence over runs of tokens in pieces of 64 with the state on the SM (csrc/state_walk.cu): mode 0 the
+    state-space form, 1 fixed decays.  The callers have checked types and shapes."""
+    lib, rows, T = library(), slots.numel(), v.shape[0]
+    ws = torch.empty(((T // lib.zb_walk_piece_tokens() + rows) * lib.zb_walk_piece_floats(mode, heads, heads_per_group, key_dim),),
+                     dtype=torch.float32, device=v.device)
+    _check(lib.zb_state_walk(
+        mode, _ptr(out), _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(dt), dt.stride(0) if dt is not None else 0,
+        _ptr(dt_bias), _ptr(a_log), _ptr(skip), _ptr(decay), _ptr(state), state.stride(0), _ptr(slots), _ptr(row_q_start),
+        _ptr(row_q_len), rows, T, heads, key_dim, value_dim, heads_per_group, state.shape[0], int(write_state), _ptr(ws), _ptr(status),
+        _stream()), "state_walk", kernels=2)
+
+
 def decayed_state_scan(mode: str, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, heads: int, key_dim: int,
                        value_dim: int, state: torch.Tensor, slots: torch.Tensor, row_q_start: torch.Tensor,
                        row_q_len: torch.Tensor, status: torch.Tensor, *, decay_logits: torch.Tensor | None = None,
@@ -761,6 +784,12 @@ def decayed_state_scan(mode: str, q: torch.Tensor, k: torch.Tensor, v: torch.Ten
             _f32_vector(vector, heads, "a per-head constant")
     out = torch.empty((T, heads * value_dim), dtype=torch.float32, device=v.device)
     rows = slots.numel()
+    if (segment is None and not gated and not fixed and v.dtype == torch.bfloat16 and T >= WALK_FROM * rows and key_dim % 8 == 0
+            and key_dim <= library().zb_walk_max_channels() and heads % heads_per_group == 0
+            and all(t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (q, k))):
+        _state_walk(0, out, q, k, v, heads, key_dim, value_dim, state, slots, row_q_start, row_q_len, status, write_state, dt=dt,
+                    dt_bias=dt_bias, a_log=a_log, skip=skip, heads_per_group=int(heads_per_group))
+        return out
     if segment is None:
         few = rows * heads * -(-value_dim // 64) <= _sm_count()
         segment = (max(SCAN_SEGMENT, -(-T // (64 * 16)) * 16)
@@ -820,6 +849,9 @@ def retention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Te
              and state.shape[1] == heads * key_dim * value_dim, "state must be float32 [slots, heads * key_dim * value_dim]")
     lib, rows = library(), slots.numel()
     out = torch.empty((T, heads * value_dim), dtype=torch.float32, device=v.device)
+    if key_dim <= lib.zb_walk_max_channels():
+        _state_walk(1, out, q, k, v, heads, key_dim, value_dim, state, slots, row_q_start, row_q_len, status, write_state, decay=decay)
+        return out
     pieces = T // lib.zb_retention_piece_tokens() + rows
     ws = torch.empty((pieces, heads * key_dim * value_dim), dtype=torch.float32, device=v.device)
     _check(lib.zb_retention(
