@@ -7,11 +7,10 @@
 // float32).  A request's new tokens of a step are cut into pieces of W tokens.  With S_in the state at a piece's start, n its
 // tokens and c_i the sum of the logarithms of its decays up to token i,
 //
-//   o_i   = e^(c_i) S_in^T q_i + sum_{j <= i} e^(c_i - c_j) s_j (q_i . k_j) v_j
-//   S_out = e^(c_n) S_in + sum_j e^(c_n - c_j) s_j k_j v_j^T
+//   o_i   = e^(c_i) S_in^T q_i + sum_{j <= i} P_ij v_j,   P_ij = e^(c_i - c_j) s_j (q_i . k_j)
+//   S_out = e^(c_n) S_in + sum_j w_j k_j v_j^T,           w_j = e^(c_n - c_j) s_j
 //
-//   walk_prepare   for all pieces side by side: the scores q . k, and what else a piece needs (sums of logarithms; the
-//                  float32 q and k as pairs of bfloat16 values)
+//   walk_prepare   for all pieces side by side: P, e^(c) and w, and q and k as the walk reads them
 //   state_walk     a CTA owns a request, a head and some value columns and walks the pieces with the state in registers
 //
 // so the state never leaves the SM, where passes over all pieces at once write and read every piece's state (2048
@@ -20,7 +19,8 @@
 // Products run on the tensor cores, float32 sums.  A bfloat16 operand is exact; beside it a float32 operand is the sum
 // of three bfloat16 values (all its 24 bits); two float32 operands (WALK_FIXED) are two bfloat16 values each, hi hi + hi lo +
 // lo hi, a relative error of about 2^-16 an operand.  The state itself is only ever touched by float32 multiply-adds.
-// Sums of logarithms are kept as two float32 values, so that a difference of two is good to a rounding of itself.
+// Sums of logarithms are formed in 64 bits and kept as two float32 values, so that a difference of two is good to a
+// rounding of itself.
 //
 // Piece p of row r has the number row_q_start[r] / W + r + p: distinct for all pieces of a step, and below
 // tokens / W + rows.
@@ -31,8 +31,9 @@ namespace zb {
 
 constexpr int W = 64;                    // tokens of a piece
 constexpr int W_THREADS = 256;
-constexpr int W_GST = W + 8;             // a row of the scores
-constexpr int W_STEP = 3 * W;            // WALK_SPACE, a head of a piece: sums of logarithms (base 2), two values each, and s
+constexpr int W_PST = W + 8;             // a row of P
+constexpr int W_STEP = 2 * W + 4;        // a head of a piece: e^(c), w, e^(c_n)
+constexpr int W_WAIT_LIMIT = 1 << 20;
 
 enum { WALK_SPACE = 0, WALK_FIXED = 1 };
 
@@ -43,14 +44,24 @@ struct WalkArgs {
   const void* dt; long long dt_stride;   // WALK_SPACE: [tokens, H], bfloat16
   const float* dt_bias; const float* a_log; const float* skip;        // WALK_SPACE: [H] each
   const float* decay;                    // WALK_FIXED: [H]
-  float* scores;                         // [pieces][qk heads][W][W_GST]
-  float* steps;                          // WALK_SPACE: [pieces][H][W_STEP]
-  __nv_bfloat16* parts;                  // WALK_FIXED: [pieces][H][q hi, q lo, k hi, k lo][W][DP + 8]
+  unsigned char* qk;                     // [pieces][qk heads][q, k][parts][W][DP + 8] bfloat16
+  unsigned char* heads;                  // [pieces][H]{P [parts][W][W_PST] bfloat16, W_STEP floats}
   float* out;                            // [tokens, H * V]
   float* state; long long slot_stride;   // slot s at state + s * slot_stride: [H][D][V]
   const int* slots; const int* row_q_start; const int* row_q_len;
   int rows, H, D, V, heads_per_group, num_slots, write_state;
+  int vectors, pairs;                    // rows of q and k move as 16-byte pieces; neighbouring values of v move together
   int* status;
+};
+
+template <int MODE, int DP>
+struct WalkParts {
+  static constexpr int PA = MODE == WALK_SPACE ? 1 : 2;      // parts of q, k and v
+  static constexpr int PB = MODE == WALK_SPACE ? 3 : 2;      // parts of P, the state and the weighted values
+  static constexpr int ST = DP + 8;
+  static constexpr int qk_bytes = 2 * PA * W * ST * 2;
+  static constexpr int p_bytes = PB * W * W_PST * 2;
+  static constexpr int head_bytes = p_bytes + W_STEP * 4;
 };
 
 __device__ __forceinline__ float walk_softplus(float z) { return fmaxf(z, 0.0f) + log1pf(expf(-fabsf(z))); }
@@ -70,36 +81,43 @@ __device__ __forceinline__ void split_parts(float x, float y, unsigned (&part)[P
 template <int PA, int PB>
 __device__ __forceinline__ constexpr bool counts(int a, int b) { return a + b < (PA > PB ? PA : PB); }
 
-// acc[N tiles of 8 columns] += A B over 16 of k: A's fragments in parts; B in parts, [k][st] tiles `part_stride` elements
-// apart, from this lane's ldmatrix address inside the first 16 x 16 block on.
-template <int N, int PA, int PB>
-__device__ __forceinline__ void walk_product(float (&acc)[N][4], const unsigned (&af)[PA][4], const __nv_bfloat16* b, int part_stride) {
+// B over 16 of k and N tiles of 8 columns: parts of [k][st] tiles `part_stride` elements apart, from this lane's ldmatrix
+// address inside the first 16 x 16 block on.
+template <int N, int PB>
+struct WalkB {
+  unsigned f[PB][N / 2][4];
+  __device__ __forceinline__ void load(const __nv_bfloat16* b, int part_stride) {
 #pragma unroll
-  for (int n = 0; n < N; n += 2) {
+    for (int pb = 0; pb < PB; ++pb)
 #pragma unroll
-    for (int pb = PB - 1; pb >= 0; --pb) {                   // the small products first
-      unsigned bf[4];
-      ldmatrix_x4_trans(bf, b + pb * part_stride + n * 8);
-#pragma unroll
-      for (int pa = PA - 1; pa >= 0; --pa)
-        if (counts<PA, PB>(pa, pb)) {
-          mma_bf16_16816(acc[n], af[pa], bf[0], bf[1]);
-          mma_bf16_16816(acc[n + 1], af[pa], bf[2], bf[3]);
-        }
-    }
+      for (int n = 0; n < N / 2; ++n) ldmatrix_x4_trans(f[pb][n], b + pb * part_stride + n * 16);
   }
+};
+// acc += A B.  The tiles take turns, so that no product waits for the one before it.
+template <int N, int PA, int PB>
+__device__ __forceinline__ void walk_product(float (&acc)[N][4], const unsigned (&af)[PA][4], const WalkB<N, PB>& b) {
+#pragma unroll
+  for (int pb = PB - 1; pb >= 0; --pb)                       // the small products first
+#pragma unroll
+    for (int pa = PA - 1; pa >= 0; --pa)
+      if (counts<PA, PB>(pa, pb)) {
+#pragma unroll
+        for (int n = 0; n < N; ++n) mma_bf16_16816(acc[n], af[pa], b.f[pb][n / 2][n % 2 * 2], b.f[pb][n / 2][n % 2 * 2 + 1]);
+      }
 }
 
 __device__ __forceinline__ int walk_first_piece(const WalkArgs& a, int row) { return a.row_q_start[row] / W + row; }
 
-// The scores of a piece for one q/k head, and its sums of logarithms (WALK_SPACE, the heads of the group) or its operands in
-// parts (WALK_FIXED).  DP: the channels padded with zeros.
+// A piece of one head.  DP: the channels padded with zeros.
 template <int MODE, int DP>
 __global__ void __launch_bounds__(W_THREADS) walk_prepare_kernel(const WalkArgs a) {
+  using Parts = WalkParts<MODE, DP>;
+  constexpr int ST = Parts::ST, PA = Parts::PA, PB = Parts::PB;
   extern __shared__ __align__(16) unsigned char w_smem[];
-  constexpr int ST = DP + 8, PA = MODE == WALK_SPACE ? 1 : 2;
   __shared__ int found;
-  const int piece = blockIdx.x, qk_head = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  __shared__ float c_hi[W], c_lo[W], s_s[W];
+  const int piece = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int qk_head = h / a.heads_per_group, qk_heads = a.H / a.heads_per_group;
   if (tid == 0) found = -1;
   __syncthreads();
   for (int r = tid; r < a.rows; r += W_THREADS) {
@@ -116,134 +134,154 @@ __global__ void __launch_bounds__(W_THREADS) walk_prepare_kernel(const WalkArgs 
   if (MODE == WALK_SPACE) {
     const __nv_bfloat16* q = static_cast<const __nv_bfloat16*>(a.q) + t0 * a.q_stride + qk_head * a.D;
     const __nv_bfloat16* k = static_cast<const __nv_bfloat16*>(a.k) + t0 * a.k_stride + qk_head * a.D;
-    for (int e = tid; e < W * (DP / 8); e += W_THREADS) {
-      const int i = e / (DP / 8), c = e % (DP / 8) * 8;
+#pragma unroll
+    for (int u = 0; u < W * (DP / 8) / W_THREADS; ++u) {
+      const int e = tid + u * W_THREADS, i = e / (DP / 8), c = e % (DP / 8) * 8;
       const bool ok = i < n && c < a.D;
       cp_async_16(q_s + i * ST + c, ok ? q + i * a.q_stride + c : q, ok);
       cp_async_16(k_s + i * ST + c, ok ? k + i * a.k_stride + c : k, ok);
     }
     cp_async_commit();
-    // Meanwhile the heads' steps and decays: a warp a head, two tokens a lane, their sum scanned in 64 bits.
-    for (int j = warp; j < a.heads_per_group; j += W_THREADS / 32) {
-      const int h = qk_head * a.heads_per_group + j;
-      const __nv_bfloat16* dt = static_cast<const __nv_bfloat16*>(a.dt) + t0 * a.dt_stride + h;
-      const float rate = expf(a.a_log[h]), bias = a.dt_bias[h];
-      float step[2];
-      double sum[2];
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int i = 2 * lane + u;
-        step[u] = i < n ? walk_softplus(__bfloat162float(dt[i * a.dt_stride]) + bias) : 0.0f;
-        // (a decay below e^-1000 is zero either way; the bound keeps the sums finite)
-        sum[u] = -fmin(static_cast<double>(rate) * static_cast<double>(step[u]), 1000.0) * 1.4426950408889634;
-      }
-      sum[1] += sum[0];
-      double before = sum[1];
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const double other = __shfl_up_sync(0xffffffffu, before, o);
-        if (lane >= o) before += other;
-      }
-      before -= sum[1];
-      float* to = a.steps + (static_cast<long long>(piece) * a.H + h) * W_STEP + 2 * lane;
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const double c = before + sum[u];
-        const float hi = static_cast<float>(c);
-        to[u] = hi;
-        to[W + u] = static_cast<float>(c - hi);
-        to[2 * W + u] = step[u];
-      }
-    }
-    cp_async_wait<0>();
   } else {
     const float* q = static_cast<const float*>(a.q) + t0 * a.q_stride + qk_head * a.D;
     const float* k = static_cast<const float*>(a.k) + t0 * a.k_stride + qk_head * a.D;
-    const bool vectors = a.D % 4 == 0 && a.q_stride % 4 == 0 && a.k_stride % 4 == 0 && reinterpret_cast<uintptr_t>(a.q) % 16 == 0 &&
-                         reinterpret_cast<uintptr_t>(a.k) % 16 == 0;
-#pragma unroll 4
-    for (int e = tid; e < 2 * W * (DP / 4); e += W_THREADS) {
-      const int which = e / (W * (DP / 4)), r = e % (W * (DP / 4)), i = r / (DP / 4), c = r % (DP / 4) * 4;
-      const float* from = which ? k + i * a.k_stride + c : q + i * a.q_stride + c;
-      float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      if (i < n && c < a.D) {
-        if (vectors) {
-          x = *reinterpret_cast<const float4*>(from);
-        } else {
-          x.x = from[0];
-          if (c + 1 < a.D) x.y = from[1];
-          if (c + 2 < a.D) x.z = from[2];
-          if (c + 3 < a.D) x.w = from[3];
+    constexpr int AHEAD = 8;             // loads on their way before the first of them is waited for
+    for (int e0 = tid; e0 < 2 * W * (DP / 4); e0 += W_THREADS * AHEAD) {
+      float4 x[AHEAD];
+#pragma unroll
+      for (int u = 0; u < AHEAD; ++u) {
+        const int e = e0 + u * W_THREADS, r = e % (W * (DP / 4)), i = r / (DP / 4), c = r % (DP / 4) * 4;
+        const float* from = e >= W * (DP / 4) ? k + i * a.k_stride + c : q + i * a.q_stride + c;
+        x[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (i < n && c < a.D) {
+          if (a.vectors) {
+            x[u] = *reinterpret_cast<const float4*>(from);
+          } else {
+            x[u].x = from[0];
+            if (c + 1 < a.D) x[u].y = from[1];
+            if (c + 2 < a.D) x[u].z = from[2];
+            if (c + 3 < a.D) x[u].w = from[3];
+          }
         }
       }
-      unsigned lo[2], hi[2];
-      split_parts<2>(x.x, x.y, lo);
-      split_parts<2>(x.z, x.w, hi);
-      __nv_bfloat16* to = (which ? k_s : q_s) + i * ST + c;
 #pragma unroll
-      for (int p = 0; p < 2; ++p) *reinterpret_cast<uint2*>(to + p * W * ST) = make_uint2(lo[p], hi[p]);
+      for (int u = 0; u < AHEAD; ++u) {
+        const int e = e0 + u * W_THREADS, r = e % (W * (DP / 4)), i = r / (DP / 4), c = r % (DP / 4) * 4;
+        unsigned lo[2], hi[2];
+        split_parts<2>(x[u].x, x[u].y, lo);
+        split_parts<2>(x[u].z, x[u].w, hi);
+        __nv_bfloat16* to = (e >= W * (DP / 4) ? k_s : q_s) + i * ST + c;
+#pragma unroll
+        for (int p = 0; p < 2; ++p) *reinterpret_cast<uint2*>(to + p * W * ST) = make_uint2(lo[p], hi[p]);
+      }
     }
   }
-  __syncthreads();
-  if (MODE == WALK_FIXED) {
-    uint4* to = reinterpret_cast<uint4*>(a.parts + (static_cast<long long>(piece) * a.H + qk_head) * 4 * W * ST);
-    const uint4* from = reinterpret_cast<const uint4*>(q_s);
-    for (int e = tid; e < 4 * W * ST / 8; e += W_THREADS) to[e] = from[e];
+  unsigned char* head = a.heads + (static_cast<long long>(piece) * a.H + h) * Parts::head_bytes;
+  if (warp == 0) {
+    // Steps and decays: two tokens a lane, the sum scanned in 64 bits (in powers of two).
+    float step[2];
+    double sum[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int i = 2 * lane + u;
+      if (MODE == WALK_SPACE) {
+        const __nv_bfloat16* dt = static_cast<const __nv_bfloat16*>(a.dt) + t0 * a.dt_stride + h;
+        step[u] = i < n ? walk_softplus(__bfloat162float(dt[i * a.dt_stride]) + a.dt_bias[h]) : 0.0f;
+        sum[u] = static_cast<double>(expf(a.a_log[h])) * static_cast<double>(step[u]) * 1.4426950408889634;
+      } else {
+        step[u] = i < n ? 1.0f : 0.0f;
+        sum[u] = i < n ? -log2(static_cast<double>(a.decay[h])) : 0.0;
+      }
+      // (a decay below 2^-1000 is zero either way; the bound keeps the sums finite)
+      sum[u] = -fmin(sum[u], 1000.0);
+    }
+    sum[1] += sum[0];
+    double before = sum[1];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double other = __shfl_up_sync(0xffffffffu, before, o);
+      if (lane >= o) before += other;
+    }
+    const double all = __shfl_sync(0xffffffffu, before, 31);
+    before -= sum[1];
+    float* steps = reinterpret_cast<float*>(head + Parts::p_bytes);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int i = 2 * lane + u;
+      const double c = before + sum[u];
+      c_hi[i] = static_cast<float>(c);
+      c_lo[i] = static_cast<float>(c - static_cast<float>(c));
+      s_s[i] = step[u];
+      steps[i] = exp2f(static_cast<float>(c));
+      steps[W + i] = exp2f(static_cast<float>(all - c)) * step[u];
+    }
+    if (lane == 0) steps[2 * W] = exp2f(static_cast<float>(all));
   }
-  // A warp owns 16 rows of the scores and 32 columns.
+  if (MODE == WALK_SPACE) cp_async_wait<0>();
+  __syncthreads();
+  if (h % a.heads_per_group == 0) {
+    uint4* to = reinterpret_cast<uint4*>(a.qk + (static_cast<long long>(piece) * qk_heads + qk_head) * Parts::qk_bytes);
+    const uint4* from = reinterpret_cast<const uint4*>(q_s);
+    for (int e = tid; e < Parts::qk_bytes / 16; e += W_THREADS) to[e] = from[e];
+  }
+  // A warp owns 16 rows of P and 32 columns; what lies behind the diagonal tile is never read.
   const int g = lane >> 2, t = lane & 3, row0 = (warp & 3) * 16, col0 = (warp >> 2) * 32;
-  const int qk_heads = a.H / a.heads_per_group;
-  float* scores = a.scores + (static_cast<long long>(piece) * qk_heads + qk_head) * W * W_GST;
   const int q_off = (row0 + (lane & 7) + ((lane >> 3) & 1) * 8) * ST + (lane >> 4) * 8;
   const int k_off = ((lane & 7) + (lane >> 4) * 8) * ST + ((lane >> 3) & 1) * 8;
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
     const int c0 = col0 + u * 16;
+    if (c0 > row0) continue;
     float s[2][4] = {};
-    if (c0 <= row0 + 15) {                                   // (later keys: never read)
 #pragma unroll
-      for (int ks = 0; ks < DP / 16; ++ks) {
-        unsigned af[PA][4], bf[PA][4];
+    for (int ks = 0; ks < DP / 16; ++ks) {
+      unsigned af[PA][4], bf[PA][4];
 #pragma unroll
-        for (int p = 0; p < PA; ++p) {
-          ldmatrix_x4(af[p], q_s + p * W * ST + q_off + ks * 16);
-          ldmatrix_x4(bf[p], k_s + p * W * ST + c0 * ST + k_off + ks * 16);
-        }
-#pragma unroll
-        for (int pa = PA - 1; pa >= 0; --pa)
-#pragma unroll
-          for (int pb = PA - 1; pb >= 0; --pb)
-            if (counts<PA, PA>(pa, pb)) {
-              mma_bf16_16816(s[0], af[pa], bf[pb][0], bf[pb][1]);
-              mma_bf16_16816(s[1], af[pa], bf[pb][2], bf[pb][3]);
-            }
+      for (int p = 0; p < PA; ++p) {
+        ldmatrix_x4(af[p], q_s + p * W * ST + q_off + ks * 16);
+        ldmatrix_x4(bf[p], k_s + p * W * ST + c0 * ST + k_off + ks * 16);
       }
+#pragma unroll
+      for (int pa = PA - 1; pa >= 0; --pa)
+#pragma unroll
+        for (int pb = PA - 1; pb >= 0; --pb)
+          if (counts<PA, PA>(pa, pb)) {
+            mma_bf16_16816(s[0], af[pa], bf[pb][0], bf[pb][1]);
+            mma_bf16_16816(s[1], af[pa], bf[pb][2], bf[pb][3]);
+          }
     }
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      float* to = scores + (row0 + g) * W_GST + c0 + 8 * i + 2 * t;
-      *reinterpret_cast<float2*>(to) = make_float2(s[i][0], s[i][1]);
-      *reinterpret_cast<float2*>(to + 8 * W_GST) = make_float2(s[i][2], s[i][3]);
-    }
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const int at = row0 + g + 8 * r, j = c0 + 8 * i + 2 * t;
+        float x[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          x[e] = j + e <= at ? s[i][2 * r + e] * (exp2f((c_hi[at] - c_hi[j + e]) + (c_lo[at] - c_lo[j + e])) * s_s[j + e]) : 0.0f;
+        unsigned part[PB];
+        split_parts<PB>(x[0], x[1], part);
+#pragma unroll
+        for (int p = 0; p < PB; ++p)
+          *reinterpret_cast<unsigned*>(head + ((p * W + at) * W_PST + j) * 2) = part[p];
+      }
   }
 }
 
 template <int MODE, int DP, int NT>
-struct WalkShape {
-  static constexpr int PA = MODE == WALK_SPACE ? 1 : 2;      // parts of q, k and v
-  static constexpr int PB = MODE == WALK_SPACE ? 3 : 2;      // parts of the state, the weights and the weighted values
-  static constexpr int ST = DP + 8, COLS = 8 * NT, CST = COLS + 8, OST = COLS + 4;
-  static constexpr int STAGES = MODE == WALK_SPACE ? 3 : 2;
-  static constexpr int qk_bytes = 2 * PA * W * ST * 2;
-  static constexpr int stage_bytes = qk_bytes + W * W_GST * 4 + (MODE == WALK_SPACE ? W_STEP * 4 : 0);
-  static constexpr int smem = STAGES * stage_bytes + PB * DP * CST * 2 + (PA + PB) * W * CST * 2 + W * OST * 4;
+struct WalkShape : WalkParts<MODE, DP> {
+  using Parts = WalkParts<MODE, DP>;
+  static constexpr int COLS = 8 * NT, CST = COLS + 8, OST = COLS + 4, STAGES = 2;
+  static constexpr int stage_bytes = Parts::qk_bytes + Parts::head_bytes;
+  static constexpr int smem =
+      STAGES * stage_bytes + Parts::PB * DP * CST * 2 + (Parts::PA + Parts::PB) * W * CST * 2 + W * OST * 4;
 };
 
 // NT: tiles of 8 value columns of a CTA.  Warp w owns the state's channels 16 w .. (C fragments); for the outputs it owns
-// tokens 16 (w % 4) .. and takes half the channels (S^T q) and every other 16 keys (the scores).  A piece:
+// tokens 16 (w % 4) .. and takes half the channels (S^T q) and every other 16 keys (P).  A piece:
 //   barrier; both terms of the outputs and the state's sums from shared memory; one half of the outputs' sums to shared memory;
 //   barrier; the other half adds it and writes; the state and the next piece's values go to shared memory in parts.
-// The next pieces' operands are copied meanwhile.
+// The next piece comes meanwhile, in two bulk copies.
 template <int MODE, int DP, int NT>
 __global__ void __launch_bounds__(W_THREADS) state_walk_kernel(const WalkArgs a) {
   using Shape = WalkShape<MODE, DP, NT>;
@@ -252,9 +290,9 @@ __global__ void __launch_bounds__(W_THREADS) state_walk_kernel(const WalkArgs a)
   extern __shared__ __align__(16) unsigned char w_smem[];
   __nv_bfloat16* s_s = reinterpret_cast<__nv_bfloat16*>(w_smem + STAGES * Shape::stage_bytes);    // [PB][DP][CST]
   __nv_bfloat16* v_s = s_s + PB * DP * CST;                  // [PA][W][CST]
-  __nv_bfloat16* wv_s = v_s + PA * W * CST;                  // [PB][W][CST]: e^(c_n - c_j) s_j v_j
+  __nv_bfloat16* wv_s = v_s + PA * W * CST;                  // [PB][W][CST]: w_j v_j
   float* o_s = reinterpret_cast<float*>(wv_s + PB * W * CST);            // [W][OST]
-  __shared__ float power_s[W + 1];                           // WALK_FIXED: a^0 .. a^W
+  __shared__ unsigned long long landed[STAGES];
   const int row = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * COLS;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int slot = a.slots[row];
@@ -265,59 +303,51 @@ __global__ void __launch_bounds__(W_THREADS) state_walk_kernel(const WalkArgs a)
   const int n_all = a.row_q_len[row], pieces = (n_all + W - 1) / W;
   const long long t0 = a.row_q_start[row];
   const int first = walk_first_piece(a, row), qk_head = h / a.heads_per_group, qk_heads = a.H / a.heads_per_group;
-  if (MODE == WALK_FIXED && tid <= W) power_s[tid] = powf(a.decay[h], static_cast<float>(tid));
-  if (MODE == WALK_SPACE && a.D < DP)                        // the channels beyond D: zeros in every stage
-    for (int e = tid; e < STAGES * 2 * W * (DP / 8); e += W_THREADS) {
-      const int c = e % (DP / 8) * 8, r = e / (DP / 8);
-      if (c >= a.D)
-        *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(w_smem + r / (2 * W) * Shape::stage_bytes) + r % (2 * W) * ST + c) =
-            make_uint4(0, 0, 0, 0);
-    }
-
-  auto copy_piece = [&](int p) {
-    unsigned char* stage = w_smem + p % STAGES * Shape::stage_bytes;
-    if (MODE == WALK_SPACE) {
-      __nv_bfloat16* q_s = reinterpret_cast<__nv_bfloat16*>(stage);
-      const int n = min(W, n_all - p * W), chunks = a.D / 8;
-      const __nv_bfloat16* q = static_cast<const __nv_bfloat16*>(a.q) + (t0 + p * W) * a.q_stride + qk_head * a.D;
-      const __nv_bfloat16* k = static_cast<const __nv_bfloat16*>(a.k) + (t0 + p * W) * a.k_stride + qk_head * a.D;
+  if (tid == 0) {
 #pragma unroll
-      for (int u = 0; u < W * (DP / 8) / W_THREADS; ++u) {
-        const int e = tid + u * W_THREADS, i = e / (DP / 8), c = e % (DP / 8);
-        if (c >= chunks) continue;
-        cp_async_16(q_s + i * ST + 8 * c, i < n ? q + i * a.q_stride + 8 * c : q, i < n);
-        cp_async_16(q_s + (W + i) * ST + 8 * c, i < n ? k + i * a.k_stride + 8 * c : k, i < n);
-      }
-      const float* steps = a.steps + (static_cast<long long>(first + p) * a.H + h) * W_STEP;
-      if (tid < W_STEP / 4) cp_async_16(stage + Shape::qk_bytes + W * W_GST * 4 + tid * 16, steps + tid * 4, true);
-    } else {
-      const __nv_bfloat16* parts = a.parts + (static_cast<long long>(first + p) * a.H + h) * 4 * W * ST;
-      for (int e = tid; e < Shape::qk_bytes / 16; e += W_THREADS) cp_async_16(stage + e * 16, parts + e * 8, true);
-    }
-    const float* scores = a.scores + (static_cast<long long>(first + p) * qk_heads + qk_head) * W * W_GST;
-    for (int e = tid; e < W * W_GST / 4; e += W_THREADS) cp_async_16(stage + Shape::qk_bytes + e * 16, scores + e * 4, true);
+    for (int i = 0; i < STAGES; ++i) mbar_init(&landed[i], 1);
+    fence_barrier_init();
+  }
+  __syncthreads();
+
+  auto copy_piece = [&](int p) {                             // one thread
+    unsigned char* stage = w_smem + p % STAGES * Shape::stage_bytes;
+    unsigned long long* bar = &landed[p % STAGES];
+    mbar_arrive_expect_tx(bar, Shape::stage_bytes);
+    bulk_copy_g2s(stage, a.qk + (static_cast<long long>(first + p) * qk_heads + qk_head) * Shape::qk_bytes, Shape::qk_bytes, bar);
+    bulk_copy_g2s(stage + Shape::qk_bytes, a.heads + (static_cast<long long>(first + p) * a.H + h) * Shape::head_bytes,
+                  Shape::head_bytes, bar);
   };
-  // This thread's values of a piece: pairs of columns (my_c, my_c + 1) of tokens my_i, my_i + W / PER, ...; with their weights.
+  // This thread's values of a piece: columns my_c and my_c + 1 of tokens my_i, my_i + TOKENS, ..., and their weights.
   constexpr int TOKENS = W / PER;
   const int my_c = tid % (COLS / 2) * 2, my_i = tid / (COLS / 2);
   float value[PER][2], weight[PER];
-  auto fetch_values = [&](int p) {
+  unsigned raw[PER];
+  const bool col0 = v0 + my_c < a.V, col1 = v0 + my_c + 1 < a.V;
+  auto fetch_values = [&](int p) {                           // (nothing here waits for what it loads)
+    const float* w = reinterpret_cast<const float*>(a.heads + (static_cast<long long>(first + p) * a.H + h) * Shape::head_bytes +
+                                                    Shape::p_bytes) + W;
 #pragma unroll
     for (int u = 0; u < PER; ++u) {
       const int i = my_i + u * TOKENS, at = p * W + i, n = min(W, n_all - p * W);
       value[u][0] = value[u][1] = weight[u] = 0.0f;
+      raw[u] = 0;
       if (p >= pieces || i >= n) continue;
+      weight[u] = w[i];
       if (MODE == WALK_SPACE) {
-        const __nv_bfloat16* v = static_cast<const __nv_bfloat16*>(a.v) + (t0 + at) * a.v_stride + h * a.V + v0 + my_c;
-        if (v0 + my_c < a.V) value[u][0] = __bfloat162float(v[0]);
-        if (v0 + my_c + 1 < a.V) value[u][1] = __bfloat162float(v[1]);
-        const float* c = a.steps + (static_cast<long long>(first + p) * a.H + h) * W_STEP;
-        weight[u] = exp2f((c[W - 1] - c[i]) + (c[2 * W - 1] - c[W + i])) * c[2 * W + i];
+        const unsigned short* v = static_cast<const unsigned short*>(a.v) + (t0 + at) * a.v_stride + h * a.V + v0 + my_c;
+        if (a.pairs && col1) raw[u] = *reinterpret_cast<const unsigned*>(v);
+        else if (col0) raw[u] = v[0] | (col1 ? static_cast<unsigned>(v[1]) << 16 : 0u);
       } else {
         const float* v = static_cast<const float*>(a.v) + (t0 + at) * a.v_stride + h * a.V + v0 + my_c;
-        if (v0 + my_c < a.V) value[u][0] = v[0];
-        if (v0 + my_c + 1 < a.V) value[u][1] = v[1];
-        weight[u] = power_s[n - 1 - i];
+        if (a.pairs && col1) {
+          const float2 x = *reinterpret_cast<const float2*>(v);
+          value[u][0] = x.x;
+          value[u][1] = x.y;
+        } else {
+          if (col0) value[u][0] = v[0];
+          if (col1) value[u][1] = v[1];
+        }
       }
     }
   };
@@ -326,7 +356,13 @@ __global__ void __launch_bounds__(W_THREADS) state_walk_kernel(const WalkArgs a)
     for (int u = 0; u < PER; ++u) {
       const int at = (my_i + u * TOKENS) * CST + my_c;
       unsigned vp[PA], wp[PB];
-      split_parts<PA>(value[u][0], value[u][1], vp);
+      if (MODE == WALK_SPACE) {
+        vp[0] = raw[u];
+        value[u][0] = __uint_as_float(raw[u] << 16);
+        value[u][1] = __uint_as_float(raw[u] & 0xffff0000u);
+      } else {
+        split_parts<PA>(value[u][0], value[u][1], vp);
+      }
       split_parts<PB>(value[u][0] * weight[u], value[u][1] * weight[u], wp);
 #pragma unroll
       for (int p = 0; p < PA; ++p) *reinterpret_cast<unsigned*>(v_s + p * W * CST + at) = vp[p];
@@ -358,80 +394,60 @@ __global__ void __launch_bounds__(W_THREADS) state_walk_kernel(const WalkArgs a)
         for (int p = 0; p < PB; ++p) *reinterpret_cast<unsigned*>(s_s + (p * DP + d0 + 8 * half) * CST + 8 * i + 2 * t) = sp[p];
       }
   };
-  if (MODE == WALK_FIXED) __syncthreads();                   // the powers
+  if (tid == 0 && pieces > 0) copy_piece(0);
   store_state();
   fetch_values(0);
   store_values();
-#pragma unroll
-  for (int p = 0; p < STAGES - 1; ++p) {
-    if (p < pieces) copy_piece(p);
-    cp_async_commit();
-  }
   const float skip = MODE == WALK_SPACE ? a.skip[h] : 0.0f;
-  // ldmatrix addresses: A rows as they lie, A transposed, B as [k][n].
-  const int a_off = ((lane & 7) + ((lane >> 3) & 1) * 8) * ST + (lane >> 4) * 8;
+  // ldmatrix addresses: A rows as they lie, P's likewise, A transposed, B as [k][n].
+  const int lrow = (lane & 7) + ((lane >> 3) & 1) * 8, lcol = (lane >> 4) * 8;
+  const int a_off = lrow * ST + lcol, p_off = lrow * W_PST + lcol, b_off = lrow * CST + lcol;
   const int at_off = ((lane & 7) + (lane >> 4) * 8) * ST + ((lane >> 3) & 1) * 8;
-  const int b_off = ((lane & 7) + ((lane >> 3) & 1) * 8) * CST + (lane >> 4) * 8;
   const int row0 = (warp & 3) * 16, half = warp >> 2;
   for (int p = 0; p < pieces; ++p) {
     const unsigned char* stage = w_smem + p % STAGES * Shape::stage_bytes;
     const __nv_bfloat16* q_s = reinterpret_cast<const __nv_bfloat16*>(stage);              // [PA][W][ST]
     const __nv_bfloat16* k_s = q_s + PA * W * ST;
-    const float* scores = reinterpret_cast<const float*>(stage + Shape::qk_bytes);
-    const float* c_s = scores + W * W_GST;
+    const __nv_bfloat16* p_s = reinterpret_cast<const __nv_bfloat16*>(stage + Shape::qk_bytes);        // [PB][W][W_PST]
+    const float* steps = reinterpret_cast<const float*>(stage + Shape::qk_bytes + Shape::p_bytes);
     const int n = min(W, n_all - p * W);
-    cp_async_wait<STAGES - 2>();
-    __syncthreads();               // the piece, the state and the values are there; the buffer of the piece before is free
-    if (p + STAGES - 1 < pieces) copy_piece(p + STAGES - 1);
-    cp_async_commit();
+    const bool here = mbar_wait(&landed[p % STAGES], (p / STAGES) & 1, W_WAIT_LIMIT);
+    // The piece, the state and the values are there; the buffer of the piece before is free.
+    if (!__syncthreads_and(here)) {
+      if (tid == 0) report(a.status, STATUS_COPY_TIMEOUT, p, row);
+      return;
+    }
+    if (tid == 0 && p + 1 < pieces) copy_piece(p + 1);
     fetch_values(p + 1);
     const int i0 = row0 + g, i1 = i0 + 8;
-    float c_hi[2] = {}, c_lo[2] = {}, lead[2];
-    if (MODE == WALK_SPACE) {
-      c_hi[0] = c_s[i0]; c_hi[1] = c_s[i1];
-      c_lo[0] = c_s[W + i0]; c_lo[1] = c_s[W + i1];
-      lead[0] = exp2f(c_hi[0] + c_lo[0]); lead[1] = exp2f(c_hi[1] + c_lo[1]);
-    } else {
-      lead[0] = power_s[i0 + 1]; lead[1] = power_s[i1 + 1];
-    }
     float o[NT][4] = {};
     if (row0 < n) {
 #pragma unroll
       for (int ks = 0; ks < DP / 32; ++ks) {
         const int d = half * (DP / 2) + ks * 16;
         unsigned af[PA][4];
+        WalkB<NT, PB> b;
 #pragma unroll
         for (int x = 0; x < PA; ++x) ldmatrix_x4(af[x], q_s + (x * W + row0) * ST + a_off + d);
-        walk_product<NT, PA, PB>(o, af, s_s + d * CST + b_off, DP * CST);
+        b.load(s_s + d * CST + b_off, DP * CST);
+        walk_product<NT, PA, PB>(o, af, b);
       }
+      const float lead0 = steps[i0], lead1 = steps[i1];
 #pragma unroll
       for (int i = 0; i < NT; ++i) {
-        o[i][0] *= lead[0]; o[i][1] *= lead[0];
-        o[i][2] *= lead[1]; o[i][3] *= lead[1];
+        o[i][0] *= lead0; o[i][1] *= lead0;
+        o[i][2] *= lead1; o[i][3] *= lead1;
       }
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         const int j0 = (half + 2 * u) * 16;
         if (j0 > row0) continue;
-        unsigned pf[PB][4];                                  // the decayed scores, in parts
+        unsigned pf[PB][4];
+        WalkB<NT, PA> b;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {                        // rows (e & 1), columns 2 t + 8 (e >> 1) and the next
-          const int i = e & 1 ? i1 : i0, j = j0 + 2 * t + 8 * (e >> 1);
-          const float2 s = *reinterpret_cast<const float2*>(scores + i * W_GST + j);
-          float x, y;
-          if (MODE == WALK_SPACE) {
-            x = j <= i ? s.x * (exp2f((c_hi[e & 1] - c_s[j]) + (c_lo[e & 1] - c_s[W + j])) * c_s[2 * W + j]) : 0.0f;
-            y = j + 1 <= i ? s.y * (exp2f((c_hi[e & 1] - c_s[j + 1]) + (c_lo[e & 1] - c_s[W + j + 1])) * c_s[2 * W + j + 1]) : 0.0f;
-          } else {
-            x = j <= i ? s.x * power_s[i - j] : 0.0f;
-            y = j + 1 <= i ? s.y * power_s[i - j - 1] : 0.0f;
-          }
-          unsigned xy[PB];
-          split_parts<PB>(x, y, xy);
-#pragma unroll
-          for (int q = 0; q < PB; ++q) pf[q][e] = xy[q];
-        }
-        walk_product<NT, PB, PA>(o, pf, v_s + j0 * CST + b_off, W * CST);
+        for (int x = 0; x < PB; ++x) ldmatrix_x4(pf[x], p_s + (x * W + row0) * W_PST + p_off + j0);
+        b.load(v_s + j0 * CST + b_off, W * CST);
+        walk_product<NT, PB, PA>(o, pf, b);
       }
       if (half == 1) {
 #pragma unroll
@@ -453,19 +469,20 @@ __global__ void __launch_bounds__(W_THREADS) state_walk_kernel(const WalkArgs a)
       float sum[NT][4] = {};
 #pragma unroll
       for (int ks = 0; ks < W / 16; ++ks) {
-        if (ks * 16 >= n) continue;
         unsigned af[PA][4];
+        WalkB<NT, PB> b;
 #pragma unroll
         for (int x = 0; x < PA; ++x) ldmatrix_x4_trans(af[x], k_s + (x * W + ks * 16) * ST + at_off + warp * 16);
-        walk_product<NT, PA, PB>(sum, af, wv_s + ks * 16 * CST + b_off, W * CST);
+        b.load(wv_s + ks * 16 * CST + b_off, W * CST);
+        walk_product<NT, PA, PB>(sum, af, b);
       }
-      const float whole = MODE == WALK_SPACE ? exp2f(c_s[W - 1] + c_s[2 * W - 1]) : power_s[n];
+      const float whole = steps[2 * W];
 #pragma unroll
       for (int i = 0; i < NT; ++i)
 #pragma unroll
         for (int e = 0; e < 4; ++e) S[i][e] = fmaf(whole, S[i][e], sum[i][e]);
     }
-    __syncthreads();               // the state's, the values' and the other half's reads are done
+    __syncthreads();               // the state's, the values' and the piece's reads are done
     store_state();
     store_values();
     if (half == 0 && row0 < n) {
@@ -486,7 +503,6 @@ __global__ void __launch_bounds__(W_THREADS) state_walk_kernel(const WalkArgs a)
         }
     }
   }
-  cp_async_wait<0>();
   if (!a.write_state || !holds) return;
 #pragma unroll
   for (int i = 0; i < NT; ++i)
@@ -501,13 +517,13 @@ template <int MODE, int DP, int NT>
 static int walk_launch(const WalkArgs& a, int pieces, cudaStream_t s) {
   using Shape = WalkShape<MODE, DP, NT>;
   static_assert(Shape::smem + 1024 <= 227 * 1024, "what a CTA keeps fits in shared memory");
-  const int prepare_smem = Shape::qk_bytes;
+  static_assert(Shape::qk_bytes % 16 == 0 && Shape::head_bytes % 16 == 0, "bulk copies move 16-byte pieces");
   auto prepare = walk_prepare_kernel<MODE, DP>;
   auto walk = state_walk_kernel<MODE, DP, NT>;
-  if (cuda_failed(cudaFuncSetAttribute(prepare, cudaFuncAttributeMaxDynamicSharedMemorySize, prepare_smem)) ||
+  if (cuda_failed(cudaFuncSetAttribute(prepare, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::qk_bytes)) ||
       cuda_failed(cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::smem)))
     return ERR_CUDA;
-  prepare<<<dim3(pieces, a.H / a.heads_per_group), W_THREADS, prepare_smem, s>>>(a);
+  prepare<<<dim3(pieces, a.H), W_THREADS, Shape::qk_bytes, s>>>(a);
   walk<<<dim3(a.rows, a.H, (a.V + Shape::COLS - 1) / Shape::COLS), W_THREADS, Shape::smem, s>>>(a);
   return launch_result();
 }
@@ -529,8 +545,12 @@ ZB_API int zb_walk_max_channels() { return 128; }
 ZB_API int zb_walk_piece_tokens() { return W; }
 // Floats of workspace a piece needs.
 ZB_API int zb_walk_piece_floats(int mode, int H, int heads_per_group, int D) {
-  const int dp = D <= 64 ? 64 : 128;
-  return mode == WALK_SPACE ? H / heads_per_group * W * W_GST + H * W_STEP : H * (W * W_GST + 2 * W * (dp + 8));
+  if (mode == WALK_SPACE) {
+    const int qk = D <= 64 ? WalkParts<WALK_SPACE, 64>::qk_bytes : WalkParts<WALK_SPACE, 128>::qk_bytes;
+    return (H / heads_per_group * qk + H * WalkParts<WALK_SPACE, 64>::head_bytes) / 4;
+  }
+  const int qk = D <= 64 ? WalkParts<WALK_FIXED, 64>::qk_bytes : WalkParts<WALK_FIXED, 128>::qk_bytes;
+  return H * (qk + WalkParts<WALK_FIXED, 64>::head_bytes) / 4;
 }
 
 // mode 0 (state space): q, k, v, dt bfloat16; q, k and their rows on 16-byte boundaries, D a multiple of 8.  mode 1 (fixed
@@ -552,14 +572,16 @@ ZB_API int zb_state_walk(int mode, float* out, const void* q, long long q_stride
       (mode == WALK_SPACE && (D % 8 != 0 || q_stride % 8 != 0 || k_stride % 8 != 0 || !aligned(q) || !aligned(k))))
     return ERR_BAD_ARGUMENT;
   const int pieces = tokens / W + rows, qk_heads = H / heads_per_group;
-  if (qk_heads > 65535) return ERR_UNSUPPORTED;
   WalkArgs a;
   a.q = q; a.q_stride = q_stride; a.k = k; a.k_stride = k_stride; a.v = v; a.v_stride = v_stride; a.dt = dt; a.dt_stride = dt_stride;
   a.dt_bias = dt_bias; a.a_log = a_log; a.skip = skip; a.decay = decay;
-  a.scores = ws;
-  a.steps = ws + static_cast<long long>(pieces) * qk_heads * W * W_GST;
-  a.parts = reinterpret_cast<__nv_bfloat16*>(a.steps);
+  a.qk = reinterpret_cast<unsigned char*>(ws);
+  const int qk_bytes = mode == WALK_SPACE ? (D <= 64 ? WalkParts<WALK_SPACE, 64>::qk_bytes : WalkParts<WALK_SPACE, 128>::qk_bytes)
+                                          : (D <= 64 ? WalkParts<WALK_FIXED, 64>::qk_bytes : WalkParts<WALK_FIXED, 128>::qk_bytes);
+  a.heads = a.qk + static_cast<long long>(pieces) * qk_heads * qk_bytes;
+  a.vectors = mode == WALK_SPACE || (D % 4 == 0 && q_stride % 4 == 0 && k_stride % 4 == 0 && aligned(q) && aligned(k));
   a.out = out; a.state = state; a.slot_stride = slot_stride; a.slots = slots; a.row_q_start = row_q_start; a.row_q_len = row_q_len;
+  a.pairs = V % 2 == 0 && v_stride % 2 == 0 && reinterpret_cast<uintptr_t>(v) % (mode == WALK_SPACE ? 4 : 8) == 0;
   a.rows = rows; a.H = H; a.D = D; a.V = V; a.heads_per_group = heads_per_group; a.num_slots = num_slots; a.write_state = write_state;
   a.status = status;
   auto s = static_cast<cudaStream_t>(stream);
