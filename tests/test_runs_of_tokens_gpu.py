@@ -111,3 +111,31 @@ def test_the_state_space_walk(cuda_device, heads, per, dim, vdim):
         # float32 sums of products that are exact, decays good to a few roundings.
         assert (out[start:start + n].cpu().double() - expected).abs().max() <= 3e-6 * max(1.0, float(expected.abs().max()))
         assert (held[slot].cpu().double() - S.reshape(-1)).abs().max() <= 3e-6 * max(1.0, float(S.abs().max()))
+
+
+@pytest.mark.parametrize("heads,dim,vdim,rot", [(3, 128, 40, 128), (2, 64, 32, 24), (5, 100, 130, 8), (1, 8, 5, 8)])
+def test_retention_turns_its_queries_and_keys(cuda_device, heads, dim, vdim, rot):
+    """The same portions with q and k turned beforehand and turned on the way into the walk."""
+    from zephyr_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(dim + vdim)
+    lengths, slots = [64, 100, 7, 130], [1, 0, 3, 2]
+    T, hd = sum(lengths), heads * dim
+    dev = lambda t: t.to(cuda_device)
+    projected = dev(torch.randn(T, (2 * hd + heads * vdim + 3) // 4 * 4, generator=g))
+    freqs = dev(10000.0 ** (-torch.arange(rot // 2) / (rot // 2)))
+    i32 = lambda values: torch.tensor(values, dtype=torch.int32, device=cuda_device)
+    positions = i32([p + 500 * r for r, n in enumerate(lengths) for p in range(n)])
+    decay = dev(1.0 - 2.0 ** -(1.0 + 3.0 * torch.arange(heads)))
+    starts = [sum(lengths[:i]) for i in range(len(lengths))]
+    status, got = ops.new_status(cuda_device), []
+    turned = ops.rotate_qk(projected, heads, dim, freqs, rot, dim ** -0.5, positions)
+    for q, k, turn in ((turned[:, :hd], turned[:, hd:], {}),
+                       (projected[:, :hd], projected[:, hd:2 * hd], dict(freqs=freqs, rot_dims=rot, k_scale=dim ** -0.5, positions=positions))):
+        assert not turn or ops.retention_turns(q, k, dim, rot)
+        state = torch.ones(4, hd * vdim, device=cuda_device)
+        got.append((ops.retention(q, k, projected[:, 2 * hd:2 * hd + heads * vdim], decay, heads, dim, vdim, state, i32(slots), i32(starts),
+                                  i32(lengths), status, **turn), state))
+    ops.check_status(status)
+    for x, y in zip(*got):       # the same float32 rotation, at most a rounding apart ahead of the split
+        assert (x - y).abs().max() <= 4e-6 * max(1.0, float(x.abs().max()))

@@ -50,6 +50,9 @@ struct WalkArgs {
   float* state; long long slot_stride;   // slot s at state + s * slot_stride: [H][D][V]
   const int* slots; const int* row_q_start; const int* row_q_len;
   int rows, H, D, V, heads_per_group, num_slots, write_state;
+  const float* freqs; const int* positions;      // WALK_FIXED: null, or q and k are still to be turned (as rotate_qk does)
+  int rot_dims;
+  float k_scale;
   int vectors, pairs;                    // rows of q and k move as 16-byte pieces; neighbouring values of v move together
   int* status;
 };
@@ -108,16 +111,20 @@ __device__ __forceinline__ void walk_product(float (&acc)[N][4], const unsigned 
 
 __device__ __forceinline__ int walk_first_piece(const WalkArgs& a, int row) { return a.row_q_start[row] / W + row; }
 
-// A piece of one head.  DP: the channels padded with zeros.
+// A piece of one q/k head and up to W_HEADS of the heads that share it (their scores are the same).  DP: the channels padded
+// with zeros.
+constexpr int W_HEADS = 4;
 template <int MODE, int DP>
 __global__ void __launch_bounds__(W_THREADS) walk_prepare_kernel(const WalkArgs a) {
   using Parts = WalkParts<MODE, DP>;
-  constexpr int ST = Parts::ST, PA = Parts::PA, PB = Parts::PB;
+  constexpr int ST = Parts::ST, PA = Parts::PA, PB = Parts::PB, HEADS = MODE == WALK_SPACE ? W_HEADS : 1;
   extern __shared__ __align__(16) unsigned char w_smem[];
   __shared__ int found;
-  __shared__ float c_hi[W], c_lo[W], s_s[W];
-  const int piece = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int qk_head = h / a.heads_per_group, qk_heads = a.H / a.heads_per_group;
+  __shared__ float c_hi[HEADS][W], c_lo[HEADS][W], s_s[HEADS][W];
+  const int piece = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int runs = (a.heads_per_group + HEADS - 1) / HEADS;              // runs of heads in a group
+  const int qk_head = blockIdx.y / runs, first_head = blockIdx.y % runs * HEADS, qk_heads = a.H / a.heads_per_group;
+  const int heads = min(HEADS, a.heads_per_group - first_head), h0 = qk_head * a.heads_per_group + first_head;
   if (tid == 0) found = -1;
   __syncthreads();
   for (int r = tid; r < a.rows; r += W_THREADS) {
@@ -145,15 +152,52 @@ __global__ void __launch_bounds__(W_THREADS) walk_prepare_kernel(const WalkArgs 
   } else {
     const float* q = static_cast<const float*>(a.q) + t0 * a.q_stride + qk_head * a.D;
     const float* k = static_cast<const float*>(a.k) + t0 * a.k_stride + qk_head * a.D;
+    const int half = a.freqs != nullptr ? a.rot_dims / 2 : 0;
+    // Values that turn: four pairs of q and four of k a thread and step, on one set of angles.
+    for (int e = tid; e < W * (half / 4); e += W_THREADS) {
+      const int i = e / (half / 4), c = e % (half / 4) * 4;
+      float4 x[2][2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+          x[u][w] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          if (i < n) x[u][w] = *reinterpret_cast<const float4*>((u ? k + i * a.k_stride : q + i * a.q_stride) + c + w * half);
+        }
+      const float pos = i < n ? static_cast<float>(a.positions[t0 + i]) : 0.0f;
+      float sn[4], cs[4];
+#pragma unroll
+      for (int w = 0; w < 4; ++w) sincosf(pos * a.freqs[c + w], &sn[w], &cs[w]);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const float scale = u ? a.k_scale : 1.0f;
+        const float4 y = x[u][0], z = x[u][1];
+        const float4 out[2] = {make_float4((y.x * cs[0] - z.x * sn[0]) * scale, (y.y * cs[1] - z.y * sn[1]) * scale,
+                                           (y.z * cs[2] - z.z * sn[2]) * scale, (y.w * cs[3] - z.w * sn[3]) * scale),
+                               make_float4((z.x * cs[0] + y.x * sn[0]) * scale, (z.y * cs[1] + y.y * sn[1]) * scale,
+                                           (z.z * cs[2] + y.z * sn[2]) * scale, (z.w * cs[3] + y.w * sn[3]) * scale)};
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+          unsigned lo[2], hi[2];
+          split_parts<2>(out[w].x, out[w].y, lo);
+          split_parts<2>(out[w].z, out[w].w, hi);
+          __nv_bfloat16* to = (u ? k_s : q_s) + i * ST + c + w * half;
+#pragma unroll
+          for (int p = 0; p < 2; ++p) *reinterpret_cast<uint2*>(to + p * W * ST) = make_uint2(lo[p], hi[p]);
+        }
+      }
+    }
+    const float passing = a.freqs != nullptr ? a.k_scale : 1.0f;         // what does not turn, k times its multiplier
+    const int from_c = 2 * half, quads = (DP - from_c) / 4;
     constexpr int AHEAD = 8;             // loads on their way before the first of them is waited for
-    for (int e0 = tid; e0 < 2 * W * (DP / 4); e0 += W_THREADS * AHEAD) {
+    for (int e0 = tid; e0 < 2 * W * quads; e0 += W_THREADS * AHEAD) {
       float4 x[AHEAD];
 #pragma unroll
       for (int u = 0; u < AHEAD; ++u) {
-        const int e = e0 + u * W_THREADS, r = e % (W * (DP / 4)), i = r / (DP / 4), c = r % (DP / 4) * 4;
-        const float* from = e >= W * (DP / 4) ? k + i * a.k_stride + c : q + i * a.q_stride + c;
+        const int e = e0 + u * W_THREADS, r = e % (W * quads), i = r / quads, c = from_c + r % quads * 4;
+        const float* from = e >= W * quads ? k + i * a.k_stride + c : q + i * a.q_stride + c;
         x[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (i < n && c < a.D) {
+        if (e < 2 * W * quads && i < n && c < a.D) {
           if (a.vectors) {
             x[u] = *reinterpret_cast<const float4*>(from);
           } else {
@@ -166,18 +210,21 @@ __global__ void __launch_bounds__(W_THREADS) walk_prepare_kernel(const WalkArgs 
       }
 #pragma unroll
       for (int u = 0; u < AHEAD; ++u) {
-        const int e = e0 + u * W_THREADS, r = e % (W * (DP / 4)), i = r / (DP / 4), c = r % (DP / 4) * 4;
+        const int e = e0 + u * W_THREADS, r = e % (W * quads), i = r / quads, c = from_c + r % quads * 4;
+        if (e >= 2 * W * quads) break;
+        const float scale = e >= W * quads ? passing : 1.0f;
         unsigned lo[2], hi[2];
-        split_parts<2>(x[u].x, x[u].y, lo);
-        split_parts<2>(x[u].z, x[u].w, hi);
-        __nv_bfloat16* to = (e >= W * (DP / 4) ? k_s : q_s) + i * ST + c;
+        split_parts<2>(x[u].x * scale, x[u].y * scale, lo);
+        split_parts<2>(x[u].z * scale, x[u].w * scale, hi);
+        __nv_bfloat16* to = (e >= W * quads ? k_s : q_s) + i * ST + c;
 #pragma unroll
         for (int p = 0; p < 2; ++p) *reinterpret_cast<uint2*>(to + p * W * ST) = make_uint2(lo[p], hi[p]);
       }
     }
   }
-  unsigned char* head = a.heads + (static_cast<long long>(piece) * a.H + h) * Parts::head_bytes;
-  if (warp == 0) {
+  unsigned char* head0 = a.heads + (static_cast<long long>(piece) * a.H + h0) * Parts::head_bytes;
+  if (warp < heads) {
+    const int h = h0 + warp;
     // Steps and decays: two tokens a lane, the sum scanned in 64 bits (in powers of two).
     float step[2];
     double sum[2];
@@ -204,14 +251,14 @@ __global__ void __launch_bounds__(W_THREADS) walk_prepare_kernel(const WalkArgs 
     }
     const double all = __shfl_sync(0xffffffffu, before, 31);
     before -= sum[1];
-    float* steps = reinterpret_cast<float*>(head + Parts::p_bytes);
+    float* steps = reinterpret_cast<float*>(head0 + warp * Parts::head_bytes + Parts::p_bytes);
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const int i = 2 * lane + u;
       const double c = before + sum[u];
-      c_hi[i] = static_cast<float>(c);
-      c_lo[i] = static_cast<float>(c - static_cast<float>(c));
-      s_s[i] = step[u];
+      c_hi[warp][i] = static_cast<float>(c);
+      c_lo[warp][i] = static_cast<float>(c - static_cast<float>(c));
+      s_s[warp][i] = step[u];
       steps[i] = exp2f(static_cast<float>(c));
       steps[W + i] = exp2f(static_cast<float>(all - c)) * step[u];
     }
@@ -219,7 +266,7 @@ __global__ void __launch_bounds__(W_THREADS) walk_prepare_kernel(const WalkArgs 
   }
   if (MODE == WALK_SPACE) cp_async_wait<0>();
   __syncthreads();
-  if (h % a.heads_per_group == 0) {
+  if (first_head == 0) {
     uint4* to = reinterpret_cast<uint4*>(a.qk + (static_cast<long long>(piece) * qk_heads + qk_head) * Parts::qk_bytes);
     const uint4* from = reinterpret_cast<const uint4*>(q_s);
     for (int e = tid; e < Parts::qk_bytes / 16; e += W_THREADS) to[e] = from[e];
@@ -250,21 +297,25 @@ __global__ void __launch_bounds__(W_THREADS) walk_prepare_kernel(const WalkArgs 
             mma_bf16_16816(s[1], af[pa], bf[pb][2], bf[pb][3]);
           }
     }
+    for (int w = 0; w < heads; ++w) {
+      unsigned char* head = head0 + w * Parts::head_bytes;
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+      for (int i = 0; i < 2; ++i)
 #pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        const int at = row0 + g + 8 * r, j = c0 + 8 * i + 2 * t;
-        float x[2];
+        for (int r = 0; r < 2; ++r) {
+          const int at = row0 + g + 8 * r, j = c0 + 8 * i + 2 * t;
+          float x[2];
 #pragma unroll
-        for (int e = 0; e < 2; ++e)
-          x[e] = j + e <= at ? s[i][2 * r + e] * (exp2f((c_hi[at] - c_hi[j + e]) + (c_lo[at] - c_lo[j + e])) * s_s[j + e]) : 0.0f;
-        unsigned part[PB];
-        split_parts<PB>(x[0], x[1], part);
+          for (int e = 0; e < 2; ++e)
+            x[e] = j + e <= at
+                       ? s[i][2 * r + e] * (exp2f((c_hi[w][at] - c_hi[w][j + e]) + (c_lo[w][at] - c_lo[w][j + e])) * s_s[w][j + e])
+                       : 0.0f;
+          unsigned part[PB];
+          split_parts<PB>(x[0], x[1], part);
 #pragma unroll
-        for (int p = 0; p < PB; ++p)
-          *reinterpret_cast<unsigned*>(head + ((p * W + at) * W_PST + j) * 2) = part[p];
-      }
+          for (int p = 0; p < PB; ++p) *reinterpret_cast<unsigned*>(head + ((p * W + at) * W_PST + j) * 2) = part[p];
+        }
+    }
   }
 }
 
@@ -523,16 +574,18 @@ static int walk_launch(const WalkArgs& a, int pieces, cudaStream_t s) {
   if (cuda_failed(cudaFuncSetAttribute(prepare, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::qk_bytes)) ||
       cuda_failed(cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::smem)))
     return ERR_CUDA;
-  prepare<<<dim3(pieces, a.H), W_THREADS, Shape::qk_bytes, s>>>(a);
+  const int heads = MODE == WALK_SPACE ? W_HEADS : 1;
+  prepare<<<dim3(pieces, a.H / a.heads_per_group * ((a.heads_per_group + heads - 1) / heads)), W_THREADS, Shape::qk_bytes, s>>>(a);
   walk<<<dim3(a.rows, a.H, (a.V + Shape::COLS - 1) / Shape::COLS), W_THREADS, Shape::smem, s>>>(a);
   return launch_result();
 }
 
 template <int MODE>
 static int walk_dispatch(const WalkArgs& a, int pieces, cudaStream_t s) {
-  // 16 value columns a CTA, 32 where that would be more CTAs than SMs: a CTA takes a whole SM's shared memory, and the
-  // second half of them would walk alone.
-  const bool wide = static_cast<long long>(a.rows) * a.H * ((a.V + 15) / 16) > 148;
+  // 16 value columns a CTA, or 32: a CTA takes an SM, and a piece 1.7 us with 16 columns and 2.7 us with 32 (state space).
+  // Up to two CTAs an SM the narrow ones are not far behind even where all rows are equally long (two rounds of 1.7 us a
+  // piece), and far ahead where one row is much the longest (2048 and 77 tokens: 90 us with the wide ones).
+  const bool wide = static_cast<long long>(a.rows) * a.H * ((a.V + 15) / 16) > 2 * 148;
   if (a.D <= 64) return wide ? walk_launch<MODE, 64, 4>(a, pieces, s) : walk_launch<MODE, 64, 2>(a, pieces, s);
   return wide ? walk_launch<MODE, 128, 4>(a, pieces, s) : walk_launch<MODE, 128, 2>(a, pieces, s);
 }
@@ -554,13 +607,15 @@ ZB_API int zb_walk_piece_floats(int mode, int H, int heads_per_group, int D) {
 }
 
 // mode 0 (state space): q, k, v, dt bfloat16; q, k and their rows on 16-byte boundaries, D a multiple of 8.  mode 1 (fixed
-// decays): q, k, v float32.  Constants float32.  ws: (tokens / piece tokens + rows) * zb_walk_piece_floats floats, 16-byte
+// decays): q, k, v float32; with `freqs` (rot_dims / 2 of them) q and k are turned by the tokens' positions first, as
+// zb_rotate_qk does, k times k_scale (rot_dims a multiple of 8, D of 4, rows on 16-byte boundaries).  Constants float32.  ws: (tokens / piece tokens + rows) * zb_walk_piece_floats floats, 16-byte
 // aligned, contents irrelevant.  The rows' tokens lie behind one another in the stream, row_q_start ascending.
 ZB_API int zb_state_walk(int mode, float* out, const void* q, long long q_stride, const void* k, long long k_stride, const void* v,
                          long long v_stride, const void* dt, long long dt_stride, const float* dt_bias, const float* a_log,
                          const float* skip, const float* decay, float* state, long long slot_stride, const int* slots,
                          const int* row_q_start, const int* row_q_len, int rows, int tokens, int H, int D, int V,
-                         int heads_per_group, int num_slots, int write_state, float* ws, int* status, void* stream) {
+                         int heads_per_group, int num_slots, int write_state, const float* freqs, int rot_dims, float k_scale,
+                         const int* positions, float* ws, int* status, void* stream) {
   if (rows < 0 || tokens < 0 || H <= 0 || D <= 0 || V <= 0 || heads_per_group <= 0 || H % heads_per_group != 0 || num_slots <= 0 ||
       (mode != WALK_SPACE && mode != WALK_FIXED) || (mode == WALK_FIXED && (decay == nullptr || heads_per_group != 1)) ||
       (mode == WALK_SPACE && (dt == nullptr || dt_bias == nullptr || a_log == nullptr || skip == nullptr)))
@@ -573,6 +628,7 @@ ZB_API int zb_state_walk(int mode, float* out, const void* q, long long q_stride
     return ERR_BAD_ARGUMENT;
   const int pieces = tokens / W + rows, qk_heads = H / heads_per_group;
   WalkArgs a;
+  a.freqs = freqs; a.positions = positions; a.rot_dims = freqs != nullptr ? rot_dims : 0; a.k_scale = k_scale;
   a.q = q; a.q_stride = q_stride; a.k = k; a.k_stride = k_stride; a.v = v; a.v_stride = v_stride; a.dt = dt; a.dt_stride = dt_stride;
   a.dt_bias = dt_bias; a.a_log = a_log; a.skip = skip; a.decay = decay;
   a.qk = reinterpret_cast<unsigned char*>(ws);
@@ -580,6 +636,8 @@ ZB_API int zb_state_walk(int mode, float* out, const void* q, long long q_stride
                                           : (D <= 64 ? WalkParts<WALK_FIXED, 64>::qk_bytes : WalkParts<WALK_FIXED, 128>::qk_bytes);
   a.heads = a.qk + static_cast<long long>(pieces) * qk_heads * qk_bytes;
   a.vectors = mode == WALK_SPACE || (D % 4 == 0 && q_stride % 4 == 0 && k_stride % 4 == 0 && aligned(q) && aligned(k));
+  if (freqs != nullptr && (mode != WALK_FIXED || !a.vectors || positions == nullptr || rot_dims < 0 || rot_dims > D || rot_dims % 8 != 0))
+    return ERR_BAD_ARGUMENT;
   a.out = out; a.state = state; a.slot_stride = slot_stride; a.slots = slots; a.row_q_start = row_q_start; a.row_q_len = row_q_len;
   a.pairs = V % 2 == 0 && v_stride % 2 == 0 && reinterpret_cast<uintptr_t>(v) % (mode == WALK_SPACE ? 4 : 8) == 0;
   a.rows = rows; a.H = H; a.D = D; a.V = V; a.heads_per_group = heads_per_group; a.num_slots = num_slots; a.write_state = write_state;

@@ -160,7 +160,7 @@ _SIGNATURES = {
     "zb_walk_piece_floats": [c_int, c_int, c_int, c_int],
     "zb_state_walk": [c_int, c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p,
                       c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-                      c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p],
+                      c_int, c_int, c_int, c_int, c_void_p, c_int, c_float, c_void_p, c_void_p, c_void_p, c_void_p],
     "zb_rotate_qk": [c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_float, c_void_p, c_int, c_int, c_int, c_void_p],
     "zb_gated_group_rms_norm": [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_int,
                                 c_float, c_int, c_int, c_int, c_void_p],
@@ -722,17 +722,19 @@ WALK_FROM = 32      # new tokens per request, on average, from which on a step's
 
 
 def _state_walk(mode: int, out, q, k, v, heads: int, key_dim: int, value_dim: int, state, slots, row_q_start, row_q_len, status,
-                write_state: bool, dt=None, dt_bias=None, a_log=None, skip=None, decay=None, heads_per_group: int = 1) -> None:
+                write_state: bool, dt=None, dt_bias=None, a_log=None, skip=None, decay=None, heads_per_group: int = 1, turn=None) -> None:
     """The recurrence over runs of tokens in pieces of 64 with the state on the SM (csrc/state_walk.cu): mode 0 the
-    state-space form, 1 fixed decays.  The callers have checked types and shapes."""
+    state-space form, 1 fixed decays (``turn``: (freqs, rot_dims, k_scale, positions) where q and k are still to be
+    turned).  The callers have checked types and shapes."""
     lib, rows, T = library(), slots.numel(), v.shape[0]
+    freqs, rot_dims, k_scale, positions = turn or (None, 0, 1.0, None)
     ws = torch.empty(((T // lib.zb_walk_piece_tokens() + rows) * lib.zb_walk_piece_floats(mode, heads, heads_per_group, key_dim),),
                      dtype=torch.float32, device=v.device)
     _check(lib.zb_state_walk(
         mode, _ptr(out), _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(dt), dt.stride(0) if dt is not None else 0,
         _ptr(dt_bias), _ptr(a_log), _ptr(skip), _ptr(decay), _ptr(state), state.stride(0), _ptr(slots), _ptr(row_q_start),
-        _ptr(row_q_len), rows, T, heads, key_dim, value_dim, heads_per_group, state.shape[0], int(write_state), _ptr(ws), _ptr(status),
-        _stream()), "state_walk", kernels=2)
+        _ptr(row_q_len), rows, T, heads, key_dim, value_dim, heads_per_group, state.shape[0], int(write_state), _ptr(freqs), int(rot_dims),
+        float(k_scale), _ptr(positions), _ptr(ws), _ptr(status), _stream()), "state_walk", kernels=2)
 
 
 def decayed_state_scan(mode: str, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, heads: int, key_dim: int,
@@ -831,11 +833,19 @@ def retention_max_channels() -> int:
     return library().zb_retention_max_channels()
 
 
+def retention_turns(q: torch.Tensor, k: torch.Tensor, key_dim: int, rot_dims: int) -> bool:
+    """True if ``retention`` turns q and k of this shape itself."""
+    return (0 < rot_dims <= key_dim <= library().zb_walk_max_channels() and rot_dims % 8 == 0 and key_dim % 4 == 0
+            and all(t.stride(0) % 4 == 0 and t.data_ptr() % 16 == 0 for t in (q, k)))
+
+
 def retention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, heads: int, key_dim: int, value_dim: int,
               state: torch.Tensor, slots: torch.Tensor, row_q_start: torch.Tensor, row_q_len: torch.Tensor,
-              status: torch.Tensor, write_state: bool = True) -> torch.Tensor:
+              status: torch.Tensor, write_state: bool = True, freqs: torch.Tensor | None = None, rot_dims: int = 0,
+              k_scale: float = 1.0, positions: torch.Tensor | None = None) -> torch.Tensor:
     """What ``decayed_state_scan`` in its "fixed" mode does, in pieces of 64 tokens on the tensor cores: for rows that
-    bring runs of tokens.  q, k, v float32 [T, .] with unit inner stride, head h at column h * width; ``decay`` float32
+    bring runs of tokens.  With ``freqs`` q and k are first turned by the tokens' ``positions`` as ``rotate_qk`` does, k times
+    ``k_scale`` (``retention_turns``: whether that is taken).  q, k, v float32 [T, .] with unit inner stride, head h at column h * width; ``decay`` float32
     [heads]; ``state`` [slots, heads * key_dim * value_dim] float32 (rows may be strided).  Each operand of a product
     is taken as two bfloat16 values.  Returns o as float32 [T, heads * value_dim]."""
     _cuda(q, k, v, decay, state, slots, row_q_start, row_q_len, status)
@@ -849,8 +859,17 @@ def retention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Te
              and state.shape[1] == heads * key_dim * value_dim, "state must be float32 [slots, heads * key_dim * value_dim]")
     lib, rows = library(), slots.numel()
     out = torch.empty((T, heads * value_dim), dtype=torch.float32, device=v.device)
+    turn = None
+    if freqs is not None:
+        _cuda(freqs, positions)
+        _require(positions is not None and positions.numel() == T, "a rotation needs every token's position")
+        _i32(positions)
+        _f32_vector(freqs, rot_dims // 2, "the frequencies")
+        _require(retention_turns(q, k, key_dim, rot_dims), "q and k of this shape are turned by rotate_qk")
+        turn = (freqs, rot_dims, k_scale, positions)
     if key_dim <= lib.zb_walk_max_channels():
-        _state_walk(1, out, q, k, v, heads, key_dim, value_dim, state, slots, row_q_start, row_q_len, status, write_state, decay=decay)
+        _state_walk(1, out, q, k, v, heads, key_dim, value_dim, state, slots, row_q_start, row_q_len, status, write_state, decay=decay,
+                    turn=turn)
         return out
     pieces = T // lib.zb_retention_piece_tokens() + rows
     ws = torch.empty((pieces, heads * key_dim * value_dim), dtype=torch.float32, device=v.device)

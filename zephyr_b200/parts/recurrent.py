@@ -331,12 +331,19 @@ class Retention(Mixer):
                                         self.vdim, ctx.caches[call.cache], ctx.state_slots, ctx.row_q_start, ctx.row_q_len,
                                         ctx.positions, ctx.status, self.dtype, write_state=call.writes_cache)
             return ops.linear(normed, self.w_o, out_dtype=out_dtype)
-        turned = ops.rotate_qk(projected, self.heads, self.dim, self.freqs, self.rot_dims, self.dim ** -0.5, ctx.positions)
-        q, k, v = turned[:, :hd], turned[:, hd:], projected[:, 2 * hd:2 * hd + hv]
+        q, k, v = projected[:, :hd], projected[:, hd:2 * hd], projected[:, 2 * hd:2 * hd + hv]
         where = (ctx.caches[call.cache], ctx.state_slots, ctx.row_q_start, ctx.row_q_len, ctx.status)
         # Runs of tokens in pieces on the tensor cores; short ones, and everything in true 32-bit, token by token.
-        if self.dtype == torch.bfloat16 and x.shape[0] >= self.PIECES_FROM * ctx.num_rows and self.dim <= ops.retention_max_channels():
-            o = ops.retention(q, k, v, self.decay, self.heads, self.dim, self.vdim, *where, write_state=call.writes_cache)
+        pieces = (self.dtype == torch.bfloat16 and x.shape[0] >= self.PIECES_FROM * ctx.num_rows
+                  and self.dim <= ops.retention_max_channels())
+        turn = {}
+        if pieces and ops.retention_turns(q, k, self.dim, self.rot_dims):
+            turn = dict(freqs=self.freqs, rot_dims=self.rot_dims, k_scale=self.dim ** -0.5, positions=ctx.positions)
+        else:
+            turned = ops.rotate_qk(projected, self.heads, self.dim, self.freqs, self.rot_dims, self.dim ** -0.5, ctx.positions)
+            q, k = turned[:, :hd], turned[:, hd:]
+        if pieces:
+            o = ops.retention(q, k, v, self.decay, self.heads, self.dim, self.vdim, *where, write_state=call.writes_cache, **turn)
         else:
             o = ops.decayed_state_scan("fixed", q, k, v, self.heads, self.dim, self.vdim, *where, decay=self.decay,
                                        write_state=call.writes_cache)
