@@ -1,0 +1,115 @@
+"""The kernels between the products that move whole pieces of four values, against the kernels that take a value at a time: the
+same calls with rows that start off a 16-byte boundary, which the latter serve."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DTYPES = {"bfloat16": torch.bfloat16, "float32": torch.float32}
+
+
+def _apart(x, y, dtype):
+    """One step of the result's type (bfloat16 keeps 8 bits: neighbours are up to 2^-7 of their value apart) between float32
+    results a few roundings apart: normed and scaled values reach 20, four roundings of 20 * 2^-24 are below 2^-17."""
+    step = 2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -20
+    x, y = x.float(), y.float()
+    return ((x - y).abs() <= step * torch.maximum(x.abs(), y.abs()) + 2.0 ** -17).all()
+
+
+class Projected:
+    """A fused projection, once with aligned rows and once a value off, with caches for the keys and values of both."""
+
+    def __init__(self, device, dtype, tokens, heads, kv_heads, kd, vd, cached, values=True, seed=0):
+        from zephyr_b200.kernels import ops
+
+        g = torch.Generator().manual_seed(seed + tokens + kd)
+        dev = lambda t: t.to(device)
+        self.width = heads * kd + (kv_heads * (kd + (vd if values else 0)) if cached else 0)
+        stride = -(-self.width // 8) * 8
+        base = torch.randn(tokens, self.width, generator=g)
+        self.rows = [dev(torch.zeros(tokens, stride))[:, :self.width], dev(torch.zeros(tokens, stride + 1))[:, 1:1 + self.width]]
+        for r in self.rows:
+            r.copy_(base)
+        page, blocks = 8, -(-tokens // 8)
+        self.table = dev((torch.randperm(blocks, generator=g) + 1).to(torch.int32).view(1, -1))
+        self.caches = [dev(torch.zeros(blocks + 1, page * kv_heads * (kd + vd), dtype=dtype)) if cached else None for _ in range(2)]
+        self.pos = dev(torch.arange(tokens, dtype=torch.int32))
+        self.row = dev(torch.zeros(tokens, dtype=torch.int32))
+        self.status = ops.new_status(device)
+        self.vector = lambda n: dev(torch.randn(n, generator=g))
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("tokens,heads,kv_heads,kd,vd,rot,form", [
+    (700, 16, 4, 128, 128, 128, "norm bias"), (5, 16, 4, 128, 128, 64, "norm"), (601, 9, 1, 20, 24, 12, "unit temp"),
+    (640, 30, 3, 100, 60, 0, "bias"), (33, 3, 2, 256, 132, 256, "norm bias temp"), (593, 7, 2, 136, 136, 8, "unit keys"),
+    (620, 4, 4, 64, 0, 32, "norm"), (12, 0, 3, 64, 64, 64, "norm"), (611, 11, 2, 64, 64, 64, "queries")])
+def test_adjacent_pairs(cuda_device, dtype, tokens, heads, kv_heads, kd, vd, rot, form):
+    from zephyr_b200.kernels import ops
+
+    dtype, keys = DTYPES[dtype], "keys" in form
+    case = Projected(cuda_device, dtype, tokens, heads, kv_heads, kd, vd, "queries" not in form, values=not keys)
+    norm = [case.vector(kd), case.vector(kd)] if "norm" in form else [None, None]
+    bias = case.vector(case.width) if "bias" in form else None
+    freqs = (1000.0 ** (-torch.arange(rot // 2) / max(rot // 2, 1))).to(cuda_device) if rot else None
+    out = [ops.qkv_pairs(rows, heads, kv_heads, kd, vd, bias, *norm, 1e-6, freqs, rot, case.pos, case.row, cache, case.table,
+                         case.status, dtype, unit_norm="unit" in form, values_from_keys=keys,
+                         q_temp=(0.1, 16) if "temp" in form else None) for rows, cache in zip(case.rows, case.caches)]
+    ops.check_status(case.status)
+    assert heads == 0 or _apart(*out, dtype)
+    assert case.caches[0] is None or (_apart(*case.caches, dtype) and case.caches[0][1:].abs().max() > 0)
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("tokens,heads,kv_heads,kd,vd,rot,form", [
+    (700, 16, 4, 128, 128, 128, "per_head bias"), (5, 16, 4, 128, 128, 64, "per_head"), (601, 9, 1, 24, 40, 16, "none unit"),
+    (640, 30, 3, 104, 64, 0, "none bias first"), (33, 3, 2, 64, 128, 48, "per_head bias"), (593, 7, 2, 120, 8, 8, "per_head unit first"),
+    (611, 11, 2, 64, 64, 64, "none queries")])
+def test_halves(cuda_device, dtype, tokens, heads, kv_heads, kd, vd, rot, form):
+    from zephyr_b200.kernels import ops
+
+    dtype, mode = DTYPES[dtype], form.split()[0]
+    case = Projected(cuda_device, dtype, tokens, heads, kv_heads, kd, vd, "queries" not in form)
+    norm = [case.vector(kd), case.vector(kd)] if mode == "per_head" else [None, None]
+    bias = case.vector(case.width) if "bias" in form else None
+    freqs = (1000.0 ** (-torch.arange(rot // 2) / max(rot // 2, 1))).to(cuda_device) if rot else None
+    first = case.vector(tokens * kv_heads * vd).view(tokens, -1) if "first" in form else None
+    out = [ops.qkv_halves(rows, heads, kv_heads, kd, vd, mode, *norm, 1e-6, freqs, rot, 1.25, "unit" in form, case.pos, case.row, cache,
+                          case.table, case.status, dtype, bias=bias, v_first=first,
+                          v_share=torch.tensor([0.3], device=cuda_device) if first is not None else None)
+           for rows, cache in zip(case.rows, case.caches)]
+    ops.check_status(case.status)
+    assert _apart(*out, dtype)
+    assert case.caches[0] is None or (_apart(*case.caches, dtype) and case.caches[0][1:].abs().max() > 0)
+
+
+@pytest.mark.parametrize("group,groups,tokens", [(4, 3, 5), (128, 2, 7), (260, 3, 9), (512, 1, 6), (516, 3, 2), (1024, 2, 33),
+                                                 (1028, 1, 3), (2048, 2, 12)])
+@pytest.mark.parametrize("gate_first", [False, True])
+def test_group_norms(cuda_device, group, groups, tokens, gate_first):
+    from zephyr_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(group + tokens)
+    width = group * groups
+    o, gate, w = torch.randn(tokens, width, generator=g), torch.randn(tokens, width + 4, generator=g), torch.randn(width, generator=g)
+    got = ops.gated_group_rms_norm(o.to(cuda_device), gate.to(cuda_device)[:, 4:], w.to(cuda_device), group, 1e-5, gate_first=gate_first)
+    act = torch.nn.functional.silu(gate[:, 4:].double())
+    x = (o.double() * (act if gate_first else 1.0)).view(tokens, groups, group)
+    want = (x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-5)).view(tokens, width) * w.double() * (1.0 if gate_first else act)
+    # The activation's exponential and five products and sums, each within a few 2^-24 of values up to 20.
+    assert (got.cpu().double() - want).abs().max() <= 4e-6 * max(1.0, float(want.abs().max()))
+
+
+@pytest.mark.parametrize("shape", [(1, 4), (3, 5), (129, 516), (1, 2049), (7, 1024)])
+def test_sums_and_biases(cuda_device, shape):
+    from zephyr_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(shape[1])
+    a, b, bias = (torch.randn(n, generator=g).to(cuda_device) for n in (shape, shape, shape[1]))
+    for out_dtype in (torch.float32, torch.bfloat16):
+        want = (0.75 * a.double() - 1.5 * b.double()).float().to(out_dtype)
+        assert _apart(ops.scaled_sum(a, b, 0.75, -1.5, out_dtype=out_dtype), want, out_dtype)
+    for dtype in (torch.float32, torch.bfloat16):
+        x = a.to(dtype)
+        assert torch.equal(ops.add_bias(x.clone(), bias), (x.float() + bias).to(dtype))

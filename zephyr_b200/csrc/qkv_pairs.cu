@@ -10,7 +10,7 @@
 // with p the token's position and f a table of float32 frequencies the host made.  Keys and values
 // may differ in width: a page holds [nkv][page_size][kd] keys and behind them [nkv][page_size][vd]
 // values; rows whose bytes are a multiple of 16 are stored with permuted 16-byte chunks (common.cuh:
-// kv_swizzle), any other width as it is.  One warp per (token, head); a lane owns adjacent pairs.
+// kv_swizzle), any other width as it is.  A warp takes a head of a token; a lane owns adjacent pairs.
 //
 // Further forms, each a parameter: a norm without scales (`unit_norm`: x / sqrt(mean(x^2) + eps) on q and
 // k); values that are the keys as projected, before their norm (`values_from_keys`: the projection has
@@ -18,6 +18,8 @@
 // 1 + coef * ln(floor((p + 1) / every) + 1) (`q_temp_*`); a cache that keeps keys only (vd = 0: its
 // reader takes the keys for values too); and no query heads at all (nh = 0: only the cache is written).
 #include "common.cuh"
+
+#include <climits>
 
 namespace zb {
 
@@ -186,6 +188,141 @@ __global__ void __launch_bounds__(QP_WARPS * 32) qkv_pairs_kernel(const QkvPairs
   }
 }
 
+// The same where the widths, the rotated part and every row start are whole pieces of four values.  A CTA takes one token:
+// its angles are worked out once, into shared memory, a warp loads all its heads' values before it uses the first, and where
+// a piece goes within a cache row is one exclusive-or.  The general kernel above is bound by instructions, not by memory:
+// two sines a lane and head and 300 instructions a head: 2125 tokens of 32
+// heads of 128 in float32 took 29.6 us and take 18.6 (its bytes: 8 us), 12 tokens 5.2 and 3.9 us.  More heads a warp alone
+// (33 us) did not help the general form.
+constexpr int QPV_WARPS = 8;
+
+__device__ __forceinline__ float4 load_piece(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load_piece(const __nv_bfloat16* p) {
+  const uint2 raw = *reinterpret_cast<const uint2*>(p);
+  return make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u), __uint_as_float(raw.y << 16),
+                     __uint_as_float(raw.y & 0xffff0000u));
+}
+__device__ __forceinline__ void store_piece(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void store_piece(__nv_bfloat16* p, float4 v) {
+  __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+  uint2 raw;
+  raw.x = *reinterpret_cast<uint32_t*>(&lo);
+  raw.y = *reinterpret_cast<uint32_t*>(&hi);
+  *reinterpret_cast<uint2*>(p) = raw;
+}
+
+template <typename IN, typename T, int ITEMS, int HEADS>
+__global__ void __launch_bounds__(QPV_WARPS * 32) qkv_pairs_vec_kernel(const QkvPairsArgs a) {
+  extern __shared__ __align__(16) float turn[];      // [rot_dims]: cosine and sine of every pair
+  const int t = blockIdx.x, lane = threadIdx.x & 31;
+  const int h0 = blockIdx.y * QPV_WARPS * HEADS + (threadIdx.x >> 5);     // and every QPV_WARPS-th behind it
+  const int total = a.cache != nullptr ? a.nh + (a.vd > 0 ? 2 : 1) * a.nkv : a.nh;
+  const int pos = a.positions[t];
+  const IN* src = static_cast<const IN*>(a.qkv) + static_cast<long long>(t) * a.stride;
+
+  float4 x[HEADS][ITEMS];
+#pragma unroll
+  for (int j = 0; j < HEADS; ++j) {
+    const int h = h0 + QPV_WARPS * j;
+    const bool is_v = h >= a.nh + a.nkv;
+    const int dim = h >= total ? 0 : (is_v ? a.vd : a.kd);
+    const int col = !is_v ? h * a.kd
+                          : (a.values_from_keys ? (h - a.nkv) * a.kd : (a.nh + a.nkv) * a.kd + (h - a.nh - a.nkv) * a.vd);
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+      const int i = 4 * (lane + 32 * k);
+      x[j][k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (i < dim) {
+        x[j][k] = load_piece(src + col + i);
+        if (a.bias != nullptr) {
+          const float4 b = load_piece(a.bias + col + i);
+          x[j][k] = make_float4(x[j][k].x + b.x, x[j][k].y + b.y, x[j][k].z + b.z, x[j][k].w + b.w);
+        }
+      }
+    }
+  }
+  for (int i = threadIdx.x; i < a.rot_dims / 2; i += QPV_WARPS * 32) {
+    float s, c;
+    sincosf(static_cast<float>(pos) * a.freqs[i], &s, &c);
+    *reinterpret_cast<float2*>(turn + 2 * i) = make_float2(c, s);
+  }
+  int page = 0;
+  if (a.cache != nullptr) {
+    const int row = a.token_row[t], block = pos / a.page_size;
+    if (row < 0 || row >= a.num_rows || block >= a.max_blocks) {
+      if (threadIdx.x == 0) report(a.status, STATUS_ROW_OUT_OF_RANGE, row, t);
+    } else {
+      page = a.block_table[static_cast<long long>(row) * a.max_blocks + block];
+      if (page <= 0 || page >= a.num_pages) {      // page 0 is the null page and is never written
+        if (threadIdx.x == 0) report(a.status, STATUS_PAGE_OUT_OF_RANGE, page, t);
+        page = 0;
+      }
+    }
+  }
+  const int slot = pos % a.page_size;
+  constexpr int CHUNK = 16 / sizeof(T);            // values a 16-byte chunk: a piece never straddles two
+  const int k_swizzle = (a.kd % CHUNK) == 0 ? kv_swizzle(pos, a.kd / CHUNK) : 0;
+  const int v_swizzle = a.vd > 0 && (a.vd % CHUNK) == 0 ? kv_swizzle(pos, a.vd / CHUNK) : 0;
+  const float q_mult = a.q_temp_coef != 0.0f
+                           ? 1.0f + a.q_temp_coef * logf(static_cast<float>((pos + 1) / a.q_temp_every) + 1.0f) : 1.0f;
+  __syncthreads();
+
+#pragma unroll
+  for (int j = 0; j < HEADS; ++j) {
+    const int h = h0 + QPV_WARPS * j;
+    if (h >= total) break;
+    const bool is_q = h < a.nh, is_v = h >= a.nh + a.nkv;
+    const int dim = is_v ? a.vd : a.kd;
+    const float* w = is_q ? a.q_norm_w : (is_v ? nullptr : a.k_norm_w);
+    if (w != nullptr || (a.unit_norm && !is_v)) {
+      float ss = 0.0f;
+#pragma unroll
+      for (int k = 0; k < ITEMS; ++k) {
+        const float4 v = x[j][k];
+        ss += (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w);
+      }
+      const float inv = 1.0f / sqrtf(warp_sum(ss) / static_cast<float>(dim) + a.eps);
+#pragma unroll
+      for (int k = 0; k < ITEMS; ++k) {
+        const int i = 4 * (lane + 32 * k);
+        const float4 v = x[j][k];
+        float4 c = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+        if (w != nullptr && i < dim) c = load_piece(w + i);
+        x[j][k] = make_float4(v.x * inv * c.x, v.y * inv * c.y, v.z * inv * c.z, v.w * inv * c.w);
+      }
+    }
+    if (!is_v) {
+#pragma unroll
+      for (int k = 0; k < ITEMS; ++k) {
+        const int i = 4 * (lane + 32 * k);
+        float4 v = x[j][k];
+        if (i < a.rot_dims) {
+          const float4 f = *reinterpret_cast<const float4*>(turn + i);      // cosine, sine of two pairs
+          v = make_float4(v.x * f.x - v.y * f.y, v.y * f.x + v.x * f.y, v.z * f.z - v.w * f.w, v.w * f.z + v.z * f.w);
+        }
+        if (is_q) v = make_float4(v.x * q_mult, v.y * q_mult, v.z * q_mult, v.w * q_mult);
+        x[j][k] = v;
+      }
+    }
+    T* dst;
+    int swizzle = 0;
+    if (is_q) {
+      dst = static_cast<T*>(a.q_out) + (static_cast<long long>(t) * a.nh + h) * a.kd;
+    } else {
+      if (page == 0) return;         // reported above; the heads that follow are keys and values too
+      const int kvh = h - a.nh - (is_v ? a.nkv : 0);
+      dst = static_cast<T*>(a.cache) + static_cast<long long>(page) * (a.nkv * a.page_size * (a.kd + a.vd)) +
+            (is_v ? a.nkv * a.page_size * a.kd : 0) + (kvh * a.page_size + slot) * dim;
+      swizzle = is_v ? v_swizzle : k_swizzle;
+    }
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+      const int i = 4 * (lane + 32 * k);
+      if (i < dim) store_piece(dst + (i ^ (swizzle * CHUNK)), x[j][k]);
+    }
+  }
+}
+
 }  // namespace zb
 
 using namespace zb;
@@ -215,6 +352,28 @@ ZB_API int zb_qkv_pairs(void* q_out, const void* qkv, long long stride, const fl
   a.pairs_aligned = kd % 2 == 0 && vd % 2 == 0 && stride % 2 == 0 && even(qkv) && even(bias) && even(q_norm_w) &&
                     even(k_norm_w) && even(q_out) && even(cache);
   const int heads = cache != nullptr ? nh + (vd > 0 ? 2 : 1) * nkv : nh;
+  auto whole = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
+  const int wide = kd > vd ? kd : vd;
+  const long long page_values = static_cast<long long>(nkv) * page_size * (kd + vd);
+  if (!(dtype == DTYPE_F32 && in_dtype != DTYPE_F32) && kd % 4 == 0 && vd % 4 == 0 && a.rot_dims % 4 == 0 && stride % 4 == 0 &&
+      whole(qkv) && whole(bias) && whole(q_norm_w) && whole(k_norm_w) && whole(q_out) && whole(cache) && wide <= 256 &&
+      page_values <= INT_MAX && a.rot_dims <= 8192) {
+    auto s = static_cast<cudaStream_t>(stream);
+    const size_t smem = sizeof(float) * a.rot_dims;
+#define ZB_QPV(ITEMS, HEADS)                                                                                             \
+  {                                                                                                                      \
+    const dim3 grid(tokens, (heads + HEADS * QPV_WARPS - 1) / (HEADS * QPV_WARPS));                                      \
+    if (dtype == DTYPE_F32) qkv_pairs_vec_kernel<float, float, ITEMS, HEADS><<<grid, QPV_WARPS * 32, smem, s>>>(a);       \
+    else if (in_dtype == DTYPE_F32) qkv_pairs_vec_kernel<float, __nv_bfloat16, ITEMS, HEADS><<<grid, QPV_WARPS * 32, smem, s>>>(a); \
+    else qkv_pairs_vec_kernel<__nv_bfloat16, __nv_bfloat16, ITEMS, HEADS><<<grid, QPV_WARPS * 32, smem, s>>>(a);          \
+  }
+    // Several heads a warp where the tokens alone give every SM a full set of warps; a decode step keeps its heads apart.
+    const bool many = tokens >= 4 * 148 && heads > QPV_WARPS;
+    if (wide <= 128) { if (many) ZB_QPV(1, 4) else ZB_QPV(1, 1) }
+    else { if (many) ZB_QPV(2, 2) else ZB_QPV(2, 1) }
+#undef ZB_QPV
+    return launch_result();
+  }
   const dim3 grid(tokens, (heads + QP_WARPS - 1) / QP_WARPS);
   auto s = static_cast<cudaStream_t>(stream);
   if (dtype == DTYPE_F32 && in_dtype != DTYPE_F32) return ERR_BAD_ARGUMENT;

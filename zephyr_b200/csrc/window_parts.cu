@@ -9,7 +9,7 @@
 //                  position * f_i (float32 products, f a table the host made);
 //                  optionally every value head divided by its root mean square (no scales), or the values mixed
 //                  with another layer's values of the same token, v <- (1 - m) v + m v_first with m from the device;
-//                  and the write of k and v into the pages.  One CTA per token; everything in float32
+//                  and the write of k and v into the pages.  One CTA per token, or a warp a head; everything in float32
 //                  with one rounding at the store.
 //   pool_blocks  entry b of a pooled store = the mean over positions b P .. b P + P - 1 of the keys and
 //                  values as the pages hold them, summed in float32 in the order of the positions; the
@@ -19,6 +19,8 @@
 //   sigmoid_gate x[t, c] *= 1 / (1 + exp(-gate[t, c / per])), the gate float32 with strided rows: value by value
 //                  (per = 1), or one gate for every run of `per` values (a head's output).
 #include "common.cuh"
+
+#include <climits>
 
 namespace zb {
 
@@ -278,6 +280,102 @@ __global__ void __launch_bounds__(QH_THREADS) qkv_halves_vec_kernel(const QkvHal
   }
 }
 
+// The same where no statistic spans the heads (any norm but NORM_WHOLE) and a head is at most a warp's 32 pieces of four
+// values: a warp takes HEADS heads of one token, loads them all before it uses the first and keeps them in registers, a
+// value's partner in the rotation comes by a shuffle, and only the token's angles, worked out once a CTA, pass through shared
+// memory.  The CTA a token above waits at two barriers between its load and its store and reads its values twice:
+// 3000 tokens of 32 heads of 128 took 38 us and take 26 (its bytes: 11 us).
+constexpr int QHH_WARPS = 8;
+
+template <typename T, int HEADS>
+__global__ void __launch_bounds__(QHH_WARPS * 32) qkv_halves_heads_kernel(const QkvHalvesArgs a) {
+  extern __shared__ __align__(16) float qh_smem[];      // [rot_dims]: cosines, then sines
+  const int t = blockIdx.x, lane = threadIdx.x & 31, i = 4 * lane;
+  const int h0 = blockIdx.y * QHH_WARPS * HEADS + (threadIdx.x >> 5);     // and every QHH_WARPS-th behind it
+  const int kv_heads = a.cache != nullptr ? a.nkv : 0;
+  const int first_v = a.nh + kv_heads, heads = first_v + kv_heads, half = a.rot_dims / 2;
+  const float* src = static_cast<const float*>(a.qkv) + static_cast<long long>(t) * a.stride;
+  const int pos = a.positions[t];
+  float4 x[HEADS];
+#pragma unroll
+  for (int j = 0; j < HEADS; ++j) {
+    const int h = h0 + QHH_WARPS * j;
+    const bool is_v = h >= first_v;
+    x[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (h < heads && i < (is_v ? a.vd : a.kd)) {
+      const int c = (is_v ? first_v * a.kd + (h - first_v) * a.vd : h * a.kd) + i;
+      x[j] = *reinterpret_cast<const float4*>(src + c);
+      if (a.bias != nullptr) {
+        const float4 b = *reinterpret_cast<const float4*>(a.bias + c);
+        x[j] = make_float4(x[j].x + b.x, x[j].y + b.y, x[j].z + b.z, x[j].w + b.w);
+      }
+    }
+  }
+  if (threadIdx.x < half) {
+    float s, c;
+    sincosf(static_cast<float>(pos) * a.freqs[threadIdx.x], &s, &c);
+    qh_smem[threadIdx.x] = c * a.rot_mult;
+    qh_smem[half + threadIdx.x] = s * a.rot_mult;
+  }
+  int page = 0;
+  if (a.cache != nullptr) {
+    const int row = a.token_row[t], block = pos / a.page_size;
+    if (row < 0 || row >= a.num_rows || block >= a.max_blocks) {
+      if (threadIdx.x == 0) report(a.status, STATUS_ROW_OUT_OF_RANGE, row, t);
+      return;
+    }
+    page = a.block_table[static_cast<long long>(row) * a.max_blocks + block];
+    if (page <= 0 || page >= a.num_pages) {
+      if (threadIdx.x == 0) report(a.status, STATUS_PAGE_OUT_OF_RANGE, page, t);
+      return;
+    }
+  }
+  const int slot = pos % a.page_size;
+  constexpr int CHUNK = 16 / sizeof(T);            // values a 16-byte chunk: a piece never straddles two
+  const int at_k = i ^ (kv_swizzle(pos, a.kd / CHUNK) * CHUNK), at_v = i ^ (kv_swizzle(pos, a.vd / CHUNK) * CHUNK);
+  T* q_row = static_cast<T*>(a.q_out) + static_cast<long long>(t) * a.nh * a.kd;
+  T* page_row = static_cast<T*>(a.cache) + static_cast<long long>(page) * (a.nkv * a.page_size * (a.kd + a.vd));
+  const float share = a.v_first != nullptr ? *a.v_share : 0.0f;
+  __syncthreads();
+  float4 cosine = make_float4(1.0f, 1.0f, 1.0f, 1.0f), sine = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  const bool turns = i < 2 * half, low = i < half;
+  const int partner = low ? lane + half / 4 : lane - half / 4;
+  if (turns) {
+    cosine = *reinterpret_cast<const float4*>(qh_smem + (low ? i : i - half));
+    sine = *reinterpret_cast<const float4*>(qh_smem + (low ? half + i : i));
+    if (low) sine = make_float4(-sine.x, -sine.y, -sine.z, -sine.w);
+  }
+#pragma unroll
+  for (int j = 0; j < HEADS; ++j) {
+    const int h = h0 + QHH_WARPS * j;
+    if (h >= heads) break;
+    const bool is_q = h < a.nh, is_v = h >= first_v;
+    const int dim = is_v ? a.vd : a.kd;
+    float4 y = x[j];
+    if (is_v ? a.value_unit_norm != 0 : a.norm_mode == NORM_PER_HEAD) {
+      const float ss = warp_sum((y.x * y.x + y.y * y.y) + (y.z * y.z + y.w * y.w));
+      const float inv = 1.0f / sqrtf(ss / static_cast<float>(dim) + a.eps);
+      y = scaled4(y, inv, is_v || i >= dim ? nullptr : (is_q ? a.q_norm_w : a.k_norm_w), i);
+    }
+    if (!is_v && half > 0) {
+      const float4 p = make_float4(__shfl_sync(~0u, y.x, partner), __shfl_sync(~0u, y.y, partner),
+                                   __shfl_sync(~0u, y.z, partner), __shfl_sync(~0u, y.w, partner));
+      if (turns)
+        y = make_float4(y.x * cosine.x + p.x * sine.x, y.y * cosine.y + p.y * sine.y, y.z * cosine.z + p.z * sine.z,
+                        y.w * cosine.w + p.w * sine.w);
+    }
+    if (i >= dim) continue;
+    if (is_v && a.v_first != nullptr) {
+      const float4 f = *reinterpret_cast<const float4*>(a.v_first + static_cast<long long>(t) * a.v_first_stride + (h - first_v) * a.vd + i);
+      const float keep = 1.0f - share;
+      y = make_float4(keep * y.x + share * f.x, keep * y.y + share * f.y, keep * y.z + share * f.z, keep * y.w + share * f.w);
+    }
+    if (is_q) store_four<T>(q_row + h * a.kd + i, y);
+    else if (is_v) store_four<T>(page_row + a.nkv * a.page_size * a.kd + ((h - first_v) * a.page_size + slot) * a.vd + at_v, y);
+    else store_four<T>(page_row + ((h - a.nh) * a.page_size + slot) * a.kd + at_k, y);
+  }
+}
+
 // ------------------------------------------------------------------------------------------------
 struct PoolBlocksArgs {
   const void* cache;          // the tokens' pages
@@ -459,6 +557,21 @@ ZB_API int zb_qkv_halves(void* q_out, const void* qkv, long long stride, const f
   auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
   if (in_dtype == DTYPE_F32 && kd % 8 == 0 && vd % 8 == 0 && rot_dims % 8 == 0 && stride % 4 == 0 && v_first_stride % 4 == 0 &&
       aligned(qkv) && aligned(bias) && aligned(q_norm_w) && aligned(k_norm_w) && aligned(v_first) && aligned(q_out) && aligned(cache)) {
+    const int heads = nh + 2 * kv_heads, widest = kv_heads > 0 && vd > kd ? vd : kd;
+    if (norm_mode != NORM_WHOLE && widest <= 128 && static_cast<long long>(nkv) * page_size * (kd + vd) <= INT_MAX) {
+      // Several heads a warp where the tokens alone give every SM a full set of warps; a decode step keeps its heads apart.
+      const bool many = tokens >= 4 * 148 && heads > QHH_WARPS;
+      const size_t turn = sizeof(float) * a.rot_dims;
+#define ZB_QHH(HEADS)                                                                                        \
+  {                                                                                                          \
+    const dim3 grid(tokens, (heads + HEADS * QHH_WARPS - 1) / (HEADS * QHH_WARPS));                          \
+    if (dtype == DTYPE_F32) qkv_halves_heads_kernel<float, HEADS><<<grid, QHH_WARPS * 32, turn, s>>>(a);      \
+    else qkv_halves_heads_kernel<__nv_bfloat16, HEADS><<<grid, QHH_WARPS * 32, turn, s>>>(a);                 \
+  }
+      if (many) ZB_QHH(4) else ZB_QHH(1)
+#undef ZB_QHH
+      return launch_result();
+    }
 #define ZB_QHV(T)                                                                                               \
   {                                                                                                             \
     auto kernel = qkv_halves_vec_kernel<T>;                                                                     \
