@@ -113,3 +113,22 @@ def test_sums_and_biases(cuda_device, shape):
     for dtype in (torch.float32, torch.bfloat16):
         x = a.to(dtype)
         assert torch.equal(ops.add_bias(x.clone(), bias), (x.float() + bias).to(dtype))
+
+
+@pytest.mark.parametrize("N,K", [(16, 8), (40, 1024), (2048, 2048), (2040, 6152), (4720, 2048), (9472, 256), (9480, 264), (9500, 4104)])
+@pytest.mark.parametrize("M", [1, 8, 9, 16, 30, 64])
+def test_few_rows_at_the_splits_of_k(cuda_device, N, K, M):
+    from zephyr_b200.kernels import ops
+
+    g = torch.Generator(device=cuda_device).manual_seed(N + K + M)
+    x = torch.randn(M, K, generator=g, device=cuda_device).to(torch.bfloat16)
+    w = (torch.randn(N, K, generator=g, device=cuda_device) / K ** 0.5).to(torch.bfloat16)
+    got, want = ops.gemm_small(x, w, out_dtype=torch.float32), x.double() @ w.double().T
+    # Exact products of about 1 / sqrt(K), float32 sums of K of them in at most K / 8 + 64 steps: below 2^-24 * sqrt(K) of sums up to 6.
+    assert (got.double() - want).abs().max() <= 6 * 2.0 ** -24 * max(16.0, K ** 0.5)
+    assert torch.equal(ops.gemm_small(x[M - 1:], w, out_dtype=torch.float32), got[M - 1:])     # a row's sums do not see the others
+    if N % 16 == 0:
+        gate, up = want.view(M, N // 16, 2, 8).unbind(2)
+        hidden = ops.gemm_small(x, w, out_dtype=torch.float32, swiglu=True)
+        want = (torch.nn.functional.silu(gate) * up).reshape(M, N // 2)
+        assert (hidden.double() - want).abs().max() <= 40 * 2.0 ** -24 * max(16.0, K ** 0.5)

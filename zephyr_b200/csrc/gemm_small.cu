@@ -8,8 +8,12 @@
 // consecutive values k = 8t .. 8t+7 of its row: one 16-byte load feeds two tensor-core products.
 // The products see k in a permuted order, the same for both operands, so the sum is unchanged.
 //
-// One CTA owns 16 rows of W; its four warps split K, and for matrices with few rows a cluster of
-// up to 8 CTAs splits K further.  Partial sums meet in (distributed) shared memory and are added in
+// One CTA owns 16 rows of W (or 32); its warps split K, and for matrices with few rows a cluster of
+// up to 8 CTAs splits K further.  A decode step's product is bound by latency before it is by bandwidth: a warp has the loads
+// of four blocks of 32 k in flight, whatever is left of its slice (one block after the other, as a loop's remainder, 2048 x
+// 6144 with 12 rows took 13.8 us; now 10.1, its bytes 3.8), and the CTAs of a cluster each finish a share of the tile with one
+// round of remote reads (one CTA for all, 2048 x 2048: 9.8 us; now 6.1).  4096 x 2048: 10.2 -> 7.9, 12288 x 2048: 14.9 -> 14.1,
+// 8192 x 4096, 12 rows: 16.9.  Partial sums meet in (distributed) shared memory and are added in
 // a fixed order, so the result does not depend on timing.  ACT takes each sum through GELU's tanh form, a
 // squared ReLU, or GELU times a value of the token's row of a table.  With SWIGLU the 16 rows are 8 gate
 // rows followed by their 8 up rows, and the epilogue writes silu(gate) * up: the activation costs
@@ -24,8 +28,6 @@ namespace zb {
 namespace cg = cooperative_groups;
 
 constexpr int ACT_TOKEN_GATE = 3;
-constexpr int GS_ROWS = 16;       // weight rows per CTA
-constexpr int GS_WARPS = 4;
 constexpr int GS_MAX_MT = 8;      // token tiles of 8: M <= 64
 constexpr int GS_MAX_KSPLIT = 8;
 
@@ -53,25 +55,30 @@ template <> __device__ __forceinline__ void store_out<__nv_bfloat16>(__nv_bfloat
   *p = __float2bfloat16_rn(v);
 }
 
-template <int MT, typename TOut, bool SWIGLU, int ACT>
-__global__ void __launch_bounds__(GS_WARPS * 32)
+template <int RT, int WARPS, int MT, typename TOut, bool SWIGLU, int ACT>
+__global__ void __launch_bounds__(WARPS * 32)
 gemm_small_kernel(const SmallGemmArgs a) {
-  // Partial sums of this CTA's warps: [warp][mt][row][token].
-  __shared__ float red[GS_WARPS][MT][GS_ROWS][8];
+  constexpr int U = RT == 1 && MT <= 2 ? 4 : 2;     // blocks of k in flight
+  constexpr int PER_WARP = RT * MT * 16 * 8;        // sums of a warp: [rt][mt][row][token]
+  __shared__ float red[WARPS][PER_WARP];
   cg::cluster_group cluster = cg::this_cluster();
   const int ksplit = gridDim.y, krank = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int n0 = blockIdx.x * GS_ROWS;
+  const int n0 = blockIdx.x * (16 * RT);
 
   const int total_blocks = (a.K + 31) / 32;
-  const int slices = GS_WARPS * ksplit, slice = krank * GS_WARPS + warp;
+  const int slices = WARPS * ksplit, slice = krank * WARPS + warp;
   const int b_begin = static_cast<int>(static_cast<long long>(total_blocks) * slice / slices);
   const int b_end = static_cast<int>(static_cast<long long>(total_blocks) * (slice + 1) / slices);
 
-  const bool lo_ok = n0 + g < a.N, hi_ok = n0 + g + 8 < a.N;
-  const __nv_bfloat16* w_lo = a.w + static_cast<size_t>(lo_ok ? n0 + g : 0) * a.ldw + 8 * t;
-  const __nv_bfloat16* w_hi = a.w + static_cast<size_t>(hi_ok ? n0 + g + 8 : 0) * a.ldw + 8 * t;
+  bool w_ok[2 * RT];
+  const __nv_bfloat16* w_row[2 * RT];
+#pragma unroll
+  for (int r = 0; r < 2 * RT; ++r) {
+    w_ok[r] = n0 + g + 8 * r < a.N;
+    w_row[r] = a.w + static_cast<size_t>(w_ok[r] ? n0 + g + 8 * r : 0) * a.ldw + 8 * t;
+  }
   const __nv_bfloat16* x_row[MT];
   bool x_ok[MT];
 #pragma unroll
@@ -80,99 +87,131 @@ gemm_small_kernel(const SmallGemmArgs a) {
     x_row[mt] = a.x + static_cast<size_t>(x_ok[mt] ? mt * 8 + g : 0) * a.ldx + 8 * t;
   }
 
-  float acc[MT][4];
+  float acc[RT][MT][4];
 #pragma unroll
-  for (int mt = 0; mt < MT; ++mt) acc[mt][0] = acc[mt][1] = acc[mt][2] = acc[mt][3] = 0.0f;
+  for (int rt = 0; rt < RT; ++rt)
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) acc[rt][mt][0] = acc[rt][mt][1] = acc[rt][mt][2] = acc[rt][mt][3] = 0.0f;
 
-#pragma unroll 8
-  for (int b = b_begin; b < b_end; ++b) {
-    const int k = b * 32;
-    const bool k_ok = k + 8 * t + 8 <= a.K;          // K is a multiple of 8: a chunk is whole or absent
-    const uint4 wl = load16_or_zero(w_lo + k, lo_ok && k_ok);
-    const uint4 wh = load16_or_zero(w_hi + k, hi_ok && k_ok);
-    const unsigned a0[4] = {wl.x, wh.x, wl.y, wh.y};
-    const unsigned a1[4] = {wl.z, wh.z, wl.w, wh.w};
+  for (int b = b_begin; b < b_end; b += U) {
+    uint4 wv[U][2 * RT], xv[U][MT];
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
-      const uint4 xv = load16_or_zero(x_row[mt] + k, x_ok[mt] && k_ok);
-      mma_bf16_16816(acc[mt], a0, xv.x, xv.y);
-      mma_bf16_16816(acc[mt], a1, xv.z, xv.w);
+    for (int u = 0; u < U; ++u) {
+      const int k = (b + u) * 32;
+      const bool k_ok = b + u < b_end && k + 8 * t + 8 <= a.K;      // K is a multiple of 8: a chunk is whole or absent
+#pragma unroll
+      for (int r = 0; r < 2 * RT; ++r) wv[u][r] = load16_or_zero(w_row[r] + k, w_ok[r] && k_ok);
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) xv[u][mt] = load16_or_zero(x_row[mt] + k, x_ok[mt] && k_ok);
     }
-  }
-
 #pragma unroll
-  for (int mt = 0; mt < MT; ++mt) {
-    red[warp][mt][g][2 * t] = acc[mt][0];
-    red[warp][mt][g][2 * t + 1] = acc[mt][1];
-    red[warp][mt][g + 8][2 * t] = acc[mt][2];
-    red[warp][mt][g + 8][2 * t + 1] = acc[mt][3];
-  }
-  // Every CTA of the cluster has its partial sums in its shared memory; a cluster of one needs only
-  // its own barrier (the cluster's costs a fence that the language-model head paid 9496 times).
-  if (ksplit == 1) __syncthreads();
-  else cluster.sync();
-
-  if (krank == 0) {
-    // The first CTA of the cluster adds all partial sums, warp by warp and CTA by CTA, and writes.
-    const float* parts[GS_MAX_KSPLIT];
-    for (int r = 0; r < ksplit; ++r) parts[r] = cluster.map_shared_rank(&red[0][0][0][0], r);
-    constexpr int PER_WARP = MT * GS_ROWS * 8;
-    TOut* y = static_cast<TOut*>(a.y);
-    if (SWIGLU) {
-      // rows 0..7 are gate rows, rows 8..15 the matching up rows
-      for (int e = threadIdx.x; e < MT * 8 * 8; e += GS_WARPS * 32) {
-        const int mt = e / 64, r = (e / 8) % 8, tok = e % 8;
-        float gate = 0.0f, up = 0.0f;
-        for (int c = 0; c < ksplit; ++c)
+    for (int u = 0; u < U; ++u)
 #pragma unroll
-          for (int w = 0; w < GS_WARPS; ++w) {
-            gate += parts[c][w * PER_WARP + (mt * GS_ROWS + r) * 8 + tok];
-            up += parts[c][w * PER_WARP + (mt * GS_ROWS + r + 8) * 8 + tok];
-          }
-        const int token = mt * 8 + tok, col = blockIdx.x * 8 + r;
-        if (token < a.M && n0 + r + 8 < a.N) {
-          float v;
-          if (a.gate.kind == GATE_BOUNDED) {
-            if (a.gate.bias != nullptr) {
-              gate += a.gate.bias[n0 + r];
-              up += a.gate.bias[n0 + r + 8];
-            }
-            v = bounded_gate<false>(gate, up, a.gate);
-          } else {
-            v = (a.gate.kind == GATE_RELU ? fmaxf(gate, 0.0f) : gate / (1.0f + expf(-gate))) * up;
-          }
-          store_out<TOut>(y + static_cast<size_t>(token) * a.ldy + col, v);
+      for (int rt = 0; rt < RT; ++rt) {
+        const uint4 wl = wv[u][2 * rt], wh = wv[u][2 * rt + 1];
+        const unsigned a0[4] = {wl.x, wh.x, wl.y, wh.y};
+        const unsigned a1[4] = {wl.z, wh.z, wl.w, wh.w};
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+          mma_bf16_16816(acc[rt][mt], a0, xv[u][mt].x, xv[u][mt].y);
+          mma_bf16_16816(acc[rt][mt], a1, xv[u][mt].z, xv[u][mt].w);
         }
       }
-    } else {
-      for (int e = threadIdx.x; e < PER_WARP; e += GS_WARPS * 32) {
-        const int mt = e / (GS_ROWS * 8), r = (e / 8) % GS_ROWS, tok = e % 8;
-        float sum = 0.0f;
-        for (int c = 0; c < ksplit; ++c)
+  }
+
 #pragma unroll
-          for (int w = 0; w < GS_WARPS; ++w) sum += parts[c][w * PER_WARP + e];
-        const int token = mt * 8 + tok;
-        if (ACT == ACT_TOKEN_GATE) {
-          if (token < a.M && n0 + r < a.N) {
-            const int id = a.token_ids[token];
-            const bool ok = id >= 0 && id < a.vocab;
-            if (!ok && n0 + r == 0) report(a.status, STATUS_TOKEN_OUT_OF_RANGE, id, token);
-            const float e = ok ? __bfloat162float(a.token_rows[static_cast<long long>(id) * a.token_stride + n0 + r]) : 0.0f;
-            store_out<TOut>(y + static_cast<size_t>(token) * a.ldy + n0 + r, gelu_tanh(sum) * e);
-          }
-        } else if (token < a.M && n0 + r < a.N)
-          store_out<TOut>(y + static_cast<size_t>(token) * a.ldy + n0 + r, ACT == ACT_GELU ? gelu_tanh(sum) : ACT == ACT_RELU2 ? relu_squared(sum) : sum);
+  for (int rt = 0; rt < RT; ++rt)
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+      float* at = &red[warp][(rt * MT + mt) * 128 + g * 8 + 2 * t];
+      *reinterpret_cast<float2*>(at) = make_float2(acc[rt][mt][0], acc[rt][mt][1]);
+      *reinterpret_cast<float2*>(at + 64) = make_float2(acc[rt][mt][2], acc[rt][mt][3]);
+    }
+  __syncthreads();
+  // A CTA adds its warps' sums in their order; a cluster's CTAs each finish a share of the tile from the sums of all, in
+  // the CTAs' order, which lie in (distributed) shared memory.
+  if (ksplit > 1) {
+    for (int e = threadIdx.x; e < PER_WARP; e += WARPS * 32) {
+      float sum = red[0][e];
+#pragma unroll
+      for (int w = 1; w < WARPS; ++w) sum += red[w][e];
+      red[0][e] = sum;
+    }
+    cluster.sync();
+  }
+  auto total_of = [&](int e) {
+    float sum;
+    if (ksplit == 1) {
+      sum = red[0][e];
+#pragma unroll
+      for (int w = 1; w < WARPS; ++w) sum += red[w][e];
+    } else {
+      float part[GS_MAX_KSPLIT];
+#pragma unroll
+      for (int c = 0; c < GS_MAX_KSPLIT; ++c) part[c] = c < ksplit ? *cluster.map_shared_rank(&red[0][e], c) : 0.0f;
+      sum = part[0];
+#pragma unroll
+      for (int c = 1; c < GS_MAX_KSPLIT; ++c) sum += part[c];
+    }
+    return sum;
+  };
+  TOut* y = static_cast<TOut*>(a.y);
+  for (int i = krank * WARPS * 32 + threadIdx.x; i < (SWIGLU ? PER_WARP / 2 : PER_WARP); i += ksplit * WARPS * 32) {
+    const int r = (i / 8) % (SWIGLU ? 8 : 16), tile = i / (SWIGLU ? 64 : 128), mt = tile % MT, rt = tile / MT;
+    const int token = mt * 8 + i % 8, row = n0 + 16 * rt + r;
+    if (token >= a.M) continue;
+    if (SWIGLU) {                          // rows 0..7 of a tile are gate rows, rows 8..15 the matching up rows
+      if (row + 8 >= a.N) continue;
+      float gate = total_of(tile * 128 + r * 8 + i % 8), up = total_of(tile * 128 + 64 + r * 8 + i % 8), v;
+      if (a.gate.kind == GATE_BOUNDED) {
+        if (a.gate.bias != nullptr) {
+          gate += a.gate.bias[row];
+          up += a.gate.bias[row + 8];
+        }
+        v = bounded_gate<false>(gate, up, a.gate);
+      } else {
+        v = (a.gate.kind == GATE_RELU ? fmaxf(gate, 0.0f) : gate / (1.0f + expf(-gate))) * up;
+      }
+      store_out<TOut>(y + static_cast<size_t>(token) * a.ldy + (blockIdx.x * RT + rt) * 8 + r, v);
+    } else {
+      if (row >= a.N) continue;
+      const float sum = total_of(i);
+      TOut* at = y + static_cast<size_t>(token) * a.ldy + row;
+      if (ACT == ACT_TOKEN_GATE) {
+        const int id = a.token_ids[token];
+        const bool ok = id >= 0 && id < a.vocab;
+        if (!ok && row == 0) report(a.status, STATUS_TOKEN_OUT_OF_RANGE, id, token);
+        const float e = ok ? __bfloat162float(a.token_rows[static_cast<long long>(id) * a.token_stride + row]) : 0.0f;
+        store_out<TOut>(at, gelu_tanh(sum) * e);
+      } else {
+        store_out<TOut>(at, ACT == ACT_GELU ? gelu_tanh(sum) : ACT == ACT_RELU2 ? relu_squared(sum) : sum);
       }
     }
   }
   if (ksplit > 1) cluster.sync();           // nobody leaves while its shared memory may still be read
 }
 
-template <int MT, typename TOut, bool SWIGLU, int ACT>
+struct SmallGemmSplit {
+  int warps, ksplit;           // of a CTA; CTAs that share K
+};
+// How K is cut, from the matrix alone: a row's sums are the same whatever rows it is computed with.  Eight warps a CTA and, up
+// to two CTAs an SM, a cluster that shares K (a power of two up to 8, two blocks of k a warp or more): with every warp's loads
+// in flight at once the latency of the last one, not the split, is what is left.  Above four such CTAs an SM a second wave
+// begins, and four warps are the better CTA (32768 x 2048, 12 rows: 29.8 us against 33.4) until K gives each of them more
+// than 32 blocks to walk (24576 x 4096: 56 us against 45).
+static SmallGemmSplit small_gemm_split(int N, int K) {
+  const int tiles = (N + 15) / 16, blocks = (K + 31) / 32;
+  if (tiles > 4 * 148) return {blocks >= 128 ? 8 : 4, 1};
+  int ksplit = 1;
+  while (ksplit < GS_MAX_KSPLIT && tiles * ksplit < 2 * 148 && blocks >= 4 * 8 * ksplit) ksplit *= 2;
+  return {8, ksplit};
+}
+
+template <int RT, int WARPS, int MT, typename TOut, bool SWIGLU, int ACT>
 int small_gemm_launch(const SmallGemmArgs& a, int ksplit, cudaStream_t stream) {
   cudaLaunchConfig_t config = {};
-  config.gridDim = dim3((a.N + GS_ROWS - 1) / GS_ROWS, ksplit, 1);
-  config.blockDim = dim3(GS_WARPS * 32, 1, 1);
+  config.gridDim = dim3((a.N + 16 * RT - 1) / (16 * RT), ksplit, 1);
+  config.blockDim = dim3(WARPS * 32, 1, 1);
   config.dynamicSmemBytes = 0;
   config.stream = stream;
   cudaLaunchAttribute attribute[1];
@@ -182,17 +221,27 @@ int small_gemm_launch(const SmallGemmArgs& a, int ksplit, cudaStream_t stream) {
   attribute[0].val.clusterDim.z = 1;
   config.attrs = attribute;
   config.numAttrs = 1;
-  if (cudaLaunchKernelEx(&config, gemm_small_kernel<MT, TOut, SWIGLU, ACT>, a) != cudaSuccess) return ERR_CUDA;
+  if (cudaLaunchKernelEx(&config, gemm_small_kernel<RT, WARPS, MT, TOut, SWIGLU, ACT>, a) != cudaSuccess) return ERR_CUDA;
   return launch_result();
 }
 
+template <int MT, typename TOut, bool SWIGLU, int ACT>
+int small_gemm_split_launch(const SmallGemmArgs& a, cudaStream_t stream) {
+  const SmallGemmSplit s = small_gemm_split(a.N, a.K);
+  if (s.warps == 8) return small_gemm_launch<1, 8, MT, TOut, SWIGLU, ACT>(a, s.ksplit, stream);
+  // Up to 8 tokens and several waves of CTAs: 32 rows a CTA read the tokens half as often (151936 x 1024, 4 rows: 50 us
+  // against 54; with 12 rows their registers cost more, 66 against 64).  The sums are the same.
+  if (MT == 1) return small_gemm_launch<2, 4, 1, TOut, SWIGLU, ACT>(a, s.ksplit, stream);
+  return small_gemm_launch<1, 4, MT, TOut, SWIGLU, ACT>(a, s.ksplit, stream);
+}
+
 template <typename TOut, bool SWIGLU, int ACT>
-int small_gemm_dispatch(const SmallGemmArgs& a, int ksplit, cudaStream_t stream) {
+int small_gemm_dispatch(const SmallGemmArgs& a, cudaStream_t stream) {
   switch ((a.M + 7) / 8) {
-    case 1: return small_gemm_launch<1, TOut, SWIGLU, ACT>(a, ksplit, stream);
-    case 2: return small_gemm_launch<2, TOut, SWIGLU, ACT>(a, ksplit, stream);
-    case 3: case 4: return small_gemm_launch<4, TOut, SWIGLU, ACT>(a, ksplit, stream);
-    default: return small_gemm_launch<8, TOut, SWIGLU, ACT>(a, ksplit, stream);
+    case 1: return small_gemm_split_launch<1, TOut, SWIGLU, ACT>(a, stream);
+    case 2: return small_gemm_split_launch<2, TOut, SWIGLU, ACT>(a, stream);
+    case 3: case 4: return small_gemm_split_launch<4, TOut, SWIGLU, ACT>(a, stream);
+    default: return small_gemm_split_launch<8, TOut, SWIGLU, ACT>(a, stream);
   }
 }
 
@@ -203,16 +252,6 @@ using namespace zb;
 // 1 if zb_gemm_small takes this problem.
 ZB_API int zb_gemm_small_supported(int M, int N, int K) {
   return M >= 1 && M <= 8 * GS_MAX_MT && N >= 1 && K >= 8 && K % 8 == 0 ? 1 : 0;
-}
-
-// How many CTAs share the K dimension of one 16-row tile: enough for the grid to fill the GPU, a
-// power of two up to 8, and no finer than one 32-wide block of k per warp.
-ZB_API int zb_gemm_small_ksplit(int N, int K) {
-  const int tiles = (N + GS_ROWS - 1) / GS_ROWS;
-  const int blocks = (K + 31) / 32;
-  int ksplit = 1;
-  while (ksplit < GS_MAX_KSPLIT && tiles * ksplit < 592 && blocks >= GS_WARPS * ksplit * 2) ksplit *= 2;
-  return ksplit;
 }
 
 // y = x w^T (swiglu = 0), or y[:, 8j + r] = silu(x w[16j + r]^T) * (x w[16j + 8 + r]^T) (swiglu = 1; 2: max(., 0) for silu;
@@ -232,19 +271,18 @@ static int small_gemm(void* y, const void* x, const void* w, int M, int N, int K
   a.w = static_cast<const __nv_bfloat16*>(w);
   a.M = M; a.N = N; a.K = K; a.ldx = ldx; a.ldw = ldw; a.ldy = ldy;
   a.gate = gate;
-  const int ksplit = zb_gemm_small_ksplit(N, K);
   auto s = static_cast<cudaStream_t>(stream);
   if (act == ACT_GELU)
-    return out_dtype == DTYPE_F32 ? small_gemm_dispatch<float, false, ACT_GELU>(a, ksplit, s)
-                                  : small_gemm_dispatch<__nv_bfloat16, false, ACT_GELU>(a, ksplit, s);
+    return out_dtype == DTYPE_F32 ? small_gemm_dispatch<float, false, ACT_GELU>(a, s)
+                                  : small_gemm_dispatch<__nv_bfloat16, false, ACT_GELU>(a, s);
   if (act == ACT_RELU2)
-    return out_dtype == DTYPE_F32 ? small_gemm_dispatch<float, false, ACT_RELU2>(a, ksplit, s)
-                                  : small_gemm_dispatch<__nv_bfloat16, false, ACT_RELU2>(a, ksplit, s);
+    return out_dtype == DTYPE_F32 ? small_gemm_dispatch<float, false, ACT_RELU2>(a, s)
+                                  : small_gemm_dispatch<__nv_bfloat16, false, ACT_RELU2>(a, s);
   if (gated)
-    return out_dtype == DTYPE_F32 ? small_gemm_dispatch<float, true, ACT_NONE>(a, ksplit, s)
-                                  : small_gemm_dispatch<__nv_bfloat16, true, ACT_NONE>(a, ksplit, s);
-  return out_dtype == DTYPE_F32 ? small_gemm_dispatch<float, false, ACT_NONE>(a, ksplit, s)
-                                : small_gemm_dispatch<__nv_bfloat16, false, ACT_NONE>(a, ksplit, s);
+    return out_dtype == DTYPE_F32 ? small_gemm_dispatch<float, true, ACT_NONE>(a, s)
+                                  : small_gemm_dispatch<__nv_bfloat16, true, ACT_NONE>(a, s);
+  return out_dtype == DTYPE_F32 ? small_gemm_dispatch<float, false, ACT_NONE>(a, s)
+                                : small_gemm_dispatch<__nv_bfloat16, false, ACT_NONE>(a, s);
 }
 
 ZB_API int zb_gemm_small(void* y, const void* x, const void* w, int M, int N, int K, long long ldx, long long ldw,
@@ -275,7 +313,7 @@ ZB_API int zb_gemm_small_token_gate(void* y, const void* x, const void* w, const
   a.M = M; a.N = N; a.K = K; a.ldx = ldx; a.ldw = ldw; a.ldy = ldy;
   a.token_rows = static_cast<const __nv_bfloat16*>(table) + offset;
   a.token_stride = table_stride; a.token_ids = ids; a.vocab = vocab; a.status = status;
-  return small_gemm_dispatch<__nv_bfloat16, false, ACT_TOKEN_GATE>(a, zb_gemm_small_ksplit(N, K), static_cast<cudaStream_t>(stream));
+  return small_gemm_dispatch<__nv_bfloat16, false, ACT_TOKEN_GATE>(a, static_cast<cudaStream_t>(stream));
 }
 
 // The gated form with the bounded gate: y[:, 8j + r] from the sums of w's rows 16j + r (gate) and 16j + 8 + r
