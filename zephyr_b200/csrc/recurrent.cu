@@ -9,7 +9,8 @@
 //     per head, S [D, V] float32 in the request's state slot, in three settings: a decay per key channel
 //     a = sigmoid(z)^(1/tau) (gated linear attention), and one decay per head a = exp(-exp(A) dt)
 //     with k = dt B, q = C and a skip term D x (the state-space form of Mamba-2), and a constant decay per
-//     head (retention; long portions of it run on tensor cores, retention.cu);
+//     head (retention); long portions with one decay per head run on tensor cores, state_walk.cu and
+//     retention.cu;
 //   * the rotation of halves on the q and k heads of a fused projection, k with a multiplier;
 //   * the RMS norm over equal groups of a row with a SiLU gate before or behind it.
 //

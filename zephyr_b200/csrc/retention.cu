@@ -12,6 +12,8 @@
 //   retention_carry    S_in of every piece, from the request's slot on, and the state behind the last into the slot
 //   retention_output   both terms of o, for all pieces side by side
 //
+// Heads of up to 128 key channels take the walk in state_walk.cu instead, which keeps the state on the SM.
+//
 // A step that brings one token a request takes one kernel from the projection to the gated output (retention_step):
 // rotation, state, read-out, unit norm and gate, all in float32.
 //

@@ -757,7 +757,9 @@ def decayed_state_scan(mode: str, q: torch.Tensor, k: torch.Tensor, v: torch.Ten
     from zero states, a carry of the state from segment to segment, a pass with the outputs: twice the
     arithmetic on many times the threads); 0: never; None: chosen, for steps whose requests bring 256
     tokens and more on average and whose requests x heads x columns / 64 do not fill the SMs (measured,
-    one request of 2048 tokens: 8 heads of 128 x 256: 712 -> 270 us; 16 heads: 720 -> 482 us)."""
+    one request of 2048 tokens: 8 heads of 128 x 256: 712 -> 270 us; 16 heads: 720 -> 482 us).  None also lets
+    the bfloat16 "state_space" form with ``WALK_FROM`` tokens a request and more, of shapes the walk over pieces
+    takes (csrc/state_walk.cu), run there on the tensor cores (2125 tokens, 32 heads of 128 x 64: 290 -> 82 us)."""
     _cuda(q, k, v, state, slots, row_q_start, row_q_len, status, decay_logits, decay_bias, dt, dt_bias, a_log, skip)
     _i32(slots, row_q_start, row_q_len)
     T = v.shape[0]
