@@ -139,3 +139,39 @@ def test_retention_turns_its_queries_and_keys(cuda_device, heads, dim, vdim, rot
     ops.check_status(status)
     for x, y in zip(*got):       # the same float32 rotation, at most a rounding apart ahead of the split
         assert (x - y).abs().max() <= 4e-6 * max(1.0, float(x.abs().max()))
+
+
+@pytest.mark.parametrize("kind", ["delta", "state_space", "retention"])
+def test_rows_whose_tokens_lie_in_another_order(cuda_device, kind):
+    """Rows may name any stretch of the stream: listed backwards or shuffled they get the bits they get in the stream's
+    order.  (Lengths at which numbers counted from a row's first token would meet: 40 and 40, the second row first.)"""
+    from zephyr_b200.kernels import ops
+
+    heads, per, dim, vdim = 4, 2 if kind != "retention" else 1, 64, 48
+    lengths = [40, 40, 200, 64, 33, 97]
+    starts, T, groups = [sum(lengths[:i]) for i in range(len(lengths))], sum(lengths), heads // per
+    g = torch.Generator().manual_seed(9)
+    dtype = torch.bfloat16 if kind == "state_space" else torch.float32
+    q, k, v, b, a = (torch.randn(T, n, generator=g).to(cuda_device) for n in (groups * dim, groups * dim, heads * vdim, heads, heads))
+    q, k, v, dt = (t.to(dtype) for t in (q, k, v, a))
+    constants = [(torch.rand(heads, generator=g) - 0.5).to(cuda_device) for _ in range(3)]
+    i32 = lambda values: torch.tensor(values, dtype=torch.int32, device=cuda_device)
+    status = ops.new_status(cuda_device)
+
+    def run(order):
+        state = torch.zeros(len(lengths), heads * dim * vdim, device=cuda_device)
+        rows = (state, i32(order), i32([starts[r] for r in order]), i32([lengths[r] for r in order]), status)
+        if kind == "delta":
+            out = ops.delta_rule(q, k, v, b, a, constants[0], constants[1], heads, groups, dim, vdim, *rows, q_scale=dim ** -0.5)
+        elif kind == "retention":
+            out = ops.retention(q, k, v, constants[0].abs() + 0.4, heads, dim, vdim, *rows)
+        else:
+            out = ops.decayed_state_scan("state_space", q, k, v, heads, dim, vdim, *rows, dt=dt, dt_bias=constants[0],
+                                         a_log=constants[1], skip=constants[2], heads_per_group=per)
+        ops.check_status(status)
+        return out, state
+
+    expected = run(list(range(len(lengths))))
+    for order in ([1, 0, 2, 3, 4, 5], [5, 4, 3, 2, 1, 0], [2, 5, 0, 4, 1, 3]):
+        for x, y in zip(run(order), expected):
+            assert torch.equal(x, y), order

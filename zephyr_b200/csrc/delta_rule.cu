@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(DS_THREADS) delta_scan_kernel(const DeltaScanA
 //   M  = P (I + A)^-1 diag(beta),  P_tj = e^(c_t - c_j) (q_t . k_j)   (o = e^(c) R_q + M v')
 //
 // and delta_block_scan walks a request's blocks.  Exponents are differences of sums within a block, never positive.
-// Tokens behind a portion's end have beta 0 and decay 1.  Block p of row r has the number row_q_start[r] / B + r + p.
+// Tokens behind a portion's end have beta 0 and decay 1.  Blocks are numbered row by row (first_piece_of_row).
 constexpr int DB = 16;                     // tokens of a block
 constexpr int DB_THREADS = 256;
 constexpr int DB_COLS = 16;                // value columns of a CTA
@@ -352,18 +352,11 @@ __global__ void __launch_bounds__(DB_THREADS) delta_blocks_kernel(const DeltaBlo
   float* t_s = p_s + DB * DB;              // [DB][DB]: (I + A)^-1 diag(beta)
   float* c_s = t_s + DB * DB;              // [DB]
   float* beta_s = c_s + DB;
-  __shared__ int found;
   const int block = blockIdx.x, group = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) found = -1;
-  __syncthreads();
-  for (int r = tid; r < a.rows; r += DB_THREADS) {
-    const int p = block - (a.row_q_start[r] / DB + r);
-    if (p >= 0 && p * DB < a.row_q_len[r]) found = r;       // at most one row
-  }
-  __syncthreads();
-  const int row = found;
+  int own;
+  const int row = row_of_piece<DB>(a.row_q_len, a.rows, block, own);
   if (row < 0) return;
-  const int begin = (block - (a.row_q_start[row] / DB + row)) * DB, n = min(DB, a.row_q_len[row] - begin);
+  const int begin = own * DB, n = min(DB, a.row_q_len[row] - begin);
   const long long t0 = a.row_q_start[row] + begin;
 #pragma unroll
   for (int u = 0; u < 2 * DB / (DB_THREADS / 32); ++u) {
@@ -550,7 +543,7 @@ __global__ void __launch_bounds__(DB_THREADS) delta_block_scan_kernel(const Delt
   }
   const int n = a.row_q_len[row], blocks = (n + DB - 1) / DB;
   const long long t0 = a.row_q_start[row];
-  const int first = a.row_q_start[row] / DB + row;
+  const int first = first_piece_of_row<DB>(a.row_q_len, row);
   const int group = head / (a.heads / a.qk_heads);
 
   auto copy_block = [&](int p, float* stage) {
@@ -785,7 +778,7 @@ static int delta_block_launch(const DeltaBlocksArgs& b, const DeltaBlockScanArgs
 }
 
 // The rule over runs of tokens, block by block.  `ws`: (tokens / block tokens + rows) * zb_delta_block_floats floats,
-// 16-byte aligned, contents irrelevant.  The rows' tokens lie behind one another in the stream, row_q_start ascending.
+// 16-byte aligned, contents irrelevant.  The rows' tokens may lie in the stream in any order.
 ZB_API int zb_delta_block_scan(float* out, const void* q, long long q_stride, const void* k, long long k_stride, const void* v,
                                long long v_stride, const float* b, const float* a, long long ba_stride, const float* a_log,
                                const float* dt_bias, float* state, long long slot_stride, const int* slots, const int* row_q_start,

@@ -25,8 +25,7 @@
 // Sums of logarithms are formed in 64 bits and kept as two float32 values, so that a difference of two is good to a
 // rounding of itself.
 //
-// Piece p of row r has the number row_q_start[r] / W + r + p: distinct for all pieces of a step, and below
-// tokens / W + rows.
+// Pieces are numbered row by row (first_piece_of_row).
 #include "common.cuh"
 #include "mma.cuh"
 
@@ -112,8 +111,6 @@ __device__ __forceinline__ void walk_product(float (&acc)[N][4], const unsigned 
       }
 }
 
-__device__ __forceinline__ int walk_first_piece(const WalkArgs& a, int row) { return a.row_q_start[row] / W + row; }
-
 // A piece of one q/k head and up to W_HEADS of the heads that share it (their scores are the same).  DP: the channels padded
 // with zeros.
 constexpr int W_HEADS = 4;
@@ -122,22 +119,15 @@ __global__ void __launch_bounds__(W_THREADS) walk_prepare_kernel(const WalkArgs 
   using Parts = WalkParts<MODE, DP>;
   constexpr int ST = Parts::ST, PA = Parts::PA, PB = Parts::PB, HEADS = MODE == WALK_SPACE ? W_HEADS : 1;
   extern __shared__ __align__(16) unsigned char w_smem[];
-  __shared__ int found;
   __shared__ float c_hi[HEADS][W], c_lo[HEADS][W], s_s[HEADS][W];
   const int piece = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int runs = (a.heads_per_group + HEADS - 1) / HEADS;              // runs of heads in a group
   const int qk_head = blockIdx.y / runs, first_head = blockIdx.y % runs * HEADS, qk_heads = a.H / a.heads_per_group;
   const int heads = min(HEADS, a.heads_per_group - first_head), h0 = qk_head * a.heads_per_group + first_head;
-  if (tid == 0) found = -1;
-  __syncthreads();
-  for (int r = tid; r < a.rows; r += W_THREADS) {
-    const int p = piece - walk_first_piece(a, r);
-    if (p >= 0 && p * W < a.row_q_len[r]) found = r;         // at most one row
-  }
-  __syncthreads();
-  const int row = found;
+  int own;
+  const int row = row_of_piece<W>(a.row_q_len, a.rows, piece, own);
   if (row < 0) return;
-  const int begin = (piece - walk_first_piece(a, row)) * W, n = min(W, a.row_q_len[row] - begin);
+  const int begin = own * W, n = min(W, a.row_q_len[row] - begin);
   const long long t0 = a.row_q_start[row] + begin;
   __nv_bfloat16* q_s = reinterpret_cast<__nv_bfloat16*>(w_smem);        // [PA][W][ST]
   __nv_bfloat16* k_s = q_s + PA * W * ST;                               // [PA][W][ST]
@@ -356,7 +346,7 @@ __global__ void __launch_bounds__(W_THREADS) state_walk_kernel(const WalkArgs a)
   }
   const int n_all = a.row_q_len[row], pieces = (n_all + W - 1) / W;
   const long long t0 = a.row_q_start[row];
-  const int first = walk_first_piece(a, row), qk_head = h / a.heads_per_group, qk_heads = a.H / a.heads_per_group;
+  const int first = first_piece_of_row<W>(a.row_q_len, row), qk_head = h / a.heads_per_group, qk_heads = a.H / a.heads_per_group;
   if (tid == 0) {
 #pragma unroll
     for (int i = 0; i < STAGES; ++i) mbar_init(&landed[i], 1);
@@ -611,8 +601,9 @@ ZB_API int zb_walk_piece_floats(int mode, int H, int heads_per_group, int D) {
 
 // mode 0 (state space): q, k, v, dt bfloat16; q, k and their rows on 16-byte boundaries, D a multiple of 8.  mode 1 (fixed
 // decays): q, k, v float32; with `freqs` (rot_dims / 2 of them) q and k are turned by the tokens' positions first, as
-// zb_rotate_qk does, k times k_scale (rot_dims a multiple of 8, D of 4, rows on 16-byte boundaries).  Constants float32.  ws: (tokens / piece tokens + rows) * zb_walk_piece_floats floats, 16-byte
-// aligned, contents irrelevant.  The rows' tokens lie behind one another in the stream, row_q_start ascending.
+// zb_rotate_qk does, k times k_scale (rot_dims a multiple of 8, D of 4, rows on 16-byte boundaries).  Constants float32.
+// ws: (tokens / piece tokens + rows) * zb_walk_piece_floats floats, 16-byte aligned, contents irrelevant.  The rows' tokens
+// may lie in the stream in any order.
 ZB_API int zb_state_walk(int mode, float* out, const void* q, long long q_stride, const void* k, long long k_stride, const void* v,
                          long long v_stride, const void* dt, long long dt_stride, const float* dt_bias, const float* a_log,
                          const float* skip, const float* decay, float* state, long long slot_stride, const int* slots,

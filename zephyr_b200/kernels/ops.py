@@ -849,7 +849,8 @@ def retention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Te
     bring runs of tokens.  With ``freqs`` q and k are first turned by the tokens' ``positions`` as ``rotate_qk`` does, k times
     ``k_scale`` (``retention_turns``: whether that is taken).  q, k, v float32 [T, .] with unit inner stride, head h at column h * width; ``decay`` float32
     [heads]; ``state`` [slots, heads * key_dim * value_dim] float32 (rows may be strided).  Each operand of a product
-    is taken as two bfloat16 values.  Returns o as float32 [T, heads * value_dim]."""
+    is taken as two bfloat16 values.  Rows may lie in the stream in any order (heads of more than 128 key channels: one behind the
+    other, ``row_q_start`` ascending).  Returns o as float32 [T, heads * value_dim]."""
     _cuda(q, k, v, decay, state, slots, row_q_start, row_q_len, status)
     _i32(slots, row_q_start, row_q_len)
     T = v.shape[0]
