@@ -1,5 +1,7 @@
 """Kernels that take runs of tokens instead of single ones, alone, at the edges of their runs and blocks."""
 
+import math
+
 import pytest
 import torch
 
@@ -175,3 +177,52 @@ def test_rows_whose_tokens_lie_in_another_order(cuda_device, kind):
     for order in ([1, 0, 2, 3, 4, 5], [5, 4, 3, 2, 1, 0], [2, 5, 0, 4, 1, 3]):
         for x, y in zip(run(order), expected):
             assert torch.equal(x, y), order
+
+
+def _delta_in_float64(q, k, v, b, a, a_log, dt_bias, heads, groups, dim, vdim, state):
+    """The plain rule, from the state [heads, vdim, dim] on: outputs [T, heads, vdim] and the state behind them."""
+    T, own = len(v), torch.arange(heads) // (heads // groups)
+    q, k, v, b, a, a_log, dt_bias, S = (t.cpu().double() for t in (q, k, v, b, a, a_log, dt_bias, state))
+    unit = lambda x: (x.view(T, groups, dim) / torch.sqrt((x.view(T, groups, dim) ** 2).sum(-1, keepdim=True) + 1e-6))[:, own]
+    q, k, v, S = unit(q) * dim ** -0.5, unit(k), v.view(T, heads, vdim), S.view(heads, vdim, dim).clone()
+    beta, decay = torch.sigmoid(b), torch.exp(-torch.exp(a_log) * torch.nn.functional.softplus(a + dt_bias))
+    out = torch.zeros(T, heads, vdim, dtype=torch.float64)
+    for t in range(T):
+        S = S * decay[t].view(-1, 1, 1)
+        u = beta[t].view(-1, 1) * (v[t] - torch.einsum("hvd,hd->hv", S, k[t]))
+        S = S + u.unsqueeze(-1) * k[t].unsqueeze(1)
+        out[t] = torch.einsum("hvd,hd->hv", S, q[t])
+    return out, S
+
+
+@pytest.mark.parametrize("dim,vdim", [(128, 64), (48, 20)])
+def test_the_delta_rule_in_blocks_keeps_float32(cuda_device, dim, vdim):
+    """With rates and steps as such models start them, blocks are as close to 64 bits as the token-by-token form, which portions
+    of 15 tokens take: sums in another order, of the same precision."""
+    from zephyr_b200.kernels import ops
+
+    heads, groups, T = 4, 2, 512
+    g = torch.Generator().manual_seed(dim)
+    q, k, v, b, a = (torch.randn(T, n, generator=g) for n in (groups * dim, groups * dim, heads * vdim, heads, heads))
+    step = torch.exp(torch.rand(heads, generator=g) * math.log(100.0) - math.log(1000.0))
+    a_log, dt_bias = torch.log(1.0 + 15.0 * torch.rand(heads, generator=g)), step + torch.log(-torch.expm1(-step))
+    ba = torch.cat([b, a], dim=1).to(cuda_device)
+    dev = lambda t: t.to(cuda_device)
+    i32 = lambda values: torch.tensor(values, dtype=torch.int32, device=cuda_device)
+    status = ops.new_status(cuda_device)
+    expected, last = _delta_in_float64(q, k, v, b, a, a_log, dt_bias, heads, groups, dim, vdim, torch.zeros(heads, vdim, dim))
+
+    def error(cuts):
+        state, out, at = torch.zeros(1, heads * dim * vdim, device=cuda_device), [], 0
+        for n in cuts:
+            part = slice(at, at + n)
+            out.append(ops.delta_rule(dev(q[part]), dev(k[part]), dev(v[part]), ba[part, :heads], ba[part, heads:], dev(a_log), dev(dt_bias),
+                                      heads, groups, dim, vdim, state, i32([0]), i32([0]), i32([n]), status, q_scale=dim ** -0.5))
+            at += n
+        ops.check_status(status)
+        got = torch.cat(out).cpu().double().view_as(expected)
+        return float((got - expected).norm() / expected.norm()), float((state.cpu().double().view_as(last) - last).norm() / last.norm())
+
+    # (measured over such inputs: 0.7 to 0.9 of the token-by-token form's error; operands of two TF32 values: 1.5 to 1.9)
+    for blocks, tokens in zip(error([T]), error([15] * (T // 15) + [T % 15])):
+        assert blocks <= 1.2 * tokens

@@ -2,7 +2,7 @@
 //
 //   S <- g S;   u = beta (v - S^T k);   S <- S + k u^T;   o = S^T q
 //
-// with one decay g and one step beta per head and token.  Two kernels:
+// with one decay g and one step beta per head and token.  Token by token, in two kernels:
 //
 //   delta_gates   per token: q and k heads (the model's type, as a convolution left them) made unit
 //                 vectors, x / sqrt(sum(x^2) + unit_eps), q also times `q_scale`, both written as
@@ -20,7 +20,7 @@
 // Where requests bring runs of tokens, two other kernels take their place (delta_blocks, delta_block_scan below): the
 // same rule, block by block of 16 tokens.
 //
-// Everything here is float32; the values v are read in the model's type.
+// Everything here is float32 multiply-adds in either form; the values v are read in the model's type.
 #include "common.cuh"
 #include "mma.cuh"
 
@@ -324,8 +324,7 @@ __global__ void __launch_bounds__(DS_THREADS) delta_scan_kernel(const DeltaScanA
 constexpr int DB = 16;                     // tokens of a block
 constexpr int DB_THREADS = 256;
 constexpr int DB_COLS = 16;                // value columns of a CTA
-constexpr int DB_CST = DB + 8;             // a row of the matrices [j][t]: the lanes of a fragment then read distinct banks
-constexpr int DB_COEF = 2 * DB * DB_CST + 2 * DB;  // Tu and M, both [j][t], e^(c_t), e^(c_B) and padding
+constexpr int DB_COEF = 2 * DB * DB + 2 * DB;      // Tu and M, both [j][t], e^(c_t), e^(c_B) and padding
 
 struct DeltaBlocksArgs {
   float* qk;               // [blocks][qk_heads][DP][2 DB]: k of the block's tokens, then q
@@ -462,12 +461,12 @@ __global__ void __launch_bounds__(DB_THREADS) delta_blocks_kernel(const DeltaBlo
     __syncthreads();
     // (threads run over the rows of the transposed matrices: t fastest)
     const int tt = tid % DB, jj = tid / DB;
-    coef[jj * DB_CST + tt] = expf(last - c_s[tt]) * t_s[tt * DB + jj];
+    coef[jj * DB + tt] = expf(last - c_s[tt]) * t_s[tt * DB + jj];
     float m = 0.0f;
     for (int i = jj; i <= tt; ++i) m = fmaf(p_s[tt * DB + i], t_s[i * DB + jj], m);
-    coef[(DB + jj) * DB_CST + tt] = m;
-    if (tid < DB) coef[2 * DB * DB_CST + tid] = expf(c_s[tid]);
-    if (tid == 0) coef[2 * DB * DB_CST + DB] = expf(last);
+    coef[(DB + jj) * DB + tt] = m;
+    if (tid < DB) coef[2 * DB * DB + tid] = expf(c_s[tid]);
+    if (tid == 0) coef[2 * DB * DB + DB] = expf(last);
   }
 }
 
@@ -482,60 +481,26 @@ struct DeltaBlockScanArgs {
   int* status;
 };
 
-// The products of the scan run on the tensor cores with operands of two TF32 values each, x = hi + lo up to 2^-21 (hi the
-// leading 11 bits, lo the rest rounded to 11, by integer instructions: NaN and infinity stay in hi), as the three
-// partial products that count, lo hi + hi lo + hi hi, each summed on its own; the state itself is only ever touched by
-// float32 multiply-adds.
-__device__ __forceinline__ void split_tf32(float x, unsigned& hi, unsigned& lo) {
-  hi = __float_as_uint(x) & 0xffffe000u;
-  lo = (__float_as_uint(x - __uint_as_float(hi)) + 0x1000u) & 0xffffe000u;
-}
-// Fragments (lane = 4 g + t): A 16 x 8: (g, t), (g + 8, t), (g, t + 4), (g + 8, t + 4); B 8 x 8: (t, g), (t + 4, g); C 16 x 8:
-// (g, 2t), (g, 2t + 1), (g + 8, 2t), (g + 8, 2t + 1).
-__device__ __forceinline__ void mma_tf32(float (&d)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
-  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-// acc += A B for one step of k: A from `at` (element (row, k) at at[row * row_step + k * k_step]), B from a tile kept as hi
-// and lo words [k][DB_BST].
-constexpr int DB_BST = DB_COLS + 8;
-constexpr int DB_STAGES = 4;               // blocks in shared memory: the present one and three on their way
-__device__ __forceinline__ void product_step(float (&hh)[4], float (&hl)[4], float (&lh)[4], const float* at, int row_step, int k_step,
-                                             const unsigned* b_hi, const unsigned* b_lo, int g, int t) {
-  unsigned ah[4], al[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) split_tf32(at[(g + (i & 1) * 8) * row_step + (t + (i >> 1) * 4) * k_step], ah[i], al[i]);
-  const unsigned h0 = b_hi[t * DB_BST + g], h1 = b_hi[(t + 4) * DB_BST + g];
-  const unsigned l0 = b_lo[t * DB_BST + g], l1 = b_lo[(t + 4) * DB_BST + g];
-  mma_tf32(lh, al, h0, h1);
-  mma_tf32(hl, ah, l0, l1);
-  mma_tf32(hh, ah, h0, h1);
-}
-
-// A CTA owns a request, a head and DB_COLS value columns; its state lies in registers (a warp 16 channels, as C fragments)
-// and, split, in shared memory for the read-outs.  A block: the read-outs of k and q (a warp a 16 x 8 tile over half
-// the channels); v' from the two halves' sums; u and o from the block's matrices (a warp a tile); the state.  The next
-// blocks' operands are copied meanwhile.  Bound by the chain of a block, four barriers with eight warps between them:
-// 1.4 us a block of 16 tokens (2048 tokens, 16 heads of 128 x 128: 181 us, and 26 us for the matrices, against 535 + 10 us
-// token by token).  With multiply-adds instead, tiles of 4 x 4 a thread, the reads of shared memory made it 224 us; blocks
-// of 32 tokens took 158 us here and 63 us for the matrices.
+// A CTA owns a request, a head and DB_COLS value columns; its state lies in registers (two channels by four columns a
+// thread) and, for the read-outs, in shared memory.  A block: every warp forms the read-outs of all 32 rows (k and q)
+// over its share of the channels, 4 x 4 a thread; the warps' sums are added and v' made; u and o from the block's
+// matrices; the state.  The next block's operands are copied meanwhile.  Bound by the reads of shared memory beside the
+// multiply-adds and by the chain of a block, four barriers with eight warps between them (2048 tokens, 16 heads of 128 x 128: 240 us
+// with the matrices, 522 token by token).  Products on the tensor cores with operands of two TF32 values each took 30 us less,
+// at 1.5 to 1.9 times the token-by-token form's error against 64 bits; this form has 0.5 to 0.9 of it.
 template <typename T, int DP>
 __global__ void __launch_bounds__(DB_THREADS) delta_block_scan_kernel(const DeltaBlockScanArgs a) {
   extern __shared__ __align__(16) float db_smem[];
-  constexpr int QK_ST = 2 * DB + 8, RED_ST = DB_COLS + 4;
+  constexpr int QK_ST = 2 * DB + 4, S_ST = DB_COLS + 4, RED_ST = 2 * DB + 4;
   constexpr int stage_floats = DP * QK_ST + DB_COEF;
-  float* stages = db_smem;                                   // [DB_STAGES] of [DP][QK_ST] and the coefficients
-  float* red_s = stages + DB_STAGES * stage_floats;          // [2][2 DB][RED_ST]: the halves' read-outs
-  float* o_s = red_s + 2 * 2 * DB * RED_ST;                  // [DB][RED_ST]: e^(c) R_q
-  unsigned* s_hi = reinterpret_cast<unsigned*>(o_s + DB * RED_ST);       // [DP][DB_BST]
-  unsigned* s_lo = s_hi + DP * DB_BST;
-  unsigned* v_hi = s_lo + DP * DB_BST;                       // [DB][DB_BST]: v'
-  unsigned* v_lo = v_hi + DB * DB_BST;
-  unsigned* u_hi = v_lo + DB * DB_BST;                       // [DB][DB_BST]: what the write takes
-  unsigned* u_lo = u_hi + DB * DB_BST;
+  float* stages = db_smem;                                   // two of [DP][QK_ST] and the coefficients
+  float* s_s = stages + 2 * stage_floats;                    // [DP][S_ST]
+  float* red_s = s_s + DP * S_ST;                            // [warps][DB_COLS][RED_ST]
+  float* vp_s = red_s + DB_THREADS / 32 * DB_COLS * RED_ST;  // [DB_COLS][DB]: v'
+  float* u_s = vp_s + DB_COLS * DB;                          // [DB][S_ST]: what the write takes
+  float* o_s = u_s + DB * S_ST;                              // [DB][S_ST]
   const int row = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * DB_COLS;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int slot = a.slots[row];
   if (slot < 0 || slot >= a.num_slots) {
     if (tid == 0) report(a.status, STATUS_ROW_OUT_OF_RANGE, slot, row);
@@ -556,113 +521,116 @@ __global__ void __launch_bounds__(DB_THREADS) delta_block_scan_kernel(const Delt
     for (int e = tid; e < DB_COEF / 4; e += DB_THREADS) cp_async_16(stage + DP * QK_ST + e * 4, coef + e * 4, true);
     cp_async_commit();
   };
-  // This thread's token and column where v' is made.
-  const int my_t = tid / DB_COLS, my_c = tid % DB_COLS;
+  // This thread's token and column in the small products.
+  const int my_t = tid % DB, my_c = tid / DB;
   const T* v = static_cast<const T*>(a.v) + t0 * a.v_stride + head * a.V + col0 + my_c;
   auto fetch_v = [&](int p) {
-    const int at = p * DB + my_t;
-    return at < n && col0 + my_c < a.V ? to_float(v[at * a.v_stride]) : 0.0f;
+    const int t = p * DB + my_t;
+    return t < n && col0 + my_c < a.V ? to_float(v[t * a.v_stride]) : 0.0f;
   };
-  // This thread's part of the state: channels d0 and d0 + 8, columns 8 i + 2 t and the next, i = 0, 1.
-  const int d0 = warp * 16 + g;
-  const bool holds = warp * 16 < DP;
+  // This thread's part of the state: channels d0 and d0 + 1, columns c0 .. c0 + 3.
+  const int d0 = tid / 4 * 2, c0 = tid % 4 * 4;
+  const bool holds = d0 < DP;
   float S[2][4];
   float* state = a.state + static_cast<long long>(slot) * a.slot_stride + (static_cast<long long>(head) * a.V + col0) * a.D;
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int d = d0 + (e >> 1) * 8, c = 8 * i + 2 * t + (e & 1);
-      S[i][e] = holds && d < a.D && col0 + c < a.V ? state[static_cast<long long>(c) * a.D + d] : 0.0f;
-    }
+    for (int c = 0; c < 4; ++c)
+      S[i][c] = holds && d0 + i < a.D && col0 + c0 + c < a.V ? state[static_cast<long long>(c0 + c) * a.D + d0 + i] : 0.0f;
   auto store_state = [&]() {
-    if (!holds) return;
+    if (holds) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint2 hi, lo;
-        split_tf32(S[i][2 * half], hi.x, lo.x);
-        split_tf32(S[i][2 * half + 1], hi.y, lo.y);
-        const int at = (d0 + 8 * half) * DB_BST + 8 * i + 2 * t;
-        *reinterpret_cast<uint2*>(s_hi + at) = hi;
-        *reinterpret_cast<uint2*>(s_lo + at) = lo;
-      }
+      for (int i = 0; i < 2; ++i) *reinterpret_cast<float4*>(s_s + (d0 + i) * S_ST + c0) = make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
+    }
   };
   store_state();
   float v_now = 0.0f;
-#pragma unroll
-  for (int p = 0; p < DB_STAGES - 1; ++p) {
-    if (p < blocks) copy_block(p, stages + p * stage_floats);
-    else cp_async_commit();
+  if (blocks > 0) {
+    copy_block(0, stages);
+    v_now = fetch_v(0);
   }
-  if (blocks > 0) v_now = fetch_v(0);
   for (int p = 0; p < blocks; ++p) {
-    const float* stage = stages + p % DB_STAGES * stage_floats;
+    const float* stage = stages + (p & 1) * stage_floats;
     const float* coef = stage + DP * QK_ST;
-    cp_async_wait<DB_STAGES - 2>();
-    __syncthreads();             // the block and the state are there; the buffer of the block before is no longer read
-    if (p + DB_STAGES - 1 < blocks) copy_block(p + DB_STAGES - 1, stages + (p + DB_STAGES - 1) % DB_STAGES * stage_floats);
-    else cp_async_commit();
-    const float v_next = p + 1 < blocks ? fetch_v(p + 1) : 0.0f;
+    cp_async_wait<0>();
+    __syncthreads();             // the block and the state are there; the other buffer is no longer read
+    float v_next = 0.0f;
+    if (p + 1 < blocks) {
+      copy_block(p + 1, stages + ((p + 1) & 1) * stage_floats);
+      v_next = fetch_v(p + 1);
+    }
     {
-      const int rows0 = (warp & 1) * DB, cols0 = (warp >> 1 & 1) * 8, half = warp >> 2;
-      float hh[4] = {}, hl[4] = {}, lh[4] = {};
+      const int i0 = (lane & 7) * 4, rc = (lane >> 3) * 4;
+      float acc[4][4];
 #pragma unroll
-      for (int ks = 0; ks < DP / 16; ++ks) {
-        const int d = half * (DP / 2) + ks * 8;
-        product_step(hh, hl, lh, stage + d * QK_ST + rows0, 1, QK_ST, s_hi + d * DB_BST + cols0, s_lo + d * DB_BST + cols0, g, t);
+      for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
+#pragma unroll
+      for (int u = 0; u < DP / 8; ++u) {
+        const int d = warp * (DP / 8) + u;
+        float x[4], y[4];
+        *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(stage + d * QK_ST + i0);
+        *reinterpret_cast<float4*>(y) = *reinterpret_cast<const float4*>(s_s + d * S_ST + rc);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) acc[c][i] = fmaf(x[i], y[c], acc[c][i]);
       }
-      float* to = red_s + (half * 2 * DB + rows0 + g) * RED_ST + cols0 + 2 * t;
-      *reinterpret_cast<float2*>(to) = make_float2((lh[0] + hl[0]) + hh[0], (lh[1] + hl[1]) + hh[1]);
-      *reinterpret_cast<float2*>(to + 8 * RED_ST) = make_float2((lh[2] + hl[2]) + hh[2], (lh[3] + hl[3]) + hh[3]);
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        *reinterpret_cast<float4*>(red_s + (warp * DB_COLS + rc + c) * RED_ST + i0) = make_float4(acc[c][0], acc[c][1], acc[c][2], acc[c][3]);
     }
     __syncthreads();
-    const float whole = coef[2 * DB * DB_CST + DB];
+    float rk = 0.0f, rq = 0.0f;
+#pragma unroll
+    for (int w = 0; w < DB_THREADS / 32; ++w) {
+      rk += red_s[(w * DB_COLS + my_c) * RED_ST + my_t];
+      rq += red_s[(w * DB_COLS + my_c) * RED_ST + DB + my_t];
+    }
+    const float lead = coef[2 * DB * DB + my_t], whole = coef[2 * DB * DB + DB];
+    vp_s[my_c * DB + my_t] = v_now - lead * rk;
+    __syncthreads();
     {
-      const float lead = coef[2 * DB * DB_CST + my_t];
-      const float* rk = red_s + my_t * RED_ST + my_c;
-      const float* rq = rk + DB * RED_ST;
-      split_tf32(v_now - lead * (rk[0] + rk[2 * DB * RED_ST]), v_hi[my_t * DB_BST + my_c], v_lo[my_t * DB_BST + my_c]);
-      o_s[my_t * RED_ST + my_c] = lead * (rq[0] + rq[2 * DB * RED_ST]);
-    }
-    __syncthreads();
-    if (warp < 4) {
-      const int cols0 = (warp & 1) * 8;
-      const bool is_o = warp >= 2;
-      float hh[4] = {}, hl[4] = {}, lh[4] = {};
+      float u = 0.0f, o = 0.0f;
 #pragma unroll
-      for (int ks = 0; ks < 2; ++ks)
-        product_step(hh, hl, lh, coef + ((is_o ? DB : 0) + ks * 8) * DB_CST, 1, DB_CST, v_hi + ks * 8 * DB_BST + cols0,
-                     v_lo + ks * 8 * DB_BST + cols0, g, t);
+      for (int j = 0; j < DB; j += 4) {
+        float x[4];
+        *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(vp_s + my_c * DB + j);
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const int tok = g + 8 * half, c = cols0 + 2 * t;
-        const float x = (lh[2 * half] + hl[2 * half]) + hh[2 * half], y = (lh[2 * half + 1] + hl[2 * half + 1]) + hh[2 * half + 1];
-        if (!is_o) {
-          uint2 hi, lo;
-          split_tf32(x, hi.x, lo.x);
-          split_tf32(y, hi.y, lo.y);
-          *reinterpret_cast<uint2*>(u_hi + tok * DB_BST + c) = hi;
-          *reinterpret_cast<uint2*>(u_lo + tok * DB_BST + c) = lo;
-        } else if (p * DB + tok < n) {
-          float* to = a.out + (t0 + p * DB + tok) * a.heads * a.V + static_cast<long long>(head) * a.V + col0 + c;
-          if (col0 + c < a.V) to[0] = o_s[tok * RED_ST + c] + x;
-          if (col0 + c + 1 < a.V) to[1] = o_s[tok * RED_ST + c + 1] + y;
+        for (int i = 0; i < 4; ++i) {
+          u = fmaf(coef[(j + i) * DB + my_t], x[i], u);
+          o = fmaf(coef[DB * DB + (j + i) * DB + my_t], x[i], o);
         }
       }
+      u_s[my_t * S_ST + my_c] = u;
+      o_s[my_t * S_ST + my_c] = fmaf(lead, rq, o);
     }
     __syncthreads();
+    {
+      const int t = p * DB + tid / DB_COLS, c = tid % DB_COLS;
+      if (t < n && col0 + c < a.V)
+        a.out[(t0 + t) * a.heads * a.V + static_cast<long long>(head) * a.V + col0 + c] = o_s[tid / DB_COLS * S_ST + c];
+    }
     if (holds) {
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        float hh[4] = {}, hl[4] = {}, lh[4] = {};
+      for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int ks = 0; ks < 2; ++ks)
-          product_step(hh, hl, lh, stage + warp * 16 * QK_ST + ks * 8, QK_ST, 1, u_hi + ks * 8 * DB_BST + 8 * i,
-                       u_lo + ks * 8 * DB_BST + 8 * i, g, t);
+        for (int c = 0; c < 4; ++c) S[i][c] *= whole;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) S[i][e] = fmaf(whole, S[i][e], (lh[e] + hl[e]) + hh[e]);
+      for (int j = 0; j < DB; j += 4) {
+        float k0[4], k1[4];
+        *reinterpret_cast<float4*>(k0) = *reinterpret_cast<const float4*>(stage + d0 * QK_ST + j);
+        *reinterpret_cast<float4*>(k1) = *reinterpret_cast<const float4*>(stage + (d0 + 1) * QK_ST + j);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          float u[4];
+          *reinterpret_cast<float4*>(u) = *reinterpret_cast<const float4*>(u_s + (j + i) * S_ST + c0);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            S[0][c] = fmaf(k0[i], u[c], S[0][c]);
+            S[1][c] = fmaf(k1[i], u[c], S[1][c]);
+          }
+        }
       }
     }
     store_state();               // (nobody reads the state's tile between the barriers above and the next one)
@@ -672,17 +640,16 @@ __global__ void __launch_bounds__(DB_THREADS) delta_block_scan_kernel(const Delt
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int d = d0 + (e >> 1) * 8, c = 8 * i + 2 * t + (e & 1);
-      if (d < a.D && col0 + c < a.V) state[static_cast<long long>(c) * a.D + d] = S[i][e];
-    }
+    for (int c = 0; c < 4; ++c)
+      if (d0 + i < a.D && col0 + c0 + c < a.V) state[static_cast<long long>(c0 + c) * a.D + d0 + i] = S[i][c];
 }
 
 template <int DP>
 constexpr size_t delta_blocks_smem() { return sizeof(float) * (2 * DB * (DP + 4) + 5 * DB * DB + 2 * DB); }
 template <int DP>
 constexpr size_t delta_block_scan_smem() {
-  return sizeof(float) * (DB_STAGES * (DP * (2 * DB + 8) + DB_COEF) + 5 * DB * (DB_COLS + 4) + 2 * DP * DB_BST + 4 * DB * DB_BST);
+  return sizeof(float) * (2 * (DP * (2 * DB + 4) + DB_COEF) + DP * (DB_COLS + 4) + DB_THREADS / 32 * DB_COLS * (2 * DB + 4) +
+                          DB_COLS * DB + 2 * DB * (DB_COLS + 4));
 }
 
 }  // namespace zb
