@@ -226,3 +226,32 @@ def test_the_delta_rule_in_blocks_keeps_float32(cuda_device, dim, vdim):
     # (measured over such inputs: 0.7 to 0.9 of the token-by-token form's error; operands of two TF32 values: 1.5 to 1.9)
     for blocks, tokens in zip(error([T]), error([15] * (T // 15) + [T % 15])):
         assert blocks <= 1.2 * tokens
+
+
+@pytest.mark.parametrize("rate", [50.0, 300.0, 3000.0, math.inf])
+def test_the_delta_rule_behind_a_token_that_forgets(cuda_device, rate):
+    """Tokens with logarithms of their decays of -rate in front of tokens that forget next to nothing: what the latter give
+    and the state behind them are as good as without the former, and a decay of exactly zero is a zero."""
+    from zephyr_b200.kernels import ops
+
+    heads, groups, dim, vdim, T = 2, 1, 64, 32, 96
+    g = torch.Generator().manual_seed(6)
+    q, k, v, b = (torch.randn(T, n, generator=g) for n in (groups * dim, groups * dim, heads * vdim, heads))
+    # A step of softplus(a) at a rate of e^3: -8 is next to no decay, a large one e^(-20 a).
+    a, a_log = torch.full((T, heads), -8.0), torch.full((heads,), 3.0)
+    strong = [0, 1, 17, 32, 33, 50, 80]
+    a[strong] = min(rate / math.exp(3.0), 3e38)
+    b += 2.0
+    ba = torch.cat([b, a], dim=1).to(cuda_device)
+    i32 = lambda values: torch.tensor(values, dtype=torch.int32, device=cuda_device)
+    state, status = torch.ones(1, heads * dim * vdim, device=cuda_device), ops.new_status(cuda_device)
+    expected, last = _delta_in_float64(q, k, v, b, a, a_log, torch.zeros(heads), heads, groups, dim, vdim, state)
+    out = ops.delta_rule(q.to(cuda_device), k.to(cuda_device), v.to(cuda_device), ba[:, :heads], ba[:, heads:], a_log.to(cuda_device),
+                         torch.zeros(heads, device=cuda_device), heads, groups, dim, vdim, state, i32([0]), i32([0]), i32([T]), status,
+                         q_scale=dim ** -0.5)
+    ops.check_status(status)
+    # Sums over 64 channels and up to 30 tokens of memory in float32: some tens of roundings of 2^-24 of the largest value.
+    behind = torch.tensor([t for t in range(T) if t not in strong])
+    got, want = out.cpu().double().view(T, heads, vdim)[behind], expected[behind]
+    assert (got - want).abs().max() <= 2e-6 * float(want.abs().max())
+    assert (state.cpu().double().view_as(last) - last).abs().max() <= 2e-6 * float(last.abs().max())

@@ -319,7 +319,9 @@ __global__ void __launch_bounds__(DS_THREADS) delta_scan_kernel(const DeltaScanA
 //   Tu = diag(e^(c_B - c_t)) (I + A)^-1 diag(beta)       (what the write takes is Tu v')
 //   M  = P (I + A)^-1 diag(beta),  P_tj = e^(c_t - c_j) (q_t . k_j)   (o = e^(c) R_q + M v')
 //
-// and delta_block_scan walks a request's blocks.  Exponents are differences of sums within a block, never positive.
+// and delta_block_scan walks a request's blocks.  Exponents are differences of sums within a block, never positive; the sums
+// are formed in 64 bits and kept as two float32 values, so that a difference is good to a rounding of itself, also behind a
+// token that forgets everything.
 // Tokens behind a portion's end have beta 0 and decay 1.  Blocks are numbered row by row (first_piece_of_row).
 constexpr int DB = 16;                     // tokens of a block
 constexpr int DB_THREADS = 256;
@@ -349,8 +351,11 @@ __global__ void __launch_bounds__(DB_THREADS) delta_blocks_kernel(const DeltaBlo
   float* a_s = qk_s + DB * DB;             // [DB][DB]: A
   float* p_s = a_s + DB * DB;              // [DB][DB]: P
   float* t_s = p_s + DB * DB;              // [DB][DB]: (I + A)^-1 diag(beta)
-  float* c_s = t_s + DB * DB;              // [DB]
-  float* beta_s = c_s + DB;
+  float* c_hi = t_s + DB * DB;             // [DB]: the sums of logarithms c_t = c_hi + c_lo
+  float* c_lo = c_hi + DB;
+  float* lead_s = c_lo + DB;               // [DB]: e^(c_t)
+  float* tail_s = lead_s + DB;             // [DB]: e^(c_B - c_t)
+  float* beta_s = tail_s + DB;
   const int block = blockIdx.x, group = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int own;
   const int row = row_of_piece<DB>(a.row_q_len, a.rows, block, own);
@@ -422,29 +427,35 @@ __global__ void __launch_bounds__(DB_THREADS) delta_blocks_kernel(const DeltaBlo
   for (int h = group * per; h < (group + 1) * per; ++h) {
     __syncthreads();                       // the products are there, and the head before is done
     if (tid < 32) {
-      float c = 0.0f, beta = 0.0f;
+      double c = 0.0;
+      float beta = 0.0f;
       if (lane < n) {
         const long long at = (t0 + lane) * a.ba_stride + h;
         beta = 1.0f / (1.0f + expf(-a.b[at]));
-        c = -expf(a.a_log[h]) * softplus_d(a.a[at] + a.dt_bias[h]);
+        c = -static_cast<double>(expf(a.a_log[h])) * static_cast<double>(softplus_d(a.a[at] + a.dt_bias[h]));
+        if (c < -1000.0) c = -1000.0;      // zero either way; the bound keeps the sums finite (a NaN passes)
       }
 #pragma unroll
       for (int o = 1; o < DB; o <<= 1) {
-        const float before = __shfl_up_sync(0xffffffffu, c, o);
+        const double before = __shfl_up_sync(0xffffffffu, c, o);
         if (lane >= o) c += before;
       }
+      const double all = __shfl_sync(0xffffffffu, c, DB - 1);
       if (lane < DB) {
-        c_s[lane] = c;
+        const float hi = static_cast<float>(c), lo = static_cast<float>(c - hi), lead = expf(hi);
+        c_hi[lane] = hi;
+        c_lo[lane] = lo;
+        lead_s[lane] = fmaf(lead, lo, lead);
+        tail_s[lane] = expf(static_cast<float>(all - c));
         beta_s[lane] = beta;
       }
     }
     __syncthreads();
-    const float decay = j <= t ? expf(c_s[t] - c_s[j]) : 0.0f;
+    const float decay = j <= t ? expf((c_hi[t] - c_hi[j]) + (c_lo[t] - c_lo[j])) : 0.0f;
     a_s[tid] = j < t ? beta_s[t] * decay * kk_s[tid] : 0.0f;
     p_s[tid] = decay * qk_s[tid];
     __syncthreads();
     float* coef = a.coef + (static_cast<long long>(block) * a.heads + h) * DB_COEF;
-    const float last = c_s[DB - 1];
     if (tid < DB) {
       // A column of the inverse by forward substitution, times beta of the column.
       float x[DB];
@@ -461,12 +472,12 @@ __global__ void __launch_bounds__(DB_THREADS) delta_blocks_kernel(const DeltaBlo
     __syncthreads();
     // (threads run over the rows of the transposed matrices: t fastest)
     const int tt = tid % DB, jj = tid / DB;
-    coef[jj * DB + tt] = expf(last - c_s[tt]) * t_s[tt * DB + jj];
+    coef[jj * DB + tt] = tail_s[tt] * t_s[tt * DB + jj];
     float m = 0.0f;
     for (int i = jj; i <= tt; ++i) m = fmaf(p_s[tt * DB + i], t_s[i * DB + jj], m);
     coef[(DB + jj) * DB + tt] = m;
-    if (tid < DB) coef[2 * DB * DB + tid] = expf(c_s[tid]);
-    if (tid == 0) coef[2 * DB * DB + DB] = expf(last);
+    if (tid < DB) coef[2 * DB * DB + tid] = lead_s[tid];
+    if (tid == 0) coef[2 * DB * DB + DB] = lead_s[DB - 1];
   }
 }
 
@@ -645,7 +656,7 @@ __global__ void __launch_bounds__(DB_THREADS) delta_block_scan_kernel(const Delt
 }
 
 template <int DP>
-constexpr size_t delta_blocks_smem() { return sizeof(float) * (2 * DB * (DP + 4) + 5 * DB * DB + 2 * DB); }
+constexpr size_t delta_blocks_smem() { return sizeof(float) * (2 * DB * (DP + 4) + 5 * DB * DB + 5 * DB); }
 template <int DP>
 constexpr size_t delta_block_scan_smem() {
   return sizeof(float) * (2 * (DP * (2 * DB + 4) + DB_COEF) + DP * (DB_COLS + 4) + DB_THREADS / 32 * DB_COLS * (2 * DB + 4) +
