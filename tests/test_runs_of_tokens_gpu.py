@@ -255,3 +255,37 @@ def test_the_delta_rule_behind_a_token_that_forgets(cuda_device, rate):
     got, want = out.cpu().double().view(T, heads, vdim)[behind], expected[behind]
     assert (got - want).abs().max() <= 2e-6 * float(want.abs().max())
     assert (state.cpu().double().view_as(last) - last).abs().max() <= 2e-6 * float(last.abs().max())
+
+
+@pytest.mark.parametrize("kind", ["delta"])
+def test_a_value_that_is_not_finite_stays_with_later_tokens(cuda_device, kind):
+    """An infinity or a NaN in one value of a token: all tokens before it, and all other columns, keep their bits."""
+    from zephyr_b200.kernels import ops
+
+    heads, per, dim, vdim, T = 4, 2 if kind != "retention" else 1, 64, 48, 150
+    groups, g = heads // per, torch.Generator().manual_seed(4)
+    dtype = torch.bfloat16 if kind == "state_space" else torch.float32
+    q, k, v, b, a = (torch.randn(T, n, generator=g).to(cuda_device) for n in (groups * dim, groups * dim, heads * vdim, heads, heads))
+    q, k, v, dt = (t.to(dtype) for t in (q, k, v, a))
+    constants = [(torch.rand(heads, generator=g) - 0.5).to(cuda_device) for _ in range(3)]
+    i32 = lambda values: torch.tensor(values, dtype=torch.int32, device=cuda_device)
+    status = ops.new_status(cuda_device)
+
+    def run(values):
+        rows = (torch.zeros(1, heads * dim * vdim, device=cuda_device), i32([0]), i32([0]), i32([T]), status)
+        if kind == "delta":
+            return ops.delta_rule(q, k, values, b, a, constants[0], constants[1], heads, groups, dim, vdim, *rows, q_scale=dim ** -0.5)
+        if kind == "retention":
+            return ops.retention(q, k, values, constants[0].abs() + 0.4, heads, dim, vdim, *rows)
+        return ops.decayed_state_scan("state_space", q, k, values, heads, dim, vdim, *rows, dt=dt, dt_bias=constants[0], a_log=constants[1],
+                                      skip=constants[2], heads_per_group=per)
+
+    clean = run(v)
+    for at, bad in ((0, math.nan), (7, math.inf), (15, -math.inf), (16, math.inf), (37, math.nan), (63, math.inf), (70, math.inf), (149, math.nan)):
+        values, column = v.clone(), (2 * at + 5) % (heads * vdim)
+        values[at, column] = bad
+        got, others = run(values), torch.arange(heads * vdim, device=cuda_device) != column
+        ops.check_status(status)
+        assert torch.equal(got[:at], clean[:at]), at
+        assert torch.equal(got[:, others], clean[:, others]), at
+        assert not torch.isfinite(got[at:, column]).any(), at

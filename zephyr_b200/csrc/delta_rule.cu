@@ -500,7 +500,7 @@ struct DeltaBlockScanArgs {
 // with the matrices, 522 token by token).  Products on the tensor cores with operands of two TF32 values each took 30 us less,
 // at 1.5 to 1.9 times the token-by-token form's error against 64 bits; this form has 0.5 to 0.9 of it.
 template <typename T, int DP>
-__global__ void __launch_bounds__(DB_THREADS) delta_block_scan_kernel(const DeltaBlockScanArgs a) {
+__global__ void __launch_bounds__(DB_THREADS, 2) delta_block_scan_kernel(const DeltaBlockScanArgs a) {
   extern __shared__ __align__(16) float db_smem[];
   constexpr int QK_ST = 2 * DB + 4, S_ST = DB_COLS + 4, RED_ST = 2 * DB + 4;
   constexpr int stage_floats = DP * QK_ST + DB_COEF;
@@ -510,8 +510,10 @@ __global__ void __launch_bounds__(DB_THREADS) delta_block_scan_kernel(const Delt
   float* vp_s = red_s + DB_THREADS / 32 * DB_COLS * RED_ST;  // [DB_COLS][DB]: v'
   float* u_s = vp_s + DB_COLS * DB;                          // [DB][S_ST]: what the write takes
   float* o_s = u_s + DB * S_ST;                              // [DB][S_ST]
+  __shared__ int wild;                                       // the last block with a v' that is not finite
   const int row = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * DB_COLS;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) wild = -1;
   const int slot = a.slots[row];
   if (slot < 0 || slot >= a.num_slots) {
     if (tid == 0) report(a.status, STATUS_ROW_OUT_OF_RANGE, slot, row);
@@ -599,18 +601,28 @@ __global__ void __launch_bounds__(DB_THREADS) delta_block_scan_kernel(const Delt
       rq += red_s[(w * DB_COLS + my_c) * RED_ST + DB + my_t];
     }
     const float lead = coef[2 * DB * DB + my_t], whole = coef[2 * DB * DB + DB];
-    vp_s[my_c * DB + my_t] = v_now - lead * rk;
+    const float vp = v_now - lead * rk;
+    vp_s[my_c * DB + my_t] = vp;
+    if (!isfinite(vp)) wild = p;
     __syncthreads();
     {
       float u = 0.0f, o = 0.0f;
+      if (wild != p) {
 #pragma unroll
-      for (int j = 0; j < DB; j += 4) {
-        float x[4];
-        *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(vp_s + my_c * DB + j);
+        for (int j = 0; j < DB; j += 4) {
+          float x[4];
+          *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(vp_s + my_c * DB + j);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          u = fmaf(coef[(j + i) * DB + my_t], x[i], u);
-          o = fmaf(coef[DB * DB + (j + i) * DB + my_t], x[i], o);
+          for (int i = 0; i < 4; ++i) {
+            u = fmaf(coef[(j + i) * DB + my_t], x[i], u);
+            o = fmaf(coef[DB * DB + (j + i) * DB + my_t], x[i], o);
+          }
+        }
+      } else {
+        // The same sums, without a zero times a later token's value.
+        for (int j = 0; j <= my_t; ++j) {
+          u = fmaf(coef[j * DB + my_t], vp_s[my_c * DB + j], u);
+          o = fmaf(coef[(DB + j) * DB + my_t], vp_s[my_c * DB + j], o);
         }
       }
       u_s[my_t * S_ST + my_c] = u;
