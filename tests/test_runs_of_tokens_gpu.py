@@ -257,7 +257,7 @@ def test_the_delta_rule_behind_a_token_that_forgets(cuda_device, rate):
     assert (state.cpu().double().view_as(last) - last).abs().max() <= 2e-6 * float(last.abs().max())
 
 
-@pytest.mark.parametrize("kind", ["delta"])
+@pytest.mark.parametrize("kind", ["delta", "state_space", "retention"])
 def test_a_value_that_is_not_finite_stays_with_later_tokens(cuda_device, kind):
     """An infinity or a NaN in one value of a token: all tokens before it, and all other columns, keep their bits."""
     from zephyr_b200.kernels import ops

@@ -22,10 +22,16 @@
 // Products run on the tensor cores, float32 sums.  A bfloat16 operand is exact; beside it a float32 operand is the sum
 // of three bfloat16 values (all its 24 bits); two float32 operands (WALK_FIXED) are two bfloat16 values each, hi hi + hi lo +
 // lo hi, a relative error of about 2^-16 an operand.  The state itself is only ever touched by float32 multiply-adds.
+// A value that is not finite must not reach the tokens before it through the zeros above P's diagonal: it is left out of the
+// product and added by hand to the outputs of the tokens from its own on.  What is behind it is not finite either, an
+// infinity or a NaN.
+//
 // Sums of logarithms are formed in 64 bits and kept as two float32 values, so that a difference of two is good to a
 // rounding of itself.
 //
 // Pieces are numbered row by row (first_piece_of_row).
+#include <type_traits>
+
 #include "common.cuh"
 #include "mma.cuh"
 
@@ -61,6 +67,7 @@ struct WalkArgs {
 
 template <int MODE, int DP>
 struct WalkParts {
+  using Value = typename std::conditional<MODE == WALK_SPACE, __nv_bfloat16, float>::type;
   static constexpr int PA = MODE == WALK_SPACE ? 1 : 2;      // parts of q, k and v
   static constexpr int PB = MODE == WALK_SPACE ? 3 : 2;      // parts of P, the state and the weighted values
   static constexpr int ST = DP + 8;
@@ -321,13 +328,38 @@ struct WalkShape : WalkParts<MODE, DP> {
       STAGES * stage_bytes + Parts::PB * DP * CST * 2 + (Parts::PA + Parts::PB) * W * CST * 2 + W * OST * 4;
 };
 
+// The values of a piece that are not finite, added to the outputs of tokens i0 and i0 + 8, columns c0 and c0 + 1 of each of `tiles`
+// tiles of 8; `v` and `out` begin at the piece's first token and the CTA's first of `cols` columns.  (A call of its own, with plain
+// arguments: inlined, its registers cost every piece 10 % of the walk.)
+template <typename T, int PB>
+__device__ __noinline__ void add_wild(float* out, long long out_stride, const T* v, long long v_stride, int n, int cols, int tiles, int i0,
+                                      int c0, float skip, const __nv_bfloat16* p_s) {
+  for (int e = 0; e < 4 * tiles; ++e) {
+    const int tok = i0 + (e & 2) * 4, c = e / 4 * 8 + c0 + (e & 1);
+    if (tok >= n || c >= cols) continue;
+    for (int j = 0; j <= tok; ++j) {
+      const float x = to_float(v[j * v_stride + c]);
+      if (isfinite(x)) continue;
+      float weight = j == tok ? skip : 0.0f;
+      for (int q = 0; q < PB; ++q) weight += __bfloat162float(p_s[(q * W + tok) * W_PST + j]);
+      out[tok * out_stride + c] = fmaf(weight, x, out[tok * out_stride + c]);
+    }
+  }
+}
+
+// Zeros in the place of values that are not finite.
+__device__ __noinline__ void drop_wild(__nv_bfloat16* v_s, int count) {
+  for (int e = threadIdx.x; e < count; e += W_THREADS)
+    if (!isfinite(__bfloat162float(v_s[e]))) v_s[e] = __float2bfloat16_rn(0.0f);
+}
+
 // NT: tiles of 8 value columns of a CTA.  Warp w owns the state's channels 16 w .. (C fragments); for the outputs it owns
 // tokens 16 (w % 4) .. and takes half the channels (S^T q) and every other 16 keys (P).  A piece:
 //   barrier; both terms of the outputs and the state's sums from shared memory; one half of the outputs' sums to shared memory;
 //   barrier; the other half adds it and writes; the state and the next piece's values go to shared memory in parts.
 // The next piece comes meanwhile, in two bulk copies.
 template <int MODE, int DP, int NT>
-__global__ void __launch_bounds__(W_THREADS) state_walk_kernel(const WalkArgs a) {
+__global__ void __launch_bounds__(W_THREADS, 2) state_walk_kernel(const WalkArgs a) {
   using Shape = WalkShape<MODE, DP, NT>;
   constexpr int PA = Shape::PA, PB = Shape::PB, ST = Shape::ST, COLS = Shape::COLS, CST = Shape::CST, OST = Shape::OST;
   constexpr int STAGES = Shape::STAGES, PER = W * COLS / W_THREADS / 2;      // pairs of values a thread brings of a piece
@@ -337,6 +369,7 @@ __global__ void __launch_bounds__(W_THREADS) state_walk_kernel(const WalkArgs a)
   __nv_bfloat16* wv_s = v_s + PA * W * CST;                  // [PB][W][CST]: w_j v_j
   float* o_s = reinterpret_cast<float*>(wv_s + PB * W * CST);            // [W][OST]
   __shared__ unsigned long long landed[STAGES];
+  __shared__ int wild;                                       // the last piece with a value that is not finite
   const int row = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * COLS;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int slot = a.slots[row];
@@ -351,6 +384,7 @@ __global__ void __launch_bounds__(W_THREADS) state_walk_kernel(const WalkArgs a)
 #pragma unroll
     for (int i = 0; i < STAGES; ++i) mbar_init(&landed[i], 1);
     fence_barrier_init();
+    wild = -1;
   }
   __syncthreads();
 
@@ -395,7 +429,8 @@ __global__ void __launch_bounds__(W_THREADS) state_walk_kernel(const WalkArgs a)
       }
     }
   };
-  auto store_values = [&]() {
+  auto store_values = [&](int p) {
+    float top = 0.0f;                                        // NaN if one of the values is not finite
 #pragma unroll
     for (int u = 0; u < PER; ++u) {
       const int at = (my_i + u * TOKENS) * CST + my_c;
@@ -407,12 +442,14 @@ __global__ void __launch_bounds__(W_THREADS) state_walk_kernel(const WalkArgs a)
       } else {
         split_parts<PA>(value[u][0], value[u][1], vp);
       }
+      top = fmaf(0.0f, value[u][0], fmaf(0.0f, value[u][1], top));
       split_parts<PB>(value[u][0] * weight[u], value[u][1] * weight[u], wp);
 #pragma unroll
-      for (int p = 0; p < PA; ++p) *reinterpret_cast<unsigned*>(v_s + p * W * CST + at) = vp[p];
+      for (int i = 0; i < PA; ++i) *reinterpret_cast<unsigned*>(v_s + i * W * CST + at) = vp[i];
 #pragma unroll
-      for (int p = 0; p < PB; ++p) *reinterpret_cast<unsigned*>(wv_s + p * W * CST + at) = wp[p];
+      for (int i = 0; i < PB; ++i) *reinterpret_cast<unsigned*>(wv_s + i * W * CST + at) = wp[i];
     }
+    if (top != 0.0f) wild = p;
   };
   // This thread's part of the state: channels d0 and d0 + 8, columns 8 i + 2 t and the next.
   const int d0 = warp * 16 + g;
@@ -441,7 +478,7 @@ __global__ void __launch_bounds__(W_THREADS) state_walk_kernel(const WalkArgs a)
   if (tid == 0 && pieces > 0) copy_piece(0);
   store_state();
   fetch_values(0);
-  store_values();
+  store_values(0);
   const float skip = MODE == WALK_SPACE ? a.skip[h] : 0.0f;
   // ldmatrix addresses: A rows as they lie, P's likewise, A transposed, B as [k][n].
   const int lrow = (lane & 7) + ((lane >> 3) & 1) * 8, lcol = (lane >> 4) * 8;
@@ -464,6 +501,11 @@ __global__ void __launch_bounds__(W_THREADS) state_walk_kernel(const WalkArgs a)
     if (tid == 0 && p + 1 < pieces) copy_piece(p + 1);
     fetch_values(p + 1);
     const int i0 = row0 + g, i1 = i0 + 8;
+    const bool tame = wild != p;
+    if (!tame) {
+      drop_wild(v_s, PA * W * CST);
+      __syncthreads();
+    }
     float o[NT][4] = {};
     if (row0 < n) {
 #pragma unroll
@@ -528,7 +570,7 @@ __global__ void __launch_bounds__(W_THREADS) state_walk_kernel(const WalkArgs a)
     }
     __syncthreads();               // the state's, the values' and the piece's reads are done
     store_state();
-    store_values();
+    store_values(p + 1);
     if (half == 0 && row0 < n) {
 #pragma unroll
       for (int i = 0; i < NT; ++i)
@@ -545,6 +587,13 @@ __global__ void __launch_bounds__(W_THREADS) state_walk_kernel(const WalkArgs a)
             if (v0 + c + 1 < a.V) to[1] = o[i][2 * r + 1] + y.y;
           }
         }
+      // (the outputs that this thread has just written; the piece's buffer is filled again behind the next barrier)
+      if (!tame) {
+        using T = typename Shape::Value;
+        const long long at = t0 + p * W;
+        add_wild<T, PB>(a.out + at * a.H * a.V + static_cast<long long>(h) * a.V + v0, static_cast<long long>(a.H) * a.V,
+                        static_cast<const T*>(a.v) + at * a.v_stride + h * a.V + v0, a.v_stride, n, a.V - v0, NT, i0, 2 * t, skip, p_s);
+      }
     }
   }
   if (!a.write_state || !holds) return;
