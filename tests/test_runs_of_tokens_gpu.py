@@ -289,3 +289,38 @@ def test_a_value_that_is_not_finite_stays_with_later_tokens(cuda_device, kind):
         assert torch.equal(got[:at], clean[:at]), at
         assert torch.equal(got[:, others], clean[:, others]), at
         assert not torch.isfinite(got[at:, column]).any(), at
+
+
+@pytest.mark.parametrize("dim,vdim", [(128, 64), (64, 40)])
+def test_the_state_space_walk_keeps_float32(cuda_device, dim, vdim):
+    """With rates and steps as such models start them, the walk over pieces is as close to 64 bits as the scan over tokens."""
+    from zephyr_b200.kernels import ops
+
+    heads, per, T = 8, 4, 700
+    groups, g = heads // per, torch.Generator().manual_seed(dim)
+    bf = lambda *shape: torch.randn(*shape, generator=g).to(torch.bfloat16)
+    q, k, v, dt = bf(T, groups * dim), bf(T, groups * dim), bf(T, heads * vdim), bf(T, heads)
+    step = torch.exp(torch.rand(heads, generator=g) * math.log(100.0) - math.log(1000.0))
+    a_log, dt_bias = torch.log(1.0 + 15.0 * torch.rand(heads, generator=g)), step + torch.log(-torch.expm1(-step))
+    skip = torch.randn(heads, generator=g)
+    dev = lambda t: t.to(cuda_device)
+    i32 = lambda values: torch.tensor(values, dtype=torch.int32, device=cuda_device)
+    status, own = ops.new_status(cuda_device), torch.arange(heads) // per
+    taken = torch.nn.functional.softplus(dt.double() + dt_bias.double())
+    decay = torch.exp(-torch.exp(a_log.double()) * taken)
+    S, expected = torch.zeros(heads, dim, vdim, dtype=torch.float64), torch.zeros(T, heads, vdim, dtype=torch.float64)
+    for t in range(T):
+        values = v[t].double().view(heads, vdim)
+        S = S * decay[t].view(-1, 1, 1) + (k[t].double().view(groups, dim)[own] * taken[t].view(-1, 1)).unsqueeze(-1) * values.unsqueeze(1)
+        expected[t] = torch.einsum("hdv,hd->hv", S, q[t].double().view(groups, dim)[own]) + skip.double().view(-1, 1) * values
+
+    def error(segment):
+        state = torch.zeros(1, heads * dim * vdim, device=cuda_device)
+        out = ops.decayed_state_scan("state_space", dev(q), dev(k), dev(v), heads, dim, vdim, state, i32([0]), i32([0]), i32([T]), status,
+                                     dt=dev(dt), dt_bias=dev(dt_bias), a_log=dev(a_log), skip=dev(skip), heads_per_group=per, segment=segment)
+        ops.check_status(status)
+        return (float((out.cpu().double().view_as(expected) - expected).norm() / expected.norm()),
+                float((state.cpu().double().view_as(S) - S).norm() / S.norm()))
+
+    for walk, scan in zip(error(None), error(0)):
+        assert walk <= 1.15 * scan, (walk, scan)

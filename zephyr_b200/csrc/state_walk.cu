@@ -19,9 +19,10 @@
 // included: 45 + 118 us, 203 in three passes and a rotation.  Bound by the pieces' way out of L2 (3.7 of about 4 TB/s, retention)
 // and by the two barriers with eight warps an SM (the state-space form).
 //
-// Products run on the tensor cores, float32 sums.  A bfloat16 operand is exact; beside it a float32 operand is the sum
-// of three bfloat16 values (all its 24 bits); two float32 operands (WALK_FIXED) are two bfloat16 values each, hi hi + hi lo +
-// lo hi, a relative error of about 2^-16 an operand.  The state itself is only ever touched by float32 multiply-adds.
+// Products run on the tensor cores, float32 sums.  A bfloat16 operand is exact; beside it a float32 operand is the sum of three
+// bfloat16 values (all its 24 bits).  The tensor cores cut a sum at every step, so there the products of the small parts have
+// a sum of their own, and scores two (error against 64 bits over 2048 and 77 tokens: 1.32e-7, 1.82e-7 with one sum each,
+// 1.29e-7 token by token).  Two float32 operands (WALK_FIXED) are two bfloat16 values each, hi hi + hi lo + lo hi, a relative error of about 2^-16 an operand.  The state itself is only ever touched by float32 multiply-adds.
 // A value that is not finite must not reach the tokens before it through the zeros above P's diagonal: it is left out of the
 // product and added by hand to the outputs of the tokens from its own on.  What is behind it is not finite either, an
 // infinity or a NaN.
@@ -105,16 +106,17 @@ struct WalkB {
       for (int n = 0; n < N / 2; ++n) ldmatrix_x4_trans(f[pb][n], b + pb * part_stride + n * 16);
   }
 };
-// acc += A B.  The tiles take turns, so that no product waits for the one before it.
+// acc + low += A B, the products of large parts in acc, all others in low (which may be acc).  The tiles take turns, so that no
+// product waits for the one before it.
 template <int N, int PA, int PB>
-__device__ __forceinline__ void walk_product(float (&acc)[N][4], const unsigned (&af)[PA][4], const WalkB<N, PB>& b) {
+__device__ __forceinline__ void walk_product(float (&acc)[N][4], float (&low)[N][4], const unsigned (&af)[PA][4], const WalkB<N, PB>& b) {
 #pragma unroll
   for (int pb = PB - 1; pb >= 0; --pb)                       // the small products first
 #pragma unroll
     for (int pa = PA - 1; pa >= 0; --pa)
       if (counts<PA, PB>(pa, pb)) {
 #pragma unroll
-        for (int n = 0; n < N; ++n) mma_bf16_16816(acc[n], af[pa], b.f[pb][n / 2][n % 2 * 2], b.f[pb][n / 2][n % 2 * 2 + 1]);
+        for (int n = 0; n < N; ++n) mma_bf16_16816(pa + pb > 0 ? low[n] : acc[n], af[pa], b.f[pb][n / 2][n % 2 * 2], b.f[pb][n / 2][n % 2 * 2 + 1]);
       }
 }
 
@@ -279,7 +281,7 @@ __global__ void __launch_bounds__(W_THREADS) walk_prepare_kernel(const WalkArgs 
   for (int u = 0; u < 2; ++u) {
     const int c0 = col0 + u * 16;
     if (c0 > row0) continue;
-    float s[2][4] = {};
+    float s2[2][2][4] = {}, s[2][4];
 #pragma unroll
     for (int ks = 0; ks < DP / 16; ++ks) {
       unsigned af[PA][4], bf[PA][4];
@@ -293,10 +295,14 @@ __global__ void __launch_bounds__(W_THREADS) walk_prepare_kernel(const WalkArgs 
 #pragma unroll
         for (int pb = PA - 1; pb >= 0; --pb)
           if (counts<PA, PA>(pa, pb)) {
-            mma_bf16_16816(s[0], af[pa], bf[pb][0], bf[pb][1]);
-            mma_bf16_16816(s[1], af[pa], bf[pb][2], bf[pb][3]);
+            mma_bf16_16816(s2[ks & 1][0], af[pa], bf[pb][0], bf[pb][1]);
+            mma_bf16_16816(s2[ks & 1][1], af[pa], bf[pb][2], bf[pb][3]);
           }
     }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) s[i][e] = s2[0][i][e] + s2[1][i][e];
     for (int w = 0; w < heads; ++w) {
       unsigned char* head = head0 + w * Parts::head_bytes;
 #pragma unroll
@@ -361,6 +367,7 @@ __device__ __noinline__ void drop_wild(__nv_bfloat16* v_s, int count) {
 template <int MODE, int DP, int NT>
 __global__ void __launch_bounds__(W_THREADS, 2) state_walk_kernel(const WalkArgs a) {
   using Shape = WalkShape<MODE, DP, NT>;
+  constexpr bool SPLIT_SUMS = MODE == WALK_SPACE;
   constexpr int PA = Shape::PA, PB = Shape::PB, ST = Shape::ST, COLS = Shape::COLS, CST = Shape::CST, OST = Shape::OST;
   constexpr int STAGES = Shape::STAGES, PER = W * COLS / W_THREADS / 2;      // pairs of values a thread brings of a piece
   extern __shared__ __align__(16) unsigned char w_smem[];
@@ -506,7 +513,8 @@ __global__ void __launch_bounds__(W_THREADS, 2) state_walk_kernel(const WalkArgs
       drop_wild(v_s, PA * W * CST);
       __syncthreads();
     }
-    float o[NT][4] = {};
+    float o[NT][4] = {}, own_low[NT][4] = {};
+    float (&low)[NT][4] = SPLIT_SUMS ? own_low : o;
     if (row0 < n) {
 #pragma unroll
       for (int ks = 0; ks < DP / 32; ++ks) {
@@ -516,13 +524,17 @@ __global__ void __launch_bounds__(W_THREADS, 2) state_walk_kernel(const WalkArgs
 #pragma unroll
         for (int x = 0; x < PA; ++x) ldmatrix_x4(af[x], q_s + (x * W + row0) * ST + a_off + d);
         b.load(s_s + d * CST + b_off, DP * CST);
-        walk_product<NT, PA, PB>(o, af, b);
+        walk_product<NT, PA, PB>(o, low, af, b);
       }
       const float lead0 = steps[i0], lead1 = steps[i1];
 #pragma unroll
       for (int i = 0; i < NT; ++i) {
         o[i][0] *= lead0; o[i][1] *= lead0;
         o[i][2] *= lead1; o[i][3] *= lead1;
+        if (SPLIT_SUMS) {
+          low[i][0] *= lead0; low[i][1] *= lead0;
+          low[i][2] *= lead1; low[i][3] *= lead1;
+        }
       }
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
@@ -533,7 +545,13 @@ __global__ void __launch_bounds__(W_THREADS, 2) state_walk_kernel(const WalkArgs
 #pragma unroll
         for (int x = 0; x < PB; ++x) ldmatrix_x4(pf[x], p_s + (x * W + row0) * W_PST + p_off + j0);
         b.load(v_s + j0 * CST + b_off, W * CST);
-        walk_product<NT, PB, PA>(o, pf, b);
+        walk_product<NT, PB, PA>(o, low, pf, b);
+      }
+      if (SPLIT_SUMS) {
+#pragma unroll
+        for (int i = 0; i < NT; ++i)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) o[i][e] += low[i][e];
       }
       if (half == 1) {
 #pragma unroll
@@ -552,7 +570,7 @@ __global__ void __launch_bounds__(W_THREADS, 2) state_walk_kernel(const WalkArgs
       }
     }
     if (holds) {
-      float sum[NT][4] = {};
+      float sum[NT][4] = {}, sum_low[NT][4] = {};
 #pragma unroll
       for (int ks = 0; ks < W / 16; ++ks) {
         unsigned af[PA][4];
@@ -560,13 +578,13 @@ __global__ void __launch_bounds__(W_THREADS, 2) state_walk_kernel(const WalkArgs
 #pragma unroll
         for (int x = 0; x < PA; ++x) ldmatrix_x4_trans(af[x], k_s + (x * W + ks * 16) * ST + at_off + warp * 16);
         b.load(wv_s + ks * 16 * CST + b_off, W * CST);
-        walk_product<NT, PA, PB>(sum, af, b);
+        walk_product<NT, PA, PB>(sum, SPLIT_SUMS ? sum_low : sum, af, b);
       }
       const float whole = steps[2 * W];
 #pragma unroll
       for (int i = 0; i < NT; ++i)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) S[i][e] = fmaf(whole, S[i][e], sum[i][e]);
+        for (int e = 0; e < 4; ++e) S[i][e] = fmaf(whole, S[i][e], SPLIT_SUMS ? sum[i][e] + sum_low[i][e] : sum[i][e]);
     }
     __syncthreads();               // the state's, the values' and the piece's reads are done
     store_state();
