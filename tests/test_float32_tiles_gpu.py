@@ -57,3 +57,32 @@ def test_attention_refuses_what_it_does_not_take(ops):
     assert ops.paged_attention_f32_supported(64, 1, 128, torch.float32)
     for nh, nkv, hd, dtype in ((65, 1, 64, torch.float32), (4, 2, 132, torch.float32), (4, 2, 30, torch.float32), (4, 2, 64, torch.bfloat16)):
         assert not ops.paged_attention_f32_supported(nh, nkv, hd, dtype)
+
+
+@pytest.mark.parametrize("nh,nkv,hd,window,chunk", [(4, 2, 64, 0, 0), (3, 1, 128, 40, 0), (2, 2, 20, 0, 50)])
+def test_values_that_are_not_finite_stay_with_the_tokens_that_see_them(ops, cuda_device, nh, nkv, hd, window, chunk):
+    """An infinity and a NaN among the values of one position: every query that does not see it keeps its bits."""
+    n, ctx, page = 150, 30, 16
+    q, cache, meta, *_ = build_paged_case(cuda_device, torch.float32, nh, nkv, hd, page, [n], [ctx], 7)
+    status, wide = ops.new_status(cuda_device), ops.paged_prefill_tile_tokens()
+
+    def run(held):
+        out = torch.empty_like(q)
+        ops.paged_attention_f32(q, held, meta["table"], *tiles_for([n], wide, cuda_device), wide, meta["row_q_start"], meta["row_q_len"],
+                                meta["row_ctx"], nh, nkv, hd, window, 1 / math.sqrt(hd), status, out, chunk=chunk)
+        ops.check_status(status)
+        return out
+
+    clean = run(cache)
+    for at in (17, 63, 64, 100, ctx + n - 1):
+        held = cache.clone()
+        held[meta["table"][0, at // page], 1, :, at % page, 0::2] = math.inf
+        held[meta["table"][0, at // page], 1, :, at % page, 1::2] = math.nan
+        got, position = run(held), torch.arange(ctx, ctx + n, device=cuda_device)
+        sees = position >= at
+        if window:
+            sees &= position - at < window
+        if chunk:
+            sees &= position // chunk == at // chunk
+        assert torch.equal(got[~sees], clean[~sees]), at
+        assert not torch.isfinite(got[sees]).any()

@@ -219,6 +219,7 @@ __global__ void __launch_bounds__(F_THREADS, 2) paged_attention_f32_kernel(const
         const float4 v = *reinterpret_cast<const float4*>(v_s + j * D + c * 64 + tx * 4);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
+          if (p4[i] == 0.0f) continue;        // a key that the row does not see: its value may be anything
           acc[i][4 * c] = fmaf(p4[i], v.x, acc[i][4 * c]);
           acc[i][4 * c + 1] = fmaf(p4[i], v.y, acc[i][4 * c + 1]);
           acc[i][4 * c + 2] = fmaf(p4[i], v.z, acc[i][4 * c + 2]);
