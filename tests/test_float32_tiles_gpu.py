@@ -86,3 +86,16 @@ def test_values_that_are_not_finite_stay_with_the_tokens_that_see_them(ops, cuda
             sees &= position // chunk == at // chunk
         assert torch.equal(got[~sees], clean[~sees]), at
         assert not torch.isfinite(got[sees]).any()
+
+
+@pytest.mark.parametrize("M,N,K,apart", [(70, 311, 200, 3), (70, 311, 203, 0), (5, 33, 64, 2), (1300, 515, 68, 1), (33, 40, 16, 4)])
+def test_a_rows_sums_do_not_depend_on_the_batch(ops, cuda_device, M, N, K, apart):
+    """Rows that lie apart by any stride, alone and in a batch, and the outputs of one row of w alone: the same bits."""
+    wide, w = rand((M, K + apart), torch.float32, cuda_device, 3), rand((N, K + apart), torch.float32, cuda_device, 4)
+    x, w = wide[:, :K], w[:, :K]
+    got = ops.gemm_nt_simt(x, w)
+    assert (got.double() - x.double() @ w.double().T).abs().max() <= 6 * 2.0 ** -24 * K
+    for i in (0, 1, M // 2, M - 1):
+        assert torch.equal(ops.gemm_nt_simt(x[i:i + 1], w), got[i:i + 1])
+    for j in (0, N - 1):
+        assert torch.equal(ops.gemm_nt_simt(x, w[j:j + 1]), got[:, j:j + 1])

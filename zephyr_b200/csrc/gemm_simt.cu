@@ -2,8 +2,8 @@
 // the true 32-bit path.  No tensor cores, hence no TF32 or other reduced-precision mode: the
 // reference's "float32" linear layers run in TF32 (deps/ttl/src/ops/matmul.cpp:269-271), which is
 // exactly what this path exists to avoid.  The order in which an output's K products are summed does
-// not depend on M, N or the tile it is made in, so a row's result does not depend on the batch around
-// it.  Inputs may be float32 or bfloat16 (read exactly); the output is float32 or the input type.
+// not depend on M, N or the tile it is made in (rows that start on 16-byte boundaries are summed in four
+// chains, others in one, by the strides alone), so a row's result does not depend on the batch around it.  Inputs may be float32 or bfloat16 (read exactly); the output is float32 or the input type.
 #include "common.cuh"
 
 namespace zb {
@@ -229,7 +229,7 @@ ZB_API int zb_gemm_nt_simt(void* y, const void* x, const void* w, int M, int N, 
   if (M == 0 || N == 0) return OK;
   auto s = static_cast<cudaStream_t>(stream);
   if (in_dtype == DTYPE_F32 && out_dtype == DTYPE_F32) {
-    const bool vectors = K % 4 == 0 && (M == 1 || ldx % 4 == 0) && (N == 1 || ldw % 4 == 0) && reinterpret_cast<uintptr_t>(x) % 16 == 0 &&
+    const bool vectors = K % 4 == 0 && ldx % 4 == 0 && ldw % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 &&
                          reinterpret_cast<uintptr_t>(w) % 16 == 0;
     auto yf = static_cast<float*>(y);
     auto xf = static_cast<const float*>(x), wf = static_cast<const float*>(w);
