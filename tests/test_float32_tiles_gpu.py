@@ -99,3 +99,34 @@ def test_a_rows_sums_do_not_depend_on_the_batch(ops, cuda_device, M, N, K, apart
         assert torch.equal(ops.gemm_nt_simt(x[i:i + 1], w), got[i:i + 1])
     for j in (0, N - 1):
         assert torch.equal(ops.gemm_nt_simt(x, w[j:j + 1]), got[:, j:j + 1])
+
+
+def test_float32_logits_do_not_depend_on_what_shares_the_step(model_folders, cuda_device):
+    """Prompts of 40, 17 and 3 tokens and single tokens behind some of them, in steps of their own and in one step with
+    many others: the same bits."""
+    from replay_util import random_tokens
+    from tiny_configs import TINY
+    from zephyr_b200.config import load_model_spec
+    from zephyr_b200.engine import ModelRunner, StepEntry
+    from zephyr_b200.parts import Model
+    from zephyr_b200.weights import Checkpoint
+
+    folder = model_folders("D", "float32")
+    model = Model.load(load_model_spec(folder), Checkpoint(folder), torch.float32, cuda_device)
+    lengths = [40, 1, 17, 3] + [1] * 12
+    tokens = [random_tokens(TINY["D"]["config"]["vocab_size"], 2 * n, seed=i) for i, n in enumerate(lengths)]
+
+    def logits(groups):
+        runner, out = ModelRunner(model, TINY["D"]["page_size"], 64, len(lengths), use_cuda_graphs=False), {}
+        for r in range(len(lengths)):
+            assert runner.add_request(r)
+        for half in (0, 1):
+            for group in groups:
+                got = runner.step([StepEntry(r, tokens[r][half * lengths[r]:(half + 1) * lengths[r]], (lengths[r] - 1,)) for r in group])
+                out.update({(r, half): got[i].clone() for i, r in enumerate(group)})
+        runner.check()
+        return out
+
+    alone, together = logits([[r] for r in range(len(lengths))]), logits([list(range(len(lengths)))])
+    for key in alone:
+        assert torch.equal(alone[key], together[key]), key

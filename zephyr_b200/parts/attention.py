@@ -66,10 +66,6 @@ from .base import POSITION_ENCODINGS, Mixer, StepContext, lookup, register_mixer
 class Attention(Mixer):
     graph_safe = True
 
-    # New tokens per request, on average, from which on a float32 step's rows with several tokens run in tiles of 64
-    # query rows: below, most of a tile would be empty (see csrc/attention_f32.cu).
-    FLOAT32_TILES_FROM = 16
-
     def __init__(self, spec: MixerSpec, weights: Mapping[str, torch.Tensor], dtype: torch.dtype,
                  device: torch.device | str):
         p = spec.params
@@ -339,8 +335,9 @@ class Attention(Mixer):
 
     def attend(self, q: torch.Tensor, ctx: StepContext, call: LayerCall) -> torch.Tensor:
         """Rows with one new token go to the split-context decode kernel, rows with several to the
-        tensor-core prompt kernel, where those kernels take this shape and type; whatever is left
-        goes to the general kernel."""
+        tensor-core prompt kernel, where those kernels take this shape and type, or in 32 bits to the
+        tiled kernel; whatever is left goes to the general kernel.  A row's kernel hangs on that row
+        alone."""
         cache = ctx.caches[call.cache]
         table = ctx.block_table(call.cache)
         if self.general and self.heads_tile_tokens > 0:
@@ -367,7 +364,7 @@ class Attention(Mixer):
                                   *common, out=out, **masks)
         if decode_done and prefill_done:
             return out
-        if self.float32_tiles and q.shape[0] >= self.FLOAT32_TILES_FROM * ctx.num_rows:
+        if self.float32_tiles:
             tile_row, tile_q0 = ctx.tiles[(self.prefill_tile_tokens, "multi")]
             prefill_done = True
             if tile_row.numel() > 0:
