@@ -324,3 +324,43 @@ def test_the_state_space_walk_keeps_float32(cuda_device, dim, vdim):
 
     for walk, scan in zip(error(None), error(0)):
         assert walk <= 1.15 * scan, (walk, scan)
+
+
+@pytest.mark.parametrize("kind", ["delta"])
+def test_what_a_row_gets_hangs_on_that_row_alone(cuda_device, kind):
+    """Portions of many sizes in one step, and each in a step of its own: the same bits, whether the host knows the rows'
+    sizes or not."""
+    from zephyr_b200.kernels import ops
+
+    heads, per, dim, vdim = 4, 2, 64, 48
+    lengths = [1, 100, 1, 1, 15, 16, 1, 300, 1, 1, 63, 64, 1, 1, 31, 32, 2, 1, 1, 1]
+    starts, T, groups = [sum(lengths[:i]) for i in range(len(lengths))], sum(lengths), heads // per
+    g = torch.Generator().manual_seed(3)
+    dtype = torch.bfloat16 if kind == "state_space" else torch.float32
+    q, k, v, b, a = (torch.randn(T, n, generator=g).to(cuda_device) for n in (groups * dim, groups * dim, heads * vdim, heads, heads))
+    q, k, v, dt = (t.to(dtype) for t in (q, k, v, a))
+    constants = [(torch.rand(heads, generator=g) - 0.5).to(cuda_device) for _ in range(3)]
+    before = torch.randn(len(lengths), heads * dim * vdim, generator=g).to(cuda_device)
+    i32 = lambda values: torch.tensor(values, dtype=torch.int32, device=cuda_device)
+    status = ops.new_status(cuda_device)
+
+    def run(rows, **more):
+        first, end = starts[rows[0]], starts[rows[-1]] + lengths[rows[-1]]
+        part, state = slice(first, end), before.clone()
+        where = (state, i32(rows), i32([starts[r] - first for r in rows]), i32([lengths[r] for r in rows]), status)
+        if kind == "delta":
+            out = ops.delta_rule(q[part], k[part], v[part], b[part], a[part], constants[0], constants[1], heads, groups, dim, vdim, *where,
+                                 q_scale=dim ** -0.5, **more)
+        else:
+            out = ops.decayed_state_scan("state_space", q[part], k[part], v[part], heads, dim, vdim, *where, dt=dt[part],
+                                         dt_bias=constants[0], a_log=constants[1], skip=constants[2], heads_per_group=per, **more)
+        ops.check_status(status)
+        return out, state
+
+    together = [run(list(range(len(lengths))), **more) for more in ({}, {"row_tokens": lengths})]
+    for out, state in together[1:]:
+        assert torch.equal(out, together[0][0]) and torch.equal(state, together[0][1])
+    for r, (start, n) in enumerate(zip(starts, lengths)):
+        out, state = run([r])
+        assert torch.equal(together[0][0][start:start + n], out), n
+        assert torch.equal(together[0][1][r], state[r]), n

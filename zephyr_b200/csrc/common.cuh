@@ -118,22 +118,25 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
-// Rows (requests) cut into pieces of SIZE tokens that are numbered row by row, whatever the order in which the rows' tokens
-// lie in the stream: a row's pieces begin behind those of all rows with a smaller number, so no two pieces share a number
-// and all are below tokens / SIZE + rows.  A whole warp calls; every lane gets the result.
+// Rows (requests) of `from` tokens and more cut into pieces of SIZE tokens that are numbered row by row, whatever the order in
+// which the rows' tokens lie in the stream: a row's pieces begin behind those of all such rows with a smaller number, so no
+// two pieces share a number and all are below tokens / SIZE + rows.  A whole warp calls; every lane gets the result.
 template <int SIZE>
-__device__ __forceinline__ int first_piece_of_row(const int* row_q_len, int row) {
+__device__ __forceinline__ int first_piece_of_row(const int* row_q_len, int row, int from) {
   int pieces = 0;
-  for (int r = threadIdx.x & 31; r < row; r += 32) pieces += (row_q_len[r] + SIZE - 1) / SIZE;
+  for (int r = threadIdx.x & 31; r < row; r += 32) {
+    const int n = row_q_len[r];
+    if (n >= from) pieces += (n + SIZE - 1) / SIZE;
+  }
   return __reduce_add_sync(0xffffffffu, pieces);
 }
 // The row that piece `piece` belongs to (-1: none) and, in `own`, its number within the row.
 template <int SIZE>
-__device__ __forceinline__ int row_of_piece(const int* row_q_len, int rows, int piece, int& own) {
+__device__ __forceinline__ int row_of_piece(const int* row_q_len, int rows, int from, int piece, int& own) {
   const int lane = threadIdx.x & 31;
   int passed = 0;
   for (int r0 = 0; r0 < rows; r0 += 32) {
-    const int count = r0 + lane < rows ? (row_q_len[r0 + lane] + SIZE - 1) / SIZE : 0;
+    const int n = r0 + lane < rows ? row_q_len[r0 + lane] : 0, count = n >= from ? (n + SIZE - 1) / SIZE : 0;
     int end = count;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {

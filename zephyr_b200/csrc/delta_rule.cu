@@ -17,8 +17,8 @@
 //                 written back at its end, so a prompt may be cut anywhere.  In the slot a head's state
 //                 lies [V][D] (a column's channels together).
 //
-// Where requests bring runs of tokens, two other kernels take their place (delta_blocks, delta_block_scan below): the
-// same rule, block by block of 16 tokens.
+// Rows that bring runs of tokens go to two other kernels (delta_blocks, delta_block_scan below): the same rule, block by
+// block of 16 tokens.
 //
 // Everything here is float32 multiply-adds in either form; the values v are read in the model's type.
 #include "common.cuh"
@@ -43,12 +43,23 @@ struct DeltaGatesArgs {
   const float* dt_bias;    // [heads]
   int qk_heads, heads, D;
   float q_scale, unit_eps;
+  const int* row_q_start;  // below > 0: only the tokens of rows with fewer than `below` tokens
+  const int* row_q_len;
+  int rows, below;
 };
 
 template <typename T>
 __global__ void __launch_bounds__(128) delta_gates_kernel(const DeltaGatesArgs a) {
   const long long t = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (a.below > 0) {
+    bool wanted = false;
+    for (int r = threadIdx.x; r < a.rows; r += blockDim.x) {
+      const int n = a.row_q_len[r];
+      wanted |= n < a.below && t >= a.row_q_start[r] && t < a.row_q_start[r] + n;
+    }
+    if (!__syncthreads_or(wanted)) return;
+  }
   for (int h = warp; h < 2 * a.qk_heads; h += 4) {
     const bool is_q = h < a.qk_heads;
     const int own = is_q ? h : h - a.qk_heads;
@@ -87,6 +98,7 @@ struct DeltaScanArgs {
   const int* row_q_start;
   const int* row_q_len;
   int heads, heads_per_group, D, V, num_slots, write_state;
+  int below;               // > 0: only rows with fewer than this many tokens
   int* status;
 };
 
@@ -119,6 +131,7 @@ __global__ void __launch_bounds__(DS_THREADS) delta_scan_kernel(const DeltaScanA
     return;
   }
   const int t0 = a.row_q_start[row], n = a.row_q_len[row];
+  if (a.below > 0 && n >= a.below) return;
   const int l = threadIdx.x % L, my_group = threadIdx.x / L;
   const int group = head / a.heads_per_group, qk_heads = a.heads / a.heads_per_group;
   // A thread's CPT columns are separate chains: one column's exchanges and writes run under the other's sums.
@@ -336,7 +349,7 @@ struct DeltaBlocksArgs {
   const float* b; const float* a; long long ba_stride;
   const float* a_log; const float* dt_bias;
   const int* row_q_start; const int* row_q_len;
-  int rows, qk_heads, heads, D;
+  int rows, from, qk_heads, heads, D;      // rows of `from` tokens and more
   float q_scale, unit_eps;
 };
 
@@ -358,7 +371,7 @@ __global__ void __launch_bounds__(DB_THREADS) delta_blocks_kernel(const DeltaBlo
   float* beta_s = tail_s + DB;
   const int block = blockIdx.x, group = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int own;
-  const int row = row_of_piece<DB>(a.row_q_len, a.rows, block, own);
+  const int row = row_of_piece<DB>(a.row_q_len, a.rows, a.from, block, own);
   if (row < 0) return;
   const int begin = own * DB, n = min(DB, a.row_q_len[row] - begin);
   const long long t0 = a.row_q_start[row] + begin;
@@ -488,7 +501,7 @@ struct DeltaBlockScanArgs {
   const void* v; long long v_stride;
   float* state; long long slot_stride;     // slot s at state + s * slot_stride: [heads][V][D]
   const int* slots; const int* row_q_start; const int* row_q_len;
-  int heads, qk_heads, D, V, num_slots, write_state;
+  int from, heads, qk_heads, D, V, num_slots, write_state;
   int* status;
 };
 
@@ -520,8 +533,9 @@ __global__ void __launch_bounds__(DB_THREADS, 2) delta_block_scan_kernel(const D
     return;
   }
   const int n = a.row_q_len[row], blocks = (n + DB - 1) / DB;
+  if (n < a.from) return;
   const long long t0 = a.row_q_start[row];
-  const int first = first_piece_of_row<DB>(a.row_q_len, row);
+  const int first = first_piece_of_row<DB>(a.row_q_len, row, a.from);
   const int group = head / (a.heads / a.qk_heads);
 
   auto copy_block = [&](int p, float* stage) {
@@ -681,16 +695,20 @@ using namespace zb;
 
 ZB_API int zb_delta_max_channels() { return 512; }
 
+// `below` > 0: only the tokens of rows with fewer than `below` tokens (here and in zb_delta_scan; zb_delta_block_scan takes the
+// others).
 ZB_API int zb_delta_gates(float* q_out, float* k_out, float* beta, float* decay, const void* q, long long q_stride,
                           const void* k, long long k_stride, const float* b, const float* a, long long ba_stride,
                           const float* a_log, const float* dt_bias, int tokens, int qk_heads, int heads, int D,
-                          float q_scale, float unit_eps, int dtype, void* stream) {
-  if (tokens < 0 || qk_heads <= 0 || heads <= 0 || D <= 0) return ERR_BAD_ARGUMENT;
+                          float q_scale, float unit_eps, const int* row_q_start, const int* row_q_len, int rows, int below, int dtype,
+                          void* stream) {
+  if (rows < 0 || tokens < 0 || qk_heads <= 0 || heads <= 0 || D <= 0) return ERR_BAD_ARGUMENT;
   if (tokens == 0) return OK;
   DeltaGatesArgs g;
   g.q_out = q_out; g.k_out = k_out; g.beta = beta; g.decay = decay; g.q = q; g.k = k; g.q_stride = q_stride;
   g.k_stride = k_stride; g.b = b; g.a = a; g.ba_stride = ba_stride; g.a_log = a_log; g.dt_bias = dt_bias;
   g.qk_heads = qk_heads; g.heads = heads; g.D = D; g.q_scale = q_scale; g.unit_eps = unit_eps;
+  g.row_q_start = row_q_start; g.row_q_len = row_q_len; g.rows = rows; g.below = below;
   auto s = static_cast<cudaStream_t>(stream);
   if (dtype == DTYPE_F32) delta_gates_kernel<float><<<tokens, 128, 0, s>>>(g);
   else delta_gates_kernel<__nv_bfloat16><<<tokens, 128, 0, s>>>(g);
@@ -735,7 +753,7 @@ static int delta_scan_dispatch(const DeltaScanArgs& a, int rows, int tokens, cud
 ZB_API int zb_delta_scan(float* out, const float* q, const float* k, const void* v, long long v_stride,
                          const float* beta, const float* decay, float* state, long long slot_stride, const int* slots,
                          const int* row_q_start, const int* row_q_len, int rows, int tokens, int heads,
-                         int heads_per_group, int D, int V, int num_slots, int write_state, int dtype, int* status,
+                         int heads_per_group, int D, int V, int num_slots, int write_state, int below, int dtype, int* status,
                          void* stream) {
   if (rows < 0 || heads <= 0 || heads_per_group <= 0 || heads % heads_per_group != 0 || D <= 0 || V <= 0)
     return ERR_BAD_ARGUMENT;
@@ -745,7 +763,7 @@ ZB_API int zb_delta_scan(float* out, const float* q, const float* k, const void*
   a.out = out; a.q = q; a.k = k; a.v = v; a.v_stride = v_stride; a.beta = beta; a.decay = decay; a.state = state;
   a.slot_stride = slot_stride; a.slots = slots; a.row_q_start = row_q_start; a.row_q_len = row_q_len;
   a.heads = heads; a.heads_per_group = heads_per_group; a.D = D; a.V = V; a.num_slots = num_slots;
-  a.write_state = write_state; a.status = status;
+  a.write_state = write_state; a.below = below; a.status = status;
   auto s = static_cast<cudaStream_t>(stream);
   return dtype == DTYPE_F32 ? delta_scan_dispatch<float>(a, rows, tokens, s)
                             : delta_scan_dispatch<__nv_bfloat16>(a, rows, tokens, s);
@@ -767,13 +785,13 @@ static int delta_block_launch(const DeltaBlocksArgs& b, const DeltaBlockScanArgs
   return launch_result();
 }
 
-// The rule over runs of tokens, block by block.  `ws`: (tokens / block tokens + rows) * zb_delta_block_floats floats,
+// The rule over rows of `from` tokens and more, block by block.  `ws`: (tokens / block tokens + rows) * zb_delta_block_floats floats,
 // 16-byte aligned, contents irrelevant.  The rows' tokens may lie in the stream in any order.
 ZB_API int zb_delta_block_scan(float* out, const void* q, long long q_stride, const void* k, long long k_stride, const void* v,
                                long long v_stride, const float* b, const float* a, long long ba_stride, const float* a_log,
                                const float* dt_bias, float* state, long long slot_stride, const int* slots, const int* row_q_start,
-                               const int* row_q_len, int rows, int tokens, int qk_heads, int heads, int D, int V, int num_slots,
-                               int write_state, float q_scale, float unit_eps, float* ws, int dtype, int* status, void* stream) {
+                               const int* row_q_len, int rows, int tokens, int from, int qk_heads, int heads, int D, int V,
+                               int num_slots, int write_state, float q_scale, float unit_eps, float* ws, int dtype, int* status, void* stream) {
   if (rows < 0 || tokens < 0 || qk_heads <= 0 || heads <= 0 || heads % qk_heads != 0 || D <= 0 || V <= 0 || num_slots <= 0)
     return ERR_BAD_ARGUMENT;
   if (D > zb_delta_block_max_channels() || heads > 65535 || (V + DB_COLS - 1) / DB_COLS > 65535) return ERR_UNSUPPORTED;
@@ -783,12 +801,12 @@ ZB_API int zb_delta_block_scan(float* out, const void* q, long long q_stride, co
   DeltaBlocksArgs g;
   g.qk = ws; g.coef = ws + static_cast<long long>(blocks) * qk_heads * dp * 2 * DB; g.q = q; g.q_stride = q_stride; g.k = k;
   g.k_stride = k_stride; g.b = b; g.a = a; g.ba_stride = ba_stride; g.a_log = a_log; g.dt_bias = dt_bias;
-  g.row_q_start = row_q_start; g.row_q_len = row_q_len; g.rows = rows; g.qk_heads = qk_heads; g.heads = heads; g.D = D;
+  g.row_q_start = row_q_start; g.row_q_len = row_q_len; g.rows = rows; g.from = from; g.qk_heads = qk_heads; g.heads = heads; g.D = D;
   g.q_scale = q_scale; g.unit_eps = unit_eps;
   DeltaBlockScanArgs c;
   c.out = out; c.qk = g.qk; c.coef = g.coef; c.v = v; c.v_stride = v_stride; c.state = state; c.slot_stride = slot_stride;
   c.slots = slots; c.row_q_start = row_q_start; c.row_q_len = row_q_len; c.heads = heads; c.qk_heads = qk_heads; c.D = D; c.V = V;
-  c.num_slots = num_slots; c.write_state = write_state; c.status = status;
+  c.num_slots = num_slots; c.write_state = write_state; c.from = from; c.status = status;
   auto s = static_cast<cudaStream_t>(stream);
   if (dtype == DTYPE_F32) return dp == 64 ? delta_block_launch<float, 64>(g, c, rows, blocks, s) : delta_block_launch<float, 128>(g, c, rows, blocks, s);
   return dp == 64 ? delta_block_launch<__nv_bfloat16, 64>(g, c, rows, blocks, s) : delta_block_launch<__nv_bfloat16, 128>(g, c, rows, blocks, s);

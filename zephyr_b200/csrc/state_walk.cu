@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(W_THREADS) walk_prepare_kernel(const WalkArgs 
   const int qk_head = blockIdx.y / runs, first_head = blockIdx.y % runs * HEADS, qk_heads = a.H / a.heads_per_group;
   const int heads = min(HEADS, a.heads_per_group - first_head), h0 = qk_head * a.heads_per_group + first_head;
   int own;
-  const int row = row_of_piece<W>(a.row_q_len, a.rows, piece, own);
+  const int row = row_of_piece<W>(a.row_q_len, a.rows, 0, piece, own);
   if (row < 0) return;
   const int begin = own * W, n = min(W, a.row_q_len[row] - begin);
   const long long t0 = a.row_q_start[row] + begin;
@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(W_THREADS, 2) state_walk_kernel(const WalkArgs
   }
   const int n_all = a.row_q_len[row], pieces = (n_all + W - 1) / W;
   const long long t0 = a.row_q_start[row];
-  const int first = first_piece_of_row<W>(a.row_q_len, row), qk_head = h / a.heads_per_group, qk_heads = a.H / a.heads_per_group;
+  const int first = first_piece_of_row<W>(a.row_q_len, row, 0), qk_head = h / a.heads_per_group, qk_heads = a.H / a.heads_per_group;
   if (tid == 0) {
 #pragma unroll
     for (int i = 0; i < STAGES; ++i) mbar_init(&landed[i], 1);

@@ -119,17 +119,17 @@ _SIGNATURES = {
     "zb_sigmoid_gate": [c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_void_p],
     "zb_delta_max_channels": [],
     "zb_delta_gates": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p,
-                       c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_int,
-                       c_void_p],
+                       c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p,
+                       c_void_p, c_int, c_int, c_int, c_void_p],
     "zb_delta_scan": [c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_longlong,
                       c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
-                      c_void_p, c_void_p],
+                      c_int, c_void_p, c_void_p],
     "zb_delta_block_max_channels": [],
     "zb_delta_block_tokens": [],
     "zb_delta_block_floats": [c_int, c_int, c_int],
     "zb_delta_block_scan": [c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p,
                             c_longlong, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
-                            c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p, c_int, c_void_p, c_void_p],
+                            c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p, c_int, c_void_p, c_void_p],
     "zb_residual_rms_norm": [c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_int, c_float, c_float, c_int,
                              c_int, c_int, c_void_p],
     "zb_route_biased": [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
@@ -1297,20 +1297,33 @@ def delta_max_channels() -> int:
     return library().zb_delta_max_channels()
 
 
-DELTA_BLOCKS_FROM = 16       # new tokens per request, on average, from which on the delta rule runs block by block
+DELTA_BLOCKS_FROM = 16       # new tokens of a row from which on the delta rule runs block by block
+
+
+def _two_forms(tokens: int, rows: int, limit: int, row_tokens: Sequence[int] | None) -> tuple[bool, bool]:
+    """Whether a step may have rows of fewer than ``limit`` tokens, and rows of ``limit`` and more; ``row_tokens`` are the
+    rows' tokens where the host knows them."""
+    if row_tokens is None and rows == 1:
+        row_tokens = [tokens]
+    if row_tokens is None:
+        return True, tokens >= limit
+    return any(0 < n < limit for n in row_tokens), any(n >= limit for n in row_tokens)
 
 
 def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b: torch.Tensor, a: torch.Tensor,
                a_log: torch.Tensor, dt_bias: torch.Tensor, heads: int, qk_heads: int, key_dim: int, value_dim: int,
                state: torch.Tensor, slots: torch.Tensor, row_q_start: torch.Tensor, row_q_len: torch.Tensor,
-               status: torch.Tensor, q_scale: float, unit_eps: float = 1e-6, write_state: bool = True) -> torch.Tensor:
+               status: torch.Tensor, q_scale: float, unit_eps: float = 1e-6, write_state: bool = True,
+               row_tokens: Sequence[int] | None = None) -> torch.Tensor:
     """The gated delta rule per head over each row's new tokens, from and to ``state`` [slots, heads *
     value_dim * key_dim] float32 (rows may be strided; a head's state lies [value_dim][key_dim]):
     S <- g S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q.  q and k [T, qk_heads * key_dim] (head h uses
     q/k head h // (heads / qk_heads)) are made unit vectors, x / sqrt(sum(x^2) + unit_eps), q times
     ``q_scale``; v [T, heads * value_dim]; beta = sigmoid(b), g = exp(-exp(a_log) softplus(a + dt_bias)) from
-    float32 b and a [T, heads].  q, k, v share a type and may be strided slices.  Returns o float32
-    [T, heads * value_dim]."""
+    float32 b and a [T, heads].  q, k, v share a type and may be strided slices.  Rows of ``DELTA_BLOCKS_FROM`` tokens and more
+    run block by block (up to 128 key channels), the others token by token: what a row gets hangs on that row alone.
+    ``row_tokens``: ``row_q_len`` on the host, where the caller has it, so that a form that no row takes is not launched.
+    Returns o float32 [T, heads * value_dim]."""
     _cuda(q, k, v, b, a, a_log, dt_bias, state, slots, row_q_start, row_q_len, status)
     _i32(slots, row_q_start, row_q_len)
     T = v.shape[0]
@@ -1327,26 +1340,30 @@ def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b: torch.Tenso
              and state.shape[1] == heads * key_dim * value_dim, "state must be float32 [slots, heads * value_dim * key_dim]")
     dev, lib, rows = v.device, library(), slots.numel()
     out = torch.empty((T, heads * value_dim), dtype=torch.float32, device=dev)
-    if T >= DELTA_BLOCKS_FROM * rows and key_dim <= lib.zb_delta_block_max_channels():
+    limit = DELTA_BLOCKS_FROM if key_dim <= lib.zb_delta_block_max_channels() else T + 1
+    short, long = _two_forms(T, rows, limit, row_tokens)
+    if long:
         ws = torch.empty(((T // lib.zb_delta_block_tokens() + rows) * lib.zb_delta_block_floats(qk_heads, heads, key_dim),),
                          dtype=torch.float32, device=dev)
         _check(lib.zb_delta_block_scan(
             _ptr(out), _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(b), _ptr(a), b.stride(0), _ptr(a_log),
-            _ptr(dt_bias), _ptr(state), state.stride(0), _ptr(slots), _ptr(row_q_start), _ptr(row_q_len), rows, T, qk_heads, heads,
-            key_dim, value_dim, state.shape[0], int(write_state), float(q_scale), float(unit_eps), _ptr(ws), DTYPE_CODE[v.dtype],
-            _ptr(status), _stream()), "delta_block_scan", kernels=2)
-        return out
-    qn = torch.empty((T, qk_heads * key_dim), dtype=torch.float32, device=dev)
-    kn = torch.empty_like(qn)
-    beta = torch.empty((T, heads), dtype=torch.float32, device=dev)
-    decay = torch.empty_like(beta)
-    _check(library().zb_delta_gates(_ptr(qn), _ptr(kn), _ptr(beta), _ptr(decay), _ptr(q), q.stride(0), _ptr(k), k.stride(0),
-                                    _ptr(b), _ptr(a), b.stride(0), _ptr(a_log), _ptr(dt_bias), T, qk_heads, heads, key_dim,
-                                    float(q_scale), float(unit_eps), DTYPE_CODE[v.dtype], _stream()), "delta_gates")
-    _check(library().zb_delta_scan(_ptr(out), _ptr(qn), _ptr(kn), _ptr(v), v.stride(0), _ptr(beta), _ptr(decay), _ptr(state),
-                                   state.stride(0), _ptr(slots), _ptr(row_q_start), _ptr(row_q_len), slots.numel(), T, heads,
-                                   heads // qk_heads, key_dim, value_dim, state.shape[0], int(write_state),
-                                   DTYPE_CODE[v.dtype], _ptr(status), _stream()), "delta_scan")
+            _ptr(dt_bias), _ptr(state), state.stride(0), _ptr(slots), _ptr(row_q_start), _ptr(row_q_len), rows, T, limit, qk_heads,
+            heads, key_dim, value_dim, state.shape[0], int(write_state), float(q_scale), float(unit_eps), _ptr(ws),
+            DTYPE_CODE[v.dtype], _ptr(status), _stream()), "delta_block_scan", kernels=2)
+    if short:
+        qn = torch.empty((T, qk_heads * key_dim), dtype=torch.float32, device=dev)
+        kn = torch.empty_like(qn)
+        beta = torch.empty((T, heads), dtype=torch.float32, device=dev)
+        decay = torch.empty_like(beta)
+        below = limit if long else 0
+        _check(lib.zb_delta_gates(_ptr(qn), _ptr(kn), _ptr(beta), _ptr(decay), _ptr(q), q.stride(0), _ptr(k), k.stride(0),
+                                  _ptr(b), _ptr(a), b.stride(0), _ptr(a_log), _ptr(dt_bias), T, qk_heads, heads, key_dim,
+                                  float(q_scale), float(unit_eps), _ptr(row_q_start), _ptr(row_q_len), rows, below,
+                                  DTYPE_CODE[v.dtype], _stream()), "delta_gates")
+        _check(lib.zb_delta_scan(_ptr(out), _ptr(qn), _ptr(kn), _ptr(v), v.stride(0), _ptr(beta), _ptr(decay), _ptr(state),
+                                 state.stride(0), _ptr(slots), _ptr(row_q_start), _ptr(row_q_len), rows, T, heads,
+                                 heads // qk_heads, key_dim, value_dim, state.shape[0], int(write_state), below,
+                                 DTYPE_CODE[v.dtype], _ptr(status), _stream()), "delta_scan")
     return out
 
 

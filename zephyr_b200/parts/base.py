@@ -68,7 +68,8 @@ class Part:
     # True if ``forward`` only launches work whose shapes depend on the step's sizes, and reads the
     # step's values (positions, tables, slots) on the device.  Steps of a model whose parts are all
     # graph-safe may be captured once and replayed.  A part that plans with host values of the
-    # step (``StepContext.host_*``) must leave this False.
+    # step (``StepContext.host_*``) must leave this False; ``host_q_len`` is one of the sizes (every graph
+    # belongs to steps whose rows bring the same numbers of tokens).
     graph_safe = False
 
     @staticmethod

@@ -271,7 +271,8 @@ class GatedDeltaRule(Mixer):
         o = ops.delta_rule(mixed[:, c[0]:c[1]], mixed[:, c[1]:c[2]], mixed[:, c[2]:c[3]], steps[:, :self.heads],
                            steps[:, self.heads:], self.a_log, self.dt_bias, self.heads, self.qk_heads, self.dim,
                            self.vdim, store[:, :self.scan_floats], ctx.state_slots, ctx.row_q_start, ctx.row_q_len,
-                           ctx.status, q_scale=self.dim ** -0.5, unit_eps=self.UNIT_EPS, write_state=call.writes_cache)
+                           ctx.status, q_scale=self.dim ** -0.5, unit_eps=self.UNIT_EPS, write_state=call.writes_cache,
+                           row_tokens=ctx.host_q_len or None)
         normed = ops.gated_group_rms_norm(o, ops.linear(x, self.w_g), self.norm, self.vdim, self.eps, gate_first=False)
         return ops.linear(normed, self.w_o, out_dtype=out_dtype)
 
