@@ -326,7 +326,7 @@ def test_the_state_space_walk_keeps_float32(cuda_device, dim, vdim):
         assert walk <= 1.15 * scan, (walk, scan)
 
 
-@pytest.mark.parametrize("kind", ["delta"])
+@pytest.mark.parametrize("kind", ["delta", "state_space"])
 def test_what_a_row_gets_hangs_on_that_row_alone(cuda_device, kind):
     """Portions of many sizes in one step, and each in a step of its own: the same bits, whether the host knows the rows'
     sizes or not."""

@@ -517,6 +517,7 @@ struct ScanArgs {
   float* out;                          // [tokens, H * V] float32
   const int* slots; const int* row_q_start; const int* row_q_len;
   int H, D, V, heads_per_group, num_slots, write_state;
+  int below;                           // > 0: only requests with fewer than this many new tokens
   float q_scale;
   // Long requests in segments that run side by side (seg_len 0: every request is one piece).  Segment g of
   // a request covers its new tokens g seg_len .. (g + 1) seg_len - 1.  A first pass runs every segment
@@ -582,6 +583,7 @@ __global__ void __launch_bounds__(512) decayed_state_scan_kernel(const ScanArgs 
     return;
   }
   int t0 = a.row_q_start[row], n = a.row_q_len[row];
+  if (a.below > 0 && n >= a.below) return;
   bool last = true;
   if (a.seg_len > 0) {
     const int begin = seg * a.seg_len;
@@ -1108,7 +1110,7 @@ ZB_API int zb_decayed_state_scan(float* out, const void* q, long long q_stride, 
                                  long long slot_stride,
                                  const int* slots, const int* row_q_start, const int* row_q_len, int rows, int tokens,
                                  int H, int D, int V, int heads_per_group, int num_slots, int write_state,
-                                 float q_scale, float inv_tau, int mode, int dtype, int seg_len, float* ws_state,
+                                 int below, float q_scale, float inv_tau, int mode, int dtype, int seg_len, float* ws_state,
                                  float* ws_decay, int* status, void* stream) {
   if (rows < 0 || tokens < 0 || H <= 0 || D <= 0 || V <= 0 || heads_per_group <= 0 || seg_len < 0 ||
       (seg_len > 0 && (ws_state == nullptr || ws_decay == nullptr)))
@@ -1129,7 +1131,7 @@ ZB_API int zb_decayed_state_scan(float* out, const void* q, long long q_stride, 
   a.a_log = a_log; a.skip = skip; a.w_dtype = w_dtype; a.state = state; a.slot_stride = slot_stride; a.out = out;
   a.slots = slots; a.row_q_start = row_q_start; a.row_q_len = row_q_len; a.H = H; a.D = D; a.V = V;
   a.heads_per_group = heads_per_group; a.num_slots = num_slots; a.write_state = write_state; a.q_scale = q_scale;
-  a.status = status;
+  a.below = below; a.status = status;
   a.seg_len = seg_len; a.segs = seg_len > 0 ? (tokens + seg_len - 1) / seg_len : 1;
   a.ws_state = ws_state; a.ws_decay = ws_decay;
   if (static_cast<long long>(rows) * a.segs > 65535) return ERR_UNSUPPORTED;

@@ -58,7 +58,7 @@ struct WalkArgs {
   float* out;                            // [tokens, H * V]
   float* state; long long slot_stride;   // slot s at state + s * slot_stride: [H][D][V]
   const int* slots; const int* row_q_start; const int* row_q_len;
-  int rows, H, D, V, heads_per_group, num_slots, write_state;
+  int rows, from, H, D, V, heads_per_group, num_slots, write_state;      // rows of `from` tokens and more
   const float* freqs; const int* positions;      // WALK_FIXED: null, or q and k are still to be turned (as rotate_qk does)
   int rot_dims;
   float k_scale;
@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(W_THREADS) walk_prepare_kernel(const WalkArgs 
   const int qk_head = blockIdx.y / runs, first_head = blockIdx.y % runs * HEADS, qk_heads = a.H / a.heads_per_group;
   const int heads = min(HEADS, a.heads_per_group - first_head), h0 = qk_head * a.heads_per_group + first_head;
   int own;
-  const int row = row_of_piece<W>(a.row_q_len, a.rows, 0, piece, own);
+  const int row = row_of_piece<W>(a.row_q_len, a.rows, a.from, piece, own);
   if (row < 0) return;
   const int begin = own * W, n = min(W, a.row_q_len[row] - begin);
   const long long t0 = a.row_q_start[row] + begin;
@@ -385,8 +385,9 @@ __global__ void __launch_bounds__(W_THREADS, 2) state_walk_kernel(const WalkArgs
     return;
   }
   const int n_all = a.row_q_len[row], pieces = (n_all + W - 1) / W;
+  if (n_all < a.from) return;
   const long long t0 = a.row_q_start[row];
-  const int first = first_piece_of_row<W>(a.row_q_len, row, 0), qk_head = h / a.heads_per_group, qk_heads = a.H / a.heads_per_group;
+  const int first = first_piece_of_row<W>(a.row_q_len, row, a.from), qk_head = h / a.heads_per_group, qk_heads = a.H / a.heads_per_group;
   if (tid == 0) {
 #pragma unroll
     for (int i = 0; i < STAGES; ++i) mbar_init(&landed[i], 1);
@@ -669,12 +670,12 @@ ZB_API int zb_walk_piece_floats(int mode, int H, int heads_per_group, int D) {
 // mode 0 (state space): q, k, v, dt bfloat16; q, k and their rows on 16-byte boundaries, D a multiple of 8.  mode 1 (fixed
 // decays): q, k, v float32; with `freqs` (rot_dims / 2 of them) q and k are turned by the tokens' positions first, as
 // zb_rotate_qk does, k times k_scale (rot_dims a multiple of 8, D of 4, rows on 16-byte boundaries).  Constants float32.
-// ws: (tokens / piece tokens + rows) * zb_walk_piece_floats floats, 16-byte aligned, contents irrelevant.  The rows' tokens
-// may lie in the stream in any order.
+// ws: (tokens / piece tokens + rows) * zb_walk_piece_floats floats, 16-byte aligned, contents irrelevant.  Rows of fewer than
+// `from` tokens are left alone; the rows' tokens may lie in the stream in any order.
 ZB_API int zb_state_walk(int mode, float* out, const void* q, long long q_stride, const void* k, long long k_stride, const void* v,
                          long long v_stride, const void* dt, long long dt_stride, const float* dt_bias, const float* a_log,
                          const float* skip, const float* decay, float* state, long long slot_stride, const int* slots,
-                         const int* row_q_start, const int* row_q_len, int rows, int tokens, int H, int D, int V,
+                         const int* row_q_start, const int* row_q_len, int rows, int tokens, int from, int H, int D, int V,
                          int heads_per_group, int num_slots, int write_state, const float* freqs, int rot_dims, float k_scale,
                          const int* positions, float* ws, int* status, void* stream) {
   if (rows < 0 || tokens < 0 || H <= 0 || D <= 0 || V <= 0 || heads_per_group <= 0 || H % heads_per_group != 0 || num_slots <= 0 ||
@@ -701,7 +702,7 @@ ZB_API int zb_state_walk(int mode, float* out, const void* q, long long q_stride
     return ERR_BAD_ARGUMENT;
   a.out = out; a.state = state; a.slot_stride = slot_stride; a.slots = slots; a.row_q_start = row_q_start; a.row_q_len = row_q_len;
   a.pairs = V % 2 == 0 && v_stride % 2 == 0 && reinterpret_cast<uintptr_t>(v) % (mode == WALK_SPACE ? 4 : 8) == 0;
-  a.rows = rows; a.H = H; a.D = D; a.V = V; a.heads_per_group = heads_per_group; a.num_slots = num_slots; a.write_state = write_state;
+  a.rows = rows; a.from = from; a.H = H; a.D = D; a.V = V; a.heads_per_group = heads_per_group; a.num_slots = num_slots; a.write_state = write_state;
   a.status = status;
   auto s = static_cast<cudaStream_t>(stream);
   return mode == WALK_SPACE ? walk_dispatch<WALK_SPACE>(a, pieces, s) : walk_dispatch<WALK_FIXED>(a, pieces, s);

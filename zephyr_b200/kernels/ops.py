@@ -148,7 +148,7 @@ _SIGNATURES = {
     "zb_decayed_state_scan": [c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p,
                               c_longlong, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
                               c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
-                              c_float, c_float, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p],
+                              c_int, c_float, c_float, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p],
     "zb_retention_piece_tokens": [],
     "zb_retention_max_channels": [],
     "zb_retention": [c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_longlong,
@@ -160,7 +160,7 @@ _SIGNATURES = {
     "zb_walk_piece_floats": [c_int, c_int, c_int, c_int],
     "zb_state_walk": [c_int, c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p,
                       c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-                      c_int, c_int, c_int, c_int, c_void_p, c_int, c_float, c_void_p, c_void_p, c_void_p, c_void_p],
+                      c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_float, c_void_p, c_void_p, c_void_p, c_void_p],
     "zb_rotate_qk": [c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_float, c_void_p, c_int, c_int, c_int, c_void_p],
     "zb_gated_group_rms_norm": [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_int,
                                 c_float, c_int, c_int, c_int, c_void_p],
@@ -718,14 +718,25 @@ def state_scan_max_channels() -> int:
     return library().zb_state_scan_max_channels()
 
 
-WALK_FROM = 32      # new tokens per request, on average, from which on a step's recurrences with one decay a head walk in pieces
+def _two_forms(tokens: int, rows: int, limit: int, row_tokens: Sequence[int] | None) -> tuple[bool, bool]:
+    """Whether a step may have rows of fewer than ``limit`` tokens, and rows of ``limit`` and more; ``row_tokens`` are the
+    rows' tokens where the host knows them."""
+    if row_tokens is None and rows == 1:
+        row_tokens = [tokens]
+    if row_tokens is None:
+        return True, tokens >= limit
+    return any(0 < n < limit for n in row_tokens), any(n >= limit for n in row_tokens)
+
+
+WALK_FROM = 32      # new tokens of a row from which on the bfloat16 state-space form walks in pieces
 
 
 def _state_walk(mode: int, out, q, k, v, heads: int, key_dim: int, value_dim: int, state, slots, row_q_start, row_q_len, status,
-                write_state: bool, dt=None, dt_bias=None, a_log=None, skip=None, decay=None, heads_per_group: int = 1, turn=None) -> None:
-    """The recurrence over runs of tokens in pieces of 64 with the state on the SM (csrc/state_walk.cu): mode 0 the
-    state-space form, 1 fixed decays (``turn``: (freqs, rot_dims, k_scale, positions) where q and k are still to be
-    turned).  The callers have checked types and shapes."""
+                write_state: bool, dt=None, dt_bias=None, a_log=None, skip=None, decay=None, heads_per_group: int = 1, turn=None,
+                limit: int = 0) -> None:
+    """The recurrence over the rows of ``limit`` tokens and more in pieces of 64 with the state on the SM (csrc/state_walk.cu):
+    mode 0 the state-space form, 1 fixed decays (``turn``: (freqs, rot_dims, k_scale, positions) where q and k are still to
+    be turned).  The callers have checked types and shapes."""
     lib, rows, T = library(), slots.numel(), v.shape[0]
     freqs, rot_dims, k_scale, positions = turn or (None, 0, 1.0, None)
     ws = torch.empty(((T // lib.zb_walk_piece_tokens() + rows) * lib.zb_walk_piece_floats(mode, heads, heads_per_group, key_dim),),
@@ -733,7 +744,7 @@ def _state_walk(mode: int, out, q, k, v, heads: int, key_dim: int, value_dim: in
     _check(lib.zb_state_walk(
         mode, _ptr(out), _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(dt), dt.stride(0) if dt is not None else 0,
         _ptr(dt_bias), _ptr(a_log), _ptr(skip), _ptr(decay), _ptr(state), state.stride(0), _ptr(slots), _ptr(row_q_start),
-        _ptr(row_q_len), rows, T, heads, key_dim, value_dim, heads_per_group, state.shape[0], int(write_state), _ptr(freqs), int(rot_dims),
+        _ptr(row_q_len), rows, T, limit, heads, key_dim, value_dim, heads_per_group, state.shape[0], int(write_state), _ptr(freqs), int(rot_dims),
         float(k_scale), _ptr(positions), _ptr(ws), _ptr(status), _stream()), "state_walk", kernels=2)
 
 
@@ -744,7 +755,8 @@ def decayed_state_scan(mode: str, q: torch.Tensor, k: torch.Tensor, v: torch.Ten
                        dt: torch.Tensor | None = None, dt_bias: torch.Tensor | None = None,
                        a_log: torch.Tensor | None = None, skip: torch.Tensor | None = None,
                        decay: torch.Tensor | None = None, heads_per_group: int = 1,
-                       write_state: bool = True, segment: int | None = None) -> torch.Tensor:
+                       write_state: bool = True, segment: int | None = None,
+                       row_tokens: Sequence[int] | None = None) -> torch.Tensor:
     """S_t = diag(a_t) S_{t-1} + k_t v_t^T, o_t = S_t^T q_t per head over each row's new tokens, from and
     to ``state`` [slots, heads * key_dim * value_dim] float32 (rows may be strided); returns o as float32
     [T, heads * value_dim].  q, k, v: [T, .] with unit inner stride, head h at column h * width.
@@ -758,8 +770,10 @@ def decayed_state_scan(mode: str, q: torch.Tensor, k: torch.Tensor, v: torch.Ten
     arithmetic on many times the threads); 0: never; None: chosen, for steps whose requests bring 256
     tokens and more on average and whose requests x heads x columns / 64 do not fill the SMs (measured,
     one request of 2048 tokens: 8 heads of 128 x 256: 712 -> 270 us; 16 heads: 720 -> 482 us).  None also lets
-    the bfloat16 "state_space" form with ``WALK_FROM`` tokens a request and more, of shapes the walk over pieces
-    takes (csrc/state_walk.cu), run there on the tensor cores (2125 tokens, 32 heads of 128 x 64: 290 -> 82 us)."""
+    the rows of ``WALK_FROM`` tokens and more of the bfloat16 "state_space" form, of shapes the walk over pieces takes
+    (csrc/state_walk.cu), run there on the tensor cores (2125 tokens, 32 heads of 128 x 64: 290 -> 82 us); the other rows
+    then run token by token, so that what a row gets hangs on that row alone.  ``row_tokens``: ``row_q_len`` on the host,
+    where the caller has it, so that a form that no row takes is not launched."""
     _cuda(q, k, v, state, slots, row_q_start, row_q_len, status, decay_logits, decay_bias, dt, dt_bias, a_log, skip)
     _i32(slots, row_q_start, row_q_len)
     T = v.shape[0]
@@ -788,12 +802,18 @@ def decayed_state_scan(mode: str, q: torch.Tensor, k: torch.Tensor, v: torch.Ten
             _f32_vector(vector, heads, "a per-head constant")
     out = torch.empty((T, heads * value_dim), dtype=torch.float32, device=v.device)
     rows = slots.numel()
-    if (segment is None and not gated and not fixed and v.dtype == torch.bfloat16 and T >= WALK_FROM * rows and key_dim % 8 == 0
+    below = 0
+    if (segment is None and not gated and not fixed and v.dtype == torch.bfloat16 and key_dim % 8 == 0
             and key_dim <= library().zb_walk_max_channels() and heads % heads_per_group == 0
             and all(t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (q, k))):
-        _state_walk(0, out, q, k, v, heads, key_dim, value_dim, state, slots, row_q_start, row_q_len, status, write_state, dt=dt,
-                    dt_bias=dt_bias, a_log=a_log, skip=skip, heads_per_group=int(heads_per_group))
-        return out
+        short, long = _two_forms(T, rows, WALK_FROM, row_tokens)
+        if long:
+            _state_walk(0, out, q, k, v, heads, key_dim, value_dim, state, slots, row_q_start, row_q_len, status, write_state, dt=dt,
+                        dt_bias=dt_bias, a_log=a_log, skip=skip, heads_per_group=int(heads_per_group), limit=WALK_FROM)
+            below = WALK_FROM
+        if not short:
+            return out
+        segment = 0
     if segment is None:
         few = rows * heads * -(-value_dim // 64) <= _sm_count()
         segment = (max(SCAN_SEGMENT, -(-T // (64 * 16)) * 16)
@@ -807,8 +827,8 @@ def decayed_state_scan(mode: str, q: torch.Tensor, k: torch.Tensor, v: torch.Ten
         _ptr(out), _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(decay_logits),
         decay_logits.stride(0) if gated else 0, _ptr(decay_bias), _ptr(dt), dt.stride(0) if dt is not None else 0,
         _ptr(dt_bias), _ptr(a_log), _ptr(skip), _ptr(decay), 0, _ptr(state), state.stride(0), _ptr(slots), _ptr(row_q_start),
-        _ptr(row_q_len), slots.numel(), T, heads, key_dim, value_dim, int(heads_per_group), state.shape[0],
-        int(write_state), float(q_scale), float(inv_tau), {"gated": 0, "state_space": 1, "fixed": 2}[mode], DTYPE_CODE[v.dtype], int(segment),
+        _ptr(row_q_len), rows, T, heads, key_dim, value_dim, int(heads_per_group), state.shape[0],
+        int(write_state), below, float(q_scale), float(inv_tau), {"gated": 0, "state_space": 1, "fixed": 2}[mode], DTYPE_CODE[v.dtype], int(segment),
         _ptr(ws_state), _ptr(ws_decay), _ptr(status), _stream()), "decayed_state_scan",
         kernels=(2 if gated else 1) + (2 if segment else 0))
     return out
@@ -1298,16 +1318,6 @@ def delta_max_channels() -> int:
 
 
 DELTA_BLOCKS_FROM = 16       # new tokens of a row from which on the delta rule runs block by block
-
-
-def _two_forms(tokens: int, rows: int, limit: int, row_tokens: Sequence[int] | None) -> tuple[bool, bool]:
-    """Whether a step may have rows of fewer than ``limit`` tokens, and rows of ``limit`` and more; ``row_tokens`` are the
-    rows' tokens where the host knows them."""
-    if row_tokens is None and rows == 1:
-        row_tokens = [tokens]
-    if row_tokens is None:
-        return True, tokens >= limit
-    return any(0 < n < limit for n in row_tokens), any(n >= limit for n in row_tokens)
 
 
 def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b: torch.Tensor, a: torch.Tensor,

@@ -193,7 +193,8 @@ class Mamba2(Mixer):
                                    self.heads, self.state, self.vdim, store[:, :self.scan_floats], ctx.state_slots,
                                    ctx.row_q_start, ctx.row_q_len, ctx.status, dt=projected[:, inner + self.channels:],
                                    dt_bias=self.dt_bias, a_log=self.a_log, skip=self.skip,
-                                   heads_per_group=self.heads // self.groups, write_state=call.writes_cache)
+                                   heads_per_group=self.heads // self.groups, write_state=call.writes_cache,
+                                   row_tokens=ctx.host_q_len or None)
         normed = ops.gated_group_rms_norm(o, projected[:, :inner], self.norm, inner // self.norm_groups, self.eps,
                                           gate_first=True)
         return ops.linear(normed, self.w_o, out_dtype=out_dtype)
