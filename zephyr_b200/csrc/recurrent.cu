@@ -99,9 +99,10 @@ __global__ void residual_layer_norm_kernel(float* residual, const T* delta, cons
 
 // The same two kernels for rows of up to LN_VEC_MAX elements whose length is a multiple of four: a thread
 // keeps its share of the row in registers as vectors of four, loads and stores move 8 or 16 bytes, and
-// nothing passes through shared memory but the two sums.  All that a row needs is asked for before the first sum (the row it
-// is added to was read behind it, the scales behind that): a decode step's few rows wait for one latency, not three, 12 rows of
-// 2048 into the residual stream 6.1 -> 3.6 us.
+// nothing passes through shared memory but the two sums.  All that a row of up to 2048 elements needs is asked for before the
+// first sum (the row it is added to was read behind it, the scales behind that): a decode step's few rows wait for one latency,
+// not three, 12 rows of 2048 into the residual stream 6.1 -> 3.6 us.  A longer row's thread would hold 64 values that way, and
+// half as many CTAs share an SM (2048 rows of 4096: 27 us, 21 read where they are used).
 constexpr int LN_VEC_THREADS = 256;
 constexpr int LN_VEC_ITEMS = 8;
 constexpr int LN_VEC_MAX = LN_VEC_THREADS * LN_VEC_ITEMS * 4;
@@ -207,13 +208,14 @@ residual_layer_norm_vec_kernel(float* residual, const T* delta, const float* w1,
   __shared__ float scratch[33];
   const size_t base = static_cast<size_t>(blockIdx.x) * H;
   const int nv = H / 4;
-  float4 r[ITEMS], old[ITEMS];
+  constexpr bool AHEAD = VecAffine<ITEMS>::KEPT;
+  float4 r[ITEMS], old[AHEAD ? ITEMS : 1];
 #pragma unroll
   for (int j = 0; j < ITEMS; ++j) {
     const int i = threadIdx.x + j * LN_VEC_THREADS;
     if (i < nv) {
       r[j] = load4(delta + base + 4 * i);
-      old[j] = load4(residual + base + 4 * i);
+      if (AHEAD) old[AHEAD ? j : 0] = load4(residual + base + 4 * i);
     }
   }
   const VecAffine<ITEMS> first(w1, b1, nv), second(out != nullptr ? w2 : nullptr, b2, nv);
@@ -223,8 +225,8 @@ residual_layer_norm_vec_kernel(float* residual, const T* delta, const float* w1,
   for (int j = 0; j < ITEMS; ++j) {
     const int i = threadIdx.x + j * LN_VEC_THREADS;
     if (i < nv) {
-      const float4 y = first(r[j], mean, rstd, j);
-      r[j] = make_float4(fmaf(mult, y.x, old[j].x), fmaf(mult, y.y, old[j].y), fmaf(mult, y.z, old[j].z), fmaf(mult, y.w, old[j].w));
+      const float4 y = first(r[j], mean, rstd, j), was = AHEAD ? old[AHEAD ? j : 0] : load4(residual + base + 4 * i);
+      r[j] = make_float4(fmaf(mult, y.x, was.x), fmaf(mult, y.y, was.y), fmaf(mult, y.z, was.z), fmaf(mult, y.w, was.w));
       store4(residual + base + 4 * i, r[j]);
       if (out != nullptr && w2 == nullptr) store4(out + base + 4 * i, r[j]);   // no second norm: the sum, rounded
     }
