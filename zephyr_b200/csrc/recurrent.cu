@@ -1082,13 +1082,15 @@ ZB_API int zb_causal_conv_silu(void* out, const void* x, long long x_stride, flo
   auto s = static_cast<cudaStream_t>(stream);
   if (tokens <= 0) return OK;
   const dim3 grid((tokens + CONV_TOKENS - 1) / CONV_TOKENS, (C + 127) / 128), per_row((C + 127) / 128, rows);
-  // Runs pay where requests bring several tokens; a step of single tokens has nothing to share.
+  // Runs pay where requests bring several tokens (a step of single tokens has nothing to share) and from half a million values
+  // on: below, runs of CONV_RUN tokens are too few CTAs.  4096 channels, 64 tokens: 8.2 us as runs, 6.2 a value at a time; 128:
+  // 8.4 and 8.5; 256: 8.9 and 12.3; 2560 channels, 128 tokens: 8.1 and 7.2; 256: 8.4 and 9.4.  The sums are the same.
   auto aligned = [&](int vec) {
     const size_t bytes = vec * (dtype == DTYPE_F32 ? 4 : 2);
     return C % vec == 0 && x_stride % vec == 0 && w_dtype == DTYPE_F32 && reinterpret_cast<uintptr_t>(x) % bytes == 0 &&
            reinterpret_cast<uintptr_t>(out) % bytes == 0;
   };
-  const bool runs = tokens >= 4 * rows && aligned(2);
+  const bool runs = tokens >= 4 * rows && static_cast<long long>(tokens) * C >= 1 << 19 && aligned(2);
   if (dtype == DTYPE_F32) {
     if (runs) conv_run_launch<float>(a, token_row, tokens, aligned(4), s);
     else causal_conv_silu_kernel<float><<<grid, 128, 0, s>>>(a, token_row, tokens);
