@@ -193,7 +193,8 @@ __global__ void __launch_bounds__(QP_WARPS * 32) qkv_pairs_kernel(const QkvPairs
 // a piece goes within a cache row is one exclusive-or.  The general kernel above is bound by instructions, not by memory:
 // two sines a lane and head and 300 instructions a head: 2125 tokens of 32
 // heads of 128 in float32 took 29.6 us and take 18.6 (its bytes: 8 us), 12 tokens 5.2 and 3.9 us.  More heads a warp alone
-// (33 us) did not help the general form.
+// (33 us) did not help the general form.  Heads of up to 64 values leave half of a warp's lanes idle here and stay with the
+// general kernel (300 tokens, 40 heads of 64: 5.1 us there, 6.0 here; 2048: 21.4 and 21.9).
 constexpr int QPV_WARPS = 8;
 
 __device__ __forceinline__ float4 load_piece(const float* p) { return *reinterpret_cast<const float4*>(p); }
@@ -356,7 +357,7 @@ ZB_API int zb_qkv_pairs(void* q_out, const void* qkv, long long stride, const fl
   const int wide = kd > vd ? kd : vd;
   const long long page_values = static_cast<long long>(nkv) * page_size * (kd + vd);
   if (!(dtype == DTYPE_F32 && in_dtype != DTYPE_F32) && kd % 4 == 0 && vd % 4 == 0 && a.rot_dims % 4 == 0 && stride % 4 == 0 &&
-      whole(qkv) && whole(bias) && whole(q_norm_w) && whole(k_norm_w) && whole(q_out) && whole(cache) && wide <= 256 &&
+      whole(qkv) && whole(bias) && whole(q_norm_w) && whole(k_norm_w) && whole(q_out) && whole(cache) && wide > 64 && wide <= 256 &&
       page_values <= INT_MAX && a.rot_dims <= 8192) {
     auto s = static_cast<cudaStream_t>(stream);
     const size_t smem = sizeof(float) * a.rot_dims;
