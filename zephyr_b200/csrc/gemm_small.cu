@@ -10,7 +10,9 @@
 //
 // One CTA owns 16 rows of W (or 32); its warps split K, and for matrices with few rows a cluster of
 // up to 8 CTAs splits K further.  A decode step's product is bound by latency before it is by bandwidth: a warp has the loads
-// of four blocks of 32 k in flight, whatever is left of its slice (one block after the other, as a loop's remainder, 2048 x
+// of several blocks of 32 k in flight, whatever is left of its slice: four up to 16 rows, two from 17 to 32 and where a CTA takes
+// 32 rows of W; above 32 rows four blocks of W alone, x at its use (with x ahead too, two blocks: 12288 x 4096, 64 rows: 92 us,
+// now 47; 6144 x 2048: 29 and 17) (one block after the other, as a loop's remainder, 2048 x
 // 6144 with 12 rows took 13.8 us; now 10.1, its bytes 3.8), and the CTAs of a cluster each finish a share of the tile with one
 // round of remote reads (one CTA for all, 2048 x 2048: 9.8 us; now 6.1).  4096 x 2048: 10.2 -> 7.9, 12288 x 2048: 14.9 -> 14.1,
 // 8192 x 4096, 12 rows: 16.9.  Partial sums meet in (distributed) shared memory and are added in
@@ -58,7 +60,8 @@ template <> __device__ __forceinline__ void store_out<__nv_bfloat16>(__nv_bfloat
 template <int RT, int WARPS, int MT, typename TOut, bool SWIGLU, int ACT>
 __global__ void __launch_bounds__(WARPS * 32)
 gemm_small_kernel(const SmallGemmArgs a) {
-  constexpr int U = RT == 1 && MT <= 2 ? 4 : 2;     // blocks of k in flight
+  constexpr bool X_AHEAD = MT <= 4;                 // (eight tiles of tokens ahead leave room for two blocks of W)
+  constexpr int U = (RT == 1 && MT <= 2) || !X_AHEAD ? 4 : 2;     // blocks of k in flight
   constexpr int PER_WARP = RT * MT * 16 * 8;        // sums of a warp: [rt][mt][row][token]
   __shared__ float red[WARPS][PER_WARP];
   cg::cluster_group cluster = cg::this_cluster();
@@ -94,7 +97,7 @@ gemm_small_kernel(const SmallGemmArgs a) {
     for (int mt = 0; mt < MT; ++mt) acc[rt][mt][0] = acc[rt][mt][1] = acc[rt][mt][2] = acc[rt][mt][3] = 0.0f;
 
   for (int b = b_begin; b < b_end; b += U) {
-    uint4 wv[U][2 * RT], xv[U][MT];
+    uint4 wv[U][2 * RT], xv[X_AHEAD ? U : 1][X_AHEAD ? MT : 1];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int k = (b + u) * 32;
@@ -102,7 +105,7 @@ gemm_small_kernel(const SmallGemmArgs a) {
 #pragma unroll
       for (int r = 0; r < 2 * RT; ++r) wv[u][r] = load16_or_zero(w_row[r] + k, w_ok[r] && k_ok);
 #pragma unroll
-      for (int mt = 0; mt < MT; ++mt) xv[u][mt] = load16_or_zero(x_row[mt] + k, x_ok[mt] && k_ok);
+      for (int mt = 0; X_AHEAD && mt < MT; ++mt) xv[u][mt] = load16_or_zero(x_row[mt] + k, x_ok[mt] && k_ok);
     }
 #pragma unroll
     for (int u = 0; u < U; ++u)
@@ -113,8 +116,11 @@ gemm_small_kernel(const SmallGemmArgs a) {
         const unsigned a1[4] = {wl.z, wh.z, wl.w, wh.w};
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt) {
-          mma_bf16_16816(acc[rt][mt], a0, xv[u][mt].x, xv[u][mt].y);
-          mma_bf16_16816(acc[rt][mt], a1, xv[u][mt].z, xv[u][mt].w);
+          const int k = (b + u) * 32;
+          const uint4 x = X_AHEAD ? xv[X_AHEAD ? u : 0][X_AHEAD ? mt : 0]
+                                  : load16_or_zero(x_row[mt] + k, x_ok[mt] && b + u < b_end && k + 8 * t + 8 <= a.K);
+          mma_bf16_16816(acc[rt][mt], a0, x.x, x.y);
+          mma_bf16_16816(acc[rt][mt], a1, x.z, x.w);
         }
       }
   }
