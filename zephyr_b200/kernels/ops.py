@@ -728,7 +728,7 @@ def _two_forms(tokens: int, rows: int, limit: int, row_tokens: Sequence[int] | N
     return any(0 < n < limit for n in row_tokens), any(n >= limit for n in row_tokens)
 
 
-WALK_FROM = 32      # new tokens of a row from which on the bfloat16 state-space form walks in pieces
+WALK_FROM = 32      # new tokens of a row from which on the bfloat16 state-space form walks in pieces, unless a caller sets its line
 
 
 def _state_walk(mode: int, out, q, k, v, heads: int, key_dim: int, value_dim: int, state, slots, row_q_start, row_q_len, status,
@@ -756,7 +756,7 @@ def decayed_state_scan(mode: str, q: torch.Tensor, k: torch.Tensor, v: torch.Ten
                        a_log: torch.Tensor | None = None, skip: torch.Tensor | None = None,
                        decay: torch.Tensor | None = None, heads_per_group: int = 1,
                        write_state: bool = True, segment: int | None = None,
-                       row_tokens: Sequence[int] | None = None) -> torch.Tensor:
+                       row_tokens: Sequence[int] | None = None, walk_from: int | None = None) -> torch.Tensor:
     """S_t = diag(a_t) S_{t-1} + k_t v_t^T, o_t = S_t^T q_t per head over each row's new tokens, from and
     to ``state`` [slots, heads * key_dim * value_dim] float32 (rows may be strided); returns o as float32
     [T, heads * value_dim].  q, k, v: [T, .] with unit inner stride, head h at column h * width.
@@ -770,7 +770,7 @@ def decayed_state_scan(mode: str, q: torch.Tensor, k: torch.Tensor, v: torch.Ten
     arithmetic on many times the threads); 0: never; None: chosen, for steps whose requests bring 256
     tokens and more on average and whose requests x heads x columns / 64 do not fill the SMs (measured,
     one request of 2048 tokens: 8 heads of 128 x 256: 712 -> 270 us; 16 heads: 720 -> 482 us).  None also lets
-    the rows of ``WALK_FROM`` tokens and more of the bfloat16 "state_space" form, of shapes the walk over pieces takes
+    the rows of ``walk_from`` (``WALK_FROM``) tokens and more of the bfloat16 "state_space" form, of shapes the walk over pieces takes
     (csrc/state_walk.cu), run there on the tensor cores (2125 tokens, 32 heads of 128 x 64: 290 -> 82 us); the other rows
     then run token by token, so that what a row gets hangs on that row alone.  ``row_tokens``: ``row_q_len`` on the host,
     where the caller has it, so that a form that no row takes is not launched."""
@@ -806,11 +806,12 @@ def decayed_state_scan(mode: str, q: torch.Tensor, k: torch.Tensor, v: torch.Ten
     if (segment is None and not gated and not fixed and v.dtype == torch.bfloat16 and key_dim % 8 == 0
             and key_dim <= library().zb_walk_max_channels() and heads % heads_per_group == 0
             and all(t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (q, k))):
-        short, long = _two_forms(T, rows, WALK_FROM, row_tokens)
+        limit = walk_from or WALK_FROM
+        short, long = _two_forms(T, rows, limit, row_tokens)
         if long:
             _state_walk(0, out, q, k, v, heads, key_dim, value_dim, state, slots, row_q_start, row_q_len, status, write_state, dt=dt,
-                        dt_bias=dt_bias, a_log=a_log, skip=skip, heads_per_group=int(heads_per_group), limit=WALK_FROM)
-            below = WALK_FROM
+                        dt_bias=dt_bias, a_log=a_log, skip=skip, heads_per_group=int(heads_per_group), limit=limit)
+            below = limit
         if not short:
             return out
         segment = 0
@@ -1317,21 +1318,21 @@ def delta_max_channels() -> int:
     return library().zb_delta_max_channels()
 
 
-DELTA_BLOCKS_FROM = 16       # new tokens of a row from which on the delta rule runs block by block
+DELTA_BLOCKS_FROM = 16       # new tokens of a row from which on the delta rule runs block by block, unless a caller sets its line
 
 
 def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b: torch.Tensor, a: torch.Tensor,
                a_log: torch.Tensor, dt_bias: torch.Tensor, heads: int, qk_heads: int, key_dim: int, value_dim: int,
                state: torch.Tensor, slots: torch.Tensor, row_q_start: torch.Tensor, row_q_len: torch.Tensor,
                status: torch.Tensor, q_scale: float, unit_eps: float = 1e-6, write_state: bool = True,
-               row_tokens: Sequence[int] | None = None) -> torch.Tensor:
+               row_tokens: Sequence[int] | None = None, blocks_from: int | None = None) -> torch.Tensor:
     """The gated delta rule per head over each row's new tokens, from and to ``state`` [slots, heads *
     value_dim * key_dim] float32 (rows may be strided; a head's state lies [value_dim][key_dim]):
     S <- g S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q.  q and k [T, qk_heads * key_dim] (head h uses
     q/k head h // (heads / qk_heads)) are made unit vectors, x / sqrt(sum(x^2) + unit_eps), q times
     ``q_scale``; v [T, heads * value_dim]; beta = sigmoid(b), g = exp(-exp(a_log) softplus(a + dt_bias)) from
-    float32 b and a [T, heads].  q, k, v share a type and may be strided slices.  Rows of ``DELTA_BLOCKS_FROM`` tokens and more
-    run block by block (up to 128 key channels), the others token by token: what a row gets hangs on that row alone.
+    float32 b and a [T, heads].  q, k, v share a type and may be strided slices.  Rows of ``blocks_from``
+    (``DELTA_BLOCKS_FROM``) tokens and more run block by block (up to 128 key channels), the others token by token: what a row gets hangs on that row alone.
     ``row_tokens``: ``row_q_len`` on the host, where the caller has it, so that a form that no row takes is not launched.
     Returns o float32 [T, heads * value_dim]."""
     _cuda(q, k, v, b, a, a_log, dt_bias, state, slots, row_q_start, row_q_len, status)
@@ -1350,7 +1351,7 @@ def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b: torch.Tenso
              and state.shape[1] == heads * key_dim * value_dim, "state must be float32 [slots, heads * value_dim * key_dim]")
     dev, lib, rows = v.device, library(), slots.numel()
     out = torch.empty((T, heads * value_dim), dtype=torch.float32, device=dev)
-    limit = DELTA_BLOCKS_FROM if key_dim <= lib.zb_delta_block_max_channels() else T + 1
+    limit = (blocks_from or DELTA_BLOCKS_FROM) if key_dim <= lib.zb_delta_block_max_channels() else T + 1
     short, long = _two_forms(T, rows, limit, row_tokens)
     if long:
         ws = torch.empty(((T // lib.zb_delta_block_tokens() + rows) * lib.zb_delta_block_floats(qk_heads, heads, key_dim),),

@@ -126,6 +126,11 @@ class Mamba2(Mixer):
     graph_safe = True
     takes_out_dtype = True
 
+    # New tokens of a row from which on it walks in pieces, whole ones from here on (32 heads of 128 x 64, one row of 64 tokens:
+    # 17 us, 31 as a scan; 8 rows: 35 and 45; 64 rows: 212 and 294; 8 heads of 64 x 128, 64 rows: 78 and 82.  Of 32 tokens: 17
+    # and 19, 33 and 26, 192 and 167, 70 and 48).
+    WALK_FROM = 64
+
     def __init__(self, spec: MixerSpec, weights: Mapping[str, torch.Tensor], dtype: torch.dtype,
                  device: torch.device | str):
         p = spec.params
@@ -194,7 +199,7 @@ class Mamba2(Mixer):
                                    ctx.row_q_start, ctx.row_q_len, ctx.status, dt=projected[:, inner + self.channels:],
                                    dt_bias=self.dt_bias, a_log=self.a_log, skip=self.skip,
                                    heads_per_group=self.heads // self.groups, write_state=call.writes_cache,
-                                   row_tokens=ctx.host_q_len or None)
+                                   row_tokens=ctx.host_q_len or None, walk_from=self.WALK_FROM)
         normed = ops.gated_group_rms_norm(o, projected[:, :inner], self.norm, inner // self.norm_groups, self.eps,
                                           gate_first=True)
         return ops.linear(normed, self.w_o, out_dtype=out_dtype)
@@ -205,6 +210,11 @@ class GatedDeltaRule(Mixer):
     takes_out_dtype = True
 
     UNIT_EPS = 1e-6      # inside the root of the unit norms of q and k: the design fixes it
+    # New tokens of a row from which on it runs in blocks.  Blocks shorten a row's chain and pay most where rows are few (16
+    # heads of 128 x 128, one row of 128 tokens: 27 us, 40 token by token; 2048: 240 and 522; 8 heads of 64 x 64, 128: 20 and
+    # 36).  Where the rows' own chains fill the SMs they are behind, least for long rows (8 rows of 128: 105 and 98; 32 rows of
+    # 64: 216 and 172), so the line lies above what a row alone would have it (24 tokens).
+    BLOCKS_FROM = 128
 
     def __init__(self, spec: MixerSpec, weights: Mapping[str, torch.Tensor], dtype: torch.dtype,
                  device: torch.device | str):
@@ -273,7 +283,7 @@ class GatedDeltaRule(Mixer):
                            steps[:, self.heads:], self.a_log, self.dt_bias, self.heads, self.qk_heads, self.dim,
                            self.vdim, store[:, :self.scan_floats], ctx.state_slots, ctx.row_q_start, ctx.row_q_len,
                            ctx.status, q_scale=self.dim ** -0.5, unit_eps=self.UNIT_EPS, write_state=call.writes_cache,
-                           row_tokens=ctx.host_q_len or None)
+                           row_tokens=ctx.host_q_len or None, blocks_from=self.BLOCKS_FROM)
         normed = ops.gated_group_rms_norm(o, ops.linear(x, self.w_g), self.norm, self.vdim, self.eps, gate_first=False)
         return ops.linear(normed, self.w_o, out_dtype=out_dtype)
 
