@@ -43,6 +43,7 @@ def test_kept_windows_and_chunks(ops, cuda_device, window, keep, chunk, softcap,
     status, got = ops.new_status(cuda_device), {}
     for tcgen05 in (True, False):
         ops.USE_TCGEN05_PREFILL = tcgen05
+        before = ops.LAUNCH_COUNTS.get("paged_prefill_tc", 0)
         try:
             got[tcgen05] = ops.paged_prefill(q, cache, meta["table"], *tiles_for(q_lens, ops.paged_prefill_tile_tokens(), cuda_device),
                                              meta["row_q_start"], meta["row_q_len"], meta["row_ctx"], nh, nkv, hd, window,
@@ -50,6 +51,7 @@ def test_kept_windows_and_chunks(ops, cuda_device, window, keep, chunk, softcap,
                                              softcap=softcap, keep_first=keep)
         finally:
             ops.USE_TCGEN05_PREFILL = True
+        assert ops.LAUNCH_COUNTS.get("paged_prefill_tc", 0) - before == int(tcgen05)      # each ran on the kernel it is about
     ops.check_status(status)
     # Weights and the result are rounded to bfloat16 (2^-9 each, of values around one to four).
     assert (got[True].float() - got[False].float()).abs().max() <= 3 * 2.0 ** -7

@@ -1673,7 +1673,7 @@ def paged_prefill(q: torch.Tensor, kv_cache: torch.Tensor, block_table: torch.Te
               _ptr(row_ctx), nh, nkv, hd, int(window))
     if tensor_memory:
         _check(library().zb_paged_prefill_tc_masked(*common, int(chunk), int(keep_first), float(scale), float(softcap), int(keys_only), _ptr(sinks),
-                                                    _ptr(r1), _ptr(r2), _ptr(status), _stream()), "paged_prefill")
+                                                    _ptr(r1), _ptr(r2), _ptr(status), _stream()), "paged_prefill_tc")
     elif windowed or r1 is not None:
         _check(library().zb_paged_prefill_windowed(*common, int(chunk), float(scale), float(softcap), int(keys_only),
                                                    _ptr(sinks), int(keep_first), int(pool), _ptr(pool_cache),
