@@ -3,10 +3,11 @@
 //
 // The general kernel reads one key value per lane and multiply-add from shared memory; here a CTA takes F_ROWS query
 // rows (the (token, head) pairs of neighbouring tokens and one key/value head) against F_KEYS keys at a time, a thread
-// 4 x 4 scores and 4 x D/16 outputs, so that a 16-byte read serves 8 to 11 multiply-adds.  Bound by those reads and by
-// the exponentials between the two products.  Keys lie transposed ([channel][key]), values as they are; a warp owns
+// 4 x 4 scores and 4 x D/16 outputs, so that a 16-byte read serves 8 to 11 multiply-adds.  Bound by those reads'
+// latency and by the exponentials between the two products, with two CTAs an SM at most (700 tokens: 192 CTAs, 0.65 of a
+// wave; shared memory busy for 52 % of the time).  Keys lie transposed ([channel][key]), values as they are; a warp owns
 // eight rows across all keys, so the weights go from one product to the other inside a warp.  700 tokens, 16 heads over 8 of 128:
-// 163 us, 776 in the general kernel.  Every row with several tokens runs here, so that its result hangs on that row alone: behind
+// 166 us, 776 in the general kernel.  Every row with several tokens runs here, so that its result hangs on that row alone: behind
 // a context of 600 two tokens take 142 us (328 in the general kernel) and fifteen 143 (553); two tokens of a new prompt, most
 // of whose tile is empty, take 22 instead of 16 us, eight rows of sixteen 31 instead of 37.
 //

@@ -15,14 +15,17 @@
 //
 // so the state never leaves the SM, where passes over all pieces at once write and read every piece's state (2048
 // tokens, 32 heads of 128 x 64: 33 MB four times), and a piece is two barriers.  Measured: the state-space form, 2048 and 77 tokens,
-// 32 heads of 128 x 64: 18 + 64 us, 290 as a scan in segments; retention, 1500 and 548 tokens, 32 heads of 128 x 128, rotation
-// included: 45 + 118 us, 203 in three passes and a rotation.  Bound by the pieces' way out of L2 (3.7 of about 4 TB/s, retention)
-// and by the two barriers with eight warps an SM (the state-space form).
+// 32 heads of 128 x 64: 19 + 68 us, 290 as a scan in segments; retention, 1500 and 548 tokens, 32 heads of 128 x 128, rotation
+// included: 44 + 122 us, 203 in three passes and a rotation.  Bound by latency with the eight warps an SM that a CTA's shared
+// memory leaves: products' results, reads of shared memory (busy for 57 to 60 % of the time) and two barriers a piece, 1.7 waves
+// of CTAs; L2 is at 14 and 18 %.
 //
 // Products run on the tensor cores, float32 sums.  A bfloat16 operand is exact; beside it a float32 operand is the sum of three
 // bfloat16 values (all its 24 bits).  The tensor cores cut a sum at every step, so there the products of the small parts have
 // a sum of their own, and scores two (error against 64 bits over 2048 and 77 tokens: 1.32e-7, 1.82e-7 with one sum each,
-// 1.29e-7 token by token).  Two float32 operands (WALK_FIXED) are two bfloat16 values each, hi hi + hi lo + lo hi, a relative error of about 2^-16 an operand.  The state itself is only ever touched by float32 multiply-adds.
+// 1.29e-7 token by token).  Two float32 operands (WALK_FIXED) are two bfloat16 values each, hi hi + hi lo + lo hi, a relative
+// error of about 2^-16 an operand.  The state itself is only ever touched by float32 multiply-adds.
+//
 // A value that is not finite must not reach the tokens before it through the zeros above P's diagonal: it is left out of the
 // product and added by hand to the outputs of the tokens from its own on.  What is behind it is not finite either, an
 // infinity or a NaN.
