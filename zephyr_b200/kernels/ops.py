@@ -1332,9 +1332,9 @@ def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b: torch.Tenso
     q/k head h // (heads / qk_heads)) are made unit vectors, x / sqrt(sum(x^2) + unit_eps), q times
     ``q_scale``; v [T, heads * value_dim]; beta = sigmoid(b), g = exp(-exp(a_log) softplus(a + dt_bias)) from
     float32 b and a [T, heads].  q, k, v share a type and may be strided slices.  Rows of ``blocks_from``
-    (``DELTA_BLOCKS_FROM``) tokens and more run block by block (up to 128 key channels), the others token by token: what a row gets hangs on that row alone.
-    ``row_tokens``: ``row_q_len`` on the host, where the caller has it, so that a form that no row takes is not launched.
-    Returns o float32 [T, heads * value_dim]."""
+    (``DELTA_BLOCKS_FROM``) tokens and more run block by block (up to 128 key channels), the others token by token, so that what
+    a row gets hangs on that row alone.  ``row_tokens``: ``row_q_len`` on the host, where the caller has it, so that a form that
+    no row takes is not launched.  Returns o float32 [T, heads * value_dim]."""
     _cuda(q, k, v, b, a, a_log, dt_bias, state, slots, row_q_start, row_q_len, status)
     _i32(slots, row_q_start, row_q_len)
     T = v.shape[0]
