@@ -98,7 +98,7 @@ struct DeltaScanArgs {
   const int* row_q_start;
   const int* row_q_len;
   int heads, heads_per_group, D, V, num_slots, write_state;
-  int below;               // > 0: only rows with fewer than this many tokens
+  int below;               // SHORT: only rows with fewer than this many tokens
   int* status;
 };
 
@@ -114,7 +114,8 @@ struct DeltaScanArgs {
 // multiply-add and the write, not the loads.  k . q is summed over the same lanes beside the two read-outs.
 // CPT: value columns a thread holds (its group's column and the one `groups` further on): two columns are two
 // chains whose waits overlap; a step of single tokens keeps one, so that its CTAs stay many.
-template <typename T, int KPL, int L, int CPT, bool ASYNC>
+// SHORT: only rows with fewer than `below` tokens (a form of its own, so that the other's loads do not wait for a row's length).
+template <typename T, int KPL, int L, int CPT, bool ASYNC, bool SHORT>
 __global__ void __launch_bounds__(DS_THREADS) delta_scan_kernel(const DeltaScanArgs a) {
   extern __shared__ __align__(16) float ds_smem[];
   constexpr int RUN = KPL + 4, DP = L * RUN;      // a lane's run and a token's row in shared memory
@@ -131,7 +132,7 @@ __global__ void __launch_bounds__(DS_THREADS) delta_scan_kernel(const DeltaScanA
     return;
   }
   const int t0 = a.row_q_start[row], n = a.row_q_len[row];
-  if (a.below > 0 && n >= a.below) return;
+  if (SHORT && n >= a.below) return;
   const int l = threadIdx.x % L, my_group = threadIdx.x / L;
   const int group = head / a.heads_per_group, qk_heads = a.heads / a.heads_per_group;
   // A thread's CPT columns are separate chains: one column's exchanges and writes run under the other's sums.
@@ -715,13 +716,13 @@ ZB_API int zb_delta_gates(float* q_out, float* k_out, float* beta, float* decay,
   return launch_result();
 }
 
-template <typename T, int KPL, int L, int CPT>
+template <typename T, int KPL, int L, int CPT, bool SHORT>
 static int delta_scan_launch(const DeltaScanArgs& a, int rows, cudaStream_t s) {
   constexpr int cols = DS_THREADS / L * CPT;
   const size_t smem = 2 * sizeof(float) * (2 * DS_TOKENS * L * (KPL + 4) + DS_TOKENS * cols + 2 * DS_TOKENS);
   const bool async = a.D % 4 == 0 && reinterpret_cast<uintptr_t>(a.q) % 16 == 0 && reinterpret_cast<uintptr_t>(a.k) % 16 == 0 &&
                      reinterpret_cast<uintptr_t>(a.state) % 16 == 0 && a.slot_stride % 4 == 0;
-  auto kernel = async ? delta_scan_kernel<T, KPL, L, CPT, true> : delta_scan_kernel<T, KPL, L, CPT, false>;
+  auto kernel = async ? delta_scan_kernel<T, KPL, L, CPT, true, SHORT> : delta_scan_kernel<T, KPL, L, CPT, false, SHORT>;
   if (smem > 48 * 1024 &&
       cuda_failed(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem))))
     return ERR_CUDA;
@@ -734,7 +735,8 @@ static int delta_scan_columns(const DeltaScanArgs& a, int rows, int tokens, cuda
   // Two columns a thread where requests bring runs of tokens (the chains hide each other's waits) and a head has
   // columns enough; one where a step is single tokens, whose time is the state's bytes.
   const bool runs = tokens >= 4 * rows && a.V >= 2 * (DS_THREADS / L);
-  return runs ? delta_scan_launch<T, KPL, L, 2>(a, rows, s) : delta_scan_launch<T, KPL, L, 1>(a, rows, s);
+  if (a.below > 0) return delta_scan_launch<T, KPL, L, 1, true>(a, rows, s);
+  return runs ? delta_scan_launch<T, KPL, L, 2, false>(a, rows, s) : delta_scan_launch<T, KPL, L, 1, false>(a, rows, s);
 }
 
 template <typename T>
