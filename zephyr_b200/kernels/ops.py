@@ -1634,14 +1634,15 @@ def paged_prefill(q: torch.Tensor, kv_cache: torch.Tensor, block_table: torch.Te
                   out: torch.Tensor, chunk: int = 0, sinks: torch.Tensor | None = None, softcap: float = 0.0,
                   keys_only: bool = False, keep_first: int = 0, pool: int = 0, pool_cache: torch.Tensor | None = None,
                   pool_table: torch.Tensor | None = None, cross_values: bool = False,
-                  by_group: bool = False,
-                  distance_bias: tuple[torch.Tensor, torch.Tensor] | None = None) -> torch.Tensor:
+                  by_group: bool = False, distance_bias: tuple[torch.Tensor, torch.Tensor] | None = None,
+                  tensor_memory: bool = True) -> torch.Tensor:
     """Tensor-core attention for rows with several new tokens, cut into tiles of
     ``paged_prefill_tile_tokens()``; writes those tokens' rows of ``out``.  ``chunk``, ``sinks``, ``softcap`` and
     ``distance_bias`` as in ``paged_attention``, ``keys_only`` as its ``shared_kv``.  Head size 128 runs on tcgen05
     with the accumulators in tensor memory, other sizes on mma.sync.  ``keep_first``, ``pool`` with its store, and
     ``cross_values`` (``out`` is then [T, nh * nkv * hd], bfloat16 or float32) as in ``paged_attention``: the last two, and
-    kept tokens or a chunk beside a distance bias, run on mma.sync.  ``by_group``: every
+    kept tokens or a chunk beside a distance bias, run on mma.sync, and so does everything without ``tensor_memory``.
+    ``by_group``: every
     tile is one new token (the tiles of single-token rows), and a CTA's query rows are the heads that share a
     key/value head: a decoded token's keys and values stream once a group."""
     _cuda(q, kv_cache, block_table, tile_row, tile_q0, row_q_start, row_q_len, row_ctx, status, out, pool_cache, pool_table)
@@ -1665,7 +1666,7 @@ def paged_prefill(q: torch.Tensor, kv_cache: torch.Tensor, block_table: torch.Te
                  and pool_cache.is_contiguous(), "a pooled store has the pages' shape and a table row per request")
         pool_pages, pool_blocks = pool_cache.shape[0], pool_table.shape[1]
     r1, r2 = _distance_bias(distance_bias, nh)
-    tensor_memory = (USE_TCGEN05_PREFILL and not (pool or cross_values or by_group or (keep_first and window <= 0))
+    tensor_memory = (tensor_memory and USE_TCGEN05_PREFILL and not (pool or cross_values or by_group or (keep_first and window <= 0))
                      and not ((softcap or keep_first or chunk) and r1 is not None)
                      and bool(library().zb_paged_prefill_tc_supported(nh, nkv, hd, DTYPE_CODE[q.dtype], page_size)))
     common = (_ptr(out), _ptr(q), _ptr(kv_cache), _ptr(block_table), block_table.shape[1], page_size, pages,
