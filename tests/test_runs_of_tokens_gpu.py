@@ -364,3 +364,24 @@ def test_what_a_row_gets_hangs_on_that_row_alone(cuda_device, kind):
         out, state = run([r])
         assert torch.equal(together[0][0][start:start + n], out), n
         assert torch.equal(together[0][1][r], state[r]), n
+
+
+@pytest.mark.parametrize("heads,dim,vdim", [(2, 64, 32), (5, 100, 130), (1, 8, 8)])
+def test_retention_walked_and_in_passes(cuda_device, heads, dim, vdim):
+    """The two forms that a layer chooses from by its state's size: the same rule, each operand two bfloat16 values."""
+    from zephyr_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(dim)
+    lengths, T = [64, 100, 7, 130], 301
+    q, k, v = (torch.randn(T, heads * n, generator=g).to(cuda_device) for n in (dim, dim, vdim))
+    i32 = lambda values: torch.tensor(values, dtype=torch.int32, device=cuda_device)
+    rows = (i32([1, 0, 3, 2]), i32([0, 64, 164, 171]), i32(lengths), ops.new_status(cuda_device))
+    decay, got = torch.full((heads,), 0.98, device=cuda_device), []
+    for walk in (True, False):
+        before, state = ops.LAUNCH_COUNTS.get("state_walk", 0), torch.ones(4, heads * dim * vdim, device=cuda_device)
+        got.append((ops.retention(q, k, v, decay, heads, dim, vdim, state, *rows, walk=walk), state))
+        assert ops.LAUNCH_COUNTS.get("state_walk", 0) - before == (2 if walk else 0)
+    ops.check_status(rows[-1])
+    # An operand is off by 2^-17 of itself at most in either form; sums of up to 130 products, of alternating signs.
+    for x, y in zip(*got):
+        assert (x - y).norm() <= 2.0 ** -15 * y.norm()

@@ -865,13 +865,14 @@ def retention_turns(q: torch.Tensor, k: torch.Tensor, key_dim: int, rot_dims: in
 def retention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, heads: int, key_dim: int, value_dim: int,
               state: torch.Tensor, slots: torch.Tensor, row_q_start: torch.Tensor, row_q_len: torch.Tensor,
               status: torch.Tensor, write_state: bool = True, freqs: torch.Tensor | None = None, rot_dims: int = 0,
-              k_scale: float = 1.0, positions: torch.Tensor | None = None) -> torch.Tensor:
+              k_scale: float = 1.0, positions: torch.Tensor | None = None, walk: bool = True) -> torch.Tensor:
     """What ``decayed_state_scan`` in its "fixed" mode does, in pieces of 64 tokens on the tensor cores: for rows that
     bring runs of tokens.  With ``freqs`` q and k are first turned by the tokens' ``positions`` as ``rotate_qk`` does, k times
     ``k_scale`` (``retention_turns``: whether that is taken).  q, k, v float32 [T, .] with unit inner stride, head h at column h * width; ``decay`` float32
     [heads]; ``state`` [slots, heads * key_dim * value_dim] float32 (rows may be strided).  Each operand of a product
-    is taken as two bfloat16 values.  Rows may lie in the stream in any order (heads of more than 128 key channels: one behind the
-    other, ``row_q_start`` ascending).  Returns o as float32 [T, heads * value_dim]."""
+    is taken as two bfloat16 values.  ``walk``: pieces one behind the other with the state on the SM (up to 128 key
+    channels; rows may then lie in the stream in any order); otherwise passes over all pieces at once (rows one behind the other,
+    ``row_q_start`` ascending).  Returns o as float32 [T, heads * value_dim]."""
     _cuda(q, k, v, decay, state, slots, row_q_start, row_q_len, status)
     _i32(slots, row_q_start, row_q_len)
     T = v.shape[0]
@@ -891,7 +892,8 @@ def retention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Te
         _f32_vector(freqs, rot_dims // 2, "the frequencies")
         _require(retention_turns(q, k, key_dim, rot_dims), "q and k of this shape are turned by rotate_qk")
         turn = (freqs, rot_dims, k_scale, positions)
-    if key_dim <= lib.zb_walk_max_channels():
+    _require(walk or turn is None, "q and k are turned on the way into the walk")
+    if walk and key_dim <= lib.zb_walk_max_channels():
         _state_walk(1, out, q, k, v, heads, key_dim, value_dim, state, slots, row_q_start, row_q_len, status, write_state, decay=decay,
                     turn=turn)
         return out

@@ -293,6 +293,17 @@ class Retention(Mixer):
     takes_out_dtype = True
 
     PIECES_FROM = 64      # new tokens per request, on average, from which on a step runs in pieces
+    # A step's pieces are walked one behind the other with the state on the SM, or in passes over all pieces at once.  The walk
+    # takes 1.75 us a piece of the longest row; 2.4 us a piece of the two longest where its CTAs of 16 value columns are nearly two
+    # an SM, which run in turn; 2.7 us in CTAs of 32, where they would be more.  The passes take 1.66 ns a token and 128 x 128
+    # values of state, and 10 us, more than the walk beside that (one row of 1024 tokens: 16 heads of 128 x 128: 44 us walked, 51 in
+    # passes; 5 of 100 x 130: 48 and 29; 2 of 64 x 32: 31 and 18; one row of 256, 2 of 64 x 32: 16 and 17; the layer with a row of
+    # 1500 beside ten single tokens, 16 heads: 186 and 162, with rows of 700 and 400: 110 and 104).
+    def _walks(self, ctx: StepContext) -> bool:
+        lengths = sorted(ctx.host_q_len or [ctx.num_tokens])
+        ctas = ctx.num_rows * self.heads * -(-self.vdim // 16)
+        walked = (1.75 * lengths[-1] if ctas <= 1.5 * 148 else 2.4 * sum(lengths[-2:]) if ctas <= 2 * 148 else 2.7 * lengths[-1]) / 64
+        return walked <= 10.0 + 1.66e-3 * ctx.num_tokens * self.heads * (self.dim * self.vdim / 128 ** 2)
 
     def __init__(self, spec: MixerSpec, weights: Mapping[str, torch.Tensor], dtype: torch.dtype,
                  device: torch.device | str):
@@ -348,14 +359,14 @@ class Retention(Mixer):
         # Runs of tokens in pieces on the tensor cores; short ones, and everything in true 32-bit, token by token.
         pieces = (self.dtype == torch.bfloat16 and x.shape[0] >= self.PIECES_FROM * ctx.num_rows
                   and self.dim <= ops.retention_max_channels())
-        turn = {}
-        if pieces and ops.retention_turns(q, k, self.dim, self.rot_dims):
+        walks, turn = pieces and self._walks(ctx), {}
+        if walks and ops.retention_turns(q, k, self.dim, self.rot_dims):
             turn = dict(freqs=self.freqs, rot_dims=self.rot_dims, k_scale=self.dim ** -0.5, positions=ctx.positions)
         else:
             turned = ops.rotate_qk(projected, self.heads, self.dim, self.freqs, self.rot_dims, self.dim ** -0.5, ctx.positions)
             q, k = turned[:, :hd], turned[:, hd:]
         if pieces:
-            o = ops.retention(q, k, v, self.decay, self.heads, self.dim, self.vdim, *where, write_state=call.writes_cache, **turn)
+            o = ops.retention(q, k, v, self.decay, self.heads, self.dim, self.vdim, *where, write_state=call.writes_cache, walk=walks, **turn)
         else:
             o = ops.decayed_state_scan("fixed", q, k, v, self.heads, self.dim, self.vdim, *where, decay=self.decay,
                                        write_state=call.writes_cache)
