@@ -210,11 +210,15 @@ class GatedDeltaRule(Mixer):
     takes_out_dtype = True
 
     UNIT_EPS = 1e-6      # inside the root of the unit norms of q and k: the design fixes it
-    # New tokens of a row from which on it runs in blocks.  Blocks shorten a row's chain and pay most where rows are few (16
-    # heads of 128 x 128, one row of 128 tokens: 27 us, 40 token by token; 2048: 240 and 522; 8 heads of 64 x 64, 128: 20 and
-    # 36).  Where the rows' own chains fill the SMs they are behind, least for long rows (8 rows of 128: 105 and 98; 32 rows of
-    # 64: 216 and 172), so the line lies above what a row alone would have it (24 tokens).
-    BLOCKS_FROM = 128
+    # New tokens of a row from which on it runs in blocks.  Blocks shorten a row's chain and pay where rows are few: 16 heads of
+    # 128 x 128, one row of 64 tokens: 19 us, 24 token by token; 2048: 239 and 520; 3 rows of 600: 199 and 244; 32 heads, one
+    # row of 2048: 420 and 559.  Where the rows' own chains fill the SMs they are behind (16 heads, 8 rows of 256: 201 and 185;
+    # 32 heads, 3 rows of 600: 375 and 326).  So in bfloat16 a step runs in blocks while their CTAs, 16 value columns each, are
+    # no more than one and a half times what the SMs hold at once, and rows of 64 to 191 tokens beside shorter ones, which
+    # take a launch of their own, stay with those (40, 3 and 90 tokens: 75 us, 87 in two launches).  In 32 bits the line looks at the row alone, so that a
+    # request's logits do not change with what shares its step; it lies where a few rows gain and many lose little (8 rows of
+    # 128: 105 and 98).
+    BLOCKS_FROM, ROW_BLOCKS_FROM, MOST_CTAS = 64, 128, 3 * 148
 
     def __init__(self, spec: MixerSpec, weights: Mapping[str, torch.Tensor], dtype: torch.dtype,
                  device: torch.device | str):
@@ -271,6 +275,13 @@ class GatedDeltaRule(Mixer):
         scan = int(p["heads"]) * int(p["key_dim"]) * int(p["value_dim"])
         return StateCacheSpec(shape=(scan + (int(p["conv"]) - 1) * channels,), dtype="float32")
 
+    def _blocks_from(self, ctx: StepContext) -> int:
+        if self.w_o.dtype == torch.float32 or not ctx.host_q_len:
+            return self.ROW_BLOCKS_FROM
+        limit = self.BLOCKS_FROM if min(ctx.host_q_len) >= self.BLOCKS_FROM else 3 * self.BLOCKS_FROM
+        rows = sum(n >= limit for n in ctx.host_q_len)
+        return limit if rows * self.heads * -(-self.vdim // 16) <= self.MOST_CTAS else ctx.num_tokens + 1
+
     def forward(self, x: torch.Tensor, ctx: StepContext, call: LayerCall,
                 out_dtype: torch.dtype | None = None) -> torch.Tensor:
         c, store = self.cuts, ctx.caches[call.cache]
@@ -283,7 +294,7 @@ class GatedDeltaRule(Mixer):
                            steps[:, self.heads:], self.a_log, self.dt_bias, self.heads, self.qk_heads, self.dim,
                            self.vdim, store[:, :self.scan_floats], ctx.state_slots, ctx.row_q_start, ctx.row_q_len,
                            ctx.status, q_scale=self.dim ** -0.5, unit_eps=self.UNIT_EPS, write_state=call.writes_cache,
-                           row_tokens=ctx.host_q_len or None, blocks_from=self.BLOCKS_FROM)
+                           row_tokens=ctx.host_q_len or None, blocks_from=self._blocks_from(ctx))
         normed = ops.gated_group_rms_norm(o, ops.linear(x, self.w_g), self.norm, self.vdim, self.eps, gate_first=False)
         return ops.linear(normed, self.w_o, out_dtype=out_dtype)
 
