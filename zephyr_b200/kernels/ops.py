@@ -187,10 +187,10 @@ _SIGNATURES = {
     "zb_paged_prefill_supported": [c_int, c_int, c_int, c_int],
     "zb_paged_prefill": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
                          c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p],
-    "zb_paged_prefill_tc_supported": [c_int, c_int, c_int, c_int, c_int],
+    "zb_paged_prefill_tc_supported": [c_int, c_int, c_int, c_int, c_int, c_int, c_int],
     "zb_paged_prefill_tc_set_trace": [c_void_p],
     "zb_paged_prefill_tc_masked": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
-                                   c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float,
+                                   c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float,
                                    c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
     "zb_paged_prefill_tc": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
                             c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p],
@@ -1637,11 +1637,12 @@ def paged_prefill(q: torch.Tensor, kv_cache: torch.Tensor, block_table: torch.Te
                   keys_only: bool = False, keep_first: int = 0, pool: int = 0, pool_cache: torch.Tensor | None = None,
                   pool_table: torch.Tensor | None = None, cross_values: bool = False,
                   by_group: bool = False, distance_bias: tuple[torch.Tensor, torch.Tensor] | None = None,
-                  tensor_memory: bool = True) -> torch.Tensor:
+                  tensor_memory: bool = True, value_dim: int = 0) -> torch.Tensor:
     """Tensor-core attention for rows with several new tokens, cut into tiles of
     ``paged_prefill_tile_tokens()``; writes those tokens' rows of ``out``.  ``chunk``, ``sinks``, ``softcap`` and
-    ``distance_bias`` as in ``paged_attention``, ``keys_only`` as its ``shared_kv``.  Head size 128 runs on tcgen05
-    with the accumulators in tensor memory, other sizes on mma.sync.  ``keep_first``, ``pool`` with its store, and
+    ``distance_bias`` as in ``paged_attention``, ``keys_only`` as its ``shared_kv``.  ``value_dim``: how many values of a row
+    of ``out`` the caller reads (0: all ``hd``); the others may stay as they are.  Head size 128, and with ``keys_only`` 160 of
+    which 128 are read, runs on tcgen05 with the accumulators in tensor memory, other sizes on mma.sync.  ``keep_first``, ``pool`` with its store, and
     ``cross_values`` (``out`` is then [T, nh * nkv * hd], bfloat16 or float32) as in ``paged_attention``: the last two, and
     kept tokens or a chunk beside a distance bias, run on mma.sync, and so does everything without ``tensor_memory``.
     ``by_group``: every
@@ -1670,12 +1671,14 @@ def paged_prefill(q: torch.Tensor, kv_cache: torch.Tensor, block_table: torch.Te
     r1, r2 = _distance_bias(distance_bias, nh)
     tensor_memory = (tensor_memory and USE_TCGEN05_PREFILL and not (pool or cross_values or by_group or (keep_first and window <= 0))
                      and not ((softcap or keep_first or chunk) and r1 is not None)
-                     and bool(library().zb_paged_prefill_tc_supported(nh, nkv, hd, DTYPE_CODE[q.dtype], page_size)))
+                     and (hd == 128 or not (keep_first or chunk or r1 is not None))
+                     and bool(library().zb_paged_prefill_tc_supported(nh, nkv, hd, value_dim or hd, int(keys_only), DTYPE_CODE[q.dtype],
+                                                                      page_size)))
     common = (_ptr(out), _ptr(q), _ptr(kv_cache), _ptr(block_table), block_table.shape[1], page_size, pages,
               block_table.shape[0], _ptr(tile_row), _ptr(tile_q0), tile_row.numel(), _ptr(row_q_start), _ptr(row_q_len),
               _ptr(row_ctx), nh, nkv, hd, int(window))
     if tensor_memory:
-        _check(library().zb_paged_prefill_tc_masked(*common, int(chunk), int(keep_first), float(scale), float(softcap), int(keys_only), _ptr(sinks),
+        _check(library().zb_paged_prefill_tc_masked(*common, value_dim or hd, int(chunk), int(keep_first), float(scale), float(softcap), int(keys_only), _ptr(sinks),
                                                     _ptr(r1), _ptr(r2), _ptr(status), _stream()), "paged_prefill_tc")
     elif windowed or r1 is not None:
         _check(library().zb_paged_prefill_windowed(*common, int(chunk), float(scale), float(softcap), int(keys_only),

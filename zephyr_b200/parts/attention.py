@@ -66,11 +66,6 @@ from .base import POSITION_ENCODINGS, Mixer, StepContext, lookup, register_mixer
 class Attention(Mixer):
     graph_safe = True
 
-    # New tokens a tile of 128, on average, from which on prompts under a chunk or a window with kept tokens run on tcgen05; below,
-    # most of a CTA's queries are padding, and the mma.sync kernel skips more of it (16/8 heads, new prompts: 30 of 20 tokens 49 us
-    # on tcgen05 and 26 there, 16 of 64 28 and 16, of 96 30 and 24, 16 of 128 24 and 26, one of 512 16 and 32).
-    MASKED_TILE_TOKENS = 112
-
     def __init__(self, spec: MixerSpec, weights: Mapping[str, torch.Tensor], dtype: torch.dtype,
                  device: torch.device | str):
         p = spec.params
@@ -366,7 +361,7 @@ class Attention(Mixer):
             prefill_done = True
             if tile_row.numel() > 0:
                 ops.paged_prefill(q, cache, table, tile_row, tile_q0, ctx.row_q_start, ctx.row_q_len, ctx.row_ctx, *common, out=out,
-                                  tensor_memory=not self.chunk or q.shape[0] >= self.MASKED_TILE_TOKENS * tile_row.numel(), **masks)
+                                  **masks)
         if decode_done and prefill_done:
             return out
         if self.float32_tiles:
@@ -428,8 +423,7 @@ class Attention(Mixer):
                                         single=True, max_context=ctx.max_decode_context)
                 elif tile_row.numel() > 0:
                     ops.paged_prefill(q, cache, table, tile_row, tile_q0, ctx.row_q_start, ctx.row_q_len, ctx.row_ctx,
-                                      *common, out=out, cross_values=mixed, by_group=by_group,
-                                      tensor_memory=q.shape[0] >= self.MASKED_TILE_TOKENS * tile_row.numel(), **masks)
+                                      *common, out=out, cross_values=mixed, by_group=by_group, **masks)
         else:
             tile_row, tile_q0 = ctx.tiles[(self.tile_tokens, "all")]
             ops.paged_attention(q, cache, table, tile_row, tile_q0, self.tile_tokens, ctx.row_q_start, ctx.row_q_len,

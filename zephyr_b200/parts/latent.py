@@ -164,7 +164,8 @@ class LatentAttention(Mixer):
         """Attention of the latent-space queries [T, heads * (rank + rot)] over the cached rows: rows with one
         new token on the split-context kernel, rows with several on a tensor-core prompt kernel, where
         those take this shape and type (the prompt kernels take more widths than the split-context one, and
-        then serve single tokens as well); whatever is left on the general kernel."""
+        then serve single tokens as well); whatever is left on the general kernel.  Of a head's values only the first
+        ``rank`` are read behind it; the tcgen05 prompt kernel leaves the others as they are."""
         out = torch.empty_like(q)
         common = (self.nh, 1, self.kw, 0, self.scale, ctx.status)
         decode_done = self.fast_decode and ctx.num_decode_rows > 0
@@ -179,14 +180,14 @@ class LatentAttention(Mixer):
             tile_row, tile_q0 = ctx.tiles[(self.prefill_tile_tokens, "all")]
             if tile_row.numel() > 0:
                 ops.paged_prefill(q, cache, table, tile_row, tile_q0, ctx.row_q_start, ctx.row_q_len, ctx.row_ctx,
-                                  *common, out=out, sinks=self.sinks, keys_only=True)
+                                  *common, out=out, sinks=self.sinks, keys_only=True, value_dim=self.rank)
             return out
         if self.fast_prefill:
             tile_row, tile_q0 = ctx.tiles[(self.prefill_tile_tokens, "multi")]
             prefill_done = True
             if tile_row.numel() > 0:
                 ops.paged_prefill(q, cache, table, tile_row, tile_q0, ctx.row_q_start, ctx.row_q_len, ctx.row_ctx,
-                                  *common, out=out, sinks=self.sinks, keys_only=True)
+                                  *common, out=out, sinks=self.sinks, keys_only=True, value_dim=self.rank)
         if decode_done and prefill_done:
             return out
         which = "multi" if decode_done else ("single" if prefill_done else "all")
