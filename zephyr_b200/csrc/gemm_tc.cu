@@ -41,9 +41,8 @@ constexpr int GT_EPI_PLAIN = 0;
 constexpr int GT_EPI_GELU = 4;             // the sums through the tanh form of GELU
 constexpr int GT_EPI_RELU_GATE = 3;        // the interface's code for the gated epilogue with max(gate, 0) in SiLU's place
 constexpr int GT_EPI_SWIGLU = 1;           // columns 16 j .. 16 j + 7 are gates, 16 j + 8 .. 16 j + 15 their ups
-constexpr int GT_EPI_SWIGLU_SCALED = 5;    // the same, both sums of a row times its scale first (GateForm::row_scale)
 constexpr int GT_EPI_RELU2 = 6;            // the square of max(sum, 0)
-constexpr int GT_EPI_BOUNDED_GATE = 7;     // the interface's code for the gated epilogue with the bounded gate (grouped products)
+constexpr int GT_EPI_BOUNDED_GATE = 7;     // the interface's code for the gated epilogue with the bounded gate
 constexpr int GT_EPI_FLOAT = 2;            // the sums as they are, float32 (logits)
 constexpr int GT_A_BYTES = GT_BM * GT_BK * 2;
 constexpr int GT_STAGING_BYTES = 32 * 128;  // an epilogue warp's 32 rows x 64 output columns on their way out; two a warp
@@ -63,9 +62,6 @@ struct GemmTcArgs {
   int M, N, K;
   int tiles_m, tiles;
   GateForm gate;                 // with the gated epilogue: what becomes of a gate sum and its up sum
-  const int* tile_group;         // null, or per tile of 128 rows the matrix of w (rows group * N .. + N) its rows take;
-                                 // a negative entry: the tile is not computed
-  int groups;                    // matrices stacked in w (1 without tile_group)
   int* status;
 };
 
@@ -84,16 +80,6 @@ __device__ __forceinline__ bool gt_wait(GemmTcShared& sh, unsigned long long* ba
   return false;
 }
 
-// x / (1 + e^-x) with the special-function unit's exp2 and reciprocal (relative error about 2^-21,
-// far inside the rounding to bfloat16 that follows): a thread has 128 of these to do per tile beside
-// the products of the next tile, and the exact forms take some fifty dependent instructions each.
-__device__ __forceinline__ float silu_fast(float x) {
-  float e, r;
-  asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(e) : "f"(-1.4426950408889634f * x));
-  asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(r) : "f"(1.0f + e));
-  return x * r;
-}
-
 // One box from shared memory to the matrix behind `map` at (x, y); x * element size is a multiple of 16
 // bytes.  Part of the thread's current bulk group.
 __device__ __forceinline__ void tiled_store_2d_s2g(const CUtensorMap* map, int x, int y, const void* smem_src) {
@@ -107,7 +93,7 @@ template <int N> __device__ __forceinline__ void bulk_wait_read() {
 }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory"); }
 
-__host__ __device__ constexpr bool gt_gated(int epilogue) { return epilogue == GT_EPI_SWIGLU || epilogue == GT_EPI_SWIGLU_SCALED; }
+__host__ __device__ constexpr bool gt_gated(int epilogue) { return epilogue == GT_EPI_SWIGLU; }
 
 // An epilogue warp's 32 rows of a tile (its TMEM lanes, accumulator columns tmem_row .. + BN) -> y:
 // the sums are read 32 columns at a time, the epilogue applied in float32, and groups of 64 output
@@ -122,8 +108,6 @@ __device__ __forceinline__ void write_out_rows(const CUtensorMap& y_map, unsigne
   constexpr int READS = GATED ? 4 : EPI == GT_EPI_FLOAT ? 1 : 2;
   constexpr int PIECES = 8 / READS;                                  // 16-byte pieces a read leaves
   constexpr int GROUP_COLUMNS = EPI == GT_EPI_FLOAT ? 32 : 64;       // output columns of a group
-  // (rows of a grouped product are whole tiles, so every row has its scale)
-  const float scale = EPI == GT_EPI_SWIGLU_SCALED ? __ldg(form.row_scale + row0 + lane) : 1.0f;
 #pragma unroll 1
   for (int group = 0; group < BN / (32 * READS); ++group) {
     const int out_col = (GATED ? n0 / 2 : n0) + group * GROUP_COLUMNS;
@@ -165,11 +149,7 @@ __device__ __forceinline__ void write_out_rows(const CUtensorMap& y_map, unsigne
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               if (GATED) {
-                float gate = __uint_as_float(v[16 * j + i]), up = __uint_as_float(v[16 * j + 8 + i]);
-                if (EPI == GT_EPI_SWIGLU_SCALED) {
-                  gate *= scale;
-                  up *= scale;
-                }
+                const float gate = __uint_as_float(v[16 * j + i]), up = __uint_as_float(v[16 * j + 8 + i]);
                 o[i] = (form.kind == GATE_RELU ? fmaxf(gate, 0.0f) : silu_fast(gate)) * up;
               } else if (EPI == GT_EPI_GELU) {
                 o[i] = gelu_tanh_fast(__uint_as_float(v[8 * j + i]));
@@ -234,8 +214,6 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tc_kernel(const __grid_con
       unsigned phase = 0;
       for (int tile = blockIdx.x; tile < a.tiles && !sh.failed; tile += gridDim.x) {
         const int m0 = (tile % a.tiles_m) * GT_BM, n0 = (tile / a.tiles_m) * BN;
-        const int group = a.tile_group != nullptr ? a.tile_group[tile % a.tiles_m] : 0;
-        if (group < 0) continue;            // every role skips the same tiles
         for (int kb = 0; kb < k_blocks; ++kb) {
           if (!gt_wait(sh, &sh.empty[stage], phase ^ 1)) {
             if (!sh.failed) report(a.status, STATUS_COPY_TIMEOUT, tile, kb);
@@ -245,7 +223,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tc_kernel(const __grid_con
           unsigned char* slot = ring + stage * Shape::STAGE_BYTES;
           mbar_arrive_expect_tx(&sh.full[stage], Shape::STAGE_BYTES);
           tiled_copy_2d_g2s(slot, &a.x_map, kb * GT_BK, m0, &sh.full[stage]);
-          tiled_copy_2d_g2s(slot + GT_A_BYTES, &a.w_map, kb * GT_BK, group * a.N + n0, &sh.full[stage]);
+          tiled_copy_2d_g2s(slot + GT_A_BYTES, &a.w_map, kb * GT_BK, n0, &sh.full[stage]);
           if (++stage == Shape::STAGES) {
             stage = 0;
             phase ^= 1;
@@ -259,7 +237,6 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tc_kernel(const __grid_con
       int stage = 0, acc = 0;
       unsigned phase = 0, acc_phase = 0;
       for (int tile = blockIdx.x; tile < a.tiles && !sh.failed; tile += gridDim.x) {
-        if (a.tile_group != nullptr && a.tile_group[tile % a.tiles_m] < 0) continue;
         if (!gt_wait(sh, &sh.acc_empty[acc], acc_phase ^ 1)) {
           if (!sh.failed) report(a.status, STATUS_BARRIER_TIMEOUT, tile, -1);
           sh.failed = 1;
@@ -298,7 +275,6 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tc_kernel(const __grid_con
     unsigned acc_phase = 0;
     for (int tile = blockIdx.x; tile < a.tiles && !sh.failed; tile += gridDim.x) {
       const int m0 = (tile % a.tiles_m) * GT_BM, n0 = (tile / a.tiles_m) * BN;
-      if (a.tile_group != nullptr && a.tile_group[tile % a.tiles_m] < 0) continue;
       if (!gt_wait(sh, &sh.acc_full[acc], acc_phase)) {
         if (!sh.failed) report(a.status, STATUS_BARRIER_TIMEOUT, tile, -3);
         sh.failed = 1;
@@ -344,52 +320,6 @@ constexpr int GP_STAGE_BYTES = 2 * GP_HALF_BYTES;
 constexpr int GP_STAGES = 6;
 constexpr int GP_SMEM_BYTES = GP_STAGES * GP_STAGE_BYTES + 8 * GT_STAGING_BYTES + 1024;
 constexpr int GP_TMEM_COLUMNS = 2 * GP_BN;
-
-__device__ __forceinline__ unsigned cluster_rank() {
-  unsigned r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-}
-// The address, in the cluster's window, of this CTA's shared-memory address `smem_address` in the CTA of rank `rank`.
-__device__ __forceinline__ unsigned in_cta_of_rank(unsigned smem_address, unsigned rank) {
-  unsigned r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(smem_address), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void mbar_arrive_in_cluster(unsigned cluster_address) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_address) : "memory");
-}
-// A tiled copy into this CTA's shared memory whose bytes are counted on a barrier of the pair's first CTA.
-__device__ __forceinline__ void tiled_copy_2d_g2s_pair(void* smem_dst, const CUtensorMap* map, int x, int y, unsigned bar_cluster_address) {
-  asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
-               ::"r"(smem_u32(smem_dst)), "l"(map), "r"(x), "r"(y), "r"(bar_cluster_address) : "memory");
-}
-__device__ __forceinline__ void tmem_alloc_pair(unsigned* smem_result, unsigned columns) {
-  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(smem_result)), "r"(columns) : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish_pair() {
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc_pair(unsigned address, unsigned columns) {
-  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(address), "r"(columns) : "memory");
-}
-__device__ __forceinline__ void tc_mma_pair(unsigned d_tmem, unsigned long long a_desc, unsigned long long b_desc,
-                                            unsigned idesc, unsigned accumulate) {
-  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-               ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-// One arrival on the barrier at this address in BOTH CTAs of the pair when every product issued so far is complete.
-__device__ __forceinline__ void tc_commit_pair(unsigned long long* bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n"
-               ::"r"(smem_u32(bar)), "h"(static_cast<unsigned short>(3)) : "memory");
-}
-// Instruction descriptor of the pair's product: as tc_idesc with M = 256.
-__host__ __device__ constexpr unsigned tc_idesc_pair(unsigned n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((256u >> 4) << 24);
-}
 
 template <int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GT_THREADS, 1) gemm_tc_pair_kernel(const __grid_constant__ GemmTcArgs a) {
@@ -524,7 +454,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GT_THREADS, 1) gemm_
 // boxes of 128 bytes (64 or 32 columns) x box_rows rows with the 128-byte swizzle.  Maps are kept: weights come back every step,
 // and so do the activations of a captured step.
 bool matrix_tensor_map(const void* base, long long rows, int cols, long long ld, int box_rows, CUtensorMap* out,
-                       int element_bytes = 2) {
+                       int element_bytes) {
   static std::mutex mutex;
   static std::map<std::tuple<const void*, long long, int, long long, int, int>, CUtensorMap> kept;
   std::lock_guard<std::mutex> lock(mutex);
@@ -553,7 +483,7 @@ bool matrix_tensor_map(const void* base, long long rows, int cols, long long ld,
 template <int BN, int EPI>
 int gemm_tc_launch(GemmTcArgs& a, const void* w, int sms, cudaStream_t stream) {
   using Shape = GemmTcShape<BN>;
-  if (!matrix_tensor_map(w, static_cast<long long>(a.N) * a.groups, a.K, a.K, BN, &a.w_map)) return ERR_CUDA;
+  if (!matrix_tensor_map(w, a.N, a.K, a.K, BN, &a.w_map, 2)) return ERR_CUDA;
   a.tiles_m = (a.M + GT_BM - 1) / GT_BM;
   a.tiles = a.tiles_m * ((a.N + BN - 1) / BN);
   if (cuda_failed(cudaFuncSetAttribute(gemm_tc_kernel<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::SMEM_BYTES)))
@@ -565,7 +495,7 @@ int gemm_tc_launch(GemmTcArgs& a, const void* w, int sms, cudaStream_t stream) {
 
 template <int EPI>
 int gemm_tc_pair_launch(GemmTcArgs& a, const void* w, int sms, cudaStream_t stream) {
-  if (!matrix_tensor_map(w, a.N, a.K, a.K, 128, &a.w_map)) return ERR_CUDA;
+  if (!matrix_tensor_map(w, a.N, a.K, a.K, 128, &a.w_map, 2)) return ERR_CUDA;
   a.tiles_m = (a.M + 255) / 256;
   a.tiles = a.tiles_m * ((a.N + GP_BN - 1) / GP_BN);
   if (cuda_failed(cudaFuncSetAttribute(gemm_tc_pair_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM_BYTES)))
@@ -621,10 +551,8 @@ static int gemm_tc_run(void* y, const void* x, const void* w, int M, int N, int 
   GemmTcArgs a;
   a.M = M; a.N = N; a.K = K;
   a.gate = gate;
-  a.tile_group = nullptr;
-  a.groups = 1;
   a.status = status;
-  if (!matrix_tensor_map(x, M, K, ldx, GT_BM, &a.x_map)) return ERR_CUDA;
+  if (!matrix_tensor_map(x, M, K, ldx, GT_BM, &a.x_map, 2)) return ERR_CUDA;
   if (!matrix_tensor_map(y, M, epilogue == GT_EPI_SWIGLU ? N / 2 : N, ldy, 32, &a.y_map, epilogue == GT_EPI_FLOAT ? 4 : 2)) return ERR_CUDA;
   const cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (block_n == GT_PAIR)
@@ -659,48 +587,4 @@ ZB_API int zb_gemm_tc_bounded(void* y, const void* x, const void* w, const float
   if (!(limit > 0.0f) || reinterpret_cast<uintptr_t>(bias) % 16 != 0) return ERR_BAD_ARGUMENT;
   return gemm_tc_run(y, x, w, M, N, K, ldx, ldy, GT_EPI_SWIGLU, GateForm{GATE_BOUNDED, bias, limit, alpha, shift, nullptr}, block_n,
                      status, stream);
-}
-
-// The same over several matrices stacked in w ([groups * N, K]): x [tiles_m * 128, K] is cut into tiles of
-// 128 rows, and tile i multiplies with matrix tile_group[i] (a device array; a negative entry leaves the
-// tile out, its rows of y unwritten).  Rows sorted by expert and padded to whole tiles make a routed
-// feed-forward's products one launch.  Tiles of one SM; epilogues as zb_gemm_tc (not 4 and
-// 6), and 7: the gated one with the bounded gate (`limit`, `alpha`, `shift`; no biases).  `row_scale`: null, or one float32
-// per row of x that goes on both sums of the gated epilogue (1 and 3).
-ZB_API int zb_gemm_tc_grouped(void* y, const void* x, const void* w, const int* tile_group, int tiles_m, int groups,
-                              int N, int K, long long ldx, int ldy, int epilogue, const float* row_scale, float limit,
-                              float alpha, float shift, int* status, void* stream) {
-  if (tiles_m <= 0 || groups <= 0 || tile_group == nullptr || epilogue == GT_EPI_GELU || epilogue == GT_EPI_RELU2)
-    return ERR_BAD_ARGUMENT;
-  const bool bounded = epilogue == GT_EPI_BOUNDED_GATE;
-  if (bounded && (row_scale != nullptr || !(limit > 0.0f))) return ERR_BAD_ARGUMENT;
-  const int M = tiles_m * GT_BM;
-  if (!zb_gemm_tc_supported(M, N, K, ldx, ldy, epilogue)) return ERR_UNSUPPORTED;
-  const int relu_gate = epilogue == GT_EPI_RELU_GATE;
-  if (relu_gate || bounded) epilogue = GT_EPI_SWIGLU;
-  if (reinterpret_cast<uintptr_t>(y) % 16 != 0 || reinterpret_cast<uintptr_t>(x) % 16 != 0 ||
-      reinterpret_cast<uintptr_t>(w) % 16 != 0)
-    return ERR_BAD_ARGUMENT;
-  int device = 0, sms = 0;
-  if (cuda_failed(cudaGetDevice(&device)) ||
-      cuda_failed(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device)))
-    return ERR_CUDA;
-  GemmTcArgs a;
-  a.M = M; a.N = N; a.K = K;
-  a.gate = bounded ? GateForm{GATE_BOUNDED, nullptr, limit, alpha, shift, nullptr} : plain_gate(relu_gate ? GATE_RELU : GATE_SILU);
-  a.gate.row_scale = row_scale;
-  a.tile_group = tile_group;
-  a.groups = groups;
-  a.status = status;
-  if (!matrix_tensor_map(x, M, K, ldx, GT_BM, &a.x_map)) return ERR_CUDA;
-  if (!matrix_tensor_map(y, M, epilogue == GT_EPI_SWIGLU ? N / 2 : N, ldy, 32, &a.y_map, epilogue == GT_EPI_FLOAT ? 4 : 2)) return ERR_CUDA;
-  const cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const bool wide = N >= 256;
-  if (epilogue == GT_EPI_FLOAT)
-    return wide ? gemm_tc_launch<256, GT_EPI_FLOAT>(a, w, sms, s) : gemm_tc_launch<128, GT_EPI_FLOAT>(a, w, sms, s);
-  if (epilogue == GT_EPI_SWIGLU && row_scale != nullptr)
-    return wide ? gemm_tc_launch<256, GT_EPI_SWIGLU_SCALED>(a, w, sms, s) : gemm_tc_launch<128, GT_EPI_SWIGLU_SCALED>(a, w, sms, s);
-  if (epilogue == GT_EPI_SWIGLU)
-    return wide ? gemm_tc_launch<256, GT_EPI_SWIGLU>(a, w, sms, s) : gemm_tc_launch<128, GT_EPI_SWIGLU>(a, w, sms, s);
-  return wide ? gemm_tc_launch<256, GT_EPI_PLAIN>(a, w, sms, s) : gemm_tc_launch<128, GT_EPI_PLAIN>(a, w, sms, s);
 }

@@ -233,41 +233,69 @@ align_kernel(int* plan, int* slots, int* place_of_slot, const int* ids, int num_
   }
 }
 
-// The same for products that run as one grouped launch of the tcgen05 kernel (gemm_tc.cu): every expert's
-// run begins on a multiple of `tile_rows` places, tile_group[i] names the expert of tile i (-1: unused),
-// and slots[place] is -1 where a place pads a run.
+// The same for products that run as one launch of the tcgen05 kernel (gemm_tc_experts.cu): an expert's tokens are cut into runs
+// of up to `run` places of equal length (a multiple of 16), plan[0] is the number of runs, plan[1 + 3 i ...] run i's expert,
+// first place and places that count, and slots[place] is -1 where a place pads a run.
 __global__ void __launch_bounds__(ALIGN_THREADS)
-align_padded_kernel(int* tile_group, int* slots, int* place_of_slot, const int* ids, int num_slots, int experts,
-                    int max_tiles, int tile_rows) {
+align_runs_kernel(int* plan, int* slots, int* place_of_slot, const int* ids, int num_slots, int experts, int max_runs, int run, int places) {
   extern __shared__ int align_smem[];
   int* count = align_smem;                 // [experts]
-  int* start = count + experts;            // [experts + 1]
-  int* fill = start + experts + 1;         // [experts]
+  int* start = count + experts;            // [experts]
+  int* fill = start + experts;             // [experts]
+  const int lane = threadIdx.x & 31;
   for (int e = threadIdx.x; e < experts; e += blockDim.x) count[e] = fill[e] = 0;
-  for (int i = threadIdx.x; i < max_tiles * tile_rows; i += blockDim.x) slots[i] = -1;
+  for (int i = threadIdx.x; i < places; i += blockDim.x) slots[i] = -1;
   __syncthreads();
-  for (int i = threadIdx.x; i < num_slots; i += blockDim.x) {
-    const int e = ids[i];
-    if (e >= 0 && e < experts) atomicAdd(&count[e], 1);
+  // One addition a warp and expert that occurs in it.
+  auto add = [&](int* to, int e, bool valid) {
+    const unsigned same = __match_any_sync(0xffffffffu, valid ? e : -1);
+    const int first = __ffs(same) - 1;
+    int before = 0;
+    if (valid && lane == first) before = atomicAdd(&to[e], __popc(same));
+    return __shfl_sync(0xffffffffu, before, first) + __popc(same & ((1u << lane) - 1));
+  };
+  for (int i0 = 0; i0 < num_slots; i0 += blockDim.x) {
+    const int i = i0 + threadIdx.x, e = i < num_slots ? ids[i] : -1;
+    add(count, e, e >= 0 && e < experts);
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int tiles = 0;
-    for (int e = 0; e < experts; ++e) {
-      start[e] = tiles * tile_rows;
-      for (int r = 0; r < count[e] && tiles < max_tiles; r += tile_rows) tile_group[tiles++] = e;
+  auto length_of = [&](int n) {            // of an expert's runs: n places in as few as it takes, all alike
+    const int pieces = (n + run - 1) / run;
+    return n > 0 ? ((n + pieces - 1) / pieces + 15) / 16 * 16 : 0;
+  };
+  if (threadIdx.x < 32) {
+    int runs = 0, first_place = 0;
+    for (int e0 = 0; e0 < experts; e0 += 32) {
+      const int e = e0 + lane, n = e < experts ? count[e] : 0, length = length_of(n), pieces = n > 0 ? (n + length - 1) / length : 0;
+      int runs_end = pieces, places_end = pieces * length;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int r = __shfl_up_sync(0xffffffffu, runs_end, o), p = __shfl_up_sync(0xffffffffu, places_end, o);
+        if (lane >= o) {
+          runs_end += r;
+          places_end += p;
+        }
+      }
+      const int at = runs + runs_end - pieces, place = first_place + places_end - pieces * length;
+      if (e < experts) start[e] = place;
+      for (int p = 0; p < pieces && at + p < max_runs; ++p) {
+        plan[1 + 3 * (at + p)] = e;
+        plan[2 + 3 * (at + p)] = place + p * length;
+        plan[3 + 3 * (at + p)] = min(length, n - p * length);
+      }
+      runs += __shfl_sync(0xffffffffu, runs_end, 31);
+      first_place += __shfl_sync(0xffffffffu, places_end, 31);
     }
-    for (; tiles < max_tiles; ++tiles) tile_group[tiles] = -1;
+    if (lane == 0) plan[0] = min(runs, max_runs);
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < num_slots; i += blockDim.x) {
-    const int e = ids[i];
-    int place = -1;
-    if (e >= 0 && e < experts) {
-      place = start[e] + atomicAdd(&fill[e], 1);
-      slots[place] = i;
-    }
-    place_of_slot[i] = place;
+  for (int i0 = 0; i0 < num_slots; i0 += blockDim.x) {
+    const int i = i0 + threadIdx.x, e = i < num_slots ? ids[i] : -1;
+    const bool valid = e >= 0 && e < experts;
+    const int nth = add(fill, e, valid);
+    const int place = valid ? start[e] + nth : -1;      // (an expert's runs lie one behind the other, without gaps between them)
+    if (place >= 0 && place < places) slots[place] = i;
+    if (i < num_slots) place_of_slot[i] = place;
   }
 }
 
@@ -585,13 +613,15 @@ ZB_API int zb_expert_product(void* out, const void* x, long long x_stride, const
   return launch_result();
 }
 
-ZB_API int zb_route_align_padded(int* tile_group, int* slots, int* place_of_slot, const int* ids, int num_slots,
-                                 int experts, int max_tiles, int tile_rows, void* stream) {
-  if (num_slots < 0 || experts <= 0 || max_tiles <= 0 || tile_rows <= 0) return ERR_BAD_ARGUMENT;
-  const size_t smem = (3 * static_cast<size_t>(experts) + 1) * sizeof(int);
+// `max_runs` >= num_slots / run + experts, `places` >= num_slots + 16 max_runs.
+ZB_API int zb_route_align_runs(int* plan, int* slots, int* place_of_slot, const int* ids, int num_slots, int experts, int max_runs,
+                               int run, int places, void* stream) {
+  if (num_slots < 0 || experts <= 0 || run <= 0 || run % 16 != 0 || max_runs < num_slots / run + experts || places < num_slots + 16 * max_runs)
+    return ERR_BAD_ARGUMENT;
+  const size_t smem = 3 * static_cast<size_t>(experts) * sizeof(int);
   if (smem > 48 * 1024) return ERR_UNSUPPORTED;
-  align_padded_kernel<<<1, ALIGN_THREADS, smem, static_cast<cudaStream_t>(stream)>>>(tile_group, slots, place_of_slot, ids,
-                                                                                       num_slots, experts, max_tiles, tile_rows);
+  align_runs_kernel<<<1, ALIGN_THREADS, smem, static_cast<cudaStream_t>(stream)>>>(plan, slots, place_of_slot, ids, num_slots, experts,
+                                                                                     max_runs, run, places);
   return launch_result();
 }
 

@@ -5,6 +5,7 @@
 
 #include "common.cuh"
 #include "mma.cuh"
+#include "tma.cuh"
 
 namespace zb {
 
@@ -113,6 +114,53 @@ __device__ __forceinline__ unsigned long long desc_k_major(unsigned smem_address
 // B MN-major if asked (bit 16), N >> 3 in 17..22, M >> 4 in 24..28.  M is 128.
 __host__ __device__ constexpr unsigned tc_idesc(bool b_mn_major, unsigned n = 128) {
   return (1u << 4) | (1u << 7) | (1u << 10) | (b_mn_major ? (1u << 16) : 0u) | ((n >> 3) << 17) | ((128u >> 4) << 24);
+}
+
+// ---- Pairs of SMs: a cluster of two CTAs, whose tensor cores work on one product (cta_group::2)
+__device__ __forceinline__ unsigned cluster_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+// The address, in the cluster's window, of this CTA's shared-memory address `smem_address` in the CTA of rank `rank`.
+__device__ __forceinline__ unsigned in_cta_of_rank(unsigned smem_address, unsigned rank) {
+  unsigned r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(smem_address), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void mbar_arrive_in_cluster(unsigned cluster_address) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_address) : "memory");
+}
+// A tiled copy into this CTA's shared memory whose bytes are counted on a barrier of the pair's first CTA.
+__device__ __forceinline__ void tiled_copy_2d_g2s_pair(void* smem_dst, const CUtensorMap* map, int x, int y, unsigned bar_cluster_address) {
+  asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
+               ::"r"(smem_u32(smem_dst)), "l"(map), "r"(x), "r"(y), "r"(bar_cluster_address) : "memory");
+}
+__device__ __forceinline__ void tmem_alloc_pair(unsigned* smem_result, unsigned columns) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(smem_result)), "r"(columns) : "memory");
+}
+__device__ __forceinline__ void tmem_relinquish_pair() {
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(unsigned address, unsigned columns) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(address), "r"(columns) : "memory");
+}
+__device__ __forceinline__ void tc_mma_pair(unsigned d_tmem, unsigned long long a_desc, unsigned long long b_desc,
+                                            unsigned idesc, unsigned accumulate) {
+  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+               ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+}
+// One arrival on the barrier at this address in BOTH CTAs of the pair when every product issued so far is complete.
+__device__ __forceinline__ void tc_commit_pair(unsigned long long* bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n"
+               ::"r"(smem_u32(bar)), "h"(static_cast<unsigned short>(3)) : "memory");
+}
+// Instruction descriptor of the pair's product: as tc_idesc with M = 256.
+__host__ __device__ constexpr unsigned tc_idesc_pair(unsigned n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((256u >> 4) << 24);
 }
 
 }  // namespace zb

@@ -82,9 +82,10 @@ _SIGNATURES = {
     "zb_route_align": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     "zb_expert_product": [c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
                           c_int, c_int, c_int, c_float, c_float, c_float, c_int, c_int, c_void_p],
-    "zb_route_align_padded": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
+    "zb_route_align_runs": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p],
     "zb_gather_places": [c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p],
-    "zb_gemm_tc_grouped": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_longlong, c_int, c_int,
+    "zb_gemm_tc_experts_run": [c_int, c_int],
+    "zb_gemm_tc_experts": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_longlong, c_longlong, c_int,
                            c_void_p, c_float, c_float, c_float, c_void_p, c_void_p],
     "zb_route_combine": [c_void_p, c_void_p, c_longlong, c_int, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_int,
                          c_int, c_int, c_int, c_void_p],
@@ -2060,10 +2061,6 @@ def route(logits: torch.Tensor, correction: torch.Tensor | None, top: int, score
     return ids, weights
 
 
-GROUPED_TILE_ROWS = 128        # rows of a tile of the tcgen05 product
-GROUPED_MIN_ROWS_PER_EXPERT = 0    # the grouped tcgen05 products from this many choices per expert on (on average)
-
-
 def interleave_gate_up(w_gate: torch.Tensor, w_up: torch.Tensor) -> torch.Tensor:
     """[E, ff, width] twice -> [E, 2 ff, width] in blocks of 8 gate rows each followed by its 8 up rows
     (ff a multiple of 8): the layout whose product can apply act(gate) * up where the sums leave the tensor
@@ -2082,8 +2079,8 @@ def routed_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w_
     nothing comes back to the host: alignment, the two products (gate/up with the activation, down) and the
     weighted sum.  ``weigh_inputs``: sum_j expert_{ids[t, j]}(weights[t, j] x[t]) instead (the gate and up sums
     are multiplied by the weight ahead of the activation; no identity experts).  ``bounded`` (without biases): the
-    bounded gate of the unrounded gate and up sums in the activation's place.  bfloat16 with many tokens per expert and the interleaved layout: each product is ONE
-    grouped launch of the tcgen05 kernel over runs padded to whole tiles; otherwise tiles on mma.sync
+    bounded gate of the unrounded gate and up sums in the activation's place.  bfloat16 with the interleaved layout: each product is ONE
+    launch of a tcgen05 kernel over runs of an expert's tokens; otherwise tiles on mma.sync
     (bfloat16) or CUDA cores (float32)."""
     _cuda(x, ids, weights, w_gate, w_up, w_down)
     T, width = x.shape
@@ -2108,27 +2105,27 @@ def routed_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w_
     code = DTYPE_CODE[x.dtype]
     out = torch.empty((T, width), dtype=x.dtype, device=device)
     place = torch.empty(max(num_slots, 1), dtype=torch.int32, device=device)
-    grouped = (USE_GROUPED_TCGEN05 and interleaved and x.dtype == torch.bfloat16 and width % 8 == 0 and x.stride(0) % 8 == 0
-               and num_slots >= GROUPED_MIN_ROWS_PER_EXPERT * E)
+    grouped = (USE_GROUPED_TCGEN05 and interleaved and x.dtype == torch.bfloat16 and width % 8 == 0 and x.stride(0) % 8 == 0)
     if grouped:
-        tiles = -(-num_slots // GROUPED_TILE_ROWS) + E
-        places = tiles * GROUPED_TILE_ROWS
-        tile_group = torch.empty(tiles, dtype=torch.int32, device=device)
+        run = lib.zb_gemm_tc_experts_run(num_slots, E)
+        runs = num_slots // run + E
+        places = num_slots + 16 * runs
+        plan = torch.empty(1 + 3 * runs, dtype=torch.int32, device=device)
         slots = torch.empty(places, dtype=torch.int32, device=device)
-        _check(lib.zb_route_align_padded(_ptr(tile_group), _ptr(slots), _ptr(place), _ptr(ids), num_slots, E, tiles,
-                                         GROUPED_TILE_ROWS, _stream()), "route_align")
+        _check(lib.zb_route_align_runs(_ptr(plan), _ptr(slots), _ptr(place), _ptr(ids), num_slots, E, runs, run, places, _stream()),
+               "route_align")
         rows = torch.empty((places, width), dtype=x.dtype, device=device)
         place_scale = torch.empty(places, dtype=torch.float32, device=device) if weigh_inputs else None
         _check(lib.zb_gather_places(_ptr(rows), _ptr(x), x.stride(0), _ptr(slots), places, width, top, _ptr(place_scale),
                                     _ptr(weights), _stream()), "gather_places")
         status = device_status(device)
         hidden = torch.empty((places, ff), dtype=x.dtype, device=device)
-        _check(lib.zb_gemm_tc_grouped(_ptr(hidden), _ptr(rows), _ptr(w_gate), _ptr(tile_group), tiles, E, 2 * ff, width, width,
-                                      ff, (1, 3, 7)[act_code], _ptr(place_scale), *bounds, _ptr(status), _stream()), "gemm_tc_grouped")
+        _check(lib.zb_gemm_tc_experts(_ptr(hidden), _ptr(rows), _ptr(w_gate), _ptr(plan), runs, run, places, E, 2 * ff, width, width, ff,
+                                      1 + act_code, _ptr(place_scale), *bounds, _ptr(status), _stream()), "gemm_tc_grouped")
         # An expert's output takes the model's type before it is weighted on every path: here the product writes it so.
         ldy = width
         y = torch.empty((places, ldy), dtype=x.dtype, device=device)
-        _check(lib.zb_gemm_tc_grouped(_ptr(y), _ptr(hidden), _ptr(w_down), _ptr(tile_group), tiles, E, width, ff, ff, ldy, 0,
+        _check(lib.zb_gemm_tc_experts(_ptr(y), _ptr(hidden), _ptr(w_down), _ptr(plan), runs, run, places, E, width, ff, ff, ldy, 0,
                                       None, *bounds, _ptr(status), _stream()), "gemm_tc_grouped")
     else:
         tile_rows = lib.zb_expert_tile_rows(code)          # CUDA-core tiles in float32, tensor-core tiles in bfloat16
