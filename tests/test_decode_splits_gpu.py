@@ -1,0 +1,48 @@
+"""How a decode step cuts its contexts: the same attention whether a context is one item or many, at the edges of tiles and of the
+rule's lines."""
+
+import math
+
+import pytest
+import torch
+
+from test_kernels_gpu import build_paged_case, ops  # noqa: F401  (ops: a fixture)
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rows,nkv,context,whole", [(1, 8, 256, True), (1, 8, 288, False), (8, 8, 2208, True), (8, 8, 2240, False),
+                                                    (12, 8, 4096, True), (12, 8, 4097, False), (37, 4, 100, True), (40, 4, 100, False)])
+def test_the_rule(ops, cuda_device, rows, nkv, context, whole):
+    if ops._sm_count() != 148:
+        pytest.skip("lines of a GPU with 148 SMs")
+    split = ops.decode_split_size(rows, nkv, context)
+    assert (split >= context) == whole
+    assert split % 32 == 0
+
+
+@pytest.mark.parametrize("nh,nkv,ctx,window,sink", [
+    (16, 8, [0, 31, 32, 33, 300, 1, 63, 64], 0, False), (16, 8, [169] * 9 + [5, 511], 0, True),
+    (8, 2, [1000, 3, 77, 500, 31, 32, 900, 12, 13, 14, 15, 16, 17, 18, 19, 20, 21, 22, 23, 24], 0, False),
+    (16, 8, [700, 699, 20, 64, 65, 66, 67], 100, False)])
+def test_whole_contexts(ops, cuda_device, nh, nkv, ctx, window, sink):
+    hd, n = 128, len(ctx)
+    q, cache, meta, Ks, Vs, qs = build_paged_case(cuda_device, torch.bfloat16, nh, nkv, hd, 16, [1] * n, ctx, 500)
+    rows, sinks = torch.arange(n, dtype=torch.int32, device=cuda_device), torch.linspace(-1, 2, nh, device=cuda_device) if sink else None
+    status = ops.new_status(cuda_device)
+    assert ops.decode_split_size(n, nkv, max(ctx) + 1, min(max(ctx) + 1, window or 1 << 30)) >= max(ctx) + 1        # one item each
+    got = {}
+    for split in (None, 0, 128):
+        got[split] = ops.paged_decode(q, cache, meta["table"], rows, meta["row_q_start"], meta["row_ctx"], max(ctx) + 1, nh, nkv, hd, window,
+                                      1 / math.sqrt(hd), status, torch.full_like(q, float("nan")), split_size=split, sinks=sinks)
+    ops.check_status(status)
+    for r in range(n):
+        lo = max(0, ctx[r] + 1 - window) if window else 0
+        for h in range(nh):
+            s = qs[r][0, h].double() @ Ks[r][lo:, h // (nh // nkv)].double().T / math.sqrt(hd)
+            if sink:
+                s = torch.cat([s, sinks[h].cpu().double().view(1)])
+            expected = torch.softmax(s, -1)[:ctx[r] + 1 - lo] @ Vs[r][lo:, h // (nh // nkv)].double()
+            # Weights and the result are rounded to bfloat16, 2^-9 each of values up to four.
+            for split in got:
+                assert (got[split][r].double().cpu().view(nh, hd)[h] - expected).abs().max() <= 3.2e-2, (split, r, h)

@@ -1470,15 +1470,27 @@ def _decode_workspace(device: torch.device, floats: int, counters: int) -> tuple
     return scratch, count
 
 
-def decode_split_size(n_rows: int, nkv: int, max_context: int) -> int:
-    """A size for fixed splits (``paged_decode(..., split_size=...)``): as many splits of a row's
-    context as give every SM one item and none two (a second round of items would leave most SMs
-    idle), and no split shorter than 128 positions.  ``paged_decode`` takes fixed splits for a
-    handful of rows (4 * rows * key/value heads <= SMs); for more, the kernel spreads the tiles of
-    all rows evenly over its CTAs.  Either way, where a row's context is cut, and with that the last
-    bits of its result, depends on how many rows are decoded beside it."""
-    per_pair = max(1, _sm_count() // max(1, n_rows * nkv))     # splits of a (row, key/value head) pair: one item per SM
-    split = -(-max_context // per_pair)
+def decode_split_size(n_rows: int, nkv: int, max_context: int, visible: int | None = None, position_bytes: int = 512) -> int:
+    """How a launch of ``paged_decode`` cuts its rows' contexts: a size for fixed splits, or 0 for balanced items (the tiles of all
+    rows spread evenly over the CTAs).  ``visible``: how much of a context a query sees at most (default: all of it).
+
+    One item a (row, key/value head) pair, no split at all, while every pair has an SM and the longest context is the shorter way:
+    a CTA streams 128-value heads at 7.9 ns a position behind 3.2 us, all of them together at the copy rate, and cutting a context
+    costs 2 us (a handful of pairs, in fixed splits) to 6 us (balanced, where a CTA's share straddles two pairs) for the merge.
+    (us, cut as below / not at all: 1 row of 160 positions 6.0 / 4.6, and of 310, though 6.4 / 5.8 back to back, 10.7 / 11.2 in a
+    step; 8 rows of 310 9.7 / 6.2, of 600 13.2 / 8.2, of 2000 20.6 / 21.0, of 2620 22.7 / 26; 12 rows of 170 12.9 / 6.9, of 1500
+    21.8 / 19.4; 16 rows of 170 8.6 / 7.9; 18 of 2500 38.6 / 33.9.)
+    Else, for a handful of rows (4 * pairs <= SMs), as many splits of a row's context as give every SM one item and none two (a
+    second round of items would leave most SMs idle), and no split shorter than 128 positions.  For more, balanced items.
+    Where a row's context is cut, and with that the last bits of its result, depends on how many rows are decoded beside it."""
+    sms, pairs = _sm_count(), max(1, n_rows * nkv)
+    few = pairs * 4 <= sms
+    ns = (7.9 - 0.079 * pairs) * position_bytes / 512          # what a position costs a CTA more than it costs them all together
+    if pairs <= sms and max_context <= 4096 and (visible or max_context) * ns <= (1900.0 if few else 6300.0):
+        return max(32, -(-max_context // 32) * 32)
+    if not few:
+        return 0
+    split = -(-max_context // (sms // pairs))
     return max(128, -(-split // 32) * 32)
 
 
@@ -1507,18 +1519,17 @@ def paged_decode(q: torch.Tensor, kv_cache: torch.Tensor, block_table: torch.Ten
 
     ``max_context`` is at least the longest context of the rows, the new token included.  ``scratch``
     (float32, any contents) and ``counters`` (int32, zero) come from a process-wide workspace unless
-    given.  ``split_size`` None or 0: balanced work items; a multiple of 32: fixed splits of that size."""
+    given.  ``split_size`` None: chosen (``decode_split_size``); 0: balanced work items; a multiple of 32: fixed splits of that size."""
     _cuda(q, kv_cache, block_table, rows, row_q_start, row_ctx, status, out)
     _i32(block_table, rows, row_q_start, row_ctx)
     _require(q.dim() == 2 and q.is_contiguous() and q.shape[1] == nh * hd and q.dtype == torch.bfloat16, "q shape")
     _require(out.shape == q.shape and out.dtype == q.dtype and out.is_contiguous(), "out must match q")
     pages, page_size = _cache_geometry(kv_cache, nkv, hd, 0, q.dtype) if keys_only else _check_cache(kv_cache, nkv, hd, q.dtype)
     n_rows = rows.numel()
-    if split_size is None and n_rows * nkv * 4 <= _sm_count():
-        # A handful of long rows: fixed splits keep every item inside one row (a CTA whose share
-        # straddles two rows pays for two merges, which shows when the shares are a few tiles).
-        split_size = decode_split_size(n_rows, nkv, max_context)
-    if split_size is None or split_size == 0:
+    if split_size is None:
+        visible = min([max_context] + [n for n in (window, chunk) if n > 0])
+        split_size = decode_split_size(n_rows, nkv, max_context, visible, (2 if keys_only else 4) * hd)
+    if split_size == 0:
         # Balanced items: the tiles of all rows spread evenly over the CTAs (see attention_decode.cu).
         split_size, max_splits = 0, max(1, math.ceil(max_context / 32))
         need = int(library().zb_paged_decode_balanced_scratch_floats(nh, nkv, hd))
@@ -1580,9 +1591,9 @@ def paged_decode_fused(qkv: torch.Tensor, kv_cache: torch.Tensor, block_table: t
                  and cos.is_contiguous() and sin.is_contiguous(), "cos/sin must be float32 [positions, head_dim/2]")
         max_positions = cos.shape[0]
     n_rows = rows.numel()
-    if split_size is None and n_rows * nkv * 4 <= _sm_count():
-        split_size = decode_split_size(n_rows, nkv, max_context)
-    if split_size is None or split_size == 0:
+    if split_size is None:
+        split_size = decode_split_size(n_rows, nkv, max_context, min([max_context] + ([window] if window > 0 else [])), 4 * hd)
+    if split_size == 0:
         split_size, max_splits = 0, max(1, math.ceil(max_context / 32))
         need = int(library().zb_paged_decode_balanced_scratch_floats(nh, nkv, hd))
     else:
