@@ -48,6 +48,8 @@ template <> __device__ __forceinline__ void store_vec<__nv_bfloat16>(__nv_bfloat
 template <typename T, bool VECTOR>
 __global__ void embedding_kernel(T* __restrict__ out, const T* __restrict__ table, const int* __restrict__ ids,
                                  int H, int V, int* status) {
+  wait_for_prior_grids();
+  let_dependents_launch();
   const int t = blockIdx.x;
   const int id = ids[t];
   if (id < 0 || id >= V) {
@@ -70,6 +72,8 @@ __global__ void embedding_kernel(T* __restrict__ out, const T* __restrict__ tabl
 template <typename T, bool VECTOR>
 __global__ void gather_rows_kernel(T* __restrict__ out, const T* __restrict__ x, const int* __restrict__ rows,
                                    int H, int num_src_rows, int* status) {
+  wait_for_prior_grids();
+  let_dependents_launch();
   const int r = blockIdx.x;
   const int src_row = rows[r];
   if (src_row < 0 || src_row >= num_src_rows) {
@@ -95,6 +99,8 @@ template <typename T, bool ADD, bool VECTOR>
 __global__ void rmsnorm_kernel(T* __restrict__ out, T* __restrict__ x, const T* __restrict__ delta,
                                const void* __restrict__ w, int w_dtype, float eps, int H,
                                long long x_stride, long long out_stride) {
+  wait_for_prior_grids();
+  let_dependents_launch();
   __shared__ float scratch[33];
   T* xr = x + static_cast<size_t>(blockIdx.x) * x_stride;
   const T* dr = ADD ? delta + static_cast<size_t>(blockIdx.x) * x_stride : nullptr;
@@ -156,6 +162,8 @@ __global__ void __launch_bounds__(NORM_ROWS_PER_BLOCK * 32)
 rmsnorm_warp_rows_kernel(__nv_bfloat16* __restrict__ out, __nv_bfloat16* __restrict__ x,
                          const __nv_bfloat16* __restrict__ delta, const void* __restrict__ w, int w_dtype, float eps,
                          int rows, int H, long long x_stride, long long out_stride) {
+  wait_for_prior_grids();
+  let_dependents_launch();
   const int lane = threadIdx.x & 31, row = blockIdx.x * NORM_ROWS_PER_BLOCK + (threadIdx.x >> 5);
   if (row >= rows) return;
   const int n_vec = H / 8;
@@ -350,6 +358,8 @@ __global__ void add_bias_kernel(T* __restrict__ y, long long ldy, const void* __
 template <typename T>
 __global__ void __launch_bounds__(256) add_bias_vec_kernel(T* __restrict__ y, long long ldy, const float* __restrict__ bias,
                                                            int T_, int N) {
+  wait_for_prior_grids();
+  let_dependents_launch();
   constexpr int N_ = Vec<T>::N;
   const int i = (blockIdx.x * 32 + threadIdx.x) * N_;
   if (i >= N) return;
@@ -380,8 +390,8 @@ int embedding_launch(void* out, const void* table, const int* ids, int T_, int H
   if (T_ == 0) return OK;
   const bool vec = aligned16<T>(out, H) && aligned16<T>(table, H);
   const int threads = 128;
-  if (vec) embedding_kernel<T, true><<<T_, threads, 0, stream>>>((T*)out, (const T*)table, ids, H, V, status);
-  else embedding_kernel<T, false><<<T_, threads, 0, stream>>>((T*)out, (const T*)table, ids, H, V, status);
+  if (vec) launch_dependent(embedding_kernel<T, true>, dim3(T_), dim3(threads), 0, stream, false, (T*)out, (const T*)table, ids, H, V, status);
+  else launch_dependent(embedding_kernel<T, false>, dim3(T_), dim3(threads), 0, stream, false, (T*)out, (const T*)table, ids, H, V, status);
   return launch_result();
 }
 
@@ -398,9 +408,9 @@ int rmsnorm_launch(void* out, void* x, const void* delta, const void* w, int w_d
     const bool add = delta != nullptr;
 #define ZB_ROWS(V_)                                                                                                  \
   do {                                                                                                               \
-    if (add) rmsnorm_warp_rows_kernel<V_, true><<<blocks, NORM_ROWS_PER_BLOCK * 32, 0, stream>>>(                    \
+    if (add) launch_dependent(rmsnorm_warp_rows_kernel<V_, true>, dim3(blocks), dim3(NORM_ROWS_PER_BLOCK * 32), 0, stream, false,                     \
         (__nv_bfloat16*)out, (__nv_bfloat16*)x, (const __nv_bfloat16*)delta, w, w_dtype, eps, rows, H, x_stride, out_stride); \
-    else rmsnorm_warp_rows_kernel<V_, false><<<blocks, NORM_ROWS_PER_BLOCK * 32, 0, stream>>>(                       \
+    else launch_dependent(rmsnorm_warp_rows_kernel<V_, false>, dim3(blocks), dim3(NORM_ROWS_PER_BLOCK * 32), 0, stream, false,                        \
         (__nv_bfloat16*)out, (__nv_bfloat16*)x, nullptr, w, w_dtype, eps, rows, H, x_stride, out_stride);           \
   } while (0)
     if (vectors <= 1) ZB_ROWS(1);
@@ -415,7 +425,7 @@ int rmsnorm_launch(void* out, void* x, const void* delta, const void* w, int w_d
   threads = threads < 32 ? 32 : (threads > 512 ? 512 : threads);
   const bool add = delta != nullptr;
 #define ZB_NORM(ADD_, VEC_)                                                                            \
-  rmsnorm_kernel<T, ADD_, VEC_><<<rows, threads, 0, stream>>>((T*)out, (T*)x, (const T*)delta, w, w_dtype, \
+  launch_dependent(rmsnorm_kernel<T, ADD_, VEC_>, dim3(rows), dim3(threads), 0, stream, false, (T*)out, (T*)x, (const T*)delta, w, w_dtype, \
                                                                eps, H, x_stride, out_stride)
   if (add && vec) ZB_NORM(true, true);
   else if (add) ZB_NORM(true, false);
@@ -465,8 +475,8 @@ ZB_API int zb_gather_rows(void* out, const void* x, const int* rows, int num_row
   const dim3 grid(num_rows, vec ? (H + piece - 1) / piece : 1);
 #define ZB_GATHER(T)                                                                                                       \
   {                                                                                                                        \
-    if (vec) gather_rows_kernel<T, true><<<grid, 128, 0, s>>>((T*)out, (const T*)x, rows, H, num_src_rows, status);         \
-    else gather_rows_kernel<T, false><<<grid, 128, 0, s>>>((T*)out, (const T*)x, rows, H, num_src_rows, status);            \
+    if (vec) launch_dependent(gather_rows_kernel<T, true>, dim3(grid), dim3(128), 0, s, false, (T*)out, (const T*)x, rows, H, num_src_rows, status);         \
+    else launch_dependent(gather_rows_kernel<T, false>, dim3(grid), dim3(128), 0, s, false, (T*)out, (const T*)x, rows, H, num_src_rows, status);            \
   }
   if (dtype == DTYPE_F32) ZB_GATHER(float) else ZB_GATHER(__nv_bfloat16)
 #undef ZB_GATHER
@@ -540,8 +550,8 @@ ZB_API int zb_add_bias(void* y, long long ldy, const void* bias, int b_dtype, in
   const int piece = dtype == DTYPE_F32 ? 4 : 8;
   if (b_dtype == DTYPE_F32 && N % piece == 0 && ldy % piece == 0 && reinterpret_cast<uintptr_t>(y) % 16 == 0) {
     const dim3 grid((N / piece + 31) / 32, std::min((T + 15) / 16, 4096)), block(32, 8);
-    if (dtype == DTYPE_F32) add_bias_vec_kernel<float><<<grid, block, 0, s>>>((float*)y, ldy, (const float*)bias, T, N);
-    else add_bias_vec_kernel<__nv_bfloat16><<<grid, block, 0, s>>>((__nv_bfloat16*)y, ldy, (const float*)bias, T, N);
+    if (dtype == DTYPE_F32) launch_dependent(add_bias_vec_kernel<float>, dim3(grid), dim3(block), 0, s, false, (float*)y, ldy, (const float*)bias, T, N);
+    else launch_dependent(add_bias_vec_kernel<__nv_bfloat16>, dim3(grid), dim3(block), 0, s, false, (__nv_bfloat16*)y, ldy, (const float*)bias, T, N);
     return launch_result();
   }
   if (dtype == DTYPE_F32) add_bias_kernel<float><<<blocks, 256, 0, s>>>((float*)y, ldy, bias, b_dtype, T, N);

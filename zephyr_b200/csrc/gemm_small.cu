@@ -32,6 +32,7 @@ namespace cg = cooperative_groups;
 constexpr int ACT_TOKEN_GATE = 3;
 constexpr int GS_MAX_MT = 8;      // token tiles of 8: M <= 64
 constexpr int GS_MAX_KSPLIT = 8;
+constexpr int GS_FETCH_AHEAD_CTAS = 4 * 148;
 
 struct SmallGemmArgs {
   void* y;
@@ -89,6 +90,23 @@ gemm_small_kernel(const SmallGemmArgs a) {
     x_ok[mt] = mt * 8 + g < a.M;
     x_row[mt] = a.x + static_cast<size_t>(x_ok[mt] ? mt * 8 + g : 0) * a.ldx + 8 * t;
   }
+
+  // While the kernel before this one still runs: the warp's rows of W are asked for as far as L2 (a fetch into the coherent cache
+  // only: what the loads below bring is right whoever wrote it last).  CTAs behind the first round of them start when their
+  // weights would be asked for anyway.  (A pass of 25 steps of 12 rows, 290 of these products and as many short kernels: 6.06 -> 5.86 ms
+  // with all of them launched as dependents.)
+  if (blockIdx.x * ksplit < GS_FETCH_AHEAD_CTAS) {
+    const int row = n0 + lane % 16;
+    const char* line = reinterpret_cast<const char*>(a.w + static_cast<size_t>(row) * a.ldw + b_begin * 32) + 128 * (lane / 16);
+    const int bytes = (min(b_end * 32, a.K) - b_begin * 32) * 2;
+#pragma unroll
+    for (int rt = 0; rt < RT; ++rt)
+      for (int at = 128 * (lane / 16); at < bytes; at += 256)
+        if (row + 16 * rt < a.N)
+          asm volatile("prefetch.global.L2 [%0];\n" ::"l"(line + static_cast<size_t>(rt) * 16 * a.ldw * 2 + (at - 128 * (lane / 16))));
+  }
+  wait_for_prior_grids();
+  let_dependents_launch();
 
   float acc[RT][MT][4];
 #pragma unroll
@@ -220,13 +238,15 @@ int small_gemm_launch(const SmallGemmArgs& a, int ksplit, cudaStream_t stream) {
   config.blockDim = dim3(WARPS * 32, 1, 1);
   config.dynamicSmemBytes = 0;
   config.stream = stream;
-  cudaLaunchAttribute attribute[1];
+  cudaLaunchAttribute attribute[2];
   attribute[0].id = cudaLaunchAttributeClusterDimension;
   attribute[0].val.clusterDim.x = 1;
   attribute[0].val.clusterDim.y = ksplit;
   attribute[0].val.clusterDim.z = 1;
+  attribute[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute[1].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attribute;
-  config.numAttrs = 1;
+  config.numAttrs = dependent_launch_enabled() ? 2 : 1;
   if (cudaLaunchKernelEx(&config, gemm_small_kernel<RT, WARPS, MT, TOut, SWIGLU, ACT>, a) != cudaSuccess) return ERR_CUDA;
   return launch_result();
 }

@@ -214,6 +214,8 @@ __device__ __forceinline__ void store_piece(__nv_bfloat16* p, float4 v) {
 
 template <typename IN, typename T, int ITEMS, int HEADS>
 __global__ void __launch_bounds__(QPV_WARPS * 32) qkv_pairs_vec_kernel(const QkvPairsArgs a) {
+  wait_for_prior_grids();
+  let_dependents_launch();
   extern __shared__ __align__(16) float turn[];      // [rot_dims]: cosine and sine of every pair
   const int t = blockIdx.x, lane = threadIdx.x & 31;
   const int h0 = blockIdx.y * QPV_WARPS * HEADS + (threadIdx.x >> 5);     // and every QPV_WARPS-th behind it
@@ -364,9 +366,9 @@ ZB_API int zb_qkv_pairs(void* q_out, const void* qkv, long long stride, const fl
 #define ZB_QPV(ITEMS, HEADS)                                                                                             \
   {                                                                                                                      \
     const dim3 grid(tokens, (heads + HEADS * QPV_WARPS - 1) / (HEADS * QPV_WARPS));                                      \
-    if (dtype == DTYPE_F32) qkv_pairs_vec_kernel<float, float, ITEMS, HEADS><<<grid, QPV_WARPS * 32, smem, s>>>(a);       \
-    else if (in_dtype == DTYPE_F32) qkv_pairs_vec_kernel<float, __nv_bfloat16, ITEMS, HEADS><<<grid, QPV_WARPS * 32, smem, s>>>(a); \
-    else qkv_pairs_vec_kernel<__nv_bfloat16, __nv_bfloat16, ITEMS, HEADS><<<grid, QPV_WARPS * 32, smem, s>>>(a);          \
+    if (dtype == DTYPE_F32) launch_dependent(qkv_pairs_vec_kernel<float, float, ITEMS, HEADS>, dim3(grid), dim3(QPV_WARPS * 32), smem, s, false, a);       \
+    else if (in_dtype == DTYPE_F32) launch_dependent(qkv_pairs_vec_kernel<float, __nv_bfloat16, ITEMS, HEADS>, dim3(grid), dim3(QPV_WARPS * 32), smem, s, false, a); \
+    else launch_dependent(qkv_pairs_vec_kernel<__nv_bfloat16, __nv_bfloat16, ITEMS, HEADS>, dim3(grid), dim3(QPV_WARPS * 32), smem, s, false, a);          \
   }
     // Several heads a warp where the tokens alone give every SM a full set of warps; a decode step keeps its heads apart.
     const bool many = tokens >= 4 * 148 && heads > QPV_WARPS;

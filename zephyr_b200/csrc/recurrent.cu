@@ -182,6 +182,8 @@ template <int ITEMS> struct VecAffine {
 template <typename X, typename T, int ITEMS>
 __global__ void __launch_bounds__(LN_VEC_THREADS)
 layer_norm_vec_kernel(T* out, const X* x, const float* w, const float* b, float eps, int H) {
+  wait_for_prior_grids();
+  let_dependents_launch();
   __shared__ float scratch[33];
   const size_t base = static_cast<size_t>(blockIdx.x) * H;
   const int nv = H / 4;
@@ -205,6 +207,8 @@ template <typename T, bool RMS, int ITEMS>
 __global__ void __launch_bounds__(LN_VEC_THREADS)
 residual_layer_norm_vec_kernel(float* residual, const T* delta, const float* w1, const float* b1, float mult, T* out,
                                const float* w2, const float* b2, float eps1, float eps2, int H) {
+  wait_for_prior_grids();
+  let_dependents_launch();
   __shared__ float scratch[33];
   const size_t base = static_cast<size_t>(blockIdx.x) * H;
   const int nv = H / 4;
@@ -267,6 +271,8 @@ __global__ void embedding_f32_kernel(float* out, T* rounded, const T* table, con
 template <typename T>
 __global__ void __launch_bounds__(128) embedding_f32_vec_kernel(float* out, T* rounded, const T* table, const int* ids, float scale,
                                                                 int H, int V, int* status) {
+  wait_for_prior_grids();
+  let_dependents_launch();
   const int t = blockIdx.x, id = ids[t], i = 4 * (blockIdx.y * 128 + threadIdx.x);
   const bool ok = id >= 0 && id < V;
   if (!ok && threadIdx.x == 0 && blockIdx.y == 0) report(status, STATUS_TOKEN_OUT_OF_RANGE, id, t);
@@ -285,7 +291,7 @@ void embedding_f32(float* out, T* rounded, const T* table, const int* ids, float
                    cudaStream_t s) {
   auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
   if (H % 4 == 0 && H <= 512 * 65535 && aligned(out) && aligned(rounded) && aligned(table))
-    embedding_f32_vec_kernel<T><<<dim3(tokens, (H + 511) / 512), 128, 0, s>>>(out, rounded, table, ids, scale, H, V, status);
+    launch_dependent(embedding_f32_vec_kernel<T>, dim3(dim3(tokens, (H + 511) / 512)), dim3(128), 0, s, false, out, rounded, table, ids, scale, H, V, status);
   else
     embedding_f32_kernel<T><<<tokens, 128, 0, s>>>(out, rounded, table, ids, scale, H, V, status);
 }
@@ -318,6 +324,8 @@ constexpr int CONV_TOKENS = 1;
 
 template <typename T>
 __global__ void causal_conv_silu_kernel(const ConvArgs a, const int* token_row, int tokens) {
+  wait_for_prior_grids();
+  let_dependents_launch();
   const int c = blockIdx.y * blockDim.x + threadIdx.x;
   if (c >= a.C) return;
   float w[CONV_MAX_TAPS];
@@ -467,6 +475,8 @@ static void conv_run_launch(const ConvArgs& a, const int* token_row, int tokens,
 // After it: every request's last taps - 1 inputs go to its state.  A thread owns a channel of one request.
 template <typename T>
 __global__ void conv_state_update_kernel(const ConvArgs a) {
+  wait_for_prior_grids();
+  let_dependents_launch();
   const int c = blockIdx.x * blockDim.x + threadIdx.x, row = blockIdx.y;
   if (c >= a.C) return;
   const int slot = a.slots[row];
@@ -561,6 +571,8 @@ __global__ void scan_carry_kernel(float* ws_state, const float* ws_decay, const 
 // z <- sigmoid(z + bias)^(1/tau), through the logarithm: exp(log_sigmoid(z + bias) / tau).
 __global__ void gated_decay_kernel(float* z, long long z_stride, const void* bias, int w_dtype, int width, float inv_tau,
                                    long long count) {
+  wait_for_prior_grids();
+  let_dependents_launch();
   const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= count) return;
   const long long t = i / width;
@@ -571,6 +583,8 @@ __global__ void gated_decay_kernel(float* z, long long z_stride, const void* bia
 
 template <typename T, int MODE, int PASS>
 __global__ void __launch_bounds__(512) decayed_state_scan_kernel(const ScanArgs a) {
+  wait_for_prior_grids();
+  let_dependents_launch();
   extern __shared__ __align__(16) float scan_smem[];
   const int D = a.D, V = a.V, nwarps = blockDim.x >> 5, Dp = nwarps * SCAN_ROWS;     // blockDim.x == 2 Dp
   float* a_s = scan_smem;                                   // [SCAN_CHUNK][Dp]
@@ -856,6 +870,8 @@ template <typename T, typename G, int ITEMS, int WARPS>      // WARPS: of a grou
 __global__ void __launch_bounds__(32 * GN_WARPS) gated_group_rms_norm_vec_kernel(T* out, const float* o, const G* gate, long long gate_stride,
                                                 const float* w, int w_len, int width, int group, float eps,
                                                 int gate_first, int tokens) {
+  wait_for_prior_grids();
+  let_dependents_launch();
   __shared__ float part[GN_WARPS];
   const int groups = width / group, warp = threadIdx.x >> 5;
   const long long item = WARPS == 1 ? static_cast<long long>(blockIdx.x) * GN_WARPS + warp : blockIdx.x;
@@ -905,8 +921,7 @@ void gated_group_rms_norm_vec(T* out, const float* o, const G* gate, long long g
                               int group, float eps, int gate_first, int tokens, cudaStream_t s) {
   const long long items = static_cast<long long>(tokens) * (width / group);
 #define ZB_GN(ITEMS, WARPS)                                                                                                  \
-  gated_group_rms_norm_vec_kernel<T, G, ITEMS, WARPS>                                                                        \
-      <<<static_cast<unsigned>((items * WARPS + GN_WARPS - 1) / GN_WARPS), 32 * GN_WARPS, 0, s>>>(                           \
+  launch_dependent(gated_group_rms_norm_vec_kernel<T, G, ITEMS, WARPS>, dim3(static_cast<unsigned>((items * WARPS + GN_WARPS - 1) / GN_WARPS)), dim3(32 * GN_WARPS), 0, s, false,                            \
           out, o, gate, gate_stride, w, w_len, width, group, eps, gate_first, tokens)
   if (group <= 128) ZB_GN(1, 1);
   else if (group <= 256) ZB_GN(2, 1);
@@ -928,6 +943,8 @@ __global__ void scaled_sum_kernel(T* out, const IN* a, const IN* b, float sa, fl
 // (2125 x 2048) in 6.2 us instead of 15.0, which one value a thread took.
 template <typename IN, typename T>
 __global__ void __launch_bounds__(256) scaled_sum_vec_kernel(T* out, const IN* a, const IN* b, float sa, float sb, long long pieces) {
+  wait_for_prior_grids();
+  let_dependents_launch();
   const long long i = static_cast<long long>(blockIdx.x) * 512 + threadIdx.x;
   float4 x[2], y[2];
 #pragma unroll
@@ -947,7 +964,7 @@ template <typename IN, typename T>
 void scaled_sum(T* out, const IN* a, const IN* b, float sa, float sb, long long n, cudaStream_t s) {
   auto aligned = [](const void* p, size_t bytes) { return reinterpret_cast<uintptr_t>(p) % bytes == 0; };
   if (n % 4 == 0 && aligned(out, 4 * sizeof(T)) && aligned(a, 4 * sizeof(IN)) && aligned(b, 4 * sizeof(IN)))
-    scaled_sum_vec_kernel<IN, T><<<static_cast<unsigned>((n / 4 + 511) / 512), 256, 0, s>>>(out, a, b, sa, sb, n / 4);
+    launch_dependent(scaled_sum_vec_kernel<IN, T>, dim3(static_cast<unsigned>((n / 4 + 511) / 512)), dim3(256), 0, s, false, out, a, b, sa, sb, n / 4);
   else
     scaled_sum_kernel<IN, T><<<static_cast<unsigned>((n + 255) / 256), 256, 0, s>>>(out, a, b, sa, sb, n);
 }
@@ -980,9 +997,9 @@ ZB_API int zb_layer_norm(void* out, const void* x, const void* w, const void* b,
 #define ZB_LNV(X, T)                                                                                                      \
   {                                                                                                                       \
     if (H <= 2 * LN_VEC_THREADS * 4)                                                                                      \
-      layer_norm_vec_kernel<X, T, 2><<<rows, LN_VEC_THREADS, 0, s>>>(static_cast<T*>(out), static_cast<const X*>(x), wf, bf, eps, H); \
+      launch_dependent(layer_norm_vec_kernel<X, T, 2>, dim3(rows), dim3(LN_VEC_THREADS), 0, s, false, static_cast<T*>(out), static_cast<const X*>(x), wf, bf, eps, H); \
     else                                                                                                                  \
-      layer_norm_vec_kernel<X, T, LN_VEC_ITEMS><<<rows, LN_VEC_THREADS, 0, s>>>(static_cast<T*>(out), static_cast<const X*>(x), wf, bf, eps, H); \
+      launch_dependent(layer_norm_vec_kernel<X, T, LN_VEC_ITEMS>, dim3(rows), dim3(LN_VEC_THREADS), 0, s, false, static_cast<T*>(out), static_cast<const X*>(x), wf, bf, eps, H); \
   }
     if (x_dtype == DTYPE_F32 && out_dtype == DTYPE_F32) ZB_LNV(float, float)
     else if (x_dtype == DTYPE_F32) ZB_LNV(float, bf16)
@@ -1020,7 +1037,7 @@ static int residual_norm_launch(float* residual, const void* delta, const void* 
     const float* f2 = static_cast<const float*>(w2);
     const float* g2 = static_cast<const float*>(b2);
 #define ZB_RN(T, ITEMS)                                                                                       \
-  residual_layer_norm_vec_kernel<T, RMS, ITEMS><<<rows, LN_VEC_THREADS, 0, s>>>(                               \
+  launch_dependent(residual_layer_norm_vec_kernel<T, RMS, ITEMS>, dim3(rows), dim3(LN_VEC_THREADS), 0, s, false,                                \
       residual, static_cast<const T*>(delta), f1, g1, mult, static_cast<T*>(out), f2, g2, eps1, eps2, H)
     const bool two = H <= 2 * LN_VEC_THREADS * 4;
     if (dtype == DTYPE_F32) { if (two) ZB_RN(float, 2); else ZB_RN(float, LN_VEC_ITEMS); }
@@ -1096,12 +1113,12 @@ ZB_API int zb_causal_conv_silu(void* out, const void* x, long long x_stride, flo
   const bool runs = tokens >= 4 * rows && static_cast<long long>(tokens) * C >= 1 << 19 && aligned(2);
   if (dtype == DTYPE_F32) {
     if (runs) conv_run_launch<float>(a, token_row, tokens, aligned(4), s);
-    else causal_conv_silu_kernel<float><<<grid, 128, 0, s>>>(a, token_row, tokens);
-    if (write_state && taps > 1) conv_state_update_kernel<float><<<per_row, 128, 0, s>>>(a);
+    else launch_dependent(causal_conv_silu_kernel<float>, dim3(grid), dim3(128), 0, s, false, a, token_row, tokens);
+    if (write_state && taps > 1) launch_dependent(conv_state_update_kernel<float>, dim3(per_row), dim3(128), 0, s, false, a);
   } else {
     if (runs) conv_run_launch<__nv_bfloat16>(a, token_row, tokens, aligned(4), s);
-    else causal_conv_silu_kernel<__nv_bfloat16><<<grid, 128, 0, s>>>(a, token_row, tokens);
-    if (write_state && taps > 1) conv_state_update_kernel<__nv_bfloat16><<<per_row, 128, 0, s>>>(a);
+    else launch_dependent(causal_conv_silu_kernel<__nv_bfloat16>, dim3(grid), dim3(128), 0, s, false, a, token_row, tokens);
+    if (write_state && taps > 1) launch_dependent(conv_state_update_kernel<__nv_bfloat16>, dim3(per_row), dim3(128), 0, s, false, a);
   }
   return launch_result();
 }
@@ -1129,7 +1146,7 @@ ZB_API int zb_decayed_state_scan(float* out, const void* q, long long q_stride, 
   auto s = static_cast<cudaStream_t>(stream);
   if (mode == SCAN_GATED) {
     const long long count = static_cast<long long>(tokens) * H * D;
-    gated_decay_kernel<<<static_cast<unsigned>((count + 255) / 256), 256, 0, s>>>(z, z_stride, z_bias, w_dtype, H * D,
+    launch_dependent(gated_decay_kernel, dim3(static_cast<unsigned>((count + 255) / 256)), dim3(256), 0, s, false, z, z_stride, z_bias, w_dtype, H * D,
                                                                                 inv_tau, count);
   }
   ScanArgs a;
@@ -1161,7 +1178,7 @@ ZB_API int zb_decayed_state_scan(float* out, const void* q, long long q_stride, 
       scan_carry_kernel<<<dim3(static_cast<unsigned>((per + 255) / 256), rows), 256, 0, s>>>(                  \
           ws_state, ws_decay, state, slot_stride, slots, row_q_len, a.segs, seg_len, H, D, V, num_slots);      \
     }                                                                                                          \
-    kernel<<<grid, warps * 32, smem, s>>>(a);                                                                  \
+    launch_dependent(kernel, grid, dim3(warps * 32), smem, s, false, a);                                       \
   }
   if (dtype == DTYPE_F32) {
     if (mode == SCAN_GATED) ZB_SCAN(float, SCAN_GATED)
