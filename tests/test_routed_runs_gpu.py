@@ -65,3 +65,17 @@ def test_every_token_to_every_expert_and_to_none(ops, cuda_device):
         t = (ids[:, j] >= E).nonzero().flatten()
         expected.index_add_(0, t, x[t].double() * weights[t, j].double().unsqueeze(1))       # an identity expert
     assert (got - expected).abs().max() <= 2.0 ** -6 * max(1.0, float(expected.abs().max()))
+
+
+@pytest.mark.parametrize("rows,outputs,k", [(65, 18, 2048), (66, 1, 64), (777, 24, 1000), (2049, 9, 72), (5000, 3, 264), (4097, 16, 64)])
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+def test_many_rows_and_few_outputs(ops, cuda_device, rows, outputs, k, out_dtype):
+    g = torch.Generator().manual_seed(33)
+    wide = torch.randn(rows, k + 8, generator=g).bfloat16().to(cuda_device)
+    x, w = wide[:, :k], (torch.randn(outputs, k, generator=g) * k ** -0.5).bfloat16().to(cuda_device)     # rows further apart than they are long
+    before = ops.LAUNCH_COUNTS.get("gemm_small", 0)
+    got = ops.linear(x, w, out_dtype=out_dtype)
+    assert ops.LAUNCH_COUNTS.get("gemm_small", 0) - before == int(rows <= 4096 or outputs % 8 != 0)
+    expected = x.double() @ w.double().T
+    # float32: k sums of products of about k^-1/2; bfloat16 rounds values of up to six.
+    assert got.dtype == out_dtype and (got.double() - expected).abs().max() <= (2.0 ** -6 if out_dtype == torch.bfloat16 else 2e-5)

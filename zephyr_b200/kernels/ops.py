@@ -196,6 +196,7 @@ _SIGNATURES = {
     "zb_paged_prefill_tc": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
                             c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p],
     "zb_gemm_small_supported": [c_int, c_int, c_int],
+    "zb_gemm_few_outputs": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int, c_void_p],
     "zb_gemm_small": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int,
                       c_int, c_void_p],
     "zb_fill_normal": [c_void_p, c_longlong, ctypes.c_ulonglong, c_float, c_float, c_int, c_void_p],
@@ -1976,11 +1977,16 @@ def fused_chain(stages: Sequence[ChainStage], tokens: int, status: torch.Tensor,
 USE_LIBRARY_PRODUCTS = True     # off: every bfloat16 product of more than a few rows runs on this package's tcgen05 kernel
 
 
+# Products of more than 64 rows with up to so many outputs (a router's) run on the few-row kernel, its sides changed, where
+# the library's is slower: numbers of outputs that it has no aligned kernel for, whatever the rows, others up to so many rows.
+FEW_OUTPUTS, FEW_OUTPUTS_ROWS = 24, 4096
+
+
 def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = None,
            bias: torch.Tensor | None = None) -> torch.Tensor:
     """y = x w^T.  float32 runs on this package's CUDA-core kernel (no TF32 anywhere).  bfloat16
     with up to 64 rows (a decode step) runs on this package's weight-streaming kernel; larger
-    bfloat16 products run on the vendor library's tensor-core product, as the reference's linear
+    bfloat16 products of more than a few outputs run on the vendor library's tensor-core product, as the reference's linear
     layers do (src/layer/linear.cpp:22-24 -> cuBLASLt), where that is the faster one; with
     ``USE_LIBRARY_PRODUCTS`` off they run on this package's tcgen05 kernel (``gemm_tc``), so that no
     library kernel is left on the path.  Accumulation is float32 everywhere.  A ``bias`` [N] is
@@ -1992,6 +1998,12 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = Non
         return gemm_nt_simt(x, w, out_dtype)
     if x.shape[0] <= SMALL_GEMM_ROWS and gemm_small_supported(x, w):
         return gemm_small(x, w, out_dtype)
+    if (w.shape[0] <= FEW_OUTPUTS and (x.shape[0] <= FEW_OUTPUTS_ROWS or w.shape[0] % 8 != 0) and x.shape[0] > w.shape[0]
+            and gemm_small_supported(w, x)):
+        out = torch.empty((x.shape[0], w.shape[0]), dtype=out_dtype or x.dtype, device=x.device)
+        _check(library().zb_gemm_few_outputs(_ptr(out), _ptr(x), _ptr(w), x.shape[0], w.shape[0], x.shape[1], x.stride(0), w.stride(0),
+                                             out.stride(0), DTYPE_CODE[out.dtype], _stream()), "gemm_small")
+        return out
     if not USE_LIBRARY_PRODUCTS and gemm_tc_supported(x, w):
         return gemm_tc(x, w, out_dtype=out_dtype)
     if out_dtype is None or out_dtype == x.dtype:
