@@ -185,20 +185,21 @@ __global__ void __launch_bounds__(HW_THREADS, BM == 32 ? 5 : 4) head_linear_whol
 #pragma unroll
     for (int c = 0; c < 4; ++c) acc[nt][c] = 0.0f;
   if (m0 < rows_here && nb < n_here) {
-    const __nv_bfloat16* a_lo = sa + (m0 + g) * ld + 2 * t;
-    const __nv_bfloat16* a_hi = a_lo + 8 * ld;
-    const __nv_bfloat16* b_row = sb + (nb + g) * ld + 2 * t;
+    // Fragments by ldmatrix, a 16 x 16 piece of x and two tiles' pieces of w a load (word by word they kept shared memory busy
+    // for as long as the products take).
+    const __nv_bfloat16* a_at = sa + (m0 + (lane & 15)) * ld + (lane >> 4) * 8;
+    const __nv_bfloat16* b_at = sb + (nb + (lane & 7) + (lane >> 4) * 8) * ld + ((lane >> 3) & 1) * 8;
+#pragma unroll 2
     for (int kk = 0; kk < K; kk += 16) {
       unsigned af[4];
-      af[0] = *reinterpret_cast<const unsigned*>(a_lo + kk);
-      af[1] = *reinterpret_cast<const unsigned*>(a_hi + kk);
-      af[2] = *reinterpret_cast<const unsigned*>(a_lo + kk + 8);
-      af[3] = *reinterpret_cast<const unsigned*>(a_hi + kk + 8);
+      ldmatrix_x4(af, a_at + kk);
 #pragma unroll
-      for (int nt = 0; nt < NT; ++nt) {
+      for (int nt = 0; nt < NT; nt += 2) {
         if (nb + nt * 8 >= n_here) break;                     // uniform over the warp
-        const __nv_bfloat16* b = b_row + nt * 8 * ld + kk;
-        mma_bf16_16816(acc[nt], af, *reinterpret_cast<const unsigned*>(b), *reinterpret_cast<const unsigned*>(b + 8));
+        unsigned b[4];
+        ldmatrix_x4(b, b_at + nt * 8 * ld + kk);
+        mma_bf16_16816(acc[nt], af, b[0], b[1]);
+        if (nb + nt * 8 + 8 < n_here) mma_bf16_16816(acc[nt + 1], af, b[2], b[3]);
       }
     }
   }
