@@ -128,6 +128,15 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
+// N of them side by side (each as warp_sum gives it).
+template <int N>
+__device__ __forceinline__ void warp_sums(float (&v)[N]) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int j = 0; j < N; ++j) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
+}
+
 // Rows (requests) of `from` tokens and more cut into pieces of SIZE tokens that are numbered row by row, whatever the order in
 // which the rows' tokens lie in the stream: a row's pieces begin behind those of all such rows with a smaller number, so no
 // two pieces share a number and all are below tokens / SIZE + rows.  A whole warp calls; every lane gets the result.

@@ -249,6 +249,37 @@ __global__ void __launch_bounds__(QPV_WARPS * 32) qkv_pairs_vec_kernel(const Qkv
     sincosf(static_cast<float>(pos) * a.freqs[i], &s, &c);
     *reinterpret_cast<float2*>(turn + 2 * i) = make_float2(c, s);
   }
+  // The norms while the page and the other threads' angles are on their way.
+  {
+    float ss[HEADS];
+#pragma unroll
+    for (int j = 0; j < HEADS; ++j) {
+      ss[j] = 0.0f;
+#pragma unroll
+      for (int k = 0; k < ITEMS; ++k) {
+        const float4 v = x[j][k];
+        ss[j] += (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w);
+      }
+    }
+    warp_sums<HEADS>(ss);
+#pragma unroll
+    for (int j = 0; j < HEADS; ++j) {
+      const int h = h0 + QPV_WARPS * j;
+      const bool is_q = h < a.nh, is_v = h >= a.nh + a.nkv;
+      const int dim = is_v ? a.vd : a.kd;
+      const float* w = is_q ? a.q_norm_w : (is_v ? nullptr : a.k_norm_w);
+      if (w == nullptr && !(a.unit_norm && !is_v)) continue;
+      const float inv = 1.0f / sqrtf(ss[j] / static_cast<float>(dim) + a.eps);
+#pragma unroll
+      for (int k = 0; k < ITEMS; ++k) {
+        const int i = 4 * (lane + 32 * k);
+        const float4 v = x[j][k];
+        float4 c = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+        if (w != nullptr && i < dim) c = load_piece(w + i);
+        x[j][k] = make_float4(v.x * inv * c.x, v.y * inv * c.y, v.z * inv * c.z, v.w * inv * c.w);
+      }
+    }
+  }
   int page = 0;
   if (a.cache != nullptr) {
     const int row = a.token_row[t], block = pos / a.page_size;
@@ -276,24 +307,6 @@ __global__ void __launch_bounds__(QPV_WARPS * 32) qkv_pairs_vec_kernel(const Qkv
     if (h >= total) break;
     const bool is_q = h < a.nh, is_v = h >= a.nh + a.nkv;
     const int dim = is_v ? a.vd : a.kd;
-    const float* w = is_q ? a.q_norm_w : (is_v ? nullptr : a.k_norm_w);
-    if (w != nullptr || (a.unit_norm && !is_v)) {
-      float ss = 0.0f;
-#pragma unroll
-      for (int k = 0; k < ITEMS; ++k) {
-        const float4 v = x[j][k];
-        ss += (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w);
-      }
-      const float inv = 1.0f / sqrtf(warp_sum(ss) / static_cast<float>(dim) + a.eps);
-#pragma unroll
-      for (int k = 0; k < ITEMS; ++k) {
-        const int i = 4 * (lane + 32 * k);
-        const float4 v = x[j][k];
-        float4 c = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
-        if (w != nullptr && i < dim) c = load_piece(w + i);
-        x[j][k] = make_float4(v.x * inv * c.x, v.y * inv * c.y, v.z * inv * c.z, v.w * inv * c.w);
-      }
-    }
     if (!is_v) {
 #pragma unroll
       for (int k = 0; k < ITEMS; ++k) {

@@ -317,6 +317,22 @@ __global__ void __launch_bounds__(QHH_WARPS * 32) qkv_halves_heads_kernel(const 
     qh_smem[threadIdx.x] = c * a.rot_mult;
     qh_smem[half + threadIdx.x] = s * a.rot_mult;
   }
+  // The norms while the page and the other threads' angles are on their way.
+  {
+    float ss[HEADS];
+#pragma unroll
+    for (int j = 0; j < HEADS; ++j) ss[j] = (x[j].x * x[j].x + x[j].y * x[j].y) + (x[j].z * x[j].z + x[j].w * x[j].w);
+    warp_sums<HEADS>(ss);
+#pragma unroll
+    for (int j = 0; j < HEADS; ++j) {
+      const int h = h0 + QHH_WARPS * j;
+      const bool is_q = h < a.nh, is_v = h >= first_v;
+      const int dim = is_v ? a.vd : a.kd;
+      if (!(is_v ? a.value_unit_norm != 0 : a.norm_mode == NORM_PER_HEAD)) continue;
+      const float inv = 1.0f / sqrtf(ss[j] / static_cast<float>(dim) + a.eps);
+      x[j] = scaled4(x[j], inv, is_v || i >= dim ? nullptr : (is_q ? a.q_norm_w : a.k_norm_w), i);
+    }
+  }
   int page = 0;
   if (a.cache != nullptr) {
     const int row = a.token_row[t], block = pos / a.page_size;
@@ -352,11 +368,6 @@ __global__ void __launch_bounds__(QHH_WARPS * 32) qkv_halves_heads_kernel(const 
     const bool is_q = h < a.nh, is_v = h >= first_v;
     const int dim = is_v ? a.vd : a.kd;
     float4 y = x[j];
-    if (is_v ? a.value_unit_norm != 0 : a.norm_mode == NORM_PER_HEAD) {
-      const float ss = warp_sum((y.x * y.x + y.y * y.y) + (y.z * y.z + y.w * y.w));
-      const float inv = 1.0f / sqrtf(ss / static_cast<float>(dim) + a.eps);
-      y = scaled4(y, inv, is_v || i >= dim ? nullptr : (is_q ? a.q_norm_w : a.k_norm_w), i);
-    }
     if (!is_v && half > 0) {
       const float4 p = make_float4(__shfl_sync(~0u, y.x, partner), __shfl_sync(~0u, y.y, partner),
                                    __shfl_sync(~0u, y.z, partner), __shfl_sync(~0u, y.w, partner));
