@@ -265,6 +265,25 @@ paged_prefill_tc_kernel(const __grid_constant__ PrefillTcArgs a) {
   __shared__ unsigned tmem_base_s;
   __shared__ volatile int abort_flag;
 
+  if (threadIdx.x == 0) {
+    abort_flag = 0;
+    for (int b = 0; b < STAGES; ++b) {
+      mbar_init(&kv_full[b], Shape::KIND_WARPS);
+      mbar_init(&kv_empty[b], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&s_full[b], 1);
+      mbar_init(&p_full[2 * b], TC_SOFTMAX_WARPS / 2);
+      mbar_init(&p_full[2 * b + 1], TC_SOFTMAX_WARPS / 2);
+      mbar_init(&o_done[b], 1);
+    }
+    mbar_init(q_full, TC_SOFTMAX_WARPS);
+    mbar_init(&edge_full, 1);
+    fence_barrier_init();
+  }
+  wait_for_prior_grids();          // tiles, queries, keys and values: all of it earlier kernels' work
+  let_dependents_launch();
+
   // The host lists the tiles by the number of keys they see, fewest first: take the list back to
   // front, and all heads of a tile before the next tile, so that the longest work of the whole
   // launch starts first and the short tiles fill the gaps at the end.
@@ -314,22 +333,6 @@ paged_prefill_tc_kernel(const __grid_constant__ PrefillTcArgs a) {
   auto slot_tiles = [&](int slot) { return split ? (n_tiles + 1 - slot) >> 1 : n_tiles; };
   auto slot_tile = [&](int slot, int i) { return split ? 2 * i + slot : i; };
 
-  if (threadIdx.x == 0) {
-    abort_flag = 0;
-    for (int b = 0; b < STAGES; ++b) {
-      mbar_init(&kv_full[b], Shape::KIND_WARPS);
-      mbar_init(&kv_empty[b], 1);
-    }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(&s_full[b], 1);
-      mbar_init(&p_full[2 * b], TC_SOFTMAX_WARPS / 2);
-      mbar_init(&p_full[2 * b + 1], TC_SOFTMAX_WARPS / 2);
-      mbar_init(&o_done[b], 1);
-    }
-    mbar_init(q_full, TC_SOFTMAX_WARPS);
-    mbar_init(&edge_full, 1);
-    fence_barrier_init();
-  }
   if (warp == TC_MMA_WARP) {
     tmem_alloc(&tmem_base_s, TC_TMEM_COLUMNS);
     tmem_relinquish();
@@ -785,8 +788,7 @@ int prefill_tc_launch(PrefillTcArgs& a, long long cache_rows, int page_size, cud
   if (cuda_failed(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::SMEM))) return ERR_CUDA;
   const long long ctas = static_cast<long long>(a.n_split) * a.nh + static_cast<long long>(a.n_tiles - a.n_split) * (a.nh / 2);
   if (ctas >= (1LL << 31)) return ERR_UNSUPPORTED;
-  kernel<<<static_cast<unsigned>(ctas), TC_THREADS, Shape::SMEM, stream>>>(a);
-  return launch_result();
+  return launch_dependent(kernel, dim3(static_cast<unsigned>(ctas)), dim3(TC_THREADS), Shape::SMEM, stream, false, a);
 }
 
 }  // namespace zb

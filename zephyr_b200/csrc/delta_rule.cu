@@ -50,6 +50,8 @@ struct DeltaGatesArgs {
 
 template <typename T>
 __global__ void __launch_bounds__(128) delta_gates_kernel(const DeltaGatesArgs a) {
+  wait_for_prior_grids();
+  let_dependents_launch();
   const long long t = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (a.below > 0) {
@@ -357,6 +359,8 @@ struct DeltaBlocksArgs {
 // DP: the channels padded with zeros.
 template <typename T, int DP>
 __global__ void __launch_bounds__(DB_THREADS) delta_blocks_kernel(const DeltaBlocksArgs a) {
+  wait_for_prior_grids();
+  let_dependents_launch();
   extern __shared__ __align__(16) float db_smem[];
   constexpr int ST = DP + 4;
   float* x_s = db_smem;                    // [2 DB][ST]: k, q
@@ -711,8 +715,8 @@ ZB_API int zb_delta_gates(float* q_out, float* k_out, float* beta, float* decay,
   g.qk_heads = qk_heads; g.heads = heads; g.D = D; g.q_scale = q_scale; g.unit_eps = unit_eps;
   g.row_q_start = row_q_start; g.row_q_len = row_q_len; g.rows = rows; g.below = below;
   auto s = static_cast<cudaStream_t>(stream);
-  if (dtype == DTYPE_F32) delta_gates_kernel<float><<<tokens, 128, 0, s>>>(g);
-  else delta_gates_kernel<__nv_bfloat16><<<tokens, 128, 0, s>>>(g);
+  if (dtype == DTYPE_F32) launch_dependent(delta_gates_kernel<float>, dim3(tokens), dim3(128), 0, s, false, g);
+  else launch_dependent(delta_gates_kernel<__nv_bfloat16>, dim3(tokens), dim3(128), 0, s, false, g);
   return launch_result();
 }
 
@@ -782,7 +786,9 @@ static int delta_block_launch(const DeltaBlocksArgs& b, const DeltaBlockScanArgs
   constexpr int first = static_cast<int>(delta_blocks_smem<DP>()), second = static_cast<int>(delta_block_scan_smem<DP>());
   if (cuda_failed(cudaFuncSetAttribute(delta_block_scan_kernel<T, DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, second)))
     return ERR_CUDA;
-  delta_blocks_kernel<T, DP><<<dim3(blocks, b.qk_heads), DB_THREADS, first, s>>>(b);
+  launch_dependent(delta_blocks_kernel<T, DP>, dim3(blocks, b.qk_heads), dim3(DB_THREADS), first, s, false, b);
+  // (Not as a dependent: its CTAs would take the SMs that the kernel before it leaves first, two a SM, while others stay empty:
+  // the layer over 2048 tokens, 16 heads 347 -> 500 us.)
   delta_block_scan_kernel<T, DP><<<dim3(rows, a.heads, (a.V + DB_COLS - 1) / DB_COLS), DB_THREADS, second, s>>>(a);
   return launch_result();
 }

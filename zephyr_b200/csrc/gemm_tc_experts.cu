@@ -102,6 +102,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GX_THREADS, 1) gemm_
   cluster_sync_all();                               // both CTAs' barriers and tensor memory are there
   tc_fence_after_sync();
   const unsigned tmem_base = sh.tmem_base;
+  wait_for_prior_grids();
+  let_dependents_launch();
   const int runs = a.plan[0], items = runs * a.row_blocks;
   // The product's columns: a run's places up to a multiple of 64, half of them in each CTA.
   auto half_columns = [](int rows) { return (rows + 63) / 64 * 32; };
@@ -263,6 +265,11 @@ int experts_launch(const ExpertsTcArgs& a, int max_runs, int sms, cudaStream_t s
   if (cuda_failed(cudaOccupancyMaxActiveClusters(&clusters, kernel, &config)) || clusters <= 0) return ERR_CUDA;
   const long long items = static_cast<long long>(max_runs) * a.row_blocks;
   config.gridDim = dim3(2 * static_cast<unsigned>(items < clusters ? items : clusters));
+  cudaLaunchAttribute attribute[1];
+  attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute[0].val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = attribute;
+  config.numAttrs = dependent_launch_enabled() ? 1 : 0;
   return cuda_failed(cudaLaunchKernelEx(&config, kernel, a)) ? ERR_CUDA : launch_result();
 }
 template <int RUN>

@@ -129,6 +129,8 @@ constexpr int HW_ROWS_32 = 384;
 // the gates per output value, which then come in as pairs.
 template <typename X, typename OUT, int BM>
 __global__ void __launch_bounds__(HW_THREADS, BM == 32 ? 5 : 4) head_linear_whole_k_kernel(const HeadLinearArgs a, int pairs) {
+  wait_for_prior_grids();
+  let_dependents_launch();
   extern __shared__ __align__(16) unsigned char hw_smem[];
   const int K = a.K, ld = K + 8, pieces = K / 8;
   __nv_bfloat16* sa = reinterpret_cast<__nv_bfloat16*>(hw_smem);      // [BM][ld]
@@ -265,8 +267,7 @@ int head_linear_whole_k_launch(const HeadLinearArgs& a, cudaStream_t s) {
   const bool pairs = tm_aligned(a.y, 2 * sizeof(OUT)) && a.y_stride % 2 == 0 && a.y_head_stride % 2 == 0;
   const bool gate_pairs = a.gate != nullptr && a.gate_per_element && tm_aligned(a.gate, 8) && a.gate_stride % 2 == 0 && a.N % 2 == 0;
   const dim3 grid((a.tokens + BM - 1) / BM, (a.N + HW_BN - 1) / HW_BN, a.heads);
-  kernel<<<grid, HW_THREADS, smem, s>>>(a, (pairs ? 1 : 0) | (gate_pairs ? 2 : 0));
-  return launch_result();
+  return launch_dependent(kernel, grid, dim3(HW_THREADS), smem, s, false, a, (pairs ? 1 : 0) | (gate_pairs ? 2 : 0));
 }
 
 }  // namespace zb

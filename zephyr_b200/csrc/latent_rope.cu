@@ -41,6 +41,8 @@ struct LatentRopeArgs {
 
 template <typename T>
 __global__ void __launch_bounds__(LR_THREADS) latent_rope_kernel(const LatentRopeArgs a) {
+  wait_for_prior_grids();
+  let_dependents_launch();
   __shared__ float cos_of[LR_MAX_HALF], sin_of[LR_MAX_HALF];
   const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int pos = a.positions[t], half = a.rot / 2, width = a.rank + a.rot;
@@ -114,7 +116,7 @@ ZB_API int zb_latent_rope(void* q_out, const float* q, long long q_stride, int q
   a.max_blocks = max_blocks; a.page_size = page_size; a.num_pages = num_pages; a.num_rows = num_rows; a.nh = nh;
   a.rank = rank; a.rot = rot; a.status = status;
   auto s = static_cast<cudaStream_t>(stream);
-  if (dtype == DTYPE_F32) latent_rope_kernel<float><<<tokens, LR_THREADS, 0, s>>>(a);
-  else latent_rope_kernel<__nv_bfloat16><<<tokens, LR_THREADS, 0, s>>>(a);
+  if (dtype == DTYPE_F32) launch_dependent(latent_rope_kernel<float>, dim3(tokens), dim3(LR_THREADS), 0, s, false, a);
+  else launch_dependent(latent_rope_kernel<__nv_bfloat16>, dim3(tokens), dim3(LR_THREADS), 0, s, false, a);
   return launch_result();
 }

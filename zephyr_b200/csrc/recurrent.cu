@@ -389,6 +389,8 @@ __device__ __forceinline__ void conv_store(T* p, const float (&y)[VEC]) {
 
 template <typename T, int VEC, int TAPS>
 __global__ void __launch_bounds__(128) causal_conv_silu_run_kernel(const ConvArgs a, const int* token_row, int tokens) {
+  wait_for_prior_grids();
+  let_dependents_launch();
   __shared__ int first_s[CONV_RUN], slot_s[CONV_RUN];         // per token: index within its request's new tokens, slot
   const int t0 = blockIdx.x * CONV_RUN, nt = min(CONV_RUN, tokens - t0);
   const int c = (blockIdx.y * blockDim.x + threadIdx.x) * VEC;
@@ -464,11 +466,11 @@ static void conv_run_launch(const ConvArgs& a, const int* token_row, int tokens,
   const int vectors = a.C / (four ? 4 : 2);
   const dim3 grid((tokens + CONV_RUN - 1) / CONV_RUN, (vectors + 127) / 128);
   if (a.taps <= 4) {
-    if (four) causal_conv_silu_run_kernel<T, 4, 4><<<grid, 128, 0, s>>>(a, token_row, tokens);
-    else causal_conv_silu_run_kernel<T, 2, 4><<<grid, 128, 0, s>>>(a, token_row, tokens);
+    if (four) launch_dependent(causal_conv_silu_run_kernel<T, 4, 4>, dim3(grid), dim3(128), 0, s, false, a, token_row, tokens);
+    else launch_dependent(causal_conv_silu_run_kernel<T, 2, 4>, dim3(grid), dim3(128), 0, s, false, a, token_row, tokens);
   } else {
-    if (four) causal_conv_silu_run_kernel<T, 4, 8><<<grid, 128, 0, s>>>(a, token_row, tokens);
-    else causal_conv_silu_run_kernel<T, 2, 8><<<grid, 128, 0, s>>>(a, token_row, tokens);
+    if (four) launch_dependent(causal_conv_silu_run_kernel<T, 4, 8>, dim3(grid), dim3(128), 0, s, false, a, token_row, tokens);
+    else launch_dependent(causal_conv_silu_run_kernel<T, 2, 8>, dim3(grid), dim3(128), 0, s, false, a, token_row, tokens);
   }
 }
 

@@ -46,6 +46,8 @@ __global__ void __launch_bounds__(ROUTE_WARPS * 32)
 route_kernel(int* ids, float* weights, const float* logits, long long logits_stride, const float* correction,
              int tokens, int outputs, int top, int score_kind, int groups, int keep, int group_top,
              float weight_scale, const float* logit_bias, int normalize) {
+  wait_for_prior_grids();
+  let_dependents_launch();
   __shared__ float choice_of[ROUTE_WARPS][32 * ROUTE_PER_LANE];
   __shared__ float mark_of[ROUTE_WARPS][32 * ROUTE_PER_LANE];
   const int warp = threadIdx.x >> 5;
@@ -238,6 +240,8 @@ align_kernel(int* plan, int* slots, int* place_of_slot, const int* ids, int num_
 // first place and places that count, and slots[place] is -1 where a place pads a run.
 __global__ void __launch_bounds__(ALIGN_THREADS)
 align_runs_kernel(int* plan, int* slots, int* place_of_slot, const int* ids, int num_slots, int experts, int max_runs, int run, int places) {
+  wait_for_prior_grids();
+  let_dependents_launch();
   extern __shared__ int align_smem[];
   int* count = align_smem;                 // [experts]
   int* start = count + experts;            // [experts]
@@ -303,6 +307,8 @@ align_runs_kernel(int* plan, int* slots, int* place_of_slot, const int* ids, int
 // With `place_scale` also the slot's weight for each place (zero for a pad).
 __global__ void gather_places_kernel(uint4* out, const uint4* x, long long x_stride16, const int* slots, int pieces, int top,
                                      float* place_scale, const float* weights) {
+  wait_for_prior_grids();
+  let_dependents_launch();
   const int place = blockIdx.x, slot = slots[place];
   if (place_scale != nullptr && threadIdx.x == 0) place_scale[place] = slot >= 0 ? weights[slot] : 0.0f;
   const uint4* src = slot >= 0 ? x + static_cast<long long>(slot / top) * x_stride16 : nullptr;
@@ -497,6 +503,8 @@ __global__ void combine_kernel(T* out, const Y* y, long long y_stride, const T* 
 constexpr int COMBINE_MAX_TOP = 16;
 __global__ void combine_pieces_kernel(uint4* out, const uint4* y, long long y_stride16, const uint4* x, long long x_stride16,
                                       const float* weights, const int* place_of_slot, int pieces, int top) {
+  wait_for_prior_grids();
+  let_dependents_launch();
   const int t = blockIdx.x;
   __shared__ int place_s[COMBINE_MAX_TOP];
   __shared__ float weight_s[COMBINE_MAX_TOP];
@@ -549,8 +557,7 @@ ZB_API int zb_route_biased(int* ids, float* weights, const float* logits, long l
     return ERR_BAD_ARGUMENT;
   if (outputs > 32 * ROUTE_PER_LANE || (groups > 1 && group_top > ROUTE_GROUP_TOP_MAX)) return ERR_UNSUPPORTED;
   if (tokens == 0) return OK;
-  route_kernel<<<(tokens + ROUTE_WARPS - 1) / ROUTE_WARPS, ROUTE_WARPS * 32, 0, static_cast<cudaStream_t>(stream)>>>(
-      ids, weights, logits, logits_stride, correction, tokens, outputs, top, sigmoid_scores, groups, keep, group_top,
+  launch_dependent(route_kernel, dim3((tokens + ROUTE_WARPS - 1) / ROUTE_WARPS), dim3(ROUTE_WARPS * 32), 0, static_cast<cudaStream_t>(stream), false, ids, weights, logits, logits_stride, correction, tokens, outputs, top, sigmoid_scores, groups, keep, group_top,
       weight_scale, logit_bias, normalize);
   return launch_result();
 }
@@ -620,7 +627,7 @@ ZB_API int zb_route_align_runs(int* plan, int* slots, int* place_of_slot, const 
     return ERR_BAD_ARGUMENT;
   const size_t smem = 3 * static_cast<size_t>(experts) * sizeof(int);
   if (smem > 48 * 1024) return ERR_UNSUPPORTED;
-  align_runs_kernel<<<1, ALIGN_THREADS, smem, static_cast<cudaStream_t>(stream)>>>(plan, slots, place_of_slot, ids, num_slots, experts,
+  launch_dependent(align_runs_kernel, dim3(1), dim3(ALIGN_THREADS), smem, static_cast<cudaStream_t>(stream), false, plan, slots, place_of_slot, ids, num_slots, experts,
                                                                                      max_runs, run, places);
   return launch_result();
 }
@@ -632,12 +639,11 @@ ZB_API int zb_gather_places(void* out, const void* x, long long x_stride, const 
       reinterpret_cast<uintptr_t>(out) % 16 != 0 || reinterpret_cast<uintptr_t>(x) % 16 != 0)
     return ERR_BAD_ARGUMENT;
   if (places == 0) return OK;
-  gather_places_kernel<<<places, 128, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<uint4*>(out), static_cast<const uint4*>(x), x_stride / 8, slots, width / 8, top, place_scale, weights);
+  launch_dependent(gather_places_kernel, dim3(places), dim3(128), 0, static_cast<cudaStream_t>(stream), false, static_cast<uint4*>(out), static_cast<const uint4*>(x), x_stride / 8, slots, width / 8, top, place_scale, weights);
   return launch_result();
 }
 
-// `weights` null: the outputs are added up as they are.  `y_dtype`: float32 sums, or the model's type (what the grouped tcgen05 product writes).
+// `weights` null: the outputs are added up as they are.  `y_dtype`: float32 sums, or the model's type (what the tcgen05 product writes).
 ZB_API int zb_route_combine(void* out, const void* y, long long y_stride, int y_dtype, const void* x, long long x_stride,
                             const int* ids, const float* weights, const int* place_of_slot, int tokens, int width, int top,
                             int dtype, void* stream) {
@@ -657,8 +663,7 @@ ZB_API int zb_route_combine(void* out, const void* y, long long y_stride, int y_
                                                            width, top);
   } else if (width % 8 == 0 && y_stride % 8 == 0 && x_stride % 8 == 0 && top <= COMBINE_MAX_TOP && tm_aligned(out, 16) &&
              tm_aligned(y, 16) && tm_aligned(x, 16)) {
-    combine_pieces_kernel<<<tokens, width >= 2048 ? 256 : 128, 0, s>>>(
-        static_cast<uint4*>(out), static_cast<const uint4*>(y), y_stride / 8, static_cast<const uint4*>(x), x_stride / 8,
+    launch_dependent(combine_pieces_kernel, dim3(tokens), dim3(width >= 2048 ? 256 : 128), 0, s, false, static_cast<uint4*>(out), static_cast<const uint4*>(y), y_stride / 8, static_cast<const uint4*>(x), x_stride / 8,
         weights, place_of_slot, width / 8, top);
   } else {
     combine_kernel<bf16, bf16><<<tokens, threads, 0, s>>>(static_cast<bf16*>(out), static_cast<const bf16*>(y), y_stride,

@@ -128,6 +128,8 @@ __device__ __forceinline__ void walk_product(float (&acc)[N][4], float (&low)[N]
 constexpr int W_HEADS = 4;
 template <int MODE, int DP>
 __global__ void __launch_bounds__(W_THREADS) walk_prepare_kernel(const WalkArgs a) {
+  wait_for_prior_grids();
+  let_dependents_launch();
   using Parts = WalkParts<MODE, DP>;
   constexpr int ST = Parts::ST, PA = Parts::PA, PB = Parts::PB, HEADS = MODE == WALK_SPACE ? W_HEADS : 1;
   extern __shared__ __align__(16) unsigned char w_smem[];
@@ -639,7 +641,8 @@ static int walk_launch(const WalkArgs& a, int pieces, cudaStream_t s) {
       cuda_failed(cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::smem)))
     return ERR_CUDA;
   const int heads = MODE == WALK_SPACE ? W_HEADS : 1;
-  prepare<<<dim3(pieces, a.H / a.heads_per_group * ((a.heads_per_group + heads - 1) / heads)), W_THREADS, Shape::qk_bytes, s>>>(a);
+  launch_dependent(prepare, dim3(pieces, a.H / a.heads_per_group * ((a.heads_per_group + heads - 1) / heads)), dim3(W_THREADS), Shape::qk_bytes, s, false, a);
+  // (Not as a dependent, which would fill the SMs that are free first instead of all of them.)
   walk<<<dim3(a.rows, a.H, (a.V + Shape::COLS - 1) / Shape::COLS), W_THREADS, Shape::smem, s>>>(a);
   return launch_result();
 }

@@ -166,6 +166,8 @@ template <typename A, typename B, typename OUT>
 __global__ void __launch_bounds__(SN_THREADS)
 sum_rms_norm_vec_kernel(OUT* out, long long out_stride, float* x, long long x_stride, const A* a, const B* b,
                         const float* bias, const void* w, int w_dtype, float eps, int H) {
+  wait_for_prior_grids();
+  let_dependents_launch();
   __shared__ float scratch[33];
   const int threads = blockDim.x;
   const long long r = blockIdx.x, summand_stride = static_cast<long long>(H) * gridDim.y;
@@ -391,7 +393,7 @@ ZB_API int zb_sum_rms_norm(void* out, long long out_stride, int out_dtype, float
 #define ZB_SN(A_, B_, OUT_)                                                                                          \
   {                                                                                                                  \
     if (vectors)                                                                                                     \
-      sum_rms_norm_vec_kernel<A_, B_, OUT_><<<grid, threads, 0, s>>>((OUT_*)out, out_stride, x, x_stride,         \
+      launch_dependent(sum_rms_norm_vec_kernel<A_, B_, OUT_>, dim3(grid), dim3(threads), 0, s, false, (OUT_*)out, out_stride, x, x_stride,         \
                                                                          (const A_*)a, (const B_*)b, bias, w, w_dtype, eps, part); \
     else                                                                                                             \
       sum_rms_norm_kernel<A_, B_, OUT_><<<grid, threads, 0, s>>>((OUT_*)out, out_stride, x, x_stride, (const A_*)a, \

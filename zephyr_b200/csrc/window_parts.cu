@@ -289,6 +289,8 @@ constexpr int QHH_WARPS = 8;
 
 template <typename T, int HEADS>
 __global__ void __launch_bounds__(QHH_WARPS * 32) qkv_halves_heads_kernel(const QkvHalvesArgs a) {
+  wait_for_prior_grids();
+  let_dependents_launch();
   extern __shared__ __align__(16) float qh_smem[];      // [rot_dims]: cosines, then sines
   const int t = blockIdx.x, lane = threadIdx.x & 31, i = 4 * lane;
   const int h0 = blockIdx.y * QHH_WARPS * HEADS + (threadIdx.x >> 5);     // and every QHH_WARPS-th behind it
@@ -521,6 +523,8 @@ sigmoid_gate_kernel(T* x, const float* gate, long long gate_stride, int width, i
 // The same for bfloat16 rows and runs of whole 16-byte pieces: a thread owns a piece and its run's gate.
 __global__ void __launch_bounds__(256)
 sigmoid_gate_pieces_kernel(uint4* x, const float* gate, long long gate_stride, int pieces, int per_pieces) {
+  wait_for_prior_grids();
+  let_dependents_launch();
   const long long t = blockIdx.x;
   for (int c = threadIdx.x; c < pieces; c += blockDim.x) {
     const float g = 1.0f / (1.0f + expf(-gate[t * gate_stride + c / per_pieces]));
@@ -576,8 +580,8 @@ ZB_API int zb_qkv_halves(void* q_out, const void* qkv, long long stride, const f
 #define ZB_QHH(HEADS)                                                                                        \
   {                                                                                                          \
     const dim3 grid(tokens, (heads + HEADS * QHH_WARPS - 1) / (HEADS * QHH_WARPS));                          \
-    if (dtype == DTYPE_F32) qkv_halves_heads_kernel<float, HEADS><<<grid, QHH_WARPS * 32, turn, s>>>(a);      \
-    else qkv_halves_heads_kernel<__nv_bfloat16, HEADS><<<grid, QHH_WARPS * 32, turn, s>>>(a);                 \
+    if (dtype == DTYPE_F32) launch_dependent(qkv_halves_heads_kernel<float, HEADS>, dim3(grid), dim3(QHH_WARPS * 32), turn, s, false, a);      \
+    else launch_dependent(qkv_halves_heads_kernel<__nv_bfloat16, HEADS>, dim3(grid), dim3(QHH_WARPS * 32), turn, s, false, a);                 \
   }
       if (many) ZB_QHH(4) else ZB_QHH(1)
 #undef ZB_QHH
@@ -648,7 +652,7 @@ ZB_API int zb_sigmoid_gate(void* x, const float* gate, long long gate_stride, in
   if (tokens == 0) return OK;
   auto s = static_cast<cudaStream_t>(stream);
   if (dtype == DTYPE_BF16 && per % 8 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0) {
-    sigmoid_gate_pieces_kernel<<<tokens, 256, 0, s>>>(static_cast<uint4*>(x), gate, gate_stride, width / 8, per / 8);
+    launch_dependent(sigmoid_gate_pieces_kernel, dim3(tokens), dim3(256), 0, s, false, static_cast<uint4*>(x), gate, gate_stride, width / 8, per / 8);
     return launch_result();
   }
   if (dtype == DTYPE_F32) sigmoid_gate_kernel<float><<<tokens, 256, 0, s>>>(static_cast<float*>(x), gate, gate_stride, width, per);
