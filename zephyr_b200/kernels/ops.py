@@ -279,7 +279,9 @@ def _check(rc: int, name: str, kernels: int = 1) -> None:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream's handle: what ``torch.cuda.current_stream().cuda_stream`` gives, without the objects that are made on the
+    way to it, which cost a launch 3 us on the host."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _ptr(t: torch.Tensor | None) -> int | None:
@@ -2133,23 +2135,24 @@ def routed_experts(x: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w_
         run = lib.zb_gemm_tc_experts_run(num_slots, E)
         runs = num_slots // run + E
         places = num_slots + 16 * runs
-        plan = torch.empty(1 + 3 * runs, dtype=torch.int32, device=device)
-        slots = torch.empty(places, dtype=torch.int32, device=device)
-        _check(lib.zb_route_align_runs(_ptr(plan), _ptr(slots), _ptr(place), _ptr(ids), num_slots, E, runs, run, places, _stream()),
-               "route_align")
-        rows = torch.empty((places, width), dtype=x.dtype, device=device)
-        place_scale = torch.empty(places, dtype=torch.float32, device=device) if weigh_inputs else None
-        _check(lib.zb_gather_places(_ptr(rows), _ptr(x), x.stride(0), _ptr(slots), places, width, top, _ptr(place_scale),
-                                    _ptr(weights), _stream()), "gather_places")
-        status = device_status(device)
-        hidden = torch.empty((places, ff), dtype=x.dtype, device=device)
-        _check(lib.zb_gemm_tc_experts(_ptr(hidden), _ptr(rows), _ptr(w_gate), _ptr(plan), runs, run, places, E, 2 * ff, width, width, ff,
-                                      1 + act_code, _ptr(place_scale), *bounds, _ptr(status), _stream()), "gemm_tc_grouped")
+        # One workspace for the plan and the places' slots, one for the gathered rows, the hidden rows and the experts' outputs
+        # (a call to the allocator costs the host more than the slices).
+        numbers = torch.empty(4 + 3 * runs + places, dtype=torch.int32, device=device)
+        plan = numbers.data_ptr()
+        slots = plan + 4 * (4 + 3 * runs)
+        stream, status = _stream(), _ptr(device_status(device))
+        _check(lib.zb_route_align_runs(plan, slots, _ptr(place), _ptr(ids), num_slots, E, runs, run, places, stream), "route_align")
+        work = torch.empty(places * (2 * width + ff), dtype=x.dtype, device=device)
         # An expert's output takes the model's type before it is weighted on every path: here the product writes it so.
-        ldy = width
-        y = torch.empty((places, ldy), dtype=x.dtype, device=device)
-        _check(lib.zb_gemm_tc_experts(_ptr(y), _ptr(hidden), _ptr(w_down), _ptr(plan), runs, run, places, E, width, ff, ff, ldy, 0,
-                                      None, *bounds, _ptr(status), _stream()), "gemm_tc_grouped")
+        y, ldy = work[:places * width].view(places, width), width
+        rows, hidden = work.data_ptr() + 2 * places * width, work.data_ptr() + 4 * places * width
+        place_scale = torch.empty(places, dtype=torch.float32, device=device) if weigh_inputs else None
+        _check(lib.zb_gather_places(rows, _ptr(x), x.stride(0), slots, places, width, top, _ptr(place_scale), _ptr(weights), stream),
+               "gather_places")
+        _check(lib.zb_gemm_tc_experts(hidden, rows, _ptr(w_gate), plan, runs, run, places, E, 2 * ff, width, width, ff, 1 + act_code,
+                                      _ptr(place_scale), *bounds, status, stream), "gemm_tc_grouped")
+        _check(lib.zb_gemm_tc_experts(_ptr(y), hidden, _ptr(w_down), plan, runs, run, places, E, width, ff, ff, ldy, 0, None, *bounds,
+                                      status, stream), "gemm_tc_grouped")
     else:
         tile_rows = lib.zb_expert_tile_rows(code)          # CUDA-core tiles in float32, tensor-core tiles in bfloat16
         max_tiles = -(-num_slots // tile_rows) + E
