@@ -130,3 +130,16 @@ def test_float32_logits_do_not_depend_on_what_shares_the_step(model_folders, cud
     alone, together = logits([[r] for r in range(len(lengths))]), logits([list(range(len(lengths)))])
     for key in alone:
         assert torch.equal(alone[key], together[key]), key
+
+
+@pytest.mark.parametrize("m,n,k", [
+    (700, 1000, 60), (1500, 1023, 36), (300, 1030, 132), (129, 4100, 68), (64, 4096, 64), (33, 6145, 20), (200, 1024, 100), (2048, 4097, 16),
+    (8, 70001, 12), (1, 5, 4),
+    (2100000, 5, 4)])
+def test_products_in_every_tile(ops, cuda_device, m, n, k):
+    """Whatever tile the sizes choose: near the exact product, and a row's sums the same to the bit as on its own."""
+    x, w = rand((m, k), torch.float32, cuda_device, 70), rand((n, k), torch.float32, cuda_device, 71)
+    got, exact = ops.gemm_nt_simt(x, w), x.double() @ w.double().T
+    assert (got.double() - exact).abs().max() <= k * 2.0 ** -24 * float((x.abs().double() @ w.abs().double().T).max())
+    for row in {0, m // 2, m - 1}:
+        assert torch.equal(got[row:row + 1], ops.gemm_nt_simt(x[row:row + 1], w))

@@ -76,15 +76,15 @@ int gemm_launch(void* y, const void* x, const void* w, int M, int N, int K, long
 // Bound by the reads of shared memory beside the multiply-adds, and at few tiles by latency.  A CTA makes a tile of
 // BM x BN with VG groups of threads: the slices of VK values of k are dealt to the groups in turn, every group sums
 // its own slices in ascending k, and the groups' sums are added in their order at the end.  That order is the same for
-// both tile sizes.  Four groups give a CTA eight warps where one group would leave an SM two (88 tiles of 64 x 128 at
+// all tile sizes.  Four groups give a CTA eight warps where one group would leave an SM two (88 tiles of 64 x 128 at
 // 700 x 1024 x 2048: 137 us, 216 us with the kernel above, 293 us with one group on tiles of 128 x 128), and four
 // short chains are closer to the exact sum than one long one (2.9e-7 against 5.7e-7 at K = 1024).
 // A thread makes 4 GM x 4 GN outputs as groups of four rows and four columns, so a step of k is GM + GN 16-byte
 // reads of shared memory for 8 GM GN paired multiply-adds.  A slice sits in one of two buffers, the next one on its way
 // into registers; a lane loads 32 bytes of one row of x or w, neighbouring lanes neighbouring rows, and stores them
 // transposed without bank conflicts.
-// Measured (us, the kernel above in brackets): 700 x 4096 x 1024 202 (259), 2048 x 6144 x 1024 716 (1017),
-// 900 x 1024 x 3072 193 (330).
+// Measured (us, the kernel above in brackets): 700 x 4096 x 1024 199 (259), 2048 x 6144 x 1024 716 (1017),
+// 900 x 1024 x 3072 189 (330).
 constexpr int VK = 16;
 constexpr int VG = 4;
 
@@ -234,11 +234,33 @@ ZB_API int zb_gemm_nt_simt(void* y, const void* x, const void* w, int M, int N, 
     auto yf = static_cast<float*>(y);
     auto xf = static_cast<const float*>(x), wf = static_cast<const float*>(w);
     if (!vectors) return gemm_launch<float, float>(y, x, w, M, N, K, ldx, ldw, ldy, s);
-    // Tiles of 64 x 128 where they give at least every other SM one, else of 32 x 32, whose CTAs are eight times as
-    // many (128 x 1024 x 2048, 16 large tiles: 41 against 136 us; 700 x 1024 x 2048, 88 of them: 169 against 137 us).
-    const long long large = static_cast<long long>((M + 63) / 64) * ((N + 127) / 128);
-    if (large >= 74) return gemm_vec_launch<64, 128, 2, 4>(yf, xf, wf, M, N, K, ldx, ldw, ldy, s);
-    return gemm_vec_launch<32, 32, 1, 1>(yf, xf, wf, M, N, K, ldx, ldw, ldy, s);
+    // The tile whose rounds over the SMs take the least time: a round costs (us at K = 1024, whatever K's share of
+    // it) 65 with tiles of 64 x 128, 50 with 64 x 96, 44 with 64 x 64, 30 with 32 x 64 and 18 with 32 x 32, which are
+    // one CTA an SM or as good as one.  (us, here / with the largest or the smallest tile alone: 700 x 6144 x 1024
+    // 249 / 264; 700 x 1024 x 2048, one round of 64 x 96 instead of one of the largest on 88 SMs, 102 / 137;
+    // 500 x 1024 x 2048 90 / 133, 300 x 1024 x 2048 89 / 100, 128 x 4096 x 1024 47 / 68, 64 x 4096 x 1024 32 / 36,
+    // 1500 x 1024 x 2048 196 / 255, 8 x 151936 x 1024 388 / 430.)
+    struct Tile { int m, n, us; };
+    constexpr Tile tiles[5] = {{64, 128, 65}, {64, 96, 50}, {64, 64, 44}, {32, 64, 30}, {32, 32, 18}};
+    int best = 0;
+    long long least = 0;
+    for (int t = 0; t < 5; ++t) {
+      const int down = (M + tiles[t].m - 1) / tiles[t].m;
+      if (t > 0 && down > 65535) continue;  // a grid holds no more
+      const long long units = static_cast<long long>(down) * ((N + tiles[t].n - 1) / tiles[t].n);
+      const long long time = (units + 147) / 148 * tiles[t].us;
+      if (t == 0 || time < least) {
+        best = t;
+        least = time;
+      }
+    }
+    switch (best) {
+      case 0: return gemm_vec_launch<64, 128, 2, 4>(yf, xf, wf, M, N, K, ldx, ldw, ldy, s);
+      case 1: return gemm_vec_launch<64, 96, 2, 3>(yf, xf, wf, M, N, K, ldx, ldw, ldy, s);
+      case 2: return gemm_vec_launch<64, 64, 2, 2>(yf, xf, wf, M, N, K, ldx, ldw, ldy, s);
+      case 3: return gemm_vec_launch<32, 64, 1, 2>(yf, xf, wf, M, N, K, ldx, ldw, ldy, s);
+      default: return gemm_vec_launch<32, 32, 1, 1>(yf, xf, wf, M, N, K, ldx, ldw, ldy, s);
+    }
   }
   if (in_dtype == DTYPE_BF16 && out_dtype == DTYPE_F32)
     return gemm_launch<__nv_bfloat16, float>(y, x, w, M, N, K, ldx, ldw, ldy, s);
