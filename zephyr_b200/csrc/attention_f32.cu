@@ -3,17 +3,24 @@
 //
 // The general kernel reads one key value per lane and multiply-add from shared memory; here a CTA takes F_ROWS query
 // rows (the (token, head) pairs of neighbouring tokens and one key/value head) against F_KEYS keys at a time, a thread
-// 4 x 4 scores and 4 x D/16 outputs, so that a 16-byte read serves 8 to 11 multiply-adds.  Bound by those reads'
-// latency and by the exponentials between the two products, with two CTAs an SM at most (700 tokens: 192 CTAs, 0.65 of a
-// wave; shared memory busy for 52 % of the time).  Keys lie transposed ([channel][key]), values as they are; a warp owns
-// eight rows across all keys, so the weights go from one product to the other inside a warp.  700 tokens, 16 heads over 8 of 128:
-// 166 us, 776 in the general kernel.  Every row with several tokens runs here, so that its result hangs on that row alone: behind
-// a context of 600 two tokens take 142 us (328 in the general kernel) and fifteen 143 (553); two tokens of a new prompt, most
-// of whose tile is empty, take 22 instead of 16 us, eight rows of sixteen 31 instead of 37.
+// 4 x 4 scores and 4 x D/16 outputs, so that a 16-byte read serves 8 to 11 multiply-adds, two of them an instruction.
+// Bound at few tiles by the serial chain of the tile that sees most keys, alone on its SM: of 10 us a step of 64 keys the
+// scores take 4, the weighted values 3, the rest barriers, exponentials and shuffles.  Two CTAs an SM are worth
+// more than registers at long prompts (4000 tokens 1699 us, 2086 with one CTA of 212 registers).  Keys lie transposed
+// ([channel][key]), values as they are; a warp owns eight rows across all keys, so the weights go from one product
+// to the other inside a warp.  A weight of zero skips its value; a tile of which a warp sees every key needs no look at
+// that.  Where a key lies in the cache is worked out once, by the lane that fetches it, and read from shared memory for
+// its value (eight divisions and table reads a thread otherwise: 700 tokens 148 us against 125).  A lane sums the weights of its own
+// keys and the lanes' sums meet at the end (125 us against 122).
+// 700 tokens, 16 heads over 8 of 128: 122 us (one multiply-add an instruction and every value's place worked out 167, the
+// general kernel 776); 4000 tokens 1678 (2241).  Every row with several tokens runs here, so that its result hangs on
+// that row alone: two tokens behind a context of 600 take 97 us (136; the general kernel 328), two tokens of a new prompt,
+// most of whose tile is empty, 16.6 (18.6; 16), eight rows of sixteen 23 (25; 37).
 //
 // Masks: causal, a window, a chunk (key and query in the same run of `chunk` positions); `sinks` join the softmax's
 // denominators; `softcap` > 0 bounds the scaled scores.  Keys and values have one width, a multiple of 4 up to 128.
 #include <initializer_list>
+#include <type_traits>
 
 #include "common.cuh"
 #include "mma.cuh"
@@ -23,6 +30,17 @@ namespace zb {
 constexpr int F_ROWS = 64;      // (token, head) pairs of a CTA
 constexpr int F_KEYS = 64;      // keys of a tile
 constexpr int F_THREADS = 256;
+
+// to[0..3] += a * b[0..3], two multiply-adds an instruction.
+__device__ __forceinline__ void multiply_add(float* to, float a, const float* b) {
+  unsigned long long twice;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(twice) : "f"(a));
+#pragma unroll
+  for (int pair = 0; pair < 2; ++pair)
+    asm("fma.rn.f32x2 %0, %1, %2, %0;"
+        : "+l"(*reinterpret_cast<unsigned long long*>(to + 2 * pair))
+        : "l"(twice), "l"(*reinterpret_cast<const unsigned long long*>(b + 2 * pair)));
+}
 
 struct AttentionF32Args {
   const float* q;           // [T, nh * d]
@@ -49,6 +67,7 @@ __global__ void __launch_bounds__(F_THREADS, 2) paged_attention_f32_kernel(const
   float* k_s = q_s + D * F_ROWS;              // [D][F_KEYS]
   float* v_s = k_s + D * F_KEYS;              // [F_KEYS][D]
   float* p_s = v_s + F_KEYS * D;              // [F_KEYS][F_ROWS]
+  auto base_s = reinterpret_cast<long long*>(p_s + F_KEYS * F_ROWS);   // [F_KEYS]: where a key begins in the cache, or -1
   constexpr int VG4 = D / 64;                 // groups of four output columns a thread
   constexpr int K_PER = F_KEYS * (D / 8) / F_THREADS;      // 32-byte pieces of a key tile a thread moves
   // The last tiles of the list see the most keys and run first.
@@ -105,6 +124,7 @@ __global__ void __launch_bounds__(F_THREADS, 2) paged_attention_f32_kernel(const
     const int pos = k0 + tid % F_KEYS;        // F_THREADS is a multiple of F_KEYS: one key a thread
     const bool ok = locate(pos, base);
     const int turn = kv_swizzle(pos, chunks);
+    if (tid < F_KEYS) base_s[tid] = ok ? static_cast<long long>(base) : -1;
 #pragma unroll
     for (int i = 0; i < K_PER; ++i)
 #pragma unroll
@@ -129,16 +149,18 @@ __global__ void __launch_bounds__(F_THREADS, 2) paged_attention_f32_kernel(const
   };
   auto copy_values = [&](int k0) {
     constexpr int per_row = D / 4;
-    for (int e = tid; e < F_KEYS * per_row; e += F_THREADS) {
-      const int j = e / per_row, c = e - j * per_row, pos = k0 + j;
-      size_t base = 0;
-      const bool ok = c < chunks && locate(pos, base);
-      cp_async_16(v_s + j * D + 4 * c, ok ? a.kv_cache + base + value_part + 4 * (c ^ kv_swizzle(pos, chunks)) : a.kv_cache, ok);
+#pragma unroll
+    for (int i = 0; i < F_KEYS * per_row / F_THREADS; ++i) {
+      const int e = tid + i * F_THREADS, j = e / per_row, c = e % per_row;
+      const long long base = base_s[j];
+      const bool ok = c < chunks && base >= 0;
+      cp_async_16(v_s + j * D + 4 * c, ok ? a.kv_cache + base + value_part + 4 * (c ^ kv_swizzle(k0 + j, chunks)) : a.kv_cache, ok);
     }
     cp_async_commit();
   };
 
-  float m[4], l[4], acc[4][4 * VG4];
+  float m[4], l[4];
+  alignas(16) float acc[4][4 * VG4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     m[i] = -INFINITY;
@@ -161,18 +183,16 @@ __global__ void __launch_bounds__(F_THREADS, 2) paged_attention_f32_kernel(const
     store_keys();
     copy_values(k0);
     __syncthreads();
-    float s[4][4];
+    alignas(16) float s[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.0f;
-#pragma unroll 8
+#pragma unroll 16
     for (int c = 0; c < D; ++c) {
-      float q4[4], k4[4];
+      alignas(16) float q4[4], k4[4];
       *reinterpret_cast<float4*>(q4) = *reinterpret_cast<const float4*>(q_s + c * F_ROWS + ty * 4);
       *reinterpret_cast<float4*>(k4) = *reinterpret_cast<const float4*>(k_s + c * F_KEYS + tx * 4);
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) s[i][j] = fmaf(q4[i], k4[j], s[i][j]);
+      for (int i = 0; i < 4; ++i) multiply_add(s[i], q4[i], k4);
     }
     if (k0 + F_KEYS < hi) fetch_keys(k0 + F_KEYS);
     float corr[4];
@@ -199,38 +219,46 @@ __global__ void __launch_bounds__(F_THREADS, 2) paged_attention_f32_kernel(const
         s[i][j] = expf(s[i][j] - from);
         sum += s[i][j];
       }
-#pragma unroll
-      for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
       l[i] = fmaf(l[i], corr[i], sum);
       m[i] = new_m;
     }
+    bool dense = true;                        // every row of the warp sees every key of the tile
+#pragma unroll
+    for (int i = 0; i < 4; ++i) dense = dense && s[i][0] > 0.0f && s[i][1] > 0.0f && s[i][2] > 0.0f && s[i][3] > 0.0f;
+    dense = __all_sync(0xffffffffu, dense);
+    // Weights: a key's groups of four rows are turned by its group of four, so that a warp's stores meet all banks.
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-      *reinterpret_cast<float4*>(p_s + (tx * 4 + j) * F_ROWS + ty * 4) = make_float4(s[0][j], s[1][j], s[2][j], s[3][j]);
+      *reinterpret_cast<float4*>(p_s + (tx * 4 + j) * F_ROWS + ((ty + tx) & 15) * 4) = make_float4(s[0][j], s[1][j], s[2][j], s[3][j]);
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int c = 0; c < 4 * VG4; ++c) acc[i][c] *= corr[i];
     cp_async_wait<0>();
     __syncthreads();                          // the values have landed; the weights of a row stay within its warp
-#pragma unroll 4
-    for (int j = 0; j < F_KEYS; ++j) {
-      float p4[4];
-      *reinterpret_cast<float4*>(p4) = *reinterpret_cast<const float4*>(p_s + j * F_ROWS + ty * 4);
+    auto weigh = [&](auto all) {
+#pragma unroll 8
+      for (int j = 0; j < F_KEYS; ++j) {
+        float p4[4];
+        *reinterpret_cast<float4*>(p4) = *reinterpret_cast<const float4*>(p_s + j * F_ROWS + ((ty + j / 4) & 15) * 4);
 #pragma unroll
-      for (int c = 0; c < VG4; ++c) {
-        const float4 v = *reinterpret_cast<const float4*>(v_s + j * D + c * 64 + tx * 4);
+        for (int c = 0; c < VG4; ++c) {
+          alignas(16) float v4[4];
+          *reinterpret_cast<float4*>(v4) = *reinterpret_cast<const float4*>(v_s + j * D + c * 64 + tx * 4);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          if (p4[i] == 0.0f) continue;        // a key that the row does not see: its value may be anything
-          acc[i][4 * c] = fmaf(p4[i], v.x, acc[i][4 * c]);
-          acc[i][4 * c + 1] = fmaf(p4[i], v.y, acc[i][4 * c + 1]);
-          acc[i][4 * c + 2] = fmaf(p4[i], v.z, acc[i][4 * c + 2]);
-          acc[i][4 * c + 3] = fmaf(p4[i], v.w, acc[i][4 * c + 3]);
+          for (int i = 0; i < 4; ++i)
+            if (all.value || p4[i] != 0.0f) multiply_add(acc[i] + 4 * c, p4[i], v4);   // (what a row does not see may be anything)
         }
       }
-    }
+    };
+    if (dense) weigh(std::true_type());
+    else weigh(std::false_type());
   }
+  // A lane has summed the weights of its own keys.
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) l[i] += __shfl_xor_sync(0xffffffffu, l[i], o);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int r = ty * 4 + i;
@@ -257,7 +285,7 @@ __global__ void __launch_bounds__(F_THREADS, 2) paged_attention_f32_kernel(const
 
 template <int D>
 static int attention_f32_launch(const AttentionF32Args& a, cudaStream_t s) {
-  constexpr int smem = static_cast<int>(sizeof(float)) * (D * F_ROWS + 2 * D * F_KEYS + F_KEYS * F_ROWS);
+  constexpr int smem = static_cast<int>(sizeof(float)) * (D * F_ROWS + 2 * D * F_KEYS + F_KEYS * F_ROWS) + 8 * F_KEYS;
   auto kernel = paged_attention_f32_kernel<D>;
   if (cuda_failed(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem))) return ERR_CUDA;
   kernel<<<dim3(a.n_tiles * a.subs * a.nkv), F_THREADS, smem, s>>>(a);
