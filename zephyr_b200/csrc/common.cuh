@@ -242,6 +242,9 @@ inline int launch_result() {
 // reads is written, before that.  `let_dependents_launch`, called after the wait, lets the next
 // kernel start in the same way (called before the wait, the order of completion would no longer be
 // a chain).  In a kernel launched the ordinary way both are no-ops.
+// In such a kernel no pointer to what another kernel writes is declared __restrict__ for reading (weights, tables and what the
+// kernel alone writes may be): that declaration promises that the data stays as it is for as long as the kernel runs, and lets it be
+// read through the cache that does not see other kernels' writes, or ahead of the wait.
 __device__ __forceinline__ void wait_for_prior_grids() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -46,8 +46,7 @@ template <> __device__ __forceinline__ void store_vec<__nv_bfloat16>(__nv_bfloat
 
 // ----------------------------------------------------------------------------- embedding
 template <typename T, bool VECTOR>
-__global__ void embedding_kernel(T* __restrict__ out, const T* __restrict__ table, const int* __restrict__ ids,
-                                 int H, int V, int* status) {
+__global__ void embedding_kernel(T* __restrict__ out, const T* __restrict__ table, const int* ids, int H, int V, int* status) {
   wait_for_prior_grids();
   let_dependents_launch();
   const int t = blockIdx.x;
@@ -70,8 +69,7 @@ __global__ void embedding_kernel(T* __restrict__ out, const T* __restrict__ tabl
 // Rows of x picked by index (the hidden states whose logits are wanted): 16 bytes a thread where rows are whole aligned pieces,
 // with a CTA for every 128 of them (12 rows of 2048: 6.9 us a value at a time, now below 2.9).
 template <typename T, bool VECTOR>
-__global__ void gather_rows_kernel(T* __restrict__ out, const T* __restrict__ x, const int* __restrict__ rows,
-                                   int H, int num_src_rows, int* status) {
+__global__ void gather_rows_kernel(T* __restrict__ out, const T* x, const int* rows, int H, int num_src_rows, int* status) {
   wait_for_prior_grids();
   let_dependents_launch();
   const int r = blockIdx.x;
@@ -96,8 +94,7 @@ __global__ void gather_rows_kernel(T* __restrict__ out, const T* __restrict__ x,
 // rounding, stored back) and the norm is taken of the stored value, so that the fused and the
 // separate form give the same bits.
 template <typename T, bool ADD, bool VECTOR>
-__global__ void rmsnorm_kernel(T* __restrict__ out, T* __restrict__ x, const T* __restrict__ delta,
-                               const void* __restrict__ w, int w_dtype, float eps, int H,
+__global__ void rmsnorm_kernel(T* __restrict__ out, T* x, const T* delta, const void* __restrict__ w, int w_dtype, float eps, int H,
                                long long x_stride, long long out_stride) {
   wait_for_prior_grids();
   let_dependents_launch();
@@ -159,9 +156,8 @@ constexpr int NORM_ROWS_PER_BLOCK = 4;
 
 template <int V, bool ADD>
 __global__ void __launch_bounds__(NORM_ROWS_PER_BLOCK * 32)
-rmsnorm_warp_rows_kernel(__nv_bfloat16* __restrict__ out, __nv_bfloat16* __restrict__ x,
-                         const __nv_bfloat16* __restrict__ delta, const void* __restrict__ w, int w_dtype, float eps,
-                         int rows, int H, long long x_stride, long long out_stride) {
+rmsnorm_warp_rows_kernel(__nv_bfloat16* __restrict__ out, __nv_bfloat16* x, const __nv_bfloat16* delta,
+                         const void* __restrict__ w, int w_dtype, float eps, int rows, int H, long long x_stride, long long out_stride) {
   wait_for_prior_grids();
   let_dependents_launch();
   const int lane = threadIdx.x & 31, row = blockIdx.x * NORM_ROWS_PER_BLOCK + (threadIdx.x >> 5);
@@ -356,8 +352,7 @@ __global__ void add_bias_kernel(T* __restrict__ y, long long ldy, const void* __
 // is read once, and eight rows at a time: 2125 x 2048 float32 in
 // 5.2 us; a value a thread, with a division each, took 13.4.
 template <typename T>
-__global__ void __launch_bounds__(256) add_bias_vec_kernel(T* __restrict__ y, long long ldy, const float* __restrict__ bias,
-                                                           int T_, int N) {
+__global__ void __launch_bounds__(256) add_bias_vec_kernel(T* y, long long ldy, const float* __restrict__ bias, int T_, int N) {
   wait_for_prior_grids();
   let_dependents_launch();
   constexpr int N_ = Vec<T>::N;

@@ -172,12 +172,12 @@ __global__ void qk_norm_rope_cache_kernel(T* __restrict__ q_out, const T* __rest
 // prompt's tokens make half as many warps: the kernel is bound by those rounds, not by bytes.
 template <int HD, int E>
 __global__ void __launch_bounds__(ROPE_WARPS * 32)
-qk_norm_rope_cache_wide_kernel(__nv_bfloat16* __restrict__ q_out, const __nv_bfloat16* __restrict__ qkv,
+qk_norm_rope_cache_wide_kernel(__nv_bfloat16* __restrict__ q_out, const __nv_bfloat16* qkv,
                                long long qkv_stride, const void* __restrict__ q_norm_w,
                                const void* __restrict__ k_norm_w, int w_dtype, float eps,
                                const float* __restrict__ cos_table, const float* __restrict__ sin_table,
-                               int max_positions, const int* __restrict__ positions,
-                               const int* __restrict__ token_row, CacheView cache, int nh, int nkv, int* status) {
+                               int max_positions, const int* positions,
+                               const int* token_row, CacheView cache, int nh, int nkv, int* status) {
   constexpr int LANES = HD / (2 * E), HEADS_PER_WARP = 32 / LANES, HALF = HD / 2, WORDS = E / 2;
   const int t = blockIdx.x;
   const int lane = threadIdx.x & 31, sub = lane % LANES;
