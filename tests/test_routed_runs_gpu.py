@@ -79,3 +79,15 @@ def test_many_rows_and_few_outputs(ops, cuda_device, rows, outputs, k, out_dtype
     expected = x.double() @ w.double().T
     # float32: k sums of products of about k^-1/2; bfloat16 rounds values of up to six.
     assert got.dtype == out_dtype and (got.double() - expected).abs().max() <= (2.0 ** -6 if out_dtype == torch.bfloat16 else 2e-5)
+
+
+@pytest.mark.parametrize("outputs,k", [(18, 2048), (18, 4096), (9, 1000), (24, 256), (1, 7168)])
+def test_a_routers_logits_do_not_depend_on_the_step(ops, cuda_device, outputs, k):
+    """The same bits for a row in a step of a few tokens and of many."""
+    g = torch.Generator().manual_seed(34)
+    x, w = torch.randn(6000, k, generator=g).bfloat16().to(cuda_device), (torch.randn(outputs, k, generator=g) * k ** -0.5).bfloat16().to(cuda_device)
+    few = ops.linear(x[:8], w, out_dtype=torch.float32)
+    for rows in (65, 333, 777, 1000) if outputs % 8 == 0 else (65, 777, 2049, 4100, 6000):
+        before = ops.LAUNCH_COUNTS.get("gemm_small", 0)
+        got = ops.linear(x[:rows], w, out_dtype=torch.float32)
+        assert ops.LAUNCH_COUNTS["gemm_small"] == before + 1 and torch.equal(got[:8], few), rows

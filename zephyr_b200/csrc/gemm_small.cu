@@ -39,6 +39,7 @@ struct SmallGemmArgs {
   const __nv_bfloat16* x;
   const __nv_bfloat16* w;
   int M, N, K;
+  int cut_rows;                        // rows of the weight matrix, which with K say how K is cut: N, or M where the sides have changed
   long long ldx, ldw, ldy;
   long long ldn;                       // between two rows of w's outputs: 1, or what a transposed result takes (ungated, no activation)
   const __nv_bfloat16* token_rows;     // ACT_TOKEN_GATE: gelu(sum) * token_rows[token_ids[token] * token_stride + column]
@@ -254,7 +255,7 @@ int small_gemm_launch(const SmallGemmArgs& a, int ksplit, cudaStream_t stream) {
 
 template <int MT, typename TOut, bool SWIGLU, int ACT>
 int small_gemm_split_launch(const SmallGemmArgs& a, cudaStream_t stream) {
-  const SmallGemmSplit s = small_gemm_split(a.N, a.K);
+  const SmallGemmSplit s = small_gemm_split(a.cut_rows, a.K);
   if (s.warps == 8) return small_gemm_launch<1, 8, MT, TOut, SWIGLU, ACT>(a, s.ksplit, stream);
   // Up to 8 tokens and several waves of CTAs: 32 rows a CTA read the tokens half as often (151936 x 1024, 4 rows: 50 us
   // against 54; with 12 rows their registers cost more, 66 against 64).  The sums are the same.
@@ -296,7 +297,7 @@ static int small_gemm(void* y, const void* x, const void* w, int M, int N, int K
   a.y = y;
   a.x = static_cast<const __nv_bfloat16*>(x);
   a.w = static_cast<const __nv_bfloat16*>(w);
-  a.M = M; a.N = N; a.K = K; a.ldx = ldx; a.ldw = ldw; a.ldy = ldy; a.ldn = 1;
+  a.M = M; a.N = a.cut_rows = N; a.K = K; a.ldx = ldx; a.ldw = ldw; a.ldy = ldy; a.ldn = 1;
   a.gate = gate;
   auto s = static_cast<cudaStream_t>(stream);
   if (act == ACT_GELU)
@@ -319,9 +320,10 @@ ZB_API int zb_gemm_small(void* y, const void* x, const void* w, int M, int N, in
 }
 
 // y [rows, outputs] = x w^T for many rows and few outputs (a router's): the kernel's sides change places, x's rows are streamed as
-// its matrix and w's are its few rows, and the result is written transposed.  (Rows of 2048 x 18 outputs, float32 out, us, the
-// library's product / here: 65 rows 5.8 / 3.8, 777 12.5 / 4.4, 2048 12.5 / 5.8, 8192 18.5 / 13.3; 8 outputs, 777 rows 5.5 / 3.3, but 8192
-// rows of 4096 13.5 / 15.7; 32 outputs, 2048 rows 4.7 / 5.9.)
+// its matrix and w's are its few rows, and the result is written transposed.  K is cut as w alone says, so that a row's sums are the
+// same as in a step of a few rows.  (Rows of 2048 x 18 outputs, float32 out, us, the
+// library's product / here: 65 rows 6.3 / 3.9, 777 12.6 / 4.6, 2048 13 / 5.9, 5000 18.1 / 14.5, 8192 18.3 / 20; cut by the number of rows
+// the last two took 11.2 and 12.3.)
 ZB_API int zb_gemm_few_outputs(void* y, const void* x, const void* w, int rows, int outputs, int K, long long ldx, long long ldw,
                                long long ldy, int out_dtype, void* stream) {
   if (!zb_gemm_small_supported(outputs, rows, K)) return ERR_UNSUPPORTED;
@@ -332,7 +334,7 @@ ZB_API int zb_gemm_few_outputs(void* y, const void* x, const void* w, int rows, 
   a.y = y;
   a.x = static_cast<const __nv_bfloat16*>(w);
   a.w = static_cast<const __nv_bfloat16*>(x);
-  a.M = outputs; a.N = rows; a.K = K; a.ldx = ldw; a.ldw = ldx; a.ldy = 1; a.ldn = ldy;
+  a.M = a.cut_rows = outputs; a.N = rows; a.K = K; a.ldx = ldw; a.ldw = ldx; a.ldy = 1; a.ldn = ldy;
   auto s = static_cast<cudaStream_t>(stream);
   return out_dtype == DTYPE_F32 ? small_gemm_dispatch<float, false, ACT_NONE>(a, s) : small_gemm_dispatch<__nv_bfloat16, false, ACT_NONE>(a, s);
 }
@@ -356,7 +358,7 @@ ZB_API int zb_gemm_small_token_gate(void* y, const void* x, const void* w, const
   a.y = y;
   a.x = static_cast<const __nv_bfloat16*>(x);
   a.w = static_cast<const __nv_bfloat16*>(w);
-  a.M = M; a.N = N; a.K = K; a.ldx = ldx; a.ldw = ldw; a.ldy = ldy; a.ldn = 1;
+  a.M = M; a.N = a.cut_rows = N; a.K = K; a.ldx = ldx; a.ldw = ldw; a.ldy = ldy; a.ldn = 1;
   a.token_rows = static_cast<const __nv_bfloat16*>(table) + offset;
   a.token_stride = table_stride; a.token_ids = ids; a.vocab = vocab; a.status = status;
   return small_gemm_dispatch<__nv_bfloat16, false, ACT_TOKEN_GATE>(a, static_cast<cudaStream_t>(stream));
