@@ -91,3 +91,16 @@ def test_a_routers_logits_do_not_depend_on_the_step(ops, cuda_device, outputs, k
         before = ops.LAUNCH_COUNTS.get("gemm_small", 0)
         got = ops.linear(x[:rows], w, out_dtype=torch.float32)
         assert ops.LAUNCH_COUNTS["gemm_small"] == before + 1 and torch.equal(got[:8], few), rows
+
+
+@pytest.mark.parametrize("outputs,rows,own", [(16, 1024, True), (16, 1025, False), (24, 2048, False), (8, 2048, True), (8, 2049, False),
+                                              (18, 6144, True), (18, 6145, False), (25, 65, False)])
+def test_where_a_routers_product_runs(ops, cuda_device, outputs, rows, own):
+    """On the few-row kernel while the library's product is the slower one."""
+    g = torch.Generator().manual_seed(35)
+    x, w = torch.randn(rows, 256, generator=g).bfloat16().to(cuda_device), torch.randn(outputs, 256, generator=g).bfloat16().to(cuda_device)
+    before = ops.LAUNCH_COUNTS.get("gemm_small", 0)
+    got = ops.linear(x, w, out_dtype=torch.float32)
+    assert ops.LAUNCH_COUNTS.get("gemm_small", 0) - before == int(own)
+    # float32 sums of 256 products of about one.
+    assert (got.double() - x.double() @ w.double().T).abs().max() <= 256 * 2.0 ** -20

@@ -1979,9 +1979,18 @@ def fused_chain(stages: Sequence[ChainStage], tokens: int, status: torch.Tensor,
 USE_LIBRARY_PRODUCTS = True     # off: every bfloat16 product of more than a few rows runs on this package's tcgen05 kernel
 
 
-# Products of more than 64 rows with up to so many outputs (a router's) run on the few-row kernel, its sides changed, where
-# the library's is slower: numbers of outputs that it has no aligned kernel for, whatever the rows, others up to so many rows.
-FEW_OUTPUTS, FEW_OUTPUTS_ROWS = 24, 4096
+FEW_OUTPUTS = 24
+
+
+def few_outputs_rows(outputs: int) -> int:
+    """Up to how many rows a product with so few outputs (a router's) runs on the few-row kernel, its sides changed: as long as the
+    library's product takes longer.  (us, the library's / here: 18 outputs, for which it has no aligned kernel, 5000 rows of 2048
+    18.1 / 14.5, 8192 18.2 / 20.0, 5000 of 4096 33 / 25, 8192 34 / 42; 8 outputs, 2048 rows of 2048 6.7 / 4.3, of 4096 10.8 / 8.0, 4096
+    of 4096 11.9 / 15.1; 16 outputs, 777 rows of 2048 5.9 / 3.8, of 4096 9.3 / 7.1, 2048 of 2048 4.8 / 7.3, of 4096 7.3 / 14.2; 24
+    outputs, 777 rows of 2048 5.4 / 4.5, 2048 5.0 / 5.8.)"""
+    if outputs > FEW_OUTPUTS:
+        return 0
+    return 6144 if outputs % 8 != 0 else 2048 if outputs <= 8 else 1024
 
 
 def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = None,
@@ -2000,8 +2009,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = Non
         return gemm_nt_simt(x, w, out_dtype)
     if x.shape[0] <= SMALL_GEMM_ROWS and gemm_small_supported(x, w):
         return gemm_small(x, w, out_dtype)
-    if (w.shape[0] <= FEW_OUTPUTS and (x.shape[0] <= FEW_OUTPUTS_ROWS or w.shape[0] % 8 != 0) and x.shape[0] > w.shape[0]
-            and gemm_small_supported(w, x)):
+    if w.shape[0] < x.shape[0] <= few_outputs_rows(w.shape[0]) and gemm_small_supported(w, x):
         out = torch.empty((x.shape[0], w.shape[0]), dtype=out_dtype or x.dtype, device=x.device)
         _check(library().zb_gemm_few_outputs(_ptr(out), _ptr(x), _ptr(w), x.shape[0], w.shape[0], x.shape[1], x.stride(0), w.stride(0),
                                              out.stride(0), DTYPE_CODE[out.dtype], _stream()), "gemm_small")
