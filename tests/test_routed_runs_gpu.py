@@ -104,3 +104,14 @@ def test_where_a_routers_product_runs(ops, cuda_device, outputs, rows, own):
     assert ops.LAUNCH_COUNTS.get("gemm_small", 0) - before == int(own)
     # float32 sums of 256 products of about one.
     assert (got.double() - x.double() @ w.double().T).abs().max() <= 256 * 2.0 ** -20
+
+
+def test_rows_that_share_memory(ops, cuda_device):
+    """One row seen as many, and rows that overlap, whatever kernel the number of outputs asks for."""
+    g = torch.Generator().manual_seed(36)
+    one, run, w = (torch.randn(*shape, generator=g).bfloat16().to(cuda_device) for shape in ((1, 64), (64 + 8 * 99,), (9, 64)))
+    for x in (one.expand(100, 64), run.as_strided((100, 64), (8, 1))):
+        for weight in (w, w[:1].expand(9, 64)):
+            got = ops.linear(x, weight, out_dtype=torch.float32)
+            # float32 sums of 64 products of about one.
+            assert (got.double() - x.double() @ weight.double().T).abs().max() <= 64 * 2.0 ** -20

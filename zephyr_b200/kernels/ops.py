@@ -2009,7 +2009,8 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = Non
         return gemm_nt_simt(x, w, out_dtype)
     if x.shape[0] <= SMALL_GEMM_ROWS and gemm_small_supported(x, w):
         return gemm_small(x, w, out_dtype)
-    if w.shape[0] < x.shape[0] <= few_outputs_rows(w.shape[0]) and gemm_small_supported(w, x):
+    if (w.shape[0] < x.shape[0] <= few_outputs_rows(w.shape[0]) and min(x.stride(0), w.stride(0)) >= x.shape[1]   # (rows side by side)
+            and gemm_small_supported(w, x)):
         out = torch.empty((x.shape[0], w.shape[0]), dtype=out_dtype or x.dtype, device=x.device)
         _check(library().zb_gemm_few_outputs(_ptr(out), _ptr(x), _ptr(w), x.shape[0], w.shape[0], x.shape[1], x.stride(0), w.stride(0),
                                              out.stride(0), DTYPE_CODE[out.dtype], _stream()), "gemm_small")
