@@ -46,3 +46,32 @@ def test_whole_contexts(ops, cuda_device, nh, nkv, ctx, window, sink):
             # Weights and the result are rounded to bfloat16, 2^-9 each of values up to four.
             for split in got:
                 assert (got[split][r].double().cpu().view(nh, hd)[h] - expected).abs().max() <= 3.2e-2, (split, r, h)
+
+
+@pytest.mark.parametrize("ctx,bound,window,whole", [
+    ([169] * 12, 4096, 0, True), ([1000] * 6 + [1020] * 6, 1024, 0, True), ([700, 690, 20, 640, 64, 650], 1024, 0, True),
+    ([4095] + [99] * 11, 4096, 0, False), ([20] * 12 + [3999], 4096, 0, False), ([1999] + [99] * 7, 2000, 0, False),
+    ([4095] + [99] * 11, 4096, 100, True)])
+def test_contexts_of_unequal_lengths(ops, cuda_device, ctx, bound, window, whole):
+    """One item a (row, key/value head) pair while the contexts are near each other in length; spread over all CTAs where one CTA would
+    stream on alone.  The lengths, not the bound on them that a captured step knows, decide."""
+    nh, nkv, hd, n = 16, 8, 128, len(ctx)
+    q, cache, meta, Ks, Vs, qs = build_paged_case(cuda_device, torch.bfloat16, nh, nkv, hd, 16, [1] * n, ctx, 520)
+    rows, status, out = torch.arange(n, dtype=torch.int32, device=cuda_device), ops.new_status(cuda_device), torch.full_like(q, float("nan"))
+    trace = torch.zeros((1024, 8), dtype=torch.int32, device=cuda_device)
+    ops.paged_decode_trace(trace)
+    for _ in range(2):                   # (the counters are left as they were found)
+        ops.paged_decode(q, cache, meta["table"], rows, meta["row_q_start"], meta["row_ctx"], bound, nh, nkv, hd, window, 1 / math.sqrt(hd),
+                         status, out)
+    ops.paged_decode_trace(None)
+    ops.check_status(status)
+    lo = [max(0, c + 1 - window) if window else 0 for c in ctx]
+    tiles = [-(-(c + 1) // 32) - l // 32 for c, l in zip(ctx, lo)]
+    most = max(tiles) if whole else -(-sum(tiles) * nkv // ops._sm_count())
+    assert int(trace[:, 6].max()) == most                             # tiles of the CTA that has the most
+    for r in range(n):
+        for h in range(nh):
+            s = qs[r][0, h].double() @ Ks[r][lo[r]:, h // 2].double().T / math.sqrt(hd)
+            expected = torch.softmax(s, -1) @ Vs[r][lo[r]:, h // 2].double()
+            # Weights and the result are rounded to bfloat16, 2^-9 each of values up to four.
+            assert (out[r].double().cpu().view(nh, hd)[h] - expected).abs().max() <= 3.2e-2, (r, h)

@@ -46,6 +46,7 @@ constexpr int DEC_TILE = 32;             // positions per tile: one consumer war
 constexpr int DEC_MAX_GROUP = 16;        // query heads per key/value head that fit one MMA tile
 constexpr int DEC_WAIT_LIMIT = 1 << 24;  // polls of an mbarrier before a warp gives up and reports
 constexpr int DEC_SMEM_BUDGET = 227 * 1024 - 1024;
+constexpr int DEC_UNEVEN_LIMIT = 3000;    // tiles of 128-value heads: see zb_paged_decode
 constexpr int DEC_MAX_BALANCED_GRID = 256;  // CTAs of a launch with balanced items: the scratch holds two slots for each
 
 struct DecodeArgs {
@@ -61,6 +62,8 @@ struct DecodeArgs {
   int* counters;                 // [n_rows, nkv] zero on entry, zero again on exit
   int max_blocks, page_shift, num_pages, num_rows, n_rows;
   int nh, nkv, window, split_size, max_splits, ring_slots, item_pages;
+  int uneven_limit;              // > 0: split_size covers whole contexts, and they are balanced items instead where the pair with the
+                                 // most tiles has more than this many hundredths of a tile beyond a hundredth of all pairs' tiles
   int chunk;                     // n > 0: the query (at position ctx_total - 1) sees only keys >= its position / n * n
   const float* sinks;            // null, or [nh]: exp(sinks[h]) joins the softmax's denominator of head h
   float scale_log2;              // scale * log2(e)
@@ -104,6 +107,10 @@ __device__ __forceinline__ int timer_ns() {
 //     begin inside one pair and end inside another, so a range owns two slots: slot 0 for a pair that
 //     began before the range, slot 1 for one that began inside it and goes on.  Every CTA streams
 //     the same number of tiles whatever the batch and the context lengths are.
+//   Either (uneven_limit > 0): whole contexts, one item a pair, where they are near each other in length, balanced where a CTA
+//     with the longest one would stream on alone.  Chosen here, from the lengths, which the host of a captured step does not know.
+//     What a launch does for that in front of its first copy shows in a step, where it starts cold: a warp's running sums of
+//     all rows cost 3 us there, two reductions a warp 0.7.
 struct DecodeItem {
   int r, row, kvh, ctx_total, begin, end, first_tile, n_tiles;
   int n_parts;          // items the pair is cut into (1: this item's result is the pair's result)
@@ -147,10 +154,11 @@ __device__ __forceinline__ void walker_init(ItemWalker& w) {
 }
 
 // The CTA's next item, the same sequence for every warp that asks.  `prefix` (balanced only): the
-// first global tile of every row, n_rows + 1 entries; `per_range`: tiles per range.
+// first global tile of every row, n_rows + 1 entries; `per_range`: tiles per range, 0 for fixed splits.
+template <bool EITHER>
 __device__ __forceinline__ bool next_item(const DecodeArgs& a, const int* prefix, int per_range, ItemWalker& w,
                                           DecodeItem& it) {
-  if (a.split_size > 0) {
+  if (EITHER ? per_range == 0 : a.split_size > 0) {
     const int n_items = a.n_rows * a.nkv * a.max_splits;
     while (w.next < n_items) {
       const int id = w.next;
@@ -210,8 +218,9 @@ __device__ __forceinline__ bool next_item(const DecodeArgs& a, const int* prefix
 }
 
 // Slot of the k-th of the pair's partial results.
+template <bool EITHER>
 __device__ __forceinline__ int part_slot(const DecodeArgs& a, const DecodeItem& it, int k, int per_range) {
-  return a.split_size > 0 ? it.merge_first + k : balanced_slot(it.pair_start, it.merge_first + k, per_range);
+  return !EITHER && a.split_size > 0 ? it.merge_first + k : balanced_slot(it.pair_start, it.merge_first + k, per_range);
 }
 
 __device__ __forceinline__ void consumer_barrier() {      // the 128 consumer threads only
@@ -383,8 +392,8 @@ __device__ __noinline__ void merge_many_parts(const MergeJob job, float* merge_o
 }
 
 // DISTANT: with the distance bias.  A form of its own: the bias's registers in the plain form cost a decode step of
-// the 0.6B shape 2.8 %.
-template <int HD, bool DISTANT>
+// the 0.6B shape 2.8 %.  EITHER: whole contexts or balanced items, as the lengths are.
+template <int HD, bool DISTANT, bool EITHER>
 __global__ void __launch_bounds__(DEC_THREADS, 1)
 paged_decode_kernel(const DecodeArgs a) {
   static_assert(HD % 32 == 0 && HD <= 128, "head sizes 32, 64, 96, 128");
@@ -434,6 +443,10 @@ paged_decode_kernel(const DecodeArgs a) {
     fence_barrier_init();
   }
   // Rows that do not exist are reported once and own no tiles.
+  const auto tiles_of = [&](int r, int row, int guess) {
+    const int ctx_total = (row == r ? guess : a.row_ctx[row]) + 1;
+    return (ctx_total + DEC_TILE - 1) / DEC_TILE - first_visible(ctx_total, a.window, a.chunk) / DEC_TILE;
+  };
   for (int r = threadIdx.x; r < a.n_rows; r += DEC_THREADS) {
     // In a step of decoding requests only, row r is request r: its context is asked for together with
     // its number, which saves a round trip to memory at the head of every launch.
@@ -443,22 +456,26 @@ paged_decode_kernel(const DecodeArgs a) {
       asm volatile("prefetch.global.L1 [%0];\n" ::"l"(a.row_ctx + r));
     const bool ok = row >= 0 && row < a.num_rows;
     if (!ok) report(a.status, STATUS_ROW_OUT_OF_RANGE, row, r);
-    if (a.split_size == 0) {
-      int tiles = 0;
-      if (ok) {
-        const int ctx_total = (row == r ? guess : a.row_ctx[row]) + 1;
-        const int lo = first_visible(ctx_total, a.window, a.chunk);
-        tiles = (ctx_total + DEC_TILE - 1) / DEC_TILE - lo / DEC_TILE;
-      }
-      prefix[r + 1] = tiles * a.nkv;
-    }
+    if (EITHER || a.split_size == 0) prefix[r + 1] = ok ? tiles_of(r, row, guess) * a.nkv : 0;
   }
   __syncthreads();
-  if (threadIdx.x == 0 && a.split_size == 0) {
+  bool balanced = a.split_size == 0;
+  if (EITHER) {                            // every warp for itself: the most tiles of a row, and all rows'
+    int longest = 0, all = 0;
+    for (int r = lane; r < a.n_rows; r += 32) {
+      longest = max(longest, prefix[r + 1]);
+      all += prefix[r + 1];
+    }
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    all = __reduce_add_sync(0xffffffffu, all);
+    balanced = 100LL * longest - static_cast<long long>(a.nkv) * all > static_cast<long long>(a.nkv) * a.uneven_limit;
+    if (balanced) __syncthreads();         // (the sums below change what the warps have read)
+  }
+  if (threadIdx.x == 0 && balanced) {
     prefix[0] = 0;
     for (int r = 0; r < a.n_rows; ++r) prefix[r + 1] += prefix[r];
   }
-  __syncthreads();
+  if (!EITHER || balanced) __syncthreads();
   fence_proxy_async();
   // Up to here nothing of an earlier kernel's output was read: the step's description is older than
   // any kernel of the step.  The queries and each row's newest key and value are an earlier kernel's
@@ -467,7 +484,8 @@ paged_decode_kernel(const DecodeArgs a) {
   // fills with old keys and values while the kernel before this one is still running.
   let_dependents_launch();
   // Balanced items: as many tiles per range as spread all tiles evenly over the CTAs.
-  const int per_range = a.split_size == 0 ? max(1, (prefix[a.n_rows] + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x)) : 0;
+  const int per_range = balanced ? max(1, (prefix[a.n_rows] + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x)) : 0;
+  if (EITHER && !balanced && blockIdx.x >= a.n_rows * a.nkv) return;      // (a CTA for balanced items that are not: its SM is free for the next kernel)
   const int page_size = 1 << a.page_shift;
   const long long page_stride = (a.keys_only ? 1LL : 2LL) * a.nkv * page_size * HD;
   const bool fused = a.qkv != nullptr;       // the new tokens' position encoding happens in this kernel
@@ -550,7 +568,7 @@ paged_decode_kernel(const DecodeArgs a) {
       __syncwarp();
       fence_proxy_async();       // the tile's bulk copies, issued next by this warp, read these rows
     };
-    while (next_item(a, prefix, per_range, walker, it)) {
+    while (next_item<EITHER>(a, prefix, per_range, walker, it)) {
       const int qb = item_seq & 1;
       if (me == 0) {
         if (!wait(&qempty[qb], ((item_seq >> 1) & 1) ^ 1)) {
@@ -645,7 +663,7 @@ paged_decode_kernel(const DecodeArgs a) {
   DecodeItem it;
   wait_for_prior_grids();      // the consumers write results, and read queries: both wait for the kernels before
   if (trace) trace[1] = trace[2] = trace[3] = timer_ns();
-  while (next_item(a, prefix, per_range, walker, it)) {
+  while (next_item<EITHER>(a, prefix, per_range, walker, it)) {
     const int qb = item_seq & 1;
     // A consumer whose wait runs out reports, raises the abort flag and keeps walking the items
     // without computing: the consumer barriers below need all four warps to the very end.
@@ -858,7 +876,7 @@ paged_decode_kernel(const DecodeArgs a) {
       MergeJob job;
       job.part_o = a.part_o; job.part_ml = a.part_ml; job.out = a.out + out_base;
       job.pair_start = it.pair_start;
-      job.n_parts = it.n_parts; job.merge_first = it.merge_first; job.per_range = per_range; job.split_size = a.split_size; job.g = g;
+      job.n_parts = it.n_parts; job.merge_first = it.merge_first; job.per_range = per_range; job.split_size = EITHER ? 0 : a.split_size; job.g = g;
       job.sinks = a.sinks; job.head0 = it.kvh * g;
       merge_many_parts<HD>(job, merge_o);
     } else {
@@ -871,7 +889,7 @@ paged_decode_kernel(const DecodeArgs a) {
           for (int k = 0; k < ROUND; ++k) {
             pm[k] = -INFINITY; pl[k] = 0.0f; po[k] = 0.0f;
             if (k < it.n_parts) {
-              const size_t slot = static_cast<size_t>(part_slot(a, it, k, per_range)) * g + h;
+              const size_t slot = static_cast<size_t>(part_slot<EITHER>(a, it, k, per_range)) * g + h;
               pm[k] = __ldcg(&a.part_ml[slot * 2]);
               pl[k] = __ldcg(&a.part_ml[slot * 2 + 1]);
               po[k] = __ldcg(&a.part_o[slot * HD + d]);
@@ -890,9 +908,9 @@ paged_decode_kernel(const DecodeArgs a) {
         } else {
           float mx = -INFINITY;
           for (int k = 0; k < it.n_parts; ++k)
-            mx = fmaxf(mx, __ldcg(&a.part_ml[(static_cast<size_t>(part_slot(a, it, k, per_range)) * g + h) * 2]));
+            mx = fmaxf(mx, __ldcg(&a.part_ml[(static_cast<size_t>(part_slot<EITHER>(a, it, k, per_range)) * g + h) * 2]));
           for (int k = 0; k < it.n_parts; ++k) {
-            const size_t slot = static_cast<size_t>(part_slot(a, it, k, per_range)) * g + h;
+            const size_t slot = static_cast<size_t>(part_slot<EITHER>(a, it, k, per_range)) * g + h;
             const float f = exp2f(__ldcg(&a.part_ml[slot * 2]) - mx);
             acc += __ldcg(&a.part_o[slot * HD + d]) * f;
             l += __ldcg(&a.part_ml[slot * 2 + 1]) * f;
@@ -932,12 +950,14 @@ int decode_launch(DecodeArgs& a, cudaStream_t stream) {
     return ERR_CUDA;
   sms = shared_sm_count(sms);
   // One persistent CTA per SM.  Fixed splits: max_splits items per pair.  Balanced: max_splits is the
-  // most tiles a pair can have, and an item is at most a pair's tiles or a range's, whichever is less.
+  // most tiles a pair can have, and an item is at most a pair's tiles or a range's, whichever is less.  Either: as for balanced
+  // items, but an item may be a pair's whole context.
   const long long units = static_cast<long long>(a.n_rows) * a.nkv * a.max_splits;
   int grid = static_cast<int>(units < sms ? units : sms);
-  if (a.split_size == 0 && grid > DEC_MAX_BALANCED_GRID) grid = DEC_MAX_BALANCED_GRID;
+  if ((a.split_size == 0 || a.uneven_limit > 0) && grid > DEC_MAX_BALANCED_GRID) grid = DEC_MAX_BALANCED_GRID;
   const long long item_tiles = a.split_size > 0 ? a.split_size / DEC_TILE + 1
                                                 : std::min<long long>(a.max_splits, (units + grid - 1) / grid) + 1;
+  if (a.uneven_limit > 0) a.max_splits = 1;
   const int item_pages = static_cast<int>((item_tiles * DEC_TILE) >> a.page_shift) + 2;
   if (decode_smem_bytes<HD>(2, g, item_pages, a.n_rows) > static_cast<size_t>(DEC_SMEM_BUDGET)) return ERR_UNSUPPORTED;
   int slots = 2;
@@ -945,7 +965,8 @@ int decode_launch(DecodeArgs& a, cudaStream_t stream) {
   a.ring_slots = slots;
   a.item_pages = item_pages;
   const size_t smem = decode_smem_bytes<HD>(slots, g, item_pages, a.n_rows);
-  auto kernel = a.bias_r1 != nullptr ? paged_decode_kernel<HD, true> : paged_decode_kernel<HD, false>;
+  auto kernel = a.uneven_limit > 0 ? (a.bias_r1 != nullptr ? paged_decode_kernel<HD, true, true> : paged_decode_kernel<HD, false, true>)
+                                   : (a.bias_r1 != nullptr ? paged_decode_kernel<HD, true, false> : paged_decode_kernel<HD, false, false>);
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
     return ERR_CUDA;
   return launch_dependent(kernel, dim3(grid), dim3(DEC_THREADS), smem, stream, false, a);
@@ -992,6 +1013,13 @@ ZB_API long long zb_paged_decode_balanced_scratch_floats(int nh, int nkv, int hd
 //     zb_paged_decode_scratch_floats(...) floats (contents irrelevant).
 //   split_size == 0: the tiles of all rows are spread evenly over the CTAs; max_splits >=
 //     ceil((longest context + 1) / 32); `scratch` holds zb_paged_decode_balanced_scratch_floats(...).
+//   `or_balanced` with split_size >= longest context + 1: one item a pair where the contexts are near each other in length, else
+//     balanced items; max_splits and `scratch` as for those.  The line: a CTA streams a tile in some 0.27 us, all of them together in
+//     0.0026 us, and balanced items cost about 8 us more for merges, so whole contexts are the shorter way while 100 tiles of the
+//     longest pair less all pairs' tiles stay below DEC_UNEVEN_LIMIT (at 128-value heads).
+//     (us, 16 heads over 8, one item a pair / balanced: 12 rows of 170 positions 7.1 / 13.0, 8 of 1024 11.7 / 15.2, 18 of 2500 33.4 /
+//     37.3, rows of 1000, 900, 300, 200 and four below 80 11.6 / 13.1; but one of 4096 beside eleven of 100 39.7 / 13.9, beside fifteen
+//     of 200 39.9 / 16.9, one of 4000 beside twelve of 20 38.8 / 23.3, one of 2000 beside seven of 100 20.5 / 12.1.)
 namespace zb {
 struct DecodeFusion {            // position encoding inside the kernel (see DecodeArgs)
   const void* qkv;
@@ -1009,12 +1037,12 @@ struct DecodeFusion {            // position encoding inside the kernel (see Dec
 static int paged_decode_entry(void* out, const void* q, const void* kv_cache, const int* block_table, int max_blocks,
                               int page_size, int num_pages, int num_rows, const int* rows, int n_rows,
                               const int* row_q_start, const int* row_ctx, int nh, int nkv, int hd, int window,
-                              float scale, int split_size, int max_splits, float* scratch, int* counters, int* status,
+                              float scale, int split_size, int max_splits, int or_balanced, float* scratch, int* counters, int* status,
                               const DecodeFusion* fusion, void* stream, int chunk = 0, const float* sinks = nullptr,
                               float softcap = 0.0f, int keys_only = 0, const float* bias_r1 = nullptr,
                               const float* bias_r2 = nullptr) {
   if ((bias_r1 == nullptr) != (bias_r2 == nullptr) || n_rows < 0 || max_splits <= 0 || split_size < 0 || split_size % DEC_TILE != 0 || page_size <= 0 || window < 0 ||
-      chunk < 0 || counters == nullptr || softcap < 0.0f || (keys_only && fusion != nullptr))
+      (or_balanced != 0 && (split_size <= 0 || max_splits > split_size / DEC_TILE)) || chunk < 0 || counters == nullptr || softcap < 0.0f || (keys_only && fusion != nullptr))
     return ERR_BAD_ARGUMENT;
   if (!zb_paged_decode_supported(nh, nkv, hd, DTYPE_BF16) || (page_size & (page_size - 1)) != 0) return ERR_UNSUPPORTED;
   if (n_rows == 0) return OK;
@@ -1027,12 +1055,13 @@ static int paged_decode_entry(void* out, const void* q, const void* kv_cache, co
   a.kv_cache = static_cast<const __nv_bfloat16*>(kv_cache);
   a.block_table = block_table; a.rows = rows; a.row_q_start = row_q_start; a.row_ctx = row_ctx;
   a.part_o = scratch;
-  a.part_ml = scratch + (split_size > 0 ? static_cast<size_t>(n_rows) * nh * max_splits * hd
+  a.part_ml = scratch + (split_size > 0 && or_balanced == 0 ? static_cast<size_t>(n_rows) * nh * max_splits * hd
                                         : static_cast<size_t>(2) * DEC_MAX_BALANCED_GRID * (nh / nkv) * hd);
   a.counters = counters;
   a.max_blocks = max_blocks; a.page_shift = page_shift; a.num_pages = num_pages; a.num_rows = num_rows;
   a.n_rows = n_rows;
   a.nh = nh; a.nkv = nkv; a.window = window; a.split_size = split_size; a.max_splits = max_splits;
+  a.uneven_limit = or_balanced ? DEC_UNEVEN_LIMIT * 128 / hd * (keys_only ? 2 : 1) : 0;
   a.chunk = chunk; a.sinks = sinks;
   a.trace = decode_trace();
   a.qkv = nullptr;
@@ -1076,10 +1105,10 @@ static int paged_decode_entry(void* out, const void* q, const void* kv_cache, co
 ZB_API int zb_paged_decode(void* out, const void* q, const void* kv_cache, const int* block_table, int max_blocks,
                            int page_size, int num_pages, int num_rows, const int* rows, int n_rows,
                            const int* row_q_start, const int* row_ctx, int nh, int nkv, int hd, int window,
-                           float scale, int split_size, int max_splits, float* scratch, int* counters, int* status,
+                           float scale, int split_size, int max_splits, int or_balanced, float* scratch, int* counters, int* status,
                            void* stream) {
   return paged_decode_entry(out, q, kv_cache, block_table, max_blocks, page_size, num_pages, num_rows, rows, n_rows,
-                            row_q_start, row_ctx, nh, nkv, hd, window, scale, split_size, max_splits, scratch, counters,
+                            row_q_start, row_ctx, nh, nkv, hd, window, scale, split_size, max_splits, or_balanced, scratch, counters,
                             status, nullptr, stream);
 }
 
@@ -1090,9 +1119,9 @@ ZB_API int zb_paged_decode_masked(void* out, const void* q, const void* kv_cache
                                   int n_rows, const int* row_q_start, const int* row_ctx, int nh, int nkv, int hd,
                                   int window, int chunk, float scale, float softcap, int keys_only,
                                   const float* sinks, const float* bias_r1, const float* bias_r2, int split_size,
-                                  int max_splits, float* scratch, int* counters, int* status, void* stream) {
+                                  int max_splits, int or_balanced, float* scratch, int* counters, int* status, void* stream) {
   return paged_decode_entry(out, q, kv_cache, block_table, max_blocks, page_size, num_pages, num_rows, rows, n_rows,
-                            row_q_start, row_ctx, nh, nkv, hd, window, scale, split_size, max_splits, scratch, counters,
+                            row_q_start, row_ctx, nh, nkv, hd, window, scale, split_size, max_splits, or_balanced, scratch, counters,
                             status, nullptr, stream, chunk, sinks, softcap, keys_only, bias_r1, bias_r2);
 }
 
@@ -1104,13 +1133,13 @@ ZB_API int zb_paged_decode_masked(void* out, const void* q, const void* kv_cache
 ZB_API int zb_paged_decode_fused(void* out, void* kv_cache, const int* block_table, int max_blocks, int page_size,
                                  int num_pages, int num_rows, const int* rows, int n_rows, const int* row_q_start,
                                  const int* row_ctx, int nh, int nkv, int hd, int window, float scale, int split_size,
-                                 int max_splits, float* scratch, int* counters, int* status, const void* qkv,
+                                 int max_splits, int or_balanced, float* scratch, int* counters, int* status, const void* qkv,
                                  long long qkv_stride, const void* q_norm_w, const void* k_norm_w, int norm_w_dtype,
                                  float norm_eps, const float* cos_table, const float* sin_table, int max_positions,
                                  void* stream) {
   const DecodeFusion fusion{qkv, qkv_stride, q_norm_w, k_norm_w, norm_w_dtype, norm_eps, cos_table, sin_table, max_positions};
   return paged_decode_entry(out, out, kv_cache, block_table, max_blocks, page_size, num_pages, num_rows, rows, n_rows,
-                            row_q_start, row_ctx, nh, nkv, hd, window, scale, split_size, max_splits, scratch, counters,
+                            row_q_start, row_ctx, nh, nkv, hd, window, scale, split_size, max_splits, or_balanced, scratch, counters,
                             status, &fusion, stream);
 }
 
@@ -1195,6 +1224,6 @@ ZB_API int zb_paged_decode_no_alloc(void* out, const void* q, const void* kv_cac
   const size_t counter_bytes = (static_cast<size_t>(n_rows) * nkv * sizeof(int) + 255) / 256 * 256;
   if (cudaMemsetAsync(scratch, 0, counter_bytes, static_cast<cudaStream_t>(stream)) != cudaSuccess) return ERR_CUDA;
   return zb_paged_decode(out, q, kv_cache, block_table, max_blocks, page_size, num_pages, num_rows, rows, n_rows,
-                         row_q_start, row_ctx, nh, nkv, hd, window, scale, split_size, max_splits,
+                         row_q_start, row_ctx, nh, nkv, hd, window, scale, split_size, max_splits, 0,
                          scratch + counter_bytes / sizeof(float), reinterpret_cast<int*>(scratch), status, stream);
 }

@@ -168,11 +168,11 @@ _SIGNATURES = {
     "zb_scaled_sum": [c_void_p, c_void_p, c_void_p, c_float, c_float, c_longlong, c_int, c_int, c_void_p],
     "zb_paged_decode_supported": [c_int, c_int, c_int, c_int],
     "zb_paged_decode": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int,
-                        c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p, c_void_p,
+                        c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_void_p, c_void_p,
                         c_void_p, c_void_p],
     "zb_paged_decode_masked": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int,
                                c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_int, c_void_p,
-                               c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p],
+                               c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p],
     "zb_paged_prefill_masked": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
                                 c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float,
                                 c_float, c_int, c_void_p, c_void_p, c_void_p],
@@ -181,7 +181,7 @@ _SIGNATURES = {
                                   c_float, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                                   c_int, c_void_p, c_void_p, c_void_p, c_void_p],
     "zb_paged_decode_fused": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p,
-                              c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
+                              c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                               c_longlong, c_void_p, c_void_p, c_int, c_float, c_void_p, c_void_p, c_int, c_void_p],
     "zb_paged_decode_set_trace": [c_void_p],
     "zb_paged_prefill_tile_tokens": [],
@@ -1482,7 +1482,8 @@ def decode_split_size(n_rows: int, nkv: int, max_context: int, visible: int | No
     costs 2 us (a handful of pairs, in fixed splits) to 6 us (balanced, where a CTA's share straddles two pairs) for the merge.
     (us, cut as below / not at all: 1 row of 160 positions 6.0 / 4.6, and of 310, though 6.4 / 5.8 back to back, 10.7 / 11.2 in a
     step; 8 rows of 310 9.7 / 6.2, of 600 13.2 / 8.2, of 2000 20.6 / 21.0, of 2620 22.7 / 26; 12 rows of 170 12.9 / 6.9, of 1500
-    21.8 / 19.4; 16 rows of 170 8.6 / 7.9; 18 of 2500 38.6 / 33.9.)
+    21.8 / 19.4; 16 rows of 170 8.6 / 7.9; 18 of 2500 38.6 / 33.9.)  That is for rows of one length: beyond a handful of pairs the kernel sees the
+    lengths and takes balanced items all the same where they are far apart (attention_decode.cu).
     Else, for a handful of rows (4 * pairs <= SMs), as many splits of a row's context as give every SM one item and none two (a
     second round of items would leave most SMs idle), and no split shorter than 128 positions.  For more, balanced items.
     Where a row's context is cut, and with that the last bits of its result, depends on how many rows are decoded beside it."""
@@ -1495,6 +1496,22 @@ def decode_split_size(n_rows: int, nkv: int, max_context: int, visible: int | No
         return 0
     split = -(-max_context // (sms // pairs))
     return max(128, -(-split // 32) * 32)
+
+
+def _decode_cut(n_rows: int, nh: int, nkv: int, hd: int, max_context: int, visible: int, position_bytes: int,
+                split_size: int | None) -> tuple[int, int, bool, int]:
+    """How a decode launch cuts its contexts: split size, items (or tiles) of a pair at most, whether the kernel may take balanced
+    items instead, and the floats of scratch that it needs."""
+    either = False
+    if split_size is None:
+        split_size = decode_split_size(n_rows, nkv, max_context, visible, position_bytes)
+        either = split_size >= max_context and 4 * n_rows * nkv > _sm_count()
+    _require(split_size >= 0, "split_size: None, 0 or a multiple of 32")
+    if split_size == 0 or either:
+        need = int(library().zb_paged_decode_balanced_scratch_floats(nh, nkv, hd))
+        return split_size, max(1, math.ceil(max_context / 32)), either, need
+    max_splits = max(1, math.ceil(max_context / split_size))
+    return split_size, max_splits, False, paged_decode_scratch_floats(n_rows, nh, hd, max_splits)
 
 
 _SM_COUNT: dict[int, int] = {}
@@ -1529,16 +1546,8 @@ def paged_decode(q: torch.Tensor, kv_cache: torch.Tensor, block_table: torch.Ten
     _require(out.shape == q.shape and out.dtype == q.dtype and out.is_contiguous(), "out must match q")
     pages, page_size = _cache_geometry(kv_cache, nkv, hd, 0, q.dtype) if keys_only else _check_cache(kv_cache, nkv, hd, q.dtype)
     n_rows = rows.numel()
-    if split_size is None:
-        visible = min([max_context] + [n for n in (window, chunk) if n > 0])
-        split_size = decode_split_size(n_rows, nkv, max_context, visible, (2 if keys_only else 4) * hd)
-    if split_size == 0:
-        # Balanced items: the tiles of all rows spread evenly over the CTAs (see attention_decode.cu).
-        split_size, max_splits = 0, max(1, math.ceil(max_context / 32))
-        need = int(library().zb_paged_decode_balanced_scratch_floats(nh, nkv, hd))
-    else:
-        max_splits = max(1, math.ceil(max_context / split_size))
-        need = paged_decode_scratch_floats(n_rows, nh, hd, max_splits)
+    split_size, max_splits, either, need = _decode_cut(n_rows, nh, nkv, hd, max_context, min([max_context] + [n for n in (window, chunk) if n > 0]),
+                                                       (2 if keys_only else 4) * hd, split_size)
     if scratch is None or counters is None:
         scratch, counters = _decode_workspace(q.device, need, n_rows * nkv)
     _require(scratch.dtype == torch.float32 and scratch.is_contiguous() and scratch.numel() >= need,
@@ -1554,12 +1563,12 @@ def paged_decode(q: torch.Tensor, kv_cache: torch.Tensor, block_table: torch.Ten
             _ptr(out), _ptr(q), _ptr(kv_cache), _ptr(block_table), block_table.shape[1], page_size, pages,
             block_table.shape[0], _ptr(rows), n_rows, _ptr(row_q_start), _ptr(row_ctx), nh, nkv, hd, int(window),
             int(chunk), float(scale), float(softcap), int(keys_only), _ptr(sinks), _ptr(r1), _ptr(r2), int(split_size), max_splits,
-            _ptr(scratch), _ptr(counters), _ptr(status), _stream()), "paged_decode")
+            int(either), _ptr(scratch), _ptr(counters), _ptr(status), _stream()), "paged_decode")
         return out
     _check(library().zb_paged_decode(
         _ptr(out), _ptr(q), _ptr(kv_cache), _ptr(block_table), block_table.shape[1], page_size, pages,
         block_table.shape[0], _ptr(rows), n_rows, _ptr(row_q_start), _ptr(row_ctx), nh, nkv, hd, int(window),
-        float(scale), int(split_size), max_splits, _ptr(scratch), _ptr(counters), _ptr(status), _stream()),
+        float(scale), int(split_size), max_splits, int(either), _ptr(scratch), _ptr(counters), _ptr(status), _stream()),
         "paged_decode")
     return out
 
@@ -1594,19 +1603,13 @@ def paged_decode_fused(qkv: torch.Tensor, kv_cache: torch.Tensor, block_table: t
                  and cos.is_contiguous() and sin.is_contiguous(), "cos/sin must be float32 [positions, head_dim/2]")
         max_positions = cos.shape[0]
     n_rows = rows.numel()
-    if split_size is None:
-        split_size = decode_split_size(n_rows, nkv, max_context, min([max_context] + ([window] if window > 0 else [])), 4 * hd)
-    if split_size == 0:
-        split_size, max_splits = 0, max(1, math.ceil(max_context / 32))
-        need = int(library().zb_paged_decode_balanced_scratch_floats(nh, nkv, hd))
-    else:
-        max_splits = max(1, math.ceil(max_context / split_size))
-        need = paged_decode_scratch_floats(n_rows, nh, hd, max_splits)
+    split_size, max_splits, either, need = _decode_cut(n_rows, nh, nkv, hd, max_context, min([max_context] + ([window] if window > 0 else [])),
+                                                       4 * hd, split_size)
     scratch, counters = _decode_workspace(qkv.device, need, n_rows * nkv)
     _check(library().zb_paged_decode_fused(
         _ptr(out), _ptr(kv_cache), _ptr(block_table), block_table.shape[1], page_size, pages, block_table.shape[0],
         _ptr(rows), n_rows, _ptr(row_q_start), _ptr(row_ctx), nh, nkv, hd, int(window), float(scale), int(split_size),
-        max_splits, _ptr(scratch), _ptr(counters), _ptr(status), _ptr(qkv), qkv.stride(0), _ptr(q_norm_w), _ptr(k_norm_w),
+        max_splits, int(either), _ptr(scratch), _ptr(counters), _ptr(status), _ptr(qkv), qkv.stride(0), _ptr(q_norm_w), _ptr(k_norm_w),
         w_code, float(eps), _ptr(cos), _ptr(sin), max_positions, _stream()), "paged_decode_fused")
     return out
 
