@@ -2,6 +2,7 @@
 rows that are keys and values at once, at the edges of its tiles, against a plain float64 attention.  The cache holds NaN wherever
 no request's row lies."""
 
+import dataclasses
 import math
 
 import pytest
@@ -121,3 +122,31 @@ def test_rows_that_are_keys_and_values(ops, cuda_device, nh, q_lens, ctx, page, 
         expected = plain(qs[r], kept, kept[..., :rank], ctx[r], 1 / math.sqrt(hd), sinks.cpu() if sink else None)
         assert (got[at:at + n].double().cpu().view(n, nh, hd)[..., :rank] - expected).abs().max() <= BOUND
         at += n
+
+
+def test_a_prompt_beside_decoding_rows(ops, cuda_device, tmp_path):
+    """Which form of a CTA a prompt's heads run in, and with that the last bits of the prompt's result, does not hang on the rows
+    that only decode beside it."""
+    from tiny_configs import tiny_config
+    from zephyr_b200 import write_random_model
+    from zephyr_b200.config import LayerCall, load_model_spec
+    from zephyr_b200.engine import ModelRunner, StepEntry
+    from zephyr_b200.parts import Model
+    from zephyr_b200.weights import Checkpoint
+
+    config = dataclasses.replace(tiny_config("A"), num_attention_heads=16, num_key_value_heads=8, head_dim=128, max_position_embeddings=4096)
+    folder = write_random_model(config, 5, tmp_path / "model", dtype=torch.bfloat16)
+    model = Model.load(load_model_spec(folder), Checkpoint(folder), torch.bfloat16, cuda_device)
+    runner, mixer, tokens = ModelRunner(model, 16, 300, 16), model.layers[0].mixer, 2048
+    projected = rand((tokens + 8, (16 + 2 * 8) * 128), torch.bfloat16, cuda_device, 530)
+    results = []
+    for beside in (0, 8):
+        names = [f"{beside} {i}" for i in range(beside + 1)]
+        for name in names:
+            assert runner.add_request(name)
+        ctx = runner.build_context([StepEntry(names[0], [1] * tokens)] + [StepEntry(name, [1]) for name in names[1:]])
+        before = ops.LAUNCH_COUNTS.get("paged_prefill_tc", 0)
+        results.append(mixer.core(projected[:tokens + beside], ctx, LayerCall(0, 0))[:tokens].clone())
+        assert ops.LAUNCH_COUNTS["paged_prefill_tc"] == before + 1
+    runner.check()
+    assert torch.equal(*results)

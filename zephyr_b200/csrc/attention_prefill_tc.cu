@@ -769,14 +769,15 @@ bool cache_tensor_map(const __nv_bfloat16* cache, long long rows, int hd, int bl
 }
 
 // How many tiles, from the longest on, run a head a CTA (see the top): all where even so every CTA gets an SM at once, or where
-// pairs of heads would not fill the SMs and rows are long, so that the longest chain is the launch's time; else none.  (us, heads
+// pairs of heads would not fill the SMs and rows are long, so that the longest chain is the launch's time; else none.  `tile_rows`:
+// the rows that these tiles come from (a step's decoding rows do not count: 2048 tokens beside four of them took 43 us in pairs).  (us, heads
 // singly / in pairs: one row of 300 tokens, 16/8 heads 11.3 / 13.9; one of 2048 33 / 43; 552 tokens behind 2048 beside a row
 // of 1496 39 / 51; but 16 rows of 128 35 / 23, 3000 tokens in a window of 1024 54 / 46, rows of 1531, 500 and 17 tokens, 32/8
 // heads, 53 / 41.  Halfway between, 25 to 75 % of the tiles, was never the best.)
-int tc_split_tiles(int nh, int nkv, int n_tiles, int num_rows, int sms) {
+int tc_split_tiles(int nh, int nkv, int n_tiles, int tile_rows, int sms) {
   if (nh / nkv % 2 != 0) return n_tiles;
   const long long single = static_cast<long long>(nh) * n_tiles;
-  return single <= sms || (single / 2 <= sms && n_tiles >= 4LL * num_rows) ? n_tiles : 0;
+  return single <= sms || (single / 2 <= sms && n_tiles >= 4LL * tile_rows) ? n_tiles : 0;
 }
 
 template <int FORM, int HD, bool SHARED>
@@ -820,6 +821,7 @@ ZB_API int zb_paged_prefill_tc_supported(int nh, int nkv, int hd, int value_dim,
 
 // Attention of the tiles' tokens (tiles of 128 new tokens of one request) over their requests'
 // pages; writes those tokens' rows of `out`.  Arguments as zb_paged_prefill_masked:
+// `tile_rows`: how many of the `num_rows` rows have tiles in the list;
 // `softcap` > 0 bounds the scaled scores by softcap * tanh(. / softcap); `keys_only`: a page holds keys alone
 // and they are the values too; `value_dim`: how many values of a row of `out` are wanted (the others may stay as they are);
 // `sinks` (null, or one float32 per query head) join the softmax's denominator;
@@ -827,7 +829,7 @@ ZB_API int zb_paged_prefill_tc_supported(int nh, int nkv, int hd, int value_dim,
 // `keep_first` (with a window): keys below this position stay visible.
 ZB_API int zb_paged_prefill_tc_masked(void* out, const void* q, const void* kv_cache, const int* block_table,
                                       int max_blocks, int page_size, int num_pages, int num_rows, const int* tile_row,
-                                      const int* tile_q0, int n_tiles, const int* row_q_start, const int* row_q_len,
+                                      const int* tile_q0, int n_tiles, int tile_rows, const int* row_q_start, const int* row_q_len,
                                       const int* row_ctx, int nh, int nkv, int hd, int window, int value_dim, int chunk, int keep_first,
                                       float scale, float softcap, int keys_only, const float* sinks, const float* bias_r1,
                                       const float* bias_r2, int* status, void* stream) {
@@ -841,12 +843,13 @@ ZB_API int zb_paged_prefill_tc_masked(void* out, const void* q, const void* kv_c
       reinterpret_cast<uintptr_t>(kv_cache) % 16 != 0)
     return ERR_BAD_ARGUMENT;
   if (n_tiles == 0) return OK;
+  if (tile_rows <= 0) return ERR_BAD_ARGUMENT;
   if (n_tiles > 65535) return ERR_UNSUPPORTED;
   int device = 0, sms = 0;
   if (cuda_failed(cudaGetDevice(&device)) || cuda_failed(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device))) return ERR_CUDA;
   PrefillTcArgs a;
   a.n_tiles = n_tiles;
-  a.n_split = tc_split_tiles(nh, nkv, n_tiles, num_rows, sms);
+  a.n_split = tc_split_tiles(nh, nkv, n_tiles, tile_rows, sms);
   a.q = static_cast<const __nv_bfloat16*>(q);
   a.out = static_cast<__nv_bfloat16*>(out);
   a.kv_cache = static_cast<const __nv_bfloat16*>(kv_cache);
@@ -878,6 +881,6 @@ ZB_API int zb_paged_prefill_tc(void* out, const void* q, const void* kv_cache, c
                                int n_tiles, const int* row_q_start, const int* row_q_len, const int* row_ctx, int nh,
                                int nkv, int hd, int window, float scale, int* status, void* stream) {
   return zb_paged_prefill_tc_masked(out, q, kv_cache, block_table, max_blocks, page_size, num_pages, num_rows, tile_row,
-                                    tile_q0, n_tiles, row_q_start, row_q_len, row_ctx, nh, nkv, hd, window, hd, 0, 0, scale, 0.0f, 0,
+                                    tile_q0, n_tiles, num_rows, row_q_start, row_q_len, row_ctx, nh, nkv, hd, window, hd, 0, 0, scale, 0.0f, 0,
                                     nullptr, nullptr, nullptr, status, stream);
 }

@@ -191,7 +191,7 @@ _SIGNATURES = {
     "zb_paged_prefill_tc_supported": [c_int, c_int, c_int, c_int, c_int, c_int, c_int],
     "zb_paged_prefill_tc_set_trace": [c_void_p],
     "zb_paged_prefill_tc_masked": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
-                                   c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float,
+                                   c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float,
                                    c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
     "zb_paged_prefill_tc": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
                             c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p],
@@ -1655,7 +1655,7 @@ def paged_prefill(q: torch.Tensor, kv_cache: torch.Tensor, block_table: torch.Te
                   keys_only: bool = False, keep_first: int = 0, pool: int = 0, pool_cache: torch.Tensor | None = None,
                   pool_table: torch.Tensor | None = None, cross_values: bool = False,
                   by_group: bool = False, distance_bias: tuple[torch.Tensor, torch.Tensor] | None = None,
-                  tensor_memory: bool = True, value_dim: int = 0) -> torch.Tensor:
+                  tensor_memory: bool = True, value_dim: int = 0, tile_rows: int | None = None) -> torch.Tensor:
     """Tensor-core attention for rows with several new tokens, cut into tiles of
     ``paged_prefill_tile_tokens()``; writes those tokens' rows of ``out``.  ``chunk``, ``sinks``, ``softcap`` and
     ``distance_bias`` as in ``paged_attention``, ``keys_only`` as its ``shared_kv``.  ``value_dim``: how many values of a row
@@ -1663,6 +1663,7 @@ def paged_prefill(q: torch.Tensor, kv_cache: torch.Tensor, block_table: torch.Te
     which 128 are read, runs on tcgen05 with the accumulators in tensor memory, other sizes on mma.sync.  ``keep_first``, ``pool`` with its store, and
     ``cross_values`` (``out`` is then [T, nh * nkv * hd], bfloat16 or float32) as in ``paged_attention``: the last two, and
     kept tokens or a chunk beside a distance bias, run on mma.sync, and so does everything without ``tensor_memory``.
+    ``tile_rows``: how many rows have tiles in the list (None: all of ``block_table``), which says how the tcgen05 kernel deals out heads.
     ``by_group``: every
     tile is one new token (the tiles of single-token rows), and a CTA's query rows are the heads that share a
     key/value head: a decoded token's keys and values stream once a group."""
@@ -1692,11 +1693,13 @@ def paged_prefill(q: torch.Tensor, kv_cache: torch.Tensor, block_table: torch.Te
                      and (hd == 128 or not (keep_first or chunk or r1 is not None))
                      and bool(library().zb_paged_prefill_tc_supported(nh, nkv, hd, value_dim or hd, int(keys_only), DTYPE_CODE[q.dtype],
                                                                       page_size)))
-    common = (_ptr(out), _ptr(q), _ptr(kv_cache), _ptr(block_table), block_table.shape[1], page_size, pages,
-              block_table.shape[0], _ptr(tile_row), _ptr(tile_q0), tile_row.numel(), _ptr(row_q_start), _ptr(row_q_len),
-              _ptr(row_ctx), nh, nkv, hd, int(window))
+    lists = (_ptr(out), _ptr(q), _ptr(kv_cache), _ptr(block_table), block_table.shape[1], page_size, pages,
+             block_table.shape[0], _ptr(tile_row), _ptr(tile_q0), tile_row.numel())
+    sizes = (_ptr(row_q_start), _ptr(row_q_len), _ptr(row_ctx), nh, nkv, hd, int(window))
+    common = lists + sizes
     if tensor_memory:
-        _check(library().zb_paged_prefill_tc_masked(*common, value_dim or hd, int(chunk), int(keep_first), float(scale), float(softcap), int(keys_only), _ptr(sinks),
+        tile_rows = block_table.shape[0] if tile_rows is None else int(tile_rows)
+        _check(library().zb_paged_prefill_tc_masked(*lists, tile_rows, *sizes, value_dim or hd, int(chunk), int(keep_first), float(scale), float(softcap), int(keys_only), _ptr(sinks),
                                                     _ptr(r1), _ptr(r2), _ptr(status), _stream()), "paged_prefill_tc")
     elif windowed or r1 is not None:
         _check(library().zb_paged_prefill_windowed(*common, int(chunk), float(scale), float(softcap), int(keys_only),

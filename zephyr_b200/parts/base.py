@@ -58,6 +58,10 @@ class StepContext:
     # What a layer hands on to later layers of the same step (values that they mix in), by a name their specs give.
     shared: dict[str, torch.Tensor] = field(default_factory=dict)
 
+    def rows_with_tiles(self, which: str) -> int:
+        """How many rows the tiles of ``tiles[(..., which)]`` come from."""
+        return {"all": self.num_rows, "single": self.num_decode_rows, "multi": self.num_rows - self.num_decode_rows}[which]
+
     def block_table(self, cache_id: int) -> torch.Tensor:
         return self.block_tables[self.group_of_cache[cache_id]]
 

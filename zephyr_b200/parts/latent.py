@@ -187,7 +187,7 @@ class LatentAttention(Mixer):
             prefill_done = True
             if tile_row.numel() > 0:
                 ops.paged_prefill(q, cache, table, tile_row, tile_q0, ctx.row_q_start, ctx.row_q_len, ctx.row_ctx,
-                                  *common, out=out, sinks=self.sinks, keys_only=True, value_dim=self.rank)
+                                  *common, out=out, sinks=self.sinks, keys_only=True, value_dim=self.rank, tile_rows=ctx.rows_with_tiles("multi"))
         if decode_done and prefill_done:
             return out
         which = "multi" if decode_done else ("single" if prefill_done else "all")
