@@ -60,3 +60,55 @@ def test_kept_windows_and_chunks(ops, cuda_device, window, keep, chunk, softcap,
         expected = plain(qs[r], Ks[r], Vs[r], ctx[r], nh, nkv, window, keep, chunk, sinks.cpu() if sink else None, softcap)
         assert (got[True][cursor:cursor + n].double().cpu().view(n, nh, hd) - expected).abs().max() <= 1.6e-2 * 2
         cursor += n
+
+
+@pytest.mark.parametrize("lengths,tcgen05", [([2], False), ([64], False), ([65], True), ([8] * 9, False), ([8] * 10, True), ([30, 200], True)])
+@pytest.mark.parametrize("kind", ["kept", "latent"])
+def test_short_prompts(ops, cuda_device, kind, lengths, tcgen05):
+    """Prompts within one step of its keys that give every head an SM of its own run on the mma.sync kernel."""
+    from zephyr_b200.config import FekotarConfig, TedulornConfig
+    from zephyr_b200.engine import ModelRunner, StepEntry
+    from zephyr_b200.parts import Model, expected_weights
+
+    rot = {"base": 10000.0, "dims": 32}
+    if kind == "kept":
+        mixer = dict(heads=16, kv_heads=8, dim=128, vdim=128, scale=128 ** -0.5, v_mix=False, rot=rot, mask={"size": 40, "keep_first": 16})
+        config = TedulornConfig(vocab=64, width=64, norm_eps=1e-6, embedding_scale=1.0, side_dim=0,
+                                layers=({"type": "attention", "mixer": mixer, "mlp": None},))
+    else:
+        mixer = dict(heads=16, dim=64, rot_dim=32, vdim=64, kv_rank=128, q_rank=64, scale=160 ** -0.5, rot=rot)
+        config = FekotarConfig(vocab=64, width=64, norm_eps=1e-6, logit_scale=1.0, bigram=None,
+                               layers=({"type": "latent_attention", "mixer": mixer, "mlp": None},))
+    spec = config.to_model_spec()
+    expected = expected_weights(spec)
+
+    class Store:
+        def names(self):
+            return tuple(expected)
+
+        def shape(self, name):
+            return tuple(expected[name].shape)
+
+        def dtype(self, name):
+            return torch.bfloat16
+
+        def read(self, name):
+            return rand(self.shape(name), torch.bfloat16, cuda_device, len(name)) * 0.1 + float(expected[name].role == "norm")
+
+    model = Model.load(spec, Store(), torch.bfloat16, cuda_device)
+    runner, call, got = ModelRunner(model, 16, 64, 16), spec.run_order[0], {}
+    for row, n in enumerate(lengths):
+        assert runner.add_request(row, n)
+    x = rand((sum(lengths), 64), torch.bfloat16, cuda_device, 9)
+    for own in (True, False):
+        ctx = runner.build_context([StepEntry(row, [0] * n) for row, n in enumerate(lengths)])
+        before = ops.LAUNCH_COUNTS.get("paged_prefill_tc", 0)
+        ops.USE_TCGEN05_PREFILL = own
+        try:
+            got[own] = model.layers[0].mixer.forward(x, ctx, call).float()
+        finally:
+            ops.USE_TCGEN05_PREFILL = True
+        assert ops.LAUNCH_COUNTS.get("paged_prefill_tc", 0) - before == int(own and tcgen05)
+    runner.check()
+    # The two kernels round probabilities and results to bfloat16, 2^-9 of them each, ahead of one more product.
+    assert (got[True] - got[False]).abs().max() <= 2.0 ** -6 * float(got[False].abs().max())

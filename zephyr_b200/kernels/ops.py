@@ -1713,6 +1713,14 @@ def paged_prefill(q: torch.Tensor, kv_cache: torch.Tensor, block_table: torch.Te
     return out
 
 
+def short_prompts(block_table: torch.Tensor, page_size: int, nh: int, tiles: int) -> bool:
+    """True where the mma.sync prompt kernel is done sooner than the tcgen05 one: no row of the step has more positions than one of its
+    steps of 64 keys, and every head of every tile has an SM.  (us, tcgen05 / mma.sync, 16 heads: new prompts of 2 to 48 tokens 8.8 /
+    6.9 to 8.2, of 64 8.8 / 8.4, of 96 9.0 / 12.0; 8 tokens behind 30 8.6 / 7.7, behind 62 8.6 / 11.8; nine of 8 tokens 9.5 / 7.1,
+    twelve 9.4 / 12.4; over rows of 160 values, 8 tokens 11.7 / 7.6, behind 62 11.4 / 12.7.)"""
+    return block_table.shape[1] * page_size <= 64 and nh * tiles <= _sm_count()
+
+
 # ------------------------------------------------------------------------ matrix products
 def gemm_nt_simt(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = None,
                  out: torch.Tensor | None = None) -> torch.Tensor:

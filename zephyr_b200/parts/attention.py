@@ -361,6 +361,7 @@ class Attention(Mixer):
             prefill_done = True
             if tile_row.numel() > 0:
                 ops.paged_prefill(q, cache, table, tile_row, tile_q0, ctx.row_q_start, ctx.row_q_len, ctx.row_ctx, *common, out=out,
+                                  tensor_memory=not (self.chunk and ops.short_prompts(table, cache.shape[3], self.nh, tile_row.numel())),
                                   tile_rows=ctx.rows_with_tiles("multi"), **masks)
         if decode_done and prefill_done:
             return out
@@ -423,7 +424,8 @@ class Attention(Mixer):
                                         single=True, max_context=ctx.max_decode_context)
                 elif tile_row.numel() > 0:
                     ops.paged_prefill(q, cache, table, tile_row, tile_q0, ctx.row_q_start, ctx.row_q_len, ctx.row_ctx,
-                                      *common, out=out, cross_values=mixed, by_group=by_group, tile_rows=ctx.rows_with_tiles(which[1]), **masks)
+                                      *common, out=out, cross_values=mixed, by_group=by_group, tile_rows=ctx.rows_with_tiles(which[1]),
+                                      tensor_memory=not ops.short_prompts(table, cache.shape[3], self.nh, tile_row.numel()), **masks)
         else:
             tile_row, tile_q0 = ctx.tiles[(self.tile_tokens, "all")]
             ops.paged_attention(q, cache, table, tile_row, tile_q0, self.tile_tokens, ctx.row_q_start, ctx.row_q_len,

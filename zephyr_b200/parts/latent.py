@@ -168,6 +168,7 @@ class LatentAttention(Mixer):
         ``rank`` are read behind it; the tcgen05 prompt kernel leaves the others as they are."""
         out = torch.empty_like(q)
         common = (self.nh, 1, self.kw, 0, self.scale, ctx.status)
+        page = cache.shape[1] // self.kw
         decode_done = self.fast_decode and ctx.num_decode_rows > 0
         if decode_done:
             ops.paged_decode(q, cache, table, ctx.decode_rows, ctx.row_q_start, ctx.row_ctx, ctx.max_decode_context,
@@ -180,14 +181,17 @@ class LatentAttention(Mixer):
             tile_row, tile_q0 = ctx.tiles[(self.prefill_tile_tokens, "all")]
             if tile_row.numel() > 0:
                 ops.paged_prefill(q, cache, table, tile_row, tile_q0, ctx.row_q_start, ctx.row_q_len, ctx.row_ctx,
-                                  *common, out=out, sinks=self.sinks, keys_only=True, value_dim=self.rank)
+                                  *common, out=out, sinks=self.sinks, keys_only=True, value_dim=self.rank,
+                                  tensor_memory=self.kw == 128 or not ops.short_prompts(table, page, self.nh, tile_row.numel()))
             return out
         if self.fast_prefill:
             tile_row, tile_q0 = ctx.tiles[(self.prefill_tile_tokens, "multi")]
             prefill_done = True
             if tile_row.numel() > 0:
                 ops.paged_prefill(q, cache, table, tile_row, tile_q0, ctx.row_q_start, ctx.row_q_len, ctx.row_ctx,
-                                  *common, out=out, sinks=self.sinks, keys_only=True, value_dim=self.rank, tile_rows=ctx.rows_with_tiles("multi"))
+                                  *common, out=out, sinks=self.sinks, keys_only=True, value_dim=self.rank,
+                                  tensor_memory=self.kw == 128 or not ops.short_prompts(table, page, self.nh, tile_row.numel()),
+                                  tile_rows=ctx.rows_with_tiles("multi"))
         if decode_done and prefill_done:
             return out
         which = "multi" if decode_done else ("single" if prefill_done else "all")
