@@ -75,3 +75,17 @@ def test_contexts_of_unequal_lengths(ops, cuda_device, ctx, bound, window, whole
             expected = torch.softmax(s, -1) @ Vs[r][lo[r]:, h // 2].double()
             # Weights and the result are rounded to bfloat16, 2^-9 each of values up to four.
             assert (out[r].double().cpu().view(nh, hd)[h] - expected).abs().max() <= 3.2e-2, (r, h)
+
+
+@pytest.mark.parametrize("options,size,most", [
+    (["--batch", "12", "--context", "170", "--split", "0"], "balanced", 4),         # 12 rows x 8 heads x 6 tiles over 148 CTAs
+    (["--batch", "12", "--context", "170"], "chosen", 6), (["--batch", "12", "--context", "170", "--split", "64"], 64, 4),     # (two items of two tiles)
+    (["--contexts", "4096,100,100,100,100,100"], "chosen", 8), (["--contexts", "4096,100,100,100,100,100", "--split", "4096"], 4096, 128)])
+def test_the_timing_program_cuts_as_it_says(ops, cuda_device, capsys, options, size, most):
+    import json
+
+    from zephyr_b200.kernels import timing
+
+    timing.main(["decode_attention", "--warmup", "1", "--iters", "2", *options])
+    line = json.loads(capsys.readouterr().out)
+    assert line["split_size"] == size and line["timeline_ns"]["tiles"][1] == most

@@ -1,6 +1,7 @@
 """Times one kernel of this package alone, on synthetic inputs, and prints what it achieves.
 
-    python -m zephyr_b200.kernels.timing decode_attention --batch 8 --context 4096
+    python -m zephyr_b200.kernels.timing decode_attention --batch 8 --context 4096 [--split 0]
+    python -m zephyr_b200.kernels.timing decode_attention --contexts 4096,100,100,100,100,100
     python -m zephyr_b200.kernels.timing prefill_attention --tokens 2048
     python -m zephyr_b200.kernels.timing gemm_small --rows 8 --n 6144 --k 1024 [--swiglu]
     python -m zephyr_b200.kernels.timing fused_chain --rows 8 --hidden 1024 --ffn 3072
@@ -84,13 +85,14 @@ def _paged_inputs(batch: int, context: int, nkv: int, hd: int, page: int, device
 
 def decode_attention(args) -> dict:
     device = torch.device("cuda")
-    nh, nkv, hd, B, ctx = args.heads, args.kv_heads, args.head_dim, args.batch, args.context
+    contexts = [int(n) for n in args.contexts.split(",")] if args.contexts else [args.context] * args.batch
+    nh, nkv, hd, B, ctx = args.heads, args.kv_heads, args.head_dim, len(contexts), max(contexts)
     caches, table = _paged_inputs(B, ctx, nkv, hd, args.page_size, device, args.keys_only)
     q = torch.randn((B, nh * hd), device=device, dtype=torch.bfloat16)
     rows = torch.arange(B, dtype=torch.int32, device=device)
-    row_ctx = torch.full((B,), ctx - 1, dtype=torch.int32, device=device)
+    row_ctx = torch.tensor([n - 1 for n in contexts], dtype=torch.int32, device=device)
     status, out = ops.new_status(device), torch.empty_like(q)
-    split = args.split or None
+    split = args.split
     chunk = getattr(args, "chunk", 0)
     masks = dict(chunk=chunk, sinks=torch.zeros(nh, device=device)) if chunk else {}
     masks.update(softcap=args.softcap, keys_only=args.keys_only)
@@ -105,12 +107,10 @@ def decode_attention(args) -> dict:
         run(i)
     ops.paged_decode_trace(None)
     ops.check_status(status, "decode_attention")
-    live = min(ctx, args.window) if args.window else ctx
-    if chunk:
-        live = min(live, (ctx - 1) % chunk + 1)
-    read = B * live * nkv * hd * 2 * (1 if args.keys_only else 2)
-    return {"kernel": "paged_decode_kernel", "softcap": args.softcap, "keys_only": args.keys_only, "batch": B, "context": ctx, "heads": nh, "kv_heads": nkv, "head_dim": hd,
-            "page_size": args.page_size, "window": args.window, "chunk": chunk, "split_size": split or "balanced", "us": round(us, 2),
+    live = [min(n, args.window or n, (n - 1) % chunk + 1 if chunk else n) for n in contexts]
+    read = sum(live) * nkv * hd * 2 * (1 if args.keys_only else 2)
+    return {"kernel": "paged_decode_kernel", "softcap": args.softcap, "keys_only": args.keys_only, "batch": B, "context": args.contexts or ctx, "heads": nh, "kv_heads": nkv, "head_dim": hd,
+            "page_size": args.page_size, "window": args.window, "chunk": chunk, "split_size": "chosen" if split is None else split or "balanced", "us": round(us, 2),
             "bytes_read": read, "gbs": round(read / us / 1e3, 1), "timeline_ns": _decode_timeline(trace)}
 
 
@@ -1048,7 +1048,8 @@ def main(argv=None) -> int:
     parser.add_argument("--mode", choices=("gated", "state_space"), default="gated")
     parser.add_argument("--side", type=int, default=256, help="plus_one_parts: width of a layer's part of the tokens' rows")
     parser.add_argument("--segment", type=int, default=-1, help="state_scan: tokens of a segment (0: one piece; -1: chosen)")
-    parser.add_argument("--split", type=int, default=0, help="fixed splits of this many positions in the decode kernel (0: balanced items)")
+    parser.add_argument("--split", type=int, help="fixed splits of this many positions in the decode kernel (0: balanced items; default: chosen)")
+    parser.add_argument("--contexts", default="", help="decode_attention: every row's context, \"4096,100,100\", instead of --batch and --context")
     parser.add_argument("--rows", type=int, default=8)
     parser.add_argument("--n", type=int, default=6144)
     parser.add_argument("--k", type=int, default=1024)
