@@ -112,3 +112,40 @@ def test_short_prompts(ops, cuda_device, kind, lengths, tcgen05):
     runner.check()
     # The two kernels round probabilities and results to bfloat16, 2^-9 of them each, ahead of one more product.
     assert (got[True] - got[False]).abs().max() <= 2.0 ** -6 * float(got[False].abs().max())
+
+
+@pytest.mark.parametrize("window,keep,chunk,bias,page", [
+    (100, 40, 0, False, 16), (64, 64, 0, False, 8), (300, 130, 0, False, 16), (60, 40, 200, False, 16), (0, 0, 100, False, 16),
+    (0, 0, 128, False, 32), (0, 0, 0, True, 16), (150, 0, 0, True, 64)])
+@pytest.mark.parametrize("heads", ["in pairs", "singly"])
+def test_masks_in_both_forms_of_a_cta(ops, cuda_device, heads, window, keep, chunk, bias, page):
+    """Kept tokens, chunks and a distance bias with two heads a CTA and with one whose tiles of keys two slots share."""
+    hd = 128
+    nh, nkv = (32, 8) if heads == "in pairs" else (4, 2)
+    q_lens, ctx = [130, 1, 127, 128, 90, 257], [0, 511, 129, 128, 64, 300]        # 9 tiles of 6 rows: 288 (head, tile) or 36
+    q, cache, meta, Ks, Vs, qs = build_paged_case(cuda_device, torch.bfloat16, nh, nkv, hd, page, q_lens, ctx, 310)
+    sinks = rand((nh,), torch.float32, cuda_device, 6)
+    r1, r2 = (torch.linspace(0.1, 2.0, nh), torch.linspace(0.01, 0.5, nh)) if bias else (None, None)
+    status, before = ops.new_status(cuda_device), ops.LAUNCH_COUNTS.get("paged_prefill_tc", 0)
+    got = ops.paged_prefill(q, cache, meta["table"], *tiles_for(q_lens, ops.paged_prefill_tile_tokens(), cuda_device), meta["row_q_start"],
+                            meta["row_q_len"], meta["row_ctx"], nh, nkv, hd, window, 1 / math.sqrt(hd), status, torch.full_like(q, float("nan")),
+                            chunk=chunk, sinks=sinks, keep_first=keep,
+                            distance_bias=(r1.to(cuda_device), r2.to(cuda_device)) if bias else None)
+    ops.check_status(status)
+    assert ops.LAUNCH_COUNTS["paged_prefill_tc"] == before + 1
+    at = 0
+    for r, n in enumerate(q_lens):
+        if bias:
+            i, j = torch.arange(ctx[r], ctx[r] + n)[:, None], torch.arange(ctx[r] + n)[None, :]
+            seen, expected = (j <= i) & ((i - j < window) if window else (j <= i)), []
+            for h in range(nh):
+                s = qs[r][:, h].double() @ Ks[r][:, h // (nh // nkv)].double().T / math.sqrt(hd) - r1[h].double() * torch.log1p(
+                    r2[h].double() * (i - j).clamp(min=0))
+                s = torch.cat([s.masked_fill(~seen, -math.inf), sinks[h].cpu().double().expand(n, 1)], dim=1)
+                expected.append(torch.softmax(s, -1)[:, :-1] @ Vs[r][:, h // (nh // nkv)].double())
+            expected = torch.stack(expected, 1)
+        else:
+            expected = plain(qs[r], Ks[r], Vs[r], ctx[r], nh, nkv, window, keep, chunk, sinks.cpu(), 0.0)
+        # Weights and the result are rounded to bfloat16 (2^-9 each, of values of up to four).
+        assert (got[at:at + n].double().cpu().view(n, nh, hd) - expected).abs().max() <= 3.2e-2
+        at += n
