@@ -1,4 +1,5 @@
-"""What a kernel that may start before the one in front of it has ended has to keep to, read from the sources."""
+"""What kernels that start before the one in front of them has ended, and kernels whose copies run beside them, have to keep to, read
+from the sources."""
 
 import re
 
@@ -42,3 +43,11 @@ def test_dependent_kernels_do_not_declare_other_kernels_results_constant():
             if "__restrict__" in parameter:
                 assert parameter.split()[-1].lstrip("*") in CONSTANT | OWN, (file, name, parameter)
         assert "__ldg(" not in body and ".nc." not in body, (file, name)
+
+
+def test_kernels_whose_wait_runs_out_let_their_copies_land():
+    """A CTA that gives up leaves its shared memory to another one only behind its own copies."""
+    copying = [k for k in kernels() if re.search(r"(bulk_copy_g2s|tiled_copy_2d_g2s(_pair)?)\(", k[3])]
+    assert len(copying) >= 7
+    for file, name, _, body in copying:
+        assert "let_copies_land()" in body, (file, name)

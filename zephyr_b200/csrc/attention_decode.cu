@@ -923,12 +923,7 @@ paged_decode_kernel(const DecodeArgs a) {
     if (ctid == 0) a.counters[it.r * a.nkv + it.kvh] = 0;    // left as it was found, for the next call
   }
   if (trace) { trace[4] = timer_ns(); trace[5] = item_seq; trace[6] = tile_base; }
-  if (abort_flag) {
-    // Something went wrong.  Give copies that are still in flight a bounded chance to land before
-    // this CTA's shared memory is handed to another.
-    for (int s = warp; s < R; s += DEC_CONSUMERS)
-      for (int i = 0; i < (1 << 14) && !mbar_try_wait(&full[s], 0) && !mbar_try_wait(&full[s], 1); ++i) {}
-  }
+  if (abort_flag) let_copies_land();
 }
 
 // Shared memory of one CTA with `slots` ring slots, and the most slots that fit.

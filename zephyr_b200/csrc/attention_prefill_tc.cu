@@ -735,6 +735,7 @@ paged_prefill_tc_kernel(const __grid_constant__ PrefillTcArgs a) {
   // Everybody meets here on every path, and the warp that took the tensor memory gives it back.
   tc_fence_before_sync();
   __syncthreads();
+  if (abort_flag) let_copies_land();
   if (warp == TC_MMA_WARP) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, TC_TMEM_COLUMNS);

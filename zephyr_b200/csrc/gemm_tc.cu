@@ -295,6 +295,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tc_kernel(const __grid_con
   // Everybody meets here on every path, and the warp that took the tensor memory gives it back.
   tc_fence_before_sync();
   __syncthreads();
+  if (sh.failed) let_copies_land();
   if (warp == 1) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, Shape::TMEM_COLUMNS);
@@ -442,6 +443,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GT_THREADS, 1) gemm_
   // then), and the warps that took the tensor memory give it back.
   tc_fence_before_sync();
   __syncthreads();
+  if (sh.failed) let_copies_land();                 // (they count on the first CTA's barriers)
   __syncwarp();
   cluster_sync_all();
   if (warp == 1) {

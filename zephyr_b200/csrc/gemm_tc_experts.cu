@@ -244,6 +244,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GX_THREADS, 1) gemm_
   // tensor memory give it back.
   tc_fence_before_sync();
   __syncthreads();
+  if (sh.failed) let_copies_land();                 // (they count on the first CTA's barriers)
+  __syncwarp();
   cluster_sync_all();
   if (warp == 1) {
     tc_fence_after_sync();

@@ -69,6 +69,13 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned pari
     if (mbar_try_wait(bar, parity)) return true;
   return false;
 }
+// For a CTA in which a wait has run out, before it leaves: time (0.2 ms, a copy takes some microseconds) for the asynchronous copies
+// that are still on their way into its shared memory, which another CTA gets next.  (Not by their barriers: which phase is due there is what
+// the failed wait has lost, and of the two parities one is always complete.)
+__device__ __forceinline__ void let_copies_land() {
+#pragma unroll 1
+  for (int i = 0; i < 200; ++i) __nanosleep(1000);
+}
 // `bytes` (a multiple of 16) from global to this CTA's shared memory, both 16-byte aligned; completion
 // is counted on `bar`.  This CTA's own shared memory is not multicast to anyone.
 __device__ __forceinline__ void bulk_copy_g2s(void* smem_dst, const void* gmem_src, unsigned bytes, unsigned long long* bar) {

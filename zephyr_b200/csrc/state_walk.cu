@@ -509,6 +509,7 @@ __global__ void __launch_bounds__(W_THREADS, 2) state_walk_kernel(const WalkArgs
     // The piece, the state and the values are there; the buffer of the piece before is free.
     if (!__syncthreads_and(here)) {
       if (tid == 0) report(a.status, STATUS_COPY_TIMEOUT, p, row);
+      let_copies_land();
       return;
     }
     if (tid == 0 && p + 1 < pieces) copy_piece(p + 1);
