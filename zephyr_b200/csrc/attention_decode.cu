@@ -485,7 +485,8 @@ paged_decode_kernel(const DecodeArgs a) {
   let_dependents_launch();
   // Balanced items: as many tiles per range as spread all tiles evenly over the CTAs.
   const int per_range = balanced ? max(1, (prefix[a.n_rows] + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x)) : 0;
-  if (EITHER && !balanced && blockIdx.x >= a.n_rows * a.nkv) return;      // (a CTA for balanced items that are not: its SM is free for the next kernel)
+  // (A CTA for balanced items that are not: its SM is free for the next kernel.)
+  if (EITHER && !balanced && blockIdx.x >= a.n_rows * a.nkv) return;
   const int page_size = 1 << a.page_shift;
   const long long page_stride = (a.keys_only ? 1LL : 2LL) * a.nkv * page_size * HD;
   const bool fused = a.qkv != nullptr;       // the new tokens' position encoding happens in this kernel
@@ -1036,8 +1037,9 @@ static int paged_decode_entry(void* out, const void* q, const void* kv_cache, co
                               const DecodeFusion* fusion, void* stream, int chunk = 0, const float* sinks = nullptr,
                               float softcap = 0.0f, int keys_only = 0, const float* bias_r1 = nullptr,
                               const float* bias_r2 = nullptr) {
-  if ((bias_r1 == nullptr) != (bias_r2 == nullptr) || n_rows < 0 || max_splits <= 0 || split_size < 0 || split_size % DEC_TILE != 0 || page_size <= 0 || window < 0 ||
-      (or_balanced != 0 && (split_size <= 0 || max_splits > split_size / DEC_TILE)) || chunk < 0 || counters == nullptr || softcap < 0.0f || (keys_only && fusion != nullptr))
+  if ((bias_r1 == nullptr) != (bias_r2 == nullptr) || n_rows < 0 || max_splits <= 0 || split_size < 0 || split_size % DEC_TILE != 0 ||
+      page_size <= 0 || window < 0 || (or_balanced != 0 && (split_size <= 0 || max_splits > split_size / DEC_TILE)) || chunk < 0 ||
+      counters == nullptr || softcap < 0.0f || (keys_only && fusion != nullptr))
     return ERR_BAD_ARGUMENT;
   if (!zb_paged_decode_supported(nh, nkv, hd, DTYPE_BF16) || (page_size & (page_size - 1)) != 0) return ERR_UNSUPPORTED;
   if (n_rows == 0) return OK;

@@ -11,9 +11,9 @@
 //   * one head whose tiles of keys the slots take by turns, even and odd, and merge at the end: half as
 //     long a chain, for the tiles that would otherwise end last (and for heads without a partner).
 // Roles:
-//   * loader warps copy a tile's rows from the cache pages (TMA tiled copies per page for tiles
-//     inside the context, 16-byte asynchronous copies at its edges, where rows have to be zero).  A
-//     cache row's 16-byte chunks are stored permuted with the position (common.cuh: kv_swizzle); for
+//   * loader warps copy a tile's rows from the cache pages (TMA tiled copies per page; at an edge of the context the values'
+//     rows beyond it are set to zero once their page has landed; 16-byte asynchronous copies for a cache of
+//     more rows than a tensor map counts).  A cache row's 16-byte chunks are stored permuted with the position (common.cuh: kv_swizzle); for
 //     rows of 256 bytes that permutation IS the 128-byte swizzle of the tensor core's canonical
 //     shared-memory layout over blocks of 64 values, for rows of 320 bytes the 64-byte swizzle over
 //     blocks of 32, so a row is copied as it lies, block by block;

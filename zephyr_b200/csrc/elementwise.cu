@@ -385,7 +385,8 @@ int embedding_launch(void* out, const void* table, const int* ids, int T_, int H
   if (T_ == 0) return OK;
   const bool vec = aligned16<T>(out, H) && aligned16<T>(table, H);
   const int threads = 128;
-  if (vec) launch_dependent(embedding_kernel<T, true>, dim3(T_), dim3(threads), 0, stream, false, (T*)out, (const T*)table, ids, H, V, status);
+  if (vec) launch_dependent(embedding_kernel<T, true>, dim3(T_), dim3(threads), 0, stream, false, (T*)out, (const T*)table,
+      ids, H, V, status);
   else launch_dependent(embedding_kernel<T, false>, dim3(T_), dim3(threads), 0, stream, false, (T*)out, (const T*)table, ids, H, V, status);
   return launch_result();
 }
@@ -403,10 +404,11 @@ int rmsnorm_launch(void* out, void* x, const void* delta, const void* w, int w_d
     const bool add = delta != nullptr;
 #define ZB_ROWS(V_)                                                                                                  \
   do {                                                                                                               \
-    if (add) launch_dependent(rmsnorm_warp_rows_kernel<V_, true>, dim3(blocks), dim3(NORM_ROWS_PER_BLOCK * 32), 0, stream, false,                     \
-        (__nv_bfloat16*)out, (__nv_bfloat16*)x, (const __nv_bfloat16*)delta, w, w_dtype, eps, rows, H, x_stride, out_stride); \
-    else launch_dependent(rmsnorm_warp_rows_kernel<V_, false>, dim3(blocks), dim3(NORM_ROWS_PER_BLOCK * 32), 0, stream, false,                        \
-        (__nv_bfloat16*)out, (__nv_bfloat16*)x, nullptr, w, w_dtype, eps, rows, H, x_stride, out_stride);           \
+    if (add) launch_dependent(rmsnorm_warp_rows_kernel<V_, true>, dim3(blocks), dim3(NORM_ROWS_PER_BLOCK * 32), 0, stream,    \
+        false, (__nv_bfloat16*)out, (__nv_bfloat16*)x, (const __nv_bfloat16*)delta, w, w_dtype, eps, rows, H, x_stride,       \
+        out_stride);                                                                                                          \
+    else launch_dependent(rmsnorm_warp_rows_kernel<V_, false>, dim3(blocks), dim3(NORM_ROWS_PER_BLOCK * 32), 0, stream,       \
+        false, (__nv_bfloat16*)out, (__nv_bfloat16*)x, nullptr, w, w_dtype, eps, rows, H, x_stride, out_stride);              \
   } while (0)
     if (vectors <= 1) ZB_ROWS(1);
     else if (vectors <= 2) ZB_ROWS(2);
@@ -420,8 +422,8 @@ int rmsnorm_launch(void* out, void* x, const void* delta, const void* w, int w_d
   threads = threads < 32 ? 32 : (threads > 512 ? 512 : threads);
   const bool add = delta != nullptr;
 #define ZB_NORM(ADD_, VEC_)                                                                            \
-  launch_dependent(rmsnorm_kernel<T, ADD_, VEC_>, dim3(rows), dim3(threads), 0, stream, false, (T*)out, (T*)x, (const T*)delta, w, w_dtype, \
-                                                               eps, H, x_stride, out_stride)
+  launch_dependent(rmsnorm_kernel<T, ADD_, VEC_>, dim3(rows), dim3(threads), 0, stream, false, (T*)out, (T*)x,                \
+      (const T*)delta, w, w_dtype, eps, H, x_stride, out_stride)
   if (add && vec) ZB_NORM(true, true);
   else if (add) ZB_NORM(true, false);
   else if (vec) ZB_NORM(false, true);
@@ -470,8 +472,10 @@ ZB_API int zb_gather_rows(void* out, const void* x, const int* rows, int num_row
   const dim3 grid(num_rows, vec ? (H + piece - 1) / piece : 1);
 #define ZB_GATHER(T)                                                                                                       \
   {                                                                                                                        \
-    if (vec) launch_dependent(gather_rows_kernel<T, true>, dim3(grid), dim3(128), 0, s, false, (T*)out, (const T*)x, rows, H, num_src_rows, status);         \
-    else launch_dependent(gather_rows_kernel<T, false>, dim3(grid), dim3(128), 0, s, false, (T*)out, (const T*)x, rows, H, num_src_rows, status);            \
+    if (vec) launch_dependent(gather_rows_kernel<T, true>, grid, dim3(128), 0, s, false, (T*)out, (const T*)x, rows, H,       \
+        num_src_rows, status);                                                                                                \
+    else launch_dependent(gather_rows_kernel<T, false>, grid, dim3(128), 0, s, false, (T*)out, (const T*)x, rows, H,          \
+        num_src_rows, status);                                                                                                \
   }
   if (dtype == DTYPE_F32) ZB_GATHER(float) else ZB_GATHER(__nv_bfloat16)
 #undef ZB_GATHER
@@ -545,8 +549,10 @@ ZB_API int zb_add_bias(void* y, long long ldy, const void* bias, int b_dtype, in
   const int piece = dtype == DTYPE_F32 ? 4 : 8;
   if (b_dtype == DTYPE_F32 && N % piece == 0 && ldy % piece == 0 && reinterpret_cast<uintptr_t>(y) % 16 == 0) {
     const dim3 grid((N / piece + 31) / 32, std::min((T + 15) / 16, 4096)), block(32, 8);
-    if (dtype == DTYPE_F32) launch_dependent(add_bias_vec_kernel<float>, dim3(grid), dim3(block), 0, s, false, (float*)y, ldy, (const float*)bias, T, N);
-    else launch_dependent(add_bias_vec_kernel<__nv_bfloat16>, dim3(grid), dim3(block), 0, s, false, (__nv_bfloat16*)y, ldy, (const float*)bias, T, N);
+    if (dtype == DTYPE_F32) launch_dependent(add_bias_vec_kernel<float>, grid, block, 0, s, false, (float*)y, ldy,
+        (const float*)bias, T, N);
+    else launch_dependent(add_bias_vec_kernel<__nv_bfloat16>, grid, block, 0, s, false, (__nv_bfloat16*)y, ldy,
+        (const float*)bias, T, N);
     return launch_result();
   }
   if (dtype == DTYPE_F32) add_bias_kernel<float><<<blocks, 256, 0, s>>>((float*)y, ldy, bias, b_dtype, T, N);

@@ -379,9 +379,12 @@ ZB_API int zb_qkv_pairs(void* q_out, const void* qkv, long long stride, const fl
 #define ZB_QPV(ITEMS, HEADS)                                                                                             \
   {                                                                                                                      \
     const dim3 grid(tokens, (heads + HEADS * QPV_WARPS - 1) / (HEADS * QPV_WARPS));                                      \
-    if (dtype == DTYPE_F32) launch_dependent(qkv_pairs_vec_kernel<float, float, ITEMS, HEADS>, dim3(grid), dim3(QPV_WARPS * 32), smem, s, false, a);       \
-    else if (in_dtype == DTYPE_F32) launch_dependent(qkv_pairs_vec_kernel<float, __nv_bfloat16, ITEMS, HEADS>, dim3(grid), dim3(QPV_WARPS * 32), smem, s, false, a); \
-    else launch_dependent(qkv_pairs_vec_kernel<__nv_bfloat16, __nv_bfloat16, ITEMS, HEADS>, dim3(grid), dim3(QPV_WARPS * 32), smem, s, false, a);          \
+    if (dtype == DTYPE_F32) launch_dependent(qkv_pairs_vec_kernel<float, float, ITEMS, HEADS>, grid, dim3(QPV_WARPS * 32),    \
+        smem, s, false, a);                                                                                                   \
+    else if (in_dtype == DTYPE_F32) launch_dependent(qkv_pairs_vec_kernel<float, __nv_bfloat16, ITEMS, HEADS>, grid,          \
+        dim3(QPV_WARPS * 32), smem, s, false, a);                                                                             \
+    else launch_dependent(qkv_pairs_vec_kernel<__nv_bfloat16, __nv_bfloat16, ITEMS, HEADS>, grid, dim3(QPV_WARPS * 32),       \
+        smem, s, false, a);                                                                                                   \
   }
     // Several heads a warp where the tokens alone give every SM a full set of warps; a decode step keeps its heads apart.
     const bool many = tokens >= 4 * 148 && heads > QPV_WARPS;

@@ -291,7 +291,8 @@ void embedding_f32(float* out, T* rounded, const T* table, const int* ids, float
                    cudaStream_t s) {
   auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
   if (H % 4 == 0 && H <= 512 * 65535 && aligned(out) && aligned(rounded) && aligned(table))
-    launch_dependent(embedding_f32_vec_kernel<T>, dim3(dim3(tokens, (H + 511) / 512)), dim3(128), 0, s, false, out, rounded, table, ids, scale, H, V, status);
+    launch_dependent(embedding_f32_vec_kernel<T>, dim3(tokens, (H + 511) / 512), dim3(128), 0, s, false, out, rounded,
+        table, ids, scale, H, V, status);
   else
     embedding_f32_kernel<T><<<tokens, 128, 0, s>>>(out, rounded, table, ids, scale, H, V, status);
 }
@@ -923,8 +924,9 @@ void gated_group_rms_norm_vec(T* out, const float* o, const G* gate, long long g
                               int group, float eps, int gate_first, int tokens, cudaStream_t s) {
   const long long items = static_cast<long long>(tokens) * (width / group);
 #define ZB_GN(ITEMS, WARPS)                                                                                                  \
-  launch_dependent(gated_group_rms_norm_vec_kernel<T, G, ITEMS, WARPS>, dim3(static_cast<unsigned>((items * WARPS + GN_WARPS - 1) / GN_WARPS)), dim3(32 * GN_WARPS), 0, s, false,                            \
-          out, o, gate, gate_stride, w, w_len, width, group, eps, gate_first, tokens)
+  launch_dependent(gated_group_rms_norm_vec_kernel<T, G, ITEMS, WARPS>,                                                       \
+      dim3(static_cast<unsigned>((items * WARPS + GN_WARPS - 1) / GN_WARPS)), dim3(32 * GN_WARPS), 0, s, false, out, o,       \
+      gate, gate_stride, w, w_len, width, group, eps, gate_first, tokens)
   if (group <= 128) ZB_GN(1, 1);
   else if (group <= 256) ZB_GN(2, 1);
   else if (group <= 512) ZB_GN(4, 1);
@@ -966,7 +968,8 @@ template <typename IN, typename T>
 void scaled_sum(T* out, const IN* a, const IN* b, float sa, float sb, long long n, cudaStream_t s) {
   auto aligned = [](const void* p, size_t bytes) { return reinterpret_cast<uintptr_t>(p) % bytes == 0; };
   if (n % 4 == 0 && aligned(out, 4 * sizeof(T)) && aligned(a, 4 * sizeof(IN)) && aligned(b, 4 * sizeof(IN)))
-    launch_dependent(scaled_sum_vec_kernel<IN, T>, dim3(static_cast<unsigned>((n / 4 + 511) / 512)), dim3(256), 0, s, false, out, a, b, sa, sb, n / 4);
+    launch_dependent(scaled_sum_vec_kernel<IN, T>, dim3(static_cast<unsigned>((n / 4 + 511) / 512)), dim3(256), 0, s, false,
+        out, a, b, sa, sb, n / 4);
   else
     scaled_sum_kernel<IN, T><<<static_cast<unsigned>((n + 255) / 256), 256, 0, s>>>(out, a, b, sa, sb, n);
 }
@@ -999,9 +1002,11 @@ ZB_API int zb_layer_norm(void* out, const void* x, const void* w, const void* b,
 #define ZB_LNV(X, T)                                                                                                      \
   {                                                                                                                       \
     if (H <= 2 * LN_VEC_THREADS * 4)                                                                                      \
-      launch_dependent(layer_norm_vec_kernel<X, T, 2>, dim3(rows), dim3(LN_VEC_THREADS), 0, s, false, static_cast<T*>(out), static_cast<const X*>(x), wf, bf, eps, H); \
+      launch_dependent(layer_norm_vec_kernel<X, T, 2>, dim3(rows), dim3(LN_VEC_THREADS), 0, s, false, static_cast<T*>(out),   \
+          static_cast<const X*>(x), wf, bf, eps, H);                                                                          \
     else                                                                                                                  \
-      launch_dependent(layer_norm_vec_kernel<X, T, LN_VEC_ITEMS>, dim3(rows), dim3(LN_VEC_THREADS), 0, s, false, static_cast<T*>(out), static_cast<const X*>(x), wf, bf, eps, H); \
+      launch_dependent(layer_norm_vec_kernel<X, T, LN_VEC_ITEMS>, dim3(rows), dim3(LN_VEC_THREADS), 0, s, false,              \
+          static_cast<T*>(out), static_cast<const X*>(x), wf, bf, eps, H);                                                    \
   }
     if (x_dtype == DTYPE_F32 && out_dtype == DTYPE_F32) ZB_LNV(float, float)
     else if (x_dtype == DTYPE_F32) ZB_LNV(float, bf16)
@@ -1039,8 +1044,8 @@ static int residual_norm_launch(float* residual, const void* delta, const void* 
     const float* f2 = static_cast<const float*>(w2);
     const float* g2 = static_cast<const float*>(b2);
 #define ZB_RN(T, ITEMS)                                                                                       \
-  launch_dependent(residual_layer_norm_vec_kernel<T, RMS, ITEMS>, dim3(rows), dim3(LN_VEC_THREADS), 0, s, false,                                \
-      residual, static_cast<const T*>(delta), f1, g1, mult, static_cast<T*>(out), f2, g2, eps1, eps2, H)
+  launch_dependent(residual_layer_norm_vec_kernel<T, RMS, ITEMS>, dim3(rows), dim3(LN_VEC_THREADS), 0, s, false, residual,    \
+      static_cast<const T*>(delta), f1, g1, mult, static_cast<T*>(out), f2, g2, eps1, eps2, H)
     const bool two = H <= 2 * LN_VEC_THREADS * 4;
     if (dtype == DTYPE_F32) { if (two) ZB_RN(float, 2); else ZB_RN(float, LN_VEC_ITEMS); }
     else { if (two) ZB_RN(__nv_bfloat16, 2); else ZB_RN(__nv_bfloat16, LN_VEC_ITEMS); }
@@ -1148,8 +1153,8 @@ ZB_API int zb_decayed_state_scan(float* out, const void* q, long long q_stride, 
   auto s = static_cast<cudaStream_t>(stream);
   if (mode == SCAN_GATED) {
     const long long count = static_cast<long long>(tokens) * H * D;
-    launch_dependent(gated_decay_kernel, dim3(static_cast<unsigned>((count + 255) / 256)), dim3(256), 0, s, false, z, z_stride, z_bias, w_dtype, H * D,
-                                                                                inv_tau, count);
+    launch_dependent(gated_decay_kernel, dim3(static_cast<unsigned>((count + 255) / 256)), dim3(256), 0, s, false, z,
+        z_stride, z_bias, w_dtype, H * D, inv_tau, count);
   }
   ScanArgs a;
   a.q = q; a.q_stride = q_stride; a.k = k; a.k_stride = k_stride; a.v = v; a.v_stride = v_stride;

@@ -557,8 +557,9 @@ ZB_API int zb_route_biased(int* ids, float* weights, const float* logits, long l
     return ERR_BAD_ARGUMENT;
   if (outputs > 32 * ROUTE_PER_LANE || (groups > 1 && group_top > ROUTE_GROUP_TOP_MAX)) return ERR_UNSUPPORTED;
   if (tokens == 0) return OK;
-  launch_dependent(route_kernel, dim3((tokens + ROUTE_WARPS - 1) / ROUTE_WARPS), dim3(ROUTE_WARPS * 32), 0, static_cast<cudaStream_t>(stream), false, ids, weights, logits, logits_stride, correction, tokens, outputs, top, sigmoid_scores, groups, keep, group_top,
-      weight_scale, logit_bias, normalize);
+  launch_dependent(route_kernel, dim3((tokens + ROUTE_WARPS - 1) / ROUTE_WARPS), dim3(ROUTE_WARPS * 32), 0,
+      static_cast<cudaStream_t>(stream), false, ids, weights, logits, logits_stride, correction, tokens, outputs, top,
+      sigmoid_scores, groups, keep, group_top, weight_scale, logit_bias, normalize);
   return launch_result();
 }
 
@@ -627,8 +628,8 @@ ZB_API int zb_route_align_runs(int* plan, int* slots, int* place_of_slot, const 
     return ERR_BAD_ARGUMENT;
   const size_t smem = 3 * static_cast<size_t>(experts) * sizeof(int);
   if (smem > 48 * 1024) return ERR_UNSUPPORTED;
-  launch_dependent(align_runs_kernel, dim3(1), dim3(ALIGN_THREADS), smem, static_cast<cudaStream_t>(stream), false, plan, slots, place_of_slot, ids, num_slots, experts,
-                                                                                     max_runs, run, places);
+  launch_dependent(align_runs_kernel, dim3(1), dim3(ALIGN_THREADS), smem, static_cast<cudaStream_t>(stream), false, plan,
+      slots, place_of_slot, ids, num_slots, experts, max_runs, run, places);
   return launch_result();
 }
 
@@ -639,7 +640,8 @@ ZB_API int zb_gather_places(void* out, const void* x, long long x_stride, const 
       reinterpret_cast<uintptr_t>(out) % 16 != 0 || reinterpret_cast<uintptr_t>(x) % 16 != 0)
     return ERR_BAD_ARGUMENT;
   if (places == 0) return OK;
-  launch_dependent(gather_places_kernel, dim3(places), dim3(128), 0, static_cast<cudaStream_t>(stream), false, static_cast<uint4*>(out), static_cast<const uint4*>(x), x_stride / 8, slots, width / 8, top, place_scale, weights);
+  launch_dependent(gather_places_kernel, dim3(places), dim3(128), 0, static_cast<cudaStream_t>(stream), false,
+      static_cast<uint4*>(out), static_cast<const uint4*>(x), x_stride / 8, slots, width / 8, top, place_scale, weights);
   return launch_result();
 }
 
@@ -663,8 +665,8 @@ ZB_API int zb_route_combine(void* out, const void* y, long long y_stride, int y_
                                                            width, top);
   } else if (width % 8 == 0 && y_stride % 8 == 0 && x_stride % 8 == 0 && top <= COMBINE_MAX_TOP && tm_aligned(out, 16) &&
              tm_aligned(y, 16) && tm_aligned(x, 16)) {
-    launch_dependent(combine_pieces_kernel, dim3(tokens), dim3(width >= 2048 ? 256 : 128), 0, s, false, static_cast<uint4*>(out), static_cast<const uint4*>(y), y_stride / 8, static_cast<const uint4*>(x), x_stride / 8,
-        weights, place_of_slot, width / 8, top);
+    launch_dependent(combine_pieces_kernel, dim3(tokens), dim3(width >= 2048 ? 256 : 128), 0, s, false, static_cast<uint4*>(out),
+        static_cast<const uint4*>(y), y_stride / 8, static_cast<const uint4*>(x), x_stride / 8, weights, place_of_slot, width / 8, top);
   } else {
     combine_kernel<bf16, bf16><<<tokens, threads, 0, s>>>(static_cast<bf16*>(out), static_cast<const bf16*>(y), y_stride,
                                                           static_cast<const bf16*>(x), x_stride, ids, weights, place_of_slot,

@@ -642,7 +642,8 @@ static int walk_launch(const WalkArgs& a, int pieces, cudaStream_t s) {
       cuda_failed(cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::smem)))
     return ERR_CUDA;
   const int heads = MODE == WALK_SPACE ? W_HEADS : 1;
-  launch_dependent(prepare, dim3(pieces, a.H / a.heads_per_group * ((a.heads_per_group + heads - 1) / heads)), dim3(W_THREADS), Shape::qk_bytes, s, false, a);
+  launch_dependent(prepare, dim3(pieces, a.H / a.heads_per_group * ((a.heads_per_group + heads - 1) / heads)),
+      dim3(W_THREADS), Shape::qk_bytes, s, false, a);
   // (Not as a dependent, which would fill the SMs that are free first instead of all of them.)
   walk<<<dim3(a.rows, a.H, (a.V + Shape::COLS - 1) / Shape::COLS), W_THREADS, Shape::smem, s>>>(a);
   return launch_result();

@@ -393,8 +393,8 @@ ZB_API int zb_sum_rms_norm(void* out, long long out_stride, int out_dtype, float
 #define ZB_SN(A_, B_, OUT_)                                                                                          \
   {                                                                                                                  \
     if (vectors)                                                                                                     \
-      launch_dependent(sum_rms_norm_vec_kernel<A_, B_, OUT_>, dim3(grid), dim3(threads), 0, s, false, (OUT_*)out, out_stride, x, x_stride,         \
-                                                                         (const A_*)a, (const B_*)b, bias, w, w_dtype, eps, part); \
+      launch_dependent(sum_rms_norm_vec_kernel<A_, B_, OUT_>, grid, dim3(threads), 0, s, false, (OUT_*)out, out_stride, x,    \
+          x_stride, (const A_*)a, (const B_*)b, bias, w, w_dtype, eps, part);                                                 \
     else                                                                                                             \
       sum_rms_norm_kernel<A_, B_, OUT_><<<grid, threads, 0, s>>>((OUT_*)out, out_stride, x, x_stride, (const A_*)a, \
                                                                      (const B_*)b, bias, w, w_dtype, eps, part);     \

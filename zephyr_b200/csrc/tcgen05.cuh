@@ -29,21 +29,7 @@ __device__ __forceinline__ void tc_mma(unsigned d_tmem, unsigned long long a_des
                ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
 // D[tmem] (+)= A[tmem] * B[smem]: A's 128 rows lie in the 128 lanes, 16 bfloat16 along K as 8 columns
-// of two (the lower index in the lower half).
-// The thread that issues the products shares its scheduler with softmax warps, and a product of
-// this size is done sooner than a dozen instructions get issued there: everything but the
-// instruction itself is taken out of the way (descriptors advance by a constant, the predicate is
-// set once).
-template <bool ACCUMULATE>
-__device__ __forceinline__ void tc_mma_ts(unsigned d_tmem, unsigned a_tmem, unsigned long long b_desc, unsigned idesc) {
-  if (ACCUMULATE)
-    asm volatile("{\n.reg .pred p;\nsetp.eq.b32 p, 0, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-                 ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc) : "memory");
-  else
-    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, 0, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-                 ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc) : "memory");
-}
-// As above, `accumulate` 0 overwrites D.
+// of two (the lower index in the lower half); `accumulate` 0 overwrites D.
 __device__ __forceinline__ void tc_mma_ts_if(unsigned d_tmem, unsigned a_tmem, unsigned long long b_desc, unsigned idesc, unsigned accumulate) {
   asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
                ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
@@ -84,12 +70,6 @@ __device__ __forceinline__ void tmem_st32(unsigned address, const unsigned (&r)[
                  "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
                  "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
                  "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-               : "memory");
-}
-__device__ __forceinline__ void tmem_st16(unsigned address, const unsigned (&r)[16]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n"
-               ::"r"(address), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-                 "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
                : "memory");
 }
 // Has the phase with this parity completed?  Never suspends the thread (try_wait may, for a while).

@@ -580,8 +580,9 @@ ZB_API int zb_qkv_halves(void* q_out, const void* qkv, long long stride, const f
 #define ZB_QHH(HEADS)                                                                                        \
   {                                                                                                          \
     const dim3 grid(tokens, (heads + HEADS * QHH_WARPS - 1) / (HEADS * QHH_WARPS));                          \
-    if (dtype == DTYPE_F32) launch_dependent(qkv_halves_heads_kernel<float, HEADS>, dim3(grid), dim3(QHH_WARPS * 32), turn, s, false, a);      \
-    else launch_dependent(qkv_halves_heads_kernel<__nv_bfloat16, HEADS>, dim3(grid), dim3(QHH_WARPS * 32), turn, s, false, a);                 \
+    if (dtype == DTYPE_F32) launch_dependent(qkv_halves_heads_kernel<float, HEADS>, grid, dim3(QHH_WARPS * 32), turn, s,      \
+        false, a);                                                                                                            \
+    else launch_dependent(qkv_halves_heads_kernel<__nv_bfloat16, HEADS>, grid, dim3(QHH_WARPS * 32), turn, s, false, a);      \
   }
       if (many) ZB_QHH(4) else ZB_QHH(1)
 #undef ZB_QHH
@@ -652,7 +653,8 @@ ZB_API int zb_sigmoid_gate(void* x, const float* gate, long long gate_stride, in
   if (tokens == 0) return OK;
   auto s = static_cast<cudaStream_t>(stream);
   if (dtype == DTYPE_BF16 && per % 8 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0) {
-    launch_dependent(sigmoid_gate_pieces_kernel, dim3(tokens), dim3(256), 0, s, false, static_cast<uint4*>(x), gate, gate_stride, width / 8, per / 8);
+    launch_dependent(sigmoid_gate_pieces_kernel, dim3(tokens), dim3(256), 0, s, false, static_cast<uint4*>(x), gate,
+        gate_stride, width / 8, per / 8);
     return launch_result();
   }
   if (dtype == DTYPE_F32) sigmoid_gate_kernel<float><<<tokens, 256, 0, s>>>(static_cast<float*>(x), gate, gate_stride, width, per);
