@@ -6,8 +6,8 @@
 // multiplied with a tile of padding, and a CTA fetches its 128 rows of w beside half of the run's rows of x.  (With the tokens on
 // the 128-row side, tiles of 128 x 256, a run of 173 tokens was two tiles that each fetched w: 777 tokens, 4 of 16 experts, 2048
 // wide, 3072 / 1536 rows: 67 and 38 us, bound by 590 and 295 MB from L2.  One SM a tile of 128 rows of w x run, 503 and
-// 250 MB: 67 and 37; on pairs, 344 and 172 MB, 45
-// and 25.  The matrices alone take 31 and 15 us at the copy rate; three rounds of 74 pairs for 2.6 rounds of work cost 14 %.)
+// 250 MB: 67 and 37; on pairs, 344 and 172 MB, 43
+// and 26.  The matrices alone take 31 and 15 us at the copy rate; three rounds of 74 pairs for 2.6 rounds of work cost 14 %.)
 // Persistent: a pair takes (256 rows of w, run) in turn, the runs of one expert next to each other in time.  Roles of a CTA's ten warps:
 //   * warp 0, one thread: per 64 elements of K a tiled copy of its 128 rows of w and one for every 32 of its half of the run's rows
 //     of x into the next stage of a ring (128-byte swizzle; what lies beyond a matrix comes as zeros, what lies beyond a run is

@@ -2010,8 +2010,8 @@ def few_outputs_rows(outputs: int) -> int:
 def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = None,
            bias: torch.Tensor | None = None) -> torch.Tensor:
     """y = x w^T.  float32 runs on this package's CUDA-core kernel (no TF32 anywhere).  bfloat16
-    with up to 64 rows (a decode step) runs on this package's weight-streaming kernel; larger
-    bfloat16 products of more than a few outputs run on the vendor library's tensor-core product, as the reference's linear
+    with up to 16 rows (a decode step) and, with few outputs, up to ``few_outputs_rows`` runs on this package's weight-streaming
+    kernel; other bfloat16 products run on the vendor library's tensor-core product, as the reference's linear
     layers do (src/layer/linear.cpp:22-24 -> cuBLASLt), where that is the faster one; with
     ``USE_LIBRARY_PRODUCTS`` off they run on this package's tcgen05 kernel (``gemm_tc``), so that no
     library kernel is left on the path.  Accumulation is float32 everywhere.  A ``bias`` [N] is
