@@ -6,7 +6,7 @@ import math
 import pytest
 import torch
 
-from test_kernels_gpu import build_paged_case, ops  # noqa: F401  (ops: a fixture)
+from test_kernels_gpu import build_paged_case, ops, rand  # noqa: F401  (ops: a fixture)
 
 pytestmark = pytest.mark.gpu
 
@@ -89,3 +89,43 @@ def test_the_timing_program_cuts_as_it_says(ops, cuda_device, capsys, options, s
     timing.main(["decode_attention", "--warmup", "1", "--iters", "2", *options])
     line = json.loads(capsys.readouterr().out)
     assert line["split_size"] == size and line["timeline_ns"]["tiles"][1] == most
+
+
+@pytest.mark.parametrize("even", [True, False])
+@pytest.mark.parametrize("form", ["narrow heads", "keys that are values", "distance bias", "bounded scores", "a chunk", "norms inside"])
+def test_the_cut_by_lengths_in_every_form(ops, cuda_device, form, even):
+    """The kernel that looks at the lengths gives what the cut that it takes gives on its own, bit for bit."""
+    hd, page, n = 64 if form == "narrow heads" else 128, 16, 12
+    nh, nkv = (48, 8) if form == "distance bias" else (16, 8)
+    ctx = [400 + 7 * r for r in range(n)] if even else [3800] + [40 + 9 * r for r in range(n - 1)]
+    keys_only, chunk = form == "keys that are values", 4000 if form == "a chunk" else 0
+    pages = [-(-(c + 1) // page) for c in ctx]
+    table, at = torch.zeros((n, max(pages)), dtype=torch.int32), 1
+    order = torch.randperm(sum(pages), generator=torch.Generator().manual_seed(3)) + 1
+    for r, count in enumerate(pages):
+        table[r, :count], at = order[at - 1:at - 1 + count], at + count
+    table = table.to(cuda_device)
+    shape = (sum(pages) + 1, nkv * page * hd) if keys_only else (sum(pages) + 1, 2, nkv, page, hd)
+    cache = rand(shape, torch.bfloat16, cuda_device, 540)
+    rows, behind = torch.arange(n, dtype=torch.int32, device=cuda_device), torch.tensor(ctx, dtype=torch.int32, device=cuda_device)
+    status, most = ops.new_status(cuda_device), max(ctx) + 1
+    options = {"distance bias": dict(distance_bias=(torch.linspace(0.1, 2, nh, device=cuda_device), torch.linspace(0.01, 0.5, nh, device=cuda_device))),
+               "bounded scores": dict(softcap=20.0, sinks=torch.linspace(-1, 2, nh, device=cuda_device))}.get(form, {})
+    if chunk:
+        options["chunk"] = chunk
+    got = {}
+    for split in (None, 4096 if even else 0):
+        out = torch.full((n, nh * hd), float("nan"), dtype=torch.bfloat16, device=cuda_device)
+        if form == "norms inside":
+            scale = rand((hd,), torch.float32, cuda_device, 541).to(torch.bfloat16)
+            qkv = rand((n, (nh + 2 * nkv) * hd), torch.bfloat16, cuda_device, 542)
+            ops.paged_decode_fused(qkv, cache, table, rows, rows, behind, most, nh, nkv, hd, 0, hd ** -0.5, scale, scale, 1e-6, None, None,
+                                   status, out, split_size=split)
+        else:
+            q = rand((n, nh * hd), torch.bfloat16, cuda_device, 543)
+            ops.paged_decode(q, cache, table, rows, rows, behind, most, nh, nkv, hd, 0, hd ** -0.5, status, out, split_size=split,
+                             keys_only=keys_only, **options)
+        got[split] = out
+    ops.check_status(status)
+    chosen, alone = got.values()
+    assert torch.isfinite(chosen).all() and torch.equal(chosen, alone)

@@ -60,7 +60,9 @@ class StepContext:
 
     def rows_with_tiles(self, which: str) -> int:
         """How many rows the tiles of ``tiles[(..., which)]`` come from."""
-        return {"all": self.num_rows, "single": self.num_decode_rows, "multi": self.num_rows - self.num_decode_rows}[which]
+        if which == "all":
+            return self.num_rows
+        return self.num_decode_rows if which == "single" else self.num_rows - self.num_decode_rows
 
     def block_table(self, cache_id: int) -> torch.Tensor:
         return self.block_tables[self.group_of_cache[cache_id]]
