@@ -85,7 +85,8 @@ def _paged_inputs(batch: int, context: int, nkv: int, hd: int, page: int, device
 
 def decode_attention(args) -> dict:
     device = torch.device("cuda")
-    contexts = [int(n) for n in args.contexts.split(",")] if args.contexts else [args.context] * args.batch
+    listed = getattr(args, "contexts", "")
+    contexts = [int(n) for n in listed.split(",")] if listed else [args.context] * args.batch
     nh, nkv, hd, B, ctx = args.heads, args.kv_heads, args.head_dim, len(contexts), max(contexts)
     caches, table = _paged_inputs(B, ctx, nkv, hd, args.page_size, device, args.keys_only)
     q = torch.randn((B, nh * hd), device=device, dtype=torch.bfloat16)
@@ -109,7 +110,7 @@ def decode_attention(args) -> dict:
     ops.check_status(status, "decode_attention")
     live = [min(n, args.window or n, (n - 1) % chunk + 1 if chunk else n) for n in contexts]
     read = sum(live) * nkv * hd * 2 * (1 if args.keys_only else 2)
-    return {"kernel": "paged_decode_kernel", "softcap": args.softcap, "keys_only": args.keys_only, "batch": B, "context": args.contexts or ctx, "heads": nh, "kv_heads": nkv, "head_dim": hd,
+    return {"kernel": "paged_decode_kernel", "softcap": args.softcap, "keys_only": args.keys_only, "batch": B, "context": listed or ctx, "heads": nh, "kv_heads": nkv, "head_dim": hd,
             "page_size": args.page_size, "window": args.window, "chunk": chunk, "split_size": "chosen" if split is None else split or "balanced", "us": round(us, 2),
             "bytes_read": read, "gbs": round(read / us / 1e3, 1), "timeline_ns": _decode_timeline(trace)}
 
