@@ -54,6 +54,12 @@ __device__ __forceinline__ void tmem_ld32(unsigned address, unsigned (&r)[32]) {
                  "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
                : "r"(address) : "memory");
 }
+__device__ __forceinline__ void tmem_ld16(unsigned address, unsigned (&r)[16]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                 "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+               : "r"(address) : "memory");
+}
 // Waits for this thread's tensor-memory loads; `r`, what a load was asked to bring, is not used before.
 __device__ __forceinline__ void tmem_wait_ld32(unsigned (&r)[32]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;\n"
@@ -61,6 +67,12 @@ __device__ __forceinline__ void tmem_wait_ld32(unsigned (&r)[32]) {
                  "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]),
                  "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]),
                  "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
+               :: "memory");
+}
+__device__ __forceinline__ void tmem_wait_ld16(unsigned (&r)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;\n"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                 "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
                :: "memory");
 }
 __device__ __forceinline__ void tmem_st32(unsigned address, const unsigned (&r)[32]) {
@@ -113,6 +125,18 @@ __device__ __forceinline__ unsigned in_cta_of_rank(unsigned smem_address, unsign
 }
 __device__ __forceinline__ void mbar_arrive_in_cluster(unsigned cluster_address) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_address) : "memory");
+}
+// One arrival that orders this CTA's accesses only: what the other CTA's thread does after it concerns this CTA's shared and tensor
+// memory through the tensor cores, not through its own loads.  (A release across the cluster waits for every load in flight.)
+__device__ __forceinline__ void mbar_arrive_at(unsigned cluster_address) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_address) : "memory");
+}
+// A look at a barrier of this CTA that the other CTA's warps arrive on too.
+__device__ __forceinline__ bool mbar_try_wait_cluster(unsigned long long* bar, unsigned parity) {
+  unsigned done;
+  asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+               : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+  return done != 0;
 }
 // A tiled copy into this CTA's shared memory whose bytes are counted on a barrier of the pair's first CTA.
 __device__ __forceinline__ void tiled_copy_2d_g2s_pair(void* smem_dst, const CUtensorMap* map, int x, int y, unsigned bar_cluster_address) {

@@ -212,6 +212,7 @@ _SIGNATURES = {
                                  c_longlong, c_longlong, c_longlong, c_void_p, c_void_p],
     "zb_gemm_nt_simt": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong,
                         c_int, c_int, c_void_p],
+    "zb_gemm_nt_f32": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_void_p, c_void_p],
     "zb_fused_chain_stage_supported": [c_int, c_int, c_int, c_int, c_int],
     "zb_fused_chain_max_stages": [],
     "zb_fused_chain_grid": [],
@@ -1724,7 +1725,8 @@ def short_prompts(block_table: torch.Tensor, page_size: int, nh: int, tiles: int
 # ------------------------------------------------------------------------ matrix products
 def gemm_nt_simt(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = None,
                  out: torch.Tensor | None = None) -> torch.Tensor:
-    """x [M, K] times w [N, K] transposed, float32 multiply-adds on CUDA cores."""
+    """x [M, K] times w [N, K] transposed: every product and sum in float32, by multiply-adds on CUDA cores or, for float32 rows that
+    start on 16-byte boundaries, from three bfloat16 parts a value on the tensor cores (as near to the exact sums, or nearer)."""
     _cuda(x, w)
     _require(x.dim() == 2 and w.dim() == 2 and x.shape[1] == w.shape[1] and x.dtype == w.dtype
              and x.dtype in DTYPE_CODE and x.stride(1) == 1 and w.stride(1) == 1, "x [M, K] and w [N, K] of one type")
@@ -1734,6 +1736,10 @@ def gemm_nt_simt(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None
     if out is None:
         out = torch.empty((M, N), dtype=out_dtype, device=x.device)
     _require(out.shape == (M, N) and out.dtype == out_dtype and out.stride(1) == 1, "out must be [M, N]")
+    if x.dtype == out_dtype == torch.float32:
+        _check(library().zb_gemm_nt_f32(_ptr(out), _ptr(x), _ptr(w), M, N, K, x.stride(0), w.stride(0), out.stride(0),
+                                        _ptr(device_status(x.device)), _stream()), "gemm_nt_simt")
+        return out
     _check(library().zb_gemm_nt_simt(_ptr(out), _ptr(x), _ptr(w), M, N, K, x.stride(0), w.stride(0), out.stride(0),
                                      DTYPE_CODE[x.dtype], DTYPE_CODE[out_dtype], _stream()), "gemm_nt_simt")
     return out
@@ -2009,7 +2015,7 @@ def few_outputs_rows(outputs: int) -> int:
 
 def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = None,
            bias: torch.Tensor | None = None) -> torch.Tensor:
-    """y = x w^T.  float32 runs on this package's CUDA-core kernel (no TF32 anywhere).  bfloat16
+    """y = x w^T.  float32 runs on this package's float32 product (no TF32 anywhere).  bfloat16
     with up to 16 rows (a decode step) and, with few outputs, up to ``few_outputs_rows`` runs on this package's weight-streaming
     kernel; other bfloat16 products run on the vendor library's tensor-core product, as the reference's linear
     layers do (src/layer/linear.cpp:22-24 -> cuBLASLt), where that is the faster one; with
