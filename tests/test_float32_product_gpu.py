@@ -1,12 +1,12 @@
-"""The float32 product on the tensor cores at the edges of its tiles and stages, near the exact sums, and over values that its three
-parts do not hold."""
+"""The float32 product and the float32 attention on the tensor cores, at the edges of their tiles and stages, near the exact sums, and over
+values that three bfloat16 parts do not hold."""
 
 import math
 
 import pytest
 import torch
 
-from test_kernels_gpu import ops, rand  # noqa: F401  (ops: a fixture)
+from test_kernels_gpu import build_paged_case, ops, rand, ref_attention_row, tiles_for  # noqa: F401  (ops: a fixture)
 
 pytestmark = pytest.mark.gpu
 
@@ -36,3 +36,39 @@ def test_values_beyond_the_parts(ops, cuda_device):
     fine = torch.arange(140, device=cuda_device) != 9
     a, b = got[rows][:, fine].double(), exact[rows][:, fine]
     assert ((a - b).norm(dim=1) <= 256 * 2.0 ** -24 * b.norm(dim=1)).all()
+
+
+@pytest.mark.parametrize("nh,nkv,hd,window,chunk,q_lens,ctx", [
+    (4, 2, 128, 0, 0, [64, 65, 2], [0, 63, 640]), (2, 2, 64, 100, 0, [129, 200], [0, 17]), (40, 1, 60, 0, 96, [7, 30], [90, 0]),
+    (64, 1, 128, 0, 0, [5], [127])])
+def test_attention_is_near_the_exact_one_and_as_finite_as_the_general_kernel(ops, cuda_device, nh, nkv, hd, window, chunk, q_lens, ctx):
+    """Rows and contexts at the edges of a CTA's pairs and of a step's keys; then keys and values that bfloat16 parts do not hold."""
+    q, cache, meta, Ks, Vs, qs = build_paged_case(cuda_device, torch.float32, nh, nkv, hd, 16, q_lens, ctx, 100)
+    status, wide, tokens = ops.new_status(cuda_device), ops.paged_prefill_tile_tokens(), ops.attention_tile_tokens(nh // nkv)
+    common = (meta["row_q_start"], meta["row_q_len"], meta["row_ctx"], nh, nkv, hd, window, 1 / math.sqrt(hd), status)
+
+    def run(held):
+        out = torch.empty_like(q)
+        ops.paged_attention_f32(q, held, meta["table"], *tiles_for(q_lens, wide, cuda_device, only_multi=True), wide, *common, out, chunk=chunk)
+        general = ops.paged_attention(q, held, meta["table"], *tiles_for(q_lens, tokens, cuda_device), tokens, *common, chunk=chunk)
+        ops.check_status(status)
+        return out, general
+
+    got, general = run(cache)
+    cursor = 0
+    for r, n in enumerate(q_lens):
+        if not chunk:
+            exact = ref_attention_row(qs[r].double(), Ks[r].double(), Vs[r].double(), ctx[r], n, window, nh, nkv).view(n, -1)
+            # A score: 8 cuts of its sum and one of the small parts', at most 2^-23 of a magnitude of a few; exponential, sum and division
+            # two roundings each; 4 cuts a step of keys of the values' sums.
+            assert (got[cursor:cursor + n].double().cpu() - exact.cpu()).norm() <= 32 * 2.0 ** -23 * exact.norm()
+        cursor += n
+    assert (got - general).abs().max() <= 2e-5
+    held, at = cache.clone(), ctx[0] + q_lens[0] // 2
+    page = meta["table"][0, at // 16]
+    held[page, 0, :, at % 16] = 3.4e38                     # a key: its scores reach infinity, of either sign
+    held[page, 1, :, at % 16, :4] = 3.4e38                 # and its values
+    got, general = run(held)
+    assert torch.equal(got.isfinite(), general.isfinite())
+    fine = got.isfinite()
+    assert ((got - general)[fine].abs() <= 2e-5 * general[fine].abs().clamp(min=1.0)).all()

@@ -61,17 +61,6 @@ struct GemmF32Args {
   int* status;
 };
 
-// x and y as three pairs of bfloat16 values whose sums they are, the largest first.
-__device__ __forceinline__ void three_parts(float x, float y, unsigned& hi, unsigned& mid, unsigned& lo) {
-  hi = pack_bf16(x, y);
-  x -= __uint_as_float(hi << 16);
-  y -= __uint_as_float(hi & 0xffff0000u);
-  mid = pack_bf16(x, y);
-  x -= __uint_as_float(mid << 16);
-  y -= __uint_as_float(mid & 0xffff0000u);
-  lo = pack_bf16(x, y);
-}
-
 // One output by multiply-adds in ascending k.
 __device__ __noinline__ float dot_f32(const float* x, const float* w, int K) {
   float sum = 0.0f;
