@@ -18,9 +18,10 @@
 //                 lies [V][D] (a column's channels together).
 //
 // Rows that bring runs of tokens go to two other kernels (delta_blocks, delta_block_scan below): the same rule, block by
-// block of 16 tokens.
+// block of 32 tokens.
 //
-// Everything here is float32 multiply-adds in either form; the values v are read in the model's type.
+// Token by token everything is float32 multiply-adds; in blocks products are formed on the tensor cores from three bfloat16 parts a value, all
+// 24 bits of it, with float32 sums.  The values v are read in the model's type.
 #include "common.cuh"
 #include "mma.cuh"
 
@@ -339,14 +340,34 @@ __global__ void __launch_bounds__(DS_THREADS) delta_scan_kernel(const DeltaScanA
 // are formed in 64 bits and kept as two float32 values, so that a difference is good to a rounding of itself, also behind a
 // token that forgets everything.
 // Tokens behind a portion's end have beta 0 and decay 1.  Blocks are numbered row by row (first_piece_of_row).
-constexpr int DB = 16;                     // tokens of a block
+constexpr int DB = 32;                     // tokens of a block
 constexpr int DB_THREADS = 256;
 constexpr int DB_COLS = 16;                // value columns of a CTA
-constexpr int DB_COEF = 2 * DB * DB + 2 * DB;      // Tu and M, both [j][t], e^(c_t), e^(c_B) and padding
+constexpr int DB_HEADS = 2;                // heads whose matrices a CTA of delta_blocks makes side by side
+constexpr int DB_MST = DB + 8;             // a row of Tu or M in bfloat16
+constexpr int DB_FST = DB + 1;             // a row of a float32 matrix
+constexpr int DB_COEF_PARTS = 3 * 2 * DB * DB_MST * 2;
+constexpr int DB_COEF_BYTES = DB_COEF_PARTS + (DB + 4) * 4;       // Tu over M, [part][t][j], then e^(c_t), e^(c_B) and padding
+constexpr float DB_LARGEST = 3.3e38f;      // beyond it a value rounds to infinity in bfloat16
+constexpr int DB_WAIT_LIMIT = 1 << 20;
+
+// DP: the channels padded with zeros.
+template <int DP>
+struct DeltaShape {
+  static constexpr int ST = DP + 8;                               // a row of k or q in bfloat16
+  static constexpr int QK_BYTES = 3 * 2 * DB * ST * 2;            // [part][k of the block's tokens, then q][ST]
+  static constexpr int STAGE_BYTES = QK_BYTES + DB_COEF_BYTES;
+  static constexpr int CST = DB_COLS + 8, FST = DB_COLS + 4;      // rows of value columns: bfloat16, float32
+  static constexpr int S_BYTES = 3 * DP * CST * 2, V_BYTES = 3 * DB * CST * 2, F_BYTES = DB * FST * 4, RED_BYTES = DP / 16 * 2 * DB * DB_COLS * 4;
+  static constexpr int BLOCKS_SMEM = QK_BYTES + (2 + 3 * DB_HEADS) * DB * DB_FST * 4 + DB_HEADS * 5 * DB * 4;
+  static constexpr int SCAN_SMEM = 2 * STAGE_BYTES + S_BYTES + 2 * V_BYTES + 2 * F_BYTES + RED_BYTES;
+  static_assert(QK_BYTES % 16 == 0 && DB_COEF_BYTES % 16 == 0, "bulk copies move 16-byte pieces");
+  static_assert(SCAN_SMEM <= 226 * 1024, "fits an SM's shared memory");
+};
 
 struct DeltaBlocksArgs {
-  float* qk;               // [blocks][qk_heads][DP][2 DB]: k of the block's tokens, then q
-  float* coef;             // [blocks][heads][DB_COEF]
+  unsigned char* qk;       // [blocks][qk_heads][QK_BYTES]
+  unsigned char* coef;     // [blocks][heads][DB_COEF_BYTES]
   const void* q; long long q_stride;
   const void* k; long long k_stride;
   const float* b; const float* a; long long ba_stride;
@@ -356,24 +377,40 @@ struct DeltaBlocksArgs {
   float q_scale, unit_eps;
 };
 
-// DP: the channels padded with zeros.
+// M products of 16 rows by NT tiles of 8 columns, operands in three parts: low += the products of parts behind hi hi, smallest first; high +=
+// hi hi.  (The tensor cores cut a sum's last bits at every step: what is cut off the small products' sum is 2^-8 of that.)  The
+// tiles take turns, so that no product waits for the one before it.
+template <int M, int NT>
+__device__ __forceinline__ void delta_products(float (&high)[M][NT][4], float (&low)[M][NT][4], const unsigned (&a)[M][3][4],
+                                               const unsigned (&b)[M][3][2 * NT]) {
+  constexpr int FIRST[6] = {2, 1, 0, 1, 0, 0}, SECOND[6] = {0, 1, 2, 0, 1, 0};
+#pragma unroll
+  for (int e = 0; e < 6; ++e)
+#pragma unroll
+    for (int m = 0; m < M; ++m)
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+        mma_bf16_16816(e < 5 ? low[m][n] : high[m][n], a[m][FIRST[e]], b[m][SECOND[e]][2 * n], b[m][SECOND[e]][2 * n + 1]);
+}
+
 template <typename T, int DP>
 __global__ void __launch_bounds__(DB_THREADS) delta_blocks_kernel(const DeltaBlocksArgs a) {
   wait_for_prior_grids();
   let_dependents_launch();
-  extern __shared__ __align__(16) float db_smem[];
-  constexpr int ST = DP + 4;
-  float* x_s = db_smem;                    // [2 DB][ST]: k, q
-  float* kk_s = x_s + 2 * DB * ST;         // [DB][DB]
-  float* qk_s = kk_s + DB * DB;
-  float* a_s = qk_s + DB * DB;             // [DB][DB]: A
-  float* p_s = a_s + DB * DB;              // [DB][DB]: P
-  float* t_s = p_s + DB * DB;              // [DB][DB]: (I + A)^-1 diag(beta)
-  float* c_hi = t_s + DB * DB;             // [DB]: the sums of logarithms c_t = c_hi + c_lo
-  float* c_lo = c_hi + DB;
-  float* lead_s = c_lo + DB;               // [DB]: e^(c_t)
-  float* tail_s = lead_s + DB;             // [DB]: e^(c_B - c_t)
-  float* beta_s = tail_s + DB;
+  using Shape = DeltaShape<DP>;
+  constexpr int ST = Shape::ST, MATRIX = DB * DB_FST;
+  extern __shared__ __align__(16) unsigned char db_smem[];
+  __nv_bfloat16* x_s = reinterpret_cast<__nv_bfloat16*>(db_smem);              // [part][k, q][ST]
+  float* kk_s = reinterpret_cast<float*>(db_smem + Shape::QK_BYTES);           // [DB][DB_FST] each
+  float* qk_s = kk_s + MATRIX;
+  float* a_s = qk_s + MATRIX;              // [head]: A
+  float* p_s = a_s + DB_HEADS * MATRIX;    // [head]: P
+  float* t_s = p_s + DB_HEADS * MATRIX;    // [head]: (I + A)^-1
+  float* c_hi = t_s + DB_HEADS * MATRIX;   // [head][DB]: the sums of logarithms c_t = c_hi + c_lo
+  float* c_lo = c_hi + DB_HEADS * DB;
+  float* lead_s = c_lo + DB_HEADS * DB;    // [head][DB]: e^(c_t)
+  float* tail_s = lead_s + DB_HEADS * DB;  // [head][DB]: e^(c_B - c_t)
+  float* beta_s = tail_s + DB_HEADS * DB;
   const int block = blockIdx.x, group = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int own;
   const int row = row_of_piece<DB>(a.row_q_len, a.rows, a.from, block, own);
@@ -382,69 +419,64 @@ __global__ void __launch_bounds__(DB_THREADS) delta_blocks_kernel(const DeltaBlo
   const long long t0 = a.row_q_start[row] + begin;
 #pragma unroll
   for (int u = 0; u < 2 * DB / (DB_THREADS / 32); ++u) {
-    const int i = warp + u * (DB_THREADS / 32);
+    const int i = warp + u * (DB_THREADS / 32), t = i % DB;
     const bool is_q = i >= DB;
-    const int t = i % DB;
     const T* src = is_q ? static_cast<const T*>(a.q) + (t0 + t) * a.q_stride + group * a.D
                         : static_cast<const T*>(a.k) + (t0 + t) * a.k_stride + group * a.D;
-    float x[DP / 32], ss = 0.0f;
+    float x[DP / 64][2], ss = 0.0f;
 #pragma unroll
-    for (int j = 0; j < DP / 32; ++j) {
-      const int d = lane + 32 * j;
-      x[j] = t < n && d < a.D ? to_float(src[d]) : 0.0f;
-      ss = fmaf(x[j], x[j], ss);
+    for (int j = 0; j < DP / 64; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int d = 64 * j + 2 * lane + e;
+        x[j][e] = t < n && d < a.D ? to_float(src[d]) : 0.0f;
+        ss = fmaf(x[j][e], x[j][e], ss);
+      }
+    const float inv = t < n ? (is_q ? a.q_scale : 1.0f) / sqrtf(warp_sum(ss) + a.unit_eps) : 0.0f;
+#pragma unroll
+    for (int j = 0; j < DP / 64; ++j) {
+      unsigned part[3];
+      three_parts(x[j][0] * inv, x[j][1] * inv, part[0], part[1], part[2]);
+#pragma unroll
+      for (int e = 0; e < 3; ++e) *reinterpret_cast<unsigned*>(x_s + (e * 2 * DB + i) * ST + 64 * j + 2 * lane) = part[e];
     }
-    const float inv = (is_q ? a.q_scale : 1.0f) / sqrtf(warp_sum(ss) + a.unit_eps);
-#pragma unroll
-    for (int j = 0; j < DP / 32; ++j) x_s[i * ST + lane + 32 * j] = t < n ? x[j] * inv : 0.0f;
   }
   __syncthreads();
-  float4* to = reinterpret_cast<float4*>(a.qk + (static_cast<long long>(block) * a.qk_heads + group) * DP * 2 * DB);
-  for (int e = tid; e < DP * 2 * DB / 4; e += DB_THREADS) {
-    const int d = e / (2 * DB / 4), i = e % (2 * DB / 4) * 4;
-    to[e] = make_float4(x_s[i * ST + d], x_s[(i + 1) * ST + d], x_s[(i + 2) * ST + d], x_s[(i + 3) * ST + d]);
-  }
+  uint4* to = reinterpret_cast<uint4*>(a.qk + (static_cast<long long>(block) * a.qk_heads + group) * Shape::QK_BYTES);
+  for (int e = tid; e < Shape::QK_BYTES / 16; e += DB_THREADS) to[e] = reinterpret_cast<const uint4*>(x_s)[e];
   {
-    // k . k and q . k: a thread takes two tokens by two over a quarter of the channels (every fourth run of four).
-    const int part = tid & 3, j0 = tid >> 2 & 7, i0 = tid >> 5;        // tokens i0, i0 + 8 against j0, j0 + 8
-    float kk[2][2] = {}, qk[2][2] = {};
+    // k . k and q . k: a warp takes 16 rows of k or q against 16 of k; what lies above the diagonal tiles is not read.
+    const int row0 = warp / 2 * 16, col0 = warp % 2 * 16, g = lane >> 2, t = lane & 3;
+    if (row0 % DB >= col0) {
+      const __nv_bfloat16* rows = x_s + (row0 + (lane & 7) + ((lane >> 3) & 1) * 8) * ST + (lane >> 4) * 8;
+      const __nv_bfloat16* columns = x_s + (col0 + (lane & 7) + (lane >> 4) * 8) * ST + ((lane >> 3) & 1) * 8;
+      float high[2][2][4] = {}, low[2][2][4] = {};
 #pragma unroll
-    for (int d = 4 * part; d < DP; d += 16) {
-      float4 kj[2], ki[2], qi[2];
+      for (int ks = 0; ks < DP / 16; ks += 2) {
+        unsigned af[2][3][4], bf[2][3][4];
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        kj[u] = *reinterpret_cast<const float4*>(x_s + (j0 + 8 * u) * ST + d);
-        ki[u] = *reinterpret_cast<const float4*>(x_s + (i0 + 8 * u) * ST + d);
-        qi[u] = *reinterpret_cast<const float4*>(x_s + (DB + i0 + 8 * u) * ST + d);
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+          for (int e = 0; e < 3; ++e) {
+            ldmatrix_x4(af[u][e], rows + e * 2 * DB * ST + (ks + u) * 16);
+            ldmatrix_x4(bf[u][e], columns + e * 2 * DB * ST + (ks + u) * 16);
+          }
+        delta_products<2, 2>(high, low, af, bf);
       }
+      float* out = row0 < DB ? kk_s : qk_s;
 #pragma unroll
-      for (int u = 0; u < 2; ++u)
+      for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int w = 0; w < 2; ++w) {
-          kk[u][w] = fmaf(ki[u].x, kj[w].x, fmaf(ki[u].y, kj[w].y, fmaf(ki[u].z, kj[w].z, fmaf(ki[u].w, kj[w].w, kk[u][w]))));
-          qk[u][w] = fmaf(qi[u].x, kj[w].x, fmaf(qi[u].y, kj[w].y, fmaf(qi[u].z, kj[w].z, fmaf(qi[u].w, kj[w].w, qk[u][w]))));
-        }
+        for (int e = 0; e < 4; ++e)
+          out[(row0 % DB + g + (e >> 1) * 8) * DB_FST + col0 + 8 * i + 2 * t + (e & 1)] = (high[0][i][e] + high[1][i][e]) + (low[0][i][e] + low[1][i][e]);
     }
-#pragma unroll
-    for (int u = 0; u < 2; ++u)
-#pragma unroll
-      for (int w = 0; w < 2; ++w) {
-#pragma unroll
-        for (int o = 1; o < 4; o <<= 1) {
-          kk[u][w] += __shfl_xor_sync(0xffffffffu, kk[u][w], o);
-          qk[u][w] += __shfl_xor_sync(0xffffffffu, qk[u][w], o);
-        }
-        if (part == 0) {
-          kk_s[(i0 + 8 * u) * DB + j0 + 8 * w] = kk[u][w];
-          qk_s[(i0 + 8 * u) * DB + j0 + 8 * w] = qk[u][w];
-        }
-      }
   }
-  const int t = tid / DB, j = tid % DB;
   const int per = a.heads / a.qk_heads;
-  for (int h = group * per; h < (group + 1) * per; ++h) {
-    __syncthreads();                       // the products are there, and the head before is done
-    if (tid < 32) {
+  for (int h0 = group * per; h0 < (group + 1) * per; h0 += DB_HEADS) {
+    const int count = min(DB_HEADS, (group + 1) * per - h0);
+    __syncthreads();                       // the products are there, and the heads before are done
+    if (warp < count) {
+      const int h = h0 + warp;
       double c = 0.0;
       float beta = 0.0f;
       if (lane < n) {
@@ -459,50 +491,109 @@ __global__ void __launch_bounds__(DB_THREADS) delta_blocks_kernel(const DeltaBlo
         if (lane >= o) c += before;
       }
       const double all = __shfl_sync(0xffffffffu, c, DB - 1);
-      if (lane < DB) {
-        const float hi = static_cast<float>(c), lo = static_cast<float>(c - hi), lead = expf(hi);
-        c_hi[lane] = hi;
-        c_lo[lane] = lo;
-        lead_s[lane] = fmaf(lead, lo, lead);
-        tail_s[lane] = expf(static_cast<float>(all - c));
-        beta_s[lane] = beta;
-      }
+      const float hi = static_cast<float>(c), lo = static_cast<float>(c - hi), lead = expf(hi);
+      const int at = warp * DB + lane;
+      c_hi[at] = hi;
+      c_lo[at] = lo;
+      lead_s[at] = fmaf(lead, lo, lead);
+      tail_s[at] = expf(static_cast<float>(all - c));
+      beta_s[at] = beta;
     }
     __syncthreads();
-    const float decay = j <= t ? expf((c_hi[t] - c_hi[j]) + (c_lo[t] - c_lo[j])) : 0.0f;
-    a_s[tid] = j < t ? beta_s[t] * decay * kk_s[tid] : 0.0f;
-    p_s[tid] = decay * qk_s[tid];
+#pragma unroll
+    for (int u = 0; u < DB_HEADS * DB * DB / DB_THREADS; ++u) {
+      const int e = tid + u * DB_THREADS, w = e / (DB * DB), t = e / DB % DB, j = e % DB;
+      if (w >= count) break;
+      const float* hi = c_hi + w * DB, * lo = c_lo + w * DB;
+      const float decay = j <= t ? expf((hi[t] - hi[j]) + (lo[t] - lo[j])) : 0.0f;
+      a_s[w * MATRIX + t * DB_FST + j] = j < t ? beta_s[w * DB + t] * decay * kk_s[t * DB_FST + j] : 0.0f;
+      p_s[w * MATRIX + t * DB_FST + j] = j <= t ? decay * qk_s[t * DB_FST + j] : 0.0f;
+    }
     __syncthreads();
-    float* coef = a.coef + (static_cast<long long>(block) * a.heads + h) * DB_COEF;
-    if (tid < DB) {
-      // A column of the inverse by forward substitution, times beta of the column.
-      float x[DB];
+    // (I + A)^-1 = [T1 0; -T2 A21 T1, T2]: a column of T1 or T2 a lane, by forward substitution.
+    if (warp < count) {
+      const int half = lane / 16, column = lane % 16;
+      const float* from = a_s + warp * MATRIX + 16 * half * (DB_FST + 1);
+      float* result = t_s + warp * MATRIX + 16 * half * (DB_FST + 1);
+      float x[16];
 #pragma unroll
-      for (int i = 0; i < DB; ++i) {
-        float sum = i == tid ? 1.0f : 0.0f;
+      for (int i = 0; i < 16; ++i) {
+        float sum = i == column ? 1.0f : 0.0f;
 #pragma unroll
-        for (int m = 0; m < i; ++m) sum = fmaf(-a_s[i * DB + m], x[m], sum);
+        for (int m = 0; m < i; ++m) sum = fmaf(-from[i * DB_FST + m], x[m], sum);
         x[i] = sum;
+        result[i * DB_FST + column] = sum;
       }
-#pragma unroll
-      for (int i = 0; i < DB; ++i) t_s[i * DB + tid] = x[i] * beta_s[tid];
     }
     __syncthreads();
-    // (threads run over the rows of the transposed matrices: t fastest)
-    const int tt = tid % DB, jj = tid / DB;
-    coef[jj * DB + tt] = tail_s[tt] * t_s[tt * DB + jj];
-    float m = 0.0f;
-    for (int i = jj; i <= tt; ++i) m = fmaf(p_s[tt * DB + i], t_s[i * DB + jj], m);
-    coef[(DB + jj) * DB + tt] = m;
-    if (tid < DB) coef[2 * DB * DB + tid] = lead_s[tid];
-    if (tid == 0) coef[2 * DB * DB + DB] = lead_s[DB - 1];
+    // A21 T1, into the quarter of A that is zero.
+    const int ti = tid / 16, tj = tid % 16;
+#pragma unroll
+    for (int w = 0; w < DB_HEADS; ++w) {
+      if (w >= count) break;
+      const float* from = a_s + w * MATRIX + (16 + ti) * DB_FST, * t1 = t_s + w * MATRIX + tj;
+      float sum = 0.0f;
+#pragma unroll
+      for (int m = 0; m < 16; ++m) sum = fmaf(from[m], t1[m * DB_FST], sum);
+      a_s[w * MATRIX + ti * DB_FST + 16 + tj] = sum;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < DB_HEADS; ++w) {
+      if (w >= count) break;
+      const float* t2 = t_s + w * MATRIX + (16 + ti) * DB_FST + 16, * from = a_s + w * MATRIX + 16 + tj;
+      float sum = 0.0f;
+#pragma unroll
+      for (int m = 0; m < 16; ++m) sum = fmaf(-t2[m], m <= ti ? from[m * DB_FST] : 0.0f, sum);      // (a later token's row may hold anything)
+      t_s[w * MATRIX + (16 + ti) * DB_FST + tj] = sum;
+      t_s[w * MATRIX + ti * DB_FST + 16 + tj] = 0.0f;
+    }
+    __syncthreads();
+    // A thread makes columns j and j + 1 of rows t, t + 8, t + 16 and t + 24 of a head's matrices.
+    static_assert(DB_HEADS * DB * DB / 8 == DB_THREADS, "eight values a thread");
+    const int w = tid / (DB_THREADS / DB_HEADS), t = tid / 16 % 8, j = tid % 16 * 2;
+    if (w < count) {
+      unsigned char* coef = a.coef + (static_cast<long long>(block) * a.heads + h0 + w) * DB_COEF_BYTES;
+      const float* inverse = t_s + w * MATRIX + j, * p = p_s + w * MATRIX + t * DB_FST;
+      float m[4][2] = {};
+#pragma unroll
+      for (int i0 = 0; i0 < DB; i0 += 8)
+#pragma unroll
+        for (int i = i0; i < i0 + 8; ++i) {
+          const float x = inverse[i * DB_FST], y = inverse[i * DB_FST + 1];
+#pragma unroll
+          for (int r = i0 / 8; r < 4; ++r) {
+            const bool seen = 8 * r > i || i - 8 * r <= t;                // (a later token's row may hold anything)
+            const float weight = p[8 * r * DB_FST + i];
+            m[r][0] = fmaf(weight, seen ? x : 0.0f, m[r][0]);
+            m[r][1] = fmaf(weight, seen ? y : 0.0f, m[r][1]);
+          }
+        }
+      const float beta0 = beta_s[w * DB + j], beta1 = beta_s[w * DB + j + 1];
+      float* steps = reinterpret_cast<float*>(coef + DB_COEF_PARTS);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int row_t = t + 8 * r;
+        const float tail = tail_s[w * DB + row_t];
+        unsigned up[3], mp[3];
+        three_parts(tail * (inverse[row_t * DB_FST] * beta0), tail * (inverse[row_t * DB_FST + 1] * beta1), up[0], up[1], up[2]);
+        three_parts(m[r][0] * beta0, m[r][1] * beta1, mp[0], mp[1], mp[2]);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          *reinterpret_cast<unsigned*>(coef + ((i * 2 * DB + row_t) * DB_MST + j) * 2) = up[i];
+          *reinterpret_cast<unsigned*>(coef + ((i * 2 * DB + DB + row_t) * DB_MST + j) * 2) = mp[i];
+        }
+        if (j == 0) steps[row_t] = lead_s[w * DB + row_t];
+      }
+      if (t == 0 && j == 0) steps[DB] = lead_s[w * DB + DB - 1];
+    }
   }
 }
 
 struct DeltaBlockScanArgs {
   float* out;              // [T, heads * V]
-  const float* qk;
-  const float* coef;
+  const unsigned char* qk;
+  const unsigned char* coef;
   const void* v; long long v_stride;
   float* state; long long slot_stride;     // slot s at state + s * slot_stride: [heads][V][D]
   const int* slots; const int* row_q_start; const int* row_q_len;
@@ -510,28 +601,46 @@ struct DeltaBlockScanArgs {
   int* status;
 };
 
-// A CTA owns a request, a head and DB_COLS value columns; its state lies in registers (two channels by four columns a
-// thread) and, for the read-outs, in shared memory.  A block: every warp forms the read-outs of all 32 rows (k and q)
-// over its share of the channels, 4 x 4 a thread; the warps' sums are added and v' made; u and o from the block's
-// matrices; the state.  The next block's operands are copied meanwhile.  Bound by the reads of shared memory beside the
-// multiply-adds and by the chain of a block, four barriers with eight warps between them (2048 tokens, 16 heads of 128 x 128: 240 us
-// with the matrices, 522 token by token).  Products on the tensor cores with operands of two TF32 values each took 30 us less,
-// at 1.5 to 1.9 times the token-by-token form's error against 64 bits; this form has 0.5 to 0.9 of it.
+// What the values v' that are not finite (or that bfloat16 parts do not hold), left out of the product, add to row `row` of Tu over M, token t.
+// (A call of its own, so that its registers cost the other blocks nothing.)
+__device__ __noinline__ float delta_wild(const __nv_bfloat16* coef, int row, int t, const float* values, int stride) {
+  float sum = 0.0f;
+  for (int j = 0; j <= t; ++j) {
+    const float x = values[j * stride];
+    if (fabsf(x) <= DB_LARGEST) continue;
+    float weight = 0.0f;
+    for (int e = 2; e >= 0; --e) weight += __bfloat162float(coef[(e * 2 * DB + row) * DB_MST + j]);
+    sum = fmaf(weight, x, sum);
+  }
+  return sum;
+}
+
+// A CTA owns a request, a head and DB_COLS value columns; its state lies in registers (a warp 16 channels) and, for the read-outs, in
+// shared memory in three parts.  A block: every warp forms the read-outs of all 64 rows (k and q) over its 16 channels;
+// the warps' sums are added and v' made; a warp a tile of u or o from the block's matrices; the state.  The next block comes meanwhile, in two
+// bulk copies.  Every product is one of float32 values in three bfloat16 parts each, all 24 bits, with sums of 16 or 32 products on the
+// tensor cores; sums across channels and blocks are float32 additions.
+// Bound by the 84 products a warp and block (of 3650 cycles a block the tensor cores take 2000, 12 a product and scheduler) between four
+// barriers; bringing operands to registers in front of the barriers made it slower (4100).  2048 tokens, 16 heads of 128 x 128: 30 us
+// for the matrices and 132 for the walk; in blocks of 16 with multiply-adds, bound by the reads of shared memory beside them, 31 and 210;
+// token by token 522.  Error against 64 bits 0.8 of the token-by-token form's, as before (4 heads of 128 x 128, 777 tokens: 1.6e-7 and 1.2e-7 of
+// the outputs and the state; blocks of 16 with multiply-adds 1.75e-7 and 1.35e-7, token by token 2.0e-7 and 1.9e-7).
 template <typename T, int DP>
-__global__ void __launch_bounds__(DB_THREADS, 2) delta_block_scan_kernel(const DeltaBlockScanArgs a) {
-  extern __shared__ __align__(16) float db_smem[];
-  constexpr int QK_ST = 2 * DB + 4, S_ST = DB_COLS + 4, RED_ST = 2 * DB + 4;
-  constexpr int stage_floats = DP * QK_ST + DB_COEF;
-  float* stages = db_smem;                                   // two of [DP][QK_ST] and the coefficients
-  float* s_s = stages + 2 * stage_floats;                    // [DP][S_ST]
-  float* red_s = s_s + DP * S_ST;                            // [warps][DB_COLS][RED_ST]
-  float* vp_s = red_s + DB_THREADS / 32 * DB_COLS * RED_ST;  // [DB_COLS][DB]: v'
-  float* u_s = vp_s + DB_COLS * DB;                          // [DB][S_ST]: what the write takes
-  float* o_s = u_s + DB * S_ST;                              // [DB][S_ST]
-  __shared__ int wild;                                       // the last block with a v' that is not finite
+__global__ void __launch_bounds__(DB_THREADS, 1) delta_block_scan_kernel(const DeltaBlockScanArgs a) {
+  using Shape = DeltaShape<DP>;
+  constexpr int ST = Shape::ST, CST = Shape::CST, FST = Shape::FST, WARPS = DP / 16;      // WARPS: that hold channels
+  extern __shared__ __align__(16) unsigned char db_smem[];
+  unsigned char* at = db_smem + 2 * Shape::STAGE_BYTES;
+  __nv_bfloat16* s_s = reinterpret_cast<__nv_bfloat16*>(at);                   // [part][DP][CST]
+  __nv_bfloat16* vp_s = reinterpret_cast<__nv_bfloat16*>(at += Shape::S_BYTES);        // [part][DB][CST]: v'
+  __nv_bfloat16* u_s = reinterpret_cast<__nv_bfloat16*>(at += Shape::V_BYTES);         // [part][DB][CST]: what the write takes
+  float* vf_s = reinterpret_cast<float*>(at += Shape::V_BYTES);                // [DB][FST]: v'
+  float* o_s = reinterpret_cast<float*>(at += Shape::F_BYTES);                 // [DB][FST]
+  float* red_s = reinterpret_cast<float*>(at += Shape::F_BYTES);               // [warps][2 DB][DB_COLS], every other pair of rows turned by 8 columns
+  __shared__ unsigned long long landed[2];
+  __shared__ int wild;                                       // the last block with a v' that is left out of the product
   const int row = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * DB_COLS;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) wild = -1;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int slot = a.slots[row];
   if (slot < 0 || slot >= a.num_slots) {
     if (tid == 0) report(a.status, STATUS_ROW_OUT_OF_RANGE, slot, row);
@@ -542,156 +651,192 @@ __global__ void __launch_bounds__(DB_THREADS, 2) delta_block_scan_kernel(const D
   const long long t0 = a.row_q_start[row];
   const int first = first_piece_of_row<DB>(a.row_q_len, row, a.from);
   const int group = head / (a.heads / a.qk_heads);
+  if (tid == 0) {
+    mbar_init(&landed[0], 1);
+    mbar_init(&landed[1], 1);
+    fence_barrier_init();
+    wild = -1;
+  }
+  __syncthreads();
 
-  auto copy_block = [&](int p, float* stage) {
-    const float* qk = a.qk + (static_cast<long long>(first + p) * a.qk_heads + group) * DP * 2 * DB;
-    for (int e = tid; e < DP * 2 * DB / 4; e += DB_THREADS) {
-      const int d = e / (2 * DB / 4), i = e % (2 * DB / 4) * 4;
-      cp_async_16(stage + d * QK_ST + i, qk + e * 4, true);
-    }
-    const float* coef = a.coef + (static_cast<long long>(first + p) * a.heads + head) * DB_COEF;
-    for (int e = tid; e < DB_COEF / 4; e += DB_THREADS) cp_async_16(stage + DP * QK_ST + e * 4, coef + e * 4, true);
-    cp_async_commit();
+  auto copy_block = [&](int p) {                             // one thread
+    unsigned char* stage = db_smem + (p & 1) * Shape::STAGE_BYTES;
+    mbar_arrive_expect_tx(&landed[p & 1], Shape::STAGE_BYTES);
+    bulk_copy_g2s(stage, a.qk + (static_cast<long long>(first + p) * a.qk_heads + group) * Shape::QK_BYTES, Shape::QK_BYTES, &landed[p & 1]);
+    bulk_copy_g2s(stage + Shape::QK_BYTES, a.coef + (static_cast<long long>(first + p) * a.heads + head) * DB_COEF_BYTES, DB_COEF_BYTES,
+                  &landed[p & 1]);
   };
-  // This thread's token and column in the small products.
-  const int my_t = tid % DB, my_c = tid / DB;
+  // This thread's token and pair of columns where v' is made.
+  const int my_t = tid / (DB_COLS / 2), my_c = tid % (DB_COLS / 2) * 2;
+  const bool live0 = col0 + my_c < a.V, live1 = col0 + my_c + 1 < a.V;
   const T* v = static_cast<const T*>(a.v) + t0 * a.v_stride + head * a.V + col0 + my_c;
   auto fetch_v = [&](int p) {
-    const int t = p * DB + my_t;
-    return t < n && col0 + my_c < a.V ? to_float(v[t * a.v_stride]) : 0.0f;
+    const int at_t = p * DB + my_t;
+    return make_float2(at_t < n && live0 ? to_float(v[at_t * a.v_stride]) : 0.0f, at_t < n && live1 ? to_float(v[at_t * a.v_stride + 1]) : 0.0f);
   };
-  // This thread's part of the state: channels d0 and d0 + 1, columns c0 .. c0 + 3.
-  const int d0 = tid / 4 * 2, c0 = tid % 4 * 4;
-  const bool holds = d0 < DP;
+  // This thread's part of the state: channels d0 and d0 + 8, columns 8 i + 2 t and the next.
+  const int d0 = warp * 16 + g;
+  const bool holds = warp < WARPS;
   float S[2][4];
   float* state = a.state + static_cast<long long>(slot) * a.slot_stride + (static_cast<long long>(head) * a.V + col0) * a.D;
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int c = 0; c < 4; ++c)
-      S[i][c] = holds && d0 + i < a.D && col0 + c0 + c < a.V ? state[static_cast<long long>(c0 + c) * a.D + d0 + i] : 0.0f;
+    for (int e = 0; e < 4; ++e) {
+      const int d = d0 + (e >> 1) * 8, c = 8 * i + 2 * t + (e & 1);
+      S[i][e] = holds && d < a.D && col0 + c < a.V ? state[static_cast<long long>(c) * a.D + d] : 0.0f;
+    }
   auto store_state = [&]() {
-    if (holds) {
+    if (!holds) return;
 #pragma unroll
-      for (int i = 0; i < 2; ++i) *reinterpret_cast<float4*>(s_s + (d0 + i) * S_ST + c0) = make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
-    }
-  };
-  store_state();
-  float v_now = 0.0f;
-  if (blocks > 0) {
-    copy_block(0, stages);
-    v_now = fetch_v(0);
-  }
-  for (int p = 0; p < blocks; ++p) {
-    const float* stage = stages + (p & 1) * stage_floats;
-    const float* coef = stage + DP * QK_ST;
-    cp_async_wait<0>();
-    __syncthreads();             // the block and the state are there; the other buffer is no longer read
-    float v_next = 0.0f;
-    if (p + 1 < blocks) {
-      copy_block(p + 1, stages + ((p + 1) & 1) * stage_floats);
-      v_next = fetch_v(p + 1);
-    }
-    {
-      const int i0 = (lane & 7) * 4, rc = (lane >> 3) * 4;
-      float acc[4][4];
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
+      for (int half = 0; half < 2; ++half) {
+        unsigned part[3];
+        three_parts(S[i][2 * half], S[i][2 * half + 1], part[0], part[1], part[2]);
 #pragma unroll
-      for (int u = 0; u < DP / 8; ++u) {
-        const int d = warp * (DP / 8) + u;
-        float x[4], y[4];
-        *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(stage + d * QK_ST + i0);
-        *reinterpret_cast<float4*>(y) = *reinterpret_cast<const float4*>(s_s + d * S_ST + rc);
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int c = 0; c < 4; ++c) acc[c][i] = fmaf(x[i], y[c], acc[c][i]);
+        for (int e = 0; e < 3; ++e) *reinterpret_cast<unsigned*>(s_s + (e * DP + d0 + 8 * half) * CST + 8 * i + 2 * t) = part[e];
       }
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-        *reinterpret_cast<float4*>(red_s + (warp * DB_COLS + rc + c) * RED_ST + i0) = make_float4(acc[c][0], acc[c][1], acc[c][2], acc[c][3]);
+  };
+  if (tid == 0 && blocks > 0) copy_block(0);
+  store_state();
+  float2 v_now = fetch_v(0);
+  // ldmatrix addresses: rows as they lie, keys transposed, value columns as [k][n].
+  const int lrow = (lane & 7) + ((lane >> 3) & 1) * 8, lcol = (lane >> 4) * 8;
+  const int a_off = lrow * ST + lcol, at_off = ((lane & 7) + (lane >> 4) * 8) * ST + ((lane >> 3) & 1) * 8, m_off = lrow * DB_MST + lcol;
+  const int b_off = lrow * CST + lcol;
+  constexpr int TILES = 2 * DB / 16, STEPS = DB / 16;
+  for (int p = 0; p < blocks; ++p) {
+    const unsigned char* stage = db_smem + (p & 1) * Shape::STAGE_BYTES;
+    const __nv_bfloat16* qk_s = reinterpret_cast<const __nv_bfloat16*>(stage);                      // [part][k, q][ST]
+    const __nv_bfloat16* coef_s = reinterpret_cast<const __nv_bfloat16*>(stage + Shape::QK_BYTES);  // [part][Tu, M][DB_MST]
+    const float* steps = reinterpret_cast<const float*>(stage + Shape::QK_BYTES + DB_COEF_PARTS);
+    const bool here = mbar_wait(&landed[p & 1], p >> 1 & 1, DB_WAIT_LIMIT);
+    // The block and the state are there; the other buffer is no longer read.
+    if (!__syncthreads_and(here)) {
+      if (tid == 0) report(a.status, STATUS_COPY_TIMEOUT, p, row);
+      let_copies_land();
+      return;
     }
-    __syncthreads();
-    float rk = 0.0f, rq = 0.0f;
+    if (tid == 0 && p + 1 < blocks) copy_block(p + 1);
+    const float2 v_next = fetch_v(p + 1);
+    if (holds) {
+      unsigned af[TILES][3][4], bf[TILES][3][4];
+      float high[TILES][2][4] = {}, low[TILES][2][4] = {};
 #pragma unroll
-    for (int w = 0; w < DB_THREADS / 32; ++w) {
-      rk += red_s[(w * DB_COLS + my_c) * RED_ST + my_t];
-      rq += red_s[(w * DB_COLS + my_c) * RED_ST + DB + my_t];
+      for (int e = 0; e < 3; ++e) {
+        ldmatrix_x4_trans(bf[0][e], s_s + (e * DP + warp * 16) * CST + b_off);
+#pragma unroll
+        for (int mt = 0; mt < TILES; ++mt) ldmatrix_x4(af[mt][e], qk_s + (e * 2 * DB + mt * 16) * ST + a_off + warp * 16);
+#pragma unroll
+        for (int mt = 1; mt < TILES; ++mt)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) bf[mt][e][i] = bf[0][e][i];
+      }
+      delta_products<TILES, 2>(high, low, af, bf);
+#pragma unroll
+      for (int mt = 0; mt < TILES; ++mt)
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            const int r = mt * 16 + g + 8 * half;
+            *reinterpret_cast<float2*>(red_s + (warp * 2 * DB + r) * DB_COLS + ((8 * i + 2 * t + (r >> 1 & 1) * 8) & 15)) =
+                make_float2(high[mt][i][2 * half] + low[mt][i][2 * half], high[mt][i][2 * half + 1] + low[mt][i][2 * half + 1]);
+          }
     }
-    const float lead = coef[2 * DB * DB + my_t], whole = coef[2 * DB * DB + DB];
-    const float vp = v_now - lead * rk;
-    vp_s[my_c * DB + my_t] = vp;
-    if (!isfinite(vp)) wild = p;
     __syncthreads();
     {
-      float u = 0.0f, o = 0.0f;
-      if (wild != p) {
+      float2 rk = make_float2(0.0f, 0.0f), rq = rk;
+      const float* from = red_s + my_t * DB_COLS + ((my_c + (my_t >> 1 & 1) * 8) & 15);
 #pragma unroll
-        for (int j = 0; j < DB; j += 4) {
-          float x[4];
-          *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(vp_s + my_c * DB + j);
+      for (int w = 0; w < WARPS; ++w) {
+        const float2 x = *reinterpret_cast<const float2*>(from + w * 2 * DB * DB_COLS);
+        const float2 y = *reinterpret_cast<const float2*>(from + (w * 2 * DB + DB) * DB_COLS);
+        rk.x += x.x; rk.y += x.y; rq.x += y.x; rq.y += y.y;
+      }
+      const float lead = steps[my_t];
+      float x = v_now.x - lead * rk.x, y = v_now.y - lead * rk.y;
+      *reinterpret_cast<float2*>(vf_s + my_t * FST + my_c) = make_float2(x, y);
+      *reinterpret_cast<float2*>(o_s + my_t * FST + my_c) = make_float2(lead * rq.x, lead * rq.y);
+      if (!(fabsf(x) <= DB_LARGEST)) { x = 0.0f; wild = p; }
+      if (!(fabsf(y) <= DB_LARGEST)) { y = 0.0f; wild = p; }
+      unsigned part[3];
+      three_parts(x, y, part[0], part[1], part[2]);
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            u = fmaf(coef[(j + i) * DB + my_t], x[i], u);
-            o = fmaf(coef[DB * DB + (j + i) * DB + my_t], x[i], o);
+      for (int e = 0; e < 3; ++e) *reinterpret_cast<unsigned*>(vp_s + (e * DB + my_t) * CST + my_c) = part[e];
+    }
+    __syncthreads();
+    {
+      // Rows 16 mt .. + 15 of Tu over M, columns 8 nt .. + 7.  (What lies above the diagonal is zeros.)
+      const int mt = warp >> 1, nt = warp & 1;
+      unsigned af[STEPS][3][4], bf[STEPS][3][2];
+      float high[STEPS][1][4] = {}, low[STEPS][1][4] = {};
+      const int b_tile = (lane & 7) + ((lane >> 3) & 1) * 8;      // (the other lanes' addresses are not used)
+#pragma unroll
+      for (int ks = 0; ks < STEPS; ++ks)
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+          ldmatrix_x4(af[ks][e], coef_s + (e * 2 * DB + mt * 16) * DB_MST + m_off + ks * 16);
+          ldmatrix_x2_trans(bf[ks][e], vp_s + (e * DB + ks * 16 + b_tile) * CST + nt * 8);
+        }
+      delta_products<STEPS, 1>(high, low, af, bf);
+      const bool tame = wild != p;
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int r = mt * 16 + g + 8 * half, tok = r % DB, c = 8 * nt + 2 * t;
+        float x = (high[0][0][2 * half] + high[1][0][2 * half]) + (low[0][0][2 * half] + low[1][0][2 * half]);
+        float y = (high[0][0][2 * half + 1] + high[1][0][2 * half + 1]) + (low[0][0][2 * half + 1] + low[1][0][2 * half + 1]);
+        if (!tame) {
+          x += delta_wild(coef_s, r, tok, vf_s + c, FST);
+          y += delta_wild(coef_s, r, tok, vf_s + c + 1, FST);
+        }
+        if (r < DB) {
+          unsigned part[3];
+          three_parts(x, y, part[0], part[1], part[2]);
+#pragma unroll
+          for (int e = 0; e < 3; ++e) *reinterpret_cast<unsigned*>(u_s + (e * DB + tok) * CST + c) = part[e];
+        } else if (p * DB + tok < n) {
+          float* to = a.out + (t0 + p * DB + tok) * a.heads * a.V + static_cast<long long>(head) * a.V + col0 + c;
+          const float2 o = *reinterpret_cast<const float2*>(o_s + tok * FST + c);
+          if (a.V % 2 == 0 && col0 + c < a.V) {
+            *reinterpret_cast<float2*>(to) = make_float2(x + o.x, y + o.y);
+          } else {
+            if (col0 + c < a.V) to[0] = x + o.x;
+            if (col0 + c + 1 < a.V) to[1] = y + o.y;
           }
         }
-      } else {
-        // The same sums, without a zero times a later token's value.
-        for (int j = 0; j <= my_t; ++j) {
-          u = fmaf(coef[j * DB + my_t], vp_s[my_c * DB + j], u);
-          o = fmaf(coef[(DB + j) * DB + my_t], vp_s[my_c * DB + j], o);
-        }
       }
-      u_s[my_t * S_ST + my_c] = u;
-      o_s[my_t * S_ST + my_c] = fmaf(lead, rq, o);
     }
     __syncthreads();
-    {
-      const int t = p * DB + tid / DB_COLS, c = tid % DB_COLS;
-      if (t < n && col0 + c < a.V)
-        a.out[(t0 + t) * a.heads * a.V + static_cast<long long>(head) * a.V + col0 + c] = o_s[tid / DB_COLS * S_ST + c];
-    }
     if (holds) {
+      unsigned af[STEPS][3][4], bf[STEPS][3][4];
+      float high[STEPS][2][4] = {}, low[STEPS][2][4] = {};
+#pragma unroll
+      for (int ks = 0; ks < STEPS; ++ks)
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+          ldmatrix_x4_trans(af[ks][e], qk_s + (e * 2 * DB + ks * 16) * ST + at_off + warp * 16);
+          ldmatrix_x4_trans(bf[ks][e], u_s + (e * DB + ks * 16) * CST + b_off);
+        }
+      delta_products<STEPS, 2>(high, low, af, bf);
+      const float whole = steps[DB];
 #pragma unroll
       for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) S[i][c] *= whole;
-#pragma unroll
-      for (int j = 0; j < DB; j += 4) {
-        float k0[4], k1[4];
-        *reinterpret_cast<float4*>(k0) = *reinterpret_cast<const float4*>(stage + d0 * QK_ST + j);
-        *reinterpret_cast<float4*>(k1) = *reinterpret_cast<const float4*>(stage + (d0 + 1) * QK_ST + j);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          float u[4];
-          *reinterpret_cast<float4*>(u) = *reinterpret_cast<const float4*>(u_s + (j + i) * S_ST + c0);
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            S[0][c] = fmaf(k0[i], u[c], S[0][c]);
-            S[1][c] = fmaf(k1[i], u[c], S[1][c]);
-          }
-        }
-      }
+        for (int e = 0; e < 4; ++e) S[i][e] = fmaf(whole, S[i][e], (high[0][i][e] + high[1][i][e]) + (low[0][i][e] + low[1][i][e]));
     }
-    store_state();               // (nobody reads the state's tile between the barriers above and the next one)
+    store_state();               // (nobody reads the state's tile between the first barrier above and the next one)
     v_now = v_next;
   }
   if (!a.write_state || !holds) return;
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int c = 0; c < 4; ++c)
-      if (d0 + i < a.D && col0 + c0 + c < a.V) state[static_cast<long long>(c0 + c) * a.D + d0 + i] = S[i][c];
-}
-
-template <int DP>
-constexpr size_t delta_blocks_smem() { return sizeof(float) * (2 * DB * (DP + 4) + 5 * DB * DB + 5 * DB); }
-template <int DP>
-constexpr size_t delta_block_scan_smem() {
-  return sizeof(float) * (2 * (DP * (2 * DB + 4) + DB_COEF) + DP * (DB_COLS + 4) + DB_THREADS / 32 * DB_COLS * (2 * DB + 4) +
-                          DB_COLS * DB + 2 * DB * (DB_COLS + 4));
+    for (int e = 0; e < 4; ++e) {
+      const int d = d0 + (e >> 1) * 8, c = 8 * i + 2 * t + (e & 1);
+      if (d < a.D && col0 + c < a.V) state[static_cast<long long>(c) * a.D + d] = S[i][e];
+    }
 }
 
 }  // namespace zb
@@ -779,17 +924,22 @@ ZB_API int zb_delta_scan(float* out, const float* q, const float* k, const void*
 ZB_API int zb_delta_block_max_channels() { return 128; }
 ZB_API int zb_delta_block_tokens() { return DB; }
 // Floats of workspace a block needs: its unit vectors and its matrices.
-ZB_API int zb_delta_block_floats(int qk_heads, int heads, int D) { return qk_heads * (D <= 64 ? 64 : 128) * 2 * DB + heads * DB_COEF; }
+ZB_API int zb_delta_block_floats(int qk_heads, int heads, int D) {
+  return (qk_heads * (D <= 64 ? DeltaShape<64>::QK_BYTES : DeltaShape<128>::QK_BYTES) + heads * DB_COEF_BYTES) / 4;
+}
 
 template <typename T, int DP>
-static int delta_block_launch(const DeltaBlocksArgs& b, const DeltaBlockScanArgs& a, int rows, int blocks, cudaStream_t s) {
-  constexpr int first = static_cast<int>(delta_blocks_smem<DP>()), second = static_cast<int>(delta_block_scan_smem<DP>());
-  if (cuda_failed(cudaFuncSetAttribute(delta_block_scan_kernel<T, DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, second)))
+static int delta_block_launch(DeltaBlocksArgs b, DeltaBlockScanArgs a, float* ws, int rows, int blocks, cudaStream_t s) {
+  using Shape = DeltaShape<DP>;
+  b.qk = reinterpret_cast<unsigned char*>(ws);
+  b.coef = b.qk + static_cast<long long>(blocks) * b.qk_heads * Shape::QK_BYTES;
+  a.qk = b.qk; a.coef = b.coef;
+  if (cuda_failed(cudaFuncSetAttribute(delta_blocks_kernel<T, DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::BLOCKS_SMEM)) ||
+      cuda_failed(cudaFuncSetAttribute(delta_block_scan_kernel<T, DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::SCAN_SMEM)))
     return ERR_CUDA;
-  launch_dependent(delta_blocks_kernel<T, DP>, dim3(blocks, b.qk_heads), dim3(DB_THREADS), first, s, false, b);
-  // (Not as a dependent: its CTAs would take the SMs that the kernel before it leaves first, two a SM, while others stay empty:
-  // the layer over 2048 tokens, 16 heads 347 -> 500 us.)
-  delta_block_scan_kernel<T, DP><<<dim3(rows, a.heads, (a.V + DB_COLS - 1) / DB_COLS), DB_THREADS, second, s>>>(a);
+  launch_dependent(delta_blocks_kernel<T, DP>, dim3(blocks, b.qk_heads), dim3(DB_THREADS), Shape::BLOCKS_SMEM, s, false, b);
+  // (Not as a dependent: its CTAs would take the SMs that the kernel before it leaves first, while others stay empty.)
+  delta_block_scan_kernel<T, DP><<<dim3(rows, a.heads, (a.V + DB_COLS - 1) / DB_COLS), DB_THREADS, Shape::SCAN_SMEM, s>>>(a);
   return launch_result();
 }
 
@@ -805,17 +955,19 @@ ZB_API int zb_delta_block_scan(float* out, const void* q, long long q_stride, co
   if (D > zb_delta_block_max_channels() || heads > 65535 || (V + DB_COLS - 1) / DB_COLS > 65535) return ERR_UNSUPPORTED;
   if (rows == 0 || tokens == 0) return OK;
   if (ws == nullptr || reinterpret_cast<uintptr_t>(ws) % 16 != 0) return ERR_BAD_ARGUMENT;
-  const int blocks = tokens / DB + rows, dp = D <= 64 ? 64 : 128;
+  const int blocks = tokens / DB + rows;
   DeltaBlocksArgs g;
-  g.qk = ws; g.coef = ws + static_cast<long long>(blocks) * qk_heads * dp * 2 * DB; g.q = q; g.q_stride = q_stride; g.k = k;
+  g.q = q; g.q_stride = q_stride; g.k = k;
   g.k_stride = k_stride; g.b = b; g.a = a; g.ba_stride = ba_stride; g.a_log = a_log; g.dt_bias = dt_bias;
   g.row_q_start = row_q_start; g.row_q_len = row_q_len; g.rows = rows; g.from = from; g.qk_heads = qk_heads; g.heads = heads; g.D = D;
   g.q_scale = q_scale; g.unit_eps = unit_eps;
   DeltaBlockScanArgs c;
-  c.out = out; c.qk = g.qk; c.coef = g.coef; c.v = v; c.v_stride = v_stride; c.state = state; c.slot_stride = slot_stride;
+  c.out = out; c.v = v; c.v_stride = v_stride; c.state = state; c.slot_stride = slot_stride;
   c.slots = slots; c.row_q_start = row_q_start; c.row_q_len = row_q_len; c.heads = heads; c.qk_heads = qk_heads; c.D = D; c.V = V;
   c.num_slots = num_slots; c.write_state = write_state; c.from = from; c.status = status;
   auto s = static_cast<cudaStream_t>(stream);
-  if (dtype == DTYPE_F32) return dp == 64 ? delta_block_launch<float, 64>(g, c, rows, blocks, s) : delta_block_launch<float, 128>(g, c, rows, blocks, s);
-  return dp == 64 ? delta_block_launch<__nv_bfloat16, 64>(g, c, rows, blocks, s) : delta_block_launch<__nv_bfloat16, 128>(g, c, rows, blocks, s);
+  if (dtype == DTYPE_F32)
+    return D <= 64 ? delta_block_launch<float, 64>(g, c, ws, rows, blocks, s) : delta_block_launch<float, 128>(g, c, ws, rows, blocks, s);
+  return D <= 64 ? delta_block_launch<__nv_bfloat16, 64>(g, c, ws, rows, blocks, s)
+                 : delta_block_launch<__nv_bfloat16, 128>(g, c, ws, rows, blocks, s);
 }

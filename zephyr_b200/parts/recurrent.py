@@ -211,13 +211,12 @@ class GatedDeltaRule(Mixer):
 
     UNIT_EPS = 1e-6      # inside the root of the unit norms of q and k: the design fixes it
     # New tokens of a row from which on it runs in blocks.  Blocks shorten a row's chain and pay where rows are few: 16 heads of
-    # 128 x 128, one row of 64 tokens: 19 us, 24 token by token; 2048: 239 and 520; 3 rows of 600: 199 and 244; 32 heads, one
-    # row of 2048: 420 and 559.  Where the rows' own chains fill the SMs they are behind (16 heads, 8 rows of 256: 201 and 185;
-    # 32 heads, 3 rows of 600: 375 and 326).  So in bfloat16 a step runs in blocks while their CTAs, 16 value columns each, are
-    # no more than one and a half times what the SMs hold at once, and rows of 64 to 191 tokens beside shorter ones, which
-    # take a launch of their own, stay with those (40, 3 and 90 tokens: 75 us, 87 in two launches).  In 32 bits the line looks at the row alone, so that a
-    # request's logits do not change with what shares its step; it lies where a few rows gain and many lose little (8 rows of
-    # 128: 105 and 98).
+    # 128 x 128, one row of 64 tokens: 19 us, 24 token by token; 2048: 167 and 520; 3 rows of 600: 155 and 244; 32 heads, one
+    # row of 500: 86 and 138.  Where the rows' own chains fill the SMs and rows are short they are behind (16 heads, 8 rows of 100: 87
+    # and 80, 16 rows of 64: 107 and 90, 16 of 128: 186 and 168; but 8 of 128 89 and 99).  So in bfloat16 a step runs in blocks while their
+    # CTAs, 16 value columns each, are no more than three an SM, and rows of 64 to 191 tokens beside shorter ones, which
+    # take a launch of their own, stay with those (40, 3 and 90 tokens: 58 us, 45).  In 32 bits the line looks at the row alone, so that a
+    # request's logits do not change with what shares its step; it lies where a few rows gain and many lose little.
     BLOCKS_FROM, ROW_BLOCKS_FROM, MOST_CTAS = 64, 128, 3 * 148
 
     def __init__(self, spec: MixerSpec, weights: Mapping[str, torch.Tensor], dtype: torch.dtype,
