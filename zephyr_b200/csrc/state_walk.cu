@@ -370,7 +370,7 @@ __device__ __noinline__ void drop_wild(__nv_bfloat16* v_s, int count) {
 //   barrier; the other half adds it and writes; the state and the next piece's values go to shared memory in parts.
 // The next piece comes meanwhile, in two bulk copies.
 template <int MODE, int DP, int NT>
-__global__ void __launch_bounds__(W_THREADS, 2) state_walk_kernel(const WalkArgs a) {
+__global__ void __launch_bounds__(W_THREADS, 1) state_walk_kernel(const WalkArgs a) {
   using Shape = WalkShape<MODE, DP, NT>;
   constexpr bool SPLIT_SUMS = MODE == WALK_SPACE;
   constexpr int PA = Shape::PA, PB = Shape::PB, ST = Shape::ST, COLS = Shape::COLS, CST = Shape::CST, OST = Shape::OST;
@@ -497,7 +497,8 @@ __global__ void __launch_bounds__(W_THREADS, 2) state_walk_kernel(const WalkArgs
   const int lrow = (lane & 7) + ((lane >> 3) & 1) * 8, lcol = (lane >> 4) * 8;
   const int a_off = lrow * ST + lcol, p_off = lrow * W_PST + lcol, b_off = lrow * CST + lcol;
   const int at_off = ((lane & 7) + (lane >> 4) * 8) * ST + ((lane >> 3) & 1) * 8;
-  const int row0 = (warp & 3) * 16, half = warp >> 2;
+  constexpr int MINE = NT / 2;                               // tiles of value columns whose outputs a warp writes
+  const int row0 = (warp & 3) * 16, half = warp >> 2, first_c = half * MINE * 8;
   for (int p = 0; p < pieces; ++p) {
     const unsigned char* stage = w_smem + p % STAGES * Shape::stage_bytes;
     const __nv_bfloat16* q_s = reinterpret_cast<const __nv_bfloat16*>(stage);              // [PA][W][ST]
@@ -512,7 +513,7 @@ __global__ void __launch_bounds__(W_THREADS, 2) state_walk_kernel(const WalkArgs
       let_copies_land();
       return;
     }
-    if (tid == 0 && p + 1 < pieces) copy_piece(p + 1);
+    if (tid == W_THREADS - 32 && p + 1 < pieces) copy_piece(p + 1);
     fetch_values(p + 1);
     const int i0 = row0 + g, i1 = i0 + 8;
     const bool tame = wild != p;
@@ -560,13 +561,14 @@ __global__ void __launch_bounds__(W_THREADS, 2) state_walk_kernel(const WalkArgs
 #pragma unroll
           for (int e = 0; e < 4; ++e) o[i][e] += low[i][e];
       }
-      if (half == 1) {
+      // The other half of the tokens' warps gets what this one has of the tiles that it writes out.
+      {
 #pragma unroll
-        for (int i = 0; i < NT; ++i)
+        for (int i = 0; i < MINE; ++i)
 #pragma unroll
           for (int r = 0; r < 2; ++r) {
-            const int tok = i0 + 8 * r, c = 8 * i + 2 * t;
-            float2 y = make_float2(o[i][2 * r], o[i][2 * r + 1]);
+            const int tok = i0 + 8 * r, c = 8 * (half == 0 ? MINE + i : i) + 2 * t;
+            float2 y = half == 0 ? make_float2(o[MINE + i][2 * r], o[MINE + i][2 * r + 1]) : make_float2(o[i][2 * r], o[i][2 * r + 1]);
             if (MODE == WALK_SPACE) {
               const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(v_s + tok * CST + c));
               y.x = fmaf(skip, v.x, y.x);
@@ -596,28 +598,30 @@ __global__ void __launch_bounds__(W_THREADS, 2) state_walk_kernel(const WalkArgs
     __syncthreads();               // the state's, the values' and the piece's reads are done
     store_state();
     store_values(p + 1);
-    if (half == 0 && row0 < n) {
+    if (row0 < n) {
 #pragma unroll
-      for (int i = 0; i < NT; ++i)
+      for (int i = 0; i < MINE; ++i)
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-          const int tok = i0 + 8 * r, c = 8 * i + 2 * t;
+          const int tok = i0 + 8 * r, c = first_c + 8 * i + 2 * t;
           if (tok >= n) continue;
           float* to = a.out + (t0 + p * W + tok) * a.H * a.V + static_cast<long long>(h) * a.V + v0 + c;
           const float2 y = *reinterpret_cast<const float2*>(o_s + tok * OST + c);
+          const float2 x = half == 0 ? make_float2(o[i][2 * r], o[i][2 * r + 1]) : make_float2(o[MINE + i][2 * r], o[MINE + i][2 * r + 1]);
           if (a.V % 2 == 0 && v0 + c < a.V) {
-            *reinterpret_cast<float2*>(to) = make_float2(o[i][2 * r] + y.x, o[i][2 * r + 1] + y.y);
+            *reinterpret_cast<float2*>(to) = make_float2(x.x + y.x, x.y + y.y);
           } else {
-            if (v0 + c < a.V) to[0] = o[i][2 * r] + y.x;
-            if (v0 + c + 1 < a.V) to[1] = o[i][2 * r + 1] + y.y;
+            if (v0 + c < a.V) to[0] = x.x + y.x;
+            if (v0 + c + 1 < a.V) to[1] = x.y + y.y;
           }
         }
       // (the outputs that this thread has just written; the piece's buffer is filled again behind the next barrier)
       if (!tame) {
         using T = typename Shape::Value;
         const long long at = t0 + p * W;
-        add_wild<T, PB>(a.out + at * a.H * a.V + static_cast<long long>(h) * a.V + v0, static_cast<long long>(a.H) * a.V,
-                        static_cast<const T*>(a.v) + at * a.v_stride + h * a.V + v0, a.v_stride, n, a.V - v0, NT, i0, 2 * t, skip, p_s);
+        add_wild<T, PB>(a.out + at * a.H * a.V + static_cast<long long>(h) * a.V + v0 + first_c, static_cast<long long>(a.H) * a.V,
+                        static_cast<const T*>(a.v) + at * a.v_stride + h * a.V + v0 + first_c, a.v_stride, n, a.V - v0 - first_c, MINE, i0, 2 * t,
+                        skip, p_s);
       }
     }
   }
