@@ -125,6 +125,12 @@ _SIGNATURES = {
     "zb_delta_scan": [c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_longlong,
                       c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                       c_int, c_void_p, c_void_p],
+    "zb_retention_tc_supported": [c_int, c_int, c_int],
+    "zb_retention_tc_piece_tokens": [],
+    "zb_retention_tc_piece_floats": [c_int],
+    "zb_retention_tc": [c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_longlong,
+                        c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_float,
+                        c_void_p, c_void_p, c_void_p, c_void_p],
     "zb_delta_block_max_channels": [],
     "zb_delta_block_tokens": [],
     "zb_delta_block_floats": [c_int, c_int, c_int],
@@ -867,6 +873,16 @@ def retention_turns(q: torch.Tensor, k: torch.Tensor, key_dim: int, rot_dims: in
             and all(t.stride(0) % 4 == 0 and t.data_ptr() % 16 == 0 for t in (q, k)))
 
 
+def _retention_in_tensor_memory(q, k, v, state, rows: int, tokens: int, heads: int, key_dim: int, value_dim: int, rot_dims: int) -> bool:
+    """True where retention's walk runs in pieces of 128 tokens on tcgen05 (csrc/retention_tc.cu): heads of 65 to 128 key channels, rows on
+    16-byte boundaries, unless a few heads' long rows leave the SMs to the walk in pieces of 64, whose chain of a row is the shorter one.
+    (us, here / there, heads of 128 x 128: 32 heads, rows of 1500 and 548 tokens 100 / 163, one of 256 24 / 33, of 64 17 / 27; 16
+    heads, one row of 2048 87 / 87, eight of 128 36 / 51, of 64 34 / 37; 8 heads, one row of 2048 81 / 70, of 700 37 / 33.)"""
+    return (bool(library().zb_retention_tc_supported(key_dim, value_dim, rot_dims))
+            and not (rows * heads * -(-value_dim // 16) <= _sm_count() // 2 and tokens >= 600 * rows)
+            and all(t.stride(0) % 4 == 0 and t.data_ptr() % 16 == 0 for t in (q, k, v, state)))
+
+
 def retention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, heads: int, key_dim: int, value_dim: int,
               state: torch.Tensor, slots: torch.Tensor, row_q_start: torch.Tensor, row_q_len: torch.Tensor,
               status: torch.Tensor, write_state: bool = True, freqs: torch.Tensor | None = None, rot_dims: int = 0,
@@ -875,7 +891,7 @@ def retention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Te
     bring runs of tokens.  With ``freqs`` q and k are first turned by the tokens' ``positions`` as ``rotate_qk`` does, k times
     ``k_scale`` (``retention_turns``: whether that is taken).  q, k, v float32 [T, .] with unit inner stride, head h at column h * width; ``decay`` float32
     [heads]; ``state`` [slots, heads * key_dim * value_dim] float32 (rows may be strided).  Each operand of a product
-    is taken as two bfloat16 values.  ``walk``: pieces one behind the other with the state on the SM (up to 128 key
+    is taken as two bfloat16 values.  ``walk``: pieces (of 64 tokens, or 128 on tcgen05) one behind the other with the state on the SM (up to 128 key
     channels; rows may then lie in the stream in any order); otherwise passes over all pieces at once (rows one behind the other,
     ``row_q_start`` ascending).  Returns o as float32 [T, heads * value_dim]."""
     _cuda(q, k, v, decay, state, slots, row_q_start, row_q_len, status)
@@ -898,6 +914,14 @@ def retention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Te
         _require(retention_turns(q, k, key_dim, rot_dims), "q and k of this shape are turned by rotate_qk")
         turn = (freqs, rot_dims, k_scale, positions)
     _require(walk or turn is None, "q and k are turned on the way into the walk")
+    if walk and _retention_in_tensor_memory(q, k, v, state, rows, T, heads, key_dim, value_dim, rot_dims if turn else 0):
+        ws = torch.empty(((T // lib.zb_retention_tc_piece_tokens() + rows) * lib.zb_retention_tc_piece_floats(heads),), dtype=torch.float32,
+                         device=v.device)
+        _check(lib.zb_retention_tc(
+            _ptr(out), _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(decay), _ptr(state), state.stride(0),
+            _ptr(slots), _ptr(row_q_start), _ptr(row_q_len), rows, T, heads, key_dim, value_dim, state.shape[0], int(write_state),
+            _ptr(freqs), int(rot_dims), float(k_scale), _ptr(positions), _ptr(ws), _ptr(status), _stream()), "retention_tc", kernels=2)
+        return out
     if walk and key_dim <= lib.zb_walk_max_channels():
         _state_walk(1, out, q, k, v, heads, key_dim, value_dim, state, slots, row_q_start, row_q_len, status, write_state, decay=decay,
                     turn=turn)
