@@ -14,11 +14,9 @@
 //   state_walk     a CTA owns a request, a head and some value columns and walks the pieces with the state in registers
 //
 // so the state never leaves the SM, where passes over all pieces at once write and read every piece's state (2048
-// tokens, 32 heads of 128 x 64: 33 MB four times), and a piece is two barriers.  Measured: the state-space form, 2048 and 77 tokens,
-// 32 heads of 128 x 64: 19 + 68 us, 290 as a scan in segments; retention, 1500 and 548 tokens, 32 heads of 128 x 128, rotation
-// included: 44 + 122 us, 203 in three passes and a rotation.  Bound by latency with the eight warps an SM that a CTA's shared
-// memory leaves: products' results, reads of shared memory (busy for 57 to 60 % of the time) and two barriers a piece, 1.7 waves
-// of CTAs; L2 is at 14 and 18 %.
+// tokens, 32 heads of 128 x 64: 33 MB four times), and a piece is one or two barriers.  Measured: the state-space form, 2048 and 77 tokens,
+// 32 heads of 128 x 64: 19 + 61 us, 290 as a scan in segments.  Retention's heads of more than 64 channels take pieces of 128 tokens on
+// tcgen05 (retention_tc.cu) but for a few heads' long rows (8 heads of 128 x 128, one row of 2048 tokens 62 us).
 //
 // Products run on the tensor cores, float32 sums.  A bfloat16 operand is exact; beside it a float32 operand is the sum of three
 // bfloat16 values (all its 24 bits).  The tensor cores cut a sum at every step, so there the products of the small parts have
@@ -42,7 +40,7 @@
 namespace zb {
 
 constexpr int W = 64;                    // tokens of a piece
-constexpr int W_THREADS = 256;
+constexpr int W_THREADS = 256;           // of a role: eight warps
 constexpr int W_PST = W + 8;             // a row of P
 constexpr int W_STEP = 2 * W + 4;        // a head of a piece: e^(c), w, e^(c_n)
 constexpr int W_WAIT_LIMIT = 1 << 20;
@@ -330,13 +328,15 @@ __global__ void __launch_bounds__(W_THREADS) walk_prepare_kernel(const WalkArgs 
   }
 }
 
-template <int MODE, int DP, int NT>
+template <int MODE, int DP, bool ROLES>
 struct WalkShape : WalkParts<MODE, DP> {
   using Parts = WalkParts<MODE, DP>;
+  static constexpr int NT = ROLES ? 2 : 4; // tiles of 8 value columns of a CTA
+  static constexpr int BUFFERS = ROLES ? 2 : 1, THREADS = ROLES ? 2 * W_THREADS : W_THREADS;
   static constexpr int COLS = 8 * NT, CST = COLS + 8, OST = COLS + 4, STAGES = 2;
   static constexpr int stage_bytes = Parts::qk_bytes + Parts::head_bytes;
-  static constexpr int smem =
-      STAGES * stage_bytes + Parts::PB * DP * CST * 2 + (Parts::PA + Parts::PB) * W * CST * 2 + W * OST * 4;
+  static constexpr int state_elems = Parts::PB * DP * CST, value_elems = (Parts::PA + Parts::PB) * W * CST;       // of a buffer each
+  static constexpr int smem = STAGES * stage_bytes + BUFFERS * (state_elems + value_elems) * 2 + W * OST * 4;
 };
 
 // The values of a piece that are not finite, added to the outputs of tokens i0 and i0 + 8, columns c0 and c0 + 1 of each of `tiles`
@@ -364,40 +364,44 @@ __device__ __noinline__ void drop_wild(__nv_bfloat16* v_s, int count) {
     if (!isfinite(__bfloat162float(v_s[e]))) v_s[e] = __float2bfloat16_rn(0.0f);
 }
 
-// NT: tiles of 8 value columns of a CTA.  Warp w owns the state's channels 16 w .. (C fragments); for the outputs it owns
-// tokens 16 (w % 4) .. and takes half the channels (S^T q) and every other 16 keys (P).  A piece:
-//   barrier; both terms of the outputs and the state's sums from shared memory; one half of the outputs' sums to shared memory;
-//   barrier; the other half adds it and writes; the state and the next piece's values go to shared memory in parts.
-// The next piece comes meanwhile, in two bulk copies.
-template <int MODE, int DP, int NT>
-__global__ void __launch_bounds__(W_THREADS, 1) state_walk_kernel(const WalkArgs a) {
-  using Shape = WalkShape<MODE, DP, NT>;
+// For the outputs, warp w owns tokens 16 (w % 4) .. and takes half the channels (S^T q) and every other 16 keys (P); the halves meet in
+// shared memory, each writing out half of the columns.  Of the state, warp w owns the channels 16 w .. (C fragments).  The next
+// piece comes meanwhile, in two bulk copies.  Two forms:
+//   * ROLES: sixteen warps and 16 value columns; eight warps make the outputs, eight carry the state on, and a piece is one barrier of all
+//     of them, behind which both work from the state's and the values' parts in one of two buffers while the state's warps
+//     fill the other: 2900 cycles a piece of the state-space form, where eight warps that did both one after the other took 3150;
+//   * else eight warps and 32 value columns: outputs and state one after the other, a barrier, the next piece's parts.
+// Bound by shared memory, ROLES at four fifths of it: 40 ldmatrix a warp of 16 columns, the parts' stores and the copies of 63 KB a piece.
+template <int MODE, int DP, bool ROLES>
+__global__ void __launch_bounds__(ROLES ? 2 * W_THREADS : W_THREADS, 1) state_walk_kernel(const WalkArgs a) {
+  using Shape = WalkShape<MODE, DP, ROLES>;
+  constexpr int NT = Shape::NT;
   constexpr bool SPLIT_SUMS = MODE == WALK_SPACE;
   constexpr int PA = Shape::PA, PB = Shape::PB, ST = Shape::ST, COLS = Shape::COLS, CST = Shape::CST, OST = Shape::OST;
   constexpr int STAGES = Shape::STAGES, PER = W * COLS / W_THREADS / 2;      // pairs of values a thread brings of a piece
   extern __shared__ __align__(16) unsigned char w_smem[];
-  __nv_bfloat16* s_s = reinterpret_cast<__nv_bfloat16*>(w_smem + STAGES * Shape::stage_bytes);    // [PB][DP][CST]
-  __nv_bfloat16* v_s = s_s + PB * DP * CST;                  // [PA][W][CST]
-  __nv_bfloat16* wv_s = v_s + PA * W * CST;                  // [PB][W][CST]: w_j v_j
-  float* o_s = reinterpret_cast<float*>(wv_s + PB * W * CST);            // [W][OST]
+  __nv_bfloat16* const state_s = reinterpret_cast<__nv_bfloat16*>(w_smem + STAGES * Shape::stage_bytes);     // [buffers][PB][DP][CST]
+  __nv_bfloat16* const values_s = state_s + Shape::BUFFERS * Shape::state_elems;      // [buffers]{v [PA][W][CST], w_j v_j [PB][W][CST]}
+  float* o_s = reinterpret_cast<float*>(values_s + Shape::BUFFERS * Shape::value_elems);        // [W][OST]
   __shared__ unsigned long long landed[STAGES];
-  __shared__ int wild;                                       // the last piece with a value that is not finite
+  __shared__ int wild[2];                                    // the last even and odd piece with a value that is not finite
   const int row = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * COLS;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const bool states = !ROLES || threadIdx.x >= W_THREADS;    // the warp's role
+  const int tid = threadIdx.x % W_THREADS, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;      // within it
   const int slot = a.slots[row];
   if (slot < 0 || slot >= a.num_slots) {
-    if (tid == 0) report(a.status, STATUS_ROW_OUT_OF_RANGE, slot, row);
+    if (threadIdx.x == 0) report(a.status, STATUS_ROW_OUT_OF_RANGE, slot, row);
     return;
   }
   const int n_all = a.row_q_len[row], pieces = (n_all + W - 1) / W;
   if (n_all < a.from) return;
   const long long t0 = a.row_q_start[row];
   const int first = first_piece_of_row<W>(a.row_q_len, row, a.from), qk_head = h / a.heads_per_group, qk_heads = a.H / a.heads_per_group;
-  if (tid == 0) {
+  if (threadIdx.x == 0) {
 #pragma unroll
     for (int i = 0; i < STAGES; ++i) mbar_init(&landed[i], 1);
     fence_barrier_init();
-    wild = -1;
+    wild[0] = wild[1] = -1;
   }
   __syncthreads();
 
@@ -443,6 +447,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) state_walk_kernel(const WalkArgs
     }
   };
   auto store_values = [&](int p) {
+    __nv_bfloat16* const v_s = values_s + p % Shape::BUFFERS * Shape::value_elems, * const wv_s = v_s + PA * W * CST;
     float top = 0.0f;                                        // NaN if one of the values is not finite
 #pragma unroll
     for (int u = 0; u < PER; ++u) {
@@ -462,11 +467,11 @@ __global__ void __launch_bounds__(W_THREADS, 1) state_walk_kernel(const WalkArgs
 #pragma unroll
       for (int i = 0; i < PB; ++i) *reinterpret_cast<unsigned*>(wv_s + i * W * CST + at) = wp[i];
     }
-    if (top != 0.0f) wild = p;
+    if (top != 0.0f) wild[p & 1] = p;
   };
   // This thread's part of the state: channels d0 and d0 + 8, columns 8 i + 2 t and the next.
   const int d0 = warp * 16 + g;
-  const bool holds = warp * 16 < DP;
+  const bool holds = states && warp * 16 < DP;
   float S[NT][4];
   float* state = a.state + static_cast<long long>(slot) * a.slot_stride + static_cast<long long>(h) * a.D * a.V + v0;
 #pragma unroll
@@ -476,8 +481,9 @@ __global__ void __launch_bounds__(W_THREADS, 1) state_walk_kernel(const WalkArgs
       const int d = d0 + (e >> 1) * 8, c = 8 * i + 2 * t + (e & 1);
       S[i][e] = holds && d < a.D && v0 + c < a.V ? state[static_cast<long long>(d) * a.V + c] : 0.0f;
     }
-  auto store_state = [&]() {
+  auto store_state = [&](int p) {                            // as piece p finds it
     if (!holds) return;
+    __nv_bfloat16* const s_s = state_s + p % Shape::BUFFERS * Shape::state_elems;
 #pragma unroll
     for (int i = 0; i < NT; ++i)
 #pragma unroll
@@ -488,10 +494,12 @@ __global__ void __launch_bounds__(W_THREADS, 1) state_walk_kernel(const WalkArgs
         for (int p = 0; p < PB; ++p) *reinterpret_cast<unsigned*>(s_s + (p * DP + d0 + 8 * half) * CST + 8 * i + 2 * t) = sp[p];
       }
   };
-  if (tid == 0 && pieces > 0) copy_piece(0);
-  store_state();
-  fetch_values(0);
-  store_values(0);
+  if (threadIdx.x == 0 && pieces > 0) copy_piece(0);
+  if (states) {
+    store_state(0);
+    fetch_values(0);
+    store_values(0);
+  }
   const float skip = MODE == WALK_SPACE ? a.skip[h] : 0.0f;
   // ldmatrix addresses: A rows as they lie, P's likewise, A transposed, B as [k][n].
   const int lrow = (lane & 7) + ((lane >> 3) & 1) * 8, lcol = (lane >> 4) * 8;
@@ -505,21 +513,51 @@ __global__ void __launch_bounds__(W_THREADS, 1) state_walk_kernel(const WalkArgs
     const __nv_bfloat16* k_s = q_s + PA * W * ST;
     const __nv_bfloat16* p_s = reinterpret_cast<const __nv_bfloat16*>(stage + Shape::qk_bytes);        // [PB][W][W_PST]
     const float* steps = reinterpret_cast<const float*>(stage + Shape::qk_bytes + Shape::p_bytes);
+    const __nv_bfloat16* s_s = state_s + p % Shape::BUFFERS * Shape::state_elems;
+    __nv_bfloat16* v_s = values_s + p % Shape::BUFFERS * Shape::value_elems;
+    const __nv_bfloat16* wv_s = v_s + PA * W * CST;
     const int n = min(W, n_all - p * W);
     const bool here = mbar_wait(&landed[p % STAGES], (p / STAGES) & 1, W_WAIT_LIMIT);
-    // The piece, the state and the values are there; the buffer of the piece before is free.
+    // The piece, the state and the values are there; the buffers of the piece before are free.
     if (!__syncthreads_and(here)) {
-      if (tid == 0) report(a.status, STATUS_COPY_TIMEOUT, p, row);
+      if (threadIdx.x == 0) report(a.status, STATUS_COPY_TIMEOUT, p, row);
       let_copies_land();
       return;
     }
-    if (tid == W_THREADS - 32 && p + 1 < pieces) copy_piece(p + 1);
-    fetch_values(p + 1);
+    if (states) {
+      if (tid == W_THREADS - 32 && p + 1 < pieces) copy_piece(p + 1);
+      fetch_values(p + 1);
+    }
+    auto carry_on = [&] {
+      if (!holds) return;
+      float sum[NT][4] = {}, sum_low[NT][4] = {};
+#pragma unroll
+      for (int ks = 0; ks < W / 16; ++ks) {
+        unsigned af[PA][4];
+        WalkB<NT, PB> b;
+#pragma unroll
+        for (int x = 0; x < PA; ++x) ldmatrix_x4_trans(af[x], k_s + (x * W + ks * 16) * ST + at_off + warp * 16);
+        b.load(wv_s + ks * 16 * CST + b_off, W * CST);
+        walk_product<NT, PA, PB>(sum, SPLIT_SUMS ? sum_low : sum, af, b);
+      }
+      const float whole = steps[2 * W];
+#pragma unroll
+      for (int i = 0; i < NT; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) S[i][e] = fmaf(whole, S[i][e], SPLIT_SUMS ? sum[i][e] + sum_low[i][e] : sum[i][e]);
+    };
+    if (ROLES && states) {
+      carry_on();
+      store_state(p + 1);
+      store_values(p + 1);
+      continue;
+    }
     const int i0 = row0 + g, i1 = i0 + 8;
-    const bool tame = wild != p;
+    const bool tame = wild[p & 1] != p;
+    auto outputs_meet = [] { asm volatile("bar.sync 1, 256;\n" ::: "memory"); };
     if (!tame) {
       drop_wild(v_s, PA * W * CST);
-      __syncthreads();
+      outputs_meet();
     }
     float o[NT][4] = {}, own_low[NT][4] = {};
     float (&low)[NT][4] = SPLIT_SUMS ? own_low : o;
@@ -578,26 +616,14 @@ __global__ void __launch_bounds__(W_THREADS, 1) state_walk_kernel(const WalkArgs
           }
       }
     }
-    if (holds) {
-      float sum[NT][4] = {}, sum_low[NT][4] = {};
-#pragma unroll
-      for (int ks = 0; ks < W / 16; ++ks) {
-        unsigned af[PA][4];
-        WalkB<NT, PB> b;
-#pragma unroll
-        for (int x = 0; x < PA; ++x) ldmatrix_x4_trans(af[x], k_s + (x * W + ks * 16) * ST + at_off + warp * 16);
-        b.load(wv_s + ks * 16 * CST + b_off, W * CST);
-        walk_product<NT, PA, PB>(sum, SPLIT_SUMS ? sum_low : sum, af, b);
-      }
-      const float whole = steps[2 * W];
-#pragma unroll
-      for (int i = 0; i < NT; ++i)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) S[i][e] = fmaf(whole, S[i][e], SPLIT_SUMS ? sum[i][e] + sum_low[i][e] : sum[i][e]);
+    if (ROLES) {
+      outputs_meet();
+    } else {
+      carry_on();
+      __syncthreads();             // the state's, the values' and the piece's reads are done
+      store_state(p + 1);
+      store_values(p + 1);
     }
-    __syncthreads();               // the state's, the values' and the piece's reads are done
-    store_state();
-    store_values(p + 1);
     if (row0 < n) {
 #pragma unroll
       for (int i = 0; i < MINE; ++i)
@@ -615,7 +641,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) state_walk_kernel(const WalkArgs
             if (v0 + c + 1 < a.V) to[1] = x.y + y.y;
           }
         }
-      // (the outputs that this thread has just written; the piece's buffer is filled again behind the next barrier)
+      // (the outputs that this thread has just written; the piece's buffer is filled again behind the next barrier of all warps)
       if (!tame) {
         using T = typename Shape::Value;
         const long long at = t0 + p * W;
@@ -635,13 +661,13 @@ __global__ void __launch_bounds__(W_THREADS, 1) state_walk_kernel(const WalkArgs
     }
 }
 
-template <int MODE, int DP, int NT>
+template <int MODE, int DP, bool ROLES>
 static int walk_launch(const WalkArgs& a, int pieces, cudaStream_t s) {
-  using Shape = WalkShape<MODE, DP, NT>;
-  static_assert(Shape::smem + 1024 <= 227 * 1024, "what a CTA keeps fits in shared memory");
+  using Shape = WalkShape<MODE, DP, ROLES>;
+  static_assert(Shape::smem + 256 <= 227 * 1024, "what a CTA keeps fits in shared memory");
   static_assert(Shape::qk_bytes % 16 == 0 && Shape::head_bytes % 16 == 0, "bulk copies move 16-byte pieces");
   auto prepare = walk_prepare_kernel<MODE, DP>;
-  auto walk = state_walk_kernel<MODE, DP, NT>;
+  auto walk = state_walk_kernel<MODE, DP, ROLES>;
   if (cuda_failed(cudaFuncSetAttribute(prepare, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::qk_bytes)) ||
       cuda_failed(cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::smem)))
     return ERR_CUDA;
@@ -649,19 +675,20 @@ static int walk_launch(const WalkArgs& a, int pieces, cudaStream_t s) {
   launch_dependent(prepare, dim3(pieces, a.H / a.heads_per_group * ((a.heads_per_group + heads - 1) / heads)),
       dim3(W_THREADS), Shape::qk_bytes, s, false, a);
   // (Not as a dependent, which would fill the SMs that are free first instead of all of them.)
-  walk<<<dim3(a.rows, a.H, (a.V + Shape::COLS - 1) / Shape::COLS), W_THREADS, Shape::smem, s>>>(a);
+  walk<<<dim3(a.rows, a.H, (a.V + Shape::COLS - 1) / Shape::COLS), Shape::THREADS, Shape::smem, s>>>(a);
   return launch_result();
 }
 
 template <int MODE>
 static int walk_dispatch(const WalkArgs& a, int pieces, cudaStream_t s) {
-  // 16 value columns a CTA, or 32: a CTA takes an SM, and a piece 1.7 us with 16 columns and 2.7 us with 32 (state space).
-  // Up to two CTAs an SM the narrow ones are not far behind even where all rows are equally long (two rounds of 1.7 us a
-  // piece), and far ahead where one row is much the longest (2048 and 77 tokens: 90 us with the wide ones).
+  // 16 value columns a CTA and a role a warp, or 32 and all of it: a CTA takes an SM.  Up to two of the narrow ones an SM they are ahead, far so where one
+  // row is much the longest (us, narrow / wide, state-space form, 32 heads of 128 x 64: 2048 and 77 tokens 74 / 90, one row of 2048 65; but twelve of
+  // 150 87 / 83, thirty of 64 121 / 97, four of 500 72 / 68; fixed decays, 32 heads of 64 x 128, three rows of 700 125 / 107).
   const bool wide = static_cast<long long>(a.rows) * a.H * ((a.V + 15) / 16) > 2 * 148;
-  if (a.D <= 64) return wide ? walk_launch<MODE, 64, 4>(a, pieces, s) : walk_launch<MODE, 64, 2>(a, pieces, s);
-  return wide ? walk_launch<MODE, 128, 4>(a, pieces, s) : walk_launch<MODE, 128, 2>(a, pieces, s);
+  if (a.D <= 64) return wide ? walk_launch<MODE, 64, false>(a, pieces, s) : walk_launch<MODE, 64, true>(a, pieces, s);
+  return wide ? walk_launch<MODE, 128, false>(a, pieces, s) : walk_launch<MODE, 128, true>(a, pieces, s);
 }
+
 
 }  // namespace zb
 
