@@ -101,6 +101,23 @@ def test_group_norms(cuda_device, group, groups, tokens, gate_first):
     assert (got.cpu().double() - want).abs().max() <= 4e-6 * max(1.0, float(want.abs().max()))
 
 
+@pytest.mark.parametrize("group,groups,tokens", [(60, 3, 1000), (64, 1, 2400), (68, 5, 700), (128, 33, 80), (132, 3, 7), (256, 2, 19)])
+def test_group_norms_side_by_side(cuda_device, group, groups, tokens):
+    """Several groups a warp, one scale for all of them, and gates far out: e^200 is infinite in float32, its inverse zero."""
+    from zephyr_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(group + tokens)
+    o, gate, w = torch.randn(tokens, group * groups, generator=g), torch.randn(tokens, group * groups, generator=g), torch.randn(group, generator=g)
+    gate[0, :4], gate[-1, -4:] = torch.tensor([200.0, -200.0, -88.0, -1e30]), torch.tensor([float("inf"), 1e30, float("-inf"), float("nan")])
+    got = ops.gated_group_rms_norm(o.to(cuda_device), gate.to(cuda_device), w.to(cuda_device), group, 1e-5, gate_first=False).cpu().double()
+    x = o.double().view(tokens, groups, group)
+    want = (x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-5)).view(tokens, -1) * w.double().repeat(groups) * torch.nn.functional.silu(gate.double())
+    assert torch.equal(got[-1, -4:].isnan(), torch.tensor([False, False, True, True])) and got[-1, -4].isinf()
+    got[-1, -4:], want[-1, -4:] = 0.0, 0.0
+    # The activation's exponential and five products and sums, each within a few 2^-24 of their own size.
+    assert ((got - want).abs() <= 4e-6 * torch.clamp(want.abs(), min=1.0)).all()
+
+
 @pytest.mark.parametrize("shape", [(1, 4), (3, 5), (129, 516), (1, 2049), (7, 1024)])
 def test_sums_and_biases(cuda_device, shape):
     from zephyr_b200.kernels import ops
@@ -132,3 +149,22 @@ def test_few_rows_at_the_splits_of_k(cuda_device, N, K, M):
         hidden = ops.gemm_small(x, w, out_dtype=torch.float32, swiglu=True)
         want = (torch.nn.functional.silu(gate) * up).reshape(M, N // 2)
         assert (hidden.double() - want).abs().max() <= 40 * 2.0 ** -24 * max(16.0, K ** 0.5)
+
+
+@pytest.mark.parametrize("tokens,heads,kv_heads,kd,vd,rot", [(64, 24, 8, 64, 64, 64), (63, 5, 3, 64, 40, 32), (70, 3, 1, 8, 8, 8), (64, 17, 3, 128, 72, 128),
+                                                             (700, 31, 5, 88, 128, 40), (2, 1, 1, 56, 64, 24)])
+@pytest.mark.parametrize("pairs", [True, False])
+def test_heads_side_by_side(cuda_device, tokens, heads, kv_heads, kd, vd, rot, pairs):
+    """Heads of a part of a warp, also where a warp holds queries beside keys and keys beside values."""
+    from zephyr_b200.kernels import ops
+
+    case = Projected(cuda_device, torch.bfloat16, tokens, heads, kv_heads, kd, vd, True)
+    norm, bias = [case.vector(kd), case.vector(kd)], case.vector(case.width)
+    freqs = (1000.0 ** (-torch.arange(rot // 2) / (rot // 2))).to(cuda_device)
+    out = []
+    for rows, cache in zip(case.rows, case.caches):
+        where = (freqs, rot), (case.pos, case.row, cache, case.table, case.status, torch.bfloat16)
+        out.append(ops.qkv_pairs(rows, heads, kv_heads, kd, vd, bias, *norm, 1e-6, *where[0], *where[1]) if pairs else
+                   ops.qkv_halves(rows, heads, kv_heads, kd, vd, "per_head", *norm, 1e-6, *where[0], 1.25, True, *where[1], bias=bias))
+    ops.check_status(case.status)
+    assert _apart(*out, torch.bfloat16) and _apart(*case.caches, torch.bfloat16) and case.caches[0][1:].abs().max() > 0

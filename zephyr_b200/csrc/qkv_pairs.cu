@@ -189,12 +189,13 @@ __global__ void __launch_bounds__(QP_WARPS * 32) qkv_pairs_kernel(const QkvPairs
 }
 
 // The same where the widths, the rotated part and every row start are whole pieces of four values.  A CTA takes one token:
-// its angles are worked out once, into shared memory, a warp loads all its heads' values before it uses the first, and where
-// a piece goes within a cache row is one exclusive-or.  The general kernel above is bound by instructions, not by memory:
-// two sines a lane and head and 300 instructions a head: 2125 tokens of 32
-// heads of 128 in float32 took 29.6 us and take 18.6 (its bytes: 8 us), 12 tokens 5.2 and 3.9 us.  More heads a warp alone
-// (33 us) did not help the general form.  Heads of up to 64 values leave half of a warp's lanes idle here and stay with the
-// general kernel (300 tokens, 40 heads of 64: 5.1 us there, 6.0 here; 2048: 21.4 and 21.9).
+// its angles are worked out once, into shared memory, a lane loads all its values before it uses the first, and where
+// a piece goes within a cache row is one exclusive-or.  Both forms are bound by instructions, not by memory: the general
+// kernel above issues two sines a lane and head and 300 instructions a head.  Here a head is LANES lanes' of eight values
+// each wherever there are tokens enough, so that a sum over lanes, a root and a row's address are issued once for the
+// heads side by side in a warp: 2125 tokens of 32 heads of 128 in float32 took 29.6 us in the general form, 18.6 as a warp a
+// head (68 % of all issue slots) and take 14.5 (its bytes: 8 us); 2048 tokens of 40 heads of 64 24.6 us in the general form
+// and 13.0 here, 12 tokens of 32 heads of 128 3.5 and 2.9 us.
 constexpr int QPV_WARPS = 8;
 
 __device__ __forceinline__ float4 load_piece(const float* p) { return *reinterpret_cast<const float4*>(p); }
@@ -212,13 +213,14 @@ __device__ __forceinline__ void store_piece(__nv_bfloat16* p, float4 v) {
   *reinterpret_cast<uint2*>(p) = raw;
 }
 
-template <typename IN, typename T, int ITEMS, int HEADS>
+template <typename IN, typename T, int LANES, int ITEMS, int HEADS>      // LANES: of a head, ITEMS pieces each; HEADS: of those lanes
 __global__ void __launch_bounds__(QPV_WARPS * 32) qkv_pairs_vec_kernel(const QkvPairsArgs a) {
   wait_for_prior_grids();
   let_dependents_launch();
   extern __shared__ __align__(16) float turn[];      // [rot_dims]: cosine and sine of every pair
-  const int t = blockIdx.x, lane = threadIdx.x & 31;
-  const int h0 = blockIdx.y * QPV_WARPS * HEADS + (threadIdx.x >> 5);     // and every QPV_WARPS-th behind it
+  constexpr int SIDE = QPV_WARPS * 32 / LANES;       // heads side by side
+  const int t = blockIdx.x, lane = threadIdx.x % LANES;
+  const int h0 = blockIdx.y * SIDE * HEADS + threadIdx.x / LANES;     // and every SIDE-th behind it
   const int total = a.cache != nullptr ? a.nh + (a.vd > 0 ? 2 : 1) * a.nkv : a.nh;
   const int pos = a.positions[t];
   const IN* src = static_cast<const IN*>(a.qkv) + static_cast<long long>(t) * a.stride;
@@ -226,14 +228,14 @@ __global__ void __launch_bounds__(QPV_WARPS * 32) qkv_pairs_vec_kernel(const Qkv
   float4 x[HEADS][ITEMS];
 #pragma unroll
   for (int j = 0; j < HEADS; ++j) {
-    const int h = h0 + QPV_WARPS * j;
+    const int h = h0 + SIDE * j;
     const bool is_v = h >= a.nh + a.nkv;
     const int dim = h >= total ? 0 : (is_v ? a.vd : a.kd);
     const int col = !is_v ? h * a.kd
                           : (a.values_from_keys ? (h - a.nkv) * a.kd : (a.nh + a.nkv) * a.kd + (h - a.nh - a.nkv) * a.vd);
 #pragma unroll
     for (int k = 0; k < ITEMS; ++k) {
-      const int i = 4 * (lane + 32 * k);
+      const int i = 4 * (lane + LANES * k);
       x[j][k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       if (i < dim) {
         x[j][k] = load_piece(src + col + i);
@@ -261,10 +263,13 @@ __global__ void __launch_bounds__(QPV_WARPS * 32) qkv_pairs_vec_kernel(const Qkv
         ss[j] += (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w);
       }
     }
-    warp_sums<HEADS>(ss);
+#pragma unroll
+    for (int d = LANES / 2; d > 0; d >>= 1)
+#pragma unroll
+      for (int j = 0; j < HEADS; ++j) ss[j] += __shfl_xor_sync(0xffffffffu, ss[j], d);
 #pragma unroll
     for (int j = 0; j < HEADS; ++j) {
-      const int h = h0 + QPV_WARPS * j;
+      const int h = h0 + SIDE * j;
       const bool is_q = h < a.nh, is_v = h >= a.nh + a.nkv;
       const int dim = is_v ? a.vd : a.kd;
       const float* w = is_q ? a.q_norm_w : (is_v ? nullptr : a.k_norm_w);
@@ -272,7 +277,7 @@ __global__ void __launch_bounds__(QPV_WARPS * 32) qkv_pairs_vec_kernel(const Qkv
       const float inv = 1.0f / sqrtf(ss[j] / static_cast<float>(dim) + a.eps);
 #pragma unroll
       for (int k = 0; k < ITEMS; ++k) {
-        const int i = 4 * (lane + 32 * k);
+        const int i = 4 * (lane + LANES * k);
         const float4 v = x[j][k];
         float4 c = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
         if (w != nullptr && i < dim) c = load_piece(w + i);
@@ -303,14 +308,14 @@ __global__ void __launch_bounds__(QPV_WARPS * 32) qkv_pairs_vec_kernel(const Qkv
 
 #pragma unroll
   for (int j = 0; j < HEADS; ++j) {
-    const int h = h0 + QPV_WARPS * j;
+    const int h = h0 + SIDE * j;
     if (h >= total) break;
     const bool is_q = h < a.nh, is_v = h >= a.nh + a.nkv;
     const int dim = is_v ? a.vd : a.kd;
     if (!is_v) {
 #pragma unroll
       for (int k = 0; k < ITEMS; ++k) {
-        const int i = 4 * (lane + 32 * k);
+        const int i = 4 * (lane + LANES * k);
         float4 v = x[j][k];
         if (i < a.rot_dims) {
           const float4 f = *reinterpret_cast<const float4*>(turn + i);      // cosine, sine of two pairs
@@ -333,7 +338,7 @@ __global__ void __launch_bounds__(QPV_WARPS * 32) qkv_pairs_vec_kernel(const Qkv
     }
 #pragma unroll
     for (int k = 0; k < ITEMS; ++k) {
-      const int i = 4 * (lane + 32 * k);
+      const int i = 4 * (lane + LANES * k);
       if (i < dim) store_piece(dst + (i ^ (swizzle * CHUNK)), x[j][k]);
     }
   }
@@ -372,24 +377,27 @@ ZB_API int zb_qkv_pairs(void* q_out, const void* qkv, long long stride, const fl
   const int wide = kd > vd ? kd : vd;
   const long long page_values = static_cast<long long>(nkv) * page_size * (kd + vd);
   if (!(dtype == DTYPE_F32 && in_dtype != DTYPE_F32) && kd % 4 == 0 && vd % 4 == 0 && a.rot_dims % 4 == 0 && stride % 4 == 0 &&
-      whole(qkv) && whole(bias) && whole(q_norm_w) && whole(k_norm_w) && whole(q_out) && whole(cache) && wide > 64 && wide <= 256 &&
+      whole(qkv) && whole(bias) && whole(q_norm_w) && whole(k_norm_w) && whole(q_out) && whole(cache) && wide <= 256 &&
       page_values <= INT_MAX && a.rot_dims <= 8192) {
     auto s = static_cast<cudaStream_t>(stream);
     const size_t smem = sizeof(float) * a.rot_dims;
-#define ZB_QPV(ITEMS, HEADS)                                                                                             \
+#define ZB_QPV(LANES, ITEMS, HEADS)                                                                                      \
   {                                                                                                                      \
-    const dim3 grid(tokens, (heads + HEADS * QPV_WARPS - 1) / (HEADS * QPV_WARPS));                                      \
-    if (dtype == DTYPE_F32) launch_dependent(qkv_pairs_vec_kernel<float, float, ITEMS, HEADS>, grid, dim3(QPV_WARPS * 32),    \
-        smem, s, false, a);                                                                                                   \
-    else if (in_dtype == DTYPE_F32) launch_dependent(qkv_pairs_vec_kernel<float, __nv_bfloat16, ITEMS, HEADS>, grid,          \
+    const dim3 grid(tokens, (heads + HEADS * (QPV_WARPS * 32 / LANES) - 1) / (HEADS * (QPV_WARPS * 32 / LANES)));        \
+    if (dtype == DTYPE_F32) launch_dependent(qkv_pairs_vec_kernel<float, float, LANES, ITEMS, HEADS>, grid,                   \
         dim3(QPV_WARPS * 32), smem, s, false, a);                                                                             \
-    else launch_dependent(qkv_pairs_vec_kernel<__nv_bfloat16, __nv_bfloat16, ITEMS, HEADS>, grid, dim3(QPV_WARPS * 32),       \
-        smem, s, false, a);                                                                                                   \
+    else if (in_dtype == DTYPE_F32) launch_dependent(qkv_pairs_vec_kernel<float, __nv_bfloat16, LANES, ITEMS, HEADS>, grid,   \
+        dim3(QPV_WARPS * 32), smem, s, false, a);                                                                             \
+    else launch_dependent(qkv_pairs_vec_kernel<__nv_bfloat16, __nv_bfloat16, LANES, ITEMS, HEADS>, grid,                      \
+        dim3(QPV_WARPS * 32), smem, s, false, a);                                                                             \
   }
-    // Several heads a warp where the tokens alone give every SM a full set of warps; a decode step keeps its heads apart.
-    const bool many = tokens >= 4 * 148 && heads > QPV_WARPS;
-    if (wide <= 128) { if (many) ZB_QPV(1, 4) else ZB_QPV(1, 1) }
-    else { if (many) ZB_QPV(2, 2) else ZB_QPV(2, 1) }
+    // Eight values a lane and several heads a warp from 64 tokens on, twice over where the tokens alone give every SM a full
+    // set of warps (300 tokens of 32 heads of 128: 4.1 us as one set, 5.3 as four values a lane; 600: 5.1 as two); a decode
+    // step keeps its heads apart.
+    const bool some = tokens >= 64, many = tokens >= 4 * 148 && heads > QPV_WARPS;
+    if (wide <= 64) { if (some) ZB_QPV(8, 2, 1) else ZB_QPV(16, 1, 1) }
+    else if (wide <= 128) { if (many) ZB_QPV(16, 2, 2) else if (some) ZB_QPV(16, 2, 1) else ZB_QPV(32, 1, 1) }
+    else { if (many) ZB_QPV(32, 2, 2) else ZB_QPV(32, 2, 1) }
 #undef ZB_QPV
     return launch_result();
   }

@@ -24,7 +24,17 @@
 
 namespace zb {
 
-__device__ __forceinline__ float silu_f(float z) { return z / (1.0f + expf(-z)); }
+// z / (1 + e^-z).  The quotient is the reciprocal's estimate times z, corrected once by its remainder (fused, so exact to
+// rounding, after Markstein: of all 2^32 inputs one differs from the divide operator's result): that operator's guarded form
+// kept a thread's values one behind the other.  Where the correction has no
+// meaning (an infinite z or e^-z), the uncorrected product is the quotient.
+__device__ __forceinline__ float silu_f(float z) {
+  const float d = 1.0f + expf(-z);
+  float r;
+  asm("rcp.approx.f32 %0, %1;\n" : "=f"(r) : "f"(d));
+  const float q = z * r, better = fmaf(fmaf(-d, q, z), r, q);
+  return better == better ? better : q;
+}
 __device__ __forceinline__ float log_sigmoid_f(float z) { return fminf(z, 0.0f) - log1pf(expf(-fabsf(z))); }
 __device__ __forceinline__ float softplus_f(float z) { return fmaxf(z, 0.0f) + log1pf(expf(-fabsf(z))); }
 
@@ -363,8 +373,9 @@ __global__ void causal_conv_silu_kernel(const ConvArgs a, const int* token_row, 
 // stream, a thread VEC neighbouring channels of them.  Bound by latency where a thread walks its tokens one load
 // behind the other, so it asks for all its inputs, the TAPS - 1 before the first token among them, before it uses any
 // (they come again from the cache for the next CTA); inputs before a request's first new token come from its state.
-// 2048 tokens: 2560 bfloat16 channels 15.5 us (21.7 us walked 32 tokens a thread), 4096 float32 channels 20.6 us (69.6 us
-// with a thread a channel and token).
+// 2125 tokens of 2560 bfloat16 channels 13.5 us (15.3 with a divide in the activation, 21.7 walked 32 tokens a thread), 2048
+// tokens of 4096 float32 channels 17.6 us (20.3; 69.6 with a thread a channel and token).  Six CTAs an SM: at five, which the
+// registers of its own choice allow, 14.2 and 17.0 us; at seven and eight registers spill, 14.5 and 17.9, 15.5 and 19.3 us.
 // TAPS: the taps of the kernel, `taps` of them in use (the others, at the old end, are skipped).
 constexpr int CONV_RUN = 8;
 
@@ -389,7 +400,7 @@ __device__ __forceinline__ void conv_store(T* p, const float (&y)[VEC]) {
 }
 
 template <typename T, int VEC, int TAPS>
-__global__ void __launch_bounds__(128) causal_conv_silu_run_kernel(const ConvArgs a, const int* token_row, int tokens) {
+__global__ void __launch_bounds__(128, VEC == 4 && TAPS == 4 ? 6 : 1) causal_conv_silu_run_kernel(const ConvArgs a, const int* token_row, int tokens) {
   wait_for_prior_grids();
   let_dependents_launch();
   __shared__ int first_s[CONV_RUN], slot_s[CONV_RUN];         // per token: index within its request's new tokens, slot
@@ -475,15 +486,17 @@ static void conv_run_launch(const ConvArgs& a, const int* token_row, int tokens,
   }
 }
 
-// After it: every request's last taps - 1 inputs go to its state.  A thread owns a channel of one request.
+// After it: every request's last taps - 1 inputs go to its state.  A thread owns a channel of one request.  All it reads is
+// older than the convolution, which only reads the state, so it reads beside it and waits for its end before it writes.
 template <typename T>
 __global__ void conv_state_update_kernel(const ConvArgs a) {
-  wait_for_prior_grids();
-  let_dependents_launch();
   const int c = blockIdx.x * blockDim.x + threadIdx.x, row = blockIdx.y;
   if (c >= a.C) return;
   const int slot = a.slots[row];
-  if (slot < 0 || slot >= a.num_slots) return;       // reported by the convolution
+  if (slot < 0 || slot >= a.num_slots) {             // reported by the convolution
+    wait_for_prior_grids();                          // what follows waits for this kernel only
+    return;
+  }
   float* state = a.state + static_cast<long long>(slot) * a.slot_stride;
   const T* x = static_cast<const T*>(a.x);
   const int t0 = a.row_q_start[row], n = a.row_q_len[row], keep = a.taps - 1;
@@ -496,6 +509,8 @@ __global__ void conv_state_update_kernel(const ConvArgs a) {
                        : state[static_cast<long long>(keep + i) * a.C + c];
     }
   }
+  wait_for_prior_grids();
+  let_dependents_launch();
 #pragma unroll
   for (int j = 0; j < CONV_MAX_TAPS; ++j)
     if (j < keep) state[static_cast<long long>(j) * a.C + c] = last[j];
@@ -862,76 +877,84 @@ __global__ void gated_group_rms_norm_kernel(T* out, const float* o, const G* gat
 }
 
 // The same for groups of up to GN_VEC_MAX columns that are a multiple of four, with aligned rows: o and the gate are
-// read once, all loads before the first use, and stay in registers.  A group of up to 512 columns is a warp's, a wider one
-// a CTA's of four warps: bound by the latency of its loads, a warp alone with 16 of them had to read the gate a second
-// time and took 22.0 us for 2125 tokens of two groups of 1024 and 10.9 us for 12; now 11.3 and 3.5 us.
+// read once, all loads before the first use, and stay in registers.  A group is LANES lanes' of a warp, eight values each and
+// more, up to 512 columns, and a CTA's of four warps beyond: what a group costs besides its values (where it lies, the sum
+// over its lanes, the root) is issued once for all the groups of a warp.  Bound by the instructions of the activation (a
+// warp a group: 79 % of all issue slots).  2048 tokens of 32 groups of 128 in bfloat16 12.8 us as a warp a group, now 10.7
+// (its bytes: 9 us); 2048 tokens of 32 groups of 64 24.6 us (with a float32 out) and 10.1; 2125 tokens of two groups of 1024
+// 11.4 and 11.3 us.
 constexpr int GN_WARPS = 4;
 constexpr int GN_VEC_ITEMS = 4;
 constexpr int GN_VEC_MAX = GN_WARPS * 32 * GN_VEC_ITEMS * 4;
 
-template <typename T, typename G, int ITEMS, int WARPS>      // WARPS: of a group
+template <typename T, typename G, int LANES, int ITEMS>      // LANES: of a group
 __global__ void __launch_bounds__(32 * GN_WARPS) gated_group_rms_norm_vec_kernel(T* out, const float* o, const G* gate, long long gate_stride,
                                                 const float* w, int w_len, int width, int group, float eps,
-                                                int gate_first, int tokens) {
+                                                int gate_first, unsigned items) {
   wait_for_prior_grids();
   let_dependents_launch();
   __shared__ float part[GN_WARPS];
-  const int groups = width / group, warp = threadIdx.x >> 5;
-  const long long item = WARPS == 1 ? static_cast<long long>(blockIdx.x) * GN_WARPS + warp : blockIdx.x;
-  if (item >= static_cast<long long>(tokens) * groups) return;
-  const int lane = WARPS == 1 ? threadIdx.x & 31 : threadIdx.x, nv = group / 4;
-  const long long t = item / groups;
+  constexpr int PER_CTA = 32 * GN_WARPS / LANES;
+  const unsigned groups = width / group, item = blockIdx.x * static_cast<unsigned>(PER_CTA) + threadIdx.x / LANES;
+  const int lane = threadIdx.x % LANES, nv = item < items ? group / 4 : 0;
+  const unsigned t = item / groups;
   const int c0 = static_cast<int>(item - t * groups) * group;
+  const float* o_row = o + static_cast<long long>(t) * width + c0;
+  const G* gate_row = gate + t * gate_stride + c0;
   float4 val[ITEMS], g[ITEMS];
 #pragma unroll
   for (int j = 0; j < ITEMS; ++j) {
-    const int i = lane + 32 * WARPS * j;
+    const int i = lane + LANES * j;
+    val[j] = g[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (i < nv) {
-      val[j] = load4(o + t * width + c0 + 4 * i);
-      g[j] = load4(gate + t * gate_stride + c0 + 4 * i);
+      val[j] = load4(o_row + 4 * i);
+      g[j] = load4(gate_row + 4 * i);
     }
   }
   float ss = 0.0f;
 #pragma unroll
   for (int j = 0; j < ITEMS; ++j) {
-    if (lane + 32 * WARPS * j < nv) {
-      g[j] = make_float4(silu_f(g[j].x), silu_f(g[j].y), silu_f(g[j].z), silu_f(g[j].w));
-      if (gate_first) val[j] = make_float4(val[j].x * g[j].x, val[j].y * g[j].y, val[j].z * g[j].z, val[j].w * g[j].w);
-      ss += (val[j].x * val[j].x + val[j].y * val[j].y) + (val[j].z * val[j].z + val[j].w * val[j].w);
-    }
+    g[j] = make_float4(silu_f(g[j].x), silu_f(g[j].y), silu_f(g[j].z), silu_f(g[j].w));
+    if (gate_first) val[j] = make_float4(val[j].x * g[j].x, val[j].y * g[j].y, val[j].z * g[j].z, val[j].w * g[j].w);
+    ss += (val[j].x * val[j].x + val[j].y * val[j].y) + (val[j].z * val[j].z + val[j].w * val[j].w);
   }
-  ss = warp_sum(ss);
-  if (WARPS > 1) {
-    if ((threadIdx.x & 31) == 0) part[warp] = ss;
+#pragma unroll
+  for (int d = (LANES < 32 ? LANES : 32) / 2; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
+  if (LANES > 32) {
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = ss;
     __syncthreads();
     ss = (part[0] + part[1]) + (part[2] + part[3]);
   }
   const float r = 1.0f / sqrtf(ss / static_cast<float>(group) + eps);
+  const int w0 = c0 < w_len ? c0 : c0 % w_len;
 #pragma unroll
   for (int j = 0; j < ITEMS; ++j) {
-    const int i = lane + 32 * WARPS * j;
+    const int i = lane + LANES * j;
     if (i < nv) {
-      const float4 wv = load4(w + (c0 + 4 * i) % w_len);
+      const int at = w0 + 4 * i;
+      const float4 wv = load4(w + (at < w_len ? at : at % w_len));
       float4 y = make_float4(val[j].x * r * wv.x, val[j].y * r * wv.y, val[j].z * r * wv.z, val[j].w * r * wv.w);
       if (!gate_first) y = make_float4(y.x * g[j].x, y.y * g[j].y, y.z * g[j].z, y.w * g[j].w);
-      store4(out + t * width + c0 + 4 * i, y);
+      store4(out + static_cast<long long>(t) * width + c0 + 4 * i, y);
     }
   }
 }
 
 template <typename T, typename G>
 void gated_group_rms_norm_vec(T* out, const float* o, const G* gate, long long gate_stride, const float* w, int w_len, int width,
-                              int group, float eps, int gate_first, int tokens, cudaStream_t s) {
-  const long long items = static_cast<long long>(tokens) * (width / group);
-#define ZB_GN(ITEMS, WARPS)                                                                                                  \
-  launch_dependent(gated_group_rms_norm_vec_kernel<T, G, ITEMS, WARPS>,                                                       \
-      dim3(static_cast<unsigned>((items * WARPS + GN_WARPS - 1) / GN_WARPS)), dim3(32 * GN_WARPS), 0, s, false, out, o,       \
-      gate, gate_stride, w, w_len, width, group, eps, gate_first, tokens)
-  if (group <= 128) ZB_GN(1, 1);
-  else if (group <= 256) ZB_GN(2, 1);
-  else if (group <= 512) ZB_GN(4, 1);
-  else if (group <= 1024) ZB_GN(2, GN_WARPS);
-  else ZB_GN(GN_VEC_ITEMS, GN_WARPS);
+                              int group, float eps, int gate_first, unsigned items, cudaStream_t s) {
+#define ZB_GN(LANES, ITEMS)                                                                                                  \
+  launch_dependent(gated_group_rms_norm_vec_kernel<T, G, LANES, ITEMS>,                                                       \
+      dim3((items - 1) / (32 * GN_WARPS / LANES) + 1), dim3(32 * GN_WARPS), 0, s, false, out, o, gate, gate_stride, w, w_len,    \
+      width, group, eps, gate_first, items)
+  // Few groups, which leave SMs idle, are a warp each: 12 tokens of 32 groups of 128 take 2.3 us, two a warp 2.7.
+  if (group <= 128 && items < 4 * 148 * GN_WARPS) ZB_GN(32, 1);
+  else if (group <= 64) ZB_GN(8, 2);
+  else if (group <= 128) ZB_GN(16, 2);
+  else if (group <= 256) ZB_GN(32, 2);
+  else if (group <= 512) ZB_GN(32, 4);
+  else if (group <= 1024) ZB_GN(128, 2);
+  else ZB_GN(128, GN_VEC_ITEMS);
 #undef ZB_GN
 }
 
@@ -1225,20 +1248,20 @@ ZB_API int zb_gated_group_rms_norm(void* out, const float* o, const void* gate, 
   const unsigned blocks = static_cast<unsigned>((items + warps - 1) / warps);
   auto s = static_cast<cudaStream_t>(stream);
   const int elem = dtype == DTYPE_F32 ? 4 : 2, gate_elem = gate_dtype == DTYPE_F32 ? 4 : 2;
-  if (group % 4 == 0 && group <= GN_VEC_MAX && w_len % 4 == 0 && w_dtype == DTYPE_F32 && gate_stride % 4 == 0 &&
+  if (items <= INT_MAX && group % 4 == 0 && group <= GN_VEC_MAX && w_len % 4 == 0 && w_dtype == DTYPE_F32 && gate_stride % 4 == 0 &&
       reinterpret_cast<uintptr_t>(gate) % (4 * gate_elem) == 0 && reinterpret_cast<uintptr_t>(o) % 16 == 0 &&
       reinterpret_cast<uintptr_t>(out) % (4 * elem) == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0) {
     const float* wf = static_cast<const float*>(w);
     using bf16 = __nv_bfloat16;
     if (dtype == DTYPE_F32)
       gated_group_rms_norm_vec(static_cast<float*>(out), o, static_cast<const float*>(gate), gate_stride, wf, w_len, width, group,
-                               eps, gate_first, tokens, s);
+                               eps, gate_first, static_cast<unsigned>(items), s);
     else if (gate_dtype == DTYPE_F32)
       gated_group_rms_norm_vec(static_cast<bf16*>(out), o, static_cast<const float*>(gate), gate_stride, wf, w_len, width, group,
-                               eps, gate_first, tokens, s);
+                               eps, gate_first, static_cast<unsigned>(items), s);
     else
       gated_group_rms_norm_vec(static_cast<bf16*>(out), o, static_cast<const bf16*>(gate), gate_stride, wf, w_len, width, group,
-                               eps, gate_first, tokens, s);
+                               eps, gate_first, static_cast<unsigned>(items), s);
     return launch_result();
   }
   if (dtype == DTYPE_F32)

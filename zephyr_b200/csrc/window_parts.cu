@@ -280,36 +280,47 @@ __global__ void __launch_bounds__(QH_THREADS) qkv_halves_vec_kernel(const QkvHal
   }
 }
 
-// The same where no statistic spans the heads (any norm but NORM_WHOLE) and a head is at most a warp's 32 pieces of four
-// values: a warp takes HEADS heads of one token, loads them all before it uses the first and keeps them in registers, a
-// value's partner in the rotation comes by a shuffle, and only the token's angles, worked out once a CTA, pass through shared
-// memory.  The CTA a token above waits at two barriers between its load and its store and reads its values twice:
-// 3000 tokens of 32 heads of 128 took 38 us and take 26 (its bytes: 11 us).
+// The same where no statistic spans the heads (any norm but NORM_WHOLE) and a head is at most 128 values: a head is LANES
+// lanes' of two pieces of four values, which it loads before it uses the first and keeps in registers; a query's and key's
+// pieces are dealt so that a lane holds a value and its partner in the rotation, and only the token's angles, worked out once
+// a CTA, pass through shared memory.  Bound by the instructions it issues (68 % of all slots as a warp a head, with partners
+// passed by shuffles): a sum over lanes, a root and a row's address now serve the heads side by side in a warp.
+// 3000 tokens of 32 heads of 128: 38 us as the CTA a token above, 24.8 as a warp a head, 20.1 now (its bytes: 11 us);
+// 2048 tokens of 40 heads of 64: 35, 28.6 and 14.3 us.
 constexpr int QHH_WARPS = 8;
 
-template <typename T, int HEADS>
+template <typename T, int LANES, int HEADS>      // LANES: of a head, two pieces each; HEADS: of those lanes
 __global__ void __launch_bounds__(QHH_WARPS * 32) qkv_halves_heads_kernel(const QkvHalvesArgs a) {
   wait_for_prior_grids();
   let_dependents_launch();
   extern __shared__ __align__(16) float qh_smem[];      // [rot_dims]: cosines, then sines
-  const int t = blockIdx.x, lane = threadIdx.x & 31, i = 4 * lane;
-  const int h0 = blockIdx.y * QHH_WARPS * HEADS + (threadIdx.x >> 5);     // and every QHH_WARPS-th behind it
+  constexpr int SIDE = QHH_WARPS * 32 / LANES;          // heads side by side
+  const int t = blockIdx.x, lane = threadIdx.x % LANES;
+  const int h0 = blockIdx.y * SIDE * HEADS + threadIdx.x / LANES;     // and every SIDE-th behind it
   const int kv_heads = a.cache != nullptr ? a.nkv : 0;
-  const int first_v = a.nh + kv_heads, heads = first_v + kv_heads, half = a.rot_dims / 2;
+  const int first_v = a.nh + kv_heads, heads = first_v + kv_heads, half = a.rot_dims / 2, turned = half / 4;
+  // A query's or key's lane: piece `lane` of the rotated values and its partner half a rotation on, or two pieces behind them.
+  const bool turns = lane < turned;
+  const int qk_at[2] = {4 * (turns ? lane : turned + lane), 4 * (turns ? lane + turned : LANES + lane)};
+  const int v_at[2] = {4 * lane, 4 * (LANES + lane)};
   const float* src = static_cast<const float*>(a.qkv) + static_cast<long long>(t) * a.stride;
-  const int pos = a.positions[t];
-  float4 x[HEADS];
+  const int pos = a.positions[t], row = a.cache != nullptr ? a.token_row[t] : 0;
+  float4 x[HEADS][2];
 #pragma unroll
   for (int j = 0; j < HEADS; ++j) {
-    const int h = h0 + QHH_WARPS * j;
+    const int h = h0 + SIDE * j;
     const bool is_v = h >= first_v;
-    x[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (h < heads && i < (is_v ? a.vd : a.kd)) {
-      const int c = (is_v ? first_v * a.kd + (h - first_v) * a.vd : h * a.kd) + i;
-      x[j] = *reinterpret_cast<const float4*>(src + c);
-      if (a.bias != nullptr) {
-        const float4 b = *reinterpret_cast<const float4*>(a.bias + c);
-        x[j] = make_float4(x[j].x + b.x, x[j].y + b.y, x[j].z + b.z, x[j].w + b.w);
+    const int dim = h >= heads ? 0 : (is_v ? a.vd : a.kd), c = is_v ? first_v * a.kd + (h - first_v) * a.vd : h * a.kd;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int i = is_v ? v_at[k] : qk_at[k];
+      x[j][k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (i < dim) {
+        x[j][k] = *reinterpret_cast<const float4*>(src + c + i);
+        if (a.bias != nullptr) {
+          const float4 b = *reinterpret_cast<const float4*>(a.bias + c + i);
+          x[j][k] = make_float4(x[j][k].x + b.x, x[j][k].y + b.y, x[j][k].z + b.z, x[j][k].w + b.w);
+        }
       }
     }
   }
@@ -323,21 +334,35 @@ __global__ void __launch_bounds__(QHH_WARPS * 32) qkv_halves_heads_kernel(const 
   {
     float ss[HEADS];
 #pragma unroll
-    for (int j = 0; j < HEADS; ++j) ss[j] = (x[j].x * x[j].x + x[j].y * x[j].y) + (x[j].z * x[j].z + x[j].w * x[j].w);
-    warp_sums<HEADS>(ss);
+    for (int j = 0; j < HEADS; ++j) {
+      ss[j] = 0.0f;
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const float4 v = x[j][k];
+        ss[j] += (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w);
+      }
+    }
+#pragma unroll
+    for (int d = LANES / 2; d > 0; d >>= 1)
+#pragma unroll
+      for (int j = 0; j < HEADS; ++j) ss[j] += __shfl_xor_sync(0xffffffffu, ss[j], d);
 #pragma unroll
     for (int j = 0; j < HEADS; ++j) {
-      const int h = h0 + QHH_WARPS * j;
+      const int h = h0 + SIDE * j;
       const bool is_q = h < a.nh, is_v = h >= first_v;
       const int dim = is_v ? a.vd : a.kd;
       if (!(is_v ? a.value_unit_norm != 0 : a.norm_mode == NORM_PER_HEAD)) continue;
       const float inv = 1.0f / sqrtf(ss[j] / static_cast<float>(dim) + a.eps);
-      x[j] = scaled4(x[j], inv, is_v || i >= dim ? nullptr : (is_q ? a.q_norm_w : a.k_norm_w), i);
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const int i = is_v ? v_at[k] : qk_at[k];
+        x[j][k] = scaled4(x[j][k], inv, is_v || i >= dim ? nullptr : (is_q ? a.q_norm_w : a.k_norm_w), i);
+      }
     }
   }
   int page = 0;
   if (a.cache != nullptr) {
-    const int row = a.token_row[t], block = pos / a.page_size;
+    const int block = pos / a.page_size;
     if (row < 0 || row >= a.num_rows || block >= a.max_blocks) {
       if (threadIdx.x == 0) report(a.status, STATUS_ROW_OUT_OF_RANGE, row, t);
       return;
@@ -350,42 +375,45 @@ __global__ void __launch_bounds__(QHH_WARPS * 32) qkv_halves_heads_kernel(const 
   }
   const int slot = pos % a.page_size;
   constexpr int CHUNK = 16 / sizeof(T);            // values a 16-byte chunk: a piece never straddles two
-  const int at_k = i ^ (kv_swizzle(pos, a.kd / CHUNK) * CHUNK), at_v = i ^ (kv_swizzle(pos, a.vd / CHUNK) * CHUNK);
+  const int k_swizzle = kv_swizzle(pos, a.kd / CHUNK) * CHUNK, v_swizzle = kv_swizzle(pos, a.vd / CHUNK) * CHUNK;
   T* q_row = static_cast<T*>(a.q_out) + static_cast<long long>(t) * a.nh * a.kd;
   T* page_row = static_cast<T*>(a.cache) + static_cast<long long>(page) * (a.nkv * a.page_size * (a.kd + a.vd));
   const float share = a.v_first != nullptr ? *a.v_share : 0.0f;
   __syncthreads();
   float4 cosine = make_float4(1.0f, 1.0f, 1.0f, 1.0f), sine = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  const bool turns = i < 2 * half, low = i < half;
-  const int partner = low ? lane + half / 4 : lane - half / 4;
   if (turns) {
-    cosine = *reinterpret_cast<const float4*>(qh_smem + (low ? i : i - half));
-    sine = *reinterpret_cast<const float4*>(qh_smem + (low ? half + i : i));
-    if (low) sine = make_float4(-sine.x, -sine.y, -sine.z, -sine.w);
+    cosine = *reinterpret_cast<const float4*>(qh_smem + 4 * lane);
+    sine = *reinterpret_cast<const float4*>(qh_smem + half + 4 * lane);
   }
 #pragma unroll
   for (int j = 0; j < HEADS; ++j) {
-    const int h = h0 + QHH_WARPS * j;
+    const int h = h0 + SIDE * j;
     if (h >= heads) break;
     const bool is_q = h < a.nh, is_v = h >= first_v;
     const int dim = is_v ? a.vd : a.kd;
-    float4 y = x[j];
-    if (!is_v && half > 0) {
-      const float4 p = make_float4(__shfl_sync(~0u, y.x, partner), __shfl_sync(~0u, y.y, partner),
-                                   __shfl_sync(~0u, y.z, partner), __shfl_sync(~0u, y.w, partner));
-      if (turns)
-        y = make_float4(y.x * cosine.x + p.x * sine.x, y.y * cosine.y + p.y * sine.y, y.z * cosine.z + p.z * sine.z,
-                        y.w * cosine.w + p.w * sine.w);
+    if (!is_v && turns) {
+      const float4 u = x[j][0], v = x[j][1];
+      x[j][0] = make_float4(u.x * cosine.x - v.x * sine.x, u.y * cosine.y - v.y * sine.y, u.z * cosine.z - v.z * sine.z,
+                            u.w * cosine.w - v.w * sine.w);
+      x[j][1] = make_float4(v.x * cosine.x + u.x * sine.x, v.y * cosine.y + u.y * sine.y, v.z * cosine.z + u.z * sine.z,
+                            v.w * cosine.w + u.w * sine.w);
     }
-    if (i >= dim) continue;
-    if (is_v && a.v_first != nullptr) {
-      const float4 f = *reinterpret_cast<const float4*>(a.v_first + static_cast<long long>(t) * a.v_first_stride + (h - first_v) * a.vd + i);
-      const float keep = 1.0f - share;
-      y = make_float4(keep * y.x + share * f.x, keep * y.y + share * f.y, keep * y.z + share * f.z, keep * y.w + share * f.w);
+    T* dst = is_q ? q_row + h * a.kd
+                  : page_row + (is_v ? a.nkv * a.page_size * a.kd + ((h - first_v) * a.page_size + slot) * a.vd
+                                     : ((h - a.nh) * a.page_size + slot) * a.kd);
+    const int swizzle = is_q ? 0 : (is_v ? v_swizzle : k_swizzle);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int i = is_v ? v_at[k] : qk_at[k];
+      if (i >= dim) continue;
+      float4 y = x[j][k];
+      if (is_v && a.v_first != nullptr) {
+        const float4 f = *reinterpret_cast<const float4*>(a.v_first + static_cast<long long>(t) * a.v_first_stride + (h - first_v) * a.vd + i);
+        const float keep = 1.0f - share;
+        y = make_float4(keep * y.x + share * f.x, keep * y.y + share * f.y, keep * y.z + share * f.z, keep * y.w + share * f.w);
+      }
+      store_four<T>(dst + (i ^ swizzle), y);
     }
-    if (is_q) store_four<T>(q_row + h * a.kd + i, y);
-    else if (is_v) store_four<T>(page_row + a.nkv * a.page_size * a.kd + ((h - first_v) * a.page_size + slot) * a.vd + at_v, y);
-    else store_four<T>(page_row + ((h - a.nh) * a.page_size + slot) * a.kd + at_k, y);
   }
 }
 
@@ -577,14 +605,16 @@ ZB_API int zb_qkv_halves(void* q_out, const void* qkv, long long stride, const f
       // Several heads a warp where the tokens alone give every SM a full set of warps; a decode step keeps its heads apart.
       const bool many = tokens >= 4 * 148 && heads > QHH_WARPS;
       const size_t turn = sizeof(float) * a.rot_dims;
-#define ZB_QHH(HEADS)                                                                                        \
+#define ZB_QHH(LANES, HEADS)                                                                                 \
   {                                                                                                          \
-    const dim3 grid(tokens, (heads + HEADS * QHH_WARPS - 1) / (HEADS * QHH_WARPS));                          \
-    if (dtype == DTYPE_F32) launch_dependent(qkv_halves_heads_kernel<float, HEADS>, grid, dim3(QHH_WARPS * 32), turn, s,      \
-        false, a);                                                                                                            \
-    else launch_dependent(qkv_halves_heads_kernel<__nv_bfloat16, HEADS>, grid, dim3(QHH_WARPS * 32), turn, s, false, a);      \
+    const dim3 grid(tokens, (heads + HEADS * (QHH_WARPS * 32 / LANES) - 1) / (HEADS * (QHH_WARPS * 32 / LANES)));             \
+    if (dtype == DTYPE_F32) launch_dependent(qkv_halves_heads_kernel<float, LANES, HEADS>, grid, dim3(QHH_WARPS * 32), turn,  \
+        s, false, a);                                                                                                         \
+    else launch_dependent(qkv_halves_heads_kernel<__nv_bfloat16, LANES, HEADS>, grid, dim3(QHH_WARPS * 32), turn, s, false, a); \
   }
-      if (many) ZB_QHH(4) else ZB_QHH(1)
+      if (widest <= 64) { ZB_QHH(8, 1) }
+      else if (many) ZB_QHH(16, 2)
+      else ZB_QHH(16, 1)
 #undef ZB_QHH
       return launch_result();
     }
