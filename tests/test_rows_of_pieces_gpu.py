@@ -151,6 +151,28 @@ def test_few_rows_at_the_splits_of_k(cuda_device, N, K, M):
         assert (hidden.double() - want).abs().max() <= 40 * 2.0 ** -24 * max(16.0, K ** 0.5)
 
 
+@pytest.mark.parametrize("N,K", [(1528, 2048), (1536, 2056), (2376, 1000), (4720, 4088), (6416, 520), (9488, 40), (9480, 3080), (23680, 1032)])
+@pytest.mark.parametrize("M", [1, 9, 17])
+def test_few_rows_streamed(cuda_device, N, K, M):
+    """Around the sizes from which a persistent kernel streams the matrix, also where K ends inside a block or is less than one a
+    slice: as exact as the tests above ask, each row alone in the same sums, and the activations behind them."""
+    from zephyr_b200.kernels import ops
+
+    g = torch.Generator(device=cuda_device).manual_seed(N + K + M)
+    x = torch.randn(M, K + 8, generator=g, device=cuda_device).to(torch.bfloat16)[:, 8:]
+    w = (torch.randn(N, K, generator=g, device=cuda_device) / K ** 0.5).to(torch.bfloat16)
+    got, want = ops.gemm_small(x, w, out_dtype=torch.float32), x.double() @ w.double().T
+    assert (got.double() - want).abs().max() <= 6 * 2.0 ** -24 * max(16.0, K ** 0.5)
+    assert torch.equal(ops.gemm_small(x[M - 1:], w, out_dtype=torch.float32), got[M - 1:])
+    assert torch.equal(ops.gemm_small(x, w), got.to(torch.bfloat16))
+    many = torch.cat([x, x, x, x[:1]] * (1 if M > 9 else 3))[:64]           # through the other kernel where the x of 33 rows and more lies
+    assert torch.equal(ops.gemm_small(many, w, out_dtype=torch.float32)[:M], got)
+    if N % 16 == 0:
+        pair = got.view(M, N // 16, 2, 8)
+        gated = ops.gemm_small(x, w, out_dtype=torch.float32, swiglu=True).view(M, N // 16, 8)
+        assert (gated - torch.nn.functional.silu(pair[:, :, 0]) * pair[:, :, 1]).abs().max() <= 2.0 ** -21 * max(1.0, float(got.abs().max())) ** 2
+
+
 @pytest.mark.parametrize("tokens,heads,kv_heads,kd,vd,rot", [(64, 24, 8, 64, 64, 64), (63, 5, 3, 64, 40, 32), (70, 3, 1, 8, 8, 8), (64, 17, 3, 128, 72, 128),
                                                              (700, 31, 5, 88, 128, 40), (2, 1, 1, 56, 64, 24)])
 @pytest.mark.parametrize("pairs", [True, False])

@@ -8,10 +8,10 @@
 // consecutive values k = 8t .. 8t+7 of its row: one 16-byte load feeds two tensor-core products.
 // The products see k in a permuted order, the same for both operands, so the sum is unchanged.
 //
-// One CTA owns 16 rows of W (or 32); its warps split K, and for matrices with few rows a cluster of
+// One CTA owns 16 rows of W; its warps split K, and for matrices with few rows a cluster of
 // up to 8 CTAs splits K further.  A decode step's product is bound by latency before it is by bandwidth: a warp has the loads
-// of several blocks of 32 k in flight, whatever is left of its slice: four up to 16 rows, two from 17 to 32 and where a CTA takes
-// 32 rows of W; above 32 rows four blocks of W alone, x at its use (with x ahead too, two blocks: 12288 x 4096, 64 rows: 92 us,
+// of several blocks of 32 k in flight, whatever is left of its slice: four up to 16 rows, two from 17 to 32;
+// above 32 rows four blocks of W alone, x at its use (with x ahead too, two blocks: 12288 x 4096, 64 rows: 92 us,
 // now 47; 6144 x 2048: 29 and 17) (one block after the other, as a loop's remainder, 2048 x
 // 6144 with 12 rows took 13.8 us; now 10.1, its bytes 3.8), and the CTAs of a cluster each finish a share of the tile with one
 // round of remote reads (one CTA for all, 2048 x 2048: 9.8 us; now 6.1).  4096 x 2048: 10.2 -> 7.9, 12288 x 2048: 14.9 -> 14.1,
@@ -19,8 +19,11 @@
 // a fixed order, so the result does not depend on timing.  ACT takes each sum through GELU's tanh form, a
 // squared ReLU, or GELU times a value of the token's row of a table.  With SWIGLU the 16 rows are 8 gate
 // rows followed by their 8 up rows, and the epilogue writes silu(gate) * up: the activation costs
-// no extra pass over memory (reference: src/layer/mlp.cpp:29-36, src/layer/activation.cu:31-33).
+// no extra pass over memory (reference: src/layer/mlp.cpp:29-36, src/layer/activation.cu:31-33).  Matrices of many rows, and
+// from 9 tokens on most, go through a persistent form with the same sums, gemm_small_stream_kernel below.
 #include <cooperative_groups.h>
+
+#include <algorithm>
 
 #include "common.cuh"
 #include "mma.cuh"
@@ -33,6 +36,8 @@ constexpr int ACT_TOKEN_GATE = 3;
 constexpr int GS_MAX_MT = 8;      // token tiles of 8: M <= 64
 constexpr int GS_MAX_KSPLIT = 8;
 constexpr int GS_FETCH_AHEAD_CTAS = 4 * 148;
+constexpr int GS_STREAM_WARPS = 16;
+constexpr size_t GS_STREAM_SMEM = 226 * 1024;
 
 struct SmallGemmArgs {
   void* y;
@@ -54,34 +59,76 @@ __device__ __forceinline__ uint4 load16_or_zero(const __nv_bfloat16* p, bool ok)
   return ok ? *reinterpret_cast<const uint4*>(p) : make_uint4(0, 0, 0, 0);
 }
 
+__device__ __forceinline__ void copy16_or_zero(unsigned to, const __nv_bfloat16* p, bool ok) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(to), "l"(p), "r"(ok ? 16 : 0) : "memory");
+}
+
 template <typename T> __device__ __forceinline__ void store_out(T* p, float v);
 template <> __device__ __forceinline__ void store_out<float>(float* p, float v) { *p = v; }
 template <> __device__ __forceinline__ void store_out<__nv_bfloat16>(__nv_bfloat16* p, float v) {
   *p = __float2bfloat16_rn(v);
 }
 
-template <int RT, int WARPS, int MT, typename TOut, bool SWIGLU, int ACT>
+// A tile's results from its sums: total_of(e) is the sum of entry e of [mt][row][token].
+template <int MT, typename TOut, bool SWIGLU, int ACT, typename Total>
+__device__ __forceinline__ void small_gemm_finish(const SmallGemmArgs& a, int n0, int first, int step, const Total& total_of) {
+  TOut* y = static_cast<TOut*>(a.y);
+  for (int i = first; i < MT * (SWIGLU ? 64 : 128); i += step) {
+    const int r = (i / 8) % (SWIGLU ? 8 : 16), mt = i / (SWIGLU ? 64 : 128);
+    const int token = mt * 8 + i % 8, row = n0 + r;
+    if (token >= a.M) continue;
+    if (SWIGLU) {                          // rows 0..7 of a tile are gate rows, rows 8..15 the matching up rows
+      if (row + 8 >= a.N) continue;
+      float gate = total_of(mt * 128 + r * 8 + i % 8), up = total_of(mt * 128 + 64 + r * 8 + i % 8), v;
+      if (a.gate.kind == GATE_BOUNDED) {
+        if (a.gate.bias != nullptr) {
+          gate += a.gate.bias[row];
+          up += a.gate.bias[row + 8];
+        }
+        v = bounded_gate<false>(gate, up, a.gate);
+      } else {
+        v = (a.gate.kind == GATE_RELU ? fmaxf(gate, 0.0f) : gate / (1.0f + expf(-gate))) * up;
+      }
+      store_out<TOut>(y + static_cast<size_t>(token) * a.ldy + n0 / 2 + r, v);
+    } else {
+      if (row >= a.N) continue;
+      const float sum = total_of(i);
+      TOut* at = y + static_cast<size_t>(token) * a.ldy + static_cast<size_t>(row) * a.ldn;
+      if (ACT == ACT_TOKEN_GATE) {
+        const int id = a.token_ids[token];
+        const bool ok = id >= 0 && id < a.vocab;
+        if (!ok && row == 0) report(a.status, STATUS_TOKEN_OUT_OF_RANGE, id, token);
+        const float e = ok ? __bfloat162float(a.token_rows[static_cast<long long>(id) * a.token_stride + row]) : 0.0f;
+        store_out<TOut>(at, gelu_tanh(sum) * e);
+      } else {
+        store_out<TOut>(at, ACT == ACT_GELU ? gelu_tanh(sum) : ACT == ACT_RELU2 ? relu_squared(sum) : sum);
+      }
+    }
+  }
+}
+
+template <int WARPS, int MT, typename TOut, bool SWIGLU, int ACT>
 __global__ void __launch_bounds__(WARPS * 32)
 gemm_small_kernel(const SmallGemmArgs a) {
   constexpr bool X_AHEAD = MT <= 4;                 // (eight tiles of tokens ahead leave room for two blocks of W)
-  constexpr int U = (RT == 1 && MT <= 2) || !X_AHEAD ? 4 : 2;     // blocks of k in flight
-  constexpr int PER_WARP = RT * MT * 16 * 8;        // sums of a warp: [rt][mt][row][token]
+  constexpr int U = MT <= 2 || !X_AHEAD ? 4 : 2;     // blocks of k in flight
+  constexpr int PER_WARP = MT * 16 * 8;             // sums of a warp: [mt][row][token]
   __shared__ float red[WARPS][PER_WARP];
   cg::cluster_group cluster = cg::this_cluster();
   const int ksplit = gridDim.y, krank = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int n0 = blockIdx.x * (16 * RT);
+  const int n0 = blockIdx.x * 16;
 
   const int total_blocks = (a.K + 31) / 32;
   const int slices = WARPS * ksplit, slice = krank * WARPS + warp;
   const int b_begin = static_cast<int>(static_cast<long long>(total_blocks) * slice / slices);
   const int b_end = static_cast<int>(static_cast<long long>(total_blocks) * (slice + 1) / slices);
 
-  bool w_ok[2 * RT];
-  const __nv_bfloat16* w_row[2 * RT];
+  bool w_ok[2];
+  const __nv_bfloat16* w_row[2];
 #pragma unroll
-  for (int r = 0; r < 2 * RT; ++r) {
+  for (int r = 0; r < 2; ++r) {
     w_ok[r] = n0 + g + 8 * r < a.N;
     w_row[r] = a.w + static_cast<size_t>(w_ok[r] ? n0 + g + 8 * r : 0) * a.ldw + 8 * t;
   }
@@ -101,58 +148,49 @@ gemm_small_kernel(const SmallGemmArgs a) {
     const int row = n0 + lane % 16;
     const char* line = reinterpret_cast<const char*>(a.w + static_cast<size_t>(row) * a.ldw + b_begin * 32) + 128 * (lane / 16);
     const int bytes = (min(b_end * 32, a.K) - b_begin * 32) * 2;
-#pragma unroll
-    for (int rt = 0; rt < RT; ++rt)
-      for (int at = 128 * (lane / 16); at < bytes; at += 256)
-        if (row + 16 * rt < a.N)
-          asm volatile("prefetch.global.L2 [%0];\n" ::"l"(line + static_cast<size_t>(rt) * 16 * a.ldw * 2 + (at - 128 * (lane / 16))));
+    for (int at = 128 * (lane / 16); at < bytes; at += 256)
+      if (row < a.N) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(line + (at - 128 * (lane / 16))));
   }
   wait_for_prior_grids();
   let_dependents_launch();
 
-  float acc[RT][MT][4];
+  float acc[MT][4];
 #pragma unroll
-  for (int rt = 0; rt < RT; ++rt)
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt) acc[rt][mt][0] = acc[rt][mt][1] = acc[rt][mt][2] = acc[rt][mt][3] = 0.0f;
+  for (int mt = 0; mt < MT; ++mt) acc[mt][0] = acc[mt][1] = acc[mt][2] = acc[mt][3] = 0.0f;
 
   for (int b = b_begin; b < b_end; b += U) {
-    uint4 wv[U][2 * RT], xv[X_AHEAD ? U : 1][X_AHEAD ? MT : 1];
+    uint4 wv[U][2], xv[X_AHEAD ? U : 1][X_AHEAD ? MT : 1];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int k = (b + u) * 32;
       const bool k_ok = b + u < b_end && k + 8 * t + 8 <= a.K;      // K is a multiple of 8: a chunk is whole or absent
 #pragma unroll
-      for (int r = 0; r < 2 * RT; ++r) wv[u][r] = load16_or_zero(w_row[r] + k, w_ok[r] && k_ok);
+      for (int r = 0; r < 2; ++r) wv[u][r] = load16_or_zero(w_row[r] + k, w_ok[r] && k_ok);
 #pragma unroll
       for (int mt = 0; X_AHEAD && mt < MT; ++mt) xv[u][mt] = load16_or_zero(x_row[mt] + k, x_ok[mt] && k_ok);
     }
 #pragma unroll
-    for (int u = 0; u < U; ++u)
+    for (int u = 0; u < U; ++u) {
+      const uint4 wl = wv[u][0], wh = wv[u][1];
+      const unsigned a0[4] = {wl.x, wh.x, wl.y, wh.y};
+      const unsigned a1[4] = {wl.z, wh.z, wl.w, wh.w};
 #pragma unroll
-      for (int rt = 0; rt < RT; ++rt) {
-        const uint4 wl = wv[u][2 * rt], wh = wv[u][2 * rt + 1];
-        const unsigned a0[4] = {wl.x, wh.x, wl.y, wh.y};
-        const unsigned a1[4] = {wl.z, wh.z, wl.w, wh.w};
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt) {
-          const int k = (b + u) * 32;
-          const uint4 x = X_AHEAD ? xv[X_AHEAD ? u : 0][X_AHEAD ? mt : 0]
-                                  : load16_or_zero(x_row[mt] + k, x_ok[mt] && b + u < b_end && k + 8 * t + 8 <= a.K);
-          mma_bf16_16816(acc[rt][mt], a0, x.x, x.y);
-          mma_bf16_16816(acc[rt][mt], a1, x.z, x.w);
-        }
+      for (int mt = 0; mt < MT; ++mt) {
+        const int k = (b + u) * 32;
+        const uint4 x = X_AHEAD ? xv[X_AHEAD ? u : 0][X_AHEAD ? mt : 0]
+                                : load16_or_zero(x_row[mt] + k, x_ok[mt] && b + u < b_end && k + 8 * t + 8 <= a.K);
+        mma_bf16_16816(acc[mt], a0, x.x, x.y);
+        mma_bf16_16816(acc[mt], a1, x.z, x.w);
       }
+    }
   }
 
 #pragma unroll
-  for (int rt = 0; rt < RT; ++rt)
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
-      float* at = &red[warp][(rt * MT + mt) * 128 + g * 8 + 2 * t];
-      *reinterpret_cast<float2*>(at) = make_float2(acc[rt][mt][0], acc[rt][mt][1]);
-      *reinterpret_cast<float2*>(at + 64) = make_float2(acc[rt][mt][2], acc[rt][mt][3]);
-    }
+  for (int mt = 0; mt < MT; ++mt) {
+    float* at = &red[warp][mt * 128 + g * 8 + 2 * t];
+    *reinterpret_cast<float2*>(at) = make_float2(acc[mt][0], acc[mt][1]);
+    *reinterpret_cast<float2*>(at + 64) = make_float2(acc[mt][2], acc[mt][3]);
+  }
   __syncthreads();
   // A CTA adds its warps' sums in their order; a cluster's CTAs each finish a share of the tile from the sums of all, in
   // the CTAs' order, which lie in (distributed) shared memory.
@@ -181,50 +219,164 @@ gemm_small_kernel(const SmallGemmArgs a) {
     }
     return sum;
   };
-  TOut* y = static_cast<TOut*>(a.y);
-  for (int i = krank * WARPS * 32 + threadIdx.x; i < (SWIGLU ? PER_WARP / 2 : PER_WARP); i += ksplit * WARPS * 32) {
-    const int r = (i / 8) % (SWIGLU ? 8 : 16), tile = i / (SWIGLU ? 64 : 128), mt = tile % MT, rt = tile / MT;
-    const int token = mt * 8 + i % 8, row = n0 + 16 * rt + r;
-    if (token >= a.M) continue;
-    if (SWIGLU) {                          // rows 0..7 of a tile are gate rows, rows 8..15 the matching up rows
-      if (row + 8 >= a.N) continue;
-      float gate = total_of(tile * 128 + r * 8 + i % 8), up = total_of(tile * 128 + 64 + r * 8 + i % 8), v;
-      if (a.gate.kind == GATE_BOUNDED) {
-        if (a.gate.bias != nullptr) {
-          gate += a.gate.bias[row];
-          up += a.gate.bias[row + 8];
-        }
-        v = bounded_gate<false>(gate, up, a.gate);
-      } else {
-        v = (a.gate.kind == GATE_RELU ? fmaxf(gate, 0.0f) : gate / (1.0f + expf(-gate))) * up;
-      }
-      store_out<TOut>(y + static_cast<size_t>(token) * a.ldy + (blockIdx.x * RT + rt) * 8 + r, v);
-    } else {
-      if (row >= a.N) continue;
-      const float sum = total_of(i);
-      TOut* at = y + static_cast<size_t>(token) * a.ldy + static_cast<size_t>(row) * a.ldn;
-      if (ACT == ACT_TOKEN_GATE) {
-        const int id = a.token_ids[token];
-        const bool ok = id >= 0 && id < a.vocab;
-        if (!ok && row == 0) report(a.status, STATUS_TOKEN_OUT_OF_RANGE, id, token);
-        const float e = ok ? __bfloat162float(a.token_rows[static_cast<long long>(id) * a.token_stride + row]) : 0.0f;
-        store_out<TOut>(at, gelu_tanh(sum) * e);
-      } else {
-        store_out<TOut>(at, ACT == ACT_GELU ? gelu_tanh(sum) : ACT == ACT_RELU2 ? relu_squared(sum) : sum);
-      }
+  small_gemm_finish<MT, TOut, SWIGLU, ACT>(a, n0, krank * WARPS * 32 + threadIdx.x, ksplit * WARPS * 32, total_of);
+  if (ksplit > 1) cluster.sync();           // nobody leaves while its shared memory may still be read
+}
+
+// The same sums with one CTA an SM that walks the tiles of 16 rows: a team of its 16 warps (SLICES of them, at most all) shares a
+// tile, a warp one slice of K or SLICES / 16 of them, added in the order in which the kernel above adds its warps and its
+// cluster's CTAs.  That kernel is bound by its waits: a warp asks for four blocks of k, waits for all of them and only then
+// asks for more, and every tile fetches the few rows of x from L2 again, as many bytes as the tile has from 16 rows on.  Here x
+// lies in shared memory once an SM, as fragments, and a warp's blocks pass through a ring of DEPTH of them that a lane fills
+// with asynchronous copies of just the 16 bytes it will use itself, so that nobody has to be told of their arrival and 64 to
+// 128 KB an SM are on their way all the time, also from one tile to the next (through registers, four blocks ahead, 32768 x
+// 2048 with 12 rows took 28.1 us).  In us, the kernel above and this one (TB/s): 32768 x 2048, 1 row 25.5 and 22.2 (6.0),
+// 12 rows 33.2 and 24.7 (5.4), 32 rows 44 and 29.8; 16384 x 2048, 8 rows 19.3 and 12.3, 12 rows 16.5 and 13.5; 24576 x 4096,
+// 12 rows 46 and 38.4; 151936 x 1024, 12 rows 67 and 52 (6.0), one row 50.3 (with 32 rows a CTA) and 49.7.
+template <int SLICES, int DEPTH, int MT, typename TOut, bool SWIGLU, int ACT>
+__global__ void __launch_bounds__(GS_STREAM_WARPS * 32, 1)
+gemm_small_stream_kernel(const SmallGemmArgs a) {
+  constexpr int TEAM = SLICES < GS_STREAM_WARPS ? SLICES : GS_STREAM_WARPS, TEAMS = GS_STREAM_WARPS / TEAM;
+  constexpr int PER_WARP = SLICES / TEAM, GROUP = SLICES < 8 ? SLICES : 8, SUMS = MT * 128;
+  extern __shared__ __align__(16) unsigned char gs_smem[];
+  const int blocks = (a.K + 31) / 32;
+  uint4* x_s = reinterpret_cast<uint4*>(gs_smem);                                  // [block of k][mt][lane]: fragments
+  float* red = reinterpret_cast<float*>(x_s + static_cast<size_t>(blocks) * MT * 32);      // [team][slice][SUMS]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, team = warp / TEAM;
+  uint4* ring = reinterpret_cast<uint4*>(red + TEAMS * SLICES * SUMS) + warp * DEPTH * 64 + lane;   // [warps][DEPTH][2][lane]
+  const int g = lane >> 2, t = lane & 3;
+  const int first_slice = warp % TEAM * PER_WARP;
+  auto slice_begin = [&](int i) { return blocks * i / SLICES; };
+  const int b_begin = slice_begin(first_slice), b_end = slice_begin(first_slice + PER_WARP);
+  const int tiles = (a.N + 15) / 16, first_tile = team * gridDim.x + blockIdx.x, tile_step = TEAMS * gridDim.x;
+
+  // While the kernel before this one still runs: the team's first tile, as far as L2 (as above).
+  {
+    const int row = first_tile * 16 + lane % 16;
+    if (row < a.N) {
+      const char* line = reinterpret_cast<const char*>(a.w + static_cast<size_t>(row) * a.ldw + b_begin * 32);
+      const int bytes = (min(b_end * 32, a.K) - b_begin * 32) * 2;
+      for (int at = 128 * (lane / 16); at < bytes; at += 256) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(line + at));
     }
   }
-  if (ksplit > 1) cluster.sync();           // nobody leaves while its shared memory may still be read
+  wait_for_prior_grids();
+  let_dependents_launch();
+
+  // Cursor of the copies: `ahead` blocks in front of the products, across the team's tiles.
+  int c_tile = first_tile, c_b = b_begin, c_slot = 0;
+  const __nv_bfloat16 *lo, *hi;
+  bool lo_ok, hi_ok;
+  auto rows_of = [&]() {
+    const int row = c_tile * 16 + g;
+    lo_ok = c_tile < tiles && row < a.N;
+    hi_ok = c_tile < tiles && row + 8 < a.N;
+    lo = a.w + static_cast<size_t>(lo_ok ? row : 0) * a.ldw;
+    hi = a.w + static_cast<size_t>(hi_ok ? row + 8 : 0) * a.ldw;
+  };
+  rows_of();
+  const unsigned ring_at = smem_u32(ring);
+  auto copy_next = [&]() {
+    const int k = c_b * 32 + 8 * t;
+    const bool k_ok = k + 8 <= a.K;
+    copy16_or_zero(ring_at + c_slot * 1024, lo + (k_ok ? k : 0), lo_ok && k_ok);
+    copy16_or_zero(ring_at + c_slot * 1024 + 512, hi + (k_ok ? k : 0), hi_ok && k_ok);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    c_slot = c_slot + 1 == DEPTH ? 0 : c_slot + 1;
+    if (++c_b >= b_end) {
+      c_b = b_begin;
+      c_tile += tile_step;
+      rows_of();
+    }
+  };
+#pragma unroll
+  for (int u = 0; u < DEPTH; ++u) copy_next();
+  for (int e = threadIdx.x; e < blocks * MT * 32; e += GS_STREAM_WARPS * 32) {
+    const int k = e / (MT * 32) * 32 + 8 * (e % 4), m = e / 32 % MT * 8 + e % 32 / 4;
+    x_s[e] = load16_or_zero(a.x + static_cast<size_t>(m < a.M ? m : 0) * a.ldx + k, m < a.M && k + 8 <= a.K);
+  }
+  __syncthreads();
+
+  auto team_barrier = [&]() { asm volatile("bar.sync %0, %1;\n" ::"r"(1 + team), "n"(TEAM * 32) : "memory"); };
+  int slot = 0;
+  for (int tile = first_tile; tile < tiles; tile += tile_step) {
+    if (tile != first_tile) team_barrier();               // the tile before has been read
+    int b = b_begin;
+#pragma unroll 1
+    for (int i = 0; i < PER_WARP; ++i) {
+      const int slice = first_slice + i;
+      float acc[MT][4];
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) acc[mt][0] = acc[mt][1] = acc[mt][2] = acc[mt][3] = 0.0f;
+      const int end = slice_begin(slice + 1);
+#pragma unroll 2
+      for (; b < end; ++b) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(DEPTH - 1) : "memory");
+        const uint4 wl = ring[slot * 64], wh = ring[slot * 64 + 32];
+        slot = slot + 1 == DEPTH ? 0 : slot + 1;
+        const unsigned a0[4] = {wl.x, wh.x, wl.y, wh.y}, a1[4] = {wl.z, wh.z, wl.w, wh.w};
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+          const uint4 x = x_s[(b * MT + mt) * 32 + lane];
+          mma_bf16_16816(acc[mt], a0, x.x, x.y);
+          mma_bf16_16816(acc[mt], a1, x.z, x.w);
+        }
+        copy_next();
+      }
+      float* mine = red + (team * SLICES + slice) * SUMS;
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) {
+        float* at = mine + mt * 128 + g * 8 + 2 * t;
+        *reinterpret_cast<float2*>(at) = make_float2(acc[mt][0], acc[mt][1]);
+        *reinterpret_cast<float2*>(at + 64) = make_float2(acc[mt][2], acc[mt][3]);
+      }
+    }
+    team_barrier();
+    const float* all = red + team * SLICES * SUMS;
+    small_gemm_finish<MT, TOut, SWIGLU, ACT>(a, tile * 16, threadIdx.x % (TEAM * 32), TEAM * 32, [&](int e) {
+      float total = 0.0f;                                 // the sums of eight slices in order, then those
+#pragma unroll
+      for (int s0 = 0; s0 < SLICES; s0 += GROUP) {
+        float sum = all[s0 * SUMS + e];
+#pragma unroll
+        for (int i = 1; i < GROUP; ++i) sum += all[(s0 + i) * SUMS + e];
+        total = s0 == 0 ? sum : total + sum;
+      }
+      return total;
+    });
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+}
+
+// The streaming kernel's shared memory but for its rings: x, and the slices' sums.
+static size_t small_gemm_stream_fixed(int K, int token_tiles, int slices) {
+  const int teams = slices < GS_STREAM_WARPS ? GS_STREAM_WARPS / slices : 1;
+  return (static_cast<size_t>((K + 31) / 32) + static_cast<size_t>(teams) * slices) * token_tiles * 512;
 }
 
 struct SmallGemmSplit {
   int warps, ksplit;           // of a CTA; CTAs that share K
 };
+
+// Whether the streaming kernel takes a product (its sums are the other kernel's, so that this may look at the number of rows):
+// always from more than four CTAs an SM on; below where its whole rounds of SMs and its one start a product are less than
+// what the other kernel loses to its waits.  Row by row of x in us, the other kernel and this one (matrices from memory,
+// launched one behind the other): 2048 x 2048, 8 rows 4.4 and 4.6, 12 rows 7.2 and 5.4; 1024 x 2048, 12 rows 3.7 and 4.8; 4096 x
+// 4096, 8 rows 9.1 and 9.5, 12 rows 11.9 and 9.2; 4736 x 2048, 12 rows 5.4 and 7.3 (exactly two CTAs an SM of the other), 32
+// rows 11.1 and 8.4; 8192 x 2048, 8 rows 7.7 and 8.2, 12 rows 9.3 and 9.0, 32 rows 13.9 and 11.0; 8192 x 4096, 8 rows 15.9 and
+// 13.2, 12 rows 18.2 and 15.2.
+static bool small_gemm_streams(int N, int K, int token_tiles, const SmallGemmSplit& s) {
+  const int tiles = (N + 15) / 16, slices = s.warps * s.ksplit;
+  if (slices > 32 || small_gemm_stream_fixed(K, token_tiles, slices) + 4 * 1024 * GS_STREAM_WARPS > GS_STREAM_SMEM) return false;
+  if (tiles > 4 * 148) return true;
+  if (token_tiles == 1) return tiles > 2 * 148 && K >= 3072;
+  if (token_tiles == 2) return tiles >= 96 && (tiles < 2 * 148 || tiles > 400);
+  return tiles > 200;
+}
 // How K is cut, from the matrix alone: a row's sums are the same whatever rows it is computed with.  Eight warps a CTA and, up
 // to two CTAs an SM, a cluster that shares K (a power of two up to 8, two blocks of k a warp or more): with every warp's loads
 // in flight at once the latency of the last one, not the split, is what is left.  Above four such CTAs an SM a second wave
 // begins, and four warps are the better CTA (32768 x 2048, 12 rows: 29.8 us against 33.4) until K gives each of them more
-// than 32 blocks to walk (24576 x 4096: 56 us against 45).
+// than 32 blocks to walk (24576 x 4096: 56 us against 45); the streaming kernel, which takes most of those, keeps the cut.
 static SmallGemmSplit small_gemm_split(int N, int K) {
   const int tiles = (N + 15) / 16, blocks = (K + 31) / 32;
   if (tiles > 4 * 148) return {blocks >= 128 ? 8 : 4, 1};
@@ -233,10 +385,10 @@ static SmallGemmSplit small_gemm_split(int N, int K) {
   return {8, ksplit};
 }
 
-template <int RT, int WARPS, int MT, typename TOut, bool SWIGLU, int ACT>
+template <int WARPS, int MT, typename TOut, bool SWIGLU, int ACT>
 int small_gemm_launch(const SmallGemmArgs& a, int ksplit, cudaStream_t stream) {
   cudaLaunchConfig_t config = {};
-  config.gridDim = dim3((a.N + 16 * RT - 1) / (16 * RT), ksplit, 1);
+  config.gridDim = dim3((a.N + 15) / 16, ksplit, 1);
   config.blockDim = dim3(WARPS * 32, 1, 1);
   config.dynamicSmemBytes = 0;
   config.stream = stream;
@@ -249,18 +401,44 @@ int small_gemm_launch(const SmallGemmArgs& a, int ksplit, cudaStream_t stream) {
   attribute[1].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attribute;
   config.numAttrs = dependent_launch_enabled() ? 2 : 1;
-  if (cudaLaunchKernelEx(&config, gemm_small_kernel<RT, WARPS, MT, TOut, SWIGLU, ACT>, a) != cudaSuccess) return ERR_CUDA;
+  if (cudaLaunchKernelEx(&config, gemm_small_kernel<WARPS, MT, TOut, SWIGLU, ACT>, a) != cudaSuccess) return ERR_CUDA;
   return launch_result();
+}
+
+template <int SLICES, int MT, typename TOut, bool SWIGLU, int ACT>
+int small_gemm_stream_launch(const SmallGemmArgs& a, cudaStream_t stream) {
+  const size_t fixed = small_gemm_stream_fixed(a.K, MT, SLICES), slot = 1024 * GS_STREAM_WARPS;
+  const bool deep = fixed + 8 * slot <= GS_STREAM_SMEM;
+  const size_t smem = fixed + (deep ? 8 : 4) * slot;
+  const dim3 grid(std::min(148, (a.N + 15) / 16)), block(GS_STREAM_WARPS * 32);
+  auto allow = [&](auto kernel) {
+    return !cuda_failed(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  };
+  if (deep) {
+    if (!allow(gemm_small_stream_kernel<SLICES, 8, MT, TOut, SWIGLU, ACT>)) return ERR_CUDA;
+    return launch_dependent(gemm_small_stream_kernel<SLICES, 8, MT, TOut, SWIGLU, ACT>, grid, block, smem, stream, false, a);
+  }
+  if (!allow(gemm_small_stream_kernel<SLICES, 4, MT, TOut, SWIGLU, ACT>)) return ERR_CUDA;
+  return launch_dependent(gemm_small_stream_kernel<SLICES, 4, MT, TOut, SWIGLU, ACT>, grid, block, smem, stream, false, a);
 }
 
 template <int MT, typename TOut, bool SWIGLU, int ACT>
 int small_gemm_split_launch(const SmallGemmArgs& a, cudaStream_t stream) {
   const SmallGemmSplit s = small_gemm_split(a.cut_rows, a.K);
-  if (s.warps == 8) return small_gemm_launch<1, 8, MT, TOut, SWIGLU, ACT>(a, s.ksplit, stream);
-  // Up to 8 tokens and several waves of CTAs: 32 rows a CTA read the tokens half as often (151936 x 1024, 4 rows: 50 us
-  // against 54; with 12 rows their registers cost more, 66 against 64).  The sums are the same.
-  if (MT == 1) return small_gemm_launch<2, 4, 1, TOut, SWIGLU, ACT>(a, s.ksplit, stream);
-  return small_gemm_launch<1, 4, MT, TOut, SWIGLU, ACT>(a, s.ksplit, stream);
+  if constexpr (MT <= 4) {
+    if (small_gemm_streams(a.cut_rows, a.K, MT, s)) {
+      const int slices = s.warps * s.ksplit;
+      if (slices == 4) return small_gemm_stream_launch<4, MT, TOut, SWIGLU, ACT>(a, stream);
+      if constexpr (MT > 1)
+        if (slices == 16) return small_gemm_stream_launch<16, MT, TOut, SWIGLU, ACT>(a, stream);
+      if constexpr (MT == 2)
+        if (slices == 32) return small_gemm_stream_launch<32, MT, TOut, SWIGLU, ACT>(a, stream);
+      return small_gemm_stream_launch<8, MT, TOut, SWIGLU, ACT>(a, stream);
+    }
+  }
+  if constexpr (MT > 2)       // (up to 16 rows, the x of a K that four warps cut finds room in the streaming kernel)
+    if (s.warps == 4) return small_gemm_launch<4, MT, TOut, SWIGLU, ACT>(a, s.ksplit, stream);
+  return small_gemm_launch<8, MT, TOut, SWIGLU, ACT>(a, s.ksplit, stream);
 }
 
 template <typename TOut, bool SWIGLU, int ACT>
