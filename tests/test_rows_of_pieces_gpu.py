@@ -151,7 +151,7 @@ def test_few_rows_at_the_splits_of_k(cuda_device, N, K, M):
         assert (hidden.double() - want).abs().max() <= 40 * 2.0 ** -24 * max(16.0, K ** 0.5)
 
 
-@pytest.mark.parametrize("N,K", [(1528, 2048), (1536, 2056), (2376, 1000), (4720, 4088), (6416, 520), (9488, 40), (9480, 3080), (23680, 1032)])
+@pytest.mark.parametrize("N,K", [(1528, 2048), (1536, 2056), (2376, 1000), (4720, 4088), (6416, 520), (9488, 40), (9480, 3080), (23680, 1032), (2384, 8200)])
 @pytest.mark.parametrize("M", [1, 9, 17])
 def test_few_rows_streamed(cuda_device, N, K, M):
     """Around the sizes from which a persistent kernel streams the matrix, also where K ends inside a block or is less than one a

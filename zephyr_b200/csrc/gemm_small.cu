@@ -230,20 +230,23 @@ gemm_small_kernel(const SmallGemmArgs a) {
 // lies in shared memory once an SM, as fragments, and a warp's blocks pass through a ring of DEPTH of them that a lane fills
 // with asynchronous copies of just the 16 bytes it will use itself, so that nobody has to be told of their arrival and 64 to
 // 128 KB an SM are on their way all the time, also from one tile to the next (through registers, four blocks ahead, 32768 x
-// 2048 with 12 rows took 28.1 us).  In us, the kernel above and this one (TB/s): 32768 x 2048, 1 row 25.5 and 22.2 (6.0),
+// 2048 with 12 rows took 28.1 us).  With X_RING, where x and four blocks a warp are more than shared memory, the rings bring
+// x's pieces beside W's.  In us, the kernel above and this one (TB/s): 32768 x 2048, 1 row 25.5 and 22.2 (6.0),
 // 12 rows 33.2 and 24.7 (5.4), 32 rows 44 and 29.8; 16384 x 2048, 8 rows 19.3 and 12.3, 12 rows 16.5 and 13.5; 24576 x 4096,
-// 12 rows 46 and 38.4; 151936 x 1024, 12 rows 67 and 52 (6.0), one row 50.3 (with 32 rows a CTA) and 49.7.
-template <int SLICES, int DEPTH, int MT, typename TOut, bool SWIGLU, int ACT>
+// 12 rows 46 and 38.4; 151936 x 1024, 12 rows 67 and 52 (6.0), one row 50.3 (with 32 rows a CTA) and 49.7; with X_RING 2048 x 8192, 12
+// rows 12.1 and 9.6, 12288 x 4096, 32 rows 47.6 and 28.5.
+template <int SLICES, int DEPTH, bool X_RING, int MT, typename TOut, bool SWIGLU, int ACT>
 __global__ void __launch_bounds__(GS_STREAM_WARPS * 32, 1)
 gemm_small_stream_kernel(const SmallGemmArgs a) {
   constexpr int TEAM = SLICES < GS_STREAM_WARPS ? SLICES : GS_STREAM_WARPS, TEAMS = GS_STREAM_WARPS / TEAM;
   constexpr int PER_WARP = SLICES / TEAM, GROUP = SLICES < 8 ? SLICES : 8, SUMS = MT * 128;
+  constexpr int SLOT = X_RING ? 2 + MT : 2;       // 512-byte pieces of a ring's slot: two of W, with X_RING x's behind them
   extern __shared__ __align__(16) unsigned char gs_smem[];
   const int blocks = (a.K + 31) / 32;
   uint4* x_s = reinterpret_cast<uint4*>(gs_smem);                                  // [block of k][mt][lane]: fragments
-  float* red = reinterpret_cast<float*>(x_s + static_cast<size_t>(blocks) * MT * 32);      // [team][slice][SUMS]
+  float* red = reinterpret_cast<float*>(x_s + (X_RING ? 0 : static_cast<size_t>(blocks) * MT * 32));      // [team][slice][SUMS]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, team = warp / TEAM;
-  uint4* ring = reinterpret_cast<uint4*>(red + TEAMS * SLICES * SUMS) + warp * DEPTH * 64 + lane;   // [warps][DEPTH][2][lane]
+  uint4* ring = reinterpret_cast<uint4*>(red + TEAMS * SLICES * SUMS) + warp * DEPTH * SLOT * 32 + lane;   // [warps][DEPTH][SLOT][lane]
   const int g = lane >> 2, t = lane & 3;
   const int first_slice = warp % TEAM * PER_WARP;
   auto slice_begin = [&](int i) { return blocks * i / SLICES; };
@@ -278,8 +281,14 @@ gemm_small_stream_kernel(const SmallGemmArgs a) {
   auto copy_next = [&]() {
     const int k = c_b * 32 + 8 * t;
     const bool k_ok = k + 8 <= a.K;
-    copy16_or_zero(ring_at + c_slot * 1024, lo + (k_ok ? k : 0), lo_ok && k_ok);
-    copy16_or_zero(ring_at + c_slot * 1024 + 512, hi + (k_ok ? k : 0), hi_ok && k_ok);
+    const unsigned to = ring_at + c_slot * (SLOT * 512);
+    copy16_or_zero(to, lo + (k_ok ? k : 0), lo_ok && k_ok);
+    copy16_or_zero(to + 512, hi + (k_ok ? k : 0), hi_ok && k_ok);
+#pragma unroll
+    for (int mt = 0; X_RING && mt < MT; ++mt) {
+      const bool ok = mt * 8 + g < a.M && k_ok && c_tile < tiles;
+      copy16_or_zero(to + 1024 + mt * 512, a.x + (ok ? static_cast<size_t>(mt * 8 + g) * a.ldx + k : 0), ok);
+    }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
     c_slot = c_slot + 1 == DEPTH ? 0 : c_slot + 1;
     if (++c_b >= b_end) {
@@ -290,11 +299,11 @@ gemm_small_stream_kernel(const SmallGemmArgs a) {
   };
 #pragma unroll
   for (int u = 0; u < DEPTH; ++u) copy_next();
-  for (int e = threadIdx.x; e < blocks * MT * 32; e += GS_STREAM_WARPS * 32) {
+  for (int e = threadIdx.x; !X_RING && e < blocks * MT * 32; e += GS_STREAM_WARPS * 32) {
     const int k = e / (MT * 32) * 32 + 8 * (e % 4), m = e / 32 % MT * 8 + e % 32 / 4;
     x_s[e] = load16_or_zero(a.x + static_cast<size_t>(m < a.M ? m : 0) * a.ldx + k, m < a.M && k + 8 <= a.K);
   }
-  __syncthreads();
+  if (!X_RING) __syncthreads();
 
   auto team_barrier = [&]() { asm volatile("bar.sync %0, %1;\n" ::"r"(1 + team), "n"(TEAM * 32) : "memory"); };
   int slot = 0;
@@ -311,12 +320,13 @@ gemm_small_stream_kernel(const SmallGemmArgs a) {
 #pragma unroll 2
       for (; b < end; ++b) {
         asm volatile("cp.async.wait_group %0;\n" ::"n"(DEPTH - 1) : "memory");
-        const uint4 wl = ring[slot * 64], wh = ring[slot * 64 + 32];
+        const uint4* now = ring + slot * (SLOT * 32);
+        const uint4 wl = now[0], wh = now[32];
         slot = slot + 1 == DEPTH ? 0 : slot + 1;
         const unsigned a0[4] = {wl.x, wh.x, wl.y, wh.y}, a1[4] = {wl.z, wh.z, wl.w, wh.w};
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt) {
-          const uint4 x = x_s[(b * MT + mt) * 32 + lane];
+          const uint4 x = X_RING ? now[64 + mt * 32] : x_s[(b * MT + mt) * 32 + lane];
           mma_bf16_16816(acc[mt], a0, x.x, x.y);
           mma_bf16_16816(acc[mt], a1, x.z, x.w);
         }
@@ -347,10 +357,11 @@ gemm_small_stream_kernel(const SmallGemmArgs a) {
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
 }
 
-// The streaming kernel's shared memory but for its rings: x, and the slices' sums.
-static size_t small_gemm_stream_fixed(int K, int token_tiles, int slices) {
-  const int teams = slices < GS_STREAM_WARPS ? GS_STREAM_WARPS / slices : 1;
-  return (static_cast<size_t>((K + 31) / 32) + static_cast<size_t>(teams) * slices) * token_tiles * 512;
+// The streaming kernel's shared memory: x where the rings do not bring it, the slices' sums, the rings.
+static size_t small_gemm_stream_smem(int K, int token_tiles, int slices, int depth, bool x_ring) {
+  const size_t teams = slices < GS_STREAM_WARPS ? GS_STREAM_WARPS / slices : 1, pieces = x_ring ? 2 + token_tiles : 2;
+  return ((x_ring ? 0 : static_cast<size_t>((K + 31) / 32) * token_tiles) + teams * slices * token_tiles +
+          GS_STREAM_WARPS * depth * pieces) * 512;
 }
 
 struct SmallGemmSplit {
@@ -366,7 +377,7 @@ struct SmallGemmSplit {
 // 13.2, 12 rows 18.2 and 15.2.
 static bool small_gemm_streams(int N, int K, int token_tiles, const SmallGemmSplit& s) {
   const int tiles = (N + 15) / 16, slices = s.warps * s.ksplit;
-  if (slices > 32 || small_gemm_stream_fixed(K, token_tiles, slices) + 4 * 1024 * GS_STREAM_WARPS > GS_STREAM_SMEM) return false;
+  if (slices > 32) return false;
   if (tiles > 4 * 148) return true;
   if (token_tiles == 1) return tiles > 2 * 148 && K >= 3072;
   if (token_tiles == 2) return tiles >= 96 && (tiles < 2 * 148 || tiles > 400);
@@ -405,21 +416,29 @@ int small_gemm_launch(const SmallGemmArgs& a, int ksplit, cudaStream_t stream) {
   return launch_result();
 }
 
-template <int SLICES, int MT, typename TOut, bool SWIGLU, int ACT>
+template <int SLICES, int DEPTH, bool X_RING, int MT, typename TOut, bool SWIGLU, int ACT>
 int small_gemm_stream_launch(const SmallGemmArgs& a, cudaStream_t stream) {
-  const size_t fixed = small_gemm_stream_fixed(a.K, MT, SLICES), slot = 1024 * GS_STREAM_WARPS;
-  const bool deep = fixed + 8 * slot <= GS_STREAM_SMEM;
-  const size_t smem = fixed + (deep ? 8 : 4) * slot;
-  const dim3 grid(std::min(148, (a.N + 15) / 16)), block(GS_STREAM_WARPS * 32);
-  auto allow = [&](auto kernel) {
-    return !cuda_failed(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  };
-  if (deep) {
-    if (!allow(gemm_small_stream_kernel<SLICES, 8, MT, TOut, SWIGLU, ACT>)) return ERR_CUDA;
-    return launch_dependent(gemm_small_stream_kernel<SLICES, 8, MT, TOut, SWIGLU, ACT>, grid, block, smem, stream, false, a);
+  const size_t smem = small_gemm_stream_smem(a.K, MT, SLICES, DEPTH, X_RING);
+  if (cuda_failed(cudaFuncSetAttribute(gemm_small_stream_kernel<SLICES, DEPTH, X_RING, MT, TOut, SWIGLU, ACT>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem))))
+    return ERR_CUDA;
+  return launch_dependent(gemm_small_stream_kernel<SLICES, DEPTH, X_RING, MT, TOut, SWIGLU, ACT>, dim3(std::min(148, (a.N + 15) / 16)),
+                          dim3(GS_STREAM_WARPS * 32), smem, stream, false, a);
+}
+
+// As many blocks on their way as shared memory has room for beside all of x; x through the rings where that leaves none.
+template <int SLICES, int MT, typename TOut, bool SWIGLU, int ACT>
+int small_gemm_stream(const SmallGemmArgs& a, cudaStream_t stream) {
+  constexpr int WITH_X = MT == 1 ? 8 : MT == 2 ? 6 : 4;
+  if (small_gemm_stream_smem(a.K, MT, SLICES, 8, false) <= GS_STREAM_SMEM)
+    return small_gemm_stream_launch<SLICES, 8, false, MT, TOut, SWIGLU, ACT>(a, stream);
+  if constexpr (SLICES == 4 && MT <= 2) {        // K below 4096
+    return small_gemm_stream_launch<SLICES, 4, false, MT, TOut, SWIGLU, ACT>(a, stream);
+  } else {
+    if (small_gemm_stream_smem(a.K, MT, SLICES, 4, false) <= GS_STREAM_SMEM)
+      return small_gemm_stream_launch<SLICES, 4, false, MT, TOut, SWIGLU, ACT>(a, stream);
+    return small_gemm_stream_launch<SLICES, WITH_X, true, MT, TOut, SWIGLU, ACT>(a, stream);
   }
-  if (!allow(gemm_small_stream_kernel<SLICES, 4, MT, TOut, SWIGLU, ACT>)) return ERR_CUDA;
-  return launch_dependent(gemm_small_stream_kernel<SLICES, 4, MT, TOut, SWIGLU, ACT>, grid, block, smem, stream, false, a);
 }
 
 template <int MT, typename TOut, bool SWIGLU, int ACT>
@@ -428,15 +447,15 @@ int small_gemm_split_launch(const SmallGemmArgs& a, cudaStream_t stream) {
   if constexpr (MT <= 4) {
     if (small_gemm_streams(a.cut_rows, a.K, MT, s)) {
       const int slices = s.warps * s.ksplit;
-      if (slices == 4) return small_gemm_stream_launch<4, MT, TOut, SWIGLU, ACT>(a, stream);
+      if (slices == 4) return small_gemm_stream<4, MT, TOut, SWIGLU, ACT>(a, stream);
       if constexpr (MT > 1)
-        if (slices == 16) return small_gemm_stream_launch<16, MT, TOut, SWIGLU, ACT>(a, stream);
+        if (slices == 16) return small_gemm_stream<16, MT, TOut, SWIGLU, ACT>(a, stream);
       if constexpr (MT == 2)
-        if (slices == 32) return small_gemm_stream_launch<32, MT, TOut, SWIGLU, ACT>(a, stream);
-      return small_gemm_stream_launch<8, MT, TOut, SWIGLU, ACT>(a, stream);
+        if (slices == 32) return small_gemm_stream<32, MT, TOut, SWIGLU, ACT>(a, stream);
+      return small_gemm_stream<8, MT, TOut, SWIGLU, ACT>(a, stream);
     }
   }
-  if constexpr (MT > 2)       // (up to 16 rows, the x of a K that four warps cut finds room in the streaming kernel)
+  if constexpr (MT > 4)       // (four warps cut matrices of many rows, which stream up to 32 tokens)
     if (s.warps == 4) return small_gemm_launch<4, MT, TOut, SWIGLU, ACT>(a, s.ksplit, stream);
   return small_gemm_launch<8, MT, TOut, SWIGLU, ACT>(a, s.ksplit, stream);
 }
