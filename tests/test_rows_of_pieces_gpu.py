@@ -190,3 +190,17 @@ def test_heads_side_by_side(cuda_device, tokens, heads, kv_heads, kd, vd, rot, p
                    ops.qkv_halves(rows, heads, kv_heads, kd, vd, "per_head", *norm, 1e-6, *where[0], 1.25, True, *where[1], bias=bias))
     ops.check_status(case.status)
     assert _apart(*out, torch.bfloat16) and _apart(*case.caches, torch.bfloat16) and case.caches[0][1:].abs().max() > 0
+
+
+@pytest.mark.parametrize("shape", [(1, 4), (3, 5), (129, 516), (12, 2048), (7, 1026)])
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+def test_a_sum_with_a_bias_is_the_sum_behind_the_bias(cuda_device, shape, out_dtype):
+    from zephyr_b200.config.errors import InvalidArgumentError
+    from zephyr_b200.kernels import ops
+
+    g = torch.Generator().manual_seed(shape[1])
+    a, b, bias = (torch.randn(n, generator=g).to(cuda_device) for n in (shape, shape, shape[1]))
+    want = ops.scaled_sum(ops.add_bias(a.clone(), bias), b, 0.75, -1.5, out_dtype=out_dtype)
+    assert torch.equal(ops.scaled_sum(a, b, 0.75, -1.5, out_dtype=out_dtype, bias_a=bias), want)
+    with pytest.raises(InvalidArgumentError):
+        ops.scaled_sum(a, b, 0.75, -1.5, bias_a=bias[:-1])

@@ -171,7 +171,7 @@ _SIGNATURES = {
     "zb_rotate_qk": [c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_float, c_void_p, c_int, c_int, c_int, c_void_p],
     "zb_gated_group_rms_norm": [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_int,
                                 c_float, c_int, c_int, c_int, c_void_p],
-    "zb_scaled_sum": [c_void_p, c_void_p, c_void_p, c_float, c_float, c_longlong, c_int, c_int, c_void_p],
+    "zb_scaled_sum": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_float, c_float, c_longlong, c_int, c_int, c_void_p],
     "zb_paged_decode_supported": [c_int, c_int, c_int, c_int],
     "zb_paged_decode": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int,
                         c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_void_p, c_void_p,
@@ -981,13 +981,16 @@ def gated_group_rms_norm(o: torch.Tensor, gate: torch.Tensor, w: torch.Tensor, g
 
 
 def scaled_sum(a: torch.Tensor, b: torch.Tensor, scale_a: float, scale_b: float,
-               out_dtype: torch.dtype | None = None) -> torch.Tensor:
-    """scale_a * a + scale_b * b in float32 with one rounding; a and b may be float32 whatever the result is."""
-    _cuda(a, b)
+               out_dtype: torch.dtype | None = None, bias_a: torch.Tensor | None = None) -> torch.Tensor:
+    """scale_a * a + scale_b * b in float32 with one rounding; a and b may be float32 whatever the result is.  ``bias_a``
+    (float32, one value a column) is added to a first, with a float32 rounding of its own."""
+    _cuda(a, b, bias_a)
     _require(a.shape == b.shape and a.dtype == b.dtype and a.dtype in DTYPE_CODE and a.is_contiguous()
              and b.is_contiguous(), "two contiguous tensors of one shape and type")
+    _require(bias_a is None or (bias_a.dtype == torch.float32 and bias_a.is_contiguous() and bias_a.shape == a.shape[-1:]),
+             "one float32 bias value per column")
     out = torch.empty(a.shape, dtype=out_dtype or a.dtype, device=a.device)
-    _check(library().zb_scaled_sum(_ptr(out), _ptr(a), _ptr(b), float(scale_a), float(scale_b), a.numel(),
+    _check(library().zb_scaled_sum(_ptr(out), _ptr(a), _ptr(b), _ptr(bias_a), a.shape[-1] if a.dim() else 0, float(scale_a), float(scale_b), a.numel(),
                                    DTYPE_CODE[a.dtype], DTYPE_CODE[out.dtype], _stream()), "scaled_sum")
     return out
 

@@ -410,6 +410,10 @@ class ParallelMixers(Mixer):
         positions = [getattr(branch, "position", None) for branch in self.branches]
         self.position = next((p for p in positions if p is not None), None)
         self.stores = [_store_count(sub) for sub, _ in branches]
+        # The first branch's output bias joins the sum in the sum's kernel instead of a pass of its own.
+        self.first_bias, first = None, self.branches[0]
+        if getattr(first, "takes_out_dtype", False) and getattr(first, "o_bias", None) is not None:
+            self.first_bias, first.o_bias = first.o_bias, None
 
     @staticmethod
     def weight_decls(spec: MixerSpec) -> dict[str, WeightDecl]:
@@ -451,7 +455,8 @@ class ParallelMixers(Mixer):
                 outputs.append(branch.forward(x, ctx, own))
         if outputs[0].dtype != outputs[1].dtype:
             outputs = [o.float() for o in outputs]
-        return ops.scaled_sum(outputs[0], outputs[1], self.scales[0], self.scales[1], out_dtype=out_dtype or self.dtype)
+        return ops.scaled_sum(outputs[0], outputs[1], self.scales[0], self.scales[1], out_dtype=out_dtype or self.dtype,
+                              bias_a=self.first_bias)
 
 
 def _store_count(sub: MixerSpec) -> int:
