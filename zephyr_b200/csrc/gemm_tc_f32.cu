@@ -13,14 +13,15 @@
 // below 2^-110 the bits below 2^-133 are lost: outputs that are not finite, or below 2^-80, are formed again by multiply-adds.
 //
 // A pair of SMs (tcgen05.mma.cta_group::2) = 256 rows of w, the tensor cores' row side, by NT rows of x, their columns; each CTA fetches 128
-// and NT / 2 of them.  Per 64 values of k: eight warps fetch the rows as float32 (the next 64 on their way in registers meanwhile), split
-// them and store the parts where the tensor cores read them (K-major, 128-byte swizzle); one thread issues the products of parts, the
-// small ones first, hi hi behind the eight warps' having taken the sums of the 64 values before; the eight warps add those to theirs
-// while the next products run.
-// Bound by the tensor cores from 192 columns on (4096^3 with 256 columns 700 us, 196 TFLOP/s and six times that of bfloat16
-// products, 0.71 of the measured peak), below by the chain of a stage: fetch, split, 24 products of at least 50 cycles, sums.  What it
-// takes beside: 700 x 4096 x 1024 44 us (multiply-adds on CUDA cores 201), 700 x 1024 x 2048 40 (103), 900 x 1024 x 3072 54 (192), 8 x
-// 151936 x 1024 201 (390), one row x 4096 x 1024 20 (19).  On single SMs (128 rows of w by 96) 62 us for the first, bound by the
+// and NT / 2 of them.  Per 64 values of k: sixteen warps (eight with 256 columns) fetch the rows as float32 (the next 64 on their way in
+// registers meanwhile), split them and store the parts where the tensor cores read them (K-major, 128-byte swizzle); one thread issues
+// the products of parts, the small ones first, hi hi behind the warps' having taken the sums of the 64 values before; the warps
+// add those to theirs while the next products run.
+// Bound by the tensor cores from 192 columns on (4096^3 587 us, 234 TFLOP/s and six times that of bfloat16
+// products, 0.86 of the measured peak; with eight warps 700 us), below by the chain of a stage: fetch, split, 24 products of at least 50
+// cycles, sums.  What it takes beside: 700 x 4096 x 1024 35 us (multiply-adds on CUDA cores 201; eight warps 44), 700 x 1024 x 2048 35
+// (103; 40), 900 x 1024 x 3072 50 (192; 54), 8 x 151936 x 1024 184 (390; 201), one row x 4096 x 1024 19 (19; 20).  On single SMs (128 rows
+// of w by 96) 62 us for the first, bound by the
 // operands' way from L2; arrivals on the pair's barriers with a release across the cluster wait for every load in flight (72 us).
 // Every wait is bounded and reports instead of hanging; tensor memory is given back on every path.
 #include "common.cuh"
@@ -34,22 +35,28 @@ namespace zb {
 
 constexpr int GF_BK = 64;                   // values of k a stage: one 128-byte row of a part
 constexpr int GF_ROWS = 128;                // rows of w of a CTA
-constexpr int GF_WARPS = 8;                 // that fetch, split and sum; one of the four behind them issues the products
-constexpr int GF_THREADS = (GF_WARPS + 4) * 32;
 constexpr int GF_WAIT_LIMIT = 1 << 18;
 constexpr float GF_SMALLEST = 8.3e-25f;      // 2^-80
 constexpr int GF_W_PART = GF_ROWS * GF_BK * 2;
-constexpr int GF_WORKER_REGISTERS = 232, GF_OTHER_REGISTERS = 40;       // of the 168 that the block is launched with: 256 x 232 + 128 x 40 = 384 x 168
 
 template <int NT> struct GemmF32Shape {
+  // That fetch, split and sum (one of the four behind them issues the products): sixteen, whose waits overlap better than eight's
+  // (700 x 4096 x 1024 in 192 columns 34.8 us against 42, 700 x 1024 x 2048 in 64 34.5 against 40), up to the columns whose sums their
+  // registers hold.
+  static constexpr int WARPS = NT <= 192 ? 16 : 8;
+  static constexpr int THREADS = (WARPS + 4) * 32;
+  // Of the 96 or 168 that the block is launched with: 512 x 104 + 128 x 64 = 640 x 96, 256 x 232 + 128 x 40 = 384 x 168.
+  static constexpr int WORKER_REGISTERS = WARPS == 16 ? 104 : 232, OTHER_REGISTERS = WARPS == 16 ? 64 : 40;
+  static constexpr int PASS = WARPS * 4;    // rows that the workers fetch at a time
+
   static constexpr int X_ROWS = NT / 2;     // of a CTA
   static constexpr int X_PART = X_ROWS * GF_BK * 2;
   static constexpr int STAGE_BYTES = 3 * (GF_W_PART + X_PART);
   static constexpr int SMEM_BYTES = 2 * STAGE_BYTES + 1024;
   static constexpr int TMEM_COLUMNS = NT <= 32 ? 64 : NT <= 64 ? 128 : NT <= 128 ? 256 : 512;      // the hi hi sums, the others
-  static constexpr int COLUMNS = NT / 2;    // of a warp
-  static constexpr int PER = (GF_ROWS + X_ROWS + 31) / 32;      // 32-byte pieces a thread fetches of a stage
-  static_assert(NT % 32 == 0 && NT <= 256, "columns of tensor memory in runs of 16 a warp");
+  static constexpr int COLUMNS = NT * 4 / WARPS;      // of a warp
+  static constexpr int PER = (GF_ROWS + X_ROWS + PASS - 1) / PASS;      // 32-byte pieces a thread fetches of a stage
+  static_assert(NT % 32 == 0 && NT <= 256 && COLUMNS % 8 == 0, "columns of tensor memory in runs of 8 a warp");
 };
 
 struct GemmF32Args {
@@ -60,6 +67,11 @@ struct GemmF32Args {
   long long ldx, ldw, ldy;
   int* status;
 };
+
+__device__ __forceinline__ void tmem_ld_run(unsigned at, unsigned (&v)[16]) { tmem_ld16(at, v); }
+__device__ __forceinline__ void tmem_ld_run(unsigned at, unsigned (&v)[8]) { tmem_ld8(at, v); }
+__device__ __forceinline__ void tmem_wait_ld_run(unsigned (&v)[16]) { tmem_wait_ld16(v); }
+__device__ __forceinline__ void tmem_wait_ld_run(unsigned (&v)[8]) { tmem_wait_ld8(v); }
 
 // One output by multiply-adds in ascending k.
 __device__ __noinline__ float dot_f32(const float* x, const float* w, int K) {
@@ -72,9 +84,9 @@ __device__ __noinline__ float dot_f32(const float* x, const float* w, int K) {
 }
 
 template <int NT>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GF_THREADS, 1) gemm_f32_tc_kernel(const GemmF32Args a) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmF32Shape<NT>::THREADS, 1) gemm_f32_tc_kernel(const GemmF32Args a) {
   using Shape = GemmF32Shape<NT>;
-  constexpr int COLUMNS = Shape::COLUMNS, PER = Shape::PER, X_PART = Shape::X_PART;
+  constexpr int COLUMNS = Shape::COLUMNS, PER = Shape::PER, X_PART = Shape::X_PART, WARPS = Shape::WARPS, PASS = Shape::PASS;
   extern __shared__ unsigned char gf_smem_raw[];
   __shared__ unsigned long long full[2], taken, done;
   __shared__ unsigned tmem_base_s;
@@ -85,14 +97,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GF_THREADS, 1) gemm_
   const int m0 = pair % a.tiles_m * NT, n0 = pair / a.tiles_m * (2 * GF_ROWS) + rank * GF_ROWS;
   const int blocks = (a.K + GF_BK - 1) / GF_BK;
   if (tid == 0) {
-    mbar_init(&full[0], 2 * GF_WARPS);
-    mbar_init(&full[1], 2 * GF_WARPS);
-    mbar_init(&taken, 2 * GF_WARPS);
+    mbar_init(&full[0], 2 * WARPS);
+    mbar_init(&full[1], 2 * WARPS);
+    mbar_init(&taken, 2 * WARPS);
     mbar_init(&done, 1);
     failed = 0;
     fence_barrier_init();
   }
-  if (warp == GF_WARPS) {
+  if (warp == WARPS) {
     tmem_alloc_pair(&tmem_base_s, Shape::TMEM_COLUMNS);
     tmem_relinquish_pair();
   }
@@ -118,9 +130,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GF_THREADS, 1) gemm_
     return ok;
   };
 
-  if (warp >= GF_WARPS) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(GF_OTHER_REGISTERS));
-    if (warp == GF_WARPS && rank == 0) {
+  if (warp >= WARPS) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(Shape::OTHER_REGISTERS));
+    if (warp == WARPS && rank == 0) {
       constexpr unsigned IDESC = tc_idesc_pair(NT);
       const bool leader = elect_one();
       for (int b = 0; b < blocks; ++b) {
@@ -150,17 +162,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GF_THREADS, 1) gemm_
       }
     }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(GF_WORKER_REGISTERS));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(Shape::WORKER_REGISTERS));
     // Piece u of this thread: 8 values of k (4 c .. and 32 + 4 c .. of the stage's 64, side by side in both operands' shared memory)
-    // of row tid / 8 + 32 u of the CTA's rows of w and, behind them, of x.
+    // of row tid / 8 + PASS u of the CTA's rows of w and, behind them, of x.
     const int c = tid & 7, r0 = tid >> 3, x0 = m0 + rank * Shape::X_ROWS;
     const float* const w_row = a.w + static_cast<long long>(n0 + r0) * a.ldw + 4 * c;
     const float* const x_row = a.x + static_cast<long long>(x0 + r0) * a.ldx + 4 * c;
     unsigned present = 0;              // bit u: its row lies within the matrix
 #pragma unroll
     for (int u = 0; u < PER; ++u) {
-      const int r = r0 + 32 * u;
-      if (32 * u < GF_ROWS ? n0 + r < a.N : x0 + r - GF_ROWS < a.M && r - GF_ROWS < Shape::X_ROWS) present |= 1u << u;
+      const int r = r0 + PASS * u;
+      if (PASS * u < GF_ROWS ? n0 + r < a.N : x0 + r - GF_ROWS < a.M && r - GF_ROWS < Shape::X_ROWS) present |= 1u << u;
     }
     float4 ahead[PER][2];
     auto fetch = [&](int b) {
@@ -169,7 +181,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GF_THREADS, 1) gemm_
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
           const int k = b * GF_BK + 32 * half;
-          const float* row = 32 * u < GF_ROWS ? w_row + 32 * u * a.ldw : x_row + (32 * u - GF_ROWS) * a.ldx;
+          const float* row = PASS * u < GF_ROWS ? w_row + PASS * u * a.ldw : x_row + (PASS * u - GF_ROWS) * a.ldx;
           ahead[u][half] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
           if ((present >> u & 1) && k + 4 * c < a.K) ahead[u][half] = *reinterpret_cast<const float4*>(row + k);
         }
@@ -177,9 +189,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GF_THREADS, 1) gemm_
     auto store = [&](unsigned char* stage) {
 #pragma unroll
       for (int u = 0; u < PER; ++u) {
-        const int r = r0 + 32 * u;
-        const bool of_w = 32 * u < GF_ROWS;
-        if (!of_w && 32 * u + 31 >= GF_ROWS + Shape::X_ROWS && r >= GF_ROWS + Shape::X_ROWS) continue;
+        const int r = r0 + PASS * u;
+        const bool of_w = PASS * u < GF_ROWS;
+        if (!of_w && PASS * u + PASS - 1 >= GF_ROWS + Shape::X_ROWS && r >= GF_ROWS + Shape::X_ROWS) continue;
         unsigned char* to = stage + (of_w ? r * 128 : 3 * GF_W_PART + (r - GF_ROWS) * 128) + ((c ^ (r & 7)) << 4);
         const int part = of_w ? GF_W_PART : X_PART;
         const float4 p = ahead[u][0], q = ahead[u][1];
@@ -193,21 +205,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GF_THREADS, 1) gemm_
         *reinterpret_cast<uint4*>(to + 2 * part) = lo;
       }
     };
-    // Sums: this thread's row of w (its lane of tensor memory) and half of the columns.
+    // Sums: this thread's row of w (its lane of tensor memory) and a warp's share of the columns.
     const int quarter = warp & 3, column0 = (warp >> 2) * COLUMNS;
     const unsigned tmem_mine = (static_cast<unsigned>(32 * quarter) << 16) + column0;
     float sum[COLUMNS];
 #pragma unroll
     for (int i = 0; i < COLUMNS; ++i) sum[i] = 0.0f;
     auto add = [&](unsigned from) {
-      unsigned v[2][16];
-      tmem_ld16(from + tmem_mine, v[0]);
+      constexpr int RUN = COLUMNS % 16 == 0 && WARPS == 8 ? 16 : 8;
+      unsigned v[2][RUN];
+      tmem_ld_run(from + tmem_mine, v[0]);
 #pragma unroll
-      for (int i = 0; i < COLUMNS / 16; ++i) {
-        tmem_wait_ld16(v[i & 1]);
-        if (i + 1 < COLUMNS / 16) tmem_ld16(from + tmem_mine + 16 * (i + 1), v[(i + 1) & 1]);
+      for (int i = 0; i < COLUMNS / RUN; ++i) {
+        tmem_wait_ld_run(v[i & 1]);
+        if (i + 1 < COLUMNS / RUN) tmem_ld_run(from + tmem_mine + RUN * (i + 1), v[(i + 1) & 1]);
 #pragma unroll
-        for (int e = 0; e < 16; ++e) sum[16 * i + e] += __uint_as_float(v[i & 1][e]);
+        for (int e = 0; e < RUN; ++e) sum[RUN * i + e] += __uint_as_float(v[i & 1][e]);
       }
     };
     const unsigned taken_at = in_cta_of_rank(smem_u32(&taken), 0), full_at = in_cta_of_rank(smem_u32(&full[0]), 0);
@@ -252,7 +265,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GF_THREADS, 1) gemm_
   if (failed) let_copies_land();        // (the products in flight)
   __syncwarp();
   cluster_sync_all();
-  if (warp == GF_WARPS) {
+  if (warp == WARPS) {
     tc_fence_after_sync();
     tmem_dealloc_pair(tmem_base, Shape::TMEM_COLUMNS);
   }
@@ -266,7 +279,7 @@ static int gemm_f32_launch(GemmF32Args a, cudaStream_t stream) {
   if (pairs >= (1LL << 30)) return ERR_UNSUPPORTED;
   auto kernel = gemm_f32_tc_kernel<NT>;
   if (cuda_failed(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::SMEM_BYTES))) return ERR_CUDA;
-  return launch_dependent(kernel, dim3(static_cast<unsigned>(2 * pairs)), dim3(GF_THREADS), Shape::SMEM_BYTES, stream, false, a);
+  return launch_dependent(kernel, dim3(static_cast<unsigned>(2 * pairs)), dim3(Shape::THREADS), Shape::SMEM_BYTES, stream, false, a);
 }
 
 }  // namespace zb
@@ -286,10 +299,10 @@ ZB_API int zb_gemm_nt_f32(float* y, const float* x, const float* w, int M, int N
   GemmF32Args a;
   a.y = y; a.x = x; a.w = w; a.M = M; a.N = N; a.K = K; a.ldx = ldx; a.ldw = ldw; a.ldy = ldy; a.status = status;
   // The tile whose rounds over the pairs of SMs take the least time (us of a full round at K = 1024, whatever K's share of it):
-  // 700 x 4096 x 1024 is one round of 64 pairs with 192 columns, 44 us (256: 50, 128: 60, 96: 51); 700 x 1024 x 2048 44 pairs with 64,
-  // 40 (32: 62, 96: 41); 2048 x 6144 x 1024 three rounds with 256, 149 (192: 162, 128: 179); 8 x 151936 x 1024 with 32, 201.
+  // 700 x 4096 x 1024 is one round of 64 pairs with 192 columns, 35 us (256: 49, 128: 48, 96: 45); 700 x 1024 x 2048 44 pairs with 64,
+  // 35 (32: 59, 96: 36); 2048 x 6144 x 1024 four rounds with 192, 133 (256: 140, 128: 141); 8 x 151936 x 1024 with 32, 184.
   struct Tile { int columns, us; };
-  constexpr Tile tiles[] = {{32, 17}, {64, 19}, {96, 22}, {128, 28}, {160, 33}, {192, 37}, {256, 45}};
+  constexpr Tile tiles[] = {{32, 17}, {64, 19}, {96, 21}, {128, 23}, {160, 28}, {192, 32}, {256, 46}};
   const long long row_blocks = (N + 2LL * GF_ROWS - 1) / (2 * GF_ROWS);
   int best = 0;
   long long least = 0;

@@ -60,6 +60,11 @@ __device__ __forceinline__ void tmem_ld16(unsigned address, unsigned (&r)[16]) {
                  "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                : "r"(address) : "memory");
 }
+__device__ __forceinline__ void tmem_ld8(unsigned address, unsigned (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(address) : "memory");
+}
 // Waits for this thread's tensor-memory loads; `r`, what a load was asked to bring, is not used before.
 __device__ __forceinline__ void tmem_wait_ld32(unsigned (&r)[32]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;\n"
@@ -74,6 +79,10 @@ __device__ __forceinline__ void tmem_wait_ld16(unsigned (&r)[16]) {
                : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
                  "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
                :: "memory");
+}
+__device__ __forceinline__ void tmem_wait_ld8(unsigned (&r)[8]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;\n"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]) :: "memory");
 }
 __device__ __forceinline__ void tmem_st32(unsigned address, const unsigned (&r)[32]) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
