@@ -72,3 +72,42 @@ def test_attention_is_near_the_exact_one_and_as_finite_as_the_general_kernel(ops
     assert torch.equal(got.isfinite(), general.isfinite())
     fine = got.isfinite()
     assert ((got - general)[fine].abs() <= 2e-5 * general[fine].abs().clamp(min=1.0)).all()
+
+
+@pytest.mark.parametrize("nh,nkv,hd,n,ctx", [(2, 1, 128, 5, 150), (8, 2, 60, 40, 130)])
+def test_large_values_weigh_what_their_keys_say(ops, cuda_device, nh, nkv, hd, n, ctx):
+    """Values that bfloat16 parts do not hold, finite and infinite, at keys of ordinary size, in a row's first step of keys and in later
+    ones whose maxima grow: the outputs as numbers, against 64 bits and the general kernel."""
+    q, cache, meta, Ks, Vs, qs = build_paged_case(cuda_device, torch.float32, nh, nkv, hd, 16, [n], [ctx], 11)
+    status, wide, tokens = ops.new_status(cuda_device), ops.paged_prefill_tile_tokens(), ops.attention_tile_tokens(nh // nkv)
+    K, V = Ks[0], Vs[0]
+    K *= (torch.arange(ctx + n) / 60.0).view(-1, 1, 1)     # (the largest score of a step grows with its place)
+    # In columns 0 .. 5 and hd - 1, each alone in its column: at position 17 (first step), 64 and 100 (second), 128 (third).
+    large = {(17, 0): 3.35e38, (17, 1): math.inf, (17, hd - 1): -3.4e38, (64, 2): -math.inf, (100, 3): 3.4e38, (100, 4): math.nan, (128, 5): 3.39e38}
+    for (p, column), value in large.items():
+        V[p, :, column] = value
+    held = cache.clone()
+    for p in range(ctx + n):
+        where = torch.argsort(ops.kv_row_permutation(p, hd, torch.float32))
+        page, off = meta["table"][0, p // 16], p % 16
+        held[page, 0, :, off], held[page, 1, :, off] = K[p][:, where].to(cuda_device), V[p][:, where].to(cuda_device)
+    common = (meta["row_q_start"], meta["row_q_len"], meta["row_ctx"], nh, nkv, hd, 0, 1 / math.sqrt(hd), status)
+    out = torch.empty_like(q)
+    ops.paged_attention_f32(q, held, meta["table"], *tiles_for([n], wide, cuda_device), wide, *common, out)
+    general = ops.paged_attention(q, held, meta["table"], *tiles_for([n], tokens, cuda_device), tokens, *common)
+    ops.check_status(status)
+    # Every query sees the large values' keys, so a plain softmax over what it sees is the reference.
+    exact = torch.empty(n, nh, hd, dtype=torch.float64)
+    for t in range(n):
+        for h in range(nh):
+            scores = K[:ctx + t + 1, h * nkv // nh].double() @ qs[0][t, h].double() / math.sqrt(hd)
+            exact[t, h] = (scores.softmax(0).unsqueeze(1) * V[:ctx + t + 1, h * nkv // nh].double()).sum(0)
+    got, general = out.cpu().double().view_as(exact), general.cpu().double().view_as(exact)
+    for x in (got, general):
+        assert torch.equal(x.isnan(), exact.isnan()) and torch.equal(x.isinf(), exact.isinf())
+        assert torch.equal(x[x.isinf()], exact[exact.isinf()])
+    # Scores of up to some 30 at errors of 2^-22 of themselves and of the sums behind them move a weight by 2^-17 of itself at most; an ordinary
+    # column's values are of about one.
+    fine = exact.isfinite()
+    assert ((got - exact).abs()[fine] <= 2.0 ** -17 * exact.abs().clamp(min=4.0)[fine]).all()
+    assert ((general - exact).abs()[fine] <= 2.0 ** -17 * exact.abs().clamp(min=4.0)[fine]).all()

@@ -400,8 +400,16 @@ __global__ void __launch_bounds__(F_THREADS, 1) paged_attention_f32_kernel(const
       }
       l = fmaf(l, corr, (sums[0] + sums[1]) + (sums[2] + sums[3]));
       m = new_m;
+      // The totals on the new maximum's scale, with the weighted values of the step before.
+      auto rescale = [&] {
+        if (i == 0) return;               // (zeros)
+        ok = arrived(&o_done, (i - 1) & 1, 3000000 + i) && ok;
+        tc_fence_after_sync();
+        take_values(corr);
+      };
       if (rare) {
         if (f32_workers_any(!ok)) break;
+        rescale();                      // (what is added by hand is on that scale)
         // The keys' place is free (their scores are complete): the weights of all rows, [key][row].
         float* weights = reinterpret_cast<float*>(k_s);
 #pragma unroll
@@ -437,14 +445,7 @@ __global__ void __launch_bounds__(F_THREADS, 1) paged_attention_f32_kernel(const
         if (lane == 0) tc_mbar_arrive(&k_full);
         fetch_keys(i + 2);
       }
-      if (i > 0) {
-        ok = arrived(&o_done, (i - 1) & 1, 3000000 + i) && ok;
-        tc_fence_after_sync();
-        take_values(corr);
-      } else {
-#pragma unroll
-        for (int e = 0; e < COLUMNS; ++e) acc[e] *= corr;      // (zeros, or what is not finite)
-      }
+      if (!rare) rescale();
       store(values, v_s);               // (free: the step before's products are complete)
       fence_proxy_async();
       {
