@@ -47,3 +47,49 @@ def test_pieces_are_near_the_recurrence_in_64_bits(cuda_device, heads, dim, vdim
         got, want = out[start:start + n].double().view(n, heads, vdim), torch.stack(expected)
         assert (got - want).norm() <= bound * want.norm(), n
         assert (state[r].double().view_as(S) - S).norm() <= bound * S.norm(), n
+
+
+@pytest.mark.parametrize("dim,vdim", [(128, 128), (100, 68)])
+def test_a_value_that_is_not_finite_stays_with_later_tokens(cuda_device, dim, vdim):
+    """Infinities, NaN and values that round to infinity in bfloat16 among the values, at the edges of pieces, of the weights' quarters and of a
+    CTA's columns, also in pieces that follow one another: all tokens before one, and all other columns, keep their bits."""
+    from zephyr_b200.kernels import ops
+
+    heads, T = 3, 300
+    g = torch.Generator().manual_seed(dim)
+    q, k, v = (torch.randn(T, n, generator=g).to(cuda_device) for n in (heads * dim, heads * dim, heads * vdim))
+    decay, status = torch.tensor([0.4, 0.9, 0.999], device=cuda_device), ops.new_status(cuda_device)
+    i32 = lambda values: torch.tensor(values, dtype=torch.int32, device=cuda_device)
+
+    def run(values):
+        state, launched = torch.zeros(1, heads * dim * vdim, device=cuda_device), ops.LAUNCH_COUNTS.get("retention_tc", 0)
+        out = ops.retention(q, k, values, decay, heads, dim, vdim, state, i32([0]), i32([0]), i32([T]), status)
+        ops.check_status(status)
+        assert ops.LAUNCH_COUNTS["retention_tc"] == launched + 2
+        return out, state.view(heads, dim, vdim)
+
+    clean, behind = run(v)
+    inf, nan = float("inf"), float("nan")
+    cases = [{(0, 0): nan}, {(31, 63): inf}, {(32, 64): -inf}, {(127, vdim - 1): nan}, {(128, vdim): inf}, {(299, 3 * vdim - 1): nan},
+             {(100, 5): inf, (130, vdim + 63): nan, (256, 2 * vdim + 64): -inf}, {(200, 1): 3.4e38, (255, vdim + 1): -3.4e38}]
+    for bad in cases:
+        values = v.clone()
+        for (at, column), value in bad.items():
+            values[at, column] = value
+        got, state = run(values)
+        touched = torch.zeros_like(got, dtype=torch.bool)
+        for (at, column), value in bad.items():
+            touched[at:, column] = True
+            # The token's own output is its value times q . k, two bfloat16 parts each, beside which the ordinary rest is nothing.
+            head = slice(column // vdim * dim, (column // vdim + 1) * dim)
+            qt, kt = q[at, head].double(), k[at, head].double()
+            want, own = float((qt @ kt * value).float()), float(got[at, column])
+            if want == want and abs(want) < inf:
+                assert abs(own - want) <= 4 * 2.0 ** -17 * float(qt.norm() * kt.norm()) * abs(value), bad
+            else:
+                assert own == want or (own != own and want != want), bad
+            if not abs(value) < inf:
+                assert not torch.isfinite(got[at:, column]).any() and not torch.isfinite(state[column // vdim, :, column % vdim]).any(), bad
+        assert torch.equal(got[~touched], clean[~touched]), bad
+        untouched = ~torch.isin(torch.arange(heads * vdim, device=cuda_device), torch.tensor([c for _, c in bad], device=cuda_device)).view(heads, 1, vdim)
+        assert torch.equal(state[untouched.expand_as(state)], behind[untouched.expand_as(behind)]), bad

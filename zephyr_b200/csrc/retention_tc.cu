@@ -363,6 +363,9 @@ __global__ void __launch_bounds__(RT_THREADS, 1) retention_tc_kernel(const Reten
       if (p + 1 < pieces) fetch_values(p + 1);
       // Scores to weights: row r, keys 32 quarter .. + 31.
       ok = arrived(&s1_done, p & 1, 4000000 + p);
+      // (Behind a piece with such a value the weights' place is read until its outputs are there, by four warps a row.  Each of them has
+      // then given the state of this piece.)
+      if (ok && p > 0 && wild[(p - 1) & 1] == p - 1) ok = arrived(&s_full, p & 1, 9000000 + p);
       if (!ok) break;
       tc_fence_after_sync();
 #pragma unroll
