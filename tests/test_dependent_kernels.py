@@ -8,6 +8,13 @@ from zephyr_b200.kernels.build import SOURCE_DIR
 # Written before any step, or by the kernel alone: the only pointers that may be declared free of other writers.
 CONSTANT = {"table", "w", "bias", "q_norm_w", "k_norm_w", "cos_table", "sin_table"}
 OWN = {"out", "q_out"}
+# What kernels index ahead of their wait: arrays of their own (barriers, shared memory, registers), ...
+LOCAL = {"consumed", "empty", "full", "page_ids", "prefix", "qempty", "qfull", "trace", "plans", "place_empty", "place_full", "place_s",
+         "half_of_row", "bars", "kv_empty", "kv_full", "note", "o_done", "p_full", "s_full", "red", "w_ok", "w_row", "x_ok", "x_row", "falling", "power",
+         "wild", "wild_token", "smem", "smem_raw", "smem_unaligned", "f_smem_raw", "gs_smem", "gx_smem_raw", "gf_smem_raw"}
+# ... the step's description, which lies there before its first kernel, weights, and the launch's own arguments.
+GIVEN = {"paged_decode_kernel": {"a.block_table", "a.row_ctx", "a.row_q_start", "a.rows", "table", "x", "y"}, "fused_chain_kernel": {"a.map", "a.stage", "a.tiled"},
+         "retention_tc_kernel": {"a.decay"}, "qk_norm_rope_cache_wide_kernel": {"positions", "token_row", "scale_x", "scale_y"}}
 
 
 def kernels():
@@ -43,6 +50,16 @@ def test_dependent_kernels_do_not_declare_other_kernels_results_constant():
             if "__restrict__" in parameter:
                 assert parameter.split()[-1].lstrip("*") in CONSTANT | OWN, (file, name, parameter)
         assert "__ldg(" not in body and ".nc." not in body, (file, name)
+
+
+def test_dependent_kernels_index_nothing_of_other_kernels_ahead_of_their_wait():
+    for file, name, _, body in kernels():
+        if "wait_for_prior_grids()" not in body:
+            continue
+        several = name in ("paged_decode_kernel", "fused_chain_kernel")          # roles, each with a wait of its own
+        ahead = body[:(body.index if several else body.rindex)("wait_for_prior_grids()")]
+        indexed = set(re.findall(r"(?<![\w.])(?:a\.)?[A-Za-z_]\w*(?=\[)", ahead))
+        assert indexed <= LOCAL | GIVEN.get(name, set()), (file, name, indexed - LOCAL)
 
 
 def test_kernels_whose_wait_runs_out_let_their_copies_land():

@@ -486,17 +486,15 @@ static void conv_run_launch(const ConvArgs& a, const int* token_row, int tokens,
   }
 }
 
-// After it: every request's last taps - 1 inputs go to its state.  A thread owns a channel of one request.  All it reads is
-// older than the convolution, which only reads the state, so it reads beside it and waits for its end before it writes.
+// After it: every request's last taps - 1 inputs go to its state.  A thread owns a channel of one request.
 template <typename T>
 __global__ void conv_state_update_kernel(const ConvArgs a) {
+  wait_for_prior_grids();
+  let_dependents_launch();
   const int c = blockIdx.x * blockDim.x + threadIdx.x, row = blockIdx.y;
   if (c >= a.C) return;
   const int slot = a.slots[row];
-  if (slot < 0 || slot >= a.num_slots) {             // reported by the convolution
-    wait_for_prior_grids();                          // what follows waits for this kernel only
-    return;
-  }
+  if (slot < 0 || slot >= a.num_slots) return;       // reported by the convolution
   float* state = a.state + static_cast<long long>(slot) * a.slot_stride;
   const T* x = static_cast<const T*>(a.x);
   const int t0 = a.row_q_start[row], n = a.row_q_len[row], keep = a.taps - 1;
@@ -509,8 +507,6 @@ __global__ void conv_state_update_kernel(const ConvArgs a) {
                        : state[static_cast<long long>(keep + i) * a.C + c];
     }
   }
-  wait_for_prior_grids();
-  let_dependents_launch();
 #pragma unroll
   for (int j = 0; j < CONV_MAX_TAPS; ++j)
     if (j < keep) state[static_cast<long long>(j) * a.C + c] = last[j];
