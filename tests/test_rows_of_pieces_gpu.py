@@ -204,3 +204,33 @@ def test_a_sum_with_a_bias_is_the_sum_behind_the_bias(cuda_device, shape, out_dt
     assert torch.equal(ops.scaled_sum(a, b, 0.75, -1.5, out_dtype=out_dtype, bias_a=bias), want)
     with pytest.raises(InvalidArgumentError):
         ops.scaled_sum(a, b, 0.75, -1.5, bias_a=bias[:-1])
+
+
+@pytest.mark.parametrize("N,K,M,streams", [
+    (32768, 1024, 8, False), (32768, 256, 1, False), (16384, 512, 8, False), (8192, 1024, 12, False), (4096, 512, 16, False), (2048, 768, 9, False),
+    (8192, 1024, 32, False), (4096, 1024, 24, False), (16384, 512, 12, False), (16384, 1024, 8, True), (65536, 512, 5, True), (4096, 1024, 12, True),
+    (8192, 512, 12, True), (20480, 256, 12, True), (6144, 1024, 32, True), (32768, 1536, 8, True), (28448, 768, 3, False), (9504, 768, 4, True), (10240, 512, 30, True), (12288, 512, 30, False)])
+def test_few_rows_take_the_faster_form(cuda_device, N, K, M, streams):
+    """On both sides of the lines between the persistent kernel and the one with bursts (32 rows of the matrix a CTA up to 8 rows): the kernel that was
+    the faster one when both were timed, near the exact sums, and the same bits where a row comes alone or with more."""
+    from torch.profiler import ProfilerActivity, profile
+
+    from zephyr_b200.kernels import ops
+
+    g = torch.Generator(device=cuda_device).manual_seed(N + K + M)
+    x = torch.randn(M, K, generator=g, device=cuda_device).to(torch.bfloat16)
+    w = (torch.randn(N, K, generator=g, device=cuda_device) / K ** 0.5).to(torch.bfloat16)
+    ops.gemm_small(x, w)
+    with profile(activities=[ProfilerActivity.CUDA]) as seen:
+        got = ops.gemm_small(x, w, out_dtype=torch.float32)
+        torch.cuda.synchronize()
+    names = [e.name for e in seen.events() if "gemm_small" in e.name]
+    assert len(names) == 1 and ("gemm_small_stream_kernel" in names[0]) == streams
+    assert (got.double() - x.double() @ w.double().T).abs().max() <= 6 * 2.0 ** -24 * max(16.0, K ** 0.5)
+    many = x.repeat(64 // M, 1)
+    for rows in (1, 9, 17, 33):
+        assert torch.equal(ops.gemm_small(many[:rows], w, out_dtype=torch.float32)[:M], got[:rows])
+    if N % 16 == 0:
+        pair = got.view(M, N // 16, 2, 8)
+        gated = ops.gemm_small(x, w, out_dtype=torch.float32, swiglu=True).view(M, N // 16, 8)
+        assert (gated - torch.nn.functional.silu(pair[:, :, 0]) * pair[:, :, 1]).abs().max() <= 2.0 ** -21 * max(1.0, float(got.abs().max())) ** 2

@@ -8,9 +8,9 @@
 // consecutive values k = 8t .. 8t+7 of its row: one 16-byte load feeds two tensor-core products.
 // The products see k in a permuted order, the same for both operands, so the sum is unchanged.
 //
-// One CTA owns 16 rows of W; its warps split K, and for matrices with few rows a cluster of
+// One CTA owns 16 rows of W (or 32); its warps split K, and for matrices with few rows a cluster of
 // up to 8 CTAs splits K further.  A decode step's product is bound by latency before it is by bandwidth: a warp has the loads
-// of several blocks of 32 k in flight, whatever is left of its slice: four up to 16 rows, two from 17 to 32;
+// of several blocks of 32 k in flight, whatever is left of its slice: four up to 16 rows, two from 17 to 32 and where a CTA takes 32 rows of W;
 // above 32 rows four blocks of W alone, x at its use (with x ahead too, two blocks: 12288 x 4096, 64 rows: 92 us,
 // now 47; 6144 x 2048: 29 and 17) (one block after the other, as a loop's remainder, 2048 x
 // 6144 with 12 rows took 13.8 us; now 10.1, its bytes 3.8), and the CTAs of a cluster each finish a share of the tile with one
@@ -19,8 +19,8 @@
 // a fixed order, so the result does not depend on timing.  ACT takes each sum through GELU's tanh form, a
 // squared ReLU, or GELU times a value of the token's row of a table.  With SWIGLU the 16 rows are 8 gate
 // rows followed by their 8 up rows, and the epilogue writes silu(gate) * up: the activation costs
-// no extra pass over memory (reference: src/layer/mlp.cpp:29-36, src/layer/activation.cu:31-33).  Matrices of many rows, and
-// from 9 tokens on most, go through a persistent form with the same sums, gemm_small_stream_kernel below.
+// no extra pass over memory (reference: src/layer/mlp.cpp:29-36, src/layer/activation.cu:31-33).  Matrices of many rows go through a
+// persistent form with the same sums, gemm_small_stream_kernel below, where small_gemm_streams says so.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -107,28 +107,28 @@ __device__ __forceinline__ void small_gemm_finish(const SmallGemmArgs& a, int n0
   }
 }
 
-template <int WARPS, int MT, typename TOut, bool SWIGLU, int ACT>
+template <int RT, int WARPS, int MT, typename TOut, bool SWIGLU, int ACT>
 __global__ void __launch_bounds__(WARPS * 32)
 gemm_small_kernel(const SmallGemmArgs a) {
   constexpr bool X_AHEAD = MT <= 4;                 // (eight tiles of tokens ahead leave room for two blocks of W)
-  constexpr int U = MT <= 2 || !X_AHEAD ? 4 : 2;     // blocks of k in flight
-  constexpr int PER_WARP = MT * 16 * 8;             // sums of a warp: [mt][row][token]
+  constexpr int U = (RT == 1 && MT <= 2) || !X_AHEAD ? 4 : 2;     // blocks of k in flight
+  constexpr int SUMS = MT * 16 * 8, PER_WARP = RT * SUMS;         // sums of a warp: [rt][mt][row][token]
   __shared__ float red[WARPS][PER_WARP];
   cg::cluster_group cluster = cg::this_cluster();
   const int ksplit = gridDim.y, krank = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int n0 = blockIdx.x * 16;
+  const int n0 = blockIdx.x * (16 * RT);
 
   const int total_blocks = (a.K + 31) / 32;
   const int slices = WARPS * ksplit, slice = krank * WARPS + warp;
   const int b_begin = static_cast<int>(static_cast<long long>(total_blocks) * slice / slices);
   const int b_end = static_cast<int>(static_cast<long long>(total_blocks) * (slice + 1) / slices);
 
-  bool w_ok[2];
-  const __nv_bfloat16* w_row[2];
+  bool w_ok[2 * RT];
+  const __nv_bfloat16* w_row[2 * RT];
 #pragma unroll
-  for (int r = 0; r < 2; ++r) {
+  for (int r = 0; r < 2 * RT; ++r) {
     w_ok[r] = n0 + g + 8 * r < a.N;
     w_row[r] = a.w + static_cast<size_t>(w_ok[r] ? n0 + g + 8 * r : 0) * a.ldw + 8 * t;
   }
@@ -148,49 +148,58 @@ gemm_small_kernel(const SmallGemmArgs a) {
     const int row = n0 + lane % 16;
     const char* line = reinterpret_cast<const char*>(a.w + static_cast<size_t>(row) * a.ldw + b_begin * 32) + 128 * (lane / 16);
     const int bytes = (min(b_end * 32, a.K) - b_begin * 32) * 2;
-    for (int at = 128 * (lane / 16); at < bytes; at += 256)
-      if (row < a.N) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(line + (at - 128 * (lane / 16))));
+#pragma unroll
+    for (int rt = 0; rt < RT; ++rt)
+      for (int at = 128 * (lane / 16); at < bytes; at += 256)
+        if (row + 16 * rt < a.N)
+          asm volatile("prefetch.global.L2 [%0];\n" ::"l"(line + static_cast<size_t>(rt) * 16 * a.ldw * 2 + (at - 128 * (lane / 16))));
   }
   wait_for_prior_grids();
   let_dependents_launch();
 
-  float acc[MT][4];
+  float acc[RT][MT][4];
 #pragma unroll
-  for (int mt = 0; mt < MT; ++mt) acc[mt][0] = acc[mt][1] = acc[mt][2] = acc[mt][3] = 0.0f;
+  for (int rt = 0; rt < RT; ++rt)
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) acc[rt][mt][0] = acc[rt][mt][1] = acc[rt][mt][2] = acc[rt][mt][3] = 0.0f;
 
   for (int b = b_begin; b < b_end; b += U) {
-    uint4 wv[U][2], xv[X_AHEAD ? U : 1][X_AHEAD ? MT : 1];
+    uint4 wv[U][2 * RT], xv[X_AHEAD ? U : 1][X_AHEAD ? MT : 1];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int k = (b + u) * 32;
       const bool k_ok = b + u < b_end && k + 8 * t + 8 <= a.K;      // K is a multiple of 8: a chunk is whole or absent
 #pragma unroll
-      for (int r = 0; r < 2; ++r) wv[u][r] = load16_or_zero(w_row[r] + k, w_ok[r] && k_ok);
+      for (int r = 0; r < 2 * RT; ++r) wv[u][r] = load16_or_zero(w_row[r] + k, w_ok[r] && k_ok);
 #pragma unroll
       for (int mt = 0; X_AHEAD && mt < MT; ++mt) xv[u][mt] = load16_or_zero(x_row[mt] + k, x_ok[mt] && k_ok);
     }
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const uint4 wl = wv[u][0], wh = wv[u][1];
-      const unsigned a0[4] = {wl.x, wh.x, wl.y, wh.y};
-      const unsigned a1[4] = {wl.z, wh.z, wl.w, wh.w};
+    for (int u = 0; u < U; ++u)
 #pragma unroll
-      for (int mt = 0; mt < MT; ++mt) {
-        const int k = (b + u) * 32;
-        const uint4 x = X_AHEAD ? xv[X_AHEAD ? u : 0][X_AHEAD ? mt : 0]
-                                : load16_or_zero(x_row[mt] + k, x_ok[mt] && b + u < b_end && k + 8 * t + 8 <= a.K);
-        mma_bf16_16816(acc[mt], a0, x.x, x.y);
-        mma_bf16_16816(acc[mt], a1, x.z, x.w);
+      for (int rt = 0; rt < RT; ++rt) {
+        const uint4 wl = wv[u][2 * rt], wh = wv[u][2 * rt + 1];
+        const unsigned a0[4] = {wl.x, wh.x, wl.y, wh.y};
+        const unsigned a1[4] = {wl.z, wh.z, wl.w, wh.w};
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+          const int k = (b + u) * 32;
+          const uint4 x = X_AHEAD ? xv[X_AHEAD ? u : 0][X_AHEAD ? mt : 0]
+                                  : load16_or_zero(x_row[mt] + k, x_ok[mt] && b + u < b_end && k + 8 * t + 8 <= a.K);
+          mma_bf16_16816(acc[rt][mt], a0, x.x, x.y);
+          mma_bf16_16816(acc[rt][mt], a1, x.z, x.w);
+        }
       }
-    }
   }
 
 #pragma unroll
-  for (int mt = 0; mt < MT; ++mt) {
-    float* at = &red[warp][mt * 128 + g * 8 + 2 * t];
-    *reinterpret_cast<float2*>(at) = make_float2(acc[mt][0], acc[mt][1]);
-    *reinterpret_cast<float2*>(at + 64) = make_float2(acc[mt][2], acc[mt][3]);
-  }
+  for (int rt = 0; rt < RT; ++rt)
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+      float* at = &red[warp][rt * SUMS + mt * 128 + g * 8 + 2 * t];
+      *reinterpret_cast<float2*>(at) = make_float2(acc[rt][mt][0], acc[rt][mt][1]);
+      *reinterpret_cast<float2*>(at + 64) = make_float2(acc[rt][mt][2], acc[rt][mt][3]);
+    }
   __syncthreads();
   // A CTA adds its warps' sums in their order; a cluster's CTAs each finish a share of the tile from the sums of all, in
   // the CTAs' order, which lie in (distributed) shared memory.
@@ -219,7 +228,10 @@ gemm_small_kernel(const SmallGemmArgs a) {
     }
     return sum;
   };
-  small_gemm_finish<MT, TOut, SWIGLU, ACT>(a, n0, krank * WARPS * 32 + threadIdx.x, ksplit * WARPS * 32, total_of);
+#pragma unroll
+  for (int rt = 0; rt < RT; ++rt)
+    small_gemm_finish<MT, TOut, SWIGLU, ACT>(a, n0 + 16 * rt, krank * WARPS * 32 + threadIdx.x, ksplit * WARPS * 32,
+                                             [&](int e) { return total_of(rt * SUMS + e); });
   if (ksplit > 1) cluster.sync();           // nobody leaves while its shared memory may still be read
 }
 
@@ -368,20 +380,39 @@ struct SmallGemmSplit {
   int warps, ksplit;           // of a CTA; CTAs that share K
 };
 
-// Whether the streaming kernel takes a product (its sums are the other kernel's, so that this may look at the number of rows):
-// always from more than four CTAs an SM on; below where its whole rounds of SMs and its one start a product are less than
-// what the other kernel loses to its waits.  Row by row of x in us, the other kernel and this one (matrices from memory,
-// launched one behind the other): 2048 x 2048, 8 rows 4.4 and 4.6, 12 rows 7.2 and 5.4; 1024 x 2048, 12 rows 3.7 and 4.8; 4096 x
-// 4096, 8 rows 9.1 and 9.5, 12 rows 11.9 and 9.2; 4736 x 2048, 12 rows 5.4 and 7.3 (exactly two CTAs an SM of the other), 32
-// rows 11.1 and 8.4; 8192 x 2048, 8 rows 7.7 and 8.2, 12 rows 9.3 and 9.0, 32 rows 13.9 and 11.0; 8192 x 4096, 8 rows 15.9 and
-// 13.2, 12 rows 18.2 and 15.2.
+// Whether the streaming kernel takes a product (its sums are the other kernel's, so that this may look at the number of rows).  It
+// starts later (x and the rings first) and then never waits for a whole burst of loads, so it is ahead where a warp of the other kernel walks
+// several bursts or its CTAs come in more than one round, and behind where one burst or one full round brings all there is.  In us, the
+// other kernel and this one, matrices from memory, launched one behind the other:
+//   more than four tiles of 16 rows an SM (K cut among four warps, bursts of 512 values of k):
+//     8 rows (32 rows of W a CTA, rounds of up to 14 tiles an SM): 65536 x 1024 24.0 and 23.5, 65536 x 512 14.0 and 12.8; 16384 x 1024 9.4
+//     and 7.7, 24576 x 1024 12.8 and 10.1, 32768 x 1024 12.1 and 12.7, 32768 x 1536 18.8 and 18.1; 24576 x 768 9.4 and 8.5, 32768 x 768 9.1
+//     and 10.2; 24576 x 512 7.0 and 7.1, 16384 x 512 4.5 and 5.6; 65536 x 256 8.2 and 8.8;
+//     12 rows (rounds of up to 7 tiles an SM): 20480 x 256 5.9 and 5.2, 65536 x 256 13.0 and 10.6; 16384 x 1024 8.4 and 8.3, 12288 x 768
+//     7.5 and 6.9, 16384 x 768 7.4 and 7.6, 10240 x 512 5.3 and 5.1, 12288 x 512 5.0 and 5.4, 16384 x 512 5.0 and 6.4;
+//     32 rows: 24576 x 512 13.3 and 10.9, 24576 x 256 8.7 and 8.6 (24 rows 7.5 and 7.8); 16384 x 1024 11.6 and 10.6, 16384 x 768 9.2 and 9.3, 10240 x 512 6.8
+//     and 6.3;
+//   fewer tiles (eight warps, and clusters that share K; bursts of 1024):
+//     8 rows: 4864 x 4096 12.5 and 11.0, 8192 x 3072 11.7 and 10.4, 8192 x 2048 7.7 and 8.2;
+//     12 rows: 2048 x 2048 7.2 and 5.4, 2048 x 1536 4.0 and 4.6, 3072 x 1536 7.5 and 6.0, 4096 x 1024 7.2 and 4.9, 2048 x 1024 3.7 and 3.7, 4096 x 768
+//     2.6 and 3.9; 4736 x 2048 5.4 and 7.3 (exactly two CTAs an SM of the other); 8192 x 512 4.8 and 4.4, 8192 x 768 5.2 and 5.6, 8192 x 1024
+//     5.8 and 6.6, 8192 x 1536 8.1 and 7.9;
+//     32 rows: 4096 x 1536 7.6 and 6.9, 4096 x 1024 5.8 and 6.2, 6144 x 1024 7.9 and 7.1, 6144 x 512 5.2 and 5.1 (24 rows 4.7 and 4.9), 8192 x 1024
+//     7.9 and 8.4.
 static bool small_gemm_streams(int N, int K, int token_tiles, const SmallGemmSplit& s) {
   const int tiles = (N + 15) / 16, slices = s.warps * s.ksplit;
   if (slices > 32) return false;
-  if (tiles > 4 * 148) return true;
+  if (tiles > 4 * 148) {
+    if (token_tiles == 1) return tiles > 14 * 148 ? K >= 512 : K >= 1536 || (K >= 768 && tiles <= 12 * 148);
+    if (token_tiles == 2) return tiles > 7 * 148 || K >= 1024 || (K >= 768 && tiles <= 6 * 148) || (K >= 512 && tiles <= 5 * 148);
+    return K >= 1024 || (K >= 512 && (tiles > 7 * 148 || tiles <= 5 * 148));
+  }
   if (token_tiles == 1) return tiles > 2 * 148 && K >= 3072;
-  if (token_tiles == 2) return tiles >= 96 && (tiles < 2 * 148 || tiles > 400);
-  return tiles > 200;
+  if (token_tiles == 2) {
+    if (tiles < 2 * 148) return tiles >= 96 && (K >= 2048 || (K >= 1024 && tiles > 148));
+    return tiles > 400 && (K >= 1536 || K <= 512);
+  }
+  return tiles > 200 && (K >= 1536 || (K >= 768 && tiles > 2 * 148 && tiles <= 400));
 }
 // How K is cut, from the matrix alone: a row's sums are the same whatever rows it is computed with.  Eight warps a CTA and, up
 // to two CTAs an SM, a cluster that shares K (a power of two up to 8, two blocks of k a warp or more): with every warp's loads
@@ -396,10 +427,10 @@ static SmallGemmSplit small_gemm_split(int N, int K) {
   return {8, ksplit};
 }
 
-template <int WARPS, int MT, typename TOut, bool SWIGLU, int ACT>
+template <int RT, int WARPS, int MT, typename TOut, bool SWIGLU, int ACT>
 int small_gemm_launch(const SmallGemmArgs& a, int ksplit, cudaStream_t stream) {
   cudaLaunchConfig_t config = {};
-  config.gridDim = dim3((a.N + 15) / 16, ksplit, 1);
+  config.gridDim = dim3((a.N + 16 * RT - 1) / (16 * RT), ksplit, 1);
   config.blockDim = dim3(WARPS * 32, 1, 1);
   config.dynamicSmemBytes = 0;
   config.stream = stream;
@@ -412,7 +443,7 @@ int small_gemm_launch(const SmallGemmArgs& a, int ksplit, cudaStream_t stream) {
   attribute[1].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attribute;
   config.numAttrs = dependent_launch_enabled() ? 2 : 1;
-  if (cudaLaunchKernelEx(&config, gemm_small_kernel<WARPS, MT, TOut, SWIGLU, ACT>, a) != cudaSuccess) return ERR_CUDA;
+  if (cudaLaunchKernelEx(&config, gemm_small_kernel<RT, WARPS, MT, TOut, SWIGLU, ACT>, a) != cudaSuccess) return ERR_CUDA;
   return launch_result();
 }
 
@@ -455,9 +486,10 @@ int small_gemm_split_launch(const SmallGemmArgs& a, cudaStream_t stream) {
       return small_gemm_stream<8, MT, TOut, SWIGLU, ACT>(a, stream);
     }
   }
-  if constexpr (MT > 4)       // (four warps cut matrices of many rows, which stream up to 32 tokens)
-    if (s.warps == 4) return small_gemm_launch<4, MT, TOut, SWIGLU, ACT>(a, s.ksplit, stream);
-  return small_gemm_launch<8, MT, TOut, SWIGLU, ACT>(a, s.ksplit, stream);
+  if (s.warps == 8) return small_gemm_launch<1, 8, MT, TOut, SWIGLU, ACT>(a, s.ksplit, stream);
+  // Up to 8 tokens 32 rows a CTA read the tokens half as often and are half as many CTAs (151936 x 1024, 4 rows: 50 us against 54; with 12
+  // rows their registers cost more, 66 against 64).  The sums are the same.
+  return small_gemm_launch<MT == 1 ? 2 : 1, 4, MT, TOut, SWIGLU, ACT>(a, s.ksplit, stream);
 }
 
 template <typename TOut, bool SWIGLU, int ACT>
