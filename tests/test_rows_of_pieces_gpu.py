@@ -207,7 +207,7 @@ def test_a_sum_with_a_bias_is_the_sum_behind_the_bias(cuda_device, shape, out_dt
 
 
 @pytest.mark.parametrize("N,K,M,streams", [
-    (32768, 1024, 8, False), (32768, 256, 1, False), (16384, 512, 8, False), (8192, 1024, 12, False), (4096, 512, 16, False), (2048, 768, 9, False),
+    (32768, 1024, 8, True), (32768, 768, 8, False), (32768, 256, 1, False), (16384, 512, 8, False), (8192, 1024, 12, False), (4096, 512, 16, False), (2048, 768, 9, False),
     (8192, 1024, 32, False), (4096, 1024, 24, False), (16384, 512, 12, False), (16384, 1024, 8, True), (65536, 512, 5, True), (4096, 1024, 12, True),
     (8192, 512, 12, True), (20480, 256, 12, True), (6144, 1024, 32, True), (32768, 1536, 8, True), (28448, 768, 3, False), (9504, 768, 4, True), (10240, 512, 30, True), (12288, 512, 30, False)])
 def test_few_rows_take_the_faster_form(cuda_device, N, K, M, streams):

@@ -385,13 +385,14 @@ struct SmallGemmSplit {
 // several bursts or its CTAs come in more than one round, and behind where one burst or one full round brings all there is.  In us, the
 // other kernel and this one, matrices from memory, launched one behind the other:
 //   more than four tiles of 16 rows an SM (K cut among four warps, bursts of 512 values of k):
-//     8 rows (32 rows of W a CTA, rounds of up to 14 tiles an SM): 65536 x 1024 24.0 and 23.5, 65536 x 512 14.0 and 12.8; 16384 x 1024 9.4
-//     and 7.7, 24576 x 1024 12.8 and 10.1, 32768 x 1024 12.1 and 12.7, 32768 x 1536 18.8 and 18.1; 24576 x 768 9.4 and 8.5, 32768 x 768 9.1
-//     and 10.2; 24576 x 512 7.0 and 7.1, 16384 x 512 4.5 and 5.6; 65536 x 256 8.2 and 8.8;
+//     8 rows (32 rows of W a CTA, rounds of up to 14 tiles an SM): 65536 x 1024 24.0 and 23.5, 65536 x 512 14.0 and 12.8; 32768 x 1536 18.8
+//     and 18.1, 16384 x 1024 9.4 and 7.7, 24576 x 1024 12.8 and 10.1, 32768 x 1024 12.1 and 12.7, but as the head of a decode step 15.5 and
+//     15.2 with what follows it 3.7 us earlier (eight requests on four layers 15.68 and 15.52 ms a pass); 24576 x 768 9.4 and 8.5, 32768 x 768
+//     9.1 and 10.2; 24576 x 512 7.0 and 7.1, 16384 x 512 4.5 and 5.6; 65536 x 256 8.2 and 8.8;
 //     12 rows (rounds of up to 7 tiles an SM): 20480 x 256 5.9 and 5.2, 65536 x 256 13.0 and 10.6; 16384 x 1024 8.4 and 8.3, 12288 x 768
 //     7.5 and 6.9, 16384 x 768 7.4 and 7.6, 10240 x 512 5.3 and 5.1, 12288 x 512 5.0 and 5.4, 16384 x 512 5.0 and 6.4;
-//     32 rows: 24576 x 512 13.3 and 10.9, 24576 x 256 8.7 and 8.6 (24 rows 7.5 and 7.8); 16384 x 1024 11.6 and 10.6, 16384 x 768 9.2 and 9.3, 10240 x 512 6.8
-//     and 6.3;
+//     32 rows: 24576 x 512 13.3 and 10.9, 24576 x 256 8.7 and 8.6 (24 rows 7.5 and 7.8); 16384 x 1024 11.6 and 10.6, 16384 x 768 9.2 and 9.3,
+//     10240 x 512 6.8 and 6.3;
 //   fewer tiles (eight warps, and clusters that share K; bursts of 1024):
 //     8 rows: 4864 x 4096 12.5 and 11.0, 8192 x 3072 11.7 and 10.4, 8192 x 2048 7.7 and 8.2;
 //     12 rows: 2048 x 2048 7.2 and 5.4, 2048 x 1536 4.0 and 4.6, 3072 x 1536 7.5 and 6.0, 4096 x 1024 7.2 and 4.9, 2048 x 1024 3.7 and 3.7, 4096 x 768
@@ -403,7 +404,7 @@ static bool small_gemm_streams(int N, int K, int token_tiles, const SmallGemmSpl
   const int tiles = (N + 15) / 16, slices = s.warps * s.ksplit;
   if (slices > 32) return false;
   if (tiles > 4 * 148) {
-    if (token_tiles == 1) return tiles > 14 * 148 ? K >= 512 : K >= 1536 || (K >= 768 && tiles <= 12 * 148);
+    if (token_tiles == 1) return tiles > 14 * 148 ? K >= 512 : K >= 1024 || (K >= 768 && tiles <= 12 * 148);
     if (token_tiles == 2) return tiles > 7 * 148 || K >= 1024 || (K >= 768 && tiles <= 6 * 148) || (K >= 512 && tiles <= 5 * 148);
     return K >= 1024 || (K >= 512 && (tiles > 7 * 148 || tiles <= 5 * 148));
   }
