@@ -47,9 +47,10 @@ __device__ __forceinline__ unsigned pack_bf16(float lo, float hi) {
   return *reinterpret_cast<const unsigned*>(&h);
 }
 
-// x and y as three pairs of bfloat16 values whose sums they are, the largest first.
+// x and y as three pairs of bfloat16 values whose sums they are, the largest first.  A value that would round to infinity keeps the largest
+// bfloat16 as its first part; an infinity's parts are that, itself and a NaN.
 __device__ __forceinline__ void three_parts(float x, float y, unsigned& hi, unsigned& mid, unsigned& lo) {
-  hi = pack_bf16(x, y);
+  asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;\n" : "=r"(hi) : "f"(y), "f"(x));
   x -= __uint_as_float(hi << 16);
   y -= __uint_as_float(hi & 0xffff0000u);
   mid = pack_bf16(x, y);
@@ -57,7 +58,6 @@ __device__ __forceinline__ void three_parts(float x, float y, unsigned& hi, unsi
   y -= __uint_as_float(mid & 0xffff0000u);
   lo = pack_bf16(x, y);
 }
-
 
 // ---- mbarrier and bulk asynchronous copy (the TMA engine, untiled form) -------------------------
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return static_cast<unsigned>(__cvta_generic_to_shared(p)); }
