@@ -9,7 +9,7 @@ from zephyr_b200.kernels.build import SOURCE_DIR
 CONSTANT = {"table", "w", "bias", "q_norm_w", "k_norm_w", "cos_table", "sin_table"}
 OWN = {"out", "q_out"}
 # What kernels index ahead of their wait: arrays of their own (barriers, shared memory, registers), ...
-LOCAL = {"consumed", "empty", "full", "page_ids", "prefix", "qempty", "qfull", "trace", "plans", "place_empty", "place_full", "place_s",
+LOCAL = {"consumed", "empty", "full", "own_full", "page_ids", "prefix", "qempty", "qfull", "trace", "plans", "place_empty", "place_full", "place_s",
          "half_of_row", "bars", "kv_empty", "kv_full", "note", "o_done", "p_full", "s_full", "red", "w_ok", "w_row", "x_ok", "x_row", "falling", "power",
          "wild", "wild_token", "smem", "smem_raw", "smem_unaligned", "f_smem_raw", "gs_smem", "gx_smem_raw", "gf_smem_raw"}
 # ... the step's description, which lies there before its first kernel, weights, and the launch's own arguments.
@@ -68,3 +68,27 @@ def test_kernels_whose_wait_runs_out_let_their_copies_land():
     assert len(copying) >= 7
     for file, name, _, body in copying:
         assert "let_copies_land()" in body, (file, name)
+
+
+def test_the_compiler_keeps_stores_in_front_of_fences_and_arrivals():
+    """A fence, a wait or an arrival that does not name memory to the compiler lets it move plain stores and loads across."""
+    ordering = re.compile(r"fence\.|mbarrier\.(?!init|test|try)|wait_group|barrier\.(cta|cluster)|\bbar\.sync|tcgen05\.(commit|wait|fence)|griddepcontrol\.")
+    seen = 0
+    for path in sorted(SOURCE_DIR.glob("*.cu*")):
+        for statement in re.findall(r"asm volatile\((.*?)\);", re.sub(r"//[^\n]*", "", path.read_text()), re.S):
+            if ordering.search(statement) and "complete_tx" not in statement:
+                seen += 1
+                assert '"memory"' in statement, (path.name, statement)
+    assert seen > 20
+
+
+def test_stores_for_a_pairs_tensor_cores_are_announced_within_their_own_cta():
+    """Behind plain stores that the tensor cores are to read comes an arrival on a barrier of the same CTA: one on the other CTA's barrier is not
+    ordered behind them."""
+    seen = 0
+    for file, name, _, body in kernels():
+        for found in re.finditer(r"fence_proxy_async\(\);", body):
+            arrival = re.search(r"\b(tc_mbar_arrive|mbar_arrive\w*|__syncthreads\w*|signal|bar_sync\w*)\(", body[found.end():])
+            seen += 1
+            assert arrival is None or arrival.group(1) not in ("mbar_arrive_at", "mbar_arrive_in_cluster"), (file, name)
+    assert seen >= 5

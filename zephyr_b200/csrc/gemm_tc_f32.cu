@@ -88,7 +88,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmF32Shape<NT>::TH
   using Shape = GemmF32Shape<NT>;
   constexpr int COLUMNS = Shape::COLUMNS, PER = Shape::PER, X_PART = Shape::X_PART, WARPS = Shape::WARPS, PASS = Shape::PASS;
   extern __shared__ unsigned char gf_smem_raw[];
-  __shared__ unsigned long long full[2], taken, done;
+  __shared__ unsigned long long full[2], taken, done, own_full[2];      // own_full: of the second CTA's own warps
   __shared__ unsigned tmem_base_s;
   __shared__ volatile int failed;
   unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(gf_smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -97,8 +97,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmF32Shape<NT>::TH
   const int m0 = pair % a.tiles_m * NT, n0 = pair / a.tiles_m * (2 * GF_ROWS) + rank * GF_ROWS;
   const int blocks = (a.K + GF_BK - 1) / GF_BK;
   if (tid == 0) {
-    mbar_init(&full[0], 2 * WARPS);
-    mbar_init(&full[1], 2 * WARPS);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&full[i], WARPS + 1);
+      mbar_init(&own_full[i], WARPS);
+    }
     mbar_init(&taken, 2 * WARPS);
     mbar_init(&done, 1);
     failed = 0;
@@ -116,10 +118,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmF32Shape<NT>::TH
   wait_for_prior_grids();
   let_dependents_launch();
 
-  auto arrived = [&](unsigned long long* bar, unsigned parity, int where) -> bool {
+  auto wait = [&](auto look, unsigned long long* bar, unsigned parity, int where) -> bool {
     bool ok = false;
     for (int i = 0; i < GF_WAIT_LIMIT && !ok; ++i) {
-      ok = mbar_try_wait_cluster(bar, parity);
+      ok = look(bar, parity);
       if (!ok && (i & 255) == 255 && failed) break;
     }
     ok = __all_sync(0xffffffffu, ok);
@@ -129,6 +131,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmF32Shape<NT>::TH
     }
     return ok;
   };
+  auto landed = [&](unsigned long long* bar, unsigned parity, int where) { return wait(mbar_try_wait, bar, parity, where); };          // this CTA's own, or a commit's
+  auto arrived = [&](unsigned long long* bar, unsigned parity, int where) { return wait(mbar_try_wait_cluster, bar, parity, where); };
 
   if (warp >= WARPS) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(Shape::OTHER_REGISTERS));
@@ -159,6 +163,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmF32Shape<NT>::TH
           for (int k = 0; k < GF_BK / 16; ++k) tc_mma_pair(tmem_base, w_hi + 2 * k, x_hi + 2 * k, IDESC, k != 0 ? 1u : 0u);
           tc_commit_pair(&done);
         }
+      }
+    } else if (warp == WARPS + 1 && rank == 1) {
+      // The second CTA's stages are announced by a thread that has seen all of its warps' stores arrive in its shared memory, where its tensor
+      // core reads them: a warp's own arrival on the other CTA's barrier is no measure of that.
+      const unsigned at = in_cta_of_rank(smem_u32(&full[0]), 0);
+      for (int b = 0; b < blocks; ++b) {
+        if (!landed(&own_full[b & 1], b >> 1 & 1, 2000000 + b)) break;
+        if (lane == 0) mbar_arrive_at(at + 8 * (b & 1));
       }
     }
   } else {
@@ -223,14 +235,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmF32Shape<NT>::TH
         for (int e = 0; e < RUN; ++e) sum[RUN * i + e] += __uint_as_float(v[i & 1][e]);
       }
     };
-    const unsigned taken_at = in_cta_of_rank(smem_u32(&taken), 0), full_at = in_cta_of_rank(smem_u32(&full[0]), 0);
+    const unsigned taken_at = in_cta_of_rank(smem_u32(&taken), 0);
     auto take = [&](int b) -> bool {           // the hi hi sums of stage b
-      if (!arrived(&done, b & 1, 1000000 + b)) return false;
+      if (!landed(&done, b & 1, 1000000 + b)) return false;
       tc_fence_after_sync();
       add(tmem_base);
       tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive_at(taken_at);
+      if (lane == 0) mbar_arrive_at(taken_at);      // (the sums are in registers, and tensor memory is all that is written behind it)
       return true;
     };
     fetch(0);
@@ -239,7 +251,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmF32Shape<NT>::TH
       store(ring + (b & 1) * Shape::STAGE_BYTES);       // (free: the stage before last's sums have been taken)
       fence_proxy_async();              // the tensor cores read the parts through the asynchronous proxy
       __syncwarp();
-      if (lane == 0) mbar_arrive_at(full_at + 8 * (b & 1));
+      if (lane == 0) tc_mbar_arrive(rank == 0 ? &full[b & 1] : &own_full[b & 1]);
       fetch(b + 1);
       if (b > 0) ok = take(b - 1);
     }

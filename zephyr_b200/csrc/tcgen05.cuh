@@ -145,8 +145,9 @@ __device__ __forceinline__ unsigned in_cta_of_rank(unsigned smem_address, unsign
 __device__ __forceinline__ void mbar_arrive_in_cluster(unsigned cluster_address) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_address) : "memory");
 }
-// One arrival that orders this CTA's accesses only: what the other CTA's thread does after it concerns this CTA's shared and tensor
-// memory through the tensor cores, not through its own loads.  (A release across the cluster waits for every load in flight.)
+// One arrival that orders nothing across the cluster: for a thread behind what is complete in its own SM already (tensor memory's loads that
+// were waited for, shared memory's stores seen through a barrier of the CTA), where what follows is the pair's tensor cores' work
+// on this SM's memory and not the other CTA's loads.  (A release across the cluster costs some 500 cycles, and waits for every load in flight.)
 __device__ __forceinline__ void mbar_arrive_at(unsigned cluster_address) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_address) : "memory");
 }
