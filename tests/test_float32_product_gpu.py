@@ -111,3 +111,25 @@ def test_large_values_weigh_what_their_keys_say(ops, cuda_device, nh, nkv, hd, n
     fine = exact.isfinite()
     assert ((got - exact).abs()[fine] <= 2.0 ** -17 * exact.abs().clamp(min=4.0)[fine]).all()
     assert ((general - exact).abs()[fine] <= 2.0 ** -17 * exact.abs().clamp(min=4.0)[fine]).all()
+
+
+@pytest.mark.parametrize("M,N,K", [(70, 300, 256), (5, 260, 64), (1500, 515, 68), (33, 40, 516)])
+def test_small_values_beside_large_ones(ops, cuda_device, M, N, K):
+    """Values below what three bfloat16 parts hold, whose outputs are of any size because the other operand is large: as exact as multiply-adds, and
+    every other output keeps its bits."""
+    x, w = rand((M, K), torch.float32, cuda_device, 13), rand((N, K), torch.float32, cuda_device, 14)
+    plain = ops.gemm_nt_simt(x, w)
+    rows = [i for i in (0, M // 2, M - 1)]
+    w[1], w[N - 1], w[2], w[N - 2] = w[1] * 2.0 ** 60, w[N - 1] * 1e25, w[2] * 2.0 ** -120, w[N - 2] * 1e-38 * 1e-4
+    w[3], w[4] = w[3] * 1e30, w[4] * 1e16                   # (and values and sums beyond the other end)
+    x[rows[0]] *= 2.0 ** -125
+    x[rows[1]] *= 1e-38
+    x[rows[1]] *= 1e-3
+    x[rows[2]] = 0.0
+    x[rows[2], K - 1] = 1.2345678 * 2.0 ** -120
+    got, exact = ops.gemm_nt_simt(x, w), x.double() @ w.double().T
+    # K products and sums, each within 2^-24 of what is there, above float32's own smallest steps.
+    assert ((got.double() - exact).abs() <= 2.0 ** -24 * K * (x.double().abs() @ w.double().abs().T) + K * 2.0 ** -149).all()
+    assert exact[rows[0], 1].abs() > 2.0 ** -80 and exact[rows[1], N - 1].float() != 0
+    others, columns = [i for i in range(M) if i not in rows], [j for j in range(N) if j not in (1, 2, 3, 4, N - 1, N - 2)]
+    assert torch.equal(got[others][:, columns], plain[others][:, columns])

@@ -6,22 +6,24 @@
 // what mid lo, lo mid and lo lo would add is below 2^-25 of the whole.  The tensor cores cut a sum's last bits at every step, so
 // the sums are kept short: hi hi is summed over 64 values of k in tensor memory, from zero each time, and those sums are added
 // to the total in registers with float32's rounding; the other five, 2^-8 and less of it, are summed over all of K where a cut
-// bit is 2^-8 of one of the total's.  Error against 64 bits (2-norm of the difference over the result's, normal values): 1.05e-7 at
-// K = 1024, 1.5e-7 at 3072, 1.7e-7 at 4096, where multiply-adds in four chains had 2.9e-7, 5.0e-7 and 5.7e-7.  The order of all this is
-// the same whatever M, N and the tile, so a row's result does not depend on the batch around it.
-// A value that is not finite, or that rounds to infinity in bfloat16, makes every output that it meets a NaN, and of a value
-// below 2^-110 the bits below 2^-133 are lost: outputs that are not finite, or below 2^-80, are formed again by multiply-adds.
+// bit is 2^-8 of one of the total's.  Error against 64 bits (2-norm of the difference over the result's, normal values): 3.7e-8 at K = 16,
+// 7.0e-8 at 64, 8.1e-8 at 256, 1.05e-7 at 1024, 1.5e-7 at 3072, 1.7e-7 at 4096, where multiply-adds in four chains had 7.4e-8, 8.4e-8,
+// 1.5e-7, 2.9e-7, 5.0e-7 and 5.7e-7.  The order of all this is the same whatever M, N and the tile, so a row's result does not depend on
+// the batch around it.
+// Values are split times 2^39, with which the parts hold every bit of float32's smallest and no part of an output is below float32's
+// range; a sum is taken back at its end.  A value from 2^88 on, or a sum from 2^50, leaves that range at its other end: outputs that
+// are not finite are formed again by multiply-adds.
 //
 // A pair of SMs (tcgen05.mma.cta_group::2) = 256 rows of w, the tensor cores' row side, by NT rows of x, their columns; each CTA fetches 128
 // and NT / 2 of them.  Per 64 values of k: sixteen warps (eight with 256 columns) fetch the rows as float32 (the next 64 on their way in
 // registers meanwhile), split them and store the parts where the tensor cores read them (K-major, 128-byte swizzle); one thread issues
 // the products of parts, the small ones first, hi hi behind the warps' having taken the sums of the 64 values before; the warps
 // add those to theirs while the next products run.
-// Bound by the tensor cores from 192 columns on (4096^3 587 us, 234 TFLOP/s and six times that of bfloat16
+// Bound by the tensor cores from 192 columns on (4096^3 584 us, 235 TFLOP/s and six times that of bfloat16
 // products, 0.86 of the measured peak; with eight warps 700 us), below by the chain of a stage: fetch, split, 24 products of at least 50
-// cycles, sums.  What it takes beside: 700 x 4096 x 1024 35 us (multiply-adds on CUDA cores 201; eight warps 44), 700 x 1024 x 2048 35
-// (103; 40), 900 x 1024 x 3072 50 (192; 54), 8 x 151936 x 1024 184 (390; 201), one row x 4096 x 1024 19 (19; 20).  On single SMs (128 rows
-// of w by 96) 62 us for the first, bound by the
+// cycles, sums.  What it takes beside: 700 x 4096 x 1024 33 us (multiply-adds on CUDA cores 197; eight warps 44), 700 x 1024 x 2048 33
+// (102; 40), 900 x 1024 x 3072 46 (189; 54), 8 x 151936 x 1024 158 (387; 201), one row x 4096 x 1024 17 (18; 20).  Four stages are little beside
+// the kernel's start and end: one row x 1024 x 256 6.2 (5.3).  On single SMs (128 rows of w by 96) 62 us for the first, bound by the
 // operands' way from L2; arrivals on the pair's barriers with a release across the cluster wait for every load in flight (72 us).
 // Every wait is bounded and reports instead of hanging; tensor memory is given back on every path.
 #include "common.cuh"
@@ -35,8 +37,8 @@ namespace zb {
 
 constexpr int GF_BK = 64;                   // values of k a stage: one 128-byte row of a part
 constexpr int GF_ROWS = 128;                // rows of w of a CTA
+constexpr int GF_AHEAD = 4;                  // stages of w that L2 is asked for ahead
 constexpr int GF_WAIT_LIMIT = 1 << 18;
-constexpr float GF_SMALLEST = 8.3e-25f;      // 2^-80
 constexpr int GF_W_PART = GF_ROWS * GF_BK * 2;
 
 template <int NT> struct GemmF32Shape {
@@ -187,6 +189,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmF32Shape<NT>::TH
       if (PASS * u < GF_ROWS ? n0 + r < a.N : x0 + r - GF_ROWS < a.M && r - GF_ROWS < Shape::X_ROWS) present |= 1u << u;
     }
     float4 ahead[PER][2];
+    // Up to 64 rows of x (in tiles of up to 64 columns) a stage is the time of its fetches, which is short from L2: w's rows are asked for that far
+    // ahead.  (One row x 4096 x 1024 19.6 -> 17.0 us, 64 x 1024 x 2048 34 -> 30; with more rows it costs 2 to 5 %.)
+    auto ask = [&](int b) {
+      if (a.M > 64) return;
+#pragma unroll
+      for (int u = 0; u < (NT <= 64 ? GF_ROWS / PASS : 0); ++u)
+        if (c < 2 && (present >> u & 1) && b * GF_BK + 32 * c < a.K)
+          asm volatile("prefetch.global.L2 [%0];\n" ::"l"(w_row + PASS * u * a.ldw + b * GF_BK + 28 * c));
+    };
     auto fetch = [&](int b) {
 #pragma unroll
       for (int u = 0; u < PER; ++u)
@@ -208,10 +219,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmF32Shape<NT>::TH
         const int part = of_w ? GF_W_PART : X_PART;
         const float4 p = ahead[u][0], q = ahead[u][1];
         uint4 hi, mid, lo;
-        three_parts(p.x, p.y, hi.x, mid.x, lo.x);
-        three_parts(p.z, p.w, hi.y, mid.y, lo.y);
-        three_parts(q.x, q.y, hi.z, mid.z, lo.z);
-        three_parts(q.z, q.w, hi.w, mid.w, lo.w);
+        three_parts_scaled(p.x, p.y, hi.x, mid.x, lo.x);
+        three_parts_scaled(p.z, p.w, hi.y, mid.y, lo.y);
+        three_parts_scaled(q.x, q.y, hi.z, mid.z, lo.z);
+        three_parts_scaled(q.z, q.w, hi.w, mid.w, lo.w);
         *reinterpret_cast<uint4*>(to) = hi;
         *reinterpret_cast<uint4*>(to + part) = mid;
         *reinterpret_cast<uint4*>(to + 2 * part) = lo;
@@ -246,6 +257,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmF32Shape<NT>::TH
       return true;
     };
     fetch(0);
+    for (int b = 1; b < GF_AHEAD; ++b) ask(b);
     bool ok = true;
     for (int b = 0; b < blocks && ok; ++b) {
       store(ring + (b & 1) * Shape::STAGE_BYTES);       // (free: the stage before last's sums have been taken)
@@ -253,6 +265,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmF32Shape<NT>::TH
       __syncwarp();
       if (lane == 0) tc_mbar_arrive(rank == 0 ? &full[b & 1] : &own_full[b & 1]);
       fetch(b + 1);
+      ask(b + GF_AHEAD);
       if (b > 0) ok = take(b - 1);
     }
     if (ok && take(blocks - 1)) {
@@ -263,8 +276,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmF32Shape<NT>::TH
       for (int i = 0; i < COLUMNS; ++i) {
         const int m = m0 + column0 + i;
         if (n >= a.N || m >= a.M) continue;
-        float v = sum[i];
-        if (!(fabsf(v) <= 3.4e38f) || (v != 0.0f && fabsf(v) < GF_SMALLEST)) v = dot_f32(a.x + m * a.ldx, a.w + n * a.ldw, a.K);
+        float v = sum[i] * PARTS_UNSCALE;
+        if (!(fabsf(sum[i]) <= 3.4e38f)) v = dot_f32(a.x + m * a.ldx, a.w + n * a.ldw, a.K);
         to[m * a.ldy] = v;
       }
     }
@@ -311,8 +324,8 @@ ZB_API int zb_gemm_nt_f32(float* y, const float* x, const float* w, int M, int N
   GemmF32Args a;
   a.y = y; a.x = x; a.w = w; a.M = M; a.N = N; a.K = K; a.ldx = ldx; a.ldw = ldw; a.ldy = ldy; a.status = status;
   // The tile whose rounds over the pairs of SMs take the least time (us of a full round at K = 1024, whatever K's share of it):
-  // 700 x 4096 x 1024 is one round of 64 pairs with 192 columns, 35 us (256: 49, 128: 48, 96: 45); 700 x 1024 x 2048 44 pairs with 64,
-  // 35 (32: 59, 96: 36); 2048 x 6144 x 1024 four rounds with 192, 133 (256: 140, 128: 141); 8 x 151936 x 1024 with 32, 184.
+  // 700 x 4096 x 1024 is one round of 64 pairs with 192 columns, 33 us (before the last change 35; 256: 49, 128: 48, 96: 45); 700 x 1024 x 2048 44
+  // pairs with 64, 33 (35; 32: 59, 96: 36); 2048 x 6144 x 1024 four rounds with 192, 129 (133; 256: 140, 128: 141); 8 x 151936 x 1024 with 32, 158.
   struct Tile { int columns, us; };
   constexpr Tile tiles[] = {{32, 17}, {64, 19}, {96, 21}, {128, 23}, {160, 28}, {192, 32}, {256, 46}};
   const long long row_blocks = (N + 2LL * GF_ROWS - 1) / (2 * GF_ROWS);

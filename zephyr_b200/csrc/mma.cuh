@@ -47,16 +47,37 @@ __device__ __forceinline__ unsigned pack_bf16(float lo, float hi) {
   return *reinterpret_cast<const unsigned*>(&h);
 }
 
-// x and y as three pairs of bfloat16 values whose sums they are, the largest first.  A value that would round to infinity keeps the largest
-// bfloat16 as its first part; an infinity's parts are that, itself and a NaN.
+// a * b + c of two values in one instruction, each with one rounding.
+__device__ __forceinline__ float2 fma_pair(float2 a, float2 b, float2 c) {
+  float2 r;
+  asm("{\n.reg .b64 a, b, c;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nmov.b64 c, {%6, %7};\nfma.rn.f32x2 a, a, b, c;\nmov.b64 {%0, %1}, a;\n}\n"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return r;
+}
+__device__ __forceinline__ float2 mul_pair(float2 a, float2 b) {
+  float2 r;
+  asm("{\n.reg .b64 a, b;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nmul.rn.f32x2 a, a, b;\nmov.b64 {%0, %1}, a;\n}\n"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+
+// x and y as three pairs of bfloat16 values whose sums they are (of a value below 2^-110 the bits below 2^-133 are lost), the largest first.  A
+// value that would round to infinity keeps the largest bfloat16 as its first part; an infinity's parts are that, itself and a NaN.
 __device__ __forceinline__ void three_parts(float x, float y, unsigned& hi, unsigned& mid, unsigned& lo) {
+  const float2 minus = make_float2(-1.0f, -1.0f);
   asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;\n" : "=r"(hi) : "f"(y), "f"(x));
-  x -= __uint_as_float(hi << 16);
-  y -= __uint_as_float(hi & 0xffff0000u);
-  mid = pack_bf16(x, y);
-  x -= __uint_as_float(mid << 16);
-  y -= __uint_as_float(mid & 0xffff0000u);
-  lo = pack_bf16(x, y);
+  float2 rest = fma_pair(make_float2(__uint_as_float(hi << 16), __uint_as_float(hi & 0xffff0000u)), minus, make_float2(x, y));
+  mid = pack_bf16(rest.x, rest.y);
+  rest = fma_pair(make_float2(__uint_as_float(mid << 16), __uint_as_float(mid & 0xffff0000u)), minus, rest);
+  lo = pack_bf16(rest.x, rest.y);
+}
+
+// The same of x and y times 2^39 = PARTS_SCALE: all bits of every float32 value below 2^88, also of the smallest; a larger one gives a NaN.
+// PARTS_UNSCALE takes a product of two such values back.
+constexpr float PARTS_SCALE = 549755813888.0f, PARTS_UNSCALE = 3.308722450212111e-24f;        // 2^39, 2^-78
+__device__ __forceinline__ void three_parts_scaled(float x, float y, unsigned& hi, unsigned& mid, unsigned& lo) {
+  const float2 scaled = mul_pair(make_float2(x, y), make_float2(PARTS_SCALE, PARTS_SCALE));
+  three_parts(scaled.x, scaled.y, hi, mid, lo);
 }
 
 // ---- mbarrier and bulk asynchronous copy (the TMA engine, untiled form) -------------------------
