@@ -133,3 +133,20 @@ def test_small_values_beside_large_ones(ops, cuda_device, M, N, K):
     assert exact[rows[0], 1].abs() > 2.0 ** -80 and exact[rows[1], N - 1].float() != 0
     others, columns = [i for i in range(M) if i not in rows], [j for j in range(N) if j not in (1, 2, 3, 4, N - 1, N - 2)]
     assert torch.equal(got[others][:, columns], plain[others][:, columns])
+
+
+@pytest.mark.parametrize("key,query,value", [(-122, 60, 0), (0, 0, -122), (-60, 20, 39), (20, 15, 41), (-140, 120, -10), (60, -122, 0)])
+def test_attention_holds_values_of_any_size(ops, cuda_device, key, query, value):
+    """Keys, queries and values times powers of two, with a scale that takes the scores back: as near the exact averages as ordinary ones."""
+    nh, nkv, hd, n, ctx = 4, 2, 68, 70, 100
+    q, cache, meta, Ks, Vs, qs = build_paged_case(cuda_device, torch.float32, nh, nkv, hd, 16, [n], [ctx], 21)
+    held = cache.clone()
+    held[:, 0], held[:, 1], q = held[:, 0] * 2.0 ** (key / 2) * 2.0 ** (key / 2), held[:, 1] * 2.0 ** value, q * 2.0 ** query
+    K, V = Ks[0] * 2.0 ** (key / 2) * 2.0 ** (key / 2), Vs[0] * 2.0 ** value
+    status, wide, scale = ops.new_status(cuda_device), ops.paged_prefill_tile_tokens(), 2.0 ** -(key + query) / math.sqrt(hd)
+    out = torch.empty_like(q)
+    ops.paged_attention_f32(q, held, meta["table"], *tiles_for([n], wide, cuda_device), wide, meta["row_q_start"], meta["row_q_len"], meta["row_ctx"],
+                            nh, nkv, hd, 0, scale, status, out)
+    ops.check_status(status)
+    exact = ref_attention_row(qs[0].double(), K.double() * 2.0 ** -key, V.double(), ctx, n, 0, nh, nkv).view(n, -1)
+    assert (out.double().cpu() - exact).norm() <= 32 * 2.0 ** -23 * exact.norm()

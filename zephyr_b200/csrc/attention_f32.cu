@@ -13,14 +13,16 @@
 //   totals; this step's values, split, to shared memory and the weights' parts to tensor memory, where the scores lay, upon which
 //   the weighted values of this step are issued.
 // Keys and values of the next step are on their way in registers meanwhile.  What does not lie in [lo, hi) comes as zeros.
-// A key's scores that are not finite are formed again by multiply-adds; a value that is not finite is left out of the product and
-// added by hand to the rows whose weight for it is not zero, so that it stays with those that see it.
+// All are split times 2^39 (gemm_tc_f32.cu), which the scores' scale and the totals take back.  Scores that are not finite then are formed
+// again by multiply-adds; a value beyond 2^40, or not finite, is left out of the product and added by hand to the rows whose weight
+// for it is not zero, so that it stays with those that see it.
 // Bound by the eight warps' part of a step, some 6500 cycles, of which the tensor cores' 72 products take 3900: scores' reads 400, maximum
 // and weights 1800, both splits 1600, values' sums 450, fetches 800.  (With the maximum taken under a branch per score, and every thread
 // looking its keys' pages up by divisions, 12000; registers spilled to an L1 of the 28 KB that the CTA's shared memory leaves,
 // 7500.)
-// 700 tokens, 16 heads over 8 of 128: 53 us (multiply-adds on CUDA cores, 64 pairs a CTA, 122); 4000 tokens 420 (1680); two tokens
-// behind a context of 600 42 (97), two tokens of a new prompt 12.4 (17.5), eight rows of sixteen 12.9 (24); 700 tokens of width 64 40 (72).
+// 700 tokens, 16 heads over 8 of 128: 54 us (multiply-adds on CUDA cores, 64 pairs a CTA, 122); 4000 tokens 428 (1680); two tokens
+// behind a context of 600 44 (97), two tokens of a new prompt 12.4 (17.5), eight rows of sixteen 12.8 (24); 700 tokens of width 64 40 (72).
+// (Splitting without the factor, which loses the last bits of values below 2^-110: 52.6 and 419.)
 // Every row with several tokens runs here, so that its result hangs on that row alone.
 //
 // Masks: causal, a window, a chunk (key and query in the same run of `chunk` positions); `sinks` join the softmax's
@@ -86,18 +88,19 @@ __device__ __forceinline__ bool f32_workers_any(bool any) {
   return r != 0;
 }
 
-// Eight values (two runs of four) as 16-byte pieces of their three parts.
+// Eight values (two runs of four) as 16-byte pieces of their three parts, times 2^39.
 __device__ __forceinline__ void f32_store_parts(float4 p, float4 q, unsigned char* to, int part) {
   unsigned hi[4], mid[4], lo[4];
   const float x[4] = {p.x, p.z, q.x, q.z}, y[4] = {p.y, p.w, q.y, q.w};
 #pragma unroll
-  for (int i = 0; i < 4; ++i) three_parts(x[i], y[i], hi[i], mid[i], lo[i]);
+  for (int i = 0; i < 4; ++i) three_parts_scaled(x[i], y[i], hi[i], mid[i], lo[i]);
   *reinterpret_cast<uint4*>(to) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
   *reinterpret_cast<uint4*>(to + part) = make_uint4(mid[0], mid[1], mid[2], mid[3]);
   *reinterpret_cast<uint4*>(to + 2 * part) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
 }
 
-__device__ __forceinline__ float zero_if_wild(float x) { return fabsf(x) <= 3.3e38f ? x : 0.0f; }
+constexpr float F_LARGEST = 1.0995116e12f;      // 2^40: 64 of them times weights of one stay below float32's end, both times 2^39
+__device__ __forceinline__ float zero_if_wild(float x) { return fabsf(x) <= F_LARGEST ? x : 0.0f; }
 
 template <int D>
 __global__ void __launch_bounds__(F_THREADS, 1) paged_attention_f32_kernel(const AttentionF32Args a) {
@@ -318,7 +321,7 @@ __global__ void __launch_bounds__(F_THREADS, 1) paged_attention_f32_kernel(const
         tmem_wait_ld16(x);
         tmem_wait_ld16(y);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) acc[i0 + i] = (acc[i0 + i] + (__uint_as_float(x[i]) + __uint_as_float(y[i]))) * by;
+        for (int i = 0; i < 16; ++i) acc[i0 + i] = fmaf(__uint_as_float(x[i]) + __uint_as_float(y[i]), PARTS_UNSCALE, acc[i0 + i]) * by;
       }
     };
     // Column i of the thread's output is this value of the row.
@@ -331,6 +334,7 @@ __global__ void __launch_bounds__(F_THREADS, 1) paged_attention_f32_kernel(const
       ok = arrived(&s_done, i & 1, 2000000 + i) && ok;
       tc_fence_after_sync();
       const unsigned tmem_s = tmem_base + lane_base + (i & 1) * 128;
+      const float score_scale = a.scale * PARTS_UNSCALE;
       float s[32];
       {
         float check = 0.0f;
@@ -343,7 +347,7 @@ __global__ void __launch_bounds__(F_THREADS, 1) paged_attention_f32_kernel(const
           tmem_wait_ld16(y);
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
-            s[j0 + j] = __uint_as_float(x[j]) + __uint_as_float(y[j]);
+            s[j0 + j] = (__uint_as_float(x[j]) + __uint_as_float(y[j])) * score_scale;
             check = fmaf(0.0f, s[j0 + j], check);
           }
         }
@@ -358,12 +362,10 @@ __global__ void __launch_bounds__(F_THREADS, 1) paged_attention_f32_kernel(const
             for (int e = 0; place >= 0 && e < d; ++e) sum = fmaf(q[e], k[kv_element_index(e, pos, d, 4)], sum);
 #pragma unroll
             for (int w = 0; w < 32; ++w)
-              if (w == j && !(fabsf(s[w]) <= 3.4e38f)) s[w] = sum;
+              if (w == j && !(fabsf(s[w]) <= 3.4e38f)) s[w] = sum * a.scale;
           }
         }
       }
-#pragma unroll
-      for (int j = 0; j < 32; ++j) s[j] *= a.scale;
       if (a.softcap > 0.0f) {
 #pragma unroll
         for (int j = 0; j < 32; ++j) s[j] = a.softcap * tanhf(s[j] / a.softcap);
@@ -387,7 +389,7 @@ __global__ void __launch_bounds__(F_THREADS, 1) paged_attention_f32_kernel(const
 #pragma unroll
           for (int e = 0; e < 4; ++e) largest = max(largest, __float_as_uint(reinterpret_cast<const float*>(&values[u][w])[e]) << 1);
       tc_fence_before_sync();           // (the halves' weights go where the other half's scores lay)
-      const bool rare = f32_workers_any(!ok || largest > __float_as_uint(3.3e38f) << 1);
+      const bool rare = f32_workers_any(!ok || largest > __float_as_uint(F_LARGEST) << 1);
       tc_fence_after_sync();
       const float new_m = fmaxf(m, fmaxf(top, half_of_row[half ^ 1][r]));
       // (a row that has seen no key yet keeps zeros: its weights are exp(-inf) of a finite difference)
@@ -451,7 +453,7 @@ __global__ void __launch_bounds__(F_THREADS, 1) paged_attention_f32_kernel(const
       {
         unsigned part[3][16];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) three_parts(s[2 * j], s[2 * j + 1], part[0][j], part[1][j], part[2][j]);
+        for (int j = 0; j < 16; ++j) three_parts_scaled(s[2 * j], s[2 * j + 1], part[0][j], part[1][j], part[2][j]);
 #pragma unroll
         for (int e = 0; e < 3; ++e) tmem_st16(tmem_s + 32 * e + 16 * half, part[e]);
         tc_wait_st();
