@@ -93,3 +93,22 @@ def test_a_value_that_is_not_finite_stays_with_later_tokens(cuda_device, dim, vd
         assert torch.equal(got[~touched], clean[~touched]), bad
         untouched = ~torch.isin(torch.arange(heads * vdim, device=cuda_device), torch.tensor([c for _, c in bad], device=cuda_device)).view(heads, 1, vdim)
         assert torch.equal(state[untouched.expand_as(state)], behind[untouched.expand_as(behind)]), bad
+
+
+# (heads, key channels, value columns, rows, in pieces of 128): us walked and in passes, rotation included.
+MEASURED = [((16, 128, 128, [1024, 1024], True), 61.0, 93.7), ((16, 128, 128, [1400, 600], True), 72.7, 93.2), ((16, 128, 128, [700, 400], True), 39.5, 49.0),
+            ((16, 128, 128, [1500, 40, 40, 40], True), 74.0, 85.3), ((16, 128, 128, [1500] + [1] * 10, True), 78.8, 96.1),
+            ((32, 128, 128, [64] * 16, True), 105.0, 137.8), ((8, 128, 128, [1500, 548], False), 49.6, 58.3), ((8, 128, 128, [1500] + [1] * 10, True), 65.0, 55.4),
+            ((5, 100, 132, [300] * 6, True), 26.0, 46.9), ((5, 100, 132, [2048], False), 64.5, 51.7), ((4, 128, 128, [1000], False), 34.5, 24.8),
+            ((2, 128, 128, [1500, 548], False), 45.7, 26.4), ((16, 64, 128, [1000], False), 28.7, 41.2), ((16, 64, 128, [1500] + [1] * 10, False), 77.3, 62.4),
+            ((4, 64, 64, [2048], False), 43.9, 23.6), ((2, 64, 32, [500], False), 18.2, 19.7)]
+
+
+@pytest.mark.parametrize("sizes,walked,passes", MEASURED)
+def test_steps_take_the_sooner_of_walk_and_passes(cuda_device, sizes, walked, passes):
+    from zephyr_b200.kernels import ops
+    from zephyr_b200.parts.recurrent import retention_walks
+
+    heads, dim, vdim, lengths, tensor_memory = sizes
+    assert ops.retention_in_tensor_memory(len(lengths), sum(lengths), heads, dim, vdim, dim // 2 // 32 * 64) == tensor_memory
+    assert retention_walks(lengths, heads, dim, vdim, tensor_memory) == (walked < passes)

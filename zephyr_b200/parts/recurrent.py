@@ -44,7 +44,7 @@ kernels (csrc/recurrent.cu); projections and the convolution's output have the m
 from __future__ import annotations
 
 import dataclasses
-from typing import Mapping
+from typing import Mapping, Sequence
 
 import torch
 
@@ -298,22 +298,40 @@ class GatedDeltaRule(Mixer):
         return ops.linear(normed, self.w_o, out_dtype=out_dtype)
 
 
+def retention_walks(lengths: Sequence[int], heads: int, dim: int, vdim: int, tensor_memory: bool) -> bool:
+    """Whether rows of these lengths run as a walk, pieces one behind the other with the state on the SM, or in passes over all pieces at once,
+    whichever these estimates (us, measured with the rotation in front, within some 10 %) say is sooner.  The walk in pieces of 128 tokens
+    (``tensor_memory``) is a CTA a row, head and 64 value columns: 8 us and 4.2 a piece, and what splits the operands.  That in pieces of 64
+    is one of 16 columns: 1.25 us a piece of the longest row (1.05 with up to 64 key channels) and what prepares the pieces; nearly two CTAs
+    an SM run in turn; CTAs of 32 columns, where they would be more, 2.7 us a piece.  The passes take a token and head's time for
+    padded channels, a row's state, and no less than 20.  (Walk / passes: 16 heads of 128 x 128, rows of 1024 and 1024 61 / 94, 1500 and
+    three of 40 74 / 85, one of 2048 79 / 94; 32 heads, sixteen rows of 64 105 / 138; 8 heads, one of 2048 61 / 58, 1500 and 548 50 / 58, 1500 and ten
+    of one 65 / 55; 4 heads, one of 1000 35 / 25; 16 heads of 64 x 128, one of 1000 29 / 41.)"""
+    tokens, longest, small = sum(lengths), max(lengths), dim <= 64
+    size = -(-dim // 64) * -(-vdim // 64) / 4
+    passes = max(19.5 if small else 22.5, 10.0 + 2.7e-3 * tokens * heads * (0.26 + 0.74 * size) + 0.05 * len(lengths) * heads * size)
+    if tensor_memory:
+        ctas = [8.0 + 4.2 * -(-n // 128) for n in lengths]
+        return 4.0 + max(max(ctas), 1.15 * heads * -(-vdim // 64) * sum(ctas) / 148) + 3.5e-4 * tokens * heads <= passes
+    ctas, pieces = len(lengths) * heads * -(-vdim // 16), -(-longest // 64)
+    if ctas <= 1.5 * 148:
+        walked = 9.0 + 1.05 * pieces + 3e-4 * tokens * heads if small else 12.0 + 1.25 * pieces + 6.5e-4 * tokens * heads
+    elif ctas <= 2 * 148:
+        walked = 9.0 + 1.7 * sum(sorted(lengths)[-2:]) / 64
+    else:
+        walked = 9.0 + 2.7 * pieces
+    return walked <= passes
+
+
 class Retention(Mixer):
     graph_safe = True
     takes_out_dtype = True
 
     PIECES_FROM = 64      # new tokens per request, on average, from which on a step runs in pieces
-    # A step's pieces are walked one behind the other with the state on the SM, or in passes over all pieces at once.  The walk
-    # takes 1.75 us a piece of the longest row; 2.4 us a piece of the two longest where its CTAs of 16 value columns are nearly two
-    # an SM, which run in turn; 2.7 us in CTAs of 32, where they would be more.  The passes take 1.66 ns a token and 128 x 128
-    # values of state, and 10 us, more than the walk beside that (one row of 1024 tokens: 16 heads of 128 x 128: 44 us walked, 51 in
-    # passes; 5 of 100 x 130: 48 and 29; 2 of 64 x 32: 31 and 18; one row of 256, 2 of 64 x 32: 16 and 17; the layer with a row of
-    # 1500 beside ten single tokens, 16 heads: 186 and 162, with rows of 700 and 400: 110 and 104).
     def _walks(self, ctx: StepContext) -> bool:
-        lengths = sorted(ctx.host_q_len or [ctx.num_tokens])
-        ctas = ctx.num_rows * self.heads * -(-self.vdim // 16)
-        walked = (1.75 * lengths[-1] if ctas <= 1.5 * 148 else 2.4 * sum(lengths[-2:]) if ctas <= 2 * 148 else 2.7 * lengths[-1]) / 64
-        return walked <= 10.0 + 1.66e-3 * ctx.num_tokens * self.heads * (self.dim * self.vdim / 128 ** 2)
+        lengths = ctx.host_q_len or [ctx.num_tokens] + [0] * (ctx.num_rows - 1)
+        return retention_walks(lengths, self.heads, self.dim, self.vdim,
+                               ops.retention_in_tensor_memory(len(lengths), sum(lengths), self.heads, self.dim, self.vdim, self.rot_dims))
 
     def __init__(self, spec: MixerSpec, weights: Mapping[str, torch.Tensor], dtype: torch.dtype,
                  device: torch.device | str):
