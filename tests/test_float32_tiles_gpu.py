@@ -1,5 +1,6 @@
-"""The 32-bit kernels that work in register tiles, alone: the product at the edges of its tiles and of its slices of k, and
-the attention over rows with several tokens against the general kernel and a plain float64 attention."""
+"""The 32-bit kernels alone: the product at the edges of its tiles and of its slices of k (on the tensor cores where rows start on 16-byte
+boundaries, in register tiles elsewhere), and the attention over rows with several tokens against the general kernel and a plain
+float64 attention."""
 
 import math
 

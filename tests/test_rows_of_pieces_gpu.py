@@ -234,3 +234,26 @@ def test_few_rows_take_the_faster_form(cuda_device, N, K, M, streams):
         pair = got.view(M, N // 16, 2, 8)
         gated = ops.gemm_small(x, w, out_dtype=torch.float32, swiglu=True).view(M, N // 16, 8)
         assert (gated - torch.nn.functional.silu(pair[:, :, 0]) * pair[:, :, 1]).abs().max() <= 2.0 ** -21 * max(1.0, float(got.abs().max())) ** 2
+
+
+@pytest.mark.parametrize("first,last,step", [(0x00000000, 0x7f800000, 1021), (0x80000000, 0xff800000, 1021), (0xc2ac0000, 0xc2d10000, 1),
+                                             (0x80000000, 0x80200000, 1), (0x00000000, 0x00200000, 1), (0xc1000000, 0xc1100000, 1)])
+def test_the_activation_over_float32(cuda_device, first, last, step):
+    """z / (1 + e^-z) alone, as a convolution of one tap of weight 1, over float32's bit patterns: all magnitudes of either sign, and every value of -86 to
+    -104.5 (where 1 + e^-z leaves float32, below which the quotient is a zero), of the smallest, and of some ordinary ones."""
+    from zephyr_b200.kernels import ops
+
+    bits = torch.arange(first, last, step, dtype=torch.int64, device=cuda_device)
+    z = torch.where(bits >= 2 ** 31, bits - 2 ** 32, bits).to(torch.int32).view(torch.float32)
+    channels = 4096
+    z = z[:len(z) // channels * channels].view(-1, channels)
+    T, i32 = z.shape[0], lambda values: torch.tensor(values, dtype=torch.int32, device=cuda_device)
+    got = ops.causal_conv_silu(z, channels, torch.ones(channels, 1, device=cuda_device), torch.zeros(channels, device=cuda_device),
+                               torch.zeros(1, 0, device=cuda_device), i32([0]), i32([0]), i32([T]), i32([0] * T), ops.new_status(cuda_device)).double()
+    e = torch.exp(-z.double())
+    edge = (z.double() + 88.72283905206835).abs() < 1e-4                      # where e^-z is float32's largest
+    want = z.double() / (1.0 + torch.where(e > torch.finfo(torch.float32).max, torch.inf, e))
+    # The exponential within two steps of 2^-23, its sum and the quotient half a step each; where 1 + e^-z has no more than a few bits as an inverse
+    # the correction still has all of them.  Results below float32's normal values: one of their steps.
+    assert ((got - want).abs() <= 3.5 * 2.0 ** -23 * want.abs() + 2.0 ** -149)[~edge].all()
+    assert (got[edge].abs() <= 1e-36).all()

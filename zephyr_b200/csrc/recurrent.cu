@@ -25,7 +25,7 @@
 namespace zb {
 
 // z / (1 + e^-z).  The quotient is the reciprocal's estimate times z, corrected once by its remainder (fused, so exact to
-// rounding, after Markstein: of all 2^32 inputs one differs from the divide operator's result): that operator's guarded form
+// rounding, after Markstein: of all 2^32 inputs none differs from the divide operator's result): that operator's guarded form
 // kept a thread's values one behind the other.  Where the correction has no
 // meaning (an infinite z or e^-z), the uncorrected product is the quotient.
 __device__ __forceinline__ float silu_f(float z) {

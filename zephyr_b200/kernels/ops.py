@@ -1766,7 +1766,7 @@ def gemm_nt_simt(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None
     _require(out.shape == (M, N) and out.dtype == out_dtype and out.stride(1) == 1, "out must be [M, N]")
     if x.dtype == out_dtype == torch.float32:
         _check(library().zb_gemm_nt_f32(_ptr(out), _ptr(x), _ptr(w), M, N, K, x.stride(0), w.stride(0), out.stride(0),
-                                        _ptr(device_status(x.device)), _stream()), "gemm_nt_simt")
+                                        _ptr(device_status(x.device)), _stream()), "gemm_nt_f32")
         return out
     _check(library().zb_gemm_nt_simt(_ptr(out), _ptr(x), _ptr(w), M, N, K, x.stride(0), w.stride(0), out.stride(0),
                                      DTYPE_CODE[x.dtype], DTYPE_CODE[out_dtype], _stream()), "gemm_nt_simt")
