@@ -150,3 +150,16 @@ def test_attention_holds_values_of_any_size(ops, cuda_device, key, query, value)
     ops.check_status(status)
     exact = ref_attention_row(qs[0].double(), K.double() * 2.0 ** -key, V.double(), ctx, n, 0, nh, nkv).view(n, -1)
     assert (out.double().cpu() - exact).norm() <= 32 * 2.0 ** -23 * exact.norm()
+
+
+def test_a_first_product_inside_a_capture(ops, cuda_device, monkeypatch):
+    """A graph captured ahead of any other call of the process makes no state that outlives it."""
+    x, w = rand((5, 64), torch.float32, cuda_device, 1), rand((70, 64), torch.float32, cuda_device, 2)
+    want = ops.gemm_nt_simt(x, w)
+    monkeypatch.setattr(ops, "_device_status", {})
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = ops.gemm_nt_simt(x, w)
+    assert not ops._device_status
+    graph.replay()
+    assert torch.equal(got, want)

@@ -349,6 +349,14 @@ def device_status(device: torch.device | str) -> torch.Tensor:
     return word
 
 
+def _device_status_pointer(device: torch.device) -> int | None:
+    """Its address for a kernel that is called without one.  A capture that finds no word yet makes none, whose memory and zeros would be that
+    graph's; the kernel then reports nowhere."""
+    if device not in _device_status and torch.cuda.is_current_stream_capturing():
+        return None
+    return _ptr(device_status(device))
+
+
 def check_status(status: torch.Tensor, where: str = "step") -> None:
     """Read the status word (this synchronises) and raise if a kernel reported an error."""
     code, detail, index, _ = status.tolist()
@@ -1766,7 +1774,7 @@ def gemm_nt_simt(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None
     _require(out.shape == (M, N) and out.dtype == out_dtype and out.stride(1) == 1, "out must be [M, N]")
     if x.dtype == out_dtype == torch.float32:
         _check(library().zb_gemm_nt_f32(_ptr(out), _ptr(x), _ptr(w), M, N, K, x.stride(0), w.stride(0), out.stride(0),
-                                        _ptr(device_status(x.device)), _stream()), "gemm_nt_f32")
+                                        _device_status_pointer(x.device), _stream()), "gemm_nt_f32")
         return out
     _check(library().zb_gemm_nt_simt(_ptr(out), _ptr(x), _ptr(w), M, N, K, x.stride(0), w.stride(0), out.stride(0),
                                      DTYPE_CODE[x.dtype], DTYPE_CODE[out_dtype], _stream()), "gemm_nt_simt")
