@@ -19,12 +19,14 @@
 // registers meanwhile), split them and store the parts where the tensor cores read them (K-major, 128-byte swizzle); one thread issues
 // the products of parts, the small ones first, hi hi behind the warps' having taken the sums of the 64 values before; the warps
 // add those to theirs while the next products run.
-// Bound by the tensor cores from 192 columns on (4096^3 584 us, 235 TFLOP/s and six times that of bfloat16
-// products, 0.86 of the measured peak; with eight warps 700 us), below by the chain of a stage: fetch, split, 24 products of at least 50
-// cycles, sums.  What it takes beside: 700 x 4096 x 1024 33 us (multiply-adds on CUDA cores 197; eight warps 44), 700 x 1024 x 2048 33
-// (102; 40), 900 x 1024 x 3072 46 (189; 54), 8 x 151936 x 1024 158 (387; 201), one row x 4096 x 1024 17 (18; 20).  Four stages are little beside
-// the kernel's start and end: one row x 1024 x 256 6.2 (5.3).  On single SMs (128 rows of w by 96) 62 us for the first, bound by the
-// operands' way from L2; arrivals on the pair's barriers with a release across the cluster wait for every load in flight (72 us).
+// Bound by the tensor cores from 192 columns on (4096^3 598 us, 230 TFLOP/s and six times that of bfloat16
+// products, 0.84 of the measured peak; with eight warps 700 us), below by the chain of a stage: fetch, split, 24 products of at least 50
+// cycles, sums.  What it takes beside: 700 x 4096 x 1024 33 us (multiply-adds on CUDA cores 197; eight warps 44), 700 x 1024 x 2048 35
+// (102; 40), 900 x 1024 x 3072 49 (189; 54), 8 x 151936 x 1024 163 (387; 201), one row x 4096 x 1024 17 (18; 20).  Four stages are little beside
+// the kernel's start and end: one row x 1024 x 256 6.5 (5.3), x 2048 x 512 10.6 (9.8).  On single SMs (128 rows of w by 96) 62 us for the first,
+// bound by the operands' way from L2.  The second SM's stages are announced by a thread of its own, which costs 1 to 3 %: its warps' own arrivals on the
+// other SM's barrier do not come behind their stores, and arrivals with a release across the cluster, by the warps or by that thread, cost
+// 500 cycles a stage (700 x 1024 x 2048 48 and 41 us).
 // Every wait is bounded and reports instead of hanging; tensor memory is given back on every path.
 #include "common.cuh"
 #include "mma.cuh"
@@ -190,7 +192,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmF32Shape<NT>::TH
     }
     float4 ahead[PER][2];
     // Up to 64 rows of x (in tiles of up to 64 columns) a stage is the time of its fetches, which is short from L2: w's rows are asked for that far
-    // ahead.  (One row x 4096 x 1024 19.6 -> 17.0 us, 64 x 1024 x 2048 34 -> 30; with more rows it costs 2 to 5 %.)
+    // ahead.  (One row x 4096 x 1024 19.6 -> 17.3 us, 64 x 1024 x 2048 34 -> 31; with more rows it costs 2 to 5 %.)
     auto ask = [&](int b) {
       if (a.M > 64) return;
 #pragma unroll
@@ -324,8 +326,8 @@ ZB_API int zb_gemm_nt_f32(float* y, const float* x, const float* w, int M, int N
   GemmF32Args a;
   a.y = y; a.x = x; a.w = w; a.M = M; a.N = N; a.K = K; a.ldx = ldx; a.ldw = ldw; a.ldy = ldy; a.status = status;
   // The tile whose rounds over the pairs of SMs take the least time (us of a full round at K = 1024, whatever K's share of it):
-  // 700 x 4096 x 1024 is one round of 64 pairs with 192 columns, 33 us (before the last change 35; 256: 49, 128: 48, 96: 45); 700 x 1024 x 2048 44
-  // pairs with 64, 33 (35; 32: 59, 96: 36); 2048 x 6144 x 1024 four rounds with 192, 129 (133; 256: 140, 128: 141); 8 x 151936 x 1024 with 32, 158.
+  // 700 x 4096 x 1024 is one round of 64 pairs with 192 columns, 35 us (256: 49, 128: 48, 96: 45); 700 x 1024 x 2048 44 pairs with 64,
+  // 35 (32: 59, 96: 36); 2048 x 6144 x 1024 four rounds with 192, 133 (256: 140, 128: 141), all at one time; 8 x 151936 x 1024 with 32, 163.
   struct Tile { int columns, us; };
   constexpr Tile tiles[] = {{32, 17}, {64, 19}, {96, 21}, {128, 23}, {160, 28}, {192, 32}, {256, 46}};
   const long long row_blocks = (N + 2LL * GF_ROWS - 1) / (2 * GF_ROWS);
