@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import contextlib
 import ctypes
+import functools
 import gc
 import math
 import os
@@ -881,14 +882,19 @@ def retention_turns(q: torch.Tensor, k: torch.Tensor, key_dim: int, rot_dims: in
             and all(t.stride(0) % 4 == 0 and t.data_ptr() % 16 == 0 for t in (q, k)))
 
 
+@functools.lru_cache(maxsize=64)
+def _retention_tc_supported(key_dim: int, value_dim: int, rot_dims: int) -> bool:
+    return bool(library().zb_retention_tc_supported(key_dim, value_dim, rot_dims))
+
+
 def retention_in_tensor_memory(rows: int, tokens: int, heads: int, key_dim: int, value_dim: int, rot_dims: int) -> bool:
     """True where retention's walk runs in pieces of 128 tokens on tcgen05 (csrc/retention_tc.cu): heads of 65 to 128 key channels, rows on
     16-byte boundaries, unless the walk in pieces of 64 has all its CTAs on the SMs at once and rows are long: its chain of a row is then the
     shorter one.  (us, here / there, heads of 128 x 128: 32 heads, rows of 1500 and 548 tokens 99 / 163, one of 2048 102 / 150, of 256 24 / 32,
     of 100 17 / 28; 16 heads, rows of 1400 and 600 73 / 99, eight of 128 36 / 56, one of 2048 87 / 82, of 1000 48 / 41, of 500 30 / 28; 8 heads,
     one row of 2048 81 / 62, of 700 37 / 32, of 300 25 / 28, two of 1024 49 / 41.)"""
-    return (bool(library().zb_retention_tc_supported(key_dim, value_dim, rot_dims))
-            and not (rows * heads * -(-value_dim // 16) <= _sm_count() and tokens >= 450 * rows))
+    return (_retention_tc_supported(key_dim, value_dim, rot_dims)
+            and not (tokens >= 450 * rows and rows * heads * -(-value_dim // 16) <= _sm_count()))
 
 
 def retention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, heads: int, key_dim: int, value_dim: int,

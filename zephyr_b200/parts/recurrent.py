@@ -304,23 +304,25 @@ def retention_walks(lengths: Sequence[int], heads: int, dim: int, vdim: int, ten
     (``tensor_memory``) is a CTA a row, head and 64 value columns: 8 us and 4.2 a piece, and what splits the operands.  That in pieces of 64
     is one of 16 columns: 1.25 us a piece of the longest row (1.05 with up to 64 key channels) and what prepares the pieces; nearly two CTAs
     an SM run in turn; CTAs of 32 columns, where they would be more, 2.7 us a piece.  The passes take a token and head's time for
-    padded channels, a row's state, and no less than 20.  (Walk / passes: 16 heads of 128 x 128, rows of 1024 and 1024 61 / 94, 1500 and
+    padded channels, a row's state, and no less than 20, or 23 and 27, as their launches from the host are three more.  (Walk / passes: 16 heads of 128 x 128, rows of 1024 and 1024 61 / 94, 1500 and
     three of 40 74 / 85, one of 2048 79 / 94; 32 heads, sixteen rows of 64 105 / 138; 8 heads, one of 2048 61 / 58, 1500 and 548 50 / 58, 1500 and ten
     of one 65 / 55; 4 heads, one of 1000 35 / 25; 16 heads of 64 x 128, one of 1000 29 / 41.)"""
-    tokens, longest, small = sum(lengths), max(lengths), dim <= 64
-    size = -(-dim // 64) * -(-vdim // 64) / 4
-    passes = max(19.5 if small else 22.5, 10.0 + 2.7e-3 * tokens * heads * (0.26 + 0.74 * size) + 0.05 * len(lengths) * heads * size)
+    tokens, least = sum(lengths), 23.0 if dim <= 64 else 27.0
     if tensor_memory:
-        ctas = [8.0 + 4.2 * -(-n // 128) for n in lengths]
-        return 4.0 + max(max(ctas), 1.15 * heads * -(-vdim // 64) * sum(ctas) / 148) + 3.5e-4 * tokens * heads <= passes
-    ctas, pieces = len(lengths) * heads * -(-vdim // 16), -(-longest // 64)
-    if ctas <= 1.5 * 148:
-        walked = 9.0 + 1.05 * pieces + 3e-4 * tokens * heads if small else 12.0 + 1.25 * pieces + 6.5e-4 * tokens * heads
-    elif ctas <= 2 * 148:
-        walked = 9.0 + 1.7 * sum(sorted(lengths)[-2:]) / 64
+        longest, ctas = 8.0 + 4.2 * -(-max(lengths) // 128), heads * -(-vdim // 64)
+        walked = 4.0 + 3.5e-4 * tokens * heads + max(longest, ctas * sum(8.0 + 4.2 * -(-n // 128) for n in lengths) / 128 if len(lengths) > 1 else 0.0)
     else:
-        walked = 9.0 + 2.7 * pieces
-    return walked <= passes
+        ctas, pieces = len(lengths) * heads * -(-vdim // 16), -(-max(lengths) // 64)
+        if ctas <= 1.5 * 148:
+            walked = 9.0 + 1.05 * pieces + 3e-4 * tokens * heads if dim <= 64 else 12.0 + 1.25 * pieces + 6.5e-4 * tokens * heads
+        elif ctas <= 2 * 148:
+            walked = 9.0 + 1.7 * sum(sorted(lengths)[-2:]) / 64
+        else:
+            walked = 9.0 + 2.7 * pieces
+    if walked <= least:
+        return True
+    size = -(-dim // 64) * -(-vdim // 64) / 4
+    return walked <= max(least, 10.0 + 2.7e-3 * tokens * heads * (0.26 + 0.74 * size) + 0.05 * len(lengths) * heads * size)
 
 
 class Retention(Mixer):
