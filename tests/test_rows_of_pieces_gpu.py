@@ -213,19 +213,13 @@ def test_a_sum_with_a_bias_is_the_sum_behind_the_bias(cuda_device, shape, out_dt
 def test_few_rows_take_the_faster_form(cuda_device, N, K, M, streams):
     """On both sides of the lines between the persistent kernel and the one with bursts (32 rows of the matrix a CTA up to 8 rows): the kernel that was
     the faster one when both were timed, near the exact sums, and the same bits where a row comes alone or with more."""
-    from torch.profiler import ProfilerActivity, profile
-
     from zephyr_b200.kernels import ops
 
     g = torch.Generator(device=cuda_device).manual_seed(N + K + M)
     x = torch.randn(M, K, generator=g, device=cuda_device).to(torch.bfloat16)
     w = (torch.randn(N, K, generator=g, device=cuda_device) / K ** 0.5).to(torch.bfloat16)
-    ops.gemm_small(x, w)
-    with profile(activities=[ProfilerActivity.CUDA]) as seen:
-        got = ops.gemm_small(x, w, out_dtype=torch.float32)
-        torch.cuda.synchronize()
-    names = [e.name for e in seen.events() if "gemm_small" in e.name]
-    assert len(names) == 1 and ("gemm_small_stream_kernel" in names[0]) == streams
+    assert ops.gemm_small_streams(M, N, K) == streams and not ops.gemm_small_streams(33, N, K)
+    got = ops.gemm_small(x, w, out_dtype=torch.float32)
     assert (got.double() - x.double() @ w.double().T).abs().max() <= 6 * 2.0 ** -24 * max(16.0, K ** 0.5)
     many = x.repeat(64 // M, 1)
     for rows in (1, 9, 17, 33):

@@ -512,6 +512,12 @@ ZB_API int zb_gemm_small_supported(int M, int N, int K) {
   return M >= 1 && M <= 8 * GS_MAX_MT && N >= 1 && K >= 8 && K % 8 == 0 ? 1 : 0;
 }
 
+// 1 if zb_gemm_small streams this problem's matrix through its persistent kernel.
+ZB_API int zb_gemm_small_streams(int M, int N, int K) {
+  if (!zb_gemm_small_supported(M, N, K) || M > 32) return 0;
+  return small_gemm_streams(N, K, M > 16 ? 4 : (M + 7) / 8, small_gemm_split(N, K)) ? 1 : 0;
+}
+
 // y = x w^T (swiglu = 0), or y[:, 8j + r] = silu(x w[16j + r]^T) * (x w[16j + 8 + r]^T) (swiglu = 1; 2: max(., 0) for silu;
 // w holds gate and up rows interleaved in blocks of 8, y has N / 2 columns).
 // x: [M, K] bfloat16 rows ldx apart (ldx, ldw multiples of 8, pointers 16-byte aligned);

@@ -203,6 +203,7 @@ _SIGNATURES = {
     "zb_paged_prefill_tc": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
                             c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p],
     "zb_gemm_small_supported": [c_int, c_int, c_int],
+    "zb_gemm_small_streams": [c_int, c_int, c_int],
     "zb_gemm_few_outputs": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int, c_void_p],
     "zb_gemm_small": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong, c_longlong, c_int,
                       c_int, c_void_p],
@@ -1814,6 +1815,11 @@ def _bounded_args(bounded: BoundedGate, rows: int) -> tuple:
     _require(bounded.limit > 0.0, "the bounded gate needs a positive limit")
     _f32_vector(bounded.bias, rows, "the gate's bias")
     return _ptr(bounded.bias), float(bounded.limit), float(bounded.alpha), float(bounded.shift)
+
+
+def gemm_small_streams(rows: int, outputs: int, k: int) -> bool:
+    """True where ``gemm_small`` streams a matrix of this size through its persistent kernel for that many rows."""
+    return bool(library().zb_gemm_small_streams(rows, outputs, k))
 
 
 def gemm_small(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype | None = None,
